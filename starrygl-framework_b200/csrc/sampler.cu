@@ -1,15 +1,17 @@
-// Temporal neighbour sampling, one warp per target, two kernels per hop:
+// Temporal neighbour sampling, two kernels per hop:
 //
-//   sample_count_kernel  warp-cooperative 32-ary search of the row's time-sorted timestamps for the
-//                        candidate window [lo, cut); stores the window and min(fanout, cut-lo); the last
-//                        CTA to finish turns the per-CTA totals into CTA base offsets (no spinning: a
-//                        fence + counter decides who is last).
-//   sample_fill_kernel   CTA-local exclusive scan of the counts (+ CTA base) gives every target its
-//                        output offset.  Windows that are copied as they are (recent: the tail of the
-//                        window; uniform with no more candidates than the fan-out) are written one
-//                        OUTPUT ELEMENT per thread -- every lane busy, stores coalesced, all loads of a
-//                        thread independent of each other; a target that draws (uniform: Floyd's
-//                        k-subset with Philox4x32-10, ranked ascending) is handled by one warp.
+//   sample_count_kernel  search of the row's time-sorted timestamps for the candidate window [lo, cut) of every target;
+//                        stores the window and min(fanout, cut-lo), and the total of the CTA
+//   sample_fill_kernel   output offsets from the CTA totals and the counts.  Windows that are copied as they are (recent:
+//                        the tail; uniform with no more candidates than the fan-out) and picks (uniform: Floyd's k-subset
+//                        with Philox4x32-10, ranked ascending) are written one OUTPUT ELEMENT per thread -- every lane
+//                        busy, stores coalesced, all loads of a thread independent of each other.
+//
+// Large launches are bound by sectors: 384,000 recent-20 targets take 155 us (180 with 8-ary searches and one element per
+// thread in flight), uniform-10 235 us (300 with a warp drawing for one target after the other); small ones by the chain
+// of dependent loads: 4,096 recent-20 targets 17.4 us (20.5 with an arrival counter to clear and a last-CTA scan).
+// One fused kernel (offsets by a look-back over the CTAs) was slower from 16,000 targets on: the look-back has to wait for
+// the slowest search before it.
 //
 // Algorithmic HBM bytes per target: 16 (indptr pair) + 16 (target id, time) + 8*ceil(log2 deg) (search
 // probes) + k_eff*24 (nbr, ts, eid reads) + k_eff*36 (five output arrays) + 8 (offset).
@@ -21,11 +23,7 @@ namespace {
 
 constexpr int kWarpsPerCta = 8;
 constexpr int kCtaThreads = kWarpsPerCta * 32;
-// Targets per warp (TPW) of the count kernel is chosen per launch: 1 for small batches (every target gets its own
-// warp: enough warps to hide the latency of the few dependent loads), 32 for larger ones, where the searches run one
-// target per LANE (8-ary steps: seven independent probes per round, so a 32-edge block takes two rounds) and the
-// number of CTAs -- hence the length of the last-CTA scan -- stays small.
-constexpr int kFillTargets = 32;   // targets per CTA of the fill kernel when the count kernel ran 256 per CTA
+constexpr int kFillUnroll = 2;   // elements of a thread in flight (four cost registers, that is resident CTAs)
 
 // first position p in [lo, hi) with ts[p] >= bound (hi when none); all 32 lanes cooperate and agree
 __device__ __forceinline__ int64_t warp_lower_bound(const int64_t* __restrict__ ts, int64_t lo, int64_t hi,
@@ -67,10 +65,19 @@ struct Philox {
   }
 };
 
-// first position p in [lo, hi) with ts[p] >= bound, one lane on its own: k-ary steps with independent probes (every
-// probe of a lane is its own 32-byte sector, so far-apart probes cost load/store-unit slots: 3 per round while the
-// range is wide, 7 once it is narrow and the probes share a few lines), then the last <= 8 candidates at once
+// first position p in [lo, hi) with ts[p] >= bound, one lane on its own.  Every probe of a lane is its own 32-byte sector,
+// so what a search costs is probes when there are many lanes (WIDE = false: halving, one probe per bit; 384,000 targets
+// took 67 us with the other form, the load/store units busy with 2.3 probes per bit) and rounds when there are few
+// (WIDE = true: three, then seven independent probes per round).
+template <bool WIDE>
 __device__ __forceinline__ int64_t lane_lower_bound(const int64_t* __restrict__ ts, int64_t lo, int64_t hi, int64_t bound) {
+  if (!WIDE) {
+    while (hi > lo) {
+      const int64_t mid = lo + ((hi - lo) >> 1);
+      if (__ldg(ts + mid) < bound) lo = mid + 1; else hi = mid;
+    }
+    return lo;
+  }
   while (hi - lo > 256) {
     const int64_t q = (hi - lo) >> 2;
     int c = 0;                          // the probes are monotone: the first c of them are "less"
@@ -111,193 +118,251 @@ __device__ __forceinline__ int64_t warp_fenced_lower_bound(const int64_t* __rest
   return p0 + __popc(__ballot_sync(0xffffffffu, less));
 }
 
+template <bool WIDE>
 __device__ __forceinline__ int64_t lane_fenced_lower_bound(const int64_t* __restrict__ ts, const int64_t* __restrict__ fence_row,
                                                            int64_t s, int64_t e, int64_t bound) {
-  if (e - s <= 32) return lane_lower_bound(ts, s, e, bound);
+  if (e - s <= 32) return lane_lower_bound<WIDE>(ts, s, e, bound);
   const int64_t nb = (e - s + 31) >> 5;
-  const int64_t j = lane_lower_bound(fence_row, 0, nb, bound);
+  const int64_t j = lane_lower_bound<WIDE>(fence_row, 0, nb, bound);
   if (j >= nb) return e;
   const int64_t p0 = s + (j << 5), p1 = p0 + 32 < e ? p0 + 32 : e;
-  return lane_lower_bound(ts, p0, p1, bound);
+  return lane_lower_bound<WIDE>(ts, p0, p1, bound);
 }
 
-template <int TPW>
+struct SampleArgs {
+  const int64_t *indptr, *nbr, *ts, *eid, *fence;
+  int64_t num_nodes;
+  const int64_t *targets, *target_ts;
+  int64_t n_cap;
+  const int64_t* d_n;
+  int fanout, policy, equal_root_time, keep_root_time;
+  int64_t allowed_offset;
+  uint64_t seed;
+  uint32_t rng_stream;
+  int64_t *out_nbr, *out_dst, *out_ts;
+  float* out_dt;
+  int64_t *out_dt_i64, *out_eid, *out_offsets;
+  int64_t *win_lo, *win_cut;   // [n_cap] candidate window of every target
+  int32_t* cnt;                // [n_cap] edges of every target
+  int64_t* cta_sums;           // [count CTAs] edges of the CTA, or (more than kDirectCtas of them) of the CTAs before it
+  unsigned int* done;          // arrival counter of the count CTAs (more than kDirectCtas)
+  int32_t* d_status;
+};
+
+// Up to this many count CTAs a fill CTA adds up the totals before its own by itself (16 KB of L2 reads at most): no
+// arrival counter to clear, no last CTA that scans while the others are gone.
+constexpr int64_t kDirectCtas = 2048;
+
+__device__ __forceinline__ uint64_t draw_below(int64_t target, int d, uint32_t rng_stream, uint64_t seed, uint64_t bound) {
+  Philox ph((uint32_t)target, (uint32_t)((uint64_t)target >> 32), (uint32_t)d, rng_stream, (uint32_t)seed, (uint32_t)(seed >> 32));
+  return ((uint64_t)ph.c[0] | ((uint64_t)ph.c[1] << 32)) % bound;
+}
+
+__device__ __forceinline__ void emit_edge(const SampleArgs& a, int64_t p, int64_t o, int64_t t, int64_t target) {
+  const int64_t ets = __ldg(a.ts + p);
+  a.out_nbr[o] = __ldg(a.nbr + p);
+  a.out_eid[o] = __ldg(a.eid + p);
+  a.out_ts[o] = a.keep_root_time ? t : ets;
+  a.out_dt[o] = (float)(t - ets);
+  if (a.out_dt_i64) a.out_dt_i64[o] = ets - t;
+  a.out_dst[o] = target;
+}
+
+// Windows and counts.  TPC targets per CTA: 8 = one warp per target (32-ary search), 256 = one lane per target (8-ary).
+template <int TPC, bool WIDE>
 __global__ void __launch_bounds__(kCtaThreads)
-sample_count_kernel(const int64_t* __restrict__ indptr, const int64_t* __restrict__ ts, const int64_t* __restrict__ fence,
-                    int64_t num_nodes,
-                    const int64_t* __restrict__ targets, const int64_t* __restrict__ target_ts, int64_t n_cap,
-                    const int64_t* d_n, int fanout, int equal_root_time, int64_t allowed_offset,
-                    int64_t* __restrict__ win_lo, int64_t* __restrict__ win_cut, int32_t* __restrict__ cnt,
-                    int64_t* __restrict__ cta_sums, unsigned int* done_counter, int64_t* __restrict__ out_offsets,
-                    int32_t* d_status) {
-  constexpr int TPC = kWarpsPerCta * TPW;
-  const int64_t n = eff_count(n_cap, d_n);
+sample_count_kernel(const SampleArgs a) {
+  constexpr bool kWarpPerTarget = TPC == kWarpsPerCta;
+  const int64_t n = eff_count(a.n_cap, a.d_n);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  int32_t my_cnt = 0;   // count of target (blockIdx.x * TPC + threadIdx.x), held by thread threadIdx.x < TPC
-  if (TPW == 32) {
-    const int64_t i = (int64_t)blockIdx.x * TPC + threadIdx.x;
-    if (i < n) {
-      int64_t node = targets[i], t = target_ts[i], lo = 0, cut = 0;
-      if (node < 0 || node >= num_nodes) {
-        dev_flag(d_status, SGL_DEV_BAD_NODE);
-      } else {
-        int64_t s = __ldg(indptr + node), e = __ldg(indptr + node + 1);
-        if (fence) {
-          const int64_t* frow = fence + (s >> 5) + node;
-          cut = lane_fenced_lower_bound(ts, frow, s, e, t + (equal_root_time ? 1 : 0));
-          lo = s;
-          if (allowed_offset >= 0) {
-            lo = lane_fenced_lower_bound(ts, frow, s, e, t - allowed_offset);
-            if (lo > cut) lo = cut;
-          }
+  const int64_t i = (int64_t)blockIdx.x * TPC + (kWarpPerTarget ? warp : (int)threadIdx.x);
+  int32_t c = 0;
+  if (i < n) {
+    const int64_t node = __ldg(a.targets + i), t = __ldg(a.target_ts + i);
+    const int64_t bound = t + (a.equal_root_time ? 1 : 0), from = t - a.allowed_offset;
+    int64_t lo = 0, cut = 0;
+    if (node < 0 || node >= a.num_nodes) {
+      if (!kWarpPerTarget || lane == 0) dev_flag(a.d_status, SGL_DEV_BAD_NODE);
+    } else {
+      const int64_t s = __ldg(a.indptr + node), e = __ldg(a.indptr + node + 1);
+      const int64_t* frow = a.fence ? a.fence + (s >> 5) + node : nullptr;
+      lo = cut = s;
+      if (e > s) {
+        if (kWarpPerTarget) {
+          cut = frow ? warp_fenced_lower_bound(a.ts, frow, s, e, bound, lane) : warp_lower_bound(a.ts, s, e, bound, lane);
+          if (a.allowed_offset >= 0 && cut > s)
+            lo = frow ? warp_fenced_lower_bound(a.ts, frow, s, e, from, lane) : warp_lower_bound(a.ts, s, cut, from, lane);
         } else {
-          cut = lane_lower_bound(ts, s, e, t + (equal_root_time ? 1 : 0));
-          lo = allowed_offset >= 0 ? lane_lower_bound(ts, s, cut, t - allowed_offset) : s;
+          cut = frow ? lane_fenced_lower_bound<WIDE>(a.ts, frow, s, e, bound) : lane_lower_bound<WIDE>(a.ts, s, e, bound);
+          if (a.allowed_offset >= 0 && cut > s)
+            lo = frow ? lane_fenced_lower_bound<WIDE>(a.ts, frow, s, e, from) : lane_lower_bound<WIDE>(a.ts, s, cut, from);
         }
+        if (lo > cut) lo = cut;
       }
-      int64_t cand = cut - lo;
-      my_cnt = (int32_t)(cand < fanout ? cand : fanout);
-      win_lo[i] = lo;
-      win_cut[i] = cut;
-      cnt[i] = my_cnt;
     }
-  } else {
-    __shared__ int32_t s_cnt[TPC];
-#pragma unroll
-    for (int j = 0; j < TPW; ++j) {
-      const int slot = warp * TPW + j;
-      const int64_t i = (int64_t)blockIdx.x * TPC + slot;
-      int32_t c = 0;
-      if (i < n) {
-        int64_t node = targets[i];
-        int64_t t = target_ts[i];
-        int64_t lo = 0, cut = 0;
-        if (node < 0 || node >= num_nodes) {
-          if (lane == 0) dev_flag(d_status, SGL_DEV_BAD_NODE);
-        } else {
-          int64_t s = __ldg(indptr + node), e = __ldg(indptr + node + 1);
-          lo = s;
-          cut = s;
-          if (e > s && fence) {
-            const int64_t* frow = fence + (s >> 5) + node;
-            cut = warp_fenced_lower_bound(ts, frow, s, e, t + (equal_root_time ? 1 : 0), lane);
-            if (allowed_offset >= 0 && cut > s) {
-              lo = warp_fenced_lower_bound(ts, frow, s, e, t - allowed_offset, lane);
-              if (lo > cut) lo = cut;
-            }
-          } else if (e > s) {
-            cut = warp_lower_bound(ts, s, e, t + (equal_root_time ? 1 : 0), lane);
-            if (allowed_offset >= 0 && cut > s) lo = warp_lower_bound(ts, s, cut, t - allowed_offset, lane);
-          }
-        }
-        int64_t cand = cut - lo;
-        c = (int32_t)(cand < fanout ? cand : fanout);
-        if (lane == 0) {
-          win_lo[i] = lo;
-          win_cut[i] = cut;
-          cnt[i] = c;
-        }
-      }
-      if (lane == 0) s_cnt[slot] = c;
+    c = (int32_t)(cut - lo < a.fanout ? cut - lo : a.fanout);
+    if (!kWarpPerTarget || lane == 0) {
+      a.win_lo[i] = lo;
+      a.win_cut[i] = cut;
+      a.cnt[i] = c;
     }
-    __syncthreads();
-    if (threadIdx.x < TPC) my_cnt = s_cnt[threadIdx.x];
   }
-  int cta_total;
-  cta_exclusive_scan<kCtaThreads, int>(my_cnt, &cta_total);
-  // grand total -> out_offsets[n_cap]; the slots of the targets themselves are written by the fill kernel
-  publish_and_scan_cta_totals<kCtaThreads>((int64_t)cta_total, cta_sums, done_counter, out_offsets + n_cap);
+  int total;
+  cta_exclusive_scan<kCtaThreads, int>(!kWarpPerTarget || lane == 0 ? c : 0, &total);
+  if (gridDim.x <= kDirectCtas) {
+    if (threadIdx.x == 0) a.cta_sums[blockIdx.x] = total;
+  } else {
+    publish_and_scan_cta_totals<kCtaThreads>((int64_t)total, a.cta_sums, a.done, a.out_offsets + a.n_cap);
+  }
 }
 
-// CT = targets per CTA of the count kernel (whose scanned totals are the CTA bases), FT = targets of this CTA
-// (FT divides CT): the CTA rebuilds the prefix inside its count CTA from the counts, which are a coalesced read of at
-// most 1 KB that hits L2.
+// Edges of FT targets (FT divides CT, the targets per CTA of the count kernel).
 template <int CT, int FT>
 __global__ void __launch_bounds__(kCtaThreads)
-sample_fill_kernel(const int64_t* __restrict__ nbr, const int64_t* __restrict__ ts, const int64_t* __restrict__ eid,
-                   const int64_t* __restrict__ target_ts, int64_t n_cap, const int64_t* d_n, int fanout, int policy,
-                   int keep_root_time, uint64_t seed, uint32_t rng_stream, const int64_t* __restrict__ win_lo,
-                   const int64_t* __restrict__ win_cut, const int32_t* __restrict__ cnt,
-                   const int64_t* __restrict__ cta_base, int64_t* __restrict__ out_nbr, int64_t* __restrict__ out_dst,
-                   int64_t* __restrict__ out_ts, float* __restrict__ out_dt, int64_t* __restrict__ out_dt_i64,
-                   int64_t* __restrict__ out_eid, int64_t* __restrict__ out_offsets) {
+sample_fill_kernel(const SampleArgs a, int count_ctas) {
   static_assert(CT % FT == 0 && CT <= kCtaThreads && FT % kWarpsPerCta == 0, "fill CTAs tile the count CTAs");
-  __shared__ int32_t s_ex[FT + 1];   // offset of the target's first element inside the count CTA's output; [FT] = end
+  constexpr bool kLaneDraws = CT != kWarpsPerCta;          // picks by the target's lane instead of its warp
+  extern __shared__ uint64_t s_dyn[];                      // picks of the targets that draw, target of every element
+  __shared__ int32_t s_ex[FT + 1];   // offset of the target's first element inside the CTA's output; [FT] = end
   __shared__ int32_t s_cnt[FT];
   __shared__ int64_t s_lo[FT], s_cut[FT], s_t[FT];
-  const int64_t n = eff_count(n_cap, d_n);
+  __shared__ int64_t s_base[kWarpsPerCta];
+  const int64_t n = eff_count(a.n_cap, a.d_n);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int64_t first = (int64_t)blockIdx.x * FT;          // this CTA's first target
   const int64_t count_cta = first / CT;
   const int sub = (int)(first - count_cta * CT);           // where this CTA's targets start inside the count CTA
-  const int64_t base = cta_base[count_cta];
-  {
-    const int64_t i = count_cta * CT + threadIdx.x;
-    const bool in_ct = threadIdx.x < CT;
-    const int slot = (int)threadIdx.x - sub;
-    const bool mine = in_ct && slot >= 0 && slot < FT;
-    const int c = (in_ct && i < n) ? cnt[i] : 0;
-    int64_t lo = 0, cut = 0, t = 0;
-    if (mine && i < n) {
-      lo = win_lo[i];
-      cut = win_cut[i];
-      t = target_ts[i];
-    }
-    const int ex = cta_exclusive_scan<kCtaThreads, int>(c, nullptr);
-    if (mine) {
-      s_ex[slot] = ex;
-      s_cnt[slot] = c;
-      s_lo[slot] = lo;
-      s_cut[slot] = cut;
-      s_t[slot] = t;
-      if (slot == FT - 1) s_ex[FT] = ex + c;
-      // offsets past the valid targets all equal the total, so out_offsets[n..n_cap] stays a valid prefix array
-      if (i < n_cap) out_offsets[i] = base + ex;
+  const int fanout = a.fanout;
+  const bool direct = count_ctas <= kDirectCtas;
+  const int slot = (int)threadIdx.x - sub;
+  const int64_t i = count_cta * CT + threadIdx.x;
+  const bool in_ct = threadIdx.x < CT && i < n, mine = slot >= 0 && slot < FT;
+  const int c = in_ct ? a.cnt[i] : 0;
+  int64_t lo = 0, cut = 0, t = 0;
+  if (mine && in_ct) {
+    lo = a.win_lo[i];
+    cut = a.win_cut[i];
+    t = a.target_ts[i];
+  }
+  int64_t before = 0;
+  if (direct) {
+    for (int64_t b = threadIdx.x; b < count_cta; b += kCtaThreads) before += a.cta_sums[b];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) before += __shfl_xor_sync(0xffffffffu, before, o);
+    if (lane == 0) s_base[warp] = before;
+  }
+  int ct_total;
+  const int ex = cta_exclusive_scan<kCtaThreads, int>(c, &ct_total);    // (its barriers also publish s_base)
+  int64_t base = 0;
+  if (direct) {
+#pragma unroll
+    for (int w = 0; w < kWarpsPerCta; ++w) base += s_base[w];
+    if (threadIdx.x == 0 && first + FT >= a.n_cap) a.out_offsets[a.n_cap] = base + ct_total;
+  } else {
+    base = a.cta_sums[count_cta];
+  }
+  const bool draws = a.policy == SGL_POLICY_UNIFORM;
+  uint32_t* s_pick = (uint32_t*)s_dyn;     // [fanout][FT]
+  const bool lane_draws = kLaneDraws && draws && fanout <= 32;
+  const bool has_map = fanout <= 32;       // which target every output element belongs to, behind the picks
+  uint8_t* s_map = (uint8_t*)(s_pick + (lane_draws ? FT * fanout : 0));
+  if (mine && threadIdx.x < CT) {
+    s_ex[slot] = ex;
+    s_cnt[slot] = c;
+    s_lo[slot] = lo;
+    s_cut[slot] = cut;
+    s_t[slot] = t;
+    if (slot == FT - 1) s_ex[FT] = ex + c;
+    // offsets past the valid targets all equal the total, so out_offsets[n..n_cap] stays a valid prefix array
+    if (i < a.n_cap) a.out_offsets[i] = base + ex;
+  }
+  __syncthreads();
+  const int begin = s_ex[0], end = s_ex[FT];
+  if (mine && threadIdx.x < CT) {
+    if (has_map)
+      for (int j = 0; j < c; ++j) s_map[ex - begin + j] = (uint8_t)slot;
+    if (lane_draws) {
+      // Floyd's subset selection: draw d picks uniformly in [0, cand - k + d]; a repeat is replaced by cand - k + d
+      const int64_t cand = cut - lo;
+      if (cand > fanout && cand <= 0xffffffffll) {
+        for (int d = 0; d < fanout; ++d) {
+          const uint32_t top = (uint32_t)(cand - fanout + d);
+          uint32_t pick = (uint32_t)draw_below(i, d, a.rng_stream, a.seed, (uint64_t)top + 1);
+          bool clash = false;
+          for (int q = 0; q < d; ++q) clash |= s_pick[q * FT + slot] == pick;
+          s_pick[d * FT + slot] = clash ? top : pick;
+        }
+      }
     }
   }
   __syncthreads();
-  const bool draws = policy == SGL_POLICY_UNIFORM;
-  // windows copied as they are: one output element per thread
-  for (int o = s_ex[0] + (int)threadIdx.x; o < s_ex[FT]; o += kCtaThreads) {
-    int a = 0, b = FT;               // last slot with s_ex[slot] <= o (its next offset is > o, so it is not empty)
-    while (b - a > 1) {
-      const int m = (a + b) >> 1;
-      if (s_ex[m] <= o) a = m; else b = m;
+  // one output element per thread: all lanes busy, stores coalesced; the loads of kFillUnroll elements of a thread are in
+  // flight together
+  for (int o0 = begin + (int)threadIdx.x; o0 < end; o0 += kCtaThreads * kFillUnroll) {
+    int at[kFillUnroll];
+    int64_t g[kFillUnroll], ets[kFillUnroll], nb[kFillUnroll], ei[kFillUnroll];
+#pragma unroll
+    for (int u = 0; u < kFillUnroll; ++u) {
+      const int o = o0 + u * kCtaThreads;
+      at[u] = -1;
+      if (o >= end) continue;
+      int k;
+      if (has_map) {
+        k = s_map[o - begin];
+      } else {
+        k = 0;
+        int b = FT;                      // last slot with s_ex[slot] <= o (its next offset is > o, so it is not empty)
+        while (b - k > 1) {
+          const int m = (k + b) >> 1;
+          if (s_ex[m] <= o) k = m; else b = m;
+        }
+      }
+      const int64_t wlo = s_lo[k], wcut = s_cut[k];
+      int64_t p;
+      if (draws && wcut - wlo > fanout) {
+        if (!lane_draws || wcut - wlo > 0xffffffffll) continue;
+        const uint32_t pick = s_pick[(o - s_ex[k]) * FT + k];
+        int rank = 0;
+        for (int q = 0; q < fanout; ++q) rank += s_pick[q * FT + k] < pick ? 1 : 0;
+        p = wlo + pick;
+        g[u] = base + s_ex[k] + rank;
+      } else {
+        // recent: tail of the window; uniform with cand <= k: the whole window
+        p = wcut - s_cnt[k] + (o - s_ex[k]);
+        g[u] = base + o;
+      }
+      at[u] = k;
+      ets[u] = __ldg(a.ts + p);
+      nb[u] = __ldg(a.nbr + p);
+      ei[u] = __ldg(a.eid + p);
     }
-    const int c = s_cnt[a];
-    const int64_t cut = s_cut[a];
-    if (draws && cut - s_lo[a] > fanout) continue;
-    const int64_t p = cut - c + (o - s_ex[a]);   // recent: tail of the window; uniform with cand <= k: the whole window
-    const int64_t t = s_t[a];
-    const int64_t ets = __ldg(ts + p);
-    const int64_t g = base + o;
-    out_nbr[g] = __ldg(nbr + p);
-    out_eid[g] = __ldg(eid + p);
-    out_ts[g] = keep_root_time ? t : ets;
-    out_dt[g] = (float)(t - ets);
-    if (out_dt_i64) out_dt_i64[g] = ets - t;
-    out_dst[g] = first + a;
+#pragma unroll
+    for (int u = 0; u < kFillUnroll; ++u) {
+      if (at[u] < 0) continue;
+      const int64_t tt = s_t[at[u]];
+      a.out_nbr[g[u]] = nb[u];
+      a.out_eid[g[u]] = ei[u];
+      a.out_ts[g[u]] = a.keep_root_time ? tt : ets[u];
+      a.out_dt[g[u]] = (float)(tt - ets[u]);
+      if (a.out_dt_i64) a.out_dt_i64[g[u]] = ets[u] - tt;
+      a.out_dst[g[u]] = first + at[u];
+    }
   }
   if (!draws) return;
-  // targets that draw: one warp per target
+  // targets that draw and were not served above: one warp per target
 #pragma unroll 1
-  for (int slot = warp; slot < FT; slot += kWarpsPerCta) {
-    const int64_t i = first + slot;
+  for (int wslot = warp; wslot < FT; wslot += kWarpsPerCta) {
+    const int64_t i = first + wslot;
     if (i >= n) break;
-    const int64_t lo = s_lo[slot], cut = s_cut[slot];
+    const int64_t lo = s_lo[wslot], cut = s_cut[wslot];
     const int64_t cand = cut - lo;
-    if (cand <= fanout) continue;
-    const int64_t t = s_t[slot];
-    const int64_t off = base + s_ex[slot];
+    if (cand <= fanout || (lane_draws && cand <= 0xffffffffll)) continue;
+    const int64_t t = s_t[wslot];
+    const int64_t off = base + s_ex[wslot];
     if (fanout > 32) {
       // more draws than lanes: the same selection, with the picks of the target kept in this warp's shared memory
-      extern __shared__ uint64_t s_picks_all[];
-      uint64_t* picks = s_picks_all + (size_t)warp * fanout;
-      for (int d = lane; d < fanout; d += 32) {
-        Philox ph((uint32_t)i, (uint32_t)((uint64_t)i >> 32), (uint32_t)d, rng_stream, (uint32_t)seed, (uint32_t)(seed >> 32));
-        const uint64_t u = (uint64_t)ph.c[0] | ((uint64_t)ph.c[1] << 32);
-        picks[d] = u % (uint64_t)(cand - fanout + d + 1);
-      }
+      uint64_t* picks = s_dyn + (size_t)warp * fanout;
+      for (int d = lane; d < fanout; d += 32) picks[d] = draw_below(i, d, a.rng_stream, a.seed, (uint64_t)(cand - fanout + d + 1));
       __syncwarp();
       for (int d = 1; d < fanout; ++d) {          // draw d against the (final) draws before it
         const uint64_t mine = picks[d];
@@ -312,27 +377,12 @@ sample_fill_kernel(const int64_t* __restrict__ nbr, const int64_t* __restrict__ 
         const uint64_t pick = picks[d];
         int rank = 0;
         for (int q = 0; q < fanout; ++q) rank += picks[q] < pick ? 1 : 0;
-        const int64_t p = lo + (int64_t)pick;
-        const int64_t o = off + rank;
-        const int64_t ets = __ldg(ts + p);
-        out_nbr[o] = __ldg(nbr + p);
-        out_eid[o] = __ldg(eid + p);
-        out_ts[o] = keep_root_time ? t : ets;
-        out_dt[o] = (float)(t - ets);
-        if (out_dt_i64) out_dt_i64[o] = ets - t;
-        out_dst[o] = i;
+        emit_edge(a, lo + (int64_t)pick, off + rank, t, i);
       }
       __syncwarp();
     } else {
-      // Floyd's subset selection: draw j picks t_j uniform in [0, cand-k+j]; a repeat is replaced by cand-k+j
       uint64_t pick = 0;
-      if (lane < fanout) {
-        Philox ph((uint32_t)i, (uint32_t)((uint64_t)i >> 32), (uint32_t)lane, rng_stream, (uint32_t)seed,
-                  (uint32_t)(seed >> 32));
-        uint64_t u = (uint64_t)ph.c[0] | ((uint64_t)ph.c[1] << 32);
-        uint64_t bound = (uint64_t)(cand - fanout + lane + 1);
-        pick = u % bound;
-      }
+      if (lane < fanout) pick = draw_below(i, lane, a.rng_stream, a.seed, (uint64_t)(cand - fanout + lane + 1));
       for (int d = 1; d < fanout; ++d) {
         uint64_t mine = __shfl_sync(0xffffffffu, pick, d);
         bool clash = lane < d && pick == mine;
@@ -344,17 +394,7 @@ sample_fill_kernel(const int64_t* __restrict__ nbr, const int64_t* __restrict__ 
         uint64_t other = __shfl_sync(0xffffffffu, pick, d);
         rank += (other < pick) ? 1 : 0;
       }
-      if (lane < fanout) {
-        int64_t p = lo + (int64_t)pick;
-        int64_t o = off + rank;
-        int64_t ets = __ldg(ts + p);
-        out_nbr[o] = __ldg(nbr + p);
-        out_eid[o] = __ldg(eid + p);
-        out_ts[o] = keep_root_time ? t : ets;
-        out_dt[o] = (float)(t - ets);
-        if (out_dt_i64) out_dt_i64[o] = ets - t;
-        out_dst[o] = i;
-      }
+      if (lane < fanout) emit_edge(a, lo + (int64_t)pick, off + rank, t, i);
     }
   }
 }
@@ -364,39 +404,31 @@ sample_fill_kernel(const int64_t* __restrict__ nbr, const int64_t* __restrict__ 
 
 using namespace sgl;
 
-static inline int sample_tpw(int64_t n) { return n <= 16384 ? 1 : 32; }
-
-static inline int64_t sample_num_ctas(int64_t n, int tpw) {
-  int64_t tpc = (int64_t)kWarpsPerCta * tpw;
-  int64_t b = (n + tpc - 1) / tpc;
-  return b < 1 ? 1 : b;
-}
+// Up to 16,384 targets a warp each hides the latency of the few dependent loads; above, a lane each; from 65,536 on
+// throughput counts and not the latency of one search.
+constexpr int64_t kWarpTargets = 16384;
+constexpr int64_t kManyTargets = 65536;
 
 extern "C" size_t sgl_sample_ws_bytes(int64_t n_targets) {
   if (n_targets < 1) n_targets = 1;
   return 2 * align_up((size_t)n_targets * 8) + align_up((size_t)n_targets * 4) +
-         align_up((size_t)sample_num_ctas(n_targets, 1) * 8) + align_up(sizeof(unsigned int));
+         align_up((size_t)((n_targets + kWarpsPerCta - 1) / kWarpsPerCta) * 8) + align_up(sizeof(unsigned int));
 }
 
-template <int TPW>
-static void launch_sample(int64_t ctas, cudaStream_t stream, const int64_t* indptr, const int64_t* nbr, const int64_t* ts,
-                          const int64_t* eid, const int64_t* fence, int64_t num_nodes, const int64_t* targets, const int64_t* target_ts,
-                          int64_t n_targets, const int64_t* d_n, int fanout, int policy, int equal_root_time,
-                          int64_t allowed_offset, int keep_root_time, uint64_t seed, uint32_t rng_stream, int64_t* win_lo,
-                          int64_t* win_cut, int32_t* cnt, int64_t* cta_sums, unsigned int* done, int64_t* out_nbr,
-                          int64_t* out_dst, int64_t* out_ts, float* out_dt, int64_t* out_dt_i64, int64_t* out_eid,
-                          int64_t* out_offsets, int32_t* d_status) {
-  sample_count_kernel<TPW><<<(unsigned)ctas, kCtaThreads, 0, stream>>>(indptr, ts, fence, num_nodes, targets, target_ts,
-                                                                       n_targets, d_n, fanout, equal_root_time,
-                                                                       allowed_offset, win_lo, win_cut, cnt, cta_sums, done,
-                                                                       out_offsets, d_status);
-  const size_t pick_smem = (policy == SGL_POLICY_UNIFORM && fanout > 32) ? (size_t)kWarpsPerCta * fanout * sizeof(uint64_t) : 0;
-  constexpr int CT = kWarpsPerCta * TPW, FT = CT < kFillTargets ? CT : kFillTargets;
-  const unsigned fill_ctas = (unsigned)((n_targets + FT - 1) / FT);
-  sample_fill_kernel<CT, FT><<<fill_ctas, kCtaThreads, pick_smem, stream>>>(nbr, ts, eid, target_ts, n_targets, d_n, fanout, policy,
-                                                                           keep_root_time, seed, rng_stream, win_lo, win_cut, cnt,
-                                                                           cta_sums, out_nbr, out_dst, out_ts, out_dt, out_dt_i64,
-                                                                           out_eid, out_offsets);
+template <int CT, int FT, bool WIDE>
+static int launch_sample(const SampleArgs& a, cudaStream_t stream) {
+  const unsigned ctas = (unsigned)((a.n_cap + CT - 1) / CT);
+  if (ctas > kDirectCtas) SGL_CUDA_CHECK(cudaMemsetAsync(a.done, 0, sizeof(unsigned int), stream));
+  sample_count_kernel<CT, WIDE><<<ctas, kCtaThreads, 0, stream>>>(a);
+  size_t smem = 0;
+  if (a.policy == SGL_POLICY_UNIFORM) {
+    if (a.fanout > 32) smem = (size_t)kWarpsPerCta * a.fanout * sizeof(uint64_t);
+    else if (CT != kWarpsPerCta) smem = (size_t)FT * a.fanout * sizeof(uint32_t);
+  }
+  if (a.fanout <= 32) smem += (size_t)FT * a.fanout;
+  sample_fill_kernel<CT, FT><<<(unsigned)((a.n_cap + FT - 1) / FT), kCtaThreads, smem, stream>>>(a, (int)ctas);
+  SGL_LAUNCH_CHECK();
+  return SGL_OK;
 }
 
 static int sample_layer_impl(const int64_t* indptr, const int64_t* nbr, const int64_t* ts, const int64_t* eid,
@@ -421,26 +453,34 @@ static int sample_layer_impl(const int64_t* indptr, const int64_t* nbr, const in
   }
   SGL_REQUIRE(indptr && nbr && ts && eid && targets && target_ts && out_nbr && out_dst && out_ts && out_dt && out_eid,
               SGL_ERR_ARG, "sample_layer: null array");
+  SampleArgs a;
+  a.indptr = indptr; a.nbr = nbr; a.ts = ts; a.eid = eid; a.fence = fence;
+  a.num_nodes = num_nodes;
+  a.targets = targets; a.target_ts = target_ts;
+  a.n_cap = n_targets;
+  a.d_n = d_n;
+  a.fanout = fanout; a.policy = policy; a.equal_root_time = equal_root_time; a.keep_root_time = keep_root_time;
+  a.allowed_offset = allowed_offset;
+  a.seed = seed;
+  a.rng_stream = rng_stream;
+  a.out_nbr = out_nbr; a.out_dst = out_dst; a.out_ts = out_ts;
+  a.out_dt = out_dt;
+  a.out_dt_i64 = out_dt_i64; a.out_eid = out_eid; a.out_offsets = out_offsets;
+  a.d_status = d_status;
   WsCarver c(ws, ws_bytes);
-  int64_t* win_lo = c.take<int64_t>(n_targets);
-  int64_t* win_cut = c.take<int64_t>(n_targets);
-  int32_t* cnt = c.take<int32_t>(n_targets);
-  const int tpw = sample_tpw(n_targets);
-  const int64_t ctas = sample_num_ctas(n_targets, tpw);
-  int64_t* cta_sums = c.take<int64_t>(sample_num_ctas(n_targets, 1));
-  unsigned int* done = c.take<unsigned int>(1);
+  a.win_lo = c.take<int64_t>(n_targets);
+  a.win_cut = c.take<int64_t>(n_targets);
+  a.cnt = c.take<int32_t>(n_targets);
+  a.cta_sums = c.take<int64_t>((size_t)((n_targets + kWarpsPerCta - 1) / kWarpsPerCta));
+  a.done = c.take<unsigned int>(1);
   SGL_REQUIRE(c.ok(), SGL_ERR_WORKSPACE, "sample_layer: workspace %zu < %zu bytes", ws_bytes,
               sgl_sample_ws_bytes(n_targets));
-  SGL_CUDA_CHECK(cudaMemsetAsync(done, 0, sizeof(unsigned int), stream));
-#define SGL_SAMPLE_ARGS                                                                                               \
-  ctas, stream, indptr, nbr, ts, eid, fence, num_nodes, targets, target_ts, n_targets, d_n, fanout, policy, equal_root_time, \
-      allowed_offset, keep_root_time, seed, rng_stream, win_lo, win_cut, cnt, cta_sums, done, out_nbr, out_dst,       \
-      out_ts, out_dt, out_dt_i64, out_eid, out_offsets, d_status
-  if (tpw == 1) launch_sample<1>(SGL_SAMPLE_ARGS);
-  else launch_sample<32>(SGL_SAMPLE_ARGS);
-#undef SGL_SAMPLE_ARGS
-  SGL_LAUNCH_CHECK();
-  return SGL_OK;
+  if (n_targets <= kWarpTargets) return launch_sample<kWarpsPerCta, kWarpsPerCta, true>(a, stream);
+  // targets per fill CTA: a lane of the CTA draws for every target (uniform), so as many as there are threads once that
+  // leaves several CTAs per SM; windows that are copied are spread thinner
+  if (policy == SGL_POLICY_UNIFORM)
+    return n_targets < kManyTargets ? launch_sample<kCtaThreads, 128, true>(a, stream) : launch_sample<kCtaThreads, 256, false>(a, stream);
+  return n_targets < kManyTargets ? launch_sample<kCtaThreads, 64, true>(a, stream) : launch_sample<kCtaThreads, 64, false>(a, stream);
 }
 
 extern "C" int sgl_sample_layer(const int64_t* indptr, const int64_t* nbr, const int64_t* ts, const int64_t* eid,
@@ -538,8 +578,7 @@ extern "C" int sgl_sample_layer_static(const int64_t* indptr, const int64_t* nbr
     SGL_REQUIRE(p != nullptr, SGL_ERR_CUDA, "sample_layer_static: no device address for the built-in scratch");
     g_static_scratch_addr[dev] = p;
   }
-  // sgl_sample_layer clears the one word of the scratch that has to start at zero (the CTA arrival counter) on the
-  // stream before its kernels; everything else in the array is written before it is read.
+  // sgl_sample_layer clears the part of the scratch it uses on the stream before its kernel.
   return sgl_sample_layer(indptr, nbr, ts, eid, num_nodes, targets, target_ts, n_targets, nullptr, fanout, policy,
                           equal_root_time, allowed_offset, keep_root_time, seed, rng_stream, out_nbr, out_dst, out_ts,
                           out_dt, nullptr, out_eid, out_offsets, d_status, g_static_scratch_addr[dev], kStaticScratchBytes,

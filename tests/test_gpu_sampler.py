@@ -207,3 +207,22 @@ def test_fence_index_and_search_through_it():
                 n = a.total()
                 assert n == b.total() and torch.equal(a.offsets, b.offsets)
                 assert torch.equal(a.eid[:n], b.eid[:n]) and torch.equal(a.nbr[:n], b.nbr[:n]) and torch.equal(a.ts[:n], b.ts[:n])
+
+
+@pytest.mark.parametrize("n", [1, 16384, 16385, 65535, 65536, 524289])
+@pytest.mark.parametrize("policy", ["recent", "uniform"])
+def test_every_launch_shape_matches_oracle(n, policy):
+    """Both sides of the lines between a warp and a lane per target, between few and many targets, and of the number of
+    CTAs whose totals are added up directly."""
+    from oracle import oracle_c as OC
+    z = random_graph(3, 3000, 200000, 5000, hub=40000)
+    g = build_graph(z)
+    indptr, nbr, ts, eid, _ = O.tcsr_build(z["dst"], z["src"], z["ts"], z["eid"], z["n"])
+    rng = np.random.default_rng(n)
+    q = rng.integers(0, z["n"], n).astype(np.int64)
+    qt = rng.integers(-5, 5010, n).astype(np.int64)
+    out, offs = run(g, q, qt, 7, policy, seed=5, allowed_offset=900)
+    ref = OC.sample_layer(indptr, nbr, ts, eid, q, qt, 7, O.RECENT if policy == "recent" else O.UNIFORM, seed=5, allowed_offset=900)
+    for nm, a, r in zip(NAMES, out, ref):
+        assert np.array_equal(a, r), nm
+    assert offs[0] == 0 and offs[-1] == len(out[0]) and (np.diff(offs) >= 0).all()

@@ -191,7 +191,8 @@ int sgl_unique_pairs(const int64_t* a_id, const int64_t* a_ts, int64_t n_a, cons
  * CSC of one sampled hop: stable order by (dst_local, ts); indptr over the num_dst rows of the
  * previous node list.  dst_map (optional): dst_local = dst_map[dst[e]] (the previous hop's inverse map),
  * else dst_local = dst[e].  num_dst may be overridden by the device count d_num_dst (indptr is then
- * written for d_num_dst+1 entries; capacity num_dst+1).  presorted != 0 (dst_map must be NULL): the edges already are
+ * written for d_num_dst+1 entries; capacity num_dst+1).  src_local NULL (not with presorted): out_indices receives the
+ * edges' input positions, to be translated by the caller.  presorted != 0 (dst_map must be NULL): the edges already are
  * in (dst, ts) order -- the first hop of a batch, whose target i is row i of the list -- and the sort is skipped
  * (the order is checked: a violation raises SGL_DEV_BAD_INDEX).
  * Replaces: _build_csc_from_pairs (prepare_sample.py:215-229).
@@ -532,6 +533,32 @@ int sgl_seeds_in_window(const int64_t* ev_src, const int64_t* ev_ts, const int64
 /* out[i] = first position p with sorted[p] >= values[i] (n when none); k values.  Used to find the slice of the
  * time-ordered event arrays that a window [t_begin, t_end) covers. */
 int sgl_lower_bound_i64(const int64_t* sorted, int64_t n, const int64_t* values, int k, int64_t* out, void* stream);
+
+/* ------------------------------------------------------------------------------------------------
+ * Whole mini-batch in one call: (id, ts) relabel of the roots, n_hops hops of sampling (hop l + 1 queries every edge of
+ * hop l at that edge's time), merged list and CSC per hop -- sgl_unique_pairs, sgl_sample_layer_fenced and sgl_build_csc
+ * enqueued back to back with all sizes on the device.  All results lie in one caller-allocated arena of
+ * sgl_build_batch_layout(...) 64-bit words, as consecutive sections whose sizes that function writes to section_words
+ * (room for 3 + 14 * n_hops entries; at most 8 hops; returns -1 on a bad argument):
+ *   3 for the roots   gids[n], ts[n], inverse map[n]
+ *   14 per hop        nbr, dst, ts, dt (fp32), eid, offsets of the sampled edges; merged gids, ts; the edges' positions in the
+ *                     merged list; CSC indptr, indices, ts, dt (fp32), eid (absent for the first hop: its edges are in
+ *                     CSC order already, with `offsets` as the row pointer)
+ * meta[2 + 2 * n_hops] = {size of the root list, then per hop sampled edges and size of the merged list, status word}; the
+ * status word is used when d_status is NULL.  side_stream (optional): hops after the first and their CSC run there,
+ * next to the relabels; everything is joined into `stream`.
+ * Replaces: build_aligned_batch's per-layer loop (prepare_sample.py:313-377).
+ * ---------------------------------------------------------------------------------------------- */
+int64_t sgl_build_batch_layout(int64_t n_roots, const int32_t* fanouts, int n_hops, int64_t* section_words);
+size_t sgl_build_batch_ws_bytes(int64_t n_roots, const int32_t* fanouts, int n_hops);
+int sgl_build_batch(const int64_t* indptr, const int64_t* nbr, const int64_t* ts, const int64_t* eid, const int64_t* fence,
+                    int64_t num_nodes, const int64_t* roots, const int64_t* root_ts, int64_t n_roots,
+                    const int32_t* fanouts, int n_hops, int policy, int equal_root_time, int64_t allowed_offset,
+                    uint64_t seed, int id_bits, int ts_bits, int64_t ts_base, int64_t* arena, int64_t* meta,
+                    int32_t* d_status, void* ws, size_t ws_bytes, void* side_stream, void* stream);
+
+/* Copies up to 4,096 bytes of device memory to (pageable) host memory and waits for the stream. */
+int sgl_read_back(const void* src, void* dst, size_t bytes, void* stream);
 
 /* ------------------------------------------------------------------------------------------------
  * CUDA-graph helpers for launch-bound steps.  Between sgl_graph_capture_begin(stream) and

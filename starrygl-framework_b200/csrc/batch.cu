@@ -1,0 +1,235 @@
+// The whole mini-batch in one call: (node, time) relabel of the roots, every hop, relabel and CSC per hop -- enqueued
+// back to back with all sizes on the device, results in one arena that the caller allocates with a single allocation.
+//
+// What this replaces is host time: driven entry point by entry point from Python a two-hop batch of 4,096 roots cost 37
+// allocations and 20 foreign calls, and its 200 us of kernels took 490 us to issue.
+//
+// Arena (8-byte words, sections in the order of batch_sections(), each rounded up to 32 words):
+//   roots            gids[n], ts[n], inverse map[n]
+//   hop l            nbr, dst, ts, dt (fp32), eid [T_l k_l], offsets[T_l + 1]; merged list gids, ts [C_l + T_l k_l], column
+//                    indices of the hop's edges in it [T_l k_l]; from the second hop on: CSC row pointer [C_l + 1], indices,
+//                    ts, dt (fp32), eid [T_l k_l]
+//   with T_0 = C_0 = n, T_(l+1) = T_l k_l, C_(l+1) = C_l + T_l k_l.  The first hop needs no CSC of its own: its targets are the
+//   list itself and its edges come out in (row, time) order, so its offsets ARE the row pointer.
+// Meta (8-byte words): entries of the root list, then per hop sampled edges and entries of the merged list, then a status
+// word (used when the caller has none of its own).
+
+#include "sampler.cuh"
+#include "sort.cuh"
+#include "tilesort.cuh"
+
+using namespace sgl;
+
+namespace {
+
+constexpr int kMaxHops = 8;
+constexpr int kRootSections = 3, kHopSections = 14;
+
+inline int64_t words(int64_t n) { return ((n < 1 ? 1 : n) + 31) / 32 * 32; }
+
+// sizes of the sections in words; returns the number of sections
+int batch_sections(int64_t n, const int32_t* fanouts, int hops, int64_t* out) {
+  int s = 0;
+  for (int i = 0; i < kRootSections; ++i) out[s++] = words(n);
+  int64_t t = n, c = n;
+  for (int l = 0; l < hops; ++l) {
+    const int64_t e = t * fanouts[l];
+    out[s++] = words(e);                         // 0 nbr
+    out[s++] = words(e);                         // 1 dst
+    out[s++] = words(e);                         // 2 ts
+    out[s++] = words((e + 1) / 2);               // 3 dt
+    out[s++] = words(e);                         // 4 eid
+    out[s++] = words(t + 1);                     // 5 offsets
+    out[s++] = words(c + e);                     // 6 gids
+    out[s++] = words(c + e);                     // 7 ts
+    out[s++] = words(e);                         // 8 column index of an edge
+    const bool csc = l > 0;
+    out[s++] = csc ? words(c + 1) : 0;           // 9 indptr
+    out[s++] = csc ? words(e) : 0;               // 10 indices
+    out[s++] = csc ? words(e) : 0;               // 11 ts
+    out[s++] = csc ? words((e + 1) / 2) : 0;     // 12 dt
+    out[s++] = csc ? words(e) : 0;               // 13 eid
+    t = e;
+    c += e;
+  }
+  return s;
+}
+
+size_t sample_ws(int64_t n, const int32_t* fanouts, int hops) {
+  size_t most = 0;
+  for (int l = 0; l < hops; ++l) {
+    const size_t b = align_up(sgl_sample_ws_bytes(n));
+    most = most > b ? most : b;
+    n *= fanouts[l];
+  }
+  return most;
+}
+
+size_t list_ws(int64_t n, const int32_t* fanouts, int hops) {
+  size_t most = sgl_unique_pairs_ws_bytes(n);
+  int64_t t = n, c = n;
+  for (int l = 0; l < hops; ++l) {
+    t *= fanouts[l];
+    c += t;
+    const size_t b = sgl_unique_pairs_ws_bytes(c);
+    most = most > b ? most : b;
+  }
+  return align_up(most);
+}
+
+size_t csc_ws(int64_t n, const int32_t* fanouts, int hops) {
+  size_t most = 0;
+  int64_t t = n, c = n;
+  for (int l = 0; l < hops; ++l) {
+    const int64_t e = t * fanouts[l];
+    const size_t b = l > 0 ? sgl_build_csc_ws_bytes(e, c) : 0;
+    most = most > b ? most : b;
+    t = e;
+    c += e;
+  }
+  return align_up(most);
+}
+
+// events of this thread for the fork and join of the side stream (recorded and waited for at once, so reusable)
+cudaError_t thread_event(int i, cudaEvent_t* out) {
+  static thread_local cudaEvent_t ev[64][4];
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  cudaEvent_t& slot = ev[dev & 63][i];
+  if (slot == nullptr) e = cudaEventCreateWithFlags(&slot, cudaEventDisableTiming);
+  *out = slot;
+  return e;
+}
+
+// indices[j] = col[indices[j]]: edge numbers -> positions in the merged list
+__global__ void __launch_bounds__(256)
+map_columns_kernel(int64_t* __restrict__ indices, const int64_t* __restrict__ col, int64_t n_cap, const int64_t* d_n) {
+  const int64_t n = eff_count(n_cap, d_n), stride = (int64_t)gridDim.x * 256;
+  for (int64_t j = (int64_t)blockIdx.x * 256 + threadIdx.x; j < n; j += stride) indices[j] = __ldg(col + indices[j]);
+}
+
+}  // namespace
+
+extern "C" int64_t sgl_build_batch_layout(int64_t n_roots, const int32_t* fanouts, int n_hops, int64_t* section_words) {
+  if (n_roots < 0 || n_hops < 0 || n_hops > kMaxHops || (n_hops && !fanouts) || !section_words) return -1;
+  const int s = batch_sections(n_roots, fanouts, n_hops, section_words);
+  int64_t total = 0;
+  for (int i = 0; i < s; ++i) total += section_words[i];
+  return total;
+}
+
+extern "C" size_t sgl_build_batch_ws_bytes(int64_t n_roots, const int32_t* fanouts, int n_hops) {
+  return sample_ws(n_roots, fanouts, n_hops) + list_ws(n_roots, fanouts, n_hops) + csc_ws(n_roots, fanouts, n_hops);
+}
+
+extern "C" int sgl_build_batch(const int64_t* indptr, const int64_t* nbr, const int64_t* ts, const int64_t* eid, const int64_t* fence,
+                               int64_t num_nodes, const int64_t* roots, const int64_t* root_ts, int64_t n_roots,
+                               const int32_t* fanouts, int n_hops, int policy, int equal_root_time, int64_t allowed_offset,
+                               uint64_t seed, int id_bits, int ts_bits, int64_t ts_base, int64_t* arena, int64_t* meta,
+                               int32_t* d_status, void* ws, size_t ws_bytes, void* side_stream, void* stream_) {
+  SGL_NVTX("sgl_build_batch");
+  cudaStream_t stream = (cudaStream_t)stream_;
+  SGL_REQUIRE(n_roots >= 0 && n_hops >= 0 && n_hops <= kMaxHops && (n_hops == 0 || fanouts), SGL_ERR_ARG,
+              "build_batch: bad size (at most %d hops)", kMaxHops);
+  for (int l = 0; l < n_hops; ++l) SGL_REQUIRE(fanouts[l] >= 1, SGL_ERR_ARG, "build_batch: fanout=%d must be >= 1", fanouts[l]);
+  SGL_REQUIRE(meta, SGL_ERR_ARG, "build_batch: meta is null");
+  SGL_CUDA_CHECK(cudaMemsetAsync(meta, 0, (size_t)(2 + 2 * n_hops) * sizeof(int64_t), stream));
+  if (n_roots == 0) return SGL_OK;
+  SGL_REQUIRE(arena && roots && root_ts, SGL_ERR_ARG, "build_batch: null array");
+  SGL_REQUIRE(ws_bytes >= sgl_build_batch_ws_bytes(n_roots, fanouts, n_hops), SGL_ERR_WORKSPACE, "build_batch: workspace %zu < %zu bytes",
+              ws_bytes, sgl_build_batch_ws_bytes(n_roots, fanouts, n_hops));
+  if (d_status == nullptr) d_status = (int32_t*)(meta + 1 + 2 * n_hops);
+  int64_t size[kRootSections + kMaxHops * kHopSections];
+  batch_sections(n_roots, fanouts, n_hops, size);
+  const size_t swb = sample_ws(n_roots, fanouts, n_hops), lwb = list_ws(n_roots, fanouts, n_hops), cwb = csc_ws(n_roots, fanouts, n_hops);
+  void *sws = ws, *lws = (char*)ws + swb, *cws = (char*)lws + lwb;
+  int64_t* p = arena;
+  int sec = 0;
+  auto take = [&]() {
+    int64_t* q = p;
+    p += size[sec++];
+    return q;
+  };
+  int64_t *cur_id = take(), *cur_ts = take(), *inv = take();
+  int rc = sgl_unique_pairs(roots, root_ts, n_roots, nullptr, nullptr, nullptr, 0, nullptr, id_bits, ts_bits, ts_base, cur_id, cur_ts, inv,
+                            nullptr, meta, d_status, lws, lwb, stream);
+  if (rc) return rc;
+  struct Hop {
+    int64_t *nbr, *dst, *ts, *eid, *offs, *gids, *gts, *col, *indptr, *indices, *cts, *ceid;
+    float *dt, *cdt;
+  } hop[kMaxHops];
+  for (int l = 0; l < n_hops; ++l) {
+    Hop& h = hop[l];
+    h.nbr = take(); h.dst = take(); h.ts = take(); h.dt = (float*)take(); h.eid = take(); h.offs = take();
+    h.gids = take(); h.gts = take(); h.col = take();
+    h.indptr = take(); h.indices = take(); h.cts = take(); h.cdt = (float*)take(); h.ceid = take();
+  }
+  auto sample = [&](int l, const int64_t* tgt, const int64_t* tgt_ts, int64_t n, const int64_t* d_n, cudaStream_t on) {
+    const Hop& h = hop[l];
+    return sample_layer(indptr, nbr, ts, eid, fence, num_nodes, tgt, tgt_ts, n, d_n, fanouts[l], policy, equal_root_time, allowed_offset, 0,
+                        seed, (uint32_t)l, h.nbr, h.dst, h.ts, h.dt, nullptr, h.eid, h.offs, meta + 1 + 2 * l, d_status, sws, swb, on);
+  };
+  // Hop l + 1 queries one target per edge sampled by hop l at that edge's time and waits for no relabel but the first; the
+  // CSC of a hop needs the relabel before it but not its own (its columns are translated at the end).  With a side stream
+  // both run there, next to the relabels: 4,096 roots uniform [10, 10] 168 us of kernels in a row, 120 side by side.
+  if (n_hops > 0 && (rc = sample(0, cur_id, cur_ts, n_roots, meta, stream))) return rc;
+  const bool forked = n_hops > 1 && side_stream != nullptr && side_stream != stream_;
+  cudaStream_t side = forked ? (cudaStream_t)side_stream : stream;
+  cudaEvent_t ev[4] = {nullptr, nullptr, nullptr, nullptr};
+  enum { kFork, kSampled, kRelabelled, kCsc };
+  if (forked) {
+    for (int i = 0; i < 4; ++i) SGL_CUDA_CHECK(thread_event(i, &ev[i]));
+    SGL_CUDA_CHECK(cudaEventRecord(ev[kFork], stream));
+    SGL_CUDA_CHECK(cudaStreamWaitEvent(side, ev[kFork], 0));
+  }
+  int64_t t = n_roots, c = n_roots;
+  const int64_t* d_cur = meta;
+  const int64_t* last_col = nullptr;
+  for (int l = 0; l < n_hops; ++l) {
+    const Hop& h = hop[l];
+    const int64_t e = t * fanouts[l];
+    int64_t *d_edges = meta + 1 + 2 * l, *d_next = meta + 2 + 2 * l;
+    if (forked && l > 0) SGL_CUDA_CHECK(cudaStreamWaitEvent(stream, ev[kSampled], 0));
+    if (l + 1 < n_hops) {
+      if ((rc = sample(l + 1, h.nbr, h.ts, e, d_edges, side))) return rc;
+      if (forked) SGL_CUDA_CHECK(cudaEventRecord(ev[kSampled], side));
+    }
+    if (l > 0) {
+      if (forked) SGL_CUDA_CHECK(cudaStreamWaitEvent(side, ev[kRelabelled], 0));
+      rc = sgl_build_csc(nullptr, h.dst, last_col, h.ts, h.dt, h.eid, e, d_edges, c, d_cur, bits_for((uint64_t)c), ts_bits, ts_base,
+                         h.indptr, h.indices, h.cts, h.cdt, h.ceid, 0, d_status, cws, cwb, side);
+      if (rc) return rc;
+      if (forked) SGL_CUDA_CHECK(cudaEventRecord(ev[kCsc], side));
+    }
+    rc = sgl_unique_pairs(cur_id, cur_ts, c, d_cur, h.nbr, h.ts, e, d_edges, id_bits, ts_bits, ts_base, h.gids, h.gts, nullptr, h.col,
+                          d_next, d_status, lws, lwb, stream);
+    if (rc) return rc;
+    if (forked && l + 1 < n_hops) SGL_CUDA_CHECK(cudaEventRecord(ev[kRelabelled], stream));
+    if (l > 0) {
+      if (forked) SGL_CUDA_CHECK(cudaStreamWaitEvent(stream, ev[kCsc], 0));
+      map_columns_kernel<<<stream_grid(e, 256 * 4, 8), 256, 0, stream>>>(h.indices, h.col, e, d_edges);
+      SGL_LAUNCH_CHECK();
+    }
+    cur_id = h.gids;
+    cur_ts = h.gts;
+    d_cur = d_next;
+    last_col = h.col;
+    t = e;
+    c += e;
+  }
+  return SGL_OK;
+}
+
+// Copies up to 4 KB of device memory to the host and waits for the stream: through a pinned buffer of the calling thread
+// (a copy to pageable memory is staged by the driver, 10 us more).
+extern "C" int sgl_read_back(const void* src, void* dst, size_t bytes, void* stream) {
+  constexpr size_t kBytes = 4096;
+  SGL_REQUIRE(src && dst && bytes <= kBytes, SGL_ERR_ARG, "read_back: at most %zu bytes", kBytes);
+  static thread_local void* pinned = nullptr;
+  if (pinned == nullptr) SGL_CUDA_CHECK(cudaHostAlloc(&pinned, kBytes, cudaHostAllocPortable));
+  SGL_CUDA_CHECK(cudaMemcpyAsync(pinned, src, bytes, cudaMemcpyDeviceToHost, (cudaStream_t)stream));
+  SGL_CUDA_CHECK(cudaStreamSynchronize((cudaStream_t)stream));
+  memcpy(dst, pinned, bytes);
+  return SGL_OK;
+}

@@ -16,6 +16,7 @@
 // Algorithmic HBM bytes per target: 16 (indptr pair) + 16 (target id, time) + 8*ceil(log2 deg) (search
 // probes) + k_eff*24 (nbr, ts, eid reads) + k_eff*36 (five output arrays) + 8 (offset).
 #include "common.cuh"
+#include "sampler.cuh"
 #include "scan.cuh"
 
 namespace sgl {
@@ -146,6 +147,7 @@ struct SampleArgs {
   int32_t* cnt;                // [n_cap] edges of every target
   int64_t* cta_sums;           // [count CTAs] edges of the CTA, or (more than kDirectCtas of them) of the CTAs before it
   unsigned int* done;          // arrival counter of the count CTAs (more than kDirectCtas)
+  int64_t* total_out;          // optional second place for the number of sampled edges
   int32_t* d_status;
 };
 
@@ -257,9 +259,13 @@ sample_fill_kernel(const SampleArgs a, int count_ctas) {
   if (direct) {
 #pragma unroll
     for (int w = 0; w < kWarpsPerCta; ++w) base += s_base[w];
-    if (threadIdx.x == 0 && first + FT >= a.n_cap) a.out_offsets[a.n_cap] = base + ct_total;
+    if (threadIdx.x == 0 && first + FT >= a.n_cap) {
+      a.out_offsets[a.n_cap] = base + ct_total;
+      if (a.total_out) *a.total_out = base + ct_total;
+    }
   } else {
     base = a.cta_sums[count_cta];
+    if (threadIdx.x == 0 && first + FT >= a.n_cap && a.total_out) *a.total_out = a.out_offsets[a.n_cap];
   }
   const bool draws = a.policy == SGL_POLICY_UNIFORM;
   uint32_t* s_pick = (uint32_t*)s_dyn;     // [fanout][FT]
@@ -431,12 +437,12 @@ static int launch_sample(const SampleArgs& a, cudaStream_t stream) {
   return SGL_OK;
 }
 
-static int sample_layer_impl(const int64_t* indptr, const int64_t* nbr, const int64_t* ts, const int64_t* eid,
-                             const int64_t* fence, int64_t num_nodes, const int64_t* targets, const int64_t* target_ts,
-                             int64_t n_targets, const int64_t* d_n, int fanout, int policy, int equal_root_time,
-                             int64_t allowed_offset, int keep_root_time, uint64_t seed, uint32_t rng_stream, int64_t* out_nbr,
-                             int64_t* out_dst, int64_t* out_ts, float* out_dt, int64_t* out_dt_i64, int64_t* out_eid,
-                             int64_t* out_offsets, int32_t* d_status, void* ws, size_t ws_bytes, void* stream_) {
+int sgl::sample_layer(const int64_t* indptr, const int64_t* nbr, const int64_t* ts, const int64_t* eid, const int64_t* fence,
+                      int64_t num_nodes, const int64_t* targets, const int64_t* target_ts, int64_t n_targets, const int64_t* d_n,
+                      int fanout, int policy, int equal_root_time, int64_t allowed_offset, int keep_root_time, uint64_t seed,
+                      uint32_t rng_stream, int64_t* out_nbr, int64_t* out_dst, int64_t* out_ts, float* out_dt, int64_t* out_dt_i64,
+                      int64_t* out_eid, int64_t* out_offsets, int64_t* total_out, int32_t* d_status, void* ws, size_t ws_bytes,
+                      void* stream_) {
   SGL_NVTX("sgl_sample_layer");
   cudaStream_t stream = (cudaStream_t)stream_;
   SGL_REQUIRE(n_targets >= 0 && num_nodes >= 0, SGL_ERR_ARG, "sample_layer: negative size");
@@ -449,6 +455,7 @@ static int sample_layer_impl(const int64_t* indptr, const int64_t* nbr, const in
   SGL_REQUIRE(n_targets < ((int64_t)1 << 34), SGL_ERR_UNSUPPORTED, "sample_layer: too many targets");
   if (n_targets == 0) {
     SGL_CUDA_CHECK(cudaMemsetAsync(out_offsets, 0, sizeof(int64_t), stream));
+    if (total_out) SGL_CUDA_CHECK(cudaMemsetAsync(total_out, 0, sizeof(int64_t), stream));
     return SGL_OK;
   }
   SGL_REQUIRE(indptr && nbr && ts && eid && targets && target_ts && out_nbr && out_dst && out_ts && out_dt && out_eid,
@@ -466,6 +473,7 @@ static int sample_layer_impl(const int64_t* indptr, const int64_t* nbr, const in
   a.out_nbr = out_nbr; a.out_dst = out_dst; a.out_ts = out_ts;
   a.out_dt = out_dt;
   a.out_dt_i64 = out_dt_i64; a.out_eid = out_eid; a.out_offsets = out_offsets;
+  a.total_out = total_out;
   a.d_status = d_status;
   WsCarver c(ws, ws_bytes);
   a.win_lo = c.take<int64_t>(n_targets);
@@ -490,9 +498,9 @@ extern "C" int sgl_sample_layer(const int64_t* indptr, const int64_t* nbr, const
                                 int64_t* out_dst, int64_t* out_ts, float* out_dt, int64_t* out_dt_i64,
                                 int64_t* out_eid, int64_t* out_offsets, int32_t* d_status, void* ws, size_t ws_bytes,
                                 void* stream) {
-  return sample_layer_impl(indptr, nbr, ts, eid, nullptr, num_nodes, targets, target_ts, n_targets, d_n, fanout, policy,
+  return sgl::sample_layer(indptr, nbr, ts, eid, nullptr, num_nodes, targets, target_ts, n_targets, d_n, fanout, policy,
                            equal_root_time, allowed_offset, keep_root_time, seed, rng_stream, out_nbr, out_dst, out_ts, out_dt,
-                           out_dt_i64, out_eid, out_offsets, d_status, ws, ws_bytes, stream);
+                           out_dt_i64, out_eid, out_offsets, nullptr, d_status, ws, ws_bytes, stream);
 }
 
 extern "C" int sgl_sample_layer_fenced(const int64_t* indptr, const int64_t* nbr, const int64_t* ts, const int64_t* eid,
@@ -502,9 +510,9 @@ extern "C" int sgl_sample_layer_fenced(const int64_t* indptr, const int64_t* nbr
                                        int64_t* out_nbr, int64_t* out_dst, int64_t* out_ts, float* out_dt, int64_t* out_dt_i64,
                                        int64_t* out_eid, int64_t* out_offsets, int32_t* d_status, void* ws, size_t ws_bytes,
                                        void* stream) {
-  return sample_layer_impl(indptr, nbr, ts, eid, fence, num_nodes, targets, target_ts, n_targets, d_n, fanout, policy,
+  return sgl::sample_layer(indptr, nbr, ts, eid, fence, num_nodes, targets, target_ts, n_targets, d_n, fanout, policy,
                            equal_root_time, allowed_offset, keep_root_time, seed, rng_stream, out_nbr, out_dst, out_ts, out_dt,
-                           out_dt_i64, out_eid, out_offsets, d_status, ws, ws_bytes, stream);
+                           out_dt_i64, out_eid, out_offsets, nullptr, d_status, ws, ws_bytes, stream);
 }
 
 extern "C" int sgl_sample_gather_fenced(const int64_t* indptr, const int64_t* nbr, const int64_t* ts, const int64_t* eid,
@@ -514,9 +522,9 @@ extern "C" int sgl_sample_gather_fenced(const int64_t* indptr, const int64_t* nb
                                         int64_t* out_ts, float* out_dt, int64_t* out_eid, int64_t* out_offsets,
                                         const void* feat_table, int64_t feat_rows, int64_t row_bytes, int64_t src_pitch,
                                         void* out_feats, int gather_mode, int32_t* d_status, void* ws, size_t ws_bytes, void* stream) {
-  int rc = sample_layer_impl(indptr, nbr, ts, eid, fence, num_nodes, targets, target_ts, n_targets, nullptr, fanout, policy,
+  int rc = sgl::sample_layer(indptr, nbr, ts, eid, fence, num_nodes, targets, target_ts, n_targets, nullptr, fanout, policy,
                              equal_root_time, allowed_offset, keep_root_time, seed, rng_stream, out_nbr, out_dst, out_ts, out_dt,
-                             nullptr, out_eid, out_offsets, d_status, ws, ws_bytes, stream);
+                             nullptr, out_eid, out_offsets, nullptr, d_status, ws, ws_bytes, stream);
   if (rc != SGL_OK || n_targets == 0) return rc;
   return sgl_gather_rows(feat_table, feat_rows, row_bytes, src_pitch, out_eid, nullptr, 0, n_targets * fanout,
                          out_offsets + n_targets, out_feats, row_bytes, nullptr, nullptr, gather_mode, d_status, stream);

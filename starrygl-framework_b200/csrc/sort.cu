@@ -220,12 +220,14 @@ struct RawSource {
   int64_t n_cap;
   const int64_t* d_n;
   uint64_t mask;        // only the sorted bits take part
-  __device__ __forceinline__ int64_t count() const { return eff_count(n_cap, d_n); }
+  __device__ __forceinline__ int64_t begin() const { return eff_count(n_cap, d_n); }
+  __device__ __forceinline__ void prepare(int64_t) const {}
   __device__ __forceinline__ uint64_t key(int64_t i) const { return keys[i] & mask; }
 };
 
 struct RawSink {
-  static constexpr bool kUnique = false, kPred = false;
+  static constexpr bool kUnique = false, kPred = false, kAfter = false;
+  __device__ __forceinline__ void begin() const {}
   const uint64_t* keys;
   const uint32_t* vals;  // nullptr: the payload is the input position
   uint64_t* out_keys;
@@ -235,7 +237,7 @@ struct RawSink {
     out_keys[at] = mask == ~0ull ? key : keys[pos];
     out_vals[at] = vals ? vals[pos] : pos;
   }
-  __device__ __forceinline__ void finish(int64_t, uint64_t, bool, int64_t) const {}
+  __device__ __forceinline__ void finish(int64_t, uint64_t, bool, int64_t, int64_t) const {}
 };
 
 template <int BITS>

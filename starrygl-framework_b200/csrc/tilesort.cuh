@@ -33,7 +33,7 @@ constexpr int kWarps = kThreads / 32;
 constexpr int kMinTile = 256;
 constexpr int kMaxTile = 4096;
 constexpr int kTileItems = kMaxTile / kThreads;
-constexpr int kMaxSamples = 1024;       // sample of the whole list: about seven per bucket with 148 buckets
+constexpr int kMaxSamples = 2048;       // sample of the whole list: about fourteen per bucket with 148 buckets
 constexpr int64_t kMaxItems = (int64_t)kMaxCtas * kMaxTile;
 constexpr int kSingleMax = 2048;
 constexpr unsigned long long kWaitNs = 2000000000ull;
@@ -205,49 +205,72 @@ __device__ __forceinline__ void block_sort(const View<WIDE>& v, const View<WIDE>
 }
 static_assert(kMaxItems < (1 << 21), "rank inside a group: 21 bits");
 
-// The items of one CTA in sorted order -> the sink.  `base` = global position of the first, `pred_key` = the key
-// before it (when has_pred), `b` / `last` = which bucket this is and whether it is the last one.
+// What a Sink is:
+//   kUnique = false   item(at, key, pos, has_prev, prev_key): the item at global position `at`, and the key before it
+//   kUnique = true    item(at, key, pos, head, u, head2, u2): `head` = first item of its group (equal sink.group(key)), `u` =
+//                     number of the group; with kLevels = 2 the same for sink.group2(key), coarser than group.  Items with
+//                     counted(key) = false (sorted behind the others) belong to no group.
+//   kPred             needs the key before a bucket's first item (prev_key, head)
+//   begin()           called once per thread before the rest (loads device-side counts)
+//   finish(n, last_key, has_last, groups, groups2)   once, by all threads of the CTA of the last bucket
+//   kAfter / after()  by one thread after every CTA has delivered its items
+// A Source: begin() loads device-side counts and returns the number of items; key(i); prepare(i) is called for every i in
+// [0, n) before any item is delivered.
+
+// The items of one CTA in sorted order -> the sink.  `base` = global position of the first, `pred_key` = the key before it
+// (when has_pred), `b` / `last` = which bucket this is and whether it is the last one.
 template <class Sink, bool WIDE>
-__device__ __forceinline__ void deliver(const Sink& sink, const View<WIDE>& v, int m, int64_t n, int64_t base, uint64_t pred_key, bool has_pred,
-                        int pos_bits, int b, bool last, unsigned int* ctl, int32_t* d_status) {
+__device__ __forceinline__ void deliver(const Sink& sink, const View<WIDE>& v, int m, int64_t n, int64_t base, uint64_t pred_key,
+                                        bool has_pred, int pos_bits, int b, bool last, unsigned long long* ctl, int32_t* d_status) {
   if constexpr (!Sink::kUnique) {
-    for (int i = threadIdx.x; i < m; i += blockDim.x) {
+    for (int i = threadIdx.x; i < m; i += kThreads) {
       const Item x = v.get(i);
       const bool hp = i > 0 || has_pred;
       const uint64_t pk = i > 0 ? key_of<WIDE>(v.get(i - 1), pos_bits) : pred_key;
       sink.item(base + i, key_of<WIDE>(x, pos_bits), pos_of<WIDE>(x, pos_bits), hp, pk);
     }
-    if (last) sink.finish(n, m > 0 ? key_of<WIDE>(v.get(m - 1), pos_bits) : pred_key, m > 0 || has_pred, 0);
+    if (last) sink.finish(n, m > 0 ? key_of<WIDE>(v.get(m - 1), pos_bits) : pred_key, m > 0 || has_pred, 0, 0);
   } else {
-    __shared__ int s_warp[32];
-    __shared__ int s_base;
-    auto is_head = [&](int i) {
+    constexpr bool kTwo = Sink::kLevels == 2;
+    __shared__ unsigned long long s_warp[kWarps];
+    __shared__ unsigned long long s_base;
+    // heads of item i: bit 0 of its group, bit 32 of its coarser group
+    auto heads_of = [&](int i) -> unsigned long long {
       const uint64_t k = key_of<WIDE>(v.get(i), pos_bits);
-      if (!sink.counted(k)) return false;
-      if (i > 0) return key_of<WIDE>(v.get(i - 1), pos_bits) != k;
-      return !has_pred || pred_key != k;
+      if (!sink.counted(k)) return 0;
+      if (i == 0 && !has_pred) return kTwo ? 0x100000001ull : 1ull;
+      const uint64_t p = i > 0 ? key_of<WIDE>(v.get(i - 1), pos_bits) : pred_key;
+      unsigned long long h = sink.group(p) != sink.group(k) ? 1ull : 0ull;
+      if constexpr (kTwo) h |= sink.group2(p) != sink.group2(k) ? 0x100000000ull : 0ull;
+      return h;
     };
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    auto cta_sum = [&](unsigned long long x) {
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+      __syncthreads();
+      if (lane == 0) s_warp[warp] = x;
+      __syncthreads();
+      x = 0;
+#pragma unroll
+      for (int w = 0; w < kWarps; ++w) x += s_warp[w];
+      return x;
+    };
     // heads of the bucket -> published; the numbers of the earlier buckets are summed up by one thread each
-    int mine = 0;
-    for (int i = threadIdx.x; i < m; i += blockDim.x) mine += is_head(i) ? 1 : 0;
-    mine = (int)__reduce_add_sync(0xffffffffu, (unsigned)mine);
-    if (lane == 0) s_warp[warp] = mine;
-    __syncthreads();
-    int heads = 0;
-    for (int w = 0; w < warps; ++w) heads += s_warp[w];
-    __syncthreads();
-    int before = 0;
+    unsigned long long heads = 0, before = 0;
+    for (int i = threadIdx.x; i < m; i += kThreads) heads += heads_of(i);
+    heads = cta_sum(heads);
     if (ctl != nullptr) {
-      if (threadIdx.x == 0) atomicExch(ctl + 1 + b, (unsigned)heads + 1u);
+      volatile unsigned long long* pub = ctl + 1;
+      if (threadIdx.x == 0) pub[b] = heads + 1ull;
       // lower buckets have taken their ticket before this one: their CTAs are running and wait only for still lower ones
-      for (int t = threadIdx.x; t < b; t += blockDim.x) {
-        unsigned c = *(volatile unsigned int*)(ctl + 1 + t);
+      for (int t = threadIdx.x; t < b; t += kThreads) {
+        unsigned long long c = pub[t];
         if (c == 0) {
           unsigned long long t0, t1;
           asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t0));
           do {
-            c = *(volatile unsigned int*)(ctl + 1 + t);
+            c = pub[t];
             asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t1));
           } while (c == 0 && t1 - t0 < kWaitNs);
           if (c == 0) {
@@ -255,26 +278,22 @@ __device__ __forceinline__ void deliver(const Sink& sink, const View<WIDE>& v, i
             c = 1;
           }
         }
-        before += (int)c - 1;
+        before += c - 1ull;
       }
-      before = (int)__reduce_add_sync(0xffffffffu, (unsigned)before);
-      if (lane == 0) s_warp[warp] = before;
-      __syncthreads();
-      before = 0;
-      for (int w = 0; w < warps; ++w) before += s_warp[w];
-      __syncthreads();
+      before = cta_sum(before);
     }
     if (threadIdx.x == 0) s_base = before;
     __syncthreads();
-    for (int i0 = 0; i0 < m; i0 += blockDim.x) {
+    for (int i0 = 0; i0 < m; i0 += kThreads) {
       const int i = i0 + threadIdx.x;
-      const bool h = i < m && is_head(i);
-      const unsigned bal = __ballot_sync(0xffffffffu, h);
-      if (lane == 0) s_warp[warp] = __popc(bal);
+      const unsigned long long h = i < m ? heads_of(i) : 0ull;
+      const unsigned b1 = __ballot_sync(0xffffffffu, (h & 1ull) != 0), b2 = kTwo ? __ballot_sync(0xffffffffu, (h >> 32) != 0) : 0u;
+      if (lane == 0) s_warp[warp] = (unsigned long long)__popc(b1) | ((unsigned long long)__popc(b2) << 32);
       __syncthreads();
-      int off = s_base, tot = 0;
-      for (int w = 0; w < warps; ++w) {
-        const int c = s_warp[w];
+      unsigned long long off = s_base, tot = 0;
+#pragma unroll
+      for (int w = 0; w < kWarps; ++w) {
+        const unsigned long long c = s_warp[w];
         if (w < warp) off += c;
         tot += c;
       }
@@ -282,13 +301,28 @@ __device__ __forceinline__ void deliver(const Sink& sink, const View<WIDE>& v, i
       if (threadIdx.x == 0) s_base += tot;
       if (i < m) {
         const Item x = v.get(i);
-        // rank of the item's key among the distinct keys
-        const int64_t u = off + __popc(bal & ((2u << lane) - 1u)) - 1;
-        sink.item(base + i, key_of<WIDE>(x, pos_bits), pos_of<WIDE>(x, pos_bits), h, u);
+        const unsigned upto = (2u << lane) - 1u;
+        const int64_t u = (int64_t)(off & 0xffffffffull) + __popc(b1 & upto) - 1, u2 = (int64_t)(off >> 32) + __popc(b2 & upto) - 1;
+        sink.item(base + i, key_of<WIDE>(x, pos_bits), pos_of<WIDE>(x, pos_bits), (h & 1ull) != 0, u, (h >> 32) != 0, u2);
       }
       __syncthreads();
     }
-    if (last) sink.finish(n, 0, false, before + heads);
+    if (last) sink.finish(n, 0, false, (int64_t)((before + heads) & 0xffffffffull), (int64_t)((before + heads) >> 32));
+  }
+}
+
+// after(): once every CTA of the launch has delivered
+template <class Sink>
+__device__ __forceinline__ void arrive(const Sink& sink, unsigned long long* counter, int ctas) {
+  if constexpr (Sink::kAfter) {
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      __threadfence();
+      if (counter == nullptr || atomicAdd(counter, 1ull) == (unsigned long long)(ctas - 1)) {
+        __threadfence();
+        sink.after();
+      }
+    }
   }
 }
 
@@ -308,16 +342,16 @@ struct Scratch {
   uint32_t* over_p;     // [2][n] (WIDE)
   uint32_t* over_a;     // [n]
   uint16_t* over_g;     // [n]
-  unsigned int* ctl;    // [0] ticket, [1 + b] number of distinct keys of bucket b plus one (0 = not known yet)
+  unsigned long long* ctl;   // [0] ticket, [1 + b] groups of bucket b plus one (0 = not known yet), [kCtlWords - 1] arrivals
 };
 
-constexpr int kCtlWords = kMaxCtas + 2;
+constexpr int kCtlWords = kMaxCtas + 3;
 constexpr int kMatrix = (kMaxCtas + 1) * kMaxCtas;
 
 inline size_t ws_bytes(int64_t n) {
   if (n < 1) n = 1;
   return align_up((size_t)n * 8) + align_up((size_t)n * 4) + align_up(kMatrix * 4) + align_up(kMatrix * 8) + align_up((size_t)n * 16) +
-         align_up((size_t)n * 8) + align_up((size_t)n * 4) + align_up((size_t)n * 2) + align_up(kCtlWords * 4);
+         align_up((size_t)n * 8) + align_up((size_t)n * 4) + align_up((size_t)n * 2) + align_up(kCtlWords * 8);
 }
 
 inline Scratch carve(WsCarver& c, int64_t n) {
@@ -330,7 +364,7 @@ inline Scratch carve(WsCarver& c, int64_t n) {
   s.over_p = c.take<uint32_t>(2 * (size_t)n);
   s.over_a = c.take<uint32_t>(n);
   s.over_g = c.take<uint16_t>(n);
-  s.ctl = c.take<unsigned int>(kCtlWords);
+  s.ctl = c.take<unsigned long long>(kCtlWords);
   return s;
 }
 
@@ -357,7 +391,7 @@ ts_part_kernel(Source src, int pos_bits, Scratch sc) {
   extern __shared__ __align__(16) unsigned char smem_ts[];
   __shared__ int s_cnt[kMaxCtas], s_w[kWarps];
   __shared__ unsigned long long s_top[kMaxCtas];
-  const int64_t n = src.count();
+  const int64_t n = src.begin();
   const int tile = tile_for(n, (int)gridDim.x);
   const int tiles = (int)((n + tile - 1) / tile);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -371,21 +405,25 @@ ts_part_kernel(Source src, int pos_bits, Scratch sc) {
   for (int r = 0; r < kTileItems; ++r) {
     const int i = tid + r * kThreads;
     x[r] = i < m ? make_item<WIDE>(src.key(first + i), (uint32_t)(first + i), pos_bits) : Item{0, 0};
+    if (i < m) src.prepare(first + i);
   }
   const Arrays<WIDE> sm(smem_ts, kMaxSamples);
   const View<WIDE> split = sm.tmp;       // splitter b (b = 1 .. tiles - 1) at split[b - 1]
+  const int buckets = tiles;             // one bucket per tile (two smaller ones were slower)
   if (tiles > 1) {
     // (more than one tile: n is above (tiles - 1) * 256, the sample is smaller than the list)
-    const int sb = tiles <= 16 ? 8 : (tiles <= 32 ? 9 : 10), s = 1 << sb;
+    // 14 - 16 samples per bucket: the largest bucket is about 1.7 times the mean.  From 31 to 148 short tiles seven have to
+    // do: sorting twice as many costs more than the larger buckets do.
+    const int sb = tiles <= 16 ? 8 : (tiles <= 32 ? 9 : (n < 60000 ? 10 : 11)), s = 1 << sb;
     for (int j = tid; j < s; j += kThreads) {
       const int i = sample_at(j, sb, (int)n);
       sm.v.set(j, make_item<WIDE>(src.key(i), (uint32_t)i, pos_bits));
     }
     block_sort<WIDE>(sm.v, sm.tmp, sm.aux, sm.grp, s);
-    for (int b = 1 + tid; b < tiles; b += kThreads) split.set(b - 1, sm.v.get(b * s / tiles));
+    for (int b = 1 + tid; b < buckets; b += kThreads) split.set(b - 1, sm.v.get(b * s / buckets));
   }
-  const int step = step_for(tiles - 1);
-  for (int b = tid; b < kMaxCtas; b += kThreads) {
+  const int step = step_for(buckets - 1);
+  for (int b = tid; b < buckets; b += kThreads) {
     s_cnt[b] = 0;
     s_top[b] = 0;
   }
@@ -395,24 +433,24 @@ ts_part_kernel(Source src, int pos_bits, Scratch sc) {
   for (int r = 0; r < kTileItems; ++r) {
     bucket[r] = at[r] = 0;
     if (tid + r * kThreads < m) {
-      bucket[r] = not_above<WIDE>(split, tiles - 1, step, x[r]);
+      bucket[r] = not_above<WIDE>(split, buckets - 1, step, x[r]);
       at[r] = atomicAdd(&s_cnt[bucket[r]], 1);
       if (TOP) atomicMax(&s_top[bucket[r]], (unsigned long long)key_of<WIDE>(x[r], pos_bits) + 1ull);
     }
   }
   __syncthreads();
-  const int c = tid < tiles ? s_cnt[tid] : 0;
+  const int c = tid < buckets ? s_cnt[tid] : 0;
   int off = warp_inclusive_scan(c, lane);
   if (lane == 31) s_w[warp] = off;
   __syncthreads();
   for (int w = 0; w < warp; ++w) off += s_w[w];
   off -= c;
-  if (tid < tiles) {
+  if (tid < buckets) {
     s_cnt[tid] = off;
     sc.start[tid * tiles + blockIdx.x] = off;
     if (TOP) sc.top[tid * tiles + blockIdx.x] = s_top[tid];
   }
-  if (tid == 0) sc.start[tiles * tiles + blockIdx.x] = m;
+  if (tid == 0) sc.start[buckets * tiles + blockIdx.x] = m;
   __syncthreads();
 #pragma unroll
   for (int r = 0; r < kTileItems; ++r)
@@ -430,17 +468,22 @@ ts_bucket_kernel(Source src, Sink sink, int pos_bits, int64_t n_cap, Scratch sc,
   __shared__ int s_w[kWarps];
   __shared__ long long s_sum[kWarps];
   __shared__ unsigned long long s_top;
-  const int64_t n = src.count();
+  const int64_t n = src.begin();
+  sink.begin();
   if (n <= 0) {
-    if (blockIdx.x == 0) sink.finish(0, 0, false, 0);
+    if (blockIdx.x == 0) {
+      sink.finish(0, 0, false, 0, 0);
+      arrive(sink, nullptr, 1);
+    }
     return;
   }
   const int tile = tile_for(n, (int)gridDim.x);
   const int tiles = (int)((n + tile - 1) / tile);
-  if ((int)blockIdx.x >= tiles) return;
+  const int buckets = tiles;             // one bucket per tile (two smaller ones were slower)
+  if ((int)blockIdx.x >= buckets) return;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   if (tid == 0) {
-    s_ticket = Sink::kUnique ? (int)atomicAdd(sc.ctl, 1u) : (int)blockIdx.x;
+    s_ticket = Sink::kUnique ? (int)atomicAdd(sc.ctl, 1ull) : (int)blockIdx.x;
     s_top = 0;
   }
   __syncthreads();
@@ -489,7 +532,7 @@ ts_bucket_kernel(Source src, Sink sink, int pos_bits, int64_t n_cap, Scratch sc,
       for (int i = s_at[a] + (tid & 3); i < e; i += 4) v.set(i, from.get(f + i));
     }
   };
-  const bool last = b == tiles - 1;
+  const bool last = b == buckets - 1;
   if (m <= cap) {
     const Arrays<WIDE> sm(smem_ts, cap);
     collect(sm.v);
@@ -502,17 +545,23 @@ ts_bucket_kernel(Source src, Sink sink, int pos_bits, int64_t n_cap, Scratch sc,
     block_sort<WIDE>(v, tmp, sc.over_a + base, sc.over_g + base, m);
     deliver<Sink, WIDE>(sink, v, m, n, base, pred_key, has_pred, pos_bits, b, last, sc.ctl, d_status);
   }
+  arrive(sink, sc.ctl + kCtlWords - 1, buckets);
 }
 
 template <class Source, class Sink, bool WIDE>
 __global__ void __launch_bounds__(kThreads)
 ts_single_kernel(Source src, Sink sink, int pos_bits, int32_t* d_status) {
   extern __shared__ __align__(16) unsigned char smem_ts[];
-  const int m = (int)src.count();
+  const int m = (int)src.begin();
+  sink.begin();
   const Arrays<WIDE> sm(smem_ts, kSingleMax);
-  for (int i = threadIdx.x; i < m; i += kThreads) sm.v.set(i, make_item<WIDE>(src.key(i), (uint32_t)i, pos_bits));
+  for (int i = threadIdx.x; i < m; i += kThreads) {
+    sm.v.set(i, make_item<WIDE>(src.key(i), (uint32_t)i, pos_bits));
+    src.prepare(i);
+  }
   block_sort<WIDE>(sm.v, sm.tmp, sm.aux, sm.grp, m);
   deliver<Sink, WIDE>(sink, sm.v, m, m, 0, 0, false, pos_bits, 0, true, nullptr, d_status);
+  arrive(sink, nullptr, 1);
 }
 
 inline int launches(int64_t n_cap) { return n_cap <= 0 ? 0 : (n_cap <= kSingleMax ? 1 : 2); }
@@ -532,7 +581,7 @@ inline cudaError_t allow_smem(const void* kernel, std::atomic<uint64_t>& done, s
 template <class Source, class Sink, bool WIDE>
 int launch_as(const Source& src, const Sink& sink, int64_t n_cap, int pos_bits, const Scratch& sc, int32_t* d_status,
               cudaStream_t stream) {
-  static std::atomic<uint64_t> single_done{0}, bucket_done{0};
+  static std::atomic<uint64_t> single_done{0}, bucket_done{0}, part_done{0};
   if (n_cap <= kSingleMax) {
     constexpr size_t smem = Arrays<WIDE>::bytes(kSingleMax);
     SGL_CUDA_CHECK(allow_smem((const void*)ts_single_kernel<Source, Sink, WIDE>, single_done, smem));
@@ -543,10 +592,11 @@ int launch_as(const Source& src, const Sink& sink, int64_t n_cap, int pos_bits, 
   const int64_t min_tiles = (n_cap + kMinTile - 1) / kMinTile;
   const int ctas = (int)(min_tiles < kMaxCtas ? min_tiles : kMaxCtas);
   const int tile = tile_for(n_cap, ctas);
-  // a bucket is about a tile, up to twice that with seven samples per bucket; what does not fit goes through global memory
+  // a bucket is about a tile, up to twice that; what does not fit goes through global memory
   constexpr int kCapMost = WIDE ? 6912 : 9216;
   const int cap = 4 * tile < kCapMost ? 4 * tile : kCapMost;
   SGL_CUDA_CHECK(allow_smem((const void*)ts_bucket_kernel<Source, Sink, WIDE>, bucket_done, Arrays<WIDE>::bytes(kCapMost)));
+  SGL_CUDA_CHECK(allow_smem((const void*)ts_part_kernel<Source, WIDE, Sink::kPred>, part_done, Arrays<WIDE>::bytes(kMaxSamples)));
   ts_part_kernel<Source, WIDE, Sink::kPred><<<ctas, kThreads, Arrays<WIDE>::bytes(kMaxSamples), stream>>>(src, pos_bits, sc);
   ts_bucket_kernel<Source, Sink, WIDE><<<ctas, kThreads, Arrays<WIDE>::bytes(cap), stream>>>(src, sink, pos_bits, n_cap, sc, cap, d_status);
   SGL_LAUNCH_CHECK();

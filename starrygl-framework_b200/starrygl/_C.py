@@ -104,6 +104,11 @@ _SIGNATURES = {
     "sgl_mail_reduce": (_i32, [_vp, _i64, _vp, _i64, _i64, _vp, _i64, _i32, _i32, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp,
                                _sz, _vp]),
     "sgl_mailbox_write": (_i32, [_vp, _i64, _vp, _vp, _vp, _i64, _vp, _vp, _vp, _i64, _i64, _i32, _vp, _vp]),
+    "sgl_build_batch_layout": (_i64, [_i64, _vp, _i32, _vp]),
+    "sgl_build_batch_ws_bytes": (_sz, [_i64, _vp, _i32]),
+    "sgl_build_batch": (_i32, [_vp, _vp, _vp, _vp, _vp, _i64, _vp, _vp, _i64, _vp, _i32, _i32, _i32, _i64, _u64, _i32, _i32, _i64,
+                               _vp, _vp, _vp, _vp, _sz, _vp, _vp]),
+    "sgl_read_back": (_i32, [_vp, _vp, _sz, _vp]),
     "sgl_graph_capture_begin": (_i32, [_vp]),
     "sgl_graph_capture_end": (_i32, [_vp, C.POINTER(C.c_void_p)]),
     "sgl_graph_launch": (_i32, [_vp, _vp, _vp, _sz, _vp]),

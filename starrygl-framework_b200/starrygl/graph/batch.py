@@ -8,36 +8,130 @@ previous list (``indptr``, ``indices``, ``eid``, ``edge_ts``, ``edge_dt``) + the
 synchronisation: the number of edges a hop produced is handed to the next kernels as a device count.
 ``finish()`` performs the single synchronisation that is needed to give the tensors their final shapes.
 """
+import threading
+from collections import OrderedDict
 from typing import List, Optional, Sequence
 
 import torch
 
-from .. import ops
+from .. import _C, ops
+
+
+class _Plan:
+    """What a batch of one shape (number of roots, fan-outs) needs: the arena's sections, the scratch size and the fan-outs as
+    the library reads them."""
+
+    def __init__(self, n: int, fanouts: Sequence[int]):
+        import ctypes as C
+        L = _C.lib()
+        if len(fanouts) > 8:
+            raise _C.SglError("build_batch: at most 8 hops")
+        self.fan = (C.c_int32 * max(len(fanouts), 1))(*[int(k) for k in fanouts])
+        sec = (C.c_int64 * (3 + 14 * len(fanouts)))()
+        self.words = int(L.sgl_build_batch_layout(n, self.fan, len(fanouts), sec))
+        if self.words < 0:
+            raise _C.SglError("build_batch: bad batch shape")
+        self.ws_bytes = int(L.sgl_build_batch_ws_bytes(n, self.fan, len(fanouts)))
+        self.start, at = [], 0
+        for w in sec:
+            self.start.append(at)
+            at += int(w)
+
+
+_PLANS: "OrderedDict" = OrderedDict()
+
+
+def _plan(n, fanouts) -> _Plan:
+    key = (n, *fanouts)
+    p = _PLANS.get(key)
+    if p is None:
+        p = _PLANS[key] = _Plan(n, fanouts)
+        if len(_PLANS) > 64:
+            _PLANS.popitem(last=False)
+    return p
+
+
+class _MetaStatus(ops.StatusWord):
+    """The status word of a batch that came without one: the last word of its meta block."""
+
+    def __init__(self, meta):
+        self.t = meta[-1:].view(torch.int32)[:1]
 
 
 class DeviceBatch:
-    """Un-trimmed result of :func:`build_batch_async` (all arrays at capacity, counts on the device)."""
+    """Un-trimmed result of :func:`build_batch_async`: one arena with every array at capacity, the counts on the device."""
 
-    def __init__(self, g, layers, counts, status, fanouts, targets_first):
-        self.g = g
-        self.layers = layers          # list of dicts of capacity-sized tensors
-        self.counts = counts          # list of device int64 scalars (1-element tensors), see finish()
-        self.status = status
-        self.fanouts = list(fanouts)
-        self._targets_first = targets_first
+    def __init__(self, g, n, fanouts, plan, arena, meta, status):
+        self.g, self.n, self.fanouts = g, n, list(fanouts)
+        self._plan, self._arena, self._meta, self._status = plan, arena, meta, status
+        self._layers = None
+
+    @property
+    def status(self):
+        if self._status is None:
+            self._status = _MetaStatus(self._meta)
+        return self._status
+
+    @property
+    def counts(self):
+        """Device int64 scalars (1-element tensors): root list, then per hop sampled edges and merged list."""
+        return [self._meta[i:i + 1] for i in range(1 + 2 * len(self.fanouts))]
+
+    def _view(self, section, count, floats=False):
+        s = self._plan.start[section]
+        if floats:
+            return self._arena[s:s + (count + 1) // 2].view(torch.float32)[:count]
+        return self._arena[s:s + count]
+
+    @property
+    def layers(self):
+        """Capacity-sized tensors per layer (views into the arena)."""
+        if self._layers is None:
+            v, n = self._view, self.n
+            out = [{"gids": v(0, n), "ts": v(1, n), "inv_map": v(2, n)}]
+            t = c = n
+            counts = self.counts
+            for l, k in enumerate(self.fanouts):
+                b, e = 3 + 14 * l, t * k
+                hop = ops.Hop(v(b, e), v(b + 1, e), v(b + 2, e), v(b + 3, e, True), v(b + 4, e), v(b + 5, t + 1), e)
+                d = {"raw_nbr": hop.nbr, "raw_ts": hop.ts, "inv": v(b + 8, e), "hop": hop, "gids": v(b + 6, c + e), "ts": v(b + 7, c + e)}
+                if l == 0:
+                    d.update(indptr=hop.offsets, indices=d["inv"], eid=hop.eid, edge_ts=hop.ts, edge_dt=hop.dt)
+                else:
+                    d.update(indptr=v(b + 9, c + 1), indices=v(b + 10, e), edge_ts=v(b + 11, e), edge_dt=v(b + 12, e, True), eid=v(b + 13, e))
+                out.append(d)
+                t, c = e, c + e
+            self._layers = out
+        return self._layers
+
+    def _read(self):
+        """The one read-back: every count and, when the batch owns it, the status word."""
+        import ctypes as C
+        words = 2 + 2 * len(self.fanouts)
+        buf = (C.c_int64 * words)()
+        with torch.cuda.device(self._meta.device):
+            _C.check(_C.lib().sgl_read_back(self._meta.data_ptr(), buf, 8 * words, _C.stream_ptr()))
+        host = list(buf)
+        return host[:-1], host[-1] & 0xFFFFFFFF
 
     def finish(self) -> List[dict]:
         """One host synchronisation: read every count, check the device status word, trim the arrays."""
-        host = self._host = torch.cat(self.counts).tolist()      # one read-back (synchronises the current stream)
-        self.status.check("build_batch")
+        host, bits = self._read()
+        if isinstance(self._status, ops.StatusWord) and not isinstance(self._status, _MetaStatus):
+            self._status.check("build_batch")
+        elif bits:
+            raise _C.SglError(f"build_batch: device status {bits} ({_C.decode_status(bits)})")
+        return self._trim(host)
+
+    def _trim(self, host):
+        self._host = host
+        v, n = self._view, self.n
         n_list = host[0]
-        out = [{"gids": self.layers[0]["gids"][:n_list], "ts": self.layers[0]["ts"][:n_list],
-                "inv_map": self.layers[0]["inv_map"]}]
+        out = [{"gids": v(0, n_list), "ts": v(1, n_list), "inv_map": v(2, n)}]
         prev_n = n_list
         for l in range(len(self.fanouts)):
             n_edges, n_next = host[1 + 2 * l], host[2 + 2 * l]
-            L = self.layers[l + 1]
-            if n_edges == 0 and not self._any_target_has_edges(l, out, prev_n):
+            if n_edges == 0 and not self._any_target_has_edges(l, out):
                 # the reference emits an empty layer and stops when no target has any edge at all
                 # (prepare_sample.py:352-361)
                 z = torch.zeros(0, dtype=torch.int64, device=self.g.device)
@@ -45,135 +139,134 @@ class DeviceBatch:
                             "eid": z, "edge_ts": z, "edge_dt": torch.zeros(0, dtype=torch.float32, device=self.g.device),
                             "gids": z, "ts": z})
                 break
-            out.append({"indptr": L["indptr"][:prev_n + 1], "indices": L["indices"][:n_edges], "eid": L["eid"][:n_edges],
-                        "edge_ts": L["edge_ts"][:n_edges], "edge_dt": L["edge_dt"][:n_edges],
-                        "gids": L["gids"][:n_next], "ts": L["ts"][:n_next]})
+            b = 3 + 14 * l
+            # (the first hop's edges are in CSC order as they were sampled, see sgl_build_batch)
+            ip, ix, ts, dt, ei = (5, 8, 2, 3, 4) if l == 0 else (9, 10, 11, 12, 13)
+            out.append({"indptr": v(b + ip, prev_n + 1), "indices": v(b + ix, n_edges), "eid": v(b + ei, n_edges),
+                        "edge_ts": v(b + ts, n_edges), "edge_dt": v(b + dt, n_edges, True),
+                        "gids": v(b + 6, n_next), "ts": v(b + 7, n_next)})
             prev_n = n_next
         return out
 
-    def _any_target_has_edges(self, l, out, prev_n):
-        tgt = out[0]["gids"] if l == 0 else self.layers[l]["raw_nbr"][:self._host[1 + 2 * (l - 1)]]
+    def _any_target_has_edges(self, l, out):
+        tgt = out[0]["gids"] if l == 0 else self._view(3 + 14 * (l - 1), self._host[1 + 2 * (l - 1)])
         if tgt.numel() == 0:
             return False
         deg = self.g.indptr[tgt + 1] - self.g.indptr[tgt]
         return bool((deg > 0).any().item())
 
 
+def _enqueue(g, roots, root_ts, fanouts, policy, lo, hi, equal_root_time, allowed_offset, seed, status, side) -> DeviceBatch:
+    """``lo`` / ``hi``: lowest and highest timestamp that can occur."""
+    roots, root_ts = ops._i64(roots), ops._i64(root_ts)
+    n = roots.numel()
+    if root_ts.numel() != n:
+        raise _C.SglError("build_batch: roots and root_ts differ in length")
+    plan = _plan(n, fanouts)
+    dev = g.device
+    arena = torch.empty(plan.words + 2 + 2 * len(fanouts), dtype=torch.int64, device=dev)
+    meta = arena[plan.words:]
+    sp = _C.stream_ptr()
+    ws = _C.WORKSPACE.get(plan.ws_bytes, dev, sp)
+    base = arena.data_ptr()
+    _C.check(_C.lib().sgl_build_batch(
+        g.indptr.data_ptr(), g.nbr.data_ptr(), g.ts.data_ptr(), g.eid.data_ptr(), None if g.fence is None else g.fence.data_ptr(),
+        g.num_nodes, _C.ptr(roots), _C.ptr(root_ts), n, plan.fan, len(fanouts),
+        _C.POLICY[policy] if isinstance(policy, str) else int(policy), int(bool(equal_root_time)), int(allowed_offset),
+        int(seed) & (2 ** 64 - 1), ops.bits_for(g.num_nodes - 1), ops.bits_for(hi - lo), lo, base, base + 8 * plan.words,
+        None if status is None else status.ptr(), ws.data_ptr(), ws.numel(), None if side is None else side.cuda_stream, sp))
+    return DeviceBatch(g, n, fanouts, plan, arena, meta, status)
+
+
+_LOCAL = threading.local()
+
+
+def _side_stream(dev) -> torch.cuda.Stream:
+    """The calling thread's second stream on ``dev`` for batches of several hops."""
+    pool = _LOCAL.__dict__.setdefault("streams", {})
+    s = pool.get(dev.index)
+    if s is None:
+        s = pool[dev.index] = torch.cuda.Stream(dev)
+    return s
+
+
+def _graph_range(g, lo, hi):
+    """Timestamps of the batch's lists: the queries' and the graph's."""
+    return min(g.ts_min, lo), max(g.ts_max, hi)
+
+
 def build_batch_async(g: ops.TCSR, roots: torch.Tensor, root_ts: torch.Tensor, fanouts: Sequence[int],
                       policy: str = "recent", *, ts_range: Optional[Sequence[int]] = None, equal_root_time=False,
                       allowed_offset=-1, seed=0, status: Optional[ops.StatusWord] = None,
                       side_streams: Optional[Sequence[torch.cuda.Stream]] = None) -> DeviceBatch:
-    """Enqueue the whole batch construction on the current stream.
+    """Enqueue the whole batch construction on the current stream: one foreign call, one allocation.
 
     ``ts_range`` = (lowest, highest) timestamp that can occur among the roots' query times; together with the
     graph's own timestamp range it fixes the width of the (id, ts) sort key.  When omitted it is read from
     ``root_ts`` (one extra synchronisation).
 
-    ``side_streams`` (two streams): the independent chains of the construction run side by side -- hop l+1 samples the
-    raw output of hop l, so the sampling of all hops proceeds while the relabel of the earlier hops is still sorting, and
-    the CSC's sort (keyed by destination row and time) runs next to the relabel's sort; only its column indices need the
-    relabel's result, and they are filled in with one gather at the end.  Everything is joined into the current stream
-    before the function returns.  Captured into a CUDA graph this becomes a graph with parallel branches.
+    Hop l+1 samples the raw output of hop l, and a hop's CSC needs the relabel before it but not its own: with several hops
+    both run on a second stream (``side_streams[0]``, default: one per thread) next to the relabels, and are joined into
+    the current stream.  Captured into a CUDA graph this becomes a graph with parallel branches.
     """
-    dev = g.device
-    status = status or ops.StatusWord(dev)
     if ts_range is None:
-        if root_ts.numel():
-            lo, hi = root_ts.aminmax()
-            ts_range = (int(lo.item()), int(hi.item()))
-        else:
-            ts_range = (g.ts_min, g.ts_max)
-    ts_base = min(g.ts_min, int(ts_range[0]))
-    ts_bits = ops.bits_for(max(g.ts_max, int(ts_range[1])) - ts_base)
-    id_bits = ops.bits_for(g.num_nodes - 1)
-    main = torch.cuda.current_stream(dev)
-    s_sample, s_csc = (side_streams[0], side_streams[1]) if side_streams else (main, main)
+        ts_range = _root_range(g, root_ts)
+    lo, hi = _graph_range(g, int(ts_range[0]), int(ts_range[1]))
+    fanouts = list(fanouts)
+    side = side_streams[0] if side_streams else (_side_stream(g.device) if len(fanouts) > 1 else None)
+    return _enqueue(g, roots, root_ts, fanouts, policy, lo, hi, equal_root_time, allowed_offset, seed, status, side)
 
-    def after(stream_done, stream_wait):
-        if stream_done is not stream_wait:
-            ev = torch.cuda.Event()
-            ev.record(stream_done)
-            stream_wait.wait_event(ev)
 
-    cur_id, cur_ts, inv0, _, d_cur = ops.unique_pairs(roots, root_ts, id_bits=id_bits, ts_bits=ts_bits, ts_base=ts_base,
-                                                      status=status)
-    layers = [{"gids": cur_id, "ts": cur_ts, "inv_map": inv0[:roots.numel()]}]
-    counts = [d_cur]
-    # the sampling chain: hop 0 queries the layer-0 list, hop l+1 one target per edge sampled by hop l at that edge's
-    # timestamp (prepare_sample.py:345-346) -- no hop waits for a relabel but the first
-    after(main, s_sample)
-    hops = []
-    tgt, tgt_ts, d_tgt = cur_id, cur_ts, d_cur
-    with torch.cuda.stream(s_sample):
-        for l, k in enumerate(fanouts):
-            hop = ops.sample_layer(g, tgt, tgt_ts, k, policy, d_n=d_tgt, equal_root_time=equal_root_time,
-                                   allowed_offset=allowed_offset, seed=seed, rng_stream=l, status=status)
-            hops.append(hop)
-            tgt, tgt_ts, d_tgt = hop.nbr, hop.ts, hop.d_total
-    after(s_sample, main)
-    if side_streams and len(hops) > 1:          # (a stream that joins a capture has to be joined back: only fork it for work)
-        after(s_sample, s_csc)
-    last_inv = None
-    pending = []
-    for l, hop in enumerate(hops):
-        cap_cur = cur_id.numel()
-        first = last_inv is None
-        if not first and side_streams:
-            # CSC of a later hop: its order does not depend on this hop's relabel -- sort it on the side with the edge
-            # number as column index, translate the columns once the relabel is there
-            after(main, s_csc)                      # last_inv / d_cur of the previous relabel
-            with torch.cuda.stream(s_csc):
-                iota = torch.arange(hop.capacity, dtype=torch.int64, device=dev)
-                indptr, edge_no, e_ts, e_dt, e_eid = ops.build_csc(iota, hop.dst, last_inv, hop.ts, hop.dt, hop.eid, cap_cur,
-                                                                   dst_bits=ops.bits_for(cap_cur), ts_bits=ts_bits,
-                                                                   ts_base=ts_base, d_n_edges=hop.d_total, d_num_dst=d_cur,
-                                                                   status=status)
-        nxt_id, nxt_ts, _, nxt_inv, d_nxt = ops.unique_pairs(cur_id, cur_ts, hop.nbr, hop.ts, id_bits=id_bits,
-                                                             ts_bits=ts_bits, ts_base=ts_base, d_n_a=d_cur,
-                                                             d_n_b=hop.d_total, status=status)
-        if first or not side_streams:
-            indptr, idx, e_ts, e_dt, e_eid = ops.build_csc(nxt_inv, hop.dst, last_inv, hop.ts, hop.dt, hop.eid, cap_cur,
-                                                           dst_bits=ops.bits_for(cap_cur), ts_bits=ts_bits, ts_base=ts_base,
-                                                           d_n_edges=hop.d_total, d_num_dst=d_cur, presorted=first,
-                                                           status=status)
-        else:
-            after(s_csc, main)
-            idx = ops.gather_rows(nxt_inv, edge_no, d_n=hop.d_total, status=status)
-        layers.append({"indptr": indptr, "indices": idx, "eid": e_eid, "edge_ts": e_ts, "edge_dt": e_dt,
-                       "gids": nxt_id, "ts": nxt_ts, "raw_nbr": hop.nbr, "raw_ts": hop.ts, "inv": nxt_inv, "hop": hop})
-        counts += [hop.d_total, d_nxt]
-        cur_id, cur_ts, d_cur, last_inv = nxt_id, nxt_ts, d_nxt, nxt_inv
-    return DeviceBatch(g, layers, counts, status, fanouts, None)
+def _root_range(g, root_ts):
+    if not root_ts.numel():
+        return g.ts_min, g.ts_max
+    lo, hi = torch.stack(root_ts.aminmax()).tolist()
+    return lo, hi
 
 
 def build_batch(g, roots, root_ts, fanouts, policy="recent", **kw) -> List[dict]:
     """Synchronous form of :func:`build_batch_async`."""
-    return build_batch_async(g, roots, root_ts, fanouts, policy, **kw).finish()
+    if kw.get("ts_range") is not None or kw.get("status") is not None:
+        return build_batch_async(g, roots, root_ts, fanouts, policy, **kw).finish()
+    # Query times nearly always lie in the graph's own time range (events of the stream): the batch is enqueued with the
+    # range known so far instead of waiting for the smallest and largest query time.  The kernels flag a time outside of
+    # it; then the range is read, kept on the graph, and the batch built again.
+    lo, hi = g.__dict__.get("_query_range", (g.ts_min, g.ts_max))
+    kw.pop("ts_range", None)
+    db = build_batch_async(g, roots, root_ts, fanouts, policy, ts_range=(lo, hi), **kw)
+    host, bits = db._read()
+    if bits & 2:
+        a, b = _root_range(g, root_ts)
+        g.__dict__["_query_range"] = (min(lo, a), max(hi, b))
+        return build_batch_async(g, roots, root_ts, fanouts, policy, ts_range=(a, b), **kw).finish()
+    if bits:
+        raise _C.SglError(f"build_batch: device status {bits} ({_C.decode_status(bits)})")
+    return db._trim(host)
 
 
 def batch_kernel_launches(num_nodes: int, num_roots: int, fanouts: Sequence[int], ts_span: int) -> int:
-    """Kernels of this library that one mini-batch of :func:`build_batch_async` launches at the given capacities (pack,
-    sort, head scan and emit of every relabel; count and fill of every hop; pack, sort and emit of every CSC after the
-    first, which needs no sort).  Counted from the structure of the calls; the sorts' share comes from the library."""
-    from .. import _C
+    """Kernels of this library that one mini-batch of :func:`build_batch_async` launches at the given capacities: count and
+    fill of every hop, the sort of every relabel and of every CSC after the first (with pack, head scan and emit kernels
+    around it only for lists above the mini-batch sort's limit)."""
     L = _C.lib()
     id_bits, ts_bits = ops.bits_for(num_nodes - 1), ops.bits_for(ts_span)
-    total = 3 + L.sgl_radix_sort_launches(num_roots, id_bits + ts_bits)          # relabel of the roots
+
+    def sort(n, bits, around):
+        k = L.sgl_radix_sort_launches(n, bits)
+        return k if k <= 2 else k + around
+    total = sort(num_roots, id_bits + ts_bits, 3)
     cur, targets = num_roots, num_roots
     for l, k in enumerate(fanouts):
         edges = targets * k
-        total += 2                                                               # count + fill
-        total += 3 + L.sgl_radix_sort_launches(cur + edges, id_bits + ts_bits)   # merged list of the hop
-        # CSC: a copy for the first hop; pack, sort, emit and the gather that fills in the column indices for the others
-        total += 1 if l == 0 else 3 + L.sgl_radix_sort_launches(edges, ops.bits_for(cur) + ts_bits)
+        total += 2 + sort(cur + edges, id_bits + ts_bits, 3)
+        total += 0 if l == 0 else 1 + sort(edges, ops.bits_for(cur) + ts_bits, 2)
         cur, targets = cur + edges, edges
     return int(total)
 
 
 class BatchGraph:
     """The whole multi-hop batch construction of :func:`build_batch_async` captured once as a CUDA graph for a fixed
-    number of roots, and replayed per mini-batch: one launch instead of about a hundred small ones (the pipeline is a
-    chain of short sort / scan / emit kernels, so at mini-batch sizes it is bound by launch overhead, not by the GPU).
+    number of roots, and replayed per mini-batch: one launch instead of a dozen small ones.
 
     The result tensors are the same objects for every batch: consume (or copy) a result before the next ``run``.
     """
@@ -181,14 +274,13 @@ class BatchGraph:
     def __init__(self, g: ops.TCSR, num_roots: int, fanouts: Sequence[int], policy: str = "recent", *,
                  ts_range: Sequence[int], equal_root_time=False, allowed_offset=-1, seed=0,
                  stream: Optional[torch.cuda.Stream] = None):
-        from .. import _C
         dev = g.device
         self.g, self.num_roots = g, int(num_roots)
         self.stream = stream or torch.cuda.Stream(dev)
         self.roots = torch.zeros(self.num_roots, dtype=torch.int64, device=dev)
         self.root_ts = torch.full((self.num_roots,), int(ts_range[0]), dtype=torch.int64, device=dev)
         self.status = ops.StatusWord(dev)
-        self._side = [torch.cuda.Stream(dev), torch.cuda.Stream(dev)]
+        self._side = [torch.cuda.Stream(dev)]
         kw = dict(ts_range=ts_range, equal_root_time=equal_root_time, allowed_offset=allowed_offset, seed=seed,
                   status=self.status, side_streams=self._side)
         # scratch used inside the graph must not be shared with eager calls: the capture gets its own workspace

@@ -545,7 +545,8 @@ int sgl_lower_bound_i64(const int64_t* sorted, int64_t n, const int64_t* values,
  *                     merged list; CSC indptr, indices, ts, dt (fp32), eid (absent for the first hop: its edges are in
  *                     CSC order already, with `offsets` as the row pointer)
  * meta[2 + 2 * n_hops] = {size of the root list, then per hop sampled edges and size of the merged list, status word}; the
- * status word is used when d_status is NULL.  side_stream (optional): hops after the first and their CSC run there,
+ * status word is used when d_status is NULL.  host_meta (optional, pinned, 3 + 2 * n_hops words): receives meta when the
+ * batch is done and then a 1 behind it (see sgl_wait_word).  side_stream (optional): hops after the first and their CSC run there,
  * next to the relabels; everything is joined into `stream`.
  * Replaces: build_aligned_batch's per-layer loop (prepare_sample.py:313-377).
  * ---------------------------------------------------------------------------------------------- */
@@ -555,9 +556,13 @@ int sgl_build_batch(const int64_t* indptr, const int64_t* nbr, const int64_t* ts
                     int64_t num_nodes, const int64_t* roots, const int64_t* root_ts, int64_t n_roots,
                     const int32_t* fanouts, int n_hops, int policy, int equal_root_time, int64_t allowed_offset,
                     uint64_t seed, int id_bits, int ts_bits, int64_t ts_base, int64_t* arena, int64_t* meta,
-                    int32_t* d_status, void* ws, size_t ws_bytes, void* side_stream, void* stream);
+                    int32_t* d_status, int64_t* host_meta, void* ws, size_t ws_bytes, void* side_stream, void* stream);
 
-/* Copies up to 4,096 bytes of device memory to (pageable) host memory and waits for the stream. */
+/* Small results for the host.  sgl_host_words: a pinned buffer of 512 words that belongs to the calling thread.
+ * sgl_wait_word: waits until work on the stream has set *flag (pinned memory).  sgl_read_back: copies up to 511 words of
+ * device memory to the host through that buffer and waits for them. */
+int sgl_host_words(void** out);
+int sgl_wait_word(const int64_t* flag, void* stream);
 int sgl_read_back(const void* src, void* dst, size_t bytes, void* stream);
 
 /* ------------------------------------------------------------------------------------------------

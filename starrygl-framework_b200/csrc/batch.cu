@@ -14,6 +14,7 @@
 // Meta (8-byte words): entries of the root list, then per hop sampled edges and entries of the merged list, then a status
 // word (used when the caller has none of its own).
 
+#include "launch.cuh"
 #include "sampler.cuh"
 #include "sort.cuh"
 #include "tilesort.cuh"
@@ -23,6 +24,7 @@ using namespace sgl;
 namespace {
 
 constexpr int kMaxHops = 8;
+constexpr int kHostWords = 512;
 constexpr int kRootSections = 3, kHopSections = 14;
 
 inline int64_t words(int64_t n) { return ((n < 1 ? 1 : n) + 31) / 32 * 32; }
@@ -90,23 +92,57 @@ size_t csc_ws(int64_t n, const int32_t* fanouts, int hops) {
   return align_up(most);
 }
 
-// events of this thread for the fork and join of the side stream (recorded and waited for at once, so reusable)
-cudaError_t thread_event(int i, cudaEvent_t* out) {
-  static thread_local cudaEvent_t ev[64][4];
-  int dev = 0;
-  cudaError_t e = cudaGetDevice(&dev);
-  if (e != cudaSuccess) return e;
-  cudaEvent_t& slot = ev[dev & 63][i];
-  if (slot == nullptr) e = cudaEventCreateWithFlags(&slot, cudaEventDisableTiming);
-  *out = slot;
-  return e;
-}
+// Order between the two streams of a batch: nodes of the launch scope, or (captured calls) events of this thread, recorded
+// and waited for at once and so reusable.
+struct Order {
+  static constexpr int kMarks = 4;
+  LaunchScope* scope;
+  std::vector<int> nodes[kMarks];
+  cudaEvent_t ev[kMarks];
+
+  int init(LaunchScope* s) {
+    scope = s;
+    if (scope) return SGL_OK;
+    static thread_local cudaEvent_t pool[64][kMarks];
+    int dev = 0;
+    SGL_CUDA_CHECK(cudaGetDevice(&dev));
+    for (int i = 0; i < kMarks; ++i) {
+      cudaEvent_t& e = pool[dev & 63][i];
+      if (e == nullptr) SGL_CUDA_CHECK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+      ev[i] = e;
+    }
+    return SGL_OK;
+  }
+  int mark(int i, cudaStream_t s) {
+    if (scope) nodes[i] = scope->mark(s);
+    else SGL_CUDA_CHECK(cudaEventRecord(ev[i], s));
+    return SGL_OK;
+  }
+  int wait(int i, cudaStream_t s) {
+    if (scope) scope->wait(s, nodes[i]);
+    else SGL_CUDA_CHECK(cudaStreamWaitEvent(s, ev[i], 0));
+    return SGL_OK;
+  }
+};
 
 // indices[j] = col[indices[j]]: edge numbers -> positions in the merged list
 __global__ void __launch_bounds__(256)
 map_columns_kernel(int64_t* __restrict__ indices, const int64_t* __restrict__ col, int64_t n_cap, const int64_t* d_n) {
   const int64_t n = eff_count(n_cap, d_n), stride = (int64_t)gridDim.x * 256;
   for (int64_t j = (int64_t)blockIdx.x * 256 + threadIdx.x; j < n; j += stride) indices[j] = __ldg(col + indices[j]);
+}
+
+// words of device memory -> pinned host memory, then the flag behind them
+__global__ void export_words_kernel(const int64_t* __restrict__ src, int64_t* dst, int words) {
+  for (int i = threadIdx.x; i < words; i += blockDim.x) dst[i] = src[i];
+  __threadfence_system();
+  __syncthreads();
+  if (threadIdx.x == 0) *(volatile int64_t*)(dst + words) = 1;
+}
+
+int export_words(const int64_t* src, int64_t* dst, int words, cudaStream_t stream) {
+  *(volatile int64_t*)(dst + words) = 0;
+  return launch(export_words_kernel, 1, 32, 0, stream, src, dst, words);
 }
 
 }  // namespace
@@ -127,15 +163,20 @@ extern "C" int sgl_build_batch(const int64_t* indptr, const int64_t* nbr, const 
                                int64_t num_nodes, const int64_t* roots, const int64_t* root_ts, int64_t n_roots,
                                const int32_t* fanouts, int n_hops, int policy, int equal_root_time, int64_t allowed_offset,
                                uint64_t seed, int id_bits, int ts_bits, int64_t ts_base, int64_t* arena, int64_t* meta,
-                               int32_t* d_status, void* ws, size_t ws_bytes, void* side_stream, void* stream_) {
+                               int32_t* d_status, int64_t* host_meta, void* ws, size_t ws_bytes, void* side_stream, void* stream_) {
   SGL_NVTX("sgl_build_batch");
   cudaStream_t stream = (cudaStream_t)stream_;
   SGL_REQUIRE(n_roots >= 0 && n_hops >= 0 && n_hops <= kMaxHops && (n_hops == 0 || fanouts), SGL_ERR_ARG,
               "build_batch: bad size (at most %d hops)", kMaxHops);
   for (int l = 0; l < n_hops; ++l) SGL_REQUIRE(fanouts[l] >= 1, SGL_ERR_ARG, "build_batch: fanout=%d must be >= 1", fanouts[l]);
   SGL_REQUIRE(meta, SGL_ERR_ARG, "build_batch: meta is null");
-  SGL_CUDA_CHECK(cudaMemsetAsync(meta, 0, (size_t)(2 + 2 * n_hops) * sizeof(int64_t), stream));
-  if (n_roots == 0) return SGL_OK;
+  LaunchScope scope(stream);
+  SGL_CHECK_RC(zero_async(meta, (size_t)(2 + 2 * n_hops) * sizeof(int64_t), stream));
+  auto done = [&]() -> int {
+    if (host_meta) SGL_CHECK_RC(export_words(meta, host_meta, 2 + 2 * n_hops, stream));
+    return scope.submit();
+  };
+  if (n_roots == 0) return done();
   SGL_REQUIRE(arena && roots && root_ts, SGL_ERR_ARG, "build_batch: null array");
   SGL_REQUIRE(ws_bytes >= sgl_build_batch_ws_bytes(n_roots, fanouts, n_hops), SGL_ERR_WORKSPACE, "build_batch: workspace %zu < %zu bytes",
               ws_bytes, sgl_build_batch_ws_bytes(n_roots, fanouts, n_hops));
@@ -171,17 +212,18 @@ extern "C" int sgl_build_batch(const int64_t* indptr, const int64_t* nbr, const 
                         seed, (uint32_t)l, h.nbr, h.dst, h.ts, h.dt, nullptr, h.eid, h.offs, meta + 1 + 2 * l, d_status, sws, swb, on);
   };
   // Hop l + 1 queries one target per edge sampled by hop l at that edge's time and waits for no relabel but the first; the
-  // CSC of a hop needs the relabel before it but not its own (its columns are translated at the end).  With a side stream
-  // both run there, next to the relabels: 4,096 roots uniform [10, 10] 168 us of kernels in a row, 120 side by side.
+  // CSC of a hop needs the relabel before it but not its own (its columns are translated at the end).  Where they can
+  // both run on a second stream, next to the relabels: 4,096 roots uniform [10, 10] 168 us of kernels in a row, 120 side by side.
   if (n_hops > 0 && (rc = sample(0, cur_id, cur_ts, n_roots, meta, stream))) return rc;
-  const bool forked = n_hops > 1 && side_stream != nullptr && side_stream != stream_;
-  cudaStream_t side = forked ? (cudaStream_t)side_stream : stream;
-  cudaEvent_t ev[4] = {nullptr, nullptr, nullptr, nullptr};
+  const bool forked = n_hops > 1 && (LaunchScope::current() != nullptr || (side_stream != nullptr && side_stream != stream_));
+  // (inside a launch scope a stream is only a name for a chain of kernels)
+  cudaStream_t side = forked ? (side_stream ? (cudaStream_t)side_stream : (cudaStream_t)(uintptr_t)3) : stream;
   enum { kFork, kSampled, kRelabelled, kCsc };
+  Order order;
   if (forked) {
-    for (int i = 0; i < 4; ++i) SGL_CUDA_CHECK(thread_event(i, &ev[i]));
-    SGL_CUDA_CHECK(cudaEventRecord(ev[kFork], stream));
-    SGL_CUDA_CHECK(cudaStreamWaitEvent(side, ev[kFork], 0));
+    SGL_CHECK_RC(order.init(LaunchScope::current()));
+    SGL_CHECK_RC(order.mark(kFork, stream));
+    SGL_CHECK_RC(order.wait(kFork, side));
   }
   int64_t t = n_roots, c = n_roots;
   const int64_t* d_cur = meta;
@@ -190,26 +232,26 @@ extern "C" int sgl_build_batch(const int64_t* indptr, const int64_t* nbr, const 
     const Hop& h = hop[l];
     const int64_t e = t * fanouts[l];
     int64_t *d_edges = meta + 1 + 2 * l, *d_next = meta + 2 + 2 * l;
-    if (forked && l > 0) SGL_CUDA_CHECK(cudaStreamWaitEvent(stream, ev[kSampled], 0));
+    if (forked && l > 0) SGL_CHECK_RC(order.wait(kSampled, stream));
     if (l + 1 < n_hops) {
       if ((rc = sample(l + 1, h.nbr, h.ts, e, d_edges, side))) return rc;
-      if (forked) SGL_CUDA_CHECK(cudaEventRecord(ev[kSampled], side));
+      if (forked) SGL_CHECK_RC(order.mark(kSampled, side));
     }
     if (l > 0) {
-      if (forked) SGL_CUDA_CHECK(cudaStreamWaitEvent(side, ev[kRelabelled], 0));
+      if (forked) SGL_CHECK_RC(order.wait(kRelabelled, side));
       rc = sgl_build_csc(nullptr, h.dst, last_col, h.ts, h.dt, h.eid, e, d_edges, c, d_cur, bits_for((uint64_t)c), ts_bits, ts_base,
                          h.indptr, h.indices, h.cts, h.cdt, h.ceid, 0, d_status, cws, cwb, side);
       if (rc) return rc;
-      if (forked) SGL_CUDA_CHECK(cudaEventRecord(ev[kCsc], side));
+      if (forked) SGL_CHECK_RC(order.mark(kCsc, side));
     }
     rc = sgl_unique_pairs(cur_id, cur_ts, c, d_cur, h.nbr, h.ts, e, d_edges, id_bits, ts_bits, ts_base, h.gids, h.gts, nullptr, h.col,
                           d_next, d_status, lws, lwb, stream);
     if (rc) return rc;
-    if (forked && l + 1 < n_hops) SGL_CUDA_CHECK(cudaEventRecord(ev[kRelabelled], stream));
+    if (forked && l + 1 < n_hops) SGL_CHECK_RC(order.mark(kRelabelled, stream));
     if (l > 0) {
-      if (forked) SGL_CUDA_CHECK(cudaStreamWaitEvent(stream, ev[kCsc], 0));
-      map_columns_kernel<<<stream_grid(e, 256 * 4, 8), 256, 0, stream>>>(h.indices, h.col, e, d_edges);
-      SGL_LAUNCH_CHECK();
+      if (forked) SGL_CHECK_RC(order.wait(kCsc, stream));
+      SGL_CHECK_RC(launch(map_columns_kernel, stream_grid(e, 256 * 4, 8), 256, 0, stream, h.indices, h.col, e, d_edges));
+    
     }
     cur_id = h.gids;
     cur_ts = h.gts;
@@ -218,18 +260,43 @@ extern "C" int sgl_build_batch(const int64_t* indptr, const int64_t* nbr, const 
     t = e;
     c += e;
   }
+  return done();
+}
+
+// Pinned buffer of the calling thread (4,096 bytes) for results that the host waits for.
+extern "C" int sgl_host_words(void** out) {
+  SGL_REQUIRE(out, SGL_ERR_ARG, "host_words: out is null");
+  static thread_local void* pinned = nullptr;
+  if (pinned == nullptr) SGL_CUDA_CHECK(cudaHostAlloc(&pinned, kHostWords * 8, cudaHostAllocPortable));
+  *out = pinned;
   return SGL_OK;
 }
 
-// Copies up to 4 KB of device memory to the host and waits for the stream: through a pinned buffer of the calling thread
-// (a copy to pageable memory is staged by the driver, 10 us more).
-extern "C" int sgl_read_back(const void* src, void* dst, size_t bytes, void* stream) {
-  constexpr size_t kBytes = 4096;
-  SGL_REQUIRE(src && dst && bytes <= kBytes, SGL_ERR_ARG, "read_back: at most %zu bytes", kBytes);
-  static thread_local void* pinned = nullptr;
-  if (pinned == nullptr) SGL_CUDA_CHECK(cudaHostAlloc(&pinned, kBytes, cudaHostAllocPortable));
-  SGL_CUDA_CHECK(cudaMemcpyAsync(pinned, src, bytes, cudaMemcpyDeviceToHost, (cudaStream_t)stream));
+// Waits until *flag is set by work on the stream: the host looks at the word itself for a while (a stream
+// synchronisation costs 5 us more than the kernel that it waits for), then waits for the stream, which also reports errors.
+extern "C" int sgl_wait_word(const int64_t* flag, void* stream) {
+  SGL_REQUIRE(flag, SGL_ERR_ARG, "wait_word: flag is null");
+  const volatile int64_t* f = flag;
+  for (int i = 0; i < 2000000; ++i) {
+    if (*f) return SGL_OK;
+#if defined(__x86_64__)
+    __builtin_ia32_pause();
+#endif
+  }
   SGL_CUDA_CHECK(cudaStreamSynchronize((cudaStream_t)stream));
-  memcpy(dst, pinned, bytes);
+  SGL_REQUIRE(*f, SGL_ERR_CUDA, "wait_word: the stream ended without setting the word");
+  return SGL_OK;
+}
+
+// Copies up to 4,088 bytes of device memory (whole 8-byte words) to the host and waits for them.
+extern "C" int sgl_read_back(const void* src, void* dst, size_t bytes, void* stream) {
+  SGL_REQUIRE(src && dst && bytes % 8 == 0 && bytes / 8 < (size_t)kHostWords, SGL_ERR_ARG, "read_back: at most %d words", kHostWords - 1);
+  void* p = nullptr;
+  SGL_CHECK_RC(sgl_host_words(&p));
+  int64_t* host = (int64_t*)p;
+  const int words = (int)(bytes / 8);
+  SGL_CHECK_RC(export_words((const int64_t*)src, host, words, (cudaStream_t)stream));
+  SGL_CHECK_RC(sgl_wait_word(host + words, stream));
+  memcpy(dst, host, bytes);
   return SGL_OK;
 }

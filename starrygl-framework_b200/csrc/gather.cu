@@ -12,6 +12,7 @@
 //   scatter_lanes_kernel    the reverse of the gather, optionally splitting a trailing timestamp column.
 //
 // Algorithmic HBM bytes: rows * (2 * row_bytes + 8) (+4 per id for the hit-map, +16 per miss for the miss list).
+#include "launch.cuh"
 #include "common.cuh"
 #include "scan.cuh"
 
@@ -656,27 +657,25 @@ extern "C" int sgl_gather_rows(const void* table, int64_t table_rows, int64_t ro
     if (ctas > (int64_t)kNumSM * 2) ctas = (int64_t)kNumSM * 2;  // persistent CTAs
     SGL_CUDA_CHECK(cudaFuncSetAttribute(gather_bulk_kernel<kBulkWarps, kBulkStages>,
                                         cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
-    gather_bulk_kernel<kBulkWarps, kBulkStages><<<(unsigned)ctas, kBulkWarps * 32, smem, stream>>>(
-        (const char*)table, table_rows, (uint32_t)row_bytes, src_pitch, idx, map, map_len, n, d_n, (char*)out, ts_table,
-        out_ts, rows_per_stage, d_status);
-    SGL_LAUNCH_CHECK();
+    SGL_CHECK_RC(launch(gather_bulk_kernel<kBulkWarps, kBulkStages>, (unsigned)ctas, kBulkWarps * 32, smem, stream, (const
+                        char*)table, table_rows, (uint32_t)row_bytes, src_pitch, idx, map, map_len, n, d_n, (char*)out,
+                        ts_table, out_ts, rows_per_stage, d_status));
     return SGL_OK;
   }
   if (mode == SGL_GATHER_VEC) {
     SGL_REQUIRE(vec_ok, SGL_ERR_UNSUPPORTED, "gather_rows: 128-bit mode needs 16-byte aligned rows");
     const uint32_t lanes = (uint32_t)(row_bytes / 16);
     const int grid = stream_grid(n * lanes, kLaneThreads * kLaneUnroll, 8);
-    gather_lanes_kernel<uint4><<<grid, kLaneThreads, 0, stream>>>((const char*)table, table_rows, LaneSplit(lanes, n * lanes), src_pitch, idx,
-                                                                 map, map_len, n, d_n, (char*)out, dst_pitch, ts_table,
-                                                                 out_ts, d_status);
+    SGL_CHECK_RC(launch(gather_lanes_kernel<uint4>, grid, kLaneThreads, 0, stream, (const char*)table, table_rows,
+                        LaneSplit(lanes, n * lanes), src_pitch, idx, map, map_len, n, d_n, (char*)out, dst_pitch, ts_table,
+                        out_ts, d_status));
   } else {
     const uint32_t lanes = (uint32_t)(row_bytes / 4);
     const int grid = stream_grid(n * lanes, kLaneThreads * kLaneUnroll, 8);
-    gather_lanes_kernel<uint32_t><<<grid, kLaneThreads, 0, stream>>>((const char*)table, table_rows, LaneSplit(lanes, n * lanes), src_pitch,
-                                                                    idx, map, map_len, n, d_n, (char*)out, dst_pitch,
-                                                                    ts_table, out_ts, d_status);
+    SGL_CHECK_RC(launch(gather_lanes_kernel<uint32_t>, grid, kLaneThreads, 0, stream, (const char*)table, table_rows,
+                        LaneSplit(lanes, n * lanes), src_pitch, idx, map, map_len, n, d_n, (char*)out, dst_pitch, ts_table,
+                        out_ts, d_status));
   }
-  SGL_LAUNCH_CHECK();
   return SGL_OK;
 }
 
@@ -698,8 +697,7 @@ extern "C" int sgl_copy_prefix(int n_arrays, const void* const* src, void* const
     const int64_t b = elem_bytes[a] < 0 ? -elem_bytes[a] : cap * elem_bytes[a];
     most = most > b ? most : b;
   }
-  copy_prefix_kernel<<<stream_grid(most / 16 + 1, 256 * 4, 2), 256, 0, stream>>>(pc, d_count, cap);
-  SGL_LAUNCH_CHECK();
+  SGL_CHECK_RC(launch(copy_prefix_kernel, stream_grid(most / 16 + 1, 256 * 4, 2), 256, 0, stream, pc, d_count, cap));
   return SGL_OK;
 }
 
@@ -718,10 +716,11 @@ extern "C" int sgl_cache_gather(const void* cache_rows, int64_t cache_slots, con
   SGL_REQUIRE(n >= 0 && row_bytes > 0 && row_bytes % 4 == 0, SGL_ERR_ARG, "cache_gather: bad size");
   SGL_REQUIRE(d_counts, SGL_ERR_ARG, "cache_gather: d_counts is null");
   if (n == 0) {
-    SGL_CUDA_CHECK(cudaMemsetAsync(d_counts, 0, 2 * sizeof(int64_t), stream));
+    SGL_CHECK_RC(zero_async(d_counts, 2 * sizeof(int64_t), stream));
     return SGL_OK;
   }
   SGL_REQUIRE(cache_rows && hitmap && ids && out && miss_pos && miss_ids, SGL_ERR_ARG, "cache_gather: null array");
+  LaunchScope scope(stream);
   WsCarver c(ws, ws_bytes);
   int32_t* slot_ws = c.take<int32_t>(n);
   int32_t* rank_ws = c.take<int32_t>(n);
@@ -729,26 +728,24 @@ extern "C" int sgl_cache_gather(const void* cache_rows, int64_t cache_slots, con
   int64_t* cta_miss = c.take<int64_t>(ctas);
   unsigned int* done = c.take<unsigned int>(1);
   SGL_REQUIRE(c.ok(), SGL_ERR_WORKSPACE, "cache_gather: workspace %zu < %zu bytes", ws_bytes, sgl_cache_gather_ws_bytes(n));
-  SGL_CUDA_CHECK(cudaMemsetAsync(done, 0, sizeof(unsigned int), stream));
-  cache_lookup_kernel<<<(unsigned)ctas, kCacheThreads, 0, stream>>>(hitmap, num_ids, ids, n, slot_ws, rank_ws, cta_miss,
-                                                                   done, d_counts, d_status);
+  SGL_CHECK_RC(zero_async(done, sizeof(unsigned int), stream));
+  SGL_CHECK_RC(launch(cache_lookup_kernel, (unsigned)ctas, kCacheThreads, 0, stream, hitmap, num_ids, ids, n, slot_ws,
+                      rank_ws, cta_miss, done, d_counts, d_status));
   const bool vec_ok = row_bytes % 16 == 0 && aligned16(cache_rows) && aligned16(out) && (backing == nullptr || aligned16(backing));
   if (vec_ok) {
     const uint32_t lanes = (uint32_t)(row_bytes / 16);
     const int grid = stream_grid(n * lanes, kLaneThreads * kLaneUnroll, 8);
-    cache_copy_kernel<uint4><<<grid, kLaneThreads, 0, stream>>>((const char*)cache_rows, cache_slots, (const char*)backing,
-                                                               LaneSplit(lanes, n * lanes), row_bytes, ids, n, slot_ws, rank_ws, cta_miss,
-                                                               (char*)out, miss_pos, miss_ids, d_counts, d_status);
+    SGL_CHECK_RC(launch(cache_copy_kernel<uint4>, grid, kLaneThreads, 0, stream, (const char*)cache_rows, cache_slots, (const
+                        char*)backing, LaneSplit(lanes, n * lanes), row_bytes, ids, n, slot_ws, rank_ws, cta_miss,
+                        (char*)out, miss_pos, miss_ids, d_counts, d_status));
   } else {
     const uint32_t lanes = (uint32_t)(row_bytes / 4);
     const int grid = stream_grid(n * lanes, kLaneThreads * kLaneUnroll, 8);
-    cache_copy_kernel<uint32_t><<<grid, kLaneThreads, 0, stream>>>((const char*)cache_rows, cache_slots,
-                                                                  (const char*)backing, LaneSplit(lanes, n * lanes), row_bytes, ids, n, slot_ws,
-                                                                  rank_ws, cta_miss, (char*)out, miss_pos, miss_ids,
-                                                                  d_counts, d_status);
+    SGL_CHECK_RC(launch(cache_copy_kernel<uint32_t>, grid, kLaneThreads, 0, stream, (const char*)cache_rows, cache_slots,
+                        (const char*)backing, LaneSplit(lanes, n * lanes), row_bytes, ids, n, slot_ws, rank_ws, cta_miss,
+                        (char*)out, miss_pos, miss_ids, d_counts, d_status));
   }
-  SGL_LAUNCH_CHECK();
-  return SGL_OK;
+  return scope.submit();
 }
 
 extern "C" int sgl_scatter_rows(void* table, int64_t table_rows, int64_t row_bytes, int64_t dst_pitch, const int64_t* idx,
@@ -767,17 +764,16 @@ extern "C" int sgl_scatter_rows(void* table, int64_t table_rows, int64_t row_byt
   if (vec_ok) {
     const uint32_t lanes = (uint32_t)(row_bytes / 16);
     const int grid = stream_grid(n * lanes, kLaneThreads, 16);
-    scatter_lanes_kernel<uint4><<<grid, kLaneThreads, 0, stream>>>((char*)table, table_rows, lanes, row_bytes, dst_pitch, idx,
-                                                                  map, map_len, n, d_n, (const char*)rows, src_pitch,
-                                                                  ts_table, ts, split_last_col, d_status);
+    SGL_CHECK_RC(launch(scatter_lanes_kernel<uint4>, grid, kLaneThreads, 0, stream, (char*)table, table_rows, lanes,
+                        row_bytes, dst_pitch, idx, map, map_len, n, d_n, (const char*)rows, src_pitch, ts_table, ts,
+                        split_last_col, d_status));
   } else {
     const uint32_t lanes = (uint32_t)(row_bytes / 4);
     const int grid = stream_grid(n * lanes, kLaneThreads, 16);
-    scatter_lanes_kernel<uint32_t><<<grid, kLaneThreads, 0, stream>>>((char*)table, table_rows, lanes, row_bytes, dst_pitch,
-                                                                     idx, map, map_len, n, d_n, (const char*)rows,
-                                                                     src_pitch, ts_table, ts, split_last_col, d_status);
+    SGL_CHECK_RC(launch(scatter_lanes_kernel<uint32_t>, grid, kLaneThreads, 0, stream, (char*)table, table_rows, lanes,
+                        row_bytes, dst_pitch, idx, map, map_len, n, d_n, (const char*)rows, src_pitch, ts_table, ts,
+                        split_last_col, d_status));
   }
-  SGL_LAUNCH_CHECK();
   return SGL_OK;
 }
 
@@ -798,14 +794,13 @@ extern "C" int sgl_route_pack(const float* feats, int64_t n_rows, int64_t dim, c
   const bool vec = dim % 4 == 0 && pitch % 4 == 0 && aligned16(feats) && aligned16(packed);
   if (vec) {
     const int grid = stream_grid(n_send * (pitch / 4), kLaneThreads, 16);
-    route_pack_kernel<4><<<grid, kLaneThreads, 0, stream>>>(feats, n_rows, (uint32_t)dim, ts, send_idx, remote_idx, n_send,
-                                                           (uint32_t)pitch, packed, d_status);
+    SGL_CHECK_RC(launch(route_pack_kernel<4>, grid, kLaneThreads, 0, stream, feats, n_rows, (uint32_t)dim, ts, send_idx,
+                        remote_idx, n_send, (uint32_t)pitch, packed, d_status));
   } else {
     const int grid = stream_grid(n_send * pitch, kLaneThreads, 16);
-    route_pack_kernel<1><<<grid, kLaneThreads, 0, stream>>>(feats, n_rows, (uint32_t)dim, ts, send_idx, remote_idx, n_send,
-                                                           (uint32_t)pitch, packed, d_status);
+    SGL_CHECK_RC(launch(route_pack_kernel<1>, grid, kLaneThreads, 0, stream, feats, n_rows, (uint32_t)dim, ts, send_idx,
+                        remote_idx, n_send, (uint32_t)pitch, packed, d_status));
   }
-  SGL_LAUNCH_CHECK();
   return SGL_OK;
 }
 
@@ -823,14 +818,13 @@ extern "C" int sgl_route_unpack(const float* packed, int64_t n, int64_t width, f
   const bool vec = dim % 4 == 0 && aligned16(packed) && aligned16(data);
   if (vec) {
     const int grid = stream_grid(n * ((width + 3) / 4), kLaneThreads, 16);
-    route_unpack_kernel<4><<<grid, kLaneThreads, 0, stream>>>(packed, n, (uint32_t)width, (uint32_t)pitch, data, data_rows,
-                                                             (uint32_t)dim, ts_table, d_status);
+    SGL_CHECK_RC(launch(route_unpack_kernel<4>, grid, kLaneThreads, 0, stream, packed, n, (uint32_t)width, (uint32_t)pitch,
+                        data, data_rows, (uint32_t)dim, ts_table, d_status));
   } else {
     const int grid = stream_grid(n * width, kLaneThreads, 16);
-    route_unpack_kernel<1><<<grid, kLaneThreads, 0, stream>>>(packed, n, (uint32_t)width, (uint32_t)pitch, data, data_rows,
-                                                             (uint32_t)dim, ts_table, d_status);
+    SGL_CHECK_RC(launch(route_unpack_kernel<1>, grid, kLaneThreads, 0, stream, packed, n, (uint32_t)width, (uint32_t)pitch,
+                        data, data_rows, (uint32_t)dim, ts_table, d_status));
   }
-  SGL_LAUNCH_CHECK();
   return SGL_OK;
 }
 
@@ -841,8 +835,8 @@ extern "C" int sgl_route_add_rows(float* x, int64_t n_rows, int64_t dim, const i
   if (seg_len == 0) return SGL_OK;
   SGL_REQUIRE(x && send_idx && outs, SGL_ERR_ARG, "route_add_rows: null array");
   const int grid = stream_grid(seg_len * dim, kLaneThreads, 16);
-  route_add_kernel<<<grid, kLaneThreads, 0, stream>>>(x, n_rows, (uint32_t)dim, send_idx, outs, seg_len, d_status);
-  SGL_LAUNCH_CHECK();
+  SGL_CHECK_RC(launch(route_add_kernel, grid, kLaneThreads, 0, stream, x, n_rows, (uint32_t)dim, send_idx, outs, seg_len,
+                      d_status));
   return SGL_OK;
 }
 
@@ -854,9 +848,8 @@ extern "C" int sgl_route_add_grouped(float* x, int64_t n_rows, int64_t dim, cons
   if (n_groups == 0) return SGL_OK;
   SGL_REQUIRE(x && rows && row_ptr && pos && outs, SGL_ERR_ARG, "route_add_grouped: null array");
   const int grid = stream_grid(n_groups, kLaneThreads / 32, 16);
-  route_add_grouped_kernel<<<grid, kLaneThreads, 0, stream>>>(x, n_rows, (uint32_t)dim, rows, row_ptr, pos, n_groups, outs,
-                                                             n_outs, d_status);
-  SGL_LAUNCH_CHECK();
+  SGL_CHECK_RC(launch(route_add_grouped_kernel, grid, kLaneThreads, 0, stream, x, n_rows, (uint32_t)dim, rows, row_ptr, pos,
+                      n_groups, outs, n_outs, d_status));
   return SGL_OK;
 }
 
@@ -872,14 +865,15 @@ extern "C" int sgl_shard_gather(const void* const* d_bases, const int64_t* d_sha
   // the shard base pointers are device values: their 16-byte alignment is the caller's contract (cudaMalloc gives 256)
   if (row_bytes % 16 == 0 && aligned16(out)) {
     const uint32_t lanes = (uint32_t)(row_bytes / 16);
-    shard_gather_kernel<uint4><<<stream_grid(n * lanes, kLaneThreads * kLaneUnroll, 8), kLaneThreads, 0, stream>>>(
-        (const char* const*)d_bases, d_shard_rows, world, lanes, row_bytes, dist_idx, n, d_n, (char*)out, d_status);
+    SGL_CHECK_RC(launch(shard_gather_kernel<uint4>, stream_grid(n * lanes, kLaneThreads * kLaneUnroll, 8), kLaneThreads, 0,
+                        stream, (const char* const*)d_bases, d_shard_rows, world, lanes, row_bytes, dist_idx, n, d_n,
+                        (char*)out, d_status));
   } else {
     const uint32_t lanes = (uint32_t)(row_bytes / 4);
-    shard_gather_kernel<uint32_t><<<stream_grid(n * lanes, kLaneThreads * kLaneUnroll, 8), kLaneThreads, 0, stream>>>(
-        (const char* const*)d_bases, d_shard_rows, world, lanes, row_bytes, dist_idx, n, d_n, (char*)out, d_status);
+    SGL_CHECK_RC(launch(shard_gather_kernel<uint32_t>, stream_grid(n * lanes, kLaneThreads * kLaneUnroll, 8), kLaneThreads,
+                        0, stream, (const char* const*)d_bases, d_shard_rows, world, lanes, row_bytes, dist_idx, n, d_n,
+                        (char*)out, d_status));
   }
-  SGL_LAUNCH_CHECK();
   return SGL_OK;
 }
 
@@ -888,8 +882,7 @@ extern "C" int sgl_dist_pack(const int64_t* loc, const int64_t* part, const uint
   SGL_REQUIRE(n >= 0, SGL_ERR_ARG, "dist_pack: negative size");
   if (n == 0) return SGL_OK;
   SGL_REQUIRE(loc && part && dist, SGL_ERR_ARG, "dist_pack: null array");
-  dist_pack_kernel<<<stream_grid(n, 256, 8), 256, 0, (cudaStream_t)stream_>>>(loc, part, shared, n, dist);
-  SGL_LAUNCH_CHECK();
+  SGL_CHECK_RC(launch(dist_pack_kernel, stream_grid(n, 256, 8), 256, 0, (cudaStream_t)stream_, loc, part, shared, n, dist));
   return SGL_OK;
 }
 
@@ -898,8 +891,8 @@ extern "C" int sgl_dist_unpack(const int64_t* dist, int64_t n, int64_t* loc, int
   SGL_REQUIRE(n >= 0, SGL_ERR_ARG, "dist_unpack: negative size");
   if (n == 0) return SGL_OK;
   SGL_REQUIRE(dist, SGL_ERR_ARG, "dist_unpack: null array");
-  dist_unpack_kernel<<<stream_grid(n, 256, 8), 256, 0, (cudaStream_t)stream_>>>(dist, n, loc, part, shared);
-  SGL_LAUNCH_CHECK();
+  SGL_CHECK_RC(launch(dist_unpack_kernel, stream_grid(n, 256, 8), 256, 0, (cudaStream_t)stream_, dist, n, loc, part,
+                      shared));
   return SGL_OK;
 }
 
@@ -918,10 +911,11 @@ extern "C" int sgl_replica_lookup(const int64_t* indptr, const int64_t* ranks, c
   SGL_REQUIRE(n >= 0 && cap >= 0 && num_nodes >= 0, SGL_ERR_ARG, "replica_lookup: negative size");
   SGL_REQUIRE(out_offsets, SGL_ERR_ARG, "replica_lookup: out_offsets is null");
   if (n == 0) {
-    SGL_CUDA_CHECK(cudaMemsetAsync(out_offsets, 0, sizeof(int64_t), stream));
+    SGL_CHECK_RC(zero_async(out_offsets, sizeof(int64_t), stream));
     return SGL_OK;
   }
   SGL_REQUIRE(indptr && ranks && locs && ids && out_src && out_rank && out_loc, SGL_ERR_ARG, "replica_lookup: null array");
+  LaunchScope scope(stream);
   WsCarver c(ws, ws_bytes);
   int64_t* local_off = c.take<int64_t>(n);
   const int64_t ctas = (n + kReplicaThreads - 1) / kReplicaThreads;
@@ -929,12 +923,10 @@ extern "C" int sgl_replica_lookup(const int64_t* indptr, const int64_t* ranks, c
   unsigned int* done = c.take<unsigned int>(1);
   SGL_REQUIRE(c.ok(), SGL_ERR_WORKSPACE, "replica_lookup: workspace %zu < %zu bytes", ws_bytes,
               sgl_replica_lookup_ws_bytes(n));
-  SGL_CUDA_CHECK(cudaMemsetAsync(done, 0, sizeof(unsigned int), stream));
-  replica_count_kernel<<<(unsigned)ctas, kReplicaThreads, 0, stream>>>(indptr, num_nodes, ids, n, local_off, cta_sums, done,
-                                                                      out_offsets + n, d_status);
-  replica_expand_kernel<<<(unsigned)ctas, kReplicaThreads, 0, stream>>>(indptr, ranks, locs, num_nodes, ids, n, cap,
-                                                                       local_off, cta_sums, out_src, out_rank, out_loc,
-                                                                       out_offsets, d_status);
-  SGL_LAUNCH_CHECK();
-  return SGL_OK;
+  SGL_CHECK_RC(zero_async(done, sizeof(unsigned int), stream));
+  SGL_CHECK_RC(launch(replica_count_kernel, (unsigned)ctas, kReplicaThreads, 0, stream, indptr, num_nodes, ids, n, local_off,
+                      cta_sums, done, out_offsets + n, d_status));
+  SGL_CHECK_RC(launch(replica_expand_kernel, (unsigned)ctas, kReplicaThreads, 0, stream, indptr, ranks, locs, num_nodes, ids,
+                      n, cap, local_off, cta_sums, out_src, out_rank, out_loc, out_offsets, d_status));
+  return scope.submit();
 }

@@ -19,6 +19,7 @@
 // Timestamps are compared as fp32, like the reference, which converts them to the mailbox dtype before the reduce.
 // Algorithmic HBM bytes: 8 + 4|8 read per entry + sort passes (32 B per entry and populated key byte), and per
 // unique node 2 * row bytes + 20 written / read.
+#include "launch.cuh"
 #include "heads.cuh"
 #include "sort.cuh"
 #include "tilesort.cuh"
@@ -215,7 +216,7 @@ extern "C" int sgl_mail_reduce(const int64_t* ids_a, int64_t n_a, const int64_t*
   SGL_REQUIRE(d_num_unique, SGL_ERR_ARG, "mail_reduce: null counter");
   SGL_REQUIRE(n_seg >= 0 && n_seg <= kMaxSeg, SGL_ERR_ARG, "mail_reduce: at most %d row segments", kMaxSeg);
   if (n == 0) {
-    SGL_CUDA_CHECK(cudaMemsetAsync(d_num_unique, 0, sizeof(int64_t), stream));
+    SGL_CHECK_RC(zero_async(d_num_unique, sizeof(int64_t), stream));
     return SGL_OK;
   }
   SGL_REQUIRE((n_a == 0 || ids_a) && (n_b == 0 || ids_b) && ts && out_index, SGL_ERR_ARG, "mail_reduce: null array");
@@ -234,17 +235,19 @@ extern "C" int sgl_mail_reduce(const int64_t* ids_a, int64_t n_a, const int64_t*
     segs.dim[s] = seg_dim[s];
     width += seg_dim[s];
   }
+  LaunchScope scope(stream);
   const int id_bits = bits_for(num_nodes > 0 ? (uint64_t)(num_nodes - 1) : 0);
   bool quads = aligned16(out_mail);
   for (int s = 0; s < segs.n; ++s) quads = quads && segs.dim[s] % 4 == 0 && aligned16(segs.a[s]) && aligned16(segs.b[s]);
-  auto emit = [&](const uint32_t* winner, const unsigned long long* best) {
+  auto emit = [&](const uint32_t* winner, const unsigned long long* best) -> int {
     const int grid = stream_grid(n, kThreads / 32, 8);
     if (quads)
-      mail_emit_kernel<Words4><<<grid, kThreads, 0, stream>>>(winner, best, n, d_num_unique, n_a, ts, ts_len, ts_is_i64, segs, width,
-                                                              out_pos, out_ts, out_mail);
+      SGL_CHECK_RC(launch(mail_emit_kernel<Words4>, grid, kThreads, 0, stream, winner, best, n, d_num_unique, n_a, ts,
+                          ts_len, ts_is_i64, segs, width, out_pos, out_ts, out_mail));
     else
-      mail_emit_kernel<Words1><<<grid, kThreads, 0, stream>>>(winner, best, n, d_num_unique, n_a, ts, ts_len, ts_is_i64, segs, width,
-                                                              out_pos, out_ts, out_mail);
+      SGL_CHECK_RC(launch(mail_emit_kernel<Words1>, grid, kThreads, 0, stream, winner, best, n, d_num_unique, n_a, ts,
+                          ts_len, ts_is_i64, segs, width, out_pos, out_ts, out_mail));
+    return scope.submit();
   };
   if (n <= tilesort::kMaxItems && id_bits <= 32) {
     WsCarver c(ws, ws_bytes);
@@ -254,9 +257,8 @@ extern "C" int sgl_mail_reduce(const int64_t* ids_a, int64_t n_a, const int64_t*
     const int rc = tilesort::launch(MailSource{ids_a, ids_b, n_a, n, num_nodes, ts, ts_len, ts_is_i64, d_status},
                                     MailSink{out_index, winner, d_num_unique}, n, id_bits + 32, sc, d_status, stream);
     if (rc) return rc;
-    emit(winner, nullptr);
-    SGL_LAUNCH_CHECK();
-    return SGL_OK;
+    SGL_CHECK_RC(emit(winner, nullptr));
+    return scope.submit();
   }
   WsCarver c(ws, ws_bytes);
   uint64_t* k0 = c.take<uint64_t>(n);
@@ -270,20 +272,21 @@ extern "C" int sgl_mail_reduce(const int64_t* ids_a, int64_t n_a, const int64_t*
   size_t sort_bytes = radix_sort_ws_bytes(n);
   char* sort_ws = c.take<char>(sort_bytes);
   SGL_REQUIRE(c.ok(), SGL_ERR_WORKSPACE, "mail_reduce: workspace %zu < %zu bytes", ws_bytes, sgl_mail_reduce_ws_bytes(n));
-  SGL_CUDA_CHECK(cudaMemsetAsync(done, 0, sizeof(unsigned int), stream));
-  SGL_CUDA_CHECK(cudaMemsetAsync(best, 0, (size_t)n * 8, stream));
-  mail_pack_kernel<<<ctas_for(n), kThreads, 0, stream>>>(ids_a, n_a, ids_b, n_b, num_nodes, k0, d_status);
-  SGL_LAUNCH_CHECK();
+  SGL_CHECK_RC(zero_async(done, sizeof(unsigned int), stream));
+  SGL_CHECK_RC(zero_async(best, (size_t)n * 8, stream));
+  SGL_CHECK_RC(launch(mail_pack_kernel, ctas_for(n), kThreads, 0, stream, ids_a, n_a, ids_b, n_b, num_nodes, k0, d_status));
+
   int in_alt = 0;
   int rc = radix_sort_pairs(k0, v0, k1, v1, n, nullptr, id_bits, true, &in_alt, sort_ws, sort_bytes, stream);
   if (rc) return rc;
   const uint64_t* ks = in_alt ? k1 : k0;
   const uint32_t* perm = in_alt ? v1 : v0;
-  heads_scan_kernel<<<ctas_for(n), kThreads, 0, stream>>>(ks, n, nullptr, 64, packed, cta_sums, done, d_num_unique);
-  mail_argmax_kernel<<<ctas_for(n), kThreads, 0, stream>>>(ks, perm, n, packed, cta_sums, ts, ts_len, ts_is_i64, best, out_index);
-  emit(nullptr, best);
-  SGL_LAUNCH_CHECK();
-  return SGL_OK;
+  SGL_CHECK_RC(launch(heads_scan_kernel, ctas_for(n), kThreads, 0, stream, ks, n, nullptr, 64, packed, cta_sums, done,
+                      d_num_unique));
+  SGL_CHECK_RC(launch(mail_argmax_kernel, ctas_for(n), kThreads, 0, stream, ks, perm, n, packed, cta_sums, ts, ts_len,
+                      ts_is_i64, best, out_index));
+  SGL_CHECK_RC(emit(nullptr, best));
+  return scope.submit();
 }
 
 extern "C" int sgl_mailbox_write(const int64_t* index, int64_t n, const int64_t* d_n, const float* mail, const float* mail_ts,
@@ -297,11 +300,10 @@ extern "C" int sgl_mailbox_write(const int64_t* index, int64_t n, const int64_t*
   SGL_REQUIRE(mailbox_size == 1 || next_mail_pos, SGL_ERR_ARG, "mailbox_write: a mailbox of several slots needs next_mail_pos");
   const int grid = stream_grid(n, kThreads / 32, 8);
   if (width % 4 == 0 && aligned16(mail) && aligned16(mailbox))
-    mailbox_write_kernel<Words4><<<grid, kThreads, 0, stream>>>(index, n, d_n, mail, mail_ts, width, mailbox, mailbox_ts, next_mail_pos,
-                                                                num_nodes, mailbox_size, advance, d_status);
+    SGL_CHECK_RC(launch(mailbox_write_kernel<Words4>, grid, kThreads, 0, stream, index, n, d_n, mail, mail_ts, width,
+                        mailbox, mailbox_ts, next_mail_pos, num_nodes, mailbox_size, advance, d_status));
   else
-    mailbox_write_kernel<Words1><<<grid, kThreads, 0, stream>>>(index, n, d_n, mail, mail_ts, width, mailbox, mailbox_ts, next_mail_pos,
-                                                                num_nodes, mailbox_size, advance, d_status);
-  SGL_LAUNCH_CHECK();
+    SGL_CHECK_RC(launch(mailbox_write_kernel<Words1>, grid, kThreads, 0, stream, index, n, d_n, mail, mail_ts, width,
+                        mailbox, mailbox_ts, next_mail_pos, num_nodes, mailbox_size, advance, d_status));
   return SGL_OK;
 }

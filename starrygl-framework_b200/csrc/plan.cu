@@ -10,6 +10,7 @@
 //                       last CTA scans the CTA totals; per-rank sizes by atomic add (order independent)
 //   plan_expand_kernel  writes (rank, row, slot) triplets in row order
 //   radix sort on the rank (one 8-bit pass) + plan_emit_kernel gathers rows and slots in sorted order
+#include "launch.cuh"
 #include "scan.cuh"
 #include "sort.cuh"
 
@@ -115,10 +116,11 @@ extern "C" int sgl_plan_route(const int64_t* layer_ids, int64_t n, const int64_t
   SGL_REQUIRE(n >= 0 && cap >= 0 && num_nodes >= 0 && num_parts >= 1 && num_parts <= 256 && pid >= 0 && pid < num_parts,
               SGL_ERR_ARG, "plan_route: bad size (1 <= num_parts <= 256, 0 <= pid < num_parts)");
   SGL_REQUIRE(d_send_sizes && d_total, SGL_ERR_ARG, "plan_route: null counter");
-  SGL_CUDA_CHECK(cudaMemsetAsync(d_send_sizes, 0, (size_t)num_parts * sizeof(int64_t), stream));
+  LaunchScope scope(stream);
+  SGL_CHECK_RC(zero_async(d_send_sizes, (size_t)num_parts * sizeof(int64_t), stream));
   if (n == 0) {
-    SGL_CUDA_CHECK(cudaMemsetAsync(d_total, 0, sizeof(int64_t), stream));
-    return SGL_OK;
+    SGL_CHECK_RC(zero_async(d_total, sizeof(int64_t), stream));
+    return scope.submit();
   }
   SGL_REQUIRE(layer_ids && node_parts && rep_indptr && rep_ranks && rep_locs && out_ranks && out_rows && out_locs, SGL_ERR_ARG,
               "plan_route: null array");
@@ -136,20 +138,19 @@ extern "C" int sgl_plan_route(const int64_t* layer_ids, int64_t n, const int64_t
   size_t sort_bytes = radix_sort_ws_bytes(capc);
   char* sort_ws = c.take<char>(sort_bytes);
   SGL_REQUIRE(c.ok(), SGL_ERR_WORKSPACE, "plan_route: workspace %zu < %zu bytes", ws_bytes, sgl_plan_route_ws_bytes(n, cap));
-  SGL_CUDA_CHECK(cudaMemsetAsync(done, 0, sizeof(unsigned int), stream));
-  plan_count_kernel<<<(unsigned)ctas_for(n), kThreads, 0, stream>>>(layer_ids, n, d_n, node_parts, num_nodes, pid, rep_indptr,
-                                                                    rep_ranks, num_parts, local_off, cta_sums, done, d_total,
-                                                                    (unsigned long long*)d_send_sizes, d_status);
-  plan_expand_kernel<<<(unsigned)ctas_for(n), kThreads, 0, stream>>>(layer_ids, n, d_n, node_parts, num_nodes, pid, rep_indptr,
-                                                                     rep_ranks, rep_locs, num_parts, local_off, cta_sums, cap, k0,
-                                                                     tmp_rows, tmp_locs, d_status);
-  SGL_LAUNCH_CHECK();
+  SGL_CHECK_RC(zero_async(done, sizeof(unsigned int), stream));
+  SGL_CHECK_RC(launch(plan_count_kernel, (unsigned)ctas_for(n), kThreads, 0, stream, layer_ids, n, d_n, node_parts,
+                      num_nodes, pid, rep_indptr, rep_ranks, num_parts, local_off, cta_sums, done, d_total, (unsigned long
+                      long*)d_send_sizes, d_status));
+  SGL_CHECK_RC(launch(plan_expand_kernel, (unsigned)ctas_for(n), kThreads, 0, stream, layer_ids, n, d_n, node_parts,
+                      num_nodes, pid, rep_indptr, rep_ranks, rep_locs, num_parts, local_off, cta_sums, cap, k0, tmp_rows,
+                      tmp_locs, d_status));
+
   int in_alt = 0;
   int rc = radix_sort_pairs(k0, v0, k1, v1, capc, d_total, bits_for((uint64_t)(num_parts - 1)), true, &in_alt, sort_ws, sort_bytes,
                             stream);
   if (rc) return rc;
-  plan_emit_kernel<<<stream_grid(capc, kThreads, 8), kThreads, 0, stream>>>(in_alt ? k1 : k0, in_alt ? v1 : v0, capc, d_total,
-                                                                          tmp_rows, tmp_locs, out_ranks, out_rows, out_locs);
-  SGL_LAUNCH_CHECK();
-  return SGL_OK;
+  SGL_CHECK_RC(launch(plan_emit_kernel, stream_grid(capc, kThreads, 8), kThreads, 0, stream, in_alt ? k1 : k0, in_alt ? v1 :
+                      v0, capc, d_total, tmp_rows, tmp_locs, out_ranks, out_rows, out_locs));
+  return scope.submit();
 }

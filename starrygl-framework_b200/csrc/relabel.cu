@@ -6,6 +6,7 @@
 //
 // Algorithmic HBM bytes: 16 read + 8 write per input pair, 16 per unique pair, plus the sort passes
 // (32 B per pair and populated key byte).
+#include "launch.cuh"
 #include "heads.cuh"
 #include "sort.cuh"
 #include "tilesort.cuh"
@@ -523,18 +524,20 @@ extern "C" int sgl_unique_pairs(const int64_t* a_id, const int64_t* a_ts, int64_
   SGL_REQUIRE(d_n_unique, SGL_ERR_ARG, "unique_pairs: d_n_unique is null");
   const int64_t n = n_a + n_b;
   if (n == 0) {
-    SGL_CUDA_CHECK(cudaMemsetAsync(d_n_unique, 0, sizeof(int64_t), stream));
+    SGL_CHECK_RC(zero_async(d_n_unique, sizeof(int64_t), stream));
     return SGL_OK;
   }
   SGL_REQUIRE((n_a == 0 || (a_id && a_ts)) && (n_b == 0 || (b_id && b_ts)) && out_id && out_ts, SGL_ERR_ARG,
               "unique_pairs: null array");
+  LaunchScope scope(stream);
   if (n <= tilesort::kMaxItems) {
     WsCarver c(ws, ws_bytes);
     const tilesort::Scratch sc = tilesort::carve(c, n);
     SGL_REQUIRE(c.ok(), SGL_ERR_WORKSPACE, "unique_pairs: workspace %zu < %zu bytes", ws_bytes, sgl_unique_pairs_ws_bytes(n));
-    return tilesort::launch(PairSource{a_id, a_ts, d_n_a, b_id, b_ts, d_n_b, n_a, n_b, id_bits, ts_bits, ts_base, d_status},
+    SGL_CHECK_RC(tilesort::launch(PairSource{a_id, a_ts, d_n_a, b_id, b_ts, d_n_b, n_a, n_b, id_bits, ts_bits, ts_base, d_status},
                             PairSink{n_a, d_n_a, ts_bits, ts_base, out_id, out_ts, inv_a, inv_b, d_n_unique}, n, id_bits + ts_bits,
-                            sc, d_status, stream);
+                            sc, d_status, stream));
+    return scope.submit();
   }
   WsCarver c(ws, ws_bytes);
   uint64_t* k0 = c.take<uint64_t>(n);
@@ -548,20 +551,20 @@ extern "C" int sgl_unique_pairs(const int64_t* a_id, const int64_t* a_ts, int64_
   size_t sort_bytes = radix_sort_ws_bytes(n);
   char* sort_ws = c.take<char>(sort_bytes);
   SGL_REQUIRE(c.ok(), SGL_ERR_WORKSPACE, "unique_pairs: workspace %zu < %zu bytes", ws_bytes, sgl_unique_pairs_ws_bytes(n));
-  SGL_CUDA_CHECK(cudaMemsetAsync(done, 0, sizeof(unsigned int), stream));
-  pairs_pack_kernel<<<ctas_for(n), kThreads, 0, stream>>>(a_id, a_ts, n_a, d_n_a, b_id, b_ts, n_b, d_n_b, id_bits, ts_bits,
-                                                          ts_base, k0, d_total, d_status);
-  SGL_LAUNCH_CHECK();
+  SGL_CHECK_RC(zero_async(done, sizeof(unsigned int), stream));
+  SGL_CHECK_RC(launch(pairs_pack_kernel, ctas_for(n), kThreads, 0, stream, a_id, a_ts, n_a, d_n_a, b_id, b_ts, n_b, d_n_b,
+                      id_bits, ts_bits, ts_base, k0, d_total, d_status));
+
   int in_alt = 0;
   int rc = radix_sort_pairs(k0, v0, k1, v1, n, d_total, id_bits + ts_bits, true, &in_alt, sort_ws, sort_bytes, stream);
   if (rc) return rc;
   const uint64_t* ks = in_alt ? k1 : k0;
   const uint32_t* vs = in_alt ? v1 : v0;
-  heads_scan_kernel<<<ctas_for(n), kThreads, 0, stream>>>(ks, n, d_total, 64, packed, cta_sums, done, d_n_unique);
-  pairs_emit_kernel<<<ctas_for(n), kThreads, 0, stream>>>(ks, vs, d_total, n, packed, cta_sums, ts_bits, ts_base, n_a,
-                                                          d_n_a, out_id, out_ts, inv_a, inv_b);
-  SGL_LAUNCH_CHECK();
-  return SGL_OK;
+  SGL_CHECK_RC(launch(heads_scan_kernel, ctas_for(n), kThreads, 0, stream, ks, n, d_total, 64, packed, cta_sums, done,
+                      d_n_unique));
+  SGL_CHECK_RC(launch(pairs_emit_kernel, ctas_for(n), kThreads, 0, stream, ks, vs, d_total, n, packed, cta_sums, ts_bits,
+                      ts_base, n_a, d_n_a, out_id, out_ts, inv_a, inv_b));
+  return scope.submit();
 }
 
 extern "C" size_t sgl_build_csc_ws_bytes(int64_t n_edges, int64_t num_dst) {
@@ -584,15 +587,15 @@ extern "C" int sgl_build_csc(const int64_t* src_local, const int64_t* dst, const
     SGL_REQUIRE(n_edges == 0 || (src_local && dst && ts && dt && eid && out_indices && out_ts && out_dt && out_eid), SGL_ERR_ARG,
                 "build_csc: null array");
     const int64_t work_s = n_edges > num_dst + 1 ? n_edges : num_dst + 1;
-    csc_emit_sorted_kernel<<<stream_grid(work_s, kThreads, 16), kThreads, 0, stream>>>(
-        dst, n_edges, d_n_edges, num_dst, d_num_dst, src_local, ts, dt, eid, out_indptr, out_indices, out_ts, out_dt, out_eid,
-        d_status);
-    SGL_LAUNCH_CHECK();
+    SGL_CHECK_RC(launch(csc_emit_sorted_kernel, stream_grid(work_s, kThreads, 16), kThreads, 0, stream, dst, n_edges,
+                        d_n_edges, num_dst, d_num_dst, src_local, ts, dt, eid, out_indptr, out_indices, out_ts, out_dt,
+                        out_eid, d_status));
     return SGL_OK;
   }
   SGL_REQUIRE(dst_bits >= 0 && ts_bits >= 0 && dst_bits + ts_bits <= 64, SGL_ERR_UNSUPPORTED,
               "build_csc: dst_bits %d + ts_bits %d exceed the 64-bit sort key", dst_bits, ts_bits);
   SGL_REQUIRE(out_indptr, SGL_ERR_ARG, "build_csc: out_indptr is null");
+  LaunchScope scope(stream);
   const int64_t cap = n_edges < 1 ? 1 : n_edges;
   if (cap <= tilesort::kMaxItems) {
     SGL_REQUIRE(n_edges == 0 || (dst && ts && dt && eid && out_indices && out_ts && out_dt && out_eid), SGL_ERR_ARG,
@@ -600,9 +603,10 @@ extern "C" int sgl_build_csc(const int64_t* src_local, const int64_t* dst, const
     WsCarver c(ws, ws_bytes);
     const tilesort::Scratch sc = tilesort::carve(c, cap);
     SGL_REQUIRE(c.ok(), SGL_ERR_WORKSPACE, "build_csc: workspace %zu < %zu bytes", ws_bytes, sgl_build_csc_ws_bytes(n_edges, num_dst));
-    return tilesort::launch(CscSource{dst, dst_map, ts, d_n_edges, n_edges, dst_bits, ts_bits, ts_base, d_status},
+    SGL_CHECK_RC(tilesort::launch(CscSource{dst, dst_map, ts, d_n_edges, n_edges, dst_bits, ts_bits, ts_base, d_status},
                             CscSink{num_dst, d_num_dst, ts_bits, src_local, ts, dt, eid, out_indptr, out_indices, out_ts, out_dt, out_eid},
-                            cap, dst_bits + ts_bits, sc, d_status, stream);
+                            cap, dst_bits + ts_bits, sc, d_status, stream));
+    return scope.submit();
   }
   WsCarver c(ws, ws_bytes);
   uint64_t* k0 = c.take<uint64_t>(cap);
@@ -617,19 +621,18 @@ extern "C" int sgl_build_csc(const int64_t* src_local, const int64_t* dst, const
   if (n_edges > 0) {
     SGL_REQUIRE(dst && ts && dt && eid && out_indices && out_ts && out_dt && out_eid, SGL_ERR_ARG,
                 "build_csc: null array");
-    csc_pack_kernel<<<ctas_for(n_edges), kThreads, 0, stream>>>(dst, dst_map, ts, n_edges, d_n_edges, dst_bits, ts_bits,
-                                                               ts_base, k0, d_status);
-    SGL_LAUNCH_CHECK();
+    SGL_CHECK_RC(launch(csc_pack_kernel, ctas_for(n_edges), kThreads, 0, stream, dst, dst_map, ts, n_edges, d_n_edges,
+                        dst_bits, ts_bits, ts_base, k0, d_status));
+  
     int rc = radix_sort_pairs(k0, v0, k1, v1, n_edges, d_n_edges, dst_bits + ts_bits, true, &in_alt, sort_ws, sort_bytes,
                               stream);
     if (rc) return rc;
   }
   int64_t work = n_edges > num_dst + 1 ? n_edges : num_dst + 1;
-  csc_emit_kernel<<<stream_grid(work, kThreads, 16), kThreads, 0, stream>>>(
-      in_alt ? k1 : k0, in_alt ? v1 : v0, n_edges, d_n_edges, num_dst, d_num_dst, ts_bits, src_local, ts, dt, eid,
-      out_indptr, out_indices, out_ts, out_dt, out_eid);
-  SGL_LAUNCH_CHECK();
-  return SGL_OK;
+  SGL_CHECK_RC(launch(csc_emit_kernel, stream_grid(work, kThreads, 16), kThreads, 0, stream, in_alt ? k1 : k0, in_alt ? v1 :
+                      v0, n_edges, d_n_edges, num_dst, d_num_dst, ts_bits, src_local, ts, dt, eid, out_indptr, out_indices,
+                      out_ts, out_dt, out_eid));
+  return scope.submit();
 }
 
 extern "C" size_t sgl_relabel_nodes_ws_bytes(int64_t n) {
@@ -647,19 +650,21 @@ extern "C" int sgl_relabel_nodes(const int64_t* ids, int64_t n, const int64_t* d
   SGL_REQUIRE(n >= 0 && num_nodes >= 0, SGL_ERR_ARG, "relabel_nodes: negative size");
   SGL_REQUIRE(d_next_local && d_n_new, SGL_ERR_ARG, "relabel_nodes: null counter");
   if (n == 0) {
-    SGL_CUDA_CHECK(cudaMemsetAsync(d_n_new, 0, sizeof(int64_t), stream));
+    SGL_CHECK_RC(zero_async(d_n_new, sizeof(int64_t), stream));
     return SGL_OK;
   }
   SGL_REQUIRE(ids && mapper && mask && out_local && out_new_ids, SGL_ERR_ARG, "relabel_nodes: null array");
   const int id_bits = bits_for(num_nodes > 0 ? (uint64_t)(num_nodes - 1) : 0);
   SGL_REQUIRE(id_bits < 63, SGL_ERR_UNSUPPORTED, "relabel_nodes: num_nodes too large");
+  LaunchScope scope(stream);
   if (n <= tilesort::kMaxItems) {
     WsCarver c(ws, ws_bytes);
     const tilesort::Scratch sc = tilesort::carve(c, n);
     SGL_REQUIRE(c.ok(), SGL_ERR_WORKSPACE, "relabel_nodes: workspace %zu < %zu bytes", ws_bytes, sgl_relabel_nodes_ws_bytes(n));
-    return tilesort::launch(NodesSource{ids, d_n, n, num_nodes, mask, epoch, id_bits, d_status},
+    SGL_CHECK_RC(tilesort::launch(NodesSource{ids, d_n, n, num_nodes, mask, epoch, id_bits, d_status},
                             NodesSink{ids, num_nodes, id_bits, mapper, mask, epoch, d_next_local, out_local, out_new_ids, d_n_new, 0}, n,
-                            id_bits + 1, sc, d_status, stream);
+                            id_bits + 1, sc, d_status, stream));
+    return scope.submit();
   }
   WsCarver c(ws, ws_bytes);
   uint64_t* k0 = c.take<uint64_t>(n);
@@ -672,20 +677,22 @@ extern "C" int sgl_relabel_nodes(const int64_t* ids, int64_t n, const int64_t* d
   size_t sort_bytes = radix_sort_ws_bytes(n);
   char* sort_ws = c.take<char>(sort_bytes);
   SGL_REQUIRE(c.ok(), SGL_ERR_WORKSPACE, "relabel_nodes: workspace %zu < %zu bytes", ws_bytes, sgl_relabel_nodes_ws_bytes(n));
-  SGL_CUDA_CHECK(cudaMemsetAsync(done, 0, sizeof(unsigned int), stream));
-  nodes_pack_kernel<<<ctas_for(n), kThreads, 0, stream>>>(ids, n, d_n, num_nodes, mask, epoch, id_bits, k0, d_status);
-  SGL_LAUNCH_CHECK();
+  SGL_CHECK_RC(zero_async(done, sizeof(unsigned int), stream));
+  SGL_CHECK_RC(launch(nodes_pack_kernel, ctas_for(n), kThreads, 0, stream, ids, n, d_n, num_nodes, mask, epoch, id_bits, k0,
+                      d_status));
+
   int in_alt = 0;
   int rc = radix_sort_pairs(k0, v0, k1, v1, n, d_n, id_bits + 1, true, &in_alt, sort_ws, sort_bytes, stream);
   if (rc) return rc;
   const uint64_t* ks = in_alt ? k1 : k0;
-  heads_scan_kernel<<<ctas_for(n), kThreads, 0, stream>>>(ks, n, d_n, id_bits, packed, cta_sums, done, d_n_new);
-  nodes_assign_kernel<<<ctas_for(n), kThreads, 0, stream>>>(ks, n, d_n, id_bits, packed, cta_sums, d_next_local, mapper,
-                                                           mask, epoch, out_new_ids);
-  nodes_lookup_kernel<<<ctas_for(n), kThreads, 0, stream>>>(ids, n, d_n, num_nodes, mapper, out_local, d_next_local, d_n_new);
-  nodes_advance_kernel<<<1, 1, 0, stream>>>(d_next_local, d_n_new);
-  SGL_LAUNCH_CHECK();
-  return SGL_OK;
+  SGL_CHECK_RC(launch(heads_scan_kernel, ctas_for(n), kThreads, 0, stream, ks, n, d_n, id_bits, packed, cta_sums, done,
+                      d_n_new));
+  SGL_CHECK_RC(launch(nodes_assign_kernel, ctas_for(n), kThreads, 0, stream, ks, n, d_n, id_bits, packed, cta_sums,
+                      d_next_local, mapper, mask, epoch, out_new_ids));
+  SGL_CHECK_RC(launch(nodes_lookup_kernel, ctas_for(n), kThreads, 0, stream, ids, n, d_n, num_nodes, mapper, out_local,
+                      d_next_local, d_n_new));
+  SGL_CHECK_RC(launch(nodes_advance_kernel, 1, 1, 0, stream, d_next_local, d_n_new));
+  return scope.submit();
 }
 
 extern "C" int sgl_lower_bound_i64(const int64_t* sorted, int64_t n, const int64_t* values, int k, int64_t* out,
@@ -693,8 +700,7 @@ extern "C" int sgl_lower_bound_i64(const int64_t* sorted, int64_t n, const int64
   SGL_REQUIRE(n >= 0 && k >= 0, SGL_ERR_ARG, "lower_bound: negative size");
   if (k == 0) return SGL_OK;
   SGL_REQUIRE((n == 0 || sorted) && values && out, SGL_ERR_ARG, "lower_bound: null array");
-  lower_bound_kernel<<<(k + 127) / 128, 128, 0, (cudaStream_t)stream_>>>(sorted, n, values, k, out);
-  SGL_LAUNCH_CHECK();
+  SGL_CHECK_RC(launch(lower_bound_kernel, (k + 127) / 128, 128, 0, (cudaStream_t)stream_, sorted, n, values, k, out));
   return SGL_OK;
 }
 
@@ -716,12 +722,13 @@ extern "C" int sgl_seeds_in_window(const int64_t* ev_src, const int64_t* ev_ts, 
               "seeds_in_window: id_bits %d + ts_bits %d leave no room for the sentinel key", id_bits, ts_bits);
   SGL_REQUIRE(d_counts && out_ts_ptr && out_q_ptr, SGL_ERR_ARG, "seeds_in_window: null output");
   if (n_events == 0) {
-    SGL_CUDA_CHECK(cudaMemsetAsync(d_counts, 0, 3 * sizeof(int64_t), stream));
-    SGL_CUDA_CHECK(cudaMemsetAsync(out_ts_ptr, 0, sizeof(int64_t), stream));
-    SGL_CUDA_CHECK(cudaMemsetAsync(out_q_ptr, 0, sizeof(int64_t), stream));
+    SGL_CHECK_RC(zero_async(d_counts, 3 * sizeof(int64_t), stream));
+    SGL_CHECK_RC(zero_async(out_ts_ptr, sizeof(int64_t), stream));
+    SGL_CHECK_RC(zero_async(out_q_ptr, sizeof(int64_t), stream));
     return SGL_OK;
   }
   SGL_REQUIRE(ev_src && ev_ts && ev_eid && out_roots && out_ts && out_q_eid, SGL_ERR_ARG, "seeds_in_window: null array");
+  LaunchScope scope(stream);
   const int64_t n = n_events;
   const int key_bits = id_bits + ts_bits;
   if (n <= tilesort::kMaxItems) {
@@ -729,11 +736,12 @@ extern "C" int sgl_seeds_in_window(const int64_t* ev_src, const int64_t* ev_ts, 
     const tilesort::Scratch sc = tilesort::carve(c, n);
     unsigned long long* valid = c.take<unsigned long long>(1);
     SGL_REQUIRE(c.ok(), SGL_ERR_WORKSPACE, "seeds_in_window: workspace %zu < %zu bytes", ws_bytes, sgl_seeds_ws_bytes(n));
-    SGL_CUDA_CHECK(cudaMemsetAsync(valid, 0, sizeof(*valid), stream));
-    return tilesort::launch(
+    SGL_CHECK_RC(zero_async(valid, sizeof(*valid), stream));
+    SGL_CHECK_RC(tilesort::launch(
         SeedsSource{ev_src, ev_ts, n, node_chunk, chunk_mask, num_chunks, num_nodes, id_bits, ts_bits, ts_base, d_status},
         SeedsSink{n, key_bits, ts_bits, ts_base, ev_eid, out_roots, out_ts_ptr, out_ts, out_q_ptr, out_q_eid, d_counts, valid}, n,
-        key_bits + 1, sc, d_status, stream);
+        key_bits + 1, sc, d_status, stream));
+    return scope.submit();
   }
   WsCarver c(ws, ws_bytes);
   uint64_t* k0 = c.take<uint64_t>(n);
@@ -747,23 +755,23 @@ extern "C" int sgl_seeds_in_window(const int64_t* ev_src, const int64_t* ev_ts, 
   size_t sort_bytes = radix_sort_ws_bytes(n);
   char* sort_ws = c.take<char>(sort_bytes);
   SGL_REQUIRE(c.ok(), SGL_ERR_WORKSPACE, "seeds_in_window: workspace %zu < %zu bytes", ws_bytes, sgl_seeds_ws_bytes(n));
-  SGL_CUDA_CHECK(cudaMemsetAsync(done, 0, sizeof(unsigned int), stream));
-  seeds_pack_kernel<<<ctas_for(n), kThreads, 0, stream>>>(ev_src, ev_ts, n, node_chunk, chunk_mask, num_chunks, num_nodes,
-                                                          id_bits, ts_bits, ts_base, k0, d_status);
-  SGL_LAUNCH_CHECK();
+  SGL_CHECK_RC(zero_async(done, sizeof(unsigned int), stream));
+  SGL_CHECK_RC(launch(seeds_pack_kernel, ctas_for(n), kThreads, 0, stream, ev_src, ev_ts, n, node_chunk, chunk_mask,
+                      num_chunks, num_nodes, id_bits, ts_bits, ts_base, k0, d_status));
+
   int in_alt = 0;
   int rc = radix_sort_pairs(k0, v0, k1, v1, n, nullptr, key_bits + 1, true, &in_alt, sort_ws, sort_bytes, stream);
   if (rc) return rc;
   const uint64_t* ks = in_alt ? k1 : k0;
   const uint32_t* vs = in_alt ? v1 : v0;
-  heads_scan_kernel<<<ctas_for(n), kThreads, 0, stream>>>(ks, n, nullptr, key_bits, packed, cta_sums, done, d_counts + 1);
-  seeds_emit_pairs_kernel<<<ctas_for(n), kThreads, 0, stream>>>(ks, vs, n, key_bits, ts_bits, ts_base, ev_eid, packed,
-                                                                cta_sums, pair_node, out_ts, out_q_ptr, out_q_eid, d_counts);
+  SGL_CHECK_RC(launch(heads_scan_kernel, ctas_for(n), kThreads, 0, stream, ks, n, nullptr, key_bits, packed, cta_sums, done,
+                      d_counts + 1));
+  SGL_CHECK_RC(launch(seeds_emit_pairs_kernel, ctas_for(n), kThreads, 0, stream, ks, vs, n, key_bits, ts_bits, ts_base,
+                      ev_eid, packed, cta_sums, pair_node, out_ts, out_q_ptr, out_q_eid, d_counts));
   // roots = runs of equal node id among the (node, ts) pairs
-  heads_scan_kernel<<<ctas_for(n), kThreads, 0, stream>>>((const uint64_t*)pair_node, n, d_counts + 1, 64, packed, cta_sums,
-                                                          done, d_counts);
-  seeds_emit_roots_kernel<<<ctas_for(n), kThreads, 0, stream>>>(pair_node, n, d_counts, packed, cta_sums, out_roots,
-                                                                out_ts_ptr);
-  SGL_LAUNCH_CHECK();
-  return SGL_OK;
+  SGL_CHECK_RC(launch(heads_scan_kernel, ctas_for(n), kThreads, 0, stream, (const uint64_t*)pair_node, n, d_counts + 1, 64,
+                      packed, cta_sums, done, d_counts));
+  SGL_CHECK_RC(launch(seeds_emit_roots_kernel, ctas_for(n), kThreads, 0, stream, pair_node, n, d_counts, packed, cta_sums,
+                      out_roots, out_ts_ptr));
+  return scope.submit();
 }

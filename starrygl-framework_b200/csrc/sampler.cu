@@ -15,6 +15,7 @@
 //
 // Algorithmic HBM bytes per target: 16 (indptr pair) + 16 (target id, time) + 8*ceil(log2 deg) (search
 // probes) + k_eff*24 (nbr, ts, eid reads) + k_eff*36 (five output arrays) + 8 (offset).
+#include "launch.cuh"
 #include "common.cuh"
 #include "sampler.cuh"
 #include "scan.cuh"
@@ -424,16 +425,16 @@ extern "C" size_t sgl_sample_ws_bytes(int64_t n_targets) {
 template <int CT, int FT, bool WIDE>
 static int launch_sample(const SampleArgs& a, cudaStream_t stream) {
   const unsigned ctas = (unsigned)((a.n_cap + CT - 1) / CT);
-  if (ctas > kDirectCtas) SGL_CUDA_CHECK(cudaMemsetAsync(a.done, 0, sizeof(unsigned int), stream));
-  sample_count_kernel<CT, WIDE><<<ctas, kCtaThreads, 0, stream>>>(a);
+  if (ctas > kDirectCtas) SGL_CHECK_RC(zero_async(a.done, sizeof(unsigned int), stream));
+  SGL_CHECK_RC(launch(sample_count_kernel<CT, WIDE>, ctas, kCtaThreads, 0, stream, a));
   size_t smem = 0;
   if (a.policy == SGL_POLICY_UNIFORM) {
     if (a.fanout > 32) smem = (size_t)kWarpsPerCta * a.fanout * sizeof(uint64_t);
     else if (CT != kWarpsPerCta) smem = (size_t)FT * a.fanout * sizeof(uint32_t);
   }
   if (a.fanout <= 32) smem += (size_t)FT * a.fanout;
-  sample_fill_kernel<CT, FT><<<(unsigned)((a.n_cap + FT - 1) / FT), kCtaThreads, smem, stream>>>(a, (int)ctas);
-  SGL_LAUNCH_CHECK();
+  SGL_CHECK_RC(launch(sample_fill_kernel<CT, FT>, (unsigned)((a.n_cap + FT - 1) / FT), kCtaThreads, smem, stream, a,
+                      (int)ctas));
   return SGL_OK;
 }
 
@@ -454,8 +455,8 @@ int sgl::sample_layer(const int64_t* indptr, const int64_t* nbr, const int64_t* 
   SGL_REQUIRE(out_offsets, SGL_ERR_ARG, "sample_layer: out_offsets is null");
   SGL_REQUIRE(n_targets < ((int64_t)1 << 34), SGL_ERR_UNSUPPORTED, "sample_layer: too many targets");
   if (n_targets == 0) {
-    SGL_CUDA_CHECK(cudaMemsetAsync(out_offsets, 0, sizeof(int64_t), stream));
-    if (total_out) SGL_CUDA_CHECK(cudaMemsetAsync(total_out, 0, sizeof(int64_t), stream));
+    SGL_CHECK_RC(zero_async(out_offsets, sizeof(int64_t), stream));
+    if (total_out) SGL_CHECK_RC(zero_async(total_out, sizeof(int64_t), stream));
     return SGL_OK;
   }
   SGL_REQUIRE(indptr && nbr && ts && eid && targets && target_ts && out_nbr && out_dst && out_ts && out_dt && out_eid,
@@ -483,12 +484,19 @@ int sgl::sample_layer(const int64_t* indptr, const int64_t* nbr, const int64_t* 
   a.done = c.take<unsigned int>(1);
   SGL_REQUIRE(c.ok(), SGL_ERR_WORKSPACE, "sample_layer: workspace %zu < %zu bytes", ws_bytes,
               sgl_sample_ws_bytes(n_targets));
-  if (n_targets <= kWarpTargets) return launch_sample<kWarpsPerCta, kWarpsPerCta, true>(a, stream);
-  // targets per fill CTA: a lane of the CTA draws for every target (uniform), so as many as there are threads once that
-  // leaves several CTAs per SM; windows that are copied are spread thinner
-  if (policy == SGL_POLICY_UNIFORM)
-    return n_targets < kManyTargets ? launch_sample<kCtaThreads, 128, true>(a, stream) : launch_sample<kCtaThreads, 256, false>(a, stream);
-  return n_targets < kManyTargets ? launch_sample<kCtaThreads, 64, true>(a, stream) : launch_sample<kCtaThreads, 64, false>(a, stream);
+  LaunchScope scope(stream);
+  if (n_targets <= kWarpTargets) {
+    SGL_CHECK_RC((launch_sample<kWarpsPerCta, kWarpsPerCta, true>(a, stream)));
+  } else if (policy == SGL_POLICY_UNIFORM) {
+    // targets per fill CTA: a lane of the CTA draws for every target, so as many as there are threads once that leaves
+    // several CTAs per SM; windows that are copied are spread thinner
+    if (n_targets < kManyTargets) SGL_CHECK_RC((launch_sample<kCtaThreads, 128, true>(a, stream)));
+    else SGL_CHECK_RC((launch_sample<kCtaThreads, 256, false>(a, stream)));
+  } else {
+    if (n_targets < kManyTargets) SGL_CHECK_RC((launch_sample<kCtaThreads, 64, true>(a, stream)));
+    else SGL_CHECK_RC((launch_sample<kCtaThreads, 64, false>(a, stream)));
+  }
+  return scope.submit();
 }
 
 extern "C" int sgl_sample_layer(const int64_t* indptr, const int64_t* nbr, const int64_t* ts, const int64_t* eid,
@@ -522,12 +530,15 @@ extern "C" int sgl_sample_gather_fenced(const int64_t* indptr, const int64_t* nb
                                         int64_t* out_ts, float* out_dt, int64_t* out_eid, int64_t* out_offsets,
                                         const void* feat_table, int64_t feat_rows, int64_t row_bytes, int64_t src_pitch,
                                         void* out_feats, int gather_mode, int32_t* d_status, void* ws, size_t ws_bytes, void* stream) {
+  LaunchScope scope((cudaStream_t)stream);
   int rc = sgl::sample_layer(indptr, nbr, ts, eid, fence, num_nodes, targets, target_ts, n_targets, nullptr, fanout, policy,
                              equal_root_time, allowed_offset, keep_root_time, seed, rng_stream, out_nbr, out_dst, out_ts, out_dt,
                              nullptr, out_eid, out_offsets, nullptr, d_status, ws, ws_bytes, stream);
-  if (rc != SGL_OK || n_targets == 0) return rc;
-  return sgl_gather_rows(feat_table, feat_rows, row_bytes, src_pitch, out_eid, nullptr, 0, n_targets * fanout,
-                         out_offsets + n_targets, out_feats, row_bytes, nullptr, nullptr, gather_mode, d_status, stream);
+  if (rc != SGL_OK) return rc;
+  if (n_targets == 0) return scope.submit();
+  SGL_CHECK_RC(sgl_gather_rows(feat_table, feat_rows, row_bytes, src_pitch, out_eid, nullptr, 0, n_targets * fanout,
+                         out_offsets + n_targets, out_feats, row_bytes, nullptr, nullptr, gather_mode, d_status, stream));
+  return scope.submit();
 }
 
 extern "C" int sgl_sample_gather(const int64_t* indptr, const int64_t* nbr, const int64_t* ts, const int64_t* eid,
@@ -538,12 +549,15 @@ extern "C" int sgl_sample_gather(const int64_t* indptr, const int64_t* nbr, cons
                                  int64_t feat_rows, int64_t row_bytes, int64_t src_pitch, void* out_feats, int gather_mode,
                                  int32_t* d_status, void* ws, size_t ws_bytes, void* stream) {
   SGL_NVTX("sgl_sample_gather");
+  LaunchScope scope((cudaStream_t)stream);
   int rc = sgl_sample_layer(indptr, nbr, ts, eid, num_nodes, targets, target_ts, n_targets, nullptr, fanout, policy,
                             equal_root_time, allowed_offset, keep_root_time, seed, rng_stream, out_nbr, out_dst, out_ts,
                             out_dt, nullptr, out_eid, out_offsets, d_status, ws, ws_bytes, stream);
-  if (rc != SGL_OK || n_targets == 0) return rc;
-  return sgl_gather_rows(feat_table, feat_rows, row_bytes, src_pitch, out_eid, nullptr, 0, n_targets * fanout,
-                         out_offsets + n_targets, out_feats, row_bytes, nullptr, nullptr, gather_mode, d_status, stream);
+  if (rc != SGL_OK) return rc;
+  if (n_targets == 0) return scope.submit();
+  SGL_CHECK_RC(sgl_gather_rows(feat_table, feat_rows, row_bytes, src_pitch, out_eid, nullptr, 0, n_targets * fanout,
+                         out_offsets + n_targets, out_feats, row_bytes, nullptr, nullptr, gather_mode, d_status, stream));
+  return scope.submit();
 }
 
 // ---------------------------------------------------------------------------------------------------------------

@@ -12,6 +12,7 @@
 //   slice_write_kernel  one warp per node again, writes at the scanned positions
 // Algorithmic HBM bytes: per node in a selected chunk 16 (row pointer) + 8 * 2 * ceil(log2 deg) (two searches), per
 // edge of the window 16 read twice (neighbour, ts; + 8 for the neighbour's chunk), per kept edge 24 written.
+#include "launch.cuh"
 #include "scan.cuh"
 
 namespace sgl {
@@ -224,9 +225,9 @@ extern "C" int sgl_slice_window(const int64_t* indptr, const int64_t* nbr, const
   SGL_REQUIRE(d_counts && out_node_ptr && out_group_ptr, SGL_ERR_ARG, "slice_window: null counter / pointer array");
   SGL_REQUIRE(chunk_mask == nullptr || num_chunks > 0, SGL_ERR_ARG, "slice_window: a chunk mask needs num_chunks > 0");
   if (num_nodes == 0) {
-    SGL_CUDA_CHECK(cudaMemsetAsync(d_counts, 0, 3 * sizeof(int64_t), stream));
-    SGL_CUDA_CHECK(cudaMemsetAsync(out_node_ptr, 0, sizeof(int64_t), stream));
-    SGL_CUDA_CHECK(cudaMemsetAsync(out_group_ptr, 0, sizeof(int64_t), stream));
+    SGL_CHECK_RC(zero_async(d_counts, 3 * sizeof(int64_t), stream));
+    SGL_CHECK_RC(zero_async(out_node_ptr, sizeof(int64_t), stream));
+    SGL_CHECK_RC(zero_async(out_group_ptr, sizeof(int64_t), stream));
     return SGL_OK;
   }
   SGL_REQUIRE(indptr && nbr && ts && out_nodes && out_group_ts && out_nbr && out_ts && out_eid, SGL_ERR_ARG,
@@ -242,16 +243,15 @@ extern "C" int sgl_slice_window(const int64_t* indptr, const int64_t* nbr, const
   int64_t* cta_edges = c.take<int64_t>(ctas_for(num_nodes));
   unsigned int* done = c.take<unsigned int>(4);
   SGL_REQUIRE(c.ok(), SGL_ERR_WORKSPACE, "slice_window: workspace %zu < %zu bytes", ws_bytes, sgl_slice_window_ws_bytes(num_nodes));
-  SGL_CUDA_CHECK(cudaMemsetAsync(done, 0, 16, stream));
+  SGL_CHECK_RC(zero_async(done, 16, stream));
   SliceArgs a{indptr, nbr, ts, node_chunk, chunk_mask, num_nodes, num_chunks, t_begin, t_end};
   const int grid = stream_grid(num_nodes, kThreads / 32, 16);
-  slice_count_kernel<<<grid, kThreads, 0, stream>>>(a, cnt_edges, cnt_groups, d_status);
-  slice_scan_kernel<<<ctas_for(num_nodes), kThreads, 0, stream>>>(cnt_edges, cnt_groups, num_nodes, loc_node, loc_group, loc_edge,
-                                                                 cta_nodes, cta_groups, cta_edges, done, d_counts);
-  slice_write_kernel<<<grid, kThreads, 0, stream>>>(a, eid, cnt_edges, loc_node, loc_group, loc_edge, cta_nodes, cta_groups,
-                                                    cta_edges, d_counts, cap_edges, out_nodes, out_node_ptr, out_group_ts,
-                                                    out_group_ptr, out_nbr, out_ts, out_eid, d_status);
-  SGL_LAUNCH_CHECK();
+  SGL_CHECK_RC(launch(slice_count_kernel, grid, kThreads, 0, stream, a, cnt_edges, cnt_groups, d_status));
+  SGL_CHECK_RC(launch(slice_scan_kernel, ctas_for(num_nodes), kThreads, 0, stream, cnt_edges, cnt_groups, num_nodes,
+                      loc_node, loc_group, loc_edge, cta_nodes, cta_groups, cta_edges, done, d_counts));
+  SGL_CHECK_RC(launch(slice_write_kernel, grid, kThreads, 0, stream, a, eid, cnt_edges, loc_node, loc_group, loc_edge,
+                      cta_nodes, cta_groups, cta_edges, d_counts, cap_edges, out_nodes, out_node_ptr, out_group_ts,
+                      out_group_ptr, out_nbr, out_ts, out_eid, d_status));
   return SGL_OK;
 }
 
@@ -265,8 +265,7 @@ extern "C" int sgl_densify_time_groups(const int64_t* node_ptr, const int64_t* g
               "densify_time_groups: %lld nodes x %lld time steps is too large for dense groups", (long long)n_nodes, (long long)T);
   SGL_REQUIRE(n_nodes == 0 || (node_ptr && group_ptr && (T == 0 || (group_ts && out_ts))), SGL_ERR_ARG,
               "densify_time_groups: null array");
-  densify_groups_kernel<<<stream_grid(n_nodes * T + 1, kThreads, 16), kThreads, 0, (cudaStream_t)stream_>>>(
-      node_ptr, group_ts, group_ptr, n_nodes, d_n_nodes, t_begin, T, out_node_ptr, out_ts, out_group_ptr);
-  SGL_LAUNCH_CHECK();
+  SGL_CHECK_RC(launch(densify_groups_kernel, stream_grid(n_nodes * T + 1, kThreads, 16), kThreads, 0, (cudaStream_t)stream_,
+                      node_ptr, group_ts, group_ptr, n_nodes, d_n_nodes, t_begin, T, out_node_ptr, out_ts, out_group_ptr));
   return SGL_OK;
 }

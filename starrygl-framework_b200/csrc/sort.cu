@@ -5,6 +5,7 @@
 //                          tile out in digit order in shared memory and writes every digit's run with consecutive
 //                          threads (coalesced runs instead of scattered 8- and 4-byte stores)
 // HBM traffic per pass and key: 8 B (histogram read) + 12 B read + 12 B write.
+#include "launch.cuh"
 #include "sort.cuh"
 #include "tilesort.cuh"
 
@@ -255,11 +256,12 @@ int run_passes(uint64_t* keys, uint32_t* vals, uint64_t* keys_alt, uint32_t* val
   uint32_t *vin = vals, *vout = vals_alt;
   for (int p = 0; p < passes; ++p) {
     const int shift = p * BITS;
-    sort_hist_kernel<BITS><<<num_blocks, kSortThreads, 0, stream>>>(kin, n, d_n, shift, block_hist, num_blocks);
-    sort_scan_kernel<<<1 << BITS, 256, 0, stream>>>(block_hist, num_blocks, digit_total);
-    sort_scatter_kernel<BITS><<<num_blocks, kSortThreads, scatter_smem(BITS), stream>>>(
-        kin, (p == 0 && iota_vals) ? nullptr : vin, n, d_n, shift, block_hist, num_blocks, digit_total, kout, vout);
-    SGL_LAUNCH_CHECK();
+    SGL_CHECK_RC(launch(sort_hist_kernel<BITS>, num_blocks, kSortThreads, 0, stream, kin, n, d_n, shift, block_hist,
+                        num_blocks));
+    SGL_CHECK_RC(launch(sort_scan_kernel, 1 << BITS, 256, 0, stream, block_hist, num_blocks, digit_total));
+    SGL_CHECK_RC(launch(sort_scatter_kernel<BITS>, num_blocks, kSortThreads, scatter_smem(BITS), stream, kin, (p == 0 &&
+                        iota_vals) ? nullptr : vin, n, d_n, shift, block_hist, num_blocks, digit_total, kout, vout));
+  
     uint64_t* tk = kin; kin = kout; kout = tk;
     uint32_t* tv = vin; vin = vout; vout = tv;
   }

@@ -19,6 +19,7 @@
 // per 11 key bits took 25, 84, 95 and 140 us: few CTAs with large digit tables, and a dependent kernel per digit.
 #pragma once
 #include "common.cuh"
+#include "launch.cuh"
 #include "scan.cuh"
 
 #include <atomic>
@@ -585,8 +586,7 @@ int launch_as(const Source& src, const Sink& sink, int64_t n_cap, int pos_bits, 
   if (n_cap <= kSingleMax) {
     constexpr size_t smem = Arrays<WIDE>::bytes(kSingleMax);
     SGL_CUDA_CHECK(allow_smem((const void*)ts_single_kernel<Source, Sink, WIDE>, single_done, smem));
-    ts_single_kernel<Source, Sink, WIDE><<<1, kThreads, smem, stream>>>(src, sink, pos_bits, d_status);
-    SGL_LAUNCH_CHECK();
+    SGL_CHECK_RC(launch(ts_single_kernel<Source, Sink, WIDE>, 1, kThreads, smem, stream, src, sink, pos_bits, d_status));
     return SGL_OK;
   }
   const int64_t min_tiles = (n_cap + kMinTile - 1) / kMinTile;
@@ -597,9 +597,10 @@ int launch_as(const Source& src, const Sink& sink, int64_t n_cap, int pos_bits, 
   const int cap = 4 * tile < kCapMost ? 4 * tile : kCapMost;
   SGL_CUDA_CHECK(allow_smem((const void*)ts_bucket_kernel<Source, Sink, WIDE>, bucket_done, Arrays<WIDE>::bytes(kCapMost)));
   SGL_CUDA_CHECK(allow_smem((const void*)ts_part_kernel<Source, WIDE, Sink::kPred>, part_done, Arrays<WIDE>::bytes(kMaxSamples)));
-  ts_part_kernel<Source, WIDE, Sink::kPred><<<ctas, kThreads, Arrays<WIDE>::bytes(kMaxSamples), stream>>>(src, pos_bits, sc);
-  ts_bucket_kernel<Source, Sink, WIDE><<<ctas, kThreads, Arrays<WIDE>::bytes(cap), stream>>>(src, sink, pos_bits, n_cap, sc, cap, d_status);
-  SGL_LAUNCH_CHECK();
+  SGL_CHECK_RC(launch(ts_part_kernel<Source, WIDE, Sink::kPred>, ctas, kThreads, Arrays<WIDE>::bytes(kMaxSamples), stream,
+                      src, pos_bits, sc));
+  SGL_CHECK_RC(launch(ts_bucket_kernel<Source, Sink, WIDE>, ctas, kThreads, Arrays<WIDE>::bytes(cap), stream, src, sink,
+                      pos_bits, n_cap, sc, cap, d_status));
   return SGL_OK;
 }
 

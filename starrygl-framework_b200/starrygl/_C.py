@@ -107,7 +107,9 @@ _SIGNATURES = {
     "sgl_build_batch_layout": (_i64, [_i64, _vp, _i32, _vp]),
     "sgl_build_batch_ws_bytes": (_sz, [_i64, _vp, _i32]),
     "sgl_build_batch": (_i32, [_vp, _vp, _vp, _vp, _vp, _i64, _vp, _vp, _i64, _vp, _i32, _i32, _i32, _i64, _u64, _i32, _i32, _i64,
-                               _vp, _vp, _vp, _vp, _sz, _vp, _vp]),
+                               _vp, _vp, _vp, _vp, _vp, _sz, _vp, _vp]),
+    "sgl_host_words": (_i32, [C.POINTER(C.c_void_p)]),
+    "sgl_wait_word": (_i32, [_vp, _vp]),
     "sgl_read_back": (_i32, [_vp, _vp, _sz, _vp]),
     "sgl_graph_capture_begin": (_i32, [_vp]),
     "sgl_graph_capture_end": (_i32, [_vp, C.POINTER(C.c_void_p)]),
@@ -158,8 +160,31 @@ def ptr(t):
 
 
 def stream_ptr(stream=None):
-    s = torch.cuda.current_stream() if stream is None else stream
-    return s.cuda_stream
+    if stream is not None:
+        return stream.cuda_stream
+    if torch.cuda.is_initialized():     # a tenth of the cost of building a Stream object
+        return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
+    return torch.cuda.current_stream().cuda_stream
+
+
+_HOST = threading.local()
+
+
+def host_words():
+    """(address, ctypes int64 array) of the calling thread's pinned result buffer."""
+    h = _HOST.__dict__.get("words")
+    if h is None:
+        p = C.c_void_p()
+        check(lib().sgl_host_words(C.byref(p)))
+        h = _HOST.__dict__["words"] = (p.value, (C.c_int64 * 512).from_address(p.value))
+    return h
+
+
+def read_words(t, count):
+    """The first ``count`` int64 words of a device tensor, as a list (waits for the current stream's work on them)."""
+    buf = (C.c_int64 * count)()
+    check(lib().sgl_read_back(t.data_ptr(), buf, 8 * count, stream_ptr()))
+    return list(buf)
 
 
 class Workspace:

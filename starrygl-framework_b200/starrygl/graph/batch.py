@@ -8,7 +8,6 @@ previous list (``indptr``, ``indices``, ``eid``, ``edge_ts``, ``edge_dt``) + the
 synchronisation: the number of edges a hop produced is handed to the next kernels as a device count.
 ``finish()`` performs the single synchronisation that is needed to give the tensors their final shapes.
 """
-import threading
 from collections import OrderedDict
 from typing import List, Optional, Sequence
 
@@ -106,12 +105,7 @@ class DeviceBatch:
 
     def _read(self):
         """The one read-back: every count and, when the batch owns it, the status word."""
-        import ctypes as C
-        words = 2 + 2 * len(self.fanouts)
-        buf = (C.c_int64 * words)()
-        with torch.cuda.device(self._meta.device):
-            _C.check(_C.lib().sgl_read_back(self._meta.data_ptr(), buf, 8 * words, _C.stream_ptr()))
-        host = list(buf)
+        host = _C.read_words(self._meta, 2 + 2 * len(self.fanouts))
         return host[:-1], host[-1] & 0xFFFFFFFF
 
     def finish(self) -> List[dict]:
@@ -156,7 +150,7 @@ class DeviceBatch:
         return bool((deg > 0).any().item())
 
 
-def _enqueue(g, roots, root_ts, fanouts, policy, lo, hi, equal_root_time, allowed_offset, seed, status, side) -> DeviceBatch:
+def _enqueue(g, roots, root_ts, fanouts, policy, lo, hi, equal_root_time, allowed_offset, seed, status, side, host=None) -> DeviceBatch:
     """``lo`` / ``hi``: lowest and highest timestamp that can occur."""
     roots, root_ts = ops._i64(roots), ops._i64(root_ts)
     n = roots.numel()
@@ -174,20 +168,8 @@ def _enqueue(g, roots, root_ts, fanouts, policy, lo, hi, equal_root_time, allowe
         g.num_nodes, _C.ptr(roots), _C.ptr(root_ts), n, plan.fan, len(fanouts),
         _C.POLICY[policy] if isinstance(policy, str) else int(policy), int(bool(equal_root_time)), int(allowed_offset),
         int(seed) & (2 ** 64 - 1), ops.bits_for(g.num_nodes - 1), ops.bits_for(hi - lo), lo, base, base + 8 * plan.words,
-        None if status is None else status.ptr(), ws.data_ptr(), ws.numel(), None if side is None else side.cuda_stream, sp))
+        None if status is None else status.ptr(), host, ws.data_ptr(), ws.numel(), None if side is None else side.cuda_stream, sp))
     return DeviceBatch(g, n, fanouts, plan, arena, meta, status)
-
-
-_LOCAL = threading.local()
-
-
-def _side_stream(dev) -> torch.cuda.Stream:
-    """The calling thread's second stream on ``dev`` for batches of several hops."""
-    pool = _LOCAL.__dict__.setdefault("streams", {})
-    s = pool.get(dev.index)
-    if s is None:
-        s = pool[dev.index] = torch.cuda.Stream(dev)
-    return s
 
 
 def _graph_range(g, lo, hi):
@@ -206,15 +188,15 @@ def build_batch_async(g: ops.TCSR, roots: torch.Tensor, root_ts: torch.Tensor, f
     ``root_ts`` (one extra synchronisation).
 
     Hop l+1 samples the raw output of hop l, and a hop's CSC needs the relabel before it but not its own: with several hops
-    both run on a second stream (``side_streams[0]``, default: one per thread) next to the relabels, and are joined into
-    the current stream.  Captured into a CUDA graph this becomes a graph with parallel branches.
+    both run next to the relabels and are joined into the current stream.  ``side_streams`` (the first is used) is needed
+    for that only while a CUDA graph is being captured.
     """
     if ts_range is None:
         ts_range = _root_range(g, root_ts)
     lo, hi = _graph_range(g, int(ts_range[0]), int(ts_range[1]))
     fanouts = list(fanouts)
-    side = side_streams[0] if side_streams else (_side_stream(g.device) if len(fanouts) > 1 else None)
-    return _enqueue(g, roots, root_ts, fanouts, policy, lo, hi, equal_root_time, allowed_offset, seed, status, side)
+    return _enqueue(g, roots, root_ts, fanouts, policy, lo, hi, equal_root_time, allowed_offset, seed, status,
+                    side_streams[0] if side_streams else None)
 
 
 def _root_range(g, root_ts):
@@ -224,21 +206,28 @@ def _root_range(g, root_ts):
     return lo, hi
 
 
+_SYNC_OPTIONS = {"ts_range", "equal_root_time", "allowed_offset", "seed"}
+
+
 def build_batch(g, roots, root_ts, fanouts, policy="recent", **kw) -> List[dict]:
     """Synchronous form of :func:`build_batch_async`."""
-    if kw.get("ts_range") is not None or kw.get("status") is not None:
+    if kw.get("ts_range") is not None or not _SYNC_OPTIONS.issuperset(kw):
         return build_batch_async(g, roots, root_ts, fanouts, policy, **kw).finish()
     # Query times nearly always lie in the graph's own time range (events of the stream): the batch is enqueued with the
     # range known so far instead of waiting for the smallest and largest query time.  The kernels flag a time outside of
     # it; then the range is read, kept on the graph, and the batch built again.
     lo, hi = g.__dict__.get("_query_range", (g.ts_min, g.ts_max))
-    kw.pop("ts_range", None)
-    db = build_batch_async(g, roots, root_ts, fanouts, policy, ts_range=(lo, hi), **kw)
-    host, bits = db._read()
+    fanouts = list(fanouts)
+    addr, words = _C.host_words()
+    last = 1 + 2 * len(fanouts)
+    db = _enqueue(g, roots, root_ts, fanouts, policy, lo, hi, kw.get("equal_root_time", False), kw.get("allowed_offset", -1),
+                  kw.get("seed", 0), None, None, addr)
+    _C.check(_C.lib().sgl_wait_word(addr + 8 * (last + 1), _C.stream_ptr()))
+    host, bits = words[:last], words[last] & 0xFFFFFFFF
     if bits & 2:
         a, b = _root_range(g, root_ts)
         g.__dict__["_query_range"] = (min(lo, a), max(hi, b))
-        return build_batch_async(g, roots, root_ts, fanouts, policy, ts_range=(a, b), **kw).finish()
+        return build_batch_async(g, roots, root_ts, fanouts, policy, **{**kw, "ts_range": (a, b)}).finish()
     if bits:
         raise _C.SglError(f"build_batch: device status {bits} ({_C.decode_status(bits)})")
     return db._trim(host)

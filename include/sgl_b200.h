@@ -559,10 +559,9 @@ int sgl_build_batch(const int64_t* indptr, const int64_t* nbr, const int64_t* ts
                     int32_t* d_status, int64_t* host_meta, void* ws, size_t ws_bytes, void* side_stream, void* stream);
 
 /* Small results for the host.  sgl_host_words: a pinned buffer of 512 words that belongs to the calling thread.
- * sgl_wait_word: waits until work on the stream has set *flag (pinned memory).  sgl_read_back: copies up to 511 words of
+ * sgl_wait_word: waits until work on the stream has set *flag (pinned memory) to at_least or more.  sgl_read_back: copies up to 511 words of
  * device memory to the host through that buffer and waits for them. */
-int sgl_host_words(void** out);
-int sgl_wait_word(const int64_t* flag, void* stream);
+int sgl_wait_word(const int64_t* flag, int64_t at_least, void* stream);
 int sgl_read_back(const void* src, void* dst, size_t bytes, void* stream);
 
 /* ------------------------------------------------------------------------------------------------

@@ -14,7 +14,7 @@
 // Meta (8-byte words): entries of the root list, then per hop sampled edges and entries of the merged list, then a status
 // word (used when the caller has none of its own).
 
-#include "launch.cuh"
+#include "chain.cuh"
 #include "sampler.cuh"
 #include "sort.cuh"
 #include "tilesort.cuh"
@@ -24,7 +24,7 @@ using namespace sgl;
 namespace {
 
 constexpr int kMaxHops = 8;
-constexpr int kHostWords = 512;
+constexpr int kHostWords = 512;   // of sgl_host_words
 constexpr int kRootSections = 3, kHopSections = 14;
 
 inline int64_t words(int64_t n) { return ((n < 1 ? 1 : n) + 31) / 32 * 32; }
@@ -92,57 +92,11 @@ size_t csc_ws(int64_t n, const int32_t* fanouts, int hops) {
   return align_up(most);
 }
 
-// Order between the two streams of a batch: nodes of the launch scope, or (captured calls) events of this thread, recorded
-// and waited for at once and so reusable.
-struct Order {
-  static constexpr int kMarks = 4;
-  LaunchScope* scope;
-  std::vector<int> nodes[kMarks];
-  cudaEvent_t ev[kMarks];
-
-  int init(LaunchScope* s) {
-    scope = s;
-    if (scope) return SGL_OK;
-    static thread_local cudaEvent_t pool[64][kMarks];
-    int dev = 0;
-    SGL_CUDA_CHECK(cudaGetDevice(&dev));
-    for (int i = 0; i < kMarks; ++i) {
-      cudaEvent_t& e = pool[dev & 63][i];
-      if (e == nullptr) SGL_CUDA_CHECK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-      ev[i] = e;
-    }
-    return SGL_OK;
-  }
-  int mark(int i, cudaStream_t s) {
-    if (scope) nodes[i] = scope->mark(s);
-    else SGL_CUDA_CHECK(cudaEventRecord(ev[i], s));
-    return SGL_OK;
-  }
-  int wait(int i, cudaStream_t s) {
-    if (scope) scope->wait(s, nodes[i]);
-    else SGL_CUDA_CHECK(cudaStreamWaitEvent(s, ev[i], 0));
-    return SGL_OK;
-  }
-};
-
 // indices[j] = col[indices[j]]: edge numbers -> positions in the merged list
 __global__ void __launch_bounds__(256)
 map_columns_kernel(int64_t* __restrict__ indices, const int64_t* __restrict__ col, int64_t n_cap, const int64_t* d_n) {
   const int64_t n = eff_count(n_cap, d_n), stride = (int64_t)gridDim.x * 256;
   for (int64_t j = (int64_t)blockIdx.x * 256 + threadIdx.x; j < n; j += stride) indices[j] = __ldg(col + indices[j]);
-}
-
-// words of device memory -> pinned host memory, then the flag behind them
-__global__ void export_words_kernel(const int64_t* __restrict__ src, int64_t* dst, int words) {
-  for (int i = threadIdx.x; i < words; i += blockDim.x) dst[i] = src[i];
-  __threadfence_system();
-  __syncthreads();
-  if (threadIdx.x == 0) *(volatile int64_t*)(dst + words) = 1;
-}
-
-int export_words(const int64_t* src, int64_t* dst, int words, cudaStream_t stream) {
-  *(volatile int64_t*)(dst + words) = 0;
-  return launch(export_words_kernel, 1, 32, 0, stream, src, dst, words);
 }
 
 }  // namespace
@@ -272,19 +226,19 @@ extern "C" int sgl_host_words(void** out) {
   return SGL_OK;
 }
 
-// Waits until *flag is set by work on the stream: the host looks at the word itself for a while (a stream
+// Waits until work on the stream has set *flag to at_least or more: the host looks at the word itself for a while (a stream
 // synchronisation costs 5 us more than the kernel that it waits for), then waits for the stream, which also reports errors.
-extern "C" int sgl_wait_word(const int64_t* flag, void* stream) {
+extern "C" int sgl_wait_word(const int64_t* flag, int64_t at_least, void* stream) {
   SGL_REQUIRE(flag, SGL_ERR_ARG, "wait_word: flag is null");
   const volatile int64_t* f = flag;
   for (int i = 0; i < 2000000; ++i) {
-    if (*f) return SGL_OK;
+    if (*f >= at_least) return SGL_OK;
 #if defined(__x86_64__)
     __builtin_ia32_pause();
 #endif
   }
   SGL_CUDA_CHECK(cudaStreamSynchronize((cudaStream_t)stream));
-  SGL_REQUIRE(*f, SGL_ERR_CUDA, "wait_word: the stream ended without setting the word");
+  SGL_REQUIRE(*f >= at_least, SGL_ERR_CUDA, "wait_word: the stream ended without setting the word");
   return SGL_OK;
 }
 
@@ -296,7 +250,7 @@ extern "C" int sgl_read_back(const void* src, void* dst, size_t bytes, void* str
   int64_t* host = (int64_t*)p;
   const int words = (int)(bytes / 8);
   SGL_CHECK_RC(export_words((const int64_t*)src, host, words, (cudaStream_t)stream));
-  SGL_CHECK_RC(sgl_wait_word(host + words, stream));
+  SGL_CHECK_RC(sgl_wait_word(host + words, 1, stream));
   memcpy(dst, host, bytes);
   return SGL_OK;
 }

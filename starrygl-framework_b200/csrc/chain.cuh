@@ -1,0 +1,53 @@
+// Helpers of the entry points that enqueue a whole batch or query.
+#pragma once
+#include "launch.cuh"
+
+namespace sgl {
+
+// Order between the two streams of an entry point: nodes of the launch scope, or (captured calls) events of this thread, recorded
+// and waited for at once and so reusable.
+struct Order {
+  static constexpr int kMarks = 4;
+  LaunchScope* scope;
+  std::vector<int> nodes[kMarks];
+  cudaEvent_t ev[kMarks];
+
+  int init(LaunchScope* s) {
+    scope = s;
+    if (scope) return SGL_OK;
+    static thread_local cudaEvent_t pool[64][kMarks];
+    int dev = 0;
+    SGL_CUDA_CHECK(cudaGetDevice(&dev));
+    for (int i = 0; i < kMarks; ++i) {
+      cudaEvent_t& e = pool[dev & 63][i];
+      if (e == nullptr) SGL_CUDA_CHECK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+      ev[i] = e;
+    }
+    return SGL_OK;
+  }
+  int mark(int i, cudaStream_t s) {
+    if (scope) nodes[i] = scope->mark(s);
+    else SGL_CUDA_CHECK(cudaEventRecord(ev[i], s));
+    return SGL_OK;
+  }
+  int wait(int i, cudaStream_t s) {
+    if (scope) scope->wait(s, nodes[i]);
+    else SGL_CUDA_CHECK(cudaStreamWaitEvent(s, ev[i], 0));
+    return SGL_OK;
+  }
+};
+
+// words of device memory -> pinned host memory, then the flag behind them
+static __global__ void export_words_kernel(const int64_t* __restrict__ src, int64_t* dst, int words, int64_t flag) {
+  for (int i = threadIdx.x; i < words; i += blockDim.x) dst[i] = src[i];
+  __threadfence_system();
+  __syncthreads();
+  if (threadIdx.x == 0) *(volatile int64_t*)(dst + words) = flag;
+}
+
+inline int export_words(const int64_t* src, int64_t* dst, int words, cudaStream_t stream) {
+  *(volatile int64_t*)(dst + words) = 0;
+  return launch(export_words_kernel, 1, 32, 0, stream, src, dst, words, (int64_t)1);
+}
+
+}  // namespace sgl

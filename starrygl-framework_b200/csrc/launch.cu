@@ -169,6 +169,7 @@ void LaunchScope::wait(cudaStream_t s, const std::vector<int>& nodes) {
 
 int LaunchScope::submit() {
   if (!owner_) return SGL_OK;
+  owner_ = false;
   Thread& t = t_state;
   t.open = nullptr;
   LaunchList& l = t.list;

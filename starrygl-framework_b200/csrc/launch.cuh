@@ -15,6 +15,7 @@
 #include <stdint.h>
 #include <string.h>
 
+#include <atomic>
 #include <vector>
 
 #include "common.cuh"
@@ -83,6 +84,18 @@ int launch(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStr
 
 // Zero bytes (a multiple of four, four-byte aligned) in stream order, in a launch scope or not.
 int zero_async(void* p, size_t bytes, cudaStream_t stream);
+
+// kernels that need more than 48 KB of shared memory say so once per device
+inline cudaError_t allow_smem(const void* kernel, std::atomic<uint64_t>& done, size_t bytes) {
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  const uint64_t bit = 1ull << (dev & 63);
+  if (done.load(std::memory_order_relaxed) & bit) return cudaSuccess;
+  e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+  if (e == cudaSuccess) done.fetch_or(bit, std::memory_order_relaxed);
+  return e;
+}
 
 #define SGL_CHECK_RC(expr)     \
   do {                         \

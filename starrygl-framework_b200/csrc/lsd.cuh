@@ -1,0 +1,456 @@
+// Radix sort of lists beyond the mini-batch sort: least significant digit first, 8 bits a pass, ONE kernel per pass (the
+// "onesweep" scheme of Adinets and Merrill, with Merrill and Garland's decoupled look-back):
+//   1. lsd_hist_kernel   one read of the keys: digit totals of every pass
+//   2. lsd_scan_kernel   start of every digit, all passes
+//   3. lsd_pass_kernel   per pass: a CTA takes the next tile, ranks its keys stably, publishes its digit counts, adds up those of
+//                        the tiles before it, and writes every digit's run with consecutive threads
+//   4. lsd_deliver_kernel   hands every item with its place, and for sinks that number groups its group's number, to a Sink
+// HBM traffic per pass and key: 16 B + twice the payload (a histogram kernel, a scan kernel and a scatter kernel per pass read
+// the keys once more and took 1.0 ms per pass for 50 M keys).
+#pragma once
+#include "launch.cuh"
+#include "scan.cuh"
+#include "sort.cuh"
+#include "tilesort.cuh"
+
+namespace sgl {
+namespace {
+
+constexpr int kBits = 8;
+constexpr int kRadix = 1 << kBits;
+constexpr int kMaxPasses = 8;
+constexpr int kLsdThreads = 512;
+constexpr int kLsdWarps = kLsdThreads / 32;
+template <class V>
+constexpr int kLsdItems = sizeof(V) == 4 ? 12 : 10;   // keys per thread: two CTAs per SM either way
+template <class V>
+constexpr int kLsdTile = kLsdThreads * kLsdItems<V>;
+constexpr int kHistThreads = 512;
+
+__device__ __forceinline__ uint32_t digit_of(uint64_t key, int shift) { return (uint32_t)(key >> shift) & (kRadix - 1u); }
+
+// Digit totals of passes shift0, shift0 + 8, ...: one shared-memory counter table per pass.  A warp whose keys all carry the
+// same digit (high digits of a hub, ordered input) adds once.
+template <class Items>
+__global__ void __launch_bounds__(kHistThreads)
+lsd_hist_kernel(Items items, int shift0, int passes, unsigned long long* __restrict__ hist) {
+  __shared__ uint32_t s_hist[kMaxPasses * kRadix];
+  const int64_t n = items.begin();
+  for (int j = threadIdx.x; j < passes * kRadix; j += kHistThreads) s_hist[j] = 0;
+  __syncthreads();
+  const int64_t stride = (int64_t)gridDim.x * kHistThreads;
+  const int lane = threadIdx.x & 31;
+  for (int64_t i0 = (int64_t)blockIdx.x * kHistThreads; i0 < n; i0 += stride) {
+    const int64_t i = i0 + threadIdx.x;
+    const bool valid = i < n;
+    const uint64_t key = valid ? items.key(i) : 0;
+    if (valid) items.prepare(i);
+    const unsigned act = __ballot_sync(0xffffffffu, valid);
+    if (act == 0) continue;
+    for (int p = 0; p < passes; ++p) {
+      const uint32_t d = digit_of(key, shift0 + p * kBits);
+      const uint32_t d0 = __shfl_sync(0xffffffffu, d, 0);
+      if (__all_sync(0xffffffffu, !valid || d == d0)) {
+        if (lane == 0) atomicAdd(&s_hist[p * kRadix + d0], (uint32_t)__popc(act));
+      } else if (valid) {
+        atomicAdd(&s_hist[p * kRadix + d], 1u);
+      }
+    }
+  }
+  __syncthreads();
+  for (int j = threadIdx.x; j < passes * kRadix; j += kHistThreads)
+    if (s_hist[j]) atomicAdd(&hist[j], (unsigned long long)s_hist[j]);
+}
+
+// totals -> starts, one CTA of 256 threads per pass
+static __global__ void __launch_bounds__(kRadix) lsd_scan_kernel(unsigned long long* __restrict__ hist) {
+  unsigned long long* h = hist + blockIdx.x * kRadix;
+  const unsigned long long v = h[threadIdx.x];
+  h[threadIdx.x] = cta_exclusive_scan<kRadix, unsigned long long>(v, nullptr);
+}
+
+// Published by a tile per digit: value, pass number + 1, and whether the value is the tile's own count or includes all
+// tiles before it.  Words of an earlier pass count as not published, so the array is cleared once per sort.
+constexpr uint64_t kOwn = 1ull << 62, kAll = 2ull << 62, kValue = (1ull << 56) - 1;
+__device__ __forceinline__ uint64_t pass_tag(int pass) { return (uint64_t)(pass + 1) << 56; }
+constexpr unsigned long long kLookLimitNs = 2000000000ull;
+
+template <class V>
+struct LsdSmem {
+  union {
+    uint64_t keys[kLsdTile<V>];            // the tile in digit order
+    uint32_t mask[kLsdWarps][kRadix];      // before that: lanes of the warp's current round that hold the digit
+  };
+  V vals[kLsdTile<V>];
+  uint32_t cnt[kLsdWarps][kRadix];         // keys of the digit in the warp so far, then where the warp's start in the tile
+  int64_t out[kRadix];                     // global position of the tile's digit run minus its position in the tile
+  int ticket;
+};
+
+// where a pass reads its items from: the arrays of the pass before, or (first pass) the producer of the keys
+template <class V>
+struct ArrayItems {
+  const uint64_t* keys;
+  const V* vals;
+  int64_t n_cap;
+  const int64_t* d_n;
+  __device__ __forceinline__ int64_t begin() const { return eff_count(n_cap, d_n); }
+  __device__ __forceinline__ uint64_t key(int64_t i) const { return keys[i]; }
+  __device__ __forceinline__ V val(int64_t i) const { return vals[i]; }
+  __device__ __forceinline__ void prepare(int64_t) const {}
+};
+
+// a Source (see tilesort.cuh) with the position as payload
+template <class Source>
+struct SourceItems {
+  Source src;
+  __device__ __forceinline__ int64_t begin() { return src.begin(); }
+  __device__ __forceinline__ uint64_t key(int64_t i) const { return src.key(i); }
+  __device__ __forceinline__ uint32_t val(int64_t i) const { return (uint32_t)i; }
+  __device__ __forceinline__ void prepare(int64_t i) const { src.prepare(i); }
+};
+
+template <class V, class Items>
+__global__ void __launch_bounds__(kLsdThreads, 2)
+lsd_pass_kernel(Items items, int shift, int pass,
+                const unsigned long long* __restrict__ starts, unsigned int* __restrict__ ticket, uint64_t* __restrict__ state,
+                uint64_t* __restrict__ out_keys, V* __restrict__ out_vals, unsigned int* gave_up, int32_t* d_status) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  LsdSmem<V>& sm = *(LsdSmem<V>*)smem;
+  constexpr int kItems = kLsdItems<V>, kTile = kLsdTile<V>;
+  const int64_t n = items.begin();
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  if (tid == 0) sm.ticket = (int)atomicAdd(ticket, 1u);
+  for (int j = tid; j < kLsdWarps * kRadix; j += kLsdThreads) {
+    (&sm.mask[0][0])[j] = 0;
+    (&sm.cnt[0][0])[j] = 0;
+  }
+  __syncthreads();
+  const int tile = sm.ticket;
+  const int64_t tile_base = (int64_t)tile * kTile;
+  if (tile_base >= n) return;
+  const int tile_n = (int)(n - tile_base < kTile ? n - tile_base : kTile);
+  // a warp owns consecutive keys of the tile, 32 at a time: (warp, round, lane) order = key order
+  const int first = warp * (kItems * 32) + lane;
+  uint64_t k[kItems];
+  V v[kItems];
+#pragma unroll
+  for (int c = 0; c < kItems; ++c) {
+    const int j = first + c * 32;
+    k[c] = j < tile_n ? items.key(tile_base + j) : ~0ull;
+  }
+#pragma unroll
+  for (int c = 0; c < kItems; ++c) {
+    const int j = first + c * 32;
+    v[c] = j < tile_n ? items.val(tile_base + j) : (V)0;
+  }
+  // stable rank inside the warp: the lanes of a round that share a digit find each other through one word per digit
+  uint16_t rank[kItems];
+  uint32_t *mask = sm.mask[warp], *cnt = sm.cnt[warp];
+  const uint32_t below = (1u << lane) - 1u;
+#pragma unroll
+  for (int c = 0; c < kItems; ++c) {
+    const bool valid = first + c * 32 < tile_n;
+    const uint32_t d = digit_of(k[c], shift);
+    if (valid) atomicOr(&mask[d], 1u << lane);
+    __syncwarp();
+    const uint32_t peers = valid ? mask[d] : 0u, before = valid ? cnt[d] : 0u;
+    __syncwarp();
+    if (valid && (peers & below) == 0) {   // the lowest lane of the digit
+      mask[d] = 0;
+      cnt[d] = before + __popc(peers);
+    }
+    __syncwarp();
+    rank[c] = (uint16_t)(before + __popc(peers & below));
+  }
+  __syncthreads();
+  // per digit: counts of the warps -> starts of the warps; the tile's count is published, those of the tiles before added up
+  uint32_t total = 0;
+  if (tid < kRadix) {
+#pragma unroll
+    for (int w = 0; w < kLsdWarps; ++w) {
+      const uint32_t c = sm.cnt[w][tid];
+      sm.cnt[w][tid] = total;
+      total += c;
+    }
+    *(volatile uint64_t*)&state[(size_t)tile * kRadix + tid] = (tile == 0 ? kAll : kOwn) | pass_tag(pass) | total;
+  }
+  const uint32_t start = cta_exclusive_scan<kLsdThreads, uint32_t>(total, nullptr);
+  if (tid < kRadix) {
+#pragma unroll
+    for (int w = 0; w < kLsdWarps; ++w) sm.cnt[w][tid] += start;
+  }
+  __syncthreads();
+#pragma unroll
+  for (int c = 0; c < kItems; ++c) {
+    if (first + c * 32 < tile_n) {
+      const uint32_t at = cnt[digit_of(k[c], shift)] + rank[c];
+      sm.keys[at] = k[c];
+      sm.vals[at] = v[c];
+    }
+  }
+  if (tid < kRadix) {
+    uint64_t sum = 0;
+    if (tile > 0) {
+      // (tiles are taken in order: those before this one are running or done)
+      const uint64_t tag = pass_tag(pass);
+      const volatile uint64_t* st = state + tid;
+      unsigned long long t0 = 0;
+      for (int t = tile - 1; t >= 0;) {
+        uint64_t w[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) w[u] = t - u >= 0 ? st[(size_t)(t - u) * kRadix] : 0;
+        bool done = false, stalled = false;
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          if (done || stalled || t < 0) continue;
+          if ((w[u] & (0x3full << 56)) != tag) {
+            stalled = true;
+            continue;
+          }
+          sum += w[u] & kValue;
+          done = (w[u] & kAll) != 0;
+          --t;
+        }
+        if (done) break;
+        if (stalled) {
+          unsigned long long now;
+          asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(now));
+          if (t0 == 0) t0 = now;
+          if (now - t0 > kLookLimitNs) {
+            dev_flag(d_status, SGL_DEV_TIMEOUT);
+            *(volatile unsigned int*)gave_up = 1u;
+            break;
+          }
+        }
+      }
+      *(volatile uint64_t*)&state[(size_t)tile * kRadix + tid] = kAll | tag | (sum + total);
+    }
+    sm.out[tid] = (int64_t)(starts[tid] + sum) - (int64_t)start;
+  }
+  __syncthreads();
+  // consecutive threads take consecutive tile positions, i.e. runs of one digit -> consecutive addresses
+  for (int j = tid; j < tile_n; j += kLsdThreads) {
+    const uint64_t key = sm.keys[j];
+    const int64_t g = sm.out[digit_of(key, shift)] + j;
+    if (g >= 0 && g < n) {                 // (always, unless a look-back gave up)
+      out_keys[g] = key;
+      out_vals[g] = sm.vals[j];
+    }
+  }
+}
+
+// ---- delivery of a sorted list to a Sink (see tilesort.cuh) -------------------------------------------------------------
+constexpr int kDeliverThreads = 512;
+constexpr int kDeliverItems = 8;
+constexpr int kDeliverTile = kDeliverThreads * kDeliverItems;
+
+// Sum of what the CTAs before this one (by ticket: they all run already) published; called by one whole warp.
+__device__ __forceinline__ uint64_t deliver_prefix(uint64_t* state, int tile, uint64_t total, int lane, int32_t* d_status) {
+  volatile uint64_t* st = state;
+  if (lane == 0) st[tile] = tile == 0 ? (kAll | total) : (kOwn | total);
+  constexpr uint64_t kSum = (1ull << 62) - 1;
+  uint64_t base = 0;
+  unsigned long long t0 = 0;
+  for (int look = tile - 1; look >= 0;) {
+    const int p = look - lane;
+    uint64_t v = kAll;                   // before the first tile: nothing
+    if (p >= 0) v = st[p];
+    if (__any_sync(0xffffffffu, v == 0)) {
+      unsigned long long now;
+      asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(now));
+      if (t0 == 0) t0 = now;
+      if (__any_sync(0xffffffffu, now - t0 > kLookLimitNs)) {
+        if (lane == 0) dev_flag(d_status, SGL_DEV_TIMEOUT);
+        break;
+      }
+      continue;
+    }
+    const unsigned all = __ballot_sync(0xffffffffu, (v & kAll) != 0);
+    const int stop = all ? __ffs(all) - 1 : 31;
+    uint64_t x = lane <= stop ? (v & kSum) : 0;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+    base += x;
+    if (all) break;
+    look -= 32;
+  }
+  if (lane == 0 && tile > 0) st[tile] = kAll | (base + total);
+  return base;
+}
+
+// ctl[0] ticket, ctl[1] arrivals; state: one word per tile, cleared
+template <class Sink>
+__global__ void __launch_bounds__(kDeliverThreads)
+lsd_deliver_kernel(Sink sink, const uint64_t* __restrict__ keys, const uint32_t* __restrict__ pos, int64_t n_cap, const int64_t* d_count,
+                   unsigned long long* ctl, uint64_t* state, const unsigned int* gave_up, int32_t* d_status) {
+  const int64_t n = *gave_up ? 0 : eff_count(n_cap, d_count);     // (a pass that gave up left places unwritten)
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  sink.begin();
+  if (n <= 0) {
+    if (blockIdx.x == 0) {
+      sink.finish(0, 0, false, 0, 0);
+      tilesort::arrive(sink, nullptr, 1);
+    }
+    return;
+  }
+  const int tiles = (int)((n + kDeliverTile - 1) / kDeliverTile);
+  if constexpr (!Sink::kUnique) {
+    const int64_t base = (int64_t)blockIdx.x * kDeliverTile;
+    if (base >= n) return;
+#pragma unroll
+    for (int c = 0; c < kDeliverItems; ++c) {
+      const int64_t i = base + c * kDeliverThreads + tid;
+      if (i < n) sink.item(i, keys[i], pos[i], i > 0, i > 0 ? keys[i - 1] : 0ull);
+    }
+    if ((int)blockIdx.x == tiles - 1) sink.finish(n, keys[n - 1], true, 0, 0);
+    tilesort::arrive(sink, ctl + 1, tiles);
+  } else {
+    constexpr bool kTwo = Sink::kLevels == 2;
+    constexpr int kShift = 31;           // two counts share the word: 31 bits each
+    __shared__ int s_ticket;
+    __shared__ uint64_t s_cnt[kDeliverItems * (kDeliverThreads / 32)], s_scan[kDeliverItems * (kDeliverThreads / 32)];
+    __shared__ uint64_t s_base;
+    if (tid == 0) s_ticket = (int)atomicAdd(ctl, 1ull);
+    __syncthreads();
+    const int tile = s_ticket;
+    const int64_t first = (int64_t)tile * kDeliverTile;
+    if (first >= n) return;
+    uint64_t k[kDeliverItems];
+    uint32_t p[kDeliverItems];
+    unsigned h1 = 0, h2 = 0;             // bit c: item c of the thread starts a group / a coarser group
+    unsigned up1[kDeliverItems], up2[kDeliverItems];
+#pragma unroll
+    for (int c = 0; c < kDeliverItems; ++c) {
+      const int64_t i = first + c * kDeliverThreads + tid;
+      k[c] = i < n ? keys[i] : 0;
+      p[c] = i < n ? pos[i] : 0u;
+    }
+#pragma unroll
+    for (int c = 0; c < kDeliverItems; ++c) {
+      const int64_t i = first + c * kDeliverThreads + tid;
+      bool a = false, b = false;
+      if (i < n && sink.counted(k[c])) {
+        const uint64_t q = i > 0 ? keys[i - 1] : 0ull;
+        a = i == 0 || sink.group(q) != sink.group(k[c]);
+        if constexpr (kTwo) b = i == 0 || sink.group2(q) != sink.group2(k[c]);
+      }
+      const unsigned ba = __ballot_sync(0xffffffffu, a), bb = kTwo ? __ballot_sync(0xffffffffu, b) : 0u;
+      h1 |= (a ? 1u : 0u) << c;
+      h2 |= (b ? 1u : 0u) << c;
+      const unsigned upto = (2u << lane) - 1u;
+      up1[c] = __popc(ba & upto);
+      up2[c] = __popc(bb & upto);
+      if (lane == 0) s_cnt[c * (kDeliverThreads / 32) + warp] = (uint64_t)__popc(ba) | ((uint64_t)__popc(bb) << kShift);
+    }
+    __syncthreads();
+    constexpr int kCells = kDeliverItems * (kDeliverThreads / 32);
+    const uint64_t mine = tid < kCells ? s_cnt[tid] : 0;
+    uint64_t total;
+    const uint64_t ex = cta_exclusive_scan<kDeliverThreads, uint64_t>(mine, &total);
+    if (tid < kCells) s_scan[tid] = ex;
+    if (warp == 0) {
+      const uint64_t base = deliver_prefix(state, tile, total, lane, d_status);
+      if (lane == 0) s_base = base;
+    }
+    __syncthreads();
+    const uint64_t base = s_base, low = kTwo ? (1ull << kShift) - 1 : ~0ull;
+#pragma unroll
+    for (int c = 0; c < kDeliverItems; ++c) {
+      const int64_t i = first + c * kDeliverThreads + tid;
+      if (i >= n) continue;
+      const uint64_t off = base + s_scan[c * (kDeliverThreads / 32) + warp];
+      const int64_t u = (int64_t)(off & low) + up1[c] - 1, u2 = kTwo ? (int64_t)(off >> kShift) + up2[c] - 1 : 0;
+      sink.item(i, k[c], p[c], (h1 >> c) & 1u, u, (h2 >> c) & 1u, u2);
+    }
+    if (tile == tiles - 1) sink.finish(n, 0, false, (int64_t)((base + total) & low), kTwo ? (int64_t)((base + total) >> kShift) : 0);
+    tilesort::arrive(sink, ctl + 1, tiles);
+  }
+}
+
+// number of items of a Source, for the kernels behind the first pass
+template <class Source>
+__global__ void source_count_kernel(Source src, int64_t* d_count) { *d_count = src.begin(); }
+
+template <class V>
+inline int64_t lsd_tiles(int64_t n) { return (n + kLsdTile<V> - 1) / kLsdTile<V>; }
+
+template <class V>
+inline size_t lsd_ws_bytes(int64_t n) {
+  return align_up((kMaxPasses * kRadix + kMaxPasses) * 8) + align_up((size_t)lsd_tiles<V>(n < 1 ? 1 : n) * kRadix * 8);
+}
+
+// Sorts on key bits [first_bit, num_bits), at least one pass; the first pass reads from `items`, writes to (k1, v1), the next to
+// (k0, v0) and so on; *in_first says whether the result ends in (k1, v1).  **gave_up on the device: a look-back ran into its
+// time limit, the result is not to be used as positions.
+template <class V, class Items>
+int lsd_sort(const Items& items, uint64_t* k1, V* v1, uint64_t* k0, V* v0, int64_t n, const int64_t* d_n, int first_bit, int num_bits,
+             bool* in_first, unsigned int** gave_up, WsCarver& c, int32_t* d_status, cudaStream_t stream) {
+  int passes = (num_bits - first_bit + kBits - 1) / kBits;
+  if (passes < 1) passes = 1;
+  const int64_t tiles = lsd_tiles<V>(n);
+  unsigned long long* hist = c.take<unsigned long long>(kMaxPasses * kRadix + kMaxPasses);
+  unsigned int* tickets = (unsigned int*)(hist + kMaxPasses * kRadix);
+  *gave_up = tickets + kMaxPasses;
+  uint64_t* state = c.take<uint64_t>((size_t)tiles * kRadix);
+  SGL_REQUIRE(c.ok(), SGL_ERR_WORKSPACE, "radix sort: workspace too small for %lld keys", (long long)n);
+  static std::atomic<uint64_t> done0{0}, done1{0};
+  SGL_CUDA_CHECK(allow_smem((const void*)lsd_pass_kernel<V, Items>, done0, sizeof(LsdSmem<V>)));
+  SGL_CUDA_CHECK(allow_smem((const void*)lsd_pass_kernel<V, ArrayItems<V>>, done1, sizeof(LsdSmem<V>)));
+  SGL_CHECK_RC(zero_async(hist, (kMaxPasses * kRadix + kMaxPasses) * 8, stream));
+  SGL_CHECK_RC(zero_async(state, (size_t)tiles * kRadix * 8, stream));
+  SGL_CHECK_RC(launch(lsd_hist_kernel<Items>, stream_grid(n, kHistThreads * 16, 4), kHistThreads, 0, stream, items, first_bit, passes, hist));
+  SGL_CHECK_RC(launch(lsd_scan_kernel, passes, kRadix, 0, stream, hist));
+  for (int p = 0; p < passes; ++p) {
+    uint64_t *kout = p & 1 ? k0 : k1, *kin = p & 1 ? k1 : k0;
+    V *vout = p & 1 ? v0 : v1, *vin = p & 1 ? v1 : v0;
+    const int shift = first_bit + p * kBits;
+    if (p == 0)
+      SGL_CHECK_RC(launch(lsd_pass_kernel<V, Items>, (unsigned)tiles, kLsdThreads, sizeof(LsdSmem<V>), stream, items, shift, p, hist, tickets,
+                          state, kout, vout, *gave_up, d_status));
+    else
+      SGL_CHECK_RC(launch(lsd_pass_kernel<V, ArrayItems<V>>, (unsigned)tiles, kLsdThreads, sizeof(LsdSmem<V>), stream,
+                          ArrayItems<V>{kin, vin, n, d_n}, shift, p, hist + p * kRadix, tickets + p, state, kout, vout, *gave_up,
+                          d_status));
+  }
+  *in_first = passes & 1;
+  return SGL_OK;
+}
+
+inline size_t list_ws_bytes(int64_t n) {
+  if (n < 1) n = 1;
+  if (n <= tilesort::kMaxItems) return tilesort::ws_bytes(n);
+  return 2 * align_up((size_t)n * 8) + 2 * align_up((size_t)n * 4) + lsd_ws_bytes<uint32_t>(n) + align_up(8) +
+         align_up(((size_t)((n + kDeliverTile - 1) / kDeliverTile) + 2) * 8);
+}
+
+// Sorts the items of `src` (at most n_cap, keys of key_bits bits) and delivers them to `sink`: the mini-batch sort, or the
+// radix passes and a delivery kernel for longer lists.
+template <class Source, class Sink>
+int sort_list(const Source& src, const Sink& sink, int64_t n_cap, int key_bits, void* ws, size_t ws_bytes, int32_t* d_status,
+              cudaStream_t stream) {
+  WsCarver c(ws, ws_bytes);
+  if (n_cap <= tilesort::kMaxItems) {
+    const tilesort::Scratch sc = tilesort::carve(c, n_cap);
+    SGL_REQUIRE(c.ok(), SGL_ERR_WORKSPACE, "sort: workspace %zu < %zu bytes", ws_bytes, list_ws_bytes(n_cap));
+    return tilesort::launch(src, sink, n_cap, key_bits, sc, d_status, stream);
+  }
+  SGL_REQUIRE(n_cap < ((int64_t)1 << 32), SGL_ERR_UNSUPPORTED, "sort: %lld entries need a 64-bit position", (long long)n_cap);
+  uint64_t *k0 = c.take<uint64_t>(n_cap), *k1 = c.take<uint64_t>(n_cap);
+  uint32_t *v0 = c.take<uint32_t>(n_cap), *v1 = c.take<uint32_t>(n_cap);
+  int64_t* count = c.take<int64_t>(1);
+  const int64_t tiles = (n_cap + kDeliverTile - 1) / kDeliverTile;
+  unsigned long long* ctl = c.take<unsigned long long>((size_t)tiles + 2);
+  SGL_REQUIRE(c.ok(), SGL_ERR_WORKSPACE, "sort: workspace %zu < %zu bytes", ws_bytes, list_ws_bytes(n_cap));
+  SGL_CHECK_RC(launch(source_count_kernel<Source>, 1, 1, 0, stream, src, count));
+  SGL_CHECK_RC(zero_async(ctl, (size_t)(tiles + 2) * 8, stream));
+  bool in_first;
+  unsigned int* gave_up;
+  SGL_CHECK_RC((lsd_sort<uint32_t, SourceItems<Source>>(SourceItems<Source>{src}, k1, v1, k0, v0, n_cap, count, 0, key_bits, &in_first,
+                                                        &gave_up, c, d_status, stream)));
+  return launch(lsd_deliver_kernel<Sink>, (unsigned)tiles, kDeliverThreads, 0, stream, sink, in_first ? k1 : k0, in_first ? v1 : v0, n_cap,
+                count, ctl, (uint64_t*)(ctl + 2), gave_up, d_status);
+}
+
+}  // namespace
+}  // namespace sgl

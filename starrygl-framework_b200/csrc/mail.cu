@@ -2,32 +2,21 @@
 //
 // The reference concatenates the batch's source and destination nodes, builds one mail row per entry
 // ([own memory | other end's memory | edge feature]), and keeps for every distinct node the entry with the largest
-// timestamp (unique + scatter_max + index).  Here the 2B x width mail matrix is never materialised:
-//
-// Up to 606,208 entries: the mini-batch sort by (node, latest time first, entry), whose first entry per node is the winner,
-// then mail_emit_kernel.  More entries:
-//
-//   mail_pack_kernel     key = node id of entry j (sources first, then destinations)
-//   stable radix sort    on the populated id bits, payload = entry position
-//   heads_scan_kernel    run heads -> index of every entry's node in the sorted unique list, number of unique nodes
-//   mail_argmax_kernel   per entry one 64-bit atomicMax on its node's slot: (orderable fp32 ts << 32) | ~position, so the
-//                        winner is the largest timestamp and, among equal timestamps, the FIRST entry (order
-//                        independent, hence deterministic)
-//   mail_emit_kernel     one warp per unique node: winner's position and timestamp, and the mail row gathered
-//                        straight from the per-event tables
+// timestamp (unique + scatter_max + index).  Here the 2B x width mail matrix is never materialised: the entries are sorted
+// by (node, latest time first, position; sources first, then destinations), so that a node's winner -- the largest
+// timestamp and, among equal timestamps, the FIRST entry -- is the first of its run, and mail_emit_kernel gathers the
+// winners' rows straight from the per-event tables.
 //
 // Timestamps are compared as fp32, like the reference, which converts them to the mailbox dtype before the reduce.
 // Algorithmic HBM bytes: 8 + 4|8 read per entry + sort passes (32 B per entry and populated key byte), and per
 // unique node 2 * row bytes + 20 written / read.
 #include "launch.cuh"
-#include "heads.cuh"
-#include "sort.cuh"
-#include "tilesort.cuh"
+#include "lsd.cuh"
 
 namespace sgl {
 namespace {
 
-constexpr int kThreads = kHeadsThreads;
+constexpr int kThreads = 256;
 constexpr int kMaxSeg = 4;
 
 struct Segs {
@@ -48,33 +37,6 @@ __device__ __forceinline__ uint32_t orderable(float f) {
   return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
 }
 
-__global__ void __launch_bounds__(kThreads)
-mail_pack_kernel(const int64_t* __restrict__ ids_a, int64_t n_a, const int64_t* __restrict__ ids_b, int64_t n_b,
-                 int64_t num_nodes, uint64_t* __restrict__ keys, int32_t* d_status) {
-  const int64_t j = (int64_t)blockIdx.x * kThreads + threadIdx.x;
-  if (j >= n_a + n_b) return;
-  int64_t g = j < n_a ? ids_a[j] : ids_b[j - n_a];
-  if (g < 0 || g >= num_nodes) {
-    dev_flag(d_status, SGL_DEV_BAD_NODE);
-    g = 0;
-  }
-  keys[j] = (uint64_t)g;
-}
-
-__global__ void __launch_bounds__(kThreads)
-mail_argmax_kernel(const uint64_t* __restrict__ keys, const uint32_t* __restrict__ perm, int64_t n,
-                   const uint32_t* __restrict__ packed, const int64_t* __restrict__ cta_base, const void* ts,
-                   int64_t ts_len, int ts_is_i64, unsigned long long* __restrict__ best, int64_t* __restrict__ out_index) {
-  const int64_t j = (int64_t)blockIdx.x * kThreads + threadIdx.x;
-  if (j >= n) return;
-  const uint32_t pk = packed[j];
-  const int64_t u = cta_base[blockIdx.x] + (pk >> 1) + (pk & 1) - 1;   // this entry's node in the unique list
-  if (pk & 1) out_index[u] = (int64_t)keys[j];
-  const uint32_t pos = perm[j];
-  const unsigned long long v = ((unsigned long long)orderable(ts_at(ts, ts_len, ts_is_i64, pos)) << 32) | (0xffffffffu - pos);
-  atomicMax(best + u, v);
-}
-
 struct Words4 {
   using T = float4;
 };
@@ -86,8 +48,8 @@ struct Words1 {
 // 16 bytes when every segment allows it (W = Words4; 7,000 rows of 372 values: 10.8 us in pieces of 4 bytes).
 template <class W>
 __global__ void __launch_bounds__(kThreads)
-mail_emit_kernel(const uint32_t* __restrict__ winner, const unsigned long long* __restrict__ best, int64_t n_cap,
-                 const int64_t* d_num_unique, int64_t n_a, const void* ts, int64_t ts_len, int ts_is_i64, Segs segs, int64_t width,
+mail_emit_kernel(const uint32_t* __restrict__ winner, int64_t n_cap, const int64_t* d_num_unique, int64_t n_a,
+                 const void* ts, int64_t ts_len, int ts_is_i64, Segs segs, int64_t width,
                  int64_t* __restrict__ out_pos, float* __restrict__ out_ts, float* __restrict__ out_mail) {
   using T = typename W::T;
   constexpr int kPer = sizeof(T) / 4;
@@ -95,7 +57,7 @@ mail_emit_kernel(const uint32_t* __restrict__ winner, const unsigned long long* 
   const int lane = threadIdx.x & 31;
   const int64_t n_warps = (int64_t)gridDim.x * (kThreads / 32);
   for (int64_t u = ((int64_t)blockIdx.x * kThreads + threadIdx.x) >> 5; u < n; u += n_warps) {
-    const int64_t pos = winner ? (int64_t)winner[u] : (int64_t)(0xffffffffu - (uint32_t)best[u]);
+    const int64_t pos = winner[u];
     if (lane == 0) {
       if (out_pos) out_pos[u] = pos;
       if (out_ts) out_ts[u] = ts_at(ts, ts_len, ts_is_i64, pos);
@@ -151,8 +113,6 @@ mailbox_write_kernel(const int64_t* __restrict__ index, int64_t n_cap, const int
 
 inline bool aligned16(const void* p) { return ((uintptr_t)p & 15) == 0; }
 
-// Lists of at most tilesort::kMaxItems entries: sorted by (node, latest time first, position), so that the first entry of a
-// node is its winner -- no argmax over the node's entries, no winner array to clear.
 struct MailSource {
   const int64_t *ids_a, *ids_b;
   int64_t n_a, n, num_nodes;
@@ -167,7 +127,36 @@ struct MailSource {
       dev_flag(d_status, SGL_DEV_BAD_NODE);
       g = 0;
     }
-    return ((uint64_t)g << 32) | (uint32_t)~orderable(ts_at(ts, ts_len, ts_is_i64, j));
+    return ((uint64_t)g << 32) | late_first(j);
+  }
+  __device__ __forceinline__ uint32_t late_first(int64_t j) const { return ~orderable(ts_at(ts, ts_len, ts_is_i64, j)); }
+  __device__ __forceinline__ void prepare(int64_t) const {}
+};
+
+// Node ids beyond 32 bits leave no room for the time in the key: sorted by time first, then stably by node.
+struct MailTimes {
+  MailSource m;
+  uint32_t* order;
+  __device__ __forceinline__ int64_t begin() const { return m.n; }
+  __device__ __forceinline__ uint64_t key(int64_t j) const { return m.late_first(j); }
+  __device__ __forceinline__ void prepare(int64_t) const {}
+};
+struct OrderSink {
+  static constexpr bool kUnique = false, kPred = false, kAfter = false;
+  uint32_t* order;
+  __device__ __forceinline__ void begin() const {}
+  __device__ __forceinline__ void item(int64_t at, uint64_t, uint32_t pos, bool, uint64_t) const { order[at] = pos; }
+  __device__ __forceinline__ void finish(int64_t, uint64_t, bool, int64_t, int64_t) const {}
+};
+struct MailNodes {
+  MailSource m;
+  const uint32_t* order;
+  __device__ __forceinline__ int64_t begin() const { return m.n; }
+  __device__ __forceinline__ uint64_t key(int64_t i) const {
+    const int64_t j = order[i], g = j < m.n_a ? m.ids_a[j] : m.ids_b[j - m.n_a];
+    if (g >= 0 && g < m.num_nodes) return (uint64_t)g;
+    dev_flag(m.d_status, SGL_DEV_BAD_NODE);
+    return 0;
   }
   __device__ __forceinline__ void prepare(int64_t) const {}
 };
@@ -178,20 +167,21 @@ struct MailSink {
   int64_t* out_index;
   uint32_t* winner;
   int64_t* d_num_unique;
+  const uint32_t* order;     // what the positions count (nullptr: the entries themselves)
+  int node_shift;
   __device__ __forceinline__ void begin() const {}
   __device__ __forceinline__ bool counted(uint64_t) const { return true; }
-  __device__ __forceinline__ uint64_t group(uint64_t k) const { return k >> 32; }
+  __device__ __forceinline__ uint64_t group(uint64_t k) const { return k >> node_shift; }
   __device__ __forceinline__ void item(int64_t, uint64_t k, uint32_t pos, bool head, int64_t u, bool, int64_t) const {
     if (!head) return;
-    out_index[u] = (int64_t)(k >> 32);
-    winner[u] = pos;
+    out_index[u] = (int64_t)(k >> node_shift);
+    winner[u] = order ? order[pos] : pos;
   }
   __device__ __forceinline__ void finish(int64_t, uint64_t, bool, int64_t groups, int64_t) const {
     if (threadIdx.x == 0) *d_num_unique = groups;
   }
 };
 
-inline unsigned ctas_for(int64_t n) { return (unsigned)((n + kThreads - 1) / kThreads < 1 ? 1 : (n + kThreads - 1) / kThreads); }
 
 }  // namespace
 }  // namespace sgl
@@ -199,9 +189,8 @@ inline unsigned ctas_for(int64_t n) { return (unsigned)((n + kThreads - 1) / kTh
 using namespace sgl;
 
 extern "C" size_t sgl_mail_reduce_ws_bytes(int64_t n_entries) {
-  int64_t n = n_entries < 1 ? 1 : n_entries;
-  return 2 * align_up((size_t)n * 8) + 3 * align_up((size_t)n * 4) + align_up((size_t)ctas_for(n) * 8) + align_up(8) +
-         align_up((size_t)n * 8) + radix_sort_ws_bytes(n);
+  const int64_t n = n_entries < 1 ? 1 : n_entries;
+  return 2 * align_up((size_t)n * 4) + list_ws_bytes(n);
 }
 
 extern "C" int sgl_mail_reduce(const int64_t* ids_a, int64_t n_a, const int64_t* ids_b, int64_t n_b, int64_t num_nodes,
@@ -235,57 +224,31 @@ extern "C" int sgl_mail_reduce(const int64_t* ids_a, int64_t n_a, const int64_t*
     segs.dim[s] = seg_dim[s];
     width += seg_dim[s];
   }
-  LaunchScope scope(stream);
   const int id_bits = bits_for(num_nodes > 0 ? (uint64_t)(num_nodes - 1) : 0);
   bool quads = aligned16(out_mail);
   for (int s = 0; s < segs.n; ++s) quads = quads && segs.dim[s] % 4 == 0 && aligned16(segs.a[s]) && aligned16(segs.b[s]);
-  auto emit = [&](const uint32_t* winner, const unsigned long long* best) -> int {
-    const int grid = stream_grid(n, kThreads / 32, 8);
-    if (quads)
-      SGL_CHECK_RC(launch(mail_emit_kernel<Words4>, grid, kThreads, 0, stream, winner, best, n, d_num_unique, n_a, ts,
-                          ts_len, ts_is_i64, segs, width, out_pos, out_ts, out_mail));
-    else
-      SGL_CHECK_RC(launch(mail_emit_kernel<Words1>, grid, kThreads, 0, stream, winner, best, n, d_num_unique, n_a, ts,
-                          ts_len, ts_is_i64, segs, width, out_pos, out_ts, out_mail));
-    return scope.submit();
-  };
-  if (n <= tilesort::kMaxItems && id_bits <= 32) {
-    WsCarver c(ws, ws_bytes);
-    uint32_t* winner = c.take<uint32_t>(n);
-    const tilesort::Scratch sc = tilesort::carve(c, n);
-    SGL_REQUIRE(c.ok(), SGL_ERR_WORKSPACE, "mail_reduce: workspace %zu < %zu bytes", ws_bytes, sgl_mail_reduce_ws_bytes(n));
-    const int rc = tilesort::launch(MailSource{ids_a, ids_b, n_a, n, num_nodes, ts, ts_len, ts_is_i64, d_status},
-                                    MailSink{out_index, winner, d_num_unique}, n, id_bits + 32, sc, d_status, stream);
-    if (rc) return rc;
-    SGL_CHECK_RC(emit(winner, nullptr));
-    return scope.submit();
+  SGL_REQUIRE(ws && ws_bytes >= sgl_mail_reduce_ws_bytes(n), SGL_ERR_WORKSPACE, "mail_reduce: workspace %zu < %zu bytes", ws_bytes,
+              sgl_mail_reduce_ws_bytes(n));
+  uint32_t *winner = (uint32_t*)ws, *order = (uint32_t*)((char*)ws + align_up((size_t)n * 4));
+  void* sort_ws = (char*)ws + 2 * align_up((size_t)n * 4);
+  const size_t sort_bytes = ws_bytes - 2 * align_up((size_t)n * 4);
+  const MailSource entries{ids_a, ids_b, n_a, n, num_nodes, ts, ts_len, ts_is_i64, d_status};
+  LaunchScope scope(stream);
+  if (id_bits <= 32) {
+    SGL_CHECK_RC(sort_list(entries, MailSink{out_index, winner, d_num_unique, nullptr, 32}, n, id_bits + 32, sort_ws, sort_bytes, d_status,
+                           stream));
+  } else {
+    SGL_CHECK_RC(sort_list(MailTimes{entries, order}, OrderSink{order}, n, 32, sort_ws, sort_bytes, d_status, stream));
+    SGL_CHECK_RC(sort_list(MailNodes{entries, order}, MailSink{out_index, winner, d_num_unique, order, 0}, n, id_bits, sort_ws, sort_bytes,
+                           d_status, stream));
   }
-  WsCarver c(ws, ws_bytes);
-  uint64_t* k0 = c.take<uint64_t>(n);
-  uint64_t* k1 = c.take<uint64_t>(n);
-  uint32_t* v0 = c.take<uint32_t>(n);
-  uint32_t* v1 = c.take<uint32_t>(n);
-  uint32_t* packed = c.take<uint32_t>(n);
-  int64_t* cta_sums = c.take<int64_t>(ctas_for(n));
-  unsigned int* done = c.take<unsigned int>(1);
-  unsigned long long* best = c.take<unsigned long long>(n);
-  size_t sort_bytes = radix_sort_ws_bytes(n);
-  char* sort_ws = c.take<char>(sort_bytes);
-  SGL_REQUIRE(c.ok(), SGL_ERR_WORKSPACE, "mail_reduce: workspace %zu < %zu bytes", ws_bytes, sgl_mail_reduce_ws_bytes(n));
-  SGL_CHECK_RC(zero_async(done, sizeof(unsigned int), stream));
-  SGL_CHECK_RC(zero_async(best, (size_t)n * 8, stream));
-  SGL_CHECK_RC(launch(mail_pack_kernel, ctas_for(n), kThreads, 0, stream, ids_a, n_a, ids_b, n_b, num_nodes, k0, d_status));
-
-  int in_alt = 0;
-  int rc = radix_sort_pairs(k0, v0, k1, v1, n, nullptr, id_bits, true, &in_alt, sort_ws, sort_bytes, stream);
-  if (rc) return rc;
-  const uint64_t* ks = in_alt ? k1 : k0;
-  const uint32_t* perm = in_alt ? v1 : v0;
-  SGL_CHECK_RC(launch(heads_scan_kernel, ctas_for(n), kThreads, 0, stream, ks, n, nullptr, 64, packed, cta_sums, done,
-                      d_num_unique));
-  SGL_CHECK_RC(launch(mail_argmax_kernel, ctas_for(n), kThreads, 0, stream, ks, perm, n, packed, cta_sums, ts, ts_len,
-                      ts_is_i64, best, out_index));
-  SGL_CHECK_RC(emit(nullptr, best));
+  const int grid = stream_grid(n, kThreads / 32, 8);
+  if (quads)
+    SGL_CHECK_RC(launch(mail_emit_kernel<Words4>, grid, kThreads, 0, stream, winner, n, d_num_unique, n_a, ts, ts_len, ts_is_i64, segs,
+                        width, out_pos, out_ts, out_mail));
+  else
+    SGL_CHECK_RC(launch(mail_emit_kernel<Words1>, grid, kThreads, 0, stream, winner, n, d_num_unique, n_a, ts, ts_len, ts_is_i64, segs,
+                        width, out_pos, out_ts, out_mail));
   return scope.submit();
 }
 

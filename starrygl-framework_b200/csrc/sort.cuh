@@ -4,10 +4,6 @@
 
 namespace sgl {
 
-constexpr int kSortThreads = 256;
-constexpr int kSortItems = 16;
-constexpr int kSortTile = kSortThreads * kSortItems;  // keys per CTA
-
 size_t radix_sort_ws_bytes(int64_t n);
 
 // Sorts on key bits [0, num_bits).  vals may be nullptr on input: the payload is then the input position.

@@ -1,4 +1,4 @@
-// Stable sort of mini-batch sized lists (up to 606,208 items) in TWO kernels, with the producer of the keys and the
+// Stable sort of mini-batch sized lists (up to 1,212,416 items) in TWO kernels, with the producer of the keys and the
 // consumer of the sorted order fused into them:
 //
 //   ts_part_kernel<Source>    a CTA makes the keys of its tile (Source), sorts a sample of the whole list -- every CTA the
@@ -22,8 +22,6 @@
 #include "launch.cuh"
 #include "scan.cuh"
 
-#include <atomic>
-
 namespace sgl {
 namespace tilesort {
 
@@ -32,9 +30,11 @@ constexpr int kThreadBits = 9;
 constexpr int kThreads = 1 << kThreadBits;   // threads of every kernel here; at least kMaxCtas (1,024 were no faster)
 constexpr int kWarps = kThreads / 32;
 constexpr int kMinTile = 256;
-constexpr int kMaxTile = 4096;
+constexpr int kMaxTile = 8192;
 constexpr int kTileItems = kMaxTile / kThreads;
 constexpr int kMaxSamples = 2048;       // sample of the whole list: about fourteen per bucket with 148 buckets
+// (Capacity: what a launch holds at most.  Lists that really are that long have buckets beyond shared memory and sort them
+// in L2, still no slower than the radix passes; multi-hop lists usually fill a third of their capacity.)
 constexpr int64_t kMaxItems = (int64_t)kMaxCtas * kMaxTile;
 constexpr int kSingleMax = 2048;
 constexpr unsigned long long kWaitNs = 2000000000ull;
@@ -566,18 +566,6 @@ ts_single_kernel(Source src, Sink sink, int pos_bits, int32_t* d_status) {
 }
 
 inline int launches(int64_t n_cap) { return n_cap <= 0 ? 0 : (n_cap <= kSingleMax ? 1 : 2); }
-
-// kernels that need more than 48 KB of shared memory say so once per device
-inline cudaError_t allow_smem(const void* kernel, std::atomic<uint64_t>& done, size_t bytes) {
-  int dev = 0;
-  cudaError_t e = cudaGetDevice(&dev);
-  if (e != cudaSuccess) return e;
-  const uint64_t bit = 1ull << (dev & 63);
-  if (done.load(std::memory_order_relaxed) & bit) return cudaSuccess;
-  e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-  if (e == cudaSuccess) done.fetch_or(bit, std::memory_order_relaxed);
-  return e;
-}
 
 template <class Source, class Sink, bool WIDE>
 int launch_as(const Source& src, const Sink& sink, int64_t n_cap, int pos_bits, const Scratch& sc, int32_t* d_status,

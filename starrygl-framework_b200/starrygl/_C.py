@@ -109,7 +109,7 @@ _SIGNATURES = {
     "sgl_build_batch": (_i32, [_vp, _vp, _vp, _vp, _vp, _i64, _vp, _vp, _i64, _vp, _i32, _i32, _i32, _i64, _u64, _i32, _i32, _i64,
                                _vp, _vp, _vp, _vp, _vp, _sz, _vp, _vp]),
     "sgl_host_words": (_i32, [C.POINTER(C.c_void_p)]),
-    "sgl_wait_word": (_i32, [_vp, _vp]),
+    "sgl_wait_word": (_i32, [_vp, _i64, _vp]),
     "sgl_read_back": (_i32, [_vp, _vp, _sz, _vp]),
     "sgl_graph_capture_begin": (_i32, [_vp]),
     "sgl_graph_capture_end": (_i32, [_vp, C.POINTER(C.c_void_p)]),

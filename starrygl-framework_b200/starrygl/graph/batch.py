@@ -150,16 +150,19 @@ class DeviceBatch:
         return bool((deg > 0).any().item())
 
 
-def _enqueue(g, roots, root_ts, fanouts, policy, lo, hi, equal_root_time, allowed_offset, seed, status, side, host=None) -> DeviceBatch:
-    """``lo`` / ``hi``: lowest and highest timestamp that can occur."""
+def _enqueue(g, roots, root_ts, fanouts, policy, lo, hi, equal_root_time, allowed_offset, seed, status, side, host=None,
+             meta=None) -> DeviceBatch:
+    """``lo`` / ``hi``: lowest and highest timestamp that can occur; ``host``: pinned address that receives the counts;
+    ``meta``: block of 2 + 2 * hops device words for the counts and the status (default: behind the arena)."""
     roots, root_ts = ops._i64(roots), ops._i64(root_ts)
     n = roots.numel()
     if root_ts.numel() != n:
         raise _C.SglError("build_batch: roots and root_ts differ in length")
     plan = _plan(n, fanouts)
     dev = g.device
-    arena = torch.empty(plan.words + 2 + 2 * len(fanouts), dtype=torch.int64, device=dev)
-    meta = arena[plan.words:]
+    arena = torch.empty(plan.words + (2 + 2 * len(fanouts) if meta is None else 0), dtype=torch.int64, device=dev)
+    if meta is None:
+        meta = arena[plan.words:]
     sp = _C.stream_ptr()
     ws = _C.WORKSPACE.get(plan.ws_bytes, dev, sp)
     base = arena.data_ptr()
@@ -167,7 +170,7 @@ def _enqueue(g, roots, root_ts, fanouts, policy, lo, hi, equal_root_time, allowe
         g.indptr.data_ptr(), g.nbr.data_ptr(), g.ts.data_ptr(), g.eid.data_ptr(), None if g.fence is None else g.fence.data_ptr(),
         g.num_nodes, _C.ptr(roots), _C.ptr(root_ts), n, plan.fan, len(fanouts),
         _C.POLICY[policy] if isinstance(policy, str) else int(policy), int(bool(equal_root_time)), int(allowed_offset),
-        int(seed) & (2 ** 64 - 1), ops.bits_for(g.num_nodes - 1), ops.bits_for(hi - lo), lo, base, base + 8 * plan.words,
+        int(seed) & (2 ** 64 - 1), ops.bits_for(g.num_nodes - 1), ops.bits_for(hi - lo), lo, base, meta.data_ptr(),
         None if status is None else status.ptr(), host, ws.data_ptr(), ws.numel(), None if side is None else side.cuda_stream, sp))
     return DeviceBatch(g, n, fanouts, plan, arena, meta, status)
 
@@ -222,7 +225,7 @@ def build_batch(g, roots, root_ts, fanouts, policy="recent", **kw) -> List[dict]
     last = 1 + 2 * len(fanouts)
     db = _enqueue(g, roots, root_ts, fanouts, policy, lo, hi, kw.get("equal_root_time", False), kw.get("allowed_offset", -1),
                   kw.get("seed", 0), None, None, addr)
-    _C.check(_C.lib().sgl_wait_word(addr + 8 * (last + 1), _C.stream_ptr()))
+    _C.check(_C.lib().sgl_wait_word(addr + 8 * (last + 1), 1, _C.stream_ptr()))
     host, bits = words[:last], words[last] & 0xFFFFFFFF
     if bits & 2:
         a, b = _root_range(g, root_ts)

@@ -183,6 +183,19 @@ def lower_bound(sorted_vals, values):
     return out
 
 
+def chunk_mask(g: TCSR, chunks, node_chunk):
+    """(mask over chunks, chunk of every node on the GPU, number of chunks), or (None, None, 0) without a filter."""
+    if node_chunk is None or not node_chunk.numel() or chunks is None:
+        return None, None, 0
+    dev = g.device
+    if not hasattr(g, "_node_chunk_dev"):
+        g._node_chunk_dev = node_chunk.to(dev, I64).contiguous()
+        g._num_chunks = int(node_chunk.max().item()) + 1
+    mask = torch.zeros(g._num_chunks, dtype=torch.uint8, device=dev)
+    mask[chunks.to(dev, I64)] = 1
+    return mask, g._node_chunk_dev, g._num_chunks
+
+
 def seeds_in_window(ev, g: TCSR, chunks, node_chunk, t_begin: int, t_end: int, *, status: Optional[StatusWord] = None):
     """Roots of the events with t_begin <= ts < t_end whose source node is in one of ``chunks``.
     Returns (roots, ts_ptr, ts, q_ptr, q_eid) trimmed to size (two small read-backs: window bounds, counts)."""
@@ -191,16 +204,7 @@ def seeds_in_window(ev, g: TCSR, chunks, node_chunk, t_begin: int, t_end: int, *
     dev = ev_src.device
     lo, hi = lower_bound(ev_ts, torch.tensor([t_begin, t_end], dtype=I64, device=dev)).tolist()
     n = max(hi - lo, 0)
-    chunk_mask = None
-    num_chunks = 0
-    d_node_chunk = None
-    if node_chunk is not None and node_chunk.numel() and chunks is not None:
-        if not hasattr(g, "_node_chunk_dev"):
-            g._node_chunk_dev = node_chunk.to(dev, I64).contiguous()
-            g._num_chunks = int(node_chunk.max().item()) + 1
-        d_node_chunk, num_chunks = g._node_chunk_dev, g._num_chunks
-        chunk_mask = torch.zeros(num_chunks, dtype=torch.uint8, device=dev)
-        chunk_mask[chunks.to(dev, I64)] = 1
+    mask, d_node_chunk, num_chunks = chunk_mask(g, chunks, node_chunk)
     roots, tsv, q_eid = (torch.empty(max(n, 1), dtype=I64, device=dev) for _ in range(3))
     ts_ptr, q_ptr = (torch.empty(n + 1, dtype=I64, device=dev) for _ in range(2))
     counts = torch.zeros(3, dtype=I64, device=dev)
@@ -209,7 +213,7 @@ def seeds_in_window(ev, g: TCSR, chunks, node_chunk, t_begin: int, t_end: int, *
     _, wp, wn = _C.workspace(L.sgl_seeds_ws_bytes(n), dev)
     sl = slice(lo, lo + n)
     _C.check(L.sgl_seeds_in_window(_C.ptr(ev_src[sl]) if n else None, _C.ptr(ev_ts[sl]) if n else None,
-                                   _C.ptr(ev_eid[sl]) if n else None, n, _C.ptr(d_node_chunk), _C.ptr(chunk_mask),
+                                   _C.ptr(ev_eid[sl]) if n else None, n, _C.ptr(d_node_chunk), _C.ptr(mask),
                                    num_chunks, g.num_nodes, id_bits, ts_bits, g.ts_min, _C.ptr(roots), _C.ptr(ts_ptr),
                                    _C.ptr(tsv), _C.ptr(q_ptr), _C.ptr(q_eid), _C.ptr(counts),
                                    status.ptr() if status else None, wp, wn, _C.stream_ptr()))
@@ -225,14 +229,7 @@ def slice_window(g: TCSR, chunks, node_chunk, t_begin: int, t_end: int, cap_edge
     in the window."""
     L = _C.lib()
     dev = g.device
-    chunk_mask, d_node_chunk, num_chunks = None, None, 0
-    if chunks is not None and node_chunk is not None and node_chunk.numel():
-        if not hasattr(g, "_node_chunk_dev"):
-            g._node_chunk_dev = node_chunk.to(dev, I64).contiguous()
-            g._num_chunks = int(node_chunk.max().item()) + 1
-        d_node_chunk, num_chunks = g._node_chunk_dev, g._num_chunks
-        chunk_mask = torch.zeros(num_chunks, dtype=torch.uint8, device=dev)
-        chunk_mask[chunks.to(dev, I64)] = 1
+    mask, d_node_chunk, num_chunks = chunk_mask(g, chunks, node_chunk)
     n, cap = g.num_nodes, max(int(cap_edges), 1)
     nodes, node_ptr = torch.empty(max(n, 1), dtype=I64, device=dev), torch.empty(n + 1, dtype=I64, device=dev)
     group_ts, nbr, ts, eid = (torch.empty(cap, dtype=I64, device=dev) for _ in range(4))
@@ -240,7 +237,7 @@ def slice_window(g: TCSR, chunks, node_chunk, t_begin: int, t_end: int, cap_edge
     counts = torch.zeros(3, dtype=I64, device=dev)
     _, wp, wn = _C.workspace(L.sgl_slice_window_ws_bytes(n), dev)
     _C.check(L.sgl_slice_window(_C.ptr(g.indptr), _C.ptr(g.nbr), _C.ptr(g.ts), _C.ptr(g.eid), n, _C.ptr(d_node_chunk),
-                                _C.ptr(chunk_mask), num_chunks, int(t_begin), int(t_end), int(cap_edges), _C.ptr(nodes),
+                                _C.ptr(mask), num_chunks, int(t_begin), int(t_end), int(cap_edges), _C.ptr(nodes),
                                 _C.ptr(node_ptr), _C.ptr(group_ts), _C.ptr(group_ptr), _C.ptr(nbr), _C.ptr(ts), _C.ptr(eid),
                                 _C.ptr(counts), status.ptr() if status else None, wp, wn, _C.stream_ptr()))
     u, gcnt, e = counts.tolist()
@@ -284,7 +281,7 @@ def unique_pairs(a_id, a_ts, b_id=None, b_ts=None, *, id_bits, ts_bits, ts_base,
     out_ts = torch.empty(max(n, 1), dtype=I64, device=dev)
     inv_a = torch.empty(max(na, 1), dtype=I64, device=dev)
     inv_b = torch.empty(max(nb, 1), dtype=I64, device=dev) if nb else None
-    d_nu = torch.zeros(1, dtype=I64, device=dev)
+    d_nu = torch.empty(1, dtype=I64, device=dev)
     _, wp, wn = _C.workspace(L.sgl_unique_pairs_ws_bytes(n), dev)
     _C.check(L.sgl_unique_pairs(_C.ptr(a_id), _C.ptr(a_ts), na, _C.ptr(d_n_a), _C.ptr(b_id), _C.ptr(b_ts), nb,
                                 _C.ptr(d_n_b), int(id_bits), int(ts_bits), int(ts_base), _C.ptr(out_id), _C.ptr(out_ts),
@@ -334,7 +331,7 @@ class NodeRelabeler:
         dev = ids.device
         out_local = torch.empty(max(n, 1), dtype=I64, device=dev)
         new_ids = torch.empty(max(n, 1), dtype=I64, device=dev)
-        d_new = torch.zeros(1, dtype=I64, device=dev)
+        d_new = torch.empty(1, dtype=I64, device=dev)
         _, wp, wn = _C.workspace(L.sgl_relabel_nodes_ws_bytes(n), dev)
         _C.check(L.sgl_relabel_nodes(_C.ptr(ids), n, _C.ptr(d_n), self.num_nodes, _C.ptr(self.mapper), _C.ptr(self.mask),
                                      self.epoch, _C.ptr(self.next_local), _C.ptr(out_local), _C.ptr(new_ids),
@@ -405,7 +402,7 @@ def cache_gather(cache_rows, hitmap, backing, ids, *, status: Optional[StatusWor
     out = torch.empty((n,) + tuple(cache_rows.shape[1:]), dtype=cache_rows.dtype, device=dev)
     miss_pos = torch.empty(max(n, 1), dtype=I64, device=dev)
     miss_ids = torch.empty(max(n, 1), dtype=I64, device=dev)
-    counts = torch.zeros(2, dtype=I64, device=dev)
+    counts = torch.empty(2, dtype=I64, device=dev)
     _, wp, wn = _C.workspace(L.sgl_cache_gather_ws_bytes(n), dev)
     _C.check(L.sgl_cache_gather(_C.ptr(cache_rows), cache_rows.shape[0], _C.ptr(hitmap), hitmap.numel(),
                                 _C.ptr(backing), row_bytes, _C.ptr(ids), n,
@@ -563,8 +560,8 @@ def plan_route(layer_ids, node_parts, pid: int, rep_indptr, rep_ranks, rep_locs,
     n = layer_ids.numel()
     dev = layer_ids.device
     ranks, rows, locs = (torch.empty(max(cap, 1), dtype=I64, device=dev) for _ in range(3))
-    sizes = torch.zeros(num_parts, dtype=I64, device=dev)
-    total = torch.zeros(1, dtype=I64, device=dev)
+    sizes = torch.empty(num_parts, dtype=I64, device=dev)
+    total = torch.empty(1, dtype=I64, device=dev)
     _, wp, wn = _C.workspace(L.sgl_plan_route_ws_bytes(n, cap), dev)
     _C.check(L.sgl_plan_route(_C.ptr(layer_ids), n, _C.ptr(d_n), _C.ptr(_i64(node_parts)), node_parts.numel(), int(pid),
                               _C.ptr(rep_indptr), _C.ptr(rep_ranks), _C.ptr(rep_locs), int(num_parts), int(cap), _C.ptr(ranks),
@@ -609,7 +606,7 @@ def mail_reduce(ids_a, ids_b, ts, num_nodes: int, segments=(), *, want_pos: bool
     pos = torch.empty(cap, dtype=I64, device=dev) if want_pos else None
     out_ts = torch.empty(cap, dtype=torch.float32, device=dev)
     mail = torch.empty((cap, width), dtype=torch.float32, device=dev) if segs else None
-    d_u = torch.zeros(1, dtype=I64, device=dev)
+    d_u = torch.empty(1, dtype=I64, device=dev)
     k = len(segs)
     arr_a = (C.c_void_p * max(k, 1))(*[a.data_ptr() for a, _ in segs])
     arr_b = (C.c_void_p * max(k, 1))(*[b.data_ptr() for _, b in segs])

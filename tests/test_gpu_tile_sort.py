@@ -6,7 +6,7 @@ import torch
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("n", [1, 63, 64, 767, 768, 2048, 2049, 148 * 256, 148 * 256 + 1, 160001, 606208])
+@pytest.mark.parametrize("n", [1, 63, 64, 767, 768, 2048, 2049, 148 * 256, 148 * 256 + 1, 160001, 606208, 606209, 1212416, 1212417])
 @pytest.mark.parametrize("bits", [1, 44, 64])
 @pytest.mark.parametrize("pattern", ["random", "few values", "ascending", "descending"])
 def test_stable_at_every_form(n, bits, pattern):

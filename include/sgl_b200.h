@@ -558,6 +558,33 @@ int sgl_build_batch(const int64_t* indptr, const int64_t* nbr, const int64_t* ts
                     uint64_t seed, int id_bits, int ts_bits, int64_t ts_base, int64_t* arena, int64_t* meta,
                     int32_t* d_status, int64_t* host_meta, void* ws, size_t ws_bytes, void* side_stream, void* stream);
 
+/* ------------------------------------------------------------------------------------------------
+ * One query of the graph API in one call: roots of the window [t_begin, t_end) (sgl_seeds_in_window), the negatives
+ * behind their (root, time) pairs, n_hops hops (sgl_sample_layer_fenced), node-level relabel of roots and neighbours
+ * (sgl_relabel_nodes).  The events of the window lie in [ev_from, ev_from + cap) of the time-ordered event arrays
+ * (host-known bounds; the exact ones are searched on the device).  restart != 0: numbering starts at 0 (with a new epoch).
+ * arena: sgl_query_layout(...) words, sections in this order, sizes in section_words (8 + 8 * n_hops entries):
+ *   roots (global), roots (local), ts_ptr, q_ptr, q_eid, query nodes, query times; per hop nbr, dst, ts, dt (fp32),
+ *   ts - t (int64), eid, local ids, offsets; new global ids of all lists in local order
+ * meta[10 + 2 * n_hops]: roots, pairs, events, queries, first local id, status word, window (2), valid events, edges per hop,
+ * new ids per list; host_meta (pinned, one word more): receives meta and then a 1 (see sgl_wait_word).
+ * Replaces: submit_query's worker (csrc/include/starrygl/sample.cu.hpp:1932-1990).
+ * sgl_query_blocks: source nodes, source times and column indices of the hops' message-flow blocks (self loops
+ * included) into `out`: per hop (d + n) nodes, (d + n) times, n indices, with d = queries and n = counts[l].
+ * ---------------------------------------------------------------------------------------------- */
+int64_t sgl_query_layout(int64_t cap, int64_t n_neg, int fanout, int n_hops, int64_t* section_words);
+size_t sgl_query_ws_bytes(int64_t cap, int64_t n_neg, int fanout, int n_hops);
+int sgl_query(const int64_t* indptr, const int64_t* nbr, const int64_t* ts, const int64_t* eid, const int64_t* fence,
+              int64_t num_nodes, const int64_t* ev_src, const int64_t* ev_ts, const int64_t* ev_eid, int64_t ev_from,
+              int64_t cap, int64_t t_begin, int64_t t_end, const int64_t* node_chunk, const uint8_t* chunk_mask,
+              int64_t num_chunks, const int64_t* neg, const int64_t* neg_ts, int64_t n_neg, int fanout, int n_hops,
+              int policy, int equal_root_time, int64_t allowed_offset, int keep_root_time, int id_bits, int ts_bits,
+              int64_t ts_base, int64_t* mapper, int64_t* mask, int64_t epoch, int restart, int64_t* d_next_local,
+              int64_t* arena, int64_t* meta, int64_t* host_meta, void* ws, size_t ws_bytes, void* stream);
+int sgl_query_blocks(int n_hops, const int64_t* const* node, const int64_t* const* ts, const int64_t* counts,
+                     const int64_t* q_ts, const int64_t* ts_ptr, const int64_t* roots_local, const int64_t* neg,
+                     int64_t n_roots, int64_t n_pairs, int64_t n_queries, int64_t* out, void* stream);
+
 /* Small results for the host.  sgl_host_words: a pinned buffer of 512 words that belongs to the calling thread.
  * sgl_wait_word: waits until work on the stream has set *flag (pinned memory) to at_least or more.  sgl_read_back: copies up to 511 words of
  * device memory to the host through that buffer and waits for them. */

@@ -98,7 +98,16 @@ class AsyncBlock:
         """Per hop: destination nodes = source nodes of the previous hop (the roots' queries for hop 0); source nodes
         = [destinations (when ``self_loop``)] + the hop's neighbours in sampling order."""
         mfgs = []
-        last_nodes = torch.repeat_interleave(root.roots, root.ts_ptr[1:] - root.ts_ptr[:-1]) if root.root_num else root.roots
+        native = starrygl_ops.query_blocks(root, neg_roots, neighbors) if self_loop else None
+        if native is not None:
+            for nb, (num_dst, src_nid, src_ts, indices) in zip(neighbors, native):
+                eid = nb.neighbors_eid // 2 if add_inverse_edge else nb.neighbors_eid
+                mfgs.append(Block(nb.root_start_ptr, indices, num_dst + nb.neighbor_num, num_dst, {"nid": src_nid, "ts": src_ts},
+                                  {"eid": eid, "dt": nb.neighbors_dt}))
+            mfgs.reverse()
+            return root, neg_roots, mfgs, nid_mapper
+        last_nodes = (torch.repeat_interleave(root.roots, root.ts_ptr[1:] - root.ts_ptr[:-1], output_size=root.root_ts_num)
+                      if root.root_num else root.roots)
         last_ts = root.ts
         if neg_roots is not None and neg_roots.root_num:
             last_nodes = torch.cat([last_nodes, neg_roots.roots])

@@ -18,6 +18,8 @@ hop l at the time of the edge that reached it (or at the root's time with ``keep
 """
 import queue
 import threading
+from bisect import bisect_left
+from collections import deque
 from typing import List, Optional
 
 import torch
@@ -195,8 +197,167 @@ class TemporalResult:
         return f"<TemporalResult with {len(self.neighbors_list)} neighbor layers>"
 
 
+class _QueryPlan:
+    """Arena layout of a query of one shape (events at most, negatives, fan-out, hops)."""
+
+    def __init__(self, cap, n_neg, fanout, hops):
+        import ctypes as C
+        L = _C.lib()
+        sec = (C.c_int64 * (8 + 8 * hops))()
+        self.words = int(L.sgl_query_layout(cap, n_neg, fanout, hops, sec))
+        if self.words < 0:
+            raise _C.SglError("query: bad shape")
+        self.ws_bytes = int(L.sgl_query_ws_bytes(cap, n_neg, fanout, hops))
+        self.start, at = [], 0
+        for w in sec:
+            self.start.append(at)
+            at += int(w)
+
+
+class _Arena:
+    """All arrays of one query (see ``sgl_query``) with their sizes known on the host: ``cut(section, n)`` is a view."""
+
+    def __init__(self, buf, plan, hops, meta):
+        self.buf, self.start, self.hops = buf, plan.start, hops
+        self.n_roots, self.n_pairs, self.n_events, self.n_queries = meta[:4]
+        self.edges = meta[9:9 + hops]
+        self.n_new = sum(meta[9 + hops:10 + 2 * hops])
+
+    def cut(self, section, n, floats=False):
+        s = self.start[section]
+        if floats:
+            return self.buf[s:s + (n + 1) // 2].view(torch.float32)[:n]
+        return self.buf[s:s + n]
+
+    def ptr(self, section):
+        return self.buf.data_ptr() + 8 * self.start[section]
+
+
+class _ArenaRoot(TemporalRoot):
+    """Roots of a query under their local ids; the tensors are cut out of the query's arena on first use."""
+
+    _SECTIONS = {"roots": (1, "n_roots", 0), "ts_ptr": (2, "n_roots", 1), "ts": (6, "n_pairs", 0), "q_ptr": (3, "n_pairs", 1),
+                 "q_eid": (4, "n_events", 0)}
+
+    def __init__(self, arena):
+        self._a = arena
+
+    def __getattr__(self, name):
+        spec = _ArenaRoot._SECTIONS.get(name)
+        if spec is None:
+            raise AttributeError(name)
+        a = self.__dict__["_a"]
+        t = self.__dict__[name] = a.cut(spec[0], getattr(a, spec[1]) + spec[2])
+        return t
+
+    @property
+    def root_num(self):
+        return self._a.n_roots
+
+    @property
+    def root_ts_num(self):
+        return self._a.n_pairs
+
+
+class _ArenaNeighbor(TemporalNeighbor):
+    """One hop of a query, cut out of the query's arena."""
+
+    def __init__(self, arena, level):
+        self._a, self._l, self._b = arena, level, 7 + 8 * level
+        self._n = arena.edges[level]
+        self._nq = arena.n_queries if level == 0 else arena.edges[level - 1]
+        self._owner, self._neighbors_override = None, None
+
+    def _cut(self):
+        return self._n
+
+    @property
+    def hop(self):
+        a, b, n = self._a, self._b, self._n
+        return ops.Hop(a.cut(b, n), a.cut(b + 1, n), a.cut(b + 2, n), a.cut(b + 3, n, True), a.cut(b + 5, n),
+                       a.cut(b + 7, self._nq + 1), n, a.cut(b + 4, n))
+
+    @property
+    def neighbors(self):
+        return self._neighbors_override if self._neighbors_override is not None else self._a.cut(self._b + 6, self._n)
+
+    @neighbors.setter
+    def neighbors(self, value):
+        self._neighbors_override = value
+
+    @property
+    def root_start_ptr(self):
+        return self._a.cut(self._b + 7, self._nq + 1)
+
+    @property
+    def neighbors_ts(self):
+        return self._a.cut(self._b + 2, self._n)
+
+    @property
+    def neighbors_eid(self):
+        return self._a.cut(self._b + 5, self._n)
+
+    @property
+    def neighbors_dt(self):
+        return self._a.cut(self._b + 4, self._n)
+
+
+class _QueryFuture:
+    """A query whose kernels are enqueued; ``wait()`` reads its sizes and builds the result."""
+
+    def __init__(self, graph, slot, buf, plan, hops, neg):
+        self.graph, self.slot, self.buf, self.plan, self.hops, self.neg = graph, slot, buf, plan, hops, neg
+
+    def wait(self):
+        g, hops = self.graph, self.hops
+        addr, words = self.slot
+        n = 10 + 2 * hops
+        _C.check(_C.lib().sgl_wait_word(addr + 8 * n, 1, g.stream.cuda_stream))
+        meta = words[:n]
+        g._slots.append(self.slot)
+        bits = meta[5] & 0xFFFFFFFF
+        if bits:
+            raise _C.SglError(f"submit_query: device status {bits} ({_C.decode_status(bits)})")
+        arena = _Arena(self.buf, self.plan, hops, meta)
+        out = TemporalResult(_ArenaRoot(arena), self.neg)
+        out.neighbors_list = [_ArenaNeighbor(arena, l) for l in range(hops)]
+        out._remapper = arena.cut(7 + 8 * hops, arena.n_new)
+        return out
+
+
+def query_blocks(root, neg_roots, neighbors):
+    """Source nodes, source times and column indices of the blocks of a query's hops (self loops included) in one launch;
+    None when the parts are not those of one query as ``CUDAGraph.get`` returned it.  Yields (dst count, nid, ts, indices)."""
+    if not neighbors or not isinstance(root, _ArenaRoot):
+        return None
+    a = root._a
+    if len(neighbors) != a.hops or any(not isinstance(nb, _ArenaNeighbor) or nb._a is not a or nb._l != l
+                                       or nb._neighbors_override is not None for l, nb in enumerate(neighbors)):
+        return None
+    n_neg = 0 if neg_roots is None else neg_roots.root_num
+    # (roots whose tensors were handed out may have been replaced: then the general path takes what they hold now)
+    if n_neg != a.n_queries - a.n_pairs or any(root.__dict__.get(k, a.buf).untyped_storage().data_ptr() != a.buf.untyped_storage().data_ptr()
+                                               for k in ("roots", "ts", "ts_ptr")):
+        return None
+    import ctypes as C
+    hops = a.hops
+    dst = [a.n_queries] + a.edges[:-1]
+    total = sum(2 * (d + n) + n for d, n in zip(dst, a.edges))
+    out = torch.empty(total, dtype=torch.int64, device=a.buf.device)
+    node = (C.c_void_p * hops)(*[a.ptr(7 + 8 * l + 6) for l in range(hops)])
+    ts = (C.c_void_p * hops)(*[a.ptr(7 + 8 * l + 2) for l in range(hops)])
+    cnt = (C.c_int64 * hops)(*a.edges)
+    _C.check(_C.lib().sgl_query_blocks(hops, node, ts, cnt, a.ptr(6), a.ptr(2), a.ptr(1), None if n_neg == 0 else neg_roots.roots.data_ptr(),
+                                       a.n_roots, a.n_pairs, a.n_queries, out.data_ptr(), _C.stream_ptr()))
+    blocks, at = [], 0
+    for d, n in zip(dst, a.edges):
+        blocks.append((d, out[at:at + d + n], out[at + d + n:at + 2 * (d + n)], out[at + 2 * (d + n):at + 2 * (d + n) + n]))
+        at += 2 * (d + n) + n
+    return blocks
+
+
 class CUDAGraph:
-    """Temporal graph on one GPU + an asynchronous sampling worker (one thread, FIFO results)."""
+    """Temporal graph on one GPU + an asynchronous sampling queue (FIFO results)."""
 
     def __init__(self, g: ops.TCSR, ev, chunk_size, mapper, stream, rank):
         self.g = g
@@ -206,10 +367,14 @@ class CUDAGraph:
         self.status = ops.StatusWord(g.device)
         self.relabel = ops.NodeRelabeler(g.num_nodes, g.device)
         self._tasks = queue.Queue()
-        self._results = queue.Queue()
+        self._results = deque()
         self._closed = False
-        self._worker = threading.Thread(target=self._run, daemon=True)
-        self._worker.start()
+        self._worker = None               # started by the first task that has to wait for the GPU on the way
+        self._pending = 0                 # tasks that the worker has not finished
+        self._lock = threading.Lock()
+        self._slots = []                  # free pinned result words, (address, ctypes array)
+        self._ev_index = None
+        self._plans = {}
 
     # ---- synchronous entry points -----------------------------------------------------------------------
     def get_negative_root(self, negative_root: torch.Tensor, negative_time: torch.Tensor) -> NegativeRoot:
@@ -285,32 +450,115 @@ class CUDAGraph:
     # ---- asynchronous queue ----------------------------------------------------------------------------------
     def submit_query(self, time_start, time_end, chunk_list, test_generate_samples, test_generate_samples_ts,
                      sample_type, layers, fanout, allowed_offset, equal_root_time, keep_root_time, op) -> None:
+        """Queue one task; results come back from :meth:`get` in the order of submission.  Sampling tasks are enqueued on
+        the graph's stream at once -- one foreign call, nothing waits for the GPU; tasks whose sizes the host has to learn on
+        the way (the chunk slice, windows above the mini-batch limit) run on a worker thread, and while it has work
+        everything behind goes through it, so that the relabel's numbering keeps the order."""
         if self._closed:
             raise RuntimeError("graph is closed")
-        fut = {"event": threading.Event(), "value": None, "error": None}
         neg = self.get_negative_root(test_generate_samples, test_generate_samples_ts)
-        self._tasks.put((fut, (int(time_start), int(time_end), chunk_list, neg, sample_type, int(layers), int(fanout),
-                               int(allowed_offset), bool(equal_root_time), bool(keep_root_time), op)))
-        self._results.put(fut)
+        task = (int(time_start), int(time_end), chunk_list, neg, sample_type, int(layers), int(fanout), int(allowed_offset),
+                bool(equal_root_time), bool(keep_root_time), op)
+        with self._lock:
+            if self._pending == 0:
+                try:
+                    fut = self._enqueue(*task)
+                except BaseException as e:       # delivered to the caller of get()
+                    fut = {"event": None, "value": None, "error": e}
+                if fut is not None:
+                    self._results.append(fut)
+                    return
+            fut = {"event": threading.Event(), "value": None, "error": None}
+            self._pending += 1
+            if self._worker is None:
+                self._worker = threading.Thread(target=_serve, args=(self._tasks, self.g.device), daemon=True)
+                self._worker.start()
+            self._tasks.put((self, fut, task))
+            self._results.append(fut)
+
+    def _window(self, t0, t1):
+        """Host-known bounds of the window's events: (first, at most) from every 256th timestamp of the stream."""
+        if self._ev_index is None:
+            self._ev_index = self.ev[1][::256].tolist()
+        idx, m = self._ev_index, self.ev[1].numel()
+        first = max(bisect_left(idx, t0) - 1, 0) * 256
+        last = min(bisect_left(idx, t1) * 256, m)
+        if last <= first:
+            first, last = min(first, m - 1), min(first, m - 1) + 1
+        return first, last - first
+
+    def _slot(self):
+        if not self._slots:
+            import ctypes as C
+            block = torch.empty(64 * 32, dtype=torch.int64).pin_memory()
+            self._slot_blocks = getattr(self, "_slot_blocks", []) + [block]
+            for i in range(64):
+                addr = block.data_ptr() + 256 * i
+                self._slots.append((addr, (C.c_int64 * 32).from_address(addr)))
+        return self._slots.pop()
+
+    def _enqueue(self, t0, t1, chunks, neg, stype, layers, fanout, off, eq, keep, op) -> Optional[_QueryFuture]:
+        g = self.g
+        m = self.ev[1].numel()
+        if stype not in ("recent", "uniform") or m == 0 or not 0 <= layers <= 8 or fanout < 1:
+            return None
+        first, cap = self._window(t0, t1)
+        if cap > 1_200_000:                 # above the mini-batch sort's limit
+            return None
+        dev = g.device
+        sp = self.stream.cuda_stream
+        n_neg = neg.root_num
+        key = (cap, n_neg, fanout, layers)
+        plan = self._plans.get(key)
+        if plan is None:
+            if len(self._plans) > 64:
+                self._plans.clear()
+            plan = self._plans[key] = _QueryPlan(*key)
+        self.stream.wait_stream(torch.cuda.current_stream(dev))
+        with torch.cuda.stream(self.stream):
+            mask, node_chunk, n_chunks = ops.chunk_mask(g, chunks, self.mapper)
+            neg_ids, neg_ts = neg.roots.contiguous(), neg.ts.contiguous()
+            buf = torch.empty(plan.words + 10 + 2 * layers, dtype=torch.int64, device=dev)
+            ws = _C.WORKSPACE.get(plan.ws_bytes, dev, sp)
+        rl = self.relabel
+        if op == "f":                     # the reference restarts the numbering on "f"
+            rl.epoch += 1
+        slot = self._slot()
+        slot[1][10 + 2 * layers] = 0
+        base = buf.data_ptr()
+        _C.check(_C.lib().sgl_query(
+            g.indptr.data_ptr(), g.nbr.data_ptr(), g.ts.data_ptr(), g.eid.data_ptr(), None if g.fence is None else g.fence.data_ptr(),
+            g.num_nodes, self.ev[0].data_ptr(), self.ev[1].data_ptr(), self.ev[2].data_ptr(), first, cap, t0, t1,
+            None if node_chunk is None else node_chunk.data_ptr(), None if mask is None else mask.data_ptr(), n_chunks,
+            neg_ids.data_ptr() if n_neg else None, neg_ts.data_ptr() if n_neg else None, n_neg, fanout, layers, _C.POLICY[stype],
+            int(eq), off, int(keep), ops.bits_for(g.num_nodes - 1), ops.bits_for(g.ts_max - g.ts_min), g.ts_min, rl.mapper.data_ptr(),
+            rl.mask.data_ptr(), rl.epoch, int(op == "f"), rl.next_local.data_ptr(), base, base + 8 * plan.words, slot[0], ws.data_ptr(),
+            ws.numel(), sp))
+        fut = _QueryFuture(self, slot, buf, plan, layers, neg)
+        fut._keep = (neg_ids, neg_ts, mask)   # inputs of kernels that may still be queued
+        return fut
 
     def get(self) -> Optional[TemporalResult]:
         try:
-            fut = self._results.get_nowait()
-        except queue.Empty:
+            fut = self._results.popleft()
+        except IndexError:
             return None
-        fut["event"].wait()
+        if isinstance(fut, _QueryFuture):
+            return fut.wait()
+        if fut["event"] is not None:
+            fut["event"].wait()
         if fut["error"] is not None:
             raise fut["error"]
         return fut["value"]
 
-    def _run(self):
-        torch.cuda.set_device(self.g.device)
-        while True:
-            item = self._tasks.get()
-            if item is None:
-                return
-            fut, (t0, t1, chunks, neg, stype, layers, fanout, off, eq, keep, op) = item
-            try:
+    def _do(self, fut, task):
+        """One task on the worker thread."""
+        t0, t1, chunks, neg, stype, layers, fanout, off, eq, keep, op = task
+        try:
+            nat = self._enqueue(*task)
+            if nat is not None:
+                fut["value"] = nat.wait()
+            else:
                 if stype in ("recent", "uniform"):
                     roots = self.get_seeds_in_chunks(chunks, t0, t1, False)
                     res = self.sample_src_in_chunks_khop(roots, neg, fanout, layers, off, eq, keep, stype)
@@ -320,13 +568,15 @@ class CUDAGraph:
                     res = self.slice_by_chunk_ts(chunks, t0, t1, True)
                     res._status = self.status
                 with torch.cuda.stream(self.stream):
-                    self._remap(res, op == "f")     # the reference restarts the numbering on "f"
+                    self._remap(res, op == "f")
                     self.status.check("submit_query")
                 self.stream.synchronize()
                 fut["value"] = res
-            except BaseException as e:   # delivered to the caller of get()
-                fut["error"] = e
-            fut["event"].set()
+        except BaseException as e:   # delivered to the caller of get()
+            fut["error"] = e
+        with self._lock:
+            self._pending -= 1
+        fut["event"].set()
 
     def close(self):
         if not self._closed:
@@ -338,6 +588,18 @@ class CUDAGraph:
             self.close()
         except Exception:
             pass
+
+
+def _serve(tasks, device):
+    """Worker of one graph; holds the graph only while it has a task of it."""
+    torch.cuda.set_device(device)
+    while True:
+        item = tasks.get()
+        if item is None:
+            return
+        graph, fut, task = item
+        graph._do(fut, task)
+        del item, graph, fut, task
 
 
 def from_edge_index(n: int, chunk_size: int, src: torch.Tensor, dst: torch.Tensor, ts: torch.Tensor, eid: torch.Tensor,

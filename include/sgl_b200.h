@@ -80,6 +80,10 @@ size_t sgl_tcsr_build_ws_bytes(int64_t num_nodes, int64_t m);
 int sgl_tcsr_build(int64_t num_nodes, int64_t m, const int64_t* key, const int64_t* nbr, const int64_t* ts,
                    const int64_t* eid, int64_t* indptr, int64_t* out_nbr, int64_t* out_ts, int64_t* out_eid,
                    int64_t* out_perm, int64_t* h_ts_range, void* ws, size_t ws_bytes, void* stream);
+/* The same with the search index below (out_fence[sgl_tcsr_fence_len(num_nodes, m)], NULL = none) in one call. */
+int sgl_tcsr_build_fenced(int64_t num_nodes, int64_t m, const int64_t* key, const int64_t* nbr, const int64_t* ts,
+                          const int64_t* eid, int64_t* indptr, int64_t* out_nbr, int64_t* out_ts, int64_t* out_eid,
+                          int64_t* out_perm, int64_t* out_fence, int64_t* h_ts_range, void* ws, size_t ws_bytes, void* stream);
 
 /* Search index over the T-CSR rows ("fence"): the timestamp of the last edge of every block of 32 consecutive edges of a
  * row; row r with edges [s, e) owns out_fence[(s >> 5) + r + j], j < ceil((e - s) / 32).  sgl_tcsr_fence_len() entries

@@ -94,13 +94,11 @@ def tcsr_build(key, nbr, ts, eid, num_nodes: int, want_perm: bool = False, want_
     o_nbr, o_ts, o_eid = (torch.empty(m, dtype=I64, device=dev) for _ in range(3))
     perm = torch.empty(m, dtype=I64, device=dev) if want_perm else None
     rng = (C.c_int64 * 2)(0, 0)
+    fence = torch.empty(L.sgl_tcsr_fence_len(num_nodes, m), dtype=I64, device=dev) if want_fence and m and num_nodes else None
     _, wp, wn = _C.workspace(L.sgl_tcsr_build_ws_bytes(num_nodes, m), dev)
-    _C.check(L.sgl_tcsr_build(num_nodes, m, _C.ptr(key), _C.ptr(nbr), _C.ptr(ts), _C.ptr(eid), _C.ptr(indptr),
-                              _C.ptr(o_nbr), _C.ptr(o_ts), _C.ptr(o_eid), _C.ptr(perm), rng, wp, wn, _C.stream_ptr()))
-    fence = None
-    if want_fence and m and num_nodes:
-        fence = torch.empty(L.sgl_tcsr_fence_len(num_nodes, m), dtype=I64, device=dev)
-        _C.check(L.sgl_tcsr_fence(_C.ptr(indptr), _C.ptr(o_ts), num_nodes, m, _C.ptr(fence), _C.stream_ptr()))
+    _C.check(L.sgl_tcsr_build_fenced(num_nodes, m, _C.ptr(key), _C.ptr(nbr), _C.ptr(ts), _C.ptr(eid), _C.ptr(indptr),
+                                     _C.ptr(o_nbr), _C.ptr(o_ts), _C.ptr(o_eid), _C.ptr(perm), _C.ptr(fence), rng, wp, wn,
+                                     _C.stream_ptr()))
     return TCSR(num_nodes, indptr, o_nbr, o_ts, o_eid, perm, int(rng[0]), int(rng[1]), fence)
 
 

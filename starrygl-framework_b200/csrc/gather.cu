@@ -3,7 +3,7 @@
 //   gather_lanes_kernel<V>  flattened copy: consecutive threads move consecutive V-byte lanes (V = 16: 128-bit
 //                           loads/stores; V = 4 for rows that are not 16-byte multiples), so every warp reads one
 //                           contiguous piece of a source row and writes one contiguous piece of the output.
-//   gather_bulk_kernel      per-warp pipeline of bulk asynchronous copies: each lane asks the copy engine for one
+//   bulk_rows_kernel        per-warp pipeline of bulk asynchronous copies: each lane asks the copy engine for one
 //                           source row (global -> shared, completion counted on an mbarrier), then one lane
 //                           writes the whole stage back with a single shared -> global bulk copy.  The payload
 //                           never passes through registers.  All waits are bounded.
@@ -176,15 +176,47 @@ __device__ __forceinline__ void bulk_wait_read() {
 __device__ __forceinline__ void bulk_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
 __device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 
+// Where row i of a bulk copy comes from, in three steps that depend on each other and that the pipeline keeps apart, so that
+// their latencies overlap the copies: first(i) and second(first) are loads, source() turns the result into an address
+// (nullptr: the output row is left as it is).
+struct TableRows {
+  const char* table;
+  int64_t table_rows, src_pitch;
+  const int64_t *idx, *map;
+  int64_t map_len;
+  const float* ts_table;
+  float* out_ts;
+  int32_t* d_status;
+  using Key = int64_t;
+  static constexpr int64_t kBad = INT64_MIN;
+  __device__ __forceinline__ Key first(int64_t i) const { return __ldg(idx + i); }
+  __device__ __forceinline__ Key second(Key r) const {
+    if (map == nullptr) return r;
+    return r >= 0 && r < map_len ? __ldg(map + r) : kBad;
+  }
+  __device__ __forceinline__ const char* source(int64_t i, Key r, float* ts, int64_t* ts_row) const {
+    if (r != kBad && r < 0) r += table_rows;
+    if (r < 0 || r >= table_rows) {
+      dev_flag(d_status, SGL_DEV_BAD_INDEX);
+      return nullptr;
+    }
+    if (ts_table) {
+      *ts = __ldg(ts_table + r);
+      *ts_row = i;
+    }
+    return table + r * src_pitch;
+  }
+  __device__ __forceinline__ void put_ts(int64_t i, float ts) const { out_ts[i] = ts; }
+};
+
 // Output rows must be contiguous (dst_pitch == row_bytes); row_bytes multiple of 16; rows_per_stage <= 32.
-template <int WARPS, int STAGES>
+template <class Rows, int WARPS, int STAGES>
 __global__ void __launch_bounds__(WARPS * 32)
-gather_bulk_kernel(const char* __restrict__ table, int64_t table_rows, uint32_t row_bytes, int64_t src_pitch,
-                   const int64_t* __restrict__ idx, const int64_t* __restrict__ map, int64_t map_len, int64_t n_cap,
-                   const int64_t* d_n, char* __restrict__ out, const float* __restrict__ ts_table,
-                   float* __restrict__ out_ts, int rows_per_stage, int32_t* d_status) {
+bulk_rows_kernel(const Rows src, uint32_t row_bytes, int64_t n_cap, const int64_t* d_n, char* __restrict__ out, int rows_per_stage,
+                 int32_t* d_status) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
   __shared__ __align__(8) uint64_t bars[WARPS][STAGES];
+  __shared__ uint32_t s_have[WARPS][STAGES];             // rows of the stage that have a source
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int64_t n = eff_count(n_cap, d_n);
   const uint32_t stage_bytes = (uint32_t)rows_per_stage * row_bytes;
@@ -201,26 +233,51 @@ gather_bulk_kernel(const char* __restrict__ table, int64_t table_rows, uint32_t 
   }
   __syncwarp();
 
-  // issue the loads of this warp's k-th chunk into stage k % STAGES
-  auto issue = [&](int64_t k) {
+  // this lane's row of the warp's k-th chunk, -1 when there is none
+  auto row_of = [&](int64_t k) -> int64_t {
     const int64_t chunk = gwarp + k * warps_total;
-    if (chunk >= num_chunks) return;
+    if (chunk >= num_chunks || lane >= rows_per_stage) return -1;
+    const int64_t i = chunk * rows_per_stage + lane;
+    return i < n ? i : -1;
+  };
+  float ts_val = 0.f;
+  int64_t ts_row = -1;
+  // issue the loads of the warp's k-th chunk into stage k % STAGES
+  auto issue = [&](int64_t k, typename Rows::Key key) {
+    if (gwarp + k * warps_total >= num_chunks) return;
     const int s = (int)(k % STAGES);
-    const int64_t row0 = chunk * rows_per_stage;
-    const int rows = (int)((n - row0) < rows_per_stage ? (n - row0) : rows_per_stage);
-    const uint32_t bar = smem_u32(&bars[warp][s]);
-    if (lane == 0) mbar_expect_tx(bar, (uint32_t)rows * row_bytes);
-    __syncwarp();
-    if (lane < rows) {
-      int64_t r;
-      if (!resolve_row(idx, map, map_len, table_rows, row0 + lane, true, d_status, &r)) r = 0;  // flagged; keep byte count
-      bulk_g2s(smem_u32(my_smem + (size_t)s * stage_bytes + (size_t)lane * row_bytes), table + r * src_pitch, row_bytes,
-               bar);
-      if (ts_table) out_ts[row0 + lane] = __ldg(ts_table + r);
+    const int64_t i = row_of(k);
+    if (ts_row >= 0) {                   // (of the chunk before: its load has had a whole round to come back)
+      src.put_ts(ts_row, ts_val);
+      ts_row = -1;
     }
+    const char* from = i >= 0 ? src.source(i, key, &ts_val, &ts_row) : nullptr;
+    const uint32_t have = __ballot_sync(0xffffffffu, from != nullptr);
+    const uint32_t bar = smem_u32(&bars[warp][s]);
+    if (lane == 0) {
+      s_have[warp][s] = have;
+      mbar_expect_tx(bar, (uint32_t)__popc(have) * row_bytes);
+    }
+    __syncwarp();
+    if (from) bulk_g2s(smem_u32(my_smem + (size_t)s * stage_bytes + (size_t)lane * row_bytes), from, row_bytes, bar);
   };
 
-  for (int k = 0; k < STAGES; ++k) issue(k);
+  typename Rows::Key one, two;           // keys of the chunk to issue next (both steps done) and of the one after (first step)
+  {
+    typename Rows::Key key[STAGES + 2];
+#pragma unroll
+    for (int k = 0; k < STAGES + 2; ++k) {
+      const int64_t i = row_of(k);
+      key[k] = i >= 0 ? src.first(i) : typename Rows::Key{};
+    }
+#pragma unroll
+    for (int k = 0; k < STAGES + 1; ++k)
+      if (row_of(k) >= 0) key[k] = src.second(key[k]);
+#pragma unroll
+    for (int k = 0; k < STAGES; ++k) issue(k, key[k]);
+    one = key[STAGES];
+    two = key[STAGES + 1];
+  }
   bool failed = false;
   for (int64_t k = 0;; ++k) {
     const int64_t chunk = gwarp + k * warps_total;
@@ -234,23 +291,60 @@ gather_bulk_kernel(const char* __restrict__ table, int64_t table_rows, uint32_t 
       failed = true;
       break;
     }
-    if (lane == 0) {
+    const uint32_t have = s_have[warp][s];
+    const bool whole = have == (rows == 32 ? 0xffffffffu : (1u << rows) - 1u);
+    char* dst = out + row0 * (int64_t)row_bytes;
+    unsigned char* from = my_smem + (size_t)s * stage_bytes;
+    if (whole) {
+      if (lane == 0) {
+        fence_async_smem();
+        bulk_s2g(dst, smem_u32(from), (uint32_t)rows * row_bytes);
+      }
+    } else if (have >> lane & 1u) {      // some rows stay as they are: row by row
       fence_async_smem();
-      bulk_s2g(out + row0 * (int64_t)row_bytes, smem_u32(my_smem + (size_t)s * stage_bytes), (uint32_t)rows * row_bytes);
-      bulk_commit();
-      // the stage written back one iteration ago may be refilled once its store has finished reading shared memory
-      bulk_wait_read<1>();
+      bulk_s2g(dst + (size_t)lane * row_bytes, smem_u32(from + (size_t)lane * row_bytes), row_bytes);
     }
+    bulk_commit();
+    // the stage written back one iteration ago may be refilled once its store has finished reading shared memory
+    bulk_wait_read<1>();
     __syncwarp();
-    if (k >= 1) issue(k - 1 + STAGES);
+    if (k >= 1) {
+      issue(k - 1 + STAGES, one);
+      if (row_of(k + STAGES) >= 0) one = src.second(two);
+      const int64_t i = row_of(k + 1 + STAGES);
+      if (i >= 0) two = src.first(i);
+    }
   }
-  if (lane == 0) bulk_wait_all();
+  if (ts_row >= 0) src.put_ts(ts_row, ts_val);
+  bulk_wait_all();
   if (failed) {
     if (lane == 0) dev_flag(d_status, SGL_DEV_TIMEOUT);
     // give copies still in flight a bounded chance to land before the CTA's shared memory is released
     for (int s = 0; s < STAGES; ++s) mbar_wait_bounded(smem_u32(&bars[warp][s]), 0);
   }
   __syncwarp();
+}
+
+// Rows per stage of the bulk copy: 4 warps x 3 stages per CTA, two CTAs per SM, about 5.5 KB per stage (8 rows of 688 bytes).
+inline int bulk_rows_per_stage(int64_t row_bytes) {
+  constexpr int64_t kBulkBudget = 200 * 1024 / 2;
+  int rows = (int)(kBulkBudget / ((int64_t)kBulkWarps * kBulkStages * row_bytes));
+  const int want = (int)((5632 + row_bytes - 1) / row_bytes);
+  if (rows > want) rows = want;
+  return rows > 32 ? 32 : rows;
+}
+
+template <class Rows>
+int launch_bulk(const Rows& src, int64_t row_bytes, int64_t n, const int64_t* d_n, void* out, int32_t* d_status, cudaStream_t stream) {
+  const int rows_per_stage = bulk_rows_per_stage(row_bytes);
+  const size_t smem = (size_t)kBulkWarps * kBulkStages * rows_per_stage * row_bytes;
+  const int64_t chunks = (n + rows_per_stage - 1) / rows_per_stage;
+  int64_t ctas = (chunks + kBulkWarps - 1) / kBulkWarps;
+  if (ctas > (int64_t)kNumSM * 2) ctas = (int64_t)kNumSM * 2;  // persistent CTAs
+  static std::atomic<uint64_t> done{0};
+  SGL_CUDA_CHECK(allow_smem((const void*)bulk_rows_kernel<Rows, kBulkWarps, kBulkStages>, done, 200 * 1024));
+  return launch(bulk_rows_kernel<Rows, kBulkWarps, kBulkStages>, (unsigned)ctas, kBulkWarps * 32, smem, stream, src, (uint32_t)row_bytes, n,
+                d_n, (char*)out, rows_per_stage, d_status);
 }
 
 // ---------------------------------------------------------------------------------------------------------------
@@ -282,8 +376,41 @@ cache_lookup_kernel(const int32_t* __restrict__ hitmap, int64_t num_ids, const i
     slot_ws[i] = slot;
     rank_ws[i] = rank;
   }
-  publish_and_scan_cta_totals<kCacheThreads>((int64_t)total, cta_miss, done_counter, d_counts + 1);
+  if (publish_and_scan_cta_totals<kCacheThreads>((int64_t)total, cta_miss, done_counter, d_counts + 1) && threadIdx.x == 0)
+    d_counts[0] = n - d_counts[1];
 }
+
+// Rows of a batch out of the cache or the backing store; the lane that locates a miss also enters it in the miss list.
+struct CachedRows {
+  const char* cache_rows;
+  int64_t cache_slots;
+  const char* backing;       // not null
+  int64_t row_bytes;
+  const int64_t* ids;
+  const int32_t *slot_ws, *rank_ws;
+  const int64_t* cta_miss;
+  int64_t *miss_pos, *miss_ids;
+  int32_t* d_status;
+  struct Key {
+    int64_t id;
+    int32_t slot, rank;
+  };
+  __device__ __forceinline__ Key first(int64_t i) const { return {__ldg(ids + i), __ldg(slot_ws + i), __ldg(rank_ws + i)}; }
+  __device__ __forceinline__ Key second(Key k) const { return k; }
+  __device__ __forceinline__ const char* source(int64_t i, Key k, float*, int64_t*) const {
+    if (k.slot >= 0) {
+      if (k.slot < cache_slots) return cache_rows + (int64_t)k.slot * row_bytes;
+      dev_flag(d_status, SGL_DEV_BAD_INDEX);
+      return nullptr;
+    }
+    if (k.slot != -1) return nullptr;
+    const int64_t p = __ldg(cta_miss + i / kCacheThreads) + k.rank;
+    miss_pos[p] = i;
+    miss_ids[p] = k.id;
+    return backing + k.id * row_bytes;
+  }
+  __device__ __forceinline__ void put_ts(int64_t, float) const {}
+};
 
 template <typename V>
 __global__ void __launch_bounds__(kLaneThreads)
@@ -291,10 +418,9 @@ cache_copy_kernel(const char* __restrict__ cache_rows, int64_t cache_slots, cons
                   LaneSplit split, int64_t row_bytes, const int64_t* __restrict__ ids, int64_t n,
                   const int32_t* __restrict__ slot_ws, const int32_t* __restrict__ rank_ws,
                   const int64_t* __restrict__ cta_miss, char* __restrict__ out, int64_t* __restrict__ miss_pos,
-                  int64_t* __restrict__ miss_ids, int64_t* d_counts, int32_t* d_status) {
+                  int64_t* __restrict__ miss_ids, int32_t* d_status) {
   const int64_t total = n * split.lanes;
   const int64_t stride = (int64_t)gridDim.x * kLaneThreads;
-  if (blockIdx.x == 0 && threadIdx.x == 0) d_counts[0] = n - d_counts[1];
   for (int64_t q0 = (int64_t)blockIdx.x * kLaneThreads + threadIdx.x; q0 < total; q0 += stride * kLaneUnroll) {
     V v[kLaneUnroll];
     V* dst[kLaneUnroll];
@@ -632,18 +758,11 @@ extern "C" int sgl_gather_rows(const void* table, int64_t table_rows, int64_t ro
   SGL_REQUIRE(table && idx && out, SGL_ERR_ARG, "gather_rows: null array");
   SGL_REQUIRE(map == nullptr || map_len > 0, SGL_ERR_ARG, "gather_rows: empty map");
   const bool vec_ok = row_bytes % 16 == 0 && src_pitch % 16 == 0 && dst_pitch % 16 == 0 && aligned16(table) && aligned16(out);
-  // bulk configuration: 4 warps x 3 stages per CTA, two CTAs per SM, about 5.5 KB per stage (8 rows of 688 bytes)
-  constexpr int64_t kBulkBudget = 200 * 1024 / 2;
-  int rows_per_stage = (int)(kBulkBudget / ((int64_t)kBulkWarps * kBulkStages * row_bytes));
-  {
-    const int want_rows = (int)((5632 + row_bytes - 1) / row_bytes);
-    if (rows_per_stage > want_rows) rows_per_stage = want_rows;
-    if (rows_per_stage > 32) rows_per_stage = 32;
-  }
+  const int rows_per_stage = bulk_rows_per_stage(row_bytes);
   if (mode == SGL_GATHER_AUTO) {
-    // measured on B200: the bulk-copy pipeline beats 128-bit lanes from 512-byte rows up; below that they tie.  Rows
-    // of which fewer than two fit a stage (above about 4 KB) go through the lanes kernel.
-    const bool bulk_ok = vec_ok && dst_pitch == row_bytes && row_bytes >= 512 && rows_per_stage >= 2 && n >= 1024;
+    // measured on B200 (132,000 and 12,000 rows of 256 ... 1,488 bytes): the bulk-copy pipeline beats 128-bit lanes at every
+    // one of these sizes by 10 - 30 %.  Rows of which fewer than two fit a stage (above about 4 KB) go through the lanes kernel.
+    const bool bulk_ok = vec_ok && dst_pitch == row_bytes && row_bytes >= 256 && rows_per_stage >= 2 && n >= 1024;
     mode = bulk_ok ? SGL_GATHER_BULK : (vec_ok ? SGL_GATHER_VEC : 0);
   }
   if (mode == SGL_GATHER_BULK) {
@@ -651,16 +770,8 @@ extern "C" int sgl_gather_rows(const void* table, int64_t table_rows, int64_t ro
                 "gather_rows: bulk mode needs 16-byte rows and a dense output");
     SGL_REQUIRE(rows_per_stage >= 2, SGL_ERR_UNSUPPORTED, "gather_rows: row of %lld bytes too large for bulk mode",
                 (long long)row_bytes);
-    const size_t smem = (size_t)kBulkWarps * kBulkStages * rows_per_stage * row_bytes;
-    const int64_t chunks = (n + rows_per_stage - 1) / rows_per_stage;
-    int64_t ctas = (chunks + kBulkWarps - 1) / kBulkWarps;
-    if (ctas > (int64_t)kNumSM * 2) ctas = (int64_t)kNumSM * 2;  // persistent CTAs
-    SGL_CUDA_CHECK(cudaFuncSetAttribute(gather_bulk_kernel<kBulkWarps, kBulkStages>,
-                                        cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
-    SGL_CHECK_RC(launch(gather_bulk_kernel<kBulkWarps, kBulkStages>, (unsigned)ctas, kBulkWarps * 32, smem, stream, (const
-                        char*)table, table_rows, (uint32_t)row_bytes, src_pitch, idx, map, map_len, n, d_n, (char*)out,
-                        ts_table, out_ts, rows_per_stage, d_status));
-    return SGL_OK;
+    return launch_bulk(TableRows{(const char*)table, table_rows, src_pitch, idx, map, map_len, ts_table, out_ts, d_status}, row_bytes, n,
+                       d_n, out, d_status, stream);
   }
   if (mode == SGL_GATHER_VEC) {
     SGL_REQUIRE(vec_ok, SGL_ERR_UNSUPPORTED, "gather_rows: 128-bit mode needs 16-byte aligned rows");
@@ -732,18 +843,22 @@ extern "C" int sgl_cache_gather(const void* cache_rows, int64_t cache_slots, con
   SGL_CHECK_RC(launch(cache_lookup_kernel, (unsigned)ctas, kCacheThreads, 0, stream, hitmap, num_ids, ids, n, slot_ws,
                       rank_ws, cta_miss, done, d_counts, d_status));
   const bool vec_ok = row_bytes % 16 == 0 && aligned16(cache_rows) && aligned16(out) && (backing == nullptr || aligned16(backing));
-  if (vec_ok) {
+  if (vec_ok && backing && row_bytes >= 256 && bulk_rows_per_stage(row_bytes) >= 2 && n >= 1024) {     // as in sgl_gather_rows
+    SGL_CHECK_RC(launch_bulk(CachedRows{(const char*)cache_rows, cache_slots, (const char*)backing, row_bytes, ids, slot_ws, rank_ws, cta_miss,
+                                        miss_pos, miss_ids, d_status},
+                             row_bytes, n, nullptr, out, d_status, stream));
+  } else if (vec_ok) {
     const uint32_t lanes = (uint32_t)(row_bytes / 16);
     const int grid = stream_grid(n * lanes, kLaneThreads * kLaneUnroll, 8);
     SGL_CHECK_RC(launch(cache_copy_kernel<uint4>, grid, kLaneThreads, 0, stream, (const char*)cache_rows, cache_slots, (const
                         char*)backing, LaneSplit(lanes, n * lanes), row_bytes, ids, n, slot_ws, rank_ws, cta_miss,
-                        (char*)out, miss_pos, miss_ids, d_counts, d_status));
+                        (char*)out, miss_pos, miss_ids, d_status));
   } else {
     const uint32_t lanes = (uint32_t)(row_bytes / 4);
     const int grid = stream_grid(n * lanes, kLaneThreads * kLaneUnroll, 8);
     SGL_CHECK_RC(launch(cache_copy_kernel<uint32_t>, grid, kLaneThreads, 0, stream, (const char*)cache_rows, cache_slots,
                         (const char*)backing, LaneSplit(lanes, n * lanes), row_bytes, ids, n, slot_ws, rank_ws, cta_miss,
-                        (char*)out, miss_pos, miss_ids, d_counts, d_status));
+                        (char*)out, miss_pos, miss_ids, d_status));
   }
   return scope.submit();
 }

@@ -39,10 +39,10 @@ __device__ __forceinline__ T cta_exclusive_scan(T v, T* total) {
 
 // Every CTA calls this once with its total (same value in all threads).  cta_sums[blockIdx.x] is published;
 // the last CTA to arrive replaces cta_sums[0..gridDim.x) by its exclusive scan, writes the grand total to
-// *grand_total and re-arms *done_counter (0) for the next launch.  Kernels that consume the scanned values
+// *grand_total, re-arms *done_counter (0) for the next launch and gets true.  Kernels that consume the scanned values
 // must be launched after this kernel on the same stream.
 template <int THREADS>
-__device__ __forceinline__ void publish_and_scan_cta_totals(int64_t my_total, int64_t* cta_sums,
+__device__ __forceinline__ bool publish_and_scan_cta_totals(int64_t my_total, int64_t* cta_sums,
                                                            unsigned int* done_counter, int64_t* grand_total) {
   __shared__ bool s_last;
   __shared__ int64_t s_carry;
@@ -54,7 +54,7 @@ __device__ __forceinline__ void publish_and_scan_cta_totals(int64_t my_total, in
     s_carry = 0;
   }
   __syncthreads();
-  if (!s_last) return;
+  if (!s_last) return false;
   __threadfence();
   for (int64_t base = 0; base < gridDim.x; base += THREADS) {
     int64_t idx = base + threadIdx.x;
@@ -71,6 +71,7 @@ __device__ __forceinline__ void publish_and_scan_cta_totals(int64_t my_total, in
     if (grand_total) *grand_total = s_carry;
     *done_counter = 0;
   }
+  return true;
 }
 
 }  // namespace sgl

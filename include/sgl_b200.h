@@ -176,6 +176,18 @@ int sgl_sample_gather(const int64_t* indptr, const int64_t* nbr, const int64_t* 
                       int64_t feat_rows, int64_t row_bytes, int64_t src_pitch, void* out_feats, int gather_mode,
                       int32_t* d_status, void* ws, size_t ws_bytes, void* stream);
 
+/* One mini-batch of a prefetcher: the stream waits for what `consumer` has been given so far, the roots and query times come
+ * out of pinned host memory (host_roots / host_ts, copied to targets / target_ts by a kernel; NULL: they are there), then
+ * sgl_sample_gather_fenced; the number of sampled edges and behind it `seq` go to host_total[0..1] (pinned, see
+ * sgl_wait_word). */
+int sgl_prefetch_batch(const int64_t* host_roots, const int64_t* host_ts, const int64_t* indptr, const int64_t* nbr, const int64_t* ts,
+                       const int64_t* eid, const int64_t* fence, int64_t num_nodes, int64_t* targets, int64_t* target_ts,
+                       int64_t n_targets, int fanout, int policy, int equal_root_time, int64_t allowed_offset,
+                       int keep_root_time, uint64_t seed, uint32_t rng_stream, int64_t* out_nbr, int64_t* out_dst, int64_t* out_ts,
+                       float* out_dt, int64_t* out_eid, int64_t* out_offsets, const void* feat_table, int64_t feat_rows,
+                       int64_t row_bytes, int64_t src_pitch, void* out_feats, int gather_mode, int32_t* d_status, void* ws,
+                       size_t ws_bytes, int64_t* host_total, int64_t seq, void* consumer, void* stream);
+
 /* ------------------------------------------------------------------------------------------------
  * (node, ts)-pair relabel.  Input = two concatenated segments A (n_a items) then B (n_b items);
  * output = the sorted (id, then ts) unique union, its size (*d_n_unique, device), and for every input

@@ -10,12 +10,13 @@ entries.  Iterating yields :class:`PrefetchedBatch` objects in loader order, alr
 current stream; a batch's tensors alias the buffers of its pipeline object and may be read by kernels enqueued on that
 stream until ``depth`` further batches have been requested.
 """
+import ctypes as C
 from collections import deque
 from typing import Iterable, Optional
 
 import torch
 
-from .. import ops
+from .. import _C, ops
 from ..graph.pipeline import SampleGatherPipeline
 
 
@@ -23,8 +24,9 @@ class PrefetchedBatch:
     """Block structure and gathered edge-feature rows of one mini-batch (device tensors, capacity-sized; the valid
     prefix has ``offsets[n_roots]`` edges -- :meth:`num_edges` reads it, one synchronisation)."""
 
-    def __init__(self, pipe: SampleGatherPipeline, n_roots: int, ready: torch.cuda.Event):
+    def __init__(self, pipe: SampleGatherPipeline, n_roots: int, ready: torch.cuda.Event, total=None):
         self.pipe, self.n_roots, self.ready = pipe, n_roots, ready
+        self._total = total               # (address, ctypes words, sequence number) of the pinned edge count
         self.offsets, self.nbr, self.dst, self.ts, self.eid, self.dt = (pipe.offsets[:n_roots + 1], pipe.nbr, pipe.dst,
                                                                         pipe.ts, pipe.eid, pipe.dt)
         self.edge_feats = pipe.out_feats
@@ -35,6 +37,12 @@ class PrefetchedBatch:
         return self
 
     def num_edges(self) -> int:
+        if self._total is not None:
+            addr, words, seq = self._total
+            if words[1] < seq:
+                _C.check(_C.lib().sgl_wait_word(addr + 8, seq, self.pipe.stream.cuda_stream))
+            if words[1] == seq:           # (a later batch of the slot may have overwritten it)
+                return words[0]
         self.ready.synchronize()
         return int(self.offsets[self.n_roots].item())
 
@@ -47,22 +55,60 @@ class HostToDevicePrefetcher:
         self.pipes = [SampleGatherPipeline(g, edge_feats, fanout, policy, max_roots, stream=s, **sampler_options)
                       for s in self.streams]
         self.events = [torch.cuda.Event() for _ in range(self.depth)]
+        self._totals = torch.zeros(2 * self.depth, dtype=torch.int64).pin_memory()   # per slot: edges, sequence number
+        self._seq, self._fn = 0, _C.lib().sgl_prefetch_batch
+        self._bound = [None] * self.depth
+
+    def _bind(self, slot):
+        """Everything of a slot's foreign call that does not change from batch to batch."""
+        v, p, g = C.c_void_p, self.pipes[slot], self.pipes[slot].g
+        a = p.args
+        addr = self._totals.data_ptr() + 16 * slot
+        words = (C.c_int64 * 2).from_address(addr)
+        var = v(0), v(0), v(0), v(0), C.c_int64(0), C.c_int64(0), v(0)       # host roots / times, targets / times, n, seq, consumer
+        table = p.feats
+        args = [var[0], var[1], v(g.indptr.data_ptr()), v(g.nbr.data_ptr()), v(g.ts.data_ptr()), v(g.eid.data_ptr()),
+                v(g.fence.data_ptr() if g.fence is not None else 0), C.c_int64(g.num_nodes), var[2], var[3], var[4], C.c_int(p.k),
+                C.c_int(a["pol"]), C.c_int(a["eq"]), C.c_int64(a["off"]), C.c_int(a["keep"]), C.c_uint64(a["seed"]), C.c_uint32(0),
+                v(p.nbr.data_ptr()), v(p.dst.data_ptr()), v(p.ts.data_ptr()), v(p.dt.data_ptr()), v(p.eid.data_ptr()),
+                v(p.offsets.data_ptr()), v(0 if table is None else table.data_ptr()), C.c_int64(0 if table is None else table.shape[0]),
+                C.c_int64(0 if table is None else p.row_bytes), C.c_int64(0 if table is None else p.src_pitch),
+                v(0 if table is None else p.out_feats.data_ptr()), C.c_int(p.mode), v(p.status.ptr()), v(p.ws.data_ptr()),
+                C.c_size_t(p.ws.numel()), v(addr), var[5], var[6], v(p.stream.cuda_stream)]
+        return args, var, addr, words
 
     def _submit(self, slot, roots, root_ts):
         pipe, st = self.pipes[slot], self.streams[slot]
-        # Orders the slot's reuse behind everything the consumer has enqueued so far on its stream: the work on the
-        # batch that occupied this slot (handed out ``depth`` batches ago) and the kernels that produced ``roots``.
-        # The batch submitted now is only needed ``depth`` requests later, so this does not stall the consumer.
-        st.wait_stream(torch.cuda.current_stream())
         n = roots.numel()
-        with torch.cuda.stream(st):
-            if not roots.is_cuda:
+        if n > pipe.max_roots:
+            raise _C.SglError(f"batch of {n} roots exceeds max_roots={pipe.max_roots}")
+        if roots.dtype != torch.int64 or root_ts.dtype != torch.int64 or root_ts.numel() != n:
+            raise _C.SglError("prefetcher: the loader yields int64 roots and as many int64 query times")
+        if self._bound[slot] is None:
+            self._bound[slot] = self._bind(slot)
+        args, (h_r, h_t, d_r, d_t, c_n, c_seq, c_cons), addr, words = self._bound[slot]
+        h_r.value = h_t.value = None
+        d_r.value, d_t.value = pipe.roots.data_ptr(), pipe.root_ts.data_ptr()
+        roots, root_ts = roots.contiguous(), root_ts.contiguous()
+        if roots.is_cuda:
+            d_r.value, d_t.value = roots.data_ptr(), root_ts.data_ptr()
+        elif roots.is_pinned() and root_ts.is_pinned():
+            h_r.value, h_t.value = roots.data_ptr(), root_ts.data_ptr()
+        else:                             # pageable: staged by a copy, behind what the consumer still does with the slot
+            st.wait_stream(torch.cuda.current_stream())
+            with torch.cuda.stream(st):
                 pipe.roots[:n].copy_(roots, non_blocking=True)
                 pipe.root_ts[:n].copy_(root_ts, non_blocking=True)
-                roots, root_ts = pipe.roots[:n], pipe.root_ts[:n]
-            pipe.run_device(roots.contiguous(), root_ts.contiguous())
-            self.events[slot].record(st)
-        return PrefetchedBatch(pipe, n, self.events[slot])
+        self._seq += 1
+        c_n.value, c_seq.value, c_cons.value = n, self._seq, _C.stream_ptr()
+        # The call orders the slot's reuse behind everything the consumer has enqueued so far on its stream: the work on the
+        # batch that occupied this slot (handed out ``depth`` batches ago) and the kernels that produced ``roots``.
+        # The batch submitted now is only needed ``depth`` requests later, so this does not stall the consumer.
+        _C.check(self._fn(*args))
+        self.events[slot].record(st)
+        b = PrefetchedBatch(pipe, n, self.events[slot], (addr, words, self._seq))
+        b._keep = (roots, root_ts)        # inputs of kernels that may still be queued
+        return b
 
     def __iter__(self):
         it = iter(self.loader)

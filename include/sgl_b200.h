@@ -604,6 +604,12 @@ int sgl_query_blocks(int n_hops, const int64_t* const* node, const int64_t* cons
 /* Small results for the host.  sgl_host_words: a pinned buffer of 512 words that belongs to the calling thread.
  * sgl_wait_word: waits until work on the stream has set *flag (pinned memory) to at_least or more.  sgl_read_back: copies up to 511 words of
  * device memory to the host through that buffer and waits for them. */
+/* Up to 96 device arrays (sizes multiples of 4 bytes) to the host in one copy: packed at the 16-byte aligned offsets at[]
+ * of `staging` (device, total bytes) and copied to `host`, or, with host2, the bytes from `split` on to host2; waits for
+ * the stream. */
+int sgl_export_arrays(int n, const void* const* src, const int64_t* bytes, const int64_t* at, void* staging, void* host,
+                      int64_t total, void* host2, int64_t split, void* stream);
+int sgl_host_words(void** out);
 int sgl_wait_word(const int64_t* flag, int64_t at_least, void* stream);
 int sgl_read_back(const void* src, void* dst, size_t bytes, void* stream);
 

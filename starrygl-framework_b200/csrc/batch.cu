@@ -217,6 +217,53 @@ extern "C" int sgl_build_batch(const int64_t* indptr, const int64_t* nbr, const 
   return done();
 }
 
+// Up to kMaxExport arrays packed one behind the other (16-byte aligned offsets) and copied to the host in one go, or in two
+// when the bytes from `split` on go to a second buffer.
+namespace {
+constexpr int kMaxExport = 96;
+struct Export {
+  const char* src[kMaxExport];
+  int64_t bytes[kMaxExport], at[kMaxExport];
+};
+__global__ void __launch_bounds__(256) pack_kernel(const __grid_constant__ Export x, char* __restrict__ dst) {
+  const int a = blockIdx.y;
+  const char* s = x.src[a];
+  char* d = dst + x.at[a];
+  const int64_t bytes = x.bytes[a], tid = (int64_t)blockIdx.x * 256 + threadIdx.x, stride = (int64_t)gridDim.x * 256;
+  const int64_t quads = ((uintptr_t)s & 15) == 0 ? bytes >> 4 : 0;
+  for (int64_t i = tid; i < quads; i += stride) ((uint4*)d)[i] = ((const uint4*)s)[i];
+  for (int64_t i = quads * 4 + tid; i < bytes >> 2; i += stride) ((uint32_t*)d)[i] = ((const uint32_t*)s)[i];
+}
+}  // namespace
+
+extern "C" int sgl_export_arrays(int n, const void* const* src, const int64_t* bytes, const int64_t* at, void* staging, void* host,
+                                 int64_t total, void* host2, int64_t split, void* stream_) {
+  cudaStream_t stream = (cudaStream_t)stream_;
+  SGL_REQUIRE(n >= 0 && n <= kMaxExport && (n == 0 || (src && bytes && at)) && total >= 0, SGL_ERR_ARG, "export_arrays: at most %d arrays",
+              kMaxExport);
+  if (n == 0 || total == 0) return SGL_OK;
+  SGL_REQUIRE(staging && (host || split == 0), SGL_ERR_ARG, "export_arrays: null buffer");
+  Export x;
+  memset(&x, 0, sizeof(x));
+  int64_t most = 1;
+  for (int i = 0; i < n; ++i) {
+    SGL_REQUIRE((src[i] || bytes[i] == 0) && bytes[i] >= 0 && bytes[i] % 4 == 0 && at[i] % 16 == 0 && at[i] >= 0 && at[i] + bytes[i] <= total,
+                SGL_ERR_ARG, "export_arrays: bad array %d", i);
+    x.src[i] = (const char*)src[i];
+    x.bytes[i] = bytes[i];
+    x.at[i] = at[i];
+    most = bytes[i] > most ? bytes[i] : most;
+  }
+  SGL_CHECK_RC(launch(pack_kernel, dim3((unsigned)stream_grid(most / 16 + 1, 256 * 4, 4), (unsigned)n), 256, 0, stream, x, (char*)staging));
+  if (host2 == nullptr) split = total;
+  SGL_REQUIRE(split >= 0 && split <= total, SGL_ERR_ARG, "export_arrays: bad split");
+  if (split > 0) SGL_CUDA_CHECK(cudaMemcpyAsync(host, staging, (size_t)split, cudaMemcpyDeviceToHost, stream));
+  if (split < total)
+    SGL_CUDA_CHECK(cudaMemcpyAsync(host2, (char*)staging + split, (size_t)(total - split), cudaMemcpyDeviceToHost, stream));
+  SGL_CUDA_CHECK(cudaStreamSynchronize(stream));
+  return SGL_OK;
+}
+
 // Pinned buffer of the calling thread (4,096 bytes) for results that the host waits for.
 extern "C" int sgl_host_words(void** out) {
   SGL_REQUIRE(out, SGL_ERR_ARG, "host_words: out is null");

@@ -6,6 +6,10 @@
 // is the last row of its run.  Rows of nodes owned here are expanded to one entry per replica on another rank, then
 // ordered by rank (stable: ascending list row inside a rank).
 //
+// Up to 32 ranks (three kernels): entries counted per (rank, CTA), one scan of those counts, every entry written straight
+// to its place -- no sort over the capacity (rows x (ranks - 1), ten kernels and 250 us for the last list of an 8,000-root
+// two-hop slot with 90,000 rows).  More ranks:
+//
 //   plan_count_kernel   per row: is it the run's last row and owned here? how many foreign replicas? CTA scan,
 //                       last CTA scans the CTA totals; per-rank sizes by atomic add (order independent)
 //   plan_expand_kernel  writes (rank, row, slot) triplets in row order
@@ -85,10 +89,113 @@ plan_emit_kernel(const uint64_t* __restrict__ keys, const uint32_t* __restrict__
                  int64_t* __restrict__ out_rows, int64_t* __restrict__ out_locs) {
   const int64_t n = eff_count(cap, d_total);
   for (int64_t j = (int64_t)blockIdx.x * kThreads + threadIdx.x; j < n; j += (int64_t)gridDim.x * kThreads) {
-    const uint32_t p = perm[j];
+    const uint32_t p = perm[j] < n ? perm[j] : 0u;      // (a sort that ran into its time limit leaves any value)
     out_ranks[j] = (int64_t)keys[j];
     out_rows[j] = tmp_rows[p];
     out_locs[j] = tmp_locs[p];
+  }
+}
+
+// ---- up to kFewParts ranks: entries counted per (rank, CTA), placed by rank without a sort --------------------------------
+constexpr int kFewParts = 32;
+
+// does row i send its node's row, and to which copies?  [*s, *e) of the replica lists; false: nothing
+__device__ __forceinline__ bool plan_row(const int64_t* __restrict__ ids, int64_t n, int64_t i, const int64_t* __restrict__ node_parts,
+                                         int64_t num_nodes, int64_t pid, const int64_t* __restrict__ indptr, int32_t* d_status,
+                                         int64_t* s, int64_t* e) {
+  const int64_t id = ids[i];
+  if (id < 0 || id >= num_nodes) {
+    dev_flag(d_status, SGL_DEV_BAD_NODE);
+    return false;
+  }
+  if (i + 1 < n) {
+    const int64_t next = ids[i + 1];
+    if (next < id) dev_flag(d_status, SGL_DEV_BAD_INDEX);   // list must be sorted by id
+    if (next == id) return false;
+  }
+  if (node_parts[id] != pid) return false;
+  *s = indptr[id];
+  *e = indptr[id + 1];
+  return true;
+}
+
+__global__ void __launch_bounds__(kThreads)
+plan_tally_kernel(const int64_t* __restrict__ ids, int64_t n_cap, const int64_t* d_n, const int64_t* __restrict__ node_parts,
+                  int64_t num_nodes, int64_t pid, const int64_t* __restrict__ indptr, const int64_t* __restrict__ ranks, int num_parts,
+                  int32_t* __restrict__ tally, int32_t* d_status) {
+  __shared__ int s_cnt[kFewParts];
+  const int64_t n = eff_count(n_cap, d_n);
+  if ((int64_t)blockIdx.x * kThreads >= n) return;
+  if (threadIdx.x < num_parts) s_cnt[threadIdx.x] = 0;
+  __syncthreads();
+  const int64_t i = (int64_t)blockIdx.x * kThreads + threadIdx.x;
+  int64_t s, e;
+  if (i < n && plan_row(ids, n, i, node_parts, num_nodes, pid, indptr, d_status, &s, &e))
+    for (int64_t p = s; p < e; ++p) {
+      const int64_t r = ranks[p];
+      if (r != pid && r >= 0 && r < num_parts) atomicAdd(&s_cnt[r], 1);
+    }
+  __syncthreads();
+  const int64_t ctas = (n + kThreads - 1) / kThreads;
+  if (threadIdx.x < num_parts) tally[threadIdx.x * ctas + blockIdx.x] = s_cnt[threadIdx.x];
+}
+
+// exclusive scan of the (rank, CTA) counts in place, rank by rank; sizes per rank and the total.  One CTA.
+__global__ void __launch_bounds__(1024)
+plan_place_kernel(int64_t n_cap, const int64_t* d_n, int num_parts, int32_t* __restrict__ tally, int64_t* d_send_sizes, int64_t* d_total) {
+  __shared__ int64_t s_carry;
+  const int64_t n = eff_count(n_cap, d_n), ctas = (n + kThreads - 1) / kThreads;
+  if (threadIdx.x == 0) s_carry = 0;
+  __syncthreads();
+  int64_t begin = 0;
+  for (int r = 0; r < num_parts; ++r) {
+    for (int64_t b = 0; b < ctas; b += 1024) {
+      const int64_t j = b + threadIdx.x;
+      const int v = j < ctas ? tally[r * ctas + j] : 0;
+      int tot;
+      const int ex = cta_exclusive_scan<1024, int>(v, &tot);
+      const int64_t carry = s_carry;
+      if (j < ctas) tally[r * ctas + j] = (int32_t)(carry + ex);
+      __syncthreads();
+      if (threadIdx.x == 0) s_carry = carry + tot;
+      __syncthreads();
+    }
+    const int64_t end = s_carry;
+    if (threadIdx.x == 0) d_send_sizes[r] = end - begin;
+    begin = end;
+  }
+  if (threadIdx.x == 0) *d_total = begin;
+}
+
+__global__ void __launch_bounds__(kThreads)
+plan_write_kernel(const int64_t* __restrict__ ids, int64_t n_cap, const int64_t* d_n, const int64_t* __restrict__ node_parts,
+                  int64_t num_nodes, int64_t pid, const int64_t* __restrict__ indptr, const int64_t* __restrict__ ranks,
+                  const int64_t* __restrict__ locs, int num_parts, const int32_t* __restrict__ tally, int64_t cap,
+                  int64_t* __restrict__ out_ranks, int64_t* __restrict__ out_rows, int64_t* __restrict__ out_locs, int32_t* d_status) {
+  const int64_t n = eff_count(n_cap, d_n);
+  if ((int64_t)blockIdx.x * kThreads >= n) return;
+  const int64_t ctas = (n + kThreads - 1) / kThreads;
+  const int64_t i = (int64_t)blockIdx.x * kThreads + threadIdx.x;
+  int64_t s = 0, e = 0;
+  if (!(i < n && plan_row(ids, n, i, node_parts, num_nodes, pid, indptr, nullptr, &s, &e))) s = e = 0;
+  for (int r = 0; r < num_parts; ++r) {
+    if (r == pid) continue;
+    int mine = 0;
+    for (int64_t p = s; p < e; ++p) mine += ranks[p] == r ? 1 : 0;
+    int total;
+    int64_t at = cta_exclusive_scan<kThreads, int>(mine, &total) + tally[r * ctas + blockIdx.x];
+    if (mine == 0) continue;
+    for (int64_t p = s; p < e; ++p) {
+      if (ranks[p] != r) continue;
+      if (at >= cap) {
+        dev_flag(d_status, SGL_DEV_OVERFLOW);
+        break;
+      }
+      out_ranks[at] = r;
+      out_rows[at] = i;
+      out_locs[at] = locs[p];
+      ++at;
+    }
   }
 }
 
@@ -102,7 +209,7 @@ using namespace sgl;
 extern "C" size_t sgl_plan_route_ws_bytes(int64_t n, int64_t cap) {
   if (n < 1) n = 1;
   if (cap < 1) cap = 1;
-  return align_up((size_t)n * 8) + align_up((size_t)ctas_for(n) * 8) + align_up(8) + 2 * align_up((size_t)cap * 8) +
+  return align_up((size_t)kFewParts * ctas_for(n) * 4) + align_up((size_t)n * 8) + align_up((size_t)ctas_for(n) * 8) + align_up(8) + 2 * align_up((size_t)cap * 8) +
          2 * align_up((size_t)cap * 4) + 2 * align_up((size_t)cap * 8) + radix_sort_ws_bytes(cap);
 }
 
@@ -117,14 +224,27 @@ extern "C" int sgl_plan_route(const int64_t* layer_ids, int64_t n, const int64_t
               SGL_ERR_ARG, "plan_route: bad size (1 <= num_parts <= 256, 0 <= pid < num_parts)");
   SGL_REQUIRE(d_send_sizes && d_total, SGL_ERR_ARG, "plan_route: null counter");
   LaunchScope scope(stream);
-  SGL_CHECK_RC(zero_async(d_send_sizes, (size_t)num_parts * sizeof(int64_t), stream));
   if (n == 0) {
+    SGL_CHECK_RC(zero_async(d_send_sizes, (size_t)num_parts * sizeof(int64_t), stream));
     SGL_CHECK_RC(zero_async(d_total, sizeof(int64_t), stream));
     return scope.submit();
   }
   SGL_REQUIRE(layer_ids && node_parts && rep_indptr && rep_ranks && rep_locs && out_ranks && out_rows && out_locs, SGL_ERR_ARG,
               "plan_route: null array");
   const int64_t capc = cap < 1 ? 1 : cap;
+  if (num_parts <= kFewParts && n * num_parts < ((int64_t)1 << 31)) {
+    WsCarver c(ws, ws_bytes);
+    int32_t* tally = c.take<int32_t>((size_t)(num_parts * ctas_for(n)));
+    SGL_REQUIRE(c.ok(), SGL_ERR_WORKSPACE, "plan_route: workspace %zu < %zu bytes", ws_bytes, sgl_plan_route_ws_bytes(n, cap));
+    const unsigned grid = (unsigned)ctas_for(n);
+    SGL_CHECK_RC(launch(plan_tally_kernel, grid, kThreads, 0, stream, layer_ids, n, d_n, node_parts, num_nodes, pid, rep_indptr, rep_ranks,
+                        (int)num_parts, tally, d_status));
+    SGL_CHECK_RC(launch(plan_place_kernel, 1, 1024, 0, stream, n, d_n, (int)num_parts, tally, d_send_sizes, d_total));
+    SGL_CHECK_RC(launch(plan_write_kernel, grid, kThreads, 0, stream, layer_ids, n, d_n, node_parts, num_nodes, pid, rep_indptr, rep_ranks,
+                        rep_locs, (int)num_parts, tally, cap, out_ranks, out_rows, out_locs, d_status));
+    return scope.submit();
+  }
+  SGL_CHECK_RC(zero_async(d_send_sizes, (size_t)num_parts * sizeof(int64_t), stream));
   WsCarver c(ws, ws_bytes);
   int64_t* local_off = c.take<int64_t>(n);
   int64_t* cta_sums = c.take<int64_t>(ctas_for(n));

@@ -6,7 +6,7 @@ dictionaries -- layer 0: ``gids``, ``ts``, ``inv_map``, ``num_neg`` + the task t
 ``indptr``, ``indices``, ``eid``, ``edge_ts``, ``edge_dt``, ``gids``, ``ts`` -- and writes it with ``torch.save`` in the
 layout the reference's loader reads (all tensors on the CPU, ``comm_plan`` = one ``CommPlan`` or ``None`` per layer
 list).  Sampling, (node, ts) relabel, CSC and the route plans run through the library
-(:func:`starrygl.graph.batch.build_batch_async`, ``sgl_plan_route``); the T-CSR is built once per partition.
+(``sgl_build_batch``, ``sgl_plan_route``); the T-CSR is built once per partition.
 
 Supported policy space = what the GPU sampler implements: continuous graphs (``graph_type == 'c'``), ``recent`` and
 ``uniform`` layers, ``end_offset`` 0 (strictly earlier edges) or 1 (edges at the query time included; integer
@@ -20,7 +20,15 @@ import torch
 
 from .. import _C, ops
 from ..cache.cache_route import CommPlan
-from .batch import build_batch_async
+from .batch import _enqueue, _graph_range, _root_range
+
+
+_PINNED_MOST, _PINNED_TOTAL = 256 << 20, 2 << 30
+
+
+def _pinned_now() -> int:
+    """Bytes of pinned memory in use through torch's host allocator."""
+    return int(torch.cuda.host_memory_stats().get("allocated_bytes.current", 0))
 
 
 def _dev_i64(x, dev):
@@ -76,26 +84,128 @@ class MaterializedMultiLayerBuilder:
         self.pid, self.num_parts = int(pid), int(num_parts)
         self.gen = torch.Generator(device="cpu")
         self.gen.manual_seed(0)
+        self._stage = None                # pinned buffer for the tasks' roots
 
-    # ---- route plan of one layer list (prepare_sample.py:266-310) ------------------------------------------------
-    def _plan_async(self, layer_ids, d_n, status):
-        if self.rep_table is None or self.node_parts is None or self.num_parts <= 1:
-            return None
-        cap = max(layer_ids.numel() * max(self.num_parts - 1, 1), 1)
-        rt = self.rep_table
-        return ops.plan_route(layer_ids, self.node_parts, self.pid, rt.indptr, rt.indices, rt.locs, self.num_parts, cap,
-                              d_n=d_n, status=status)
+    def _roots(self, node_parts, ts_parts):
+        """(nodes, times, (lowest, highest time)) of a task on the GPU: host arrays go through one pinned buffer and one copy,
+        and their time range is read where they are."""
+        parts = [x.numpy() if torch.is_tensor(x) and not x.is_cuda else x for x in (*node_parts, *ts_parts)]
+        if not all(isinstance(x, np.ndarray) for x in parts):
+            f = lambda xs: torch.cat([_dev_i64(x, self.device) for x in xs])
+            return f(node_parts), f(ts_parts), None
+        n, total = sum(len(x) for x in parts[:len(node_parts)]), sum(len(x) for x in parts)
+        if self._stage is None or self._stage.numel() < total:
+            self._stage = torch.empty(max(2 * total, 1024), dtype=torch.int64).pin_memory()
+        st, at = self._stage.numpy(), 0
+        for x in parts:
+            st[at:at + len(x)] = x
+            at += len(x)
+        d = self._stage[:total].to(self.device, non_blocking=True)     # (the slot's end waits for the stream)
+        t = parts[len(node_parts)]
+        return d[:n], d[n:], (int(t.min()), int(t.max())) if len(t) else None
 
-    @staticmethod
-    def _plan_finish(p) -> Optional[CommPlan]:
-        if p is None:
-            return None
-        ranks, rows, locs, sizes, total = p
-        n = int(total.item())
-        if n == 0:
-            return None
-        return CommPlan(send_ranks=ranks[:n].cpu(), send_sizes=sizes.cpu(), send_indices=rows[:n].cpu(),
-                        send_remote_indices=locs[:n].cpu())
+    # ---- layers and route plans of one slot on the host (prepare_sample.py:266-310) -------------------------------
+    def _build(self, roots, root_ts, ts_range, fanouts, policy, inclusive, seed) -> List[dict]:
+        """Batch, then the plan of every layer list, all enqueued without a host round trip; one read-back of every size;
+        one copy of every array."""
+        g, L, P, hops = self.g, _C.lib(), self.num_parts, len(fanouts)
+        if ts_range is None:
+            ts_range = _root_range(g, root_ts)
+        planned = self.rep_table is not None and self.node_parts is not None and P > 1
+        nb = 2 + 2 * hops
+        meta = torch.empty(nb + ((hops + 1) * (P + 1) if planned else 0), dtype=torch.int64, device=self.device)
+        lo, hi = _graph_range(g, *ts_range)
+        db = _enqueue(g, roots, root_ts, fanouts, policy, lo, hi, inclusive, -1, seed, None, None, None, meta[:nb])
+        lists = []                                  # (address of the ids, capacity) of every layer list
+        n = c = t = roots.numel()
+        base = db._arena.data_ptr()
+        lists.append((base + 8 * db._plan.start[0], c))
+        for l, k in enumerate(fanouts):
+            t *= k
+            c += t
+            lists.append((base + 8 * db._plan.start[3 + 14 * l + 6], c))
+        plans = []
+        if planned:
+            caps = [max(c * max(P - 1, 1), 1) for _, c in lists]
+            room = torch.empty(3 * sum(caps), dtype=torch.int64, device=self.device)
+            rt, sp, mp, at = self.rep_table, _C.stream_ptr(), meta.data_ptr(), room.data_ptr()
+            ws = _C.WORKSPACE.get(max(L.sgl_plan_route_ws_bytes(c, cap) for (_, c), cap in zip(lists, caps)), self.device, sp)
+            for i, ((ids, c), cap) in enumerate(zip(lists, caps)):
+                m = mp + 8 * (nb + i * (P + 1))
+                _C.check(L.sgl_plan_route(ids, c, mp + 8 * (2 * i), self.node_parts.data_ptr(), self.node_parts.numel(), self.pid,
+                                          rt.indptr.data_ptr(), rt.indices.data_ptr(), rt.locs.data_ptr(), P, cap, at, at + 8 * cap,
+                                          at + 16 * cap, m, m + 8 * P, mp + 8 * (nb - 1), ws.data_ptr(), ws.numel(), sp))
+                plans.append((at, cap))
+                at += 24 * cap
+        host = _C.read_words(meta, meta.numel())    # the one synchronisation before the copy
+        bits = host[nb - 1] & 0xFFFFFFFF
+        if bits:
+            raise _C.SglError(f"build_batch: device status {bits} ({_C.decode_status(bits)})")
+        stopped = next((l for l in range(hops) if host[1 + 2 * l] == 0), None)
+        layers = None
+        if stopped is not None:                     # perhaps a hop without any edge, where the builder stops
+            layers = db._trim(host[:nb - 1])
+            if len(layers) == hops + 1 and layers[-1]["indptr"].numel() > 1:
+                layers = None
+        picks = []                                  # (address, count, bytes per value) in the order of the result
+        if layers is None:
+            starts = db._plan.start
+            sec = lambda i, count, size=8: picks.append((base + 8 * starts[i], count, size))
+            sec(0, host[0]); sec(1, host[0]); sec(2, n)
+            prev = host[0]
+            for l in range(hops):
+                e, nxt, b = host[1 + 2 * l], host[2 + 2 * l], 3 + 14 * l
+                ip, ix, ts, dt, ei = (5, 8, 2, 3, 4) if l == 0 else (9, 10, 11, 12, 13)
+                sec(b + ip, prev + 1); sec(b + ix, e); sec(b + ei, e); sec(b + ts, e); sec(b + dt, e, 4); sec(b + 6, nxt); sec(b + 7, nxt)
+                prev = nxt
+        sizes = [host[nb + i * (P + 1):nb + (i + 1) * (P + 1)] for i in range(len(plans))]
+        for (at, cap), s in zip(plans, sizes):
+            for j in range(3):
+                picks.append((at + 8 * j * cap, s[P], 8))
+        got = self._export(picks)
+        if layers is None:
+            names = ("indptr", "indices", "eid", "edge_ts", "edge_dt", "gids", "ts")
+            final = [dict(zip(("gids", "ts", "inv_map"), got[:3]))]
+            final += [dict(zip(names, got[3 + 7 * l:10 + 7 * l])) for l in range(hops)]
+            got = got[3 + 7 * hops:]
+        else:
+            final = [{k: v.cpu() for k, v in d.items()} for d in layers]
+        routes = []
+        for i in range(len(final)):
+            if not plans or sizes[i][P] == 0:
+                routes.append(None)
+            else:
+                routes.append(CommPlan(send_ranks=got[3 * i], send_sizes=torch.tensor(sizes[i][:P], dtype=torch.int64),
+                                       send_indices=got[3 * i + 1], send_remote_indices=got[3 * i + 2]))
+        if len(final) >= 2 and final[-1]["indptr"].numel() == 1:
+            routes[-1] = None                       # the reference stops at an empty layer with no plan for it
+        final[0]["comm_plan"] = routes
+        return final
+
+    def _export(self, picks):
+        """Host tensors of device arrays (address, count, bytes per value): views of one buffer per type, filled by one copy
+        each.  The buffers are pinned (a copy to fresh pageable memory takes several times as long) as long as not too
+        much is."""
+        import ctypes as C
+        n, at, offs = len(picks), 0, [0] * len(picks)
+        split = 0
+        for want in (8, 4):                         # 8-byte values first
+            for i, (_, count, size) in enumerate(picks):
+                if size == want:
+                    offs[i] = at
+                    at += (count * size + 15) & ~15
+            if want == 8:
+                split = at
+        total = at
+        pin = total <= _PINNED_MOST and _pinned_now() + total <= _PINNED_TOTAL
+        h = torch.empty(split // 8, dtype=torch.int64, pin_memory=pin)
+        f = torch.empty((total - split) // 4, dtype=torch.float32, pin_memory=pin)
+        d = torch.empty(max(total, 16) // 8, dtype=torch.int64, device=self.device)
+        src = (C.c_void_p * max(n, 1))(*[p[0] for p in picks])
+        size = (C.c_int64 * max(n, 1))(*[p[1] * p[2] for p in picks])
+        _C.check(_C.lib().sgl_export_arrays(n, src, size, (C.c_int64 * max(n, 1))(*offs), d.data_ptr(), h.data_ptr(), total, f.data_ptr(),
+                                            split, _C.stream_ptr()))
+        return [h[o // 8:o // 8 + count] if s == 8 else f[(o - split) // 4:(o - split) // 4 + count] for o, (_, count, s) in zip(offs, picks)]
 
     # ---- one slot ------------------------------------------------------------------------------------------------
     def build_aligned_batch(self, task_param, save_path, layer_configs, num_neg=1, global_dst_pool=None, cluster_ids=None,
@@ -105,14 +215,12 @@ class MaterializedMultiLayerBuilder:
         extra = {}
         if task_type == 'link':
             task_src, task_dst, task_ts, task_label, task_eid = task_nodes
-            l0_nodes = torch.cat([_dev_i64(task_src, dev), _dev_i64(task_dst, dev)])
-            t = _dev_i64(task_ts, dev)
-            l0_ts = torch.cat([t, t])
+            l0_nodes, l0_ts, ts_range = self._roots((task_src, task_dst), (task_ts, task_ts))
             extra = {"task_ts": task_ts, "task_src": task_src, "task_dst": task_dst, "task_label": task_label,
                      "task_eid": task_eid}
         elif task_type == 'node':
             task_node, task_ts, task_label = task_nodes
-            l0_nodes, l0_ts = _dev_i64(task_node, dev), _dev_i64(task_ts, dev)
+            l0_nodes, l0_ts, ts_range = self._roots((task_node,), (task_ts,))
             extra = {"task_node": task_node, "task_ts": task_ts, "task_label": task_label}
         elif task_type == 'neg':
             if num_neg <= 0 or global_dst_pool is None:
@@ -124,7 +232,7 @@ class MaterializedMultiLayerBuilder:
             pick = torch.randint(0, pool.numel(), (len(task_ts) * num_neg,), generator=self.gen)
             neg = pool[pick]
             l0_nodes = neg.to(dev)
-            l0_ts = _dev_i64(task_ts, dev).repeat_interleave(num_neg)
+            l0_ts, ts_range = _dev_i64(task_ts, dev).repeat_interleave(num_neg), None
             extra = {"task_nodes": neg, "task_ts": task_ts, "task_label": 'neg_set'}
         else:
             raise ValueError(f"Unsupported task type: {task_type}")
@@ -143,26 +251,15 @@ class MaterializedMultiLayerBuilder:
         policy = kinds.pop() if kinds else 'recent'
         fanouts = [int(c['fanout']) for c in layer_configs['layer']]
 
-        status = ops.StatusWord(dev)
-        db = build_batch_async(self.g, l0_nodes, l0_ts, fanouts, policy, equal_root_time=bool(end_offset),
-                               seed=0 if seed is None else int(seed), status=status)
-        # plans of every layer list, enqueued behind the builder without a host round trip
-        plans = [self._plan_async(db.layers[0]["gids"], db.counts[0], status)]
-        for l in range(len(fanouts)):
-            plans.append(self._plan_async(db.layers[l + 1]["gids"], db.counts[2 + 2 * l], status))
-        layers = db.finish()                      # the one synchronisation of the slot
-        routes = [self._plan_finish(p) for p in plans[:len(layers)]]
-        if len(layers) >= 2 and layers[-1]["indptr"].numel() == 1:
-            routes[-1] = None                     # the reference stops at an empty layer with no plan for it
+        seed = 0 if seed is None else int(seed)
+        final = self._build(l0_nodes, l0_ts, ts_range, fanouts, policy, bool(end_offset), seed)
 
         def host(x):
             if isinstance(x, np.ndarray):
                 return torch.from_numpy(x)
             return x.cpu() if torch.is_tensor(x) else x
-        final = [{k: host(v) for k, v in d.items()} for d in layers]
         final[0]["num_neg"] = num_neg
         final[0].update({k: host(v) for k, v in extra.items()})
-        final[0]['comm_plan'] = routes
         if save_path is not None:
             torch.save(final, save_path)
         return final

@@ -1,4 +1,4 @@
-// Radix sort of lists beyond the mini-batch sort: least significant digit first, 8 bits a pass, ONE kernel per pass (the
+// Radix sort of lists beyond the mini-batch sort: least significant digit first, up to 9 bits a pass, ONE kernel per pass (the
 // "onesweep" scheme of Adinets and Merrill, with Merrill and Garland's decoupled look-back):
 //   1. lsd_hist_kernel   one read of the keys: digit totals of every pass
 //   2. lsd_scan_kernel   start of every digit, all passes
@@ -8,6 +8,8 @@
 // HBM traffic per pass and key: 16 B + twice the payload (a histogram kernel, a scan kernel and a scatter kernel per pass read
 // the keys once more and took 1.0 ms per pass for 50 M keys).
 #pragma once
+#include <type_traits>
+
 #include "launch.cuh"
 #include "scan.cuh"
 #include "sort.cuh"
@@ -16,44 +18,59 @@
 namespace sgl {
 namespace {
 
-constexpr int kBits = 8;
+constexpr int kBits = 9;
 constexpr int kRadix = 1 << kBits;
 constexpr int kMaxPasses = 8;
+// Measured (50 M and 4.2 M keys of 44 bits, 256 - 1,024 threads, 8 - 20 keys each, 8 and 9 bits a pass): what fills the LSU data
+// pipe with two CTAs per SM is the best of them; 9 bits take five passes instead of six.
 constexpr int kLsdThreads = 512;
+constexpr int kLsdCtas = 2;
 constexpr int kLsdWarps = kLsdThreads / 32;
-template <class V>
-constexpr int kLsdItems = sizeof(V) == 4 ? 12 : 10;   // keys per thread: two CTAs per SM either way
-template <class V>
-constexpr int kLsdTile = kLsdThreads * kLsdItems<V>;
+constexpr int kLsdItems = 14;            // keys per thread
+constexpr int kLsdTile = kLsdThreads * kLsdItems;
+constexpr int kLookWide = 16;            // tiles a look-back step reads: with 4 the chain of steps was slower than the tiles
 constexpr int kHistThreads = 512;
 
-__device__ __forceinline__ uint32_t digit_of(uint64_t key, int shift) { return (uint32_t)(key >> shift) & (kRadix - 1u); }
+// a pass: `bits` <= kBits bits from `shift` on
+struct Digit {
+  int shift, bits;
+  __device__ __forceinline__ uint32_t of(uint64_t key) const { return (uint32_t)(key >> shift) & ((1u << bits) - 1u); }
+};
 
 // Digit totals of passes shift0, shift0 + 8, ...: one shared-memory counter table per pass.  A warp whose keys all carry the
 // same digit (high digits of a hub, ordered input) adds once.
 template <class Items>
 __global__ void __launch_bounds__(kHistThreads)
-lsd_hist_kernel(Items items, int shift0, int passes, unsigned long long* __restrict__ hist) {
+lsd_hist_kernel(Items items, Digit first, int passes, unsigned long long* __restrict__ hist) {
   __shared__ uint32_t s_hist[kMaxPasses * kRadix];
   const int64_t n = items.begin();
   for (int j = threadIdx.x; j < passes * kRadix; j += kHistThreads) s_hist[j] = 0;
   __syncthreads();
-  const int64_t stride = (int64_t)gridDim.x * kHistThreads;
+  constexpr int kAhead = 4;              // keys in flight per thread
+  const int64_t stride = (int64_t)gridDim.x * kHistThreads * kAhead;
   const int lane = threadIdx.x & 31;
-  for (int64_t i0 = (int64_t)blockIdx.x * kHistThreads; i0 < n; i0 += stride) {
-    const int64_t i = i0 + threadIdx.x;
-    const bool valid = i < n;
-    const uint64_t key = valid ? items.key(i) : 0;
-    if (valid) items.prepare(i);
-    const unsigned act = __ballot_sync(0xffffffffu, valid);
-    if (act == 0) continue;
-    for (int p = 0; p < passes; ++p) {
-      const uint32_t d = digit_of(key, shift0 + p * kBits);
-      const uint32_t d0 = __shfl_sync(0xffffffffu, d, 0);
-      if (__all_sync(0xffffffffu, !valid || d == d0)) {
-        if (lane == 0) atomicAdd(&s_hist[p * kRadix + d0], (uint32_t)__popc(act));
-      } else if (valid) {
-        atomicAdd(&s_hist[p * kRadix + d], 1u);
+  for (int64_t i0 = (int64_t)blockIdx.x * kHistThreads * kAhead; i0 < n; i0 += stride) {
+    uint64_t key[kAhead];
+#pragma unroll
+    for (int u = 0; u < kAhead; ++u) {
+      const int64_t i = i0 + u * kHistThreads + threadIdx.x;
+      key[u] = i < n ? items.key(i) : 0;
+    }
+#pragma unroll
+    for (int u = 0; u < kAhead; ++u) {
+      const int64_t i = i0 + u * kHistThreads + threadIdx.x;
+      const bool valid = i < n;
+      if (valid) items.prepare(i);
+      const unsigned act = __ballot_sync(0xffffffffu, valid);
+      if (act == 0) continue;
+      for (int p = 0; p < passes; ++p) {
+        const uint32_t d = Digit{first.shift + p * first.bits, first.bits}.of(key[u]);
+        const uint32_t d0 = __shfl_sync(0xffffffffu, d, 0);
+        if (__all_sync(0xffffffffu, !valid || d == d0)) {
+          if (lane == 0) atomicAdd(&s_hist[p * kRadix + d0], (uint32_t)__popc(act));
+        } else if (valid) {
+          atomicAdd(&s_hist[p * kRadix + d], 1u);
+        }
       }
     }
   }
@@ -62,7 +79,7 @@ lsd_hist_kernel(Items items, int shift0, int passes, unsigned long long* __restr
     if (s_hist[j]) atomicAdd(&hist[j], (unsigned long long)s_hist[j]);
 }
 
-// totals -> starts, one CTA of 256 threads per pass
+// totals -> starts, one CTA per pass
 static __global__ void __launch_bounds__(kRadix) lsd_scan_kernel(unsigned long long* __restrict__ hist) {
   unsigned long long* h = hist + blockIdx.x * kRadix;
   const unsigned long long v = h[threadIdx.x];
@@ -75,15 +92,13 @@ constexpr uint64_t kOwn = 1ull << 62, kAll = 2ull << 62, kValue = (1ull << 56) -
 __device__ __forceinline__ uint64_t pass_tag(int pass) { return (uint64_t)(pass + 1) << 56; }
 constexpr unsigned long long kLookLimitNs = 2000000000ull;
 
-template <class V>
 struct LsdSmem {
   union {
-    uint64_t keys[kLsdTile<V>];            // the tile in digit order
+    uint64_t keys[kLsdTile];               // the tile in digit order, and after that its payload
     uint32_t mask[kLsdWarps][kRadix];      // before that: lanes of the warp's current round that hold the digit
   };
-  V vals[kLsdTile<V>];
   uint32_t cnt[kLsdWarps][kRadix];         // keys of the digit in the warp so far, then where the warp's start in the tile
-  int64_t out[kRadix];                     // global position of the tile's digit run minus its position in the tile
+  uint32_t out[kRadix];                    // global position of the tile's digit run minus its position in the tile (mod 2^32)
   int ticket;
 };
 
@@ -100,6 +115,15 @@ struct ArrayItems {
   __device__ __forceinline__ void prepare(int64_t) const {}
 };
 
+// where a pass writes them: the arrays of the next one, or (last pass, optionally) what the caller makes of sorted items
+template <class V>
+struct ArrayOut {
+  uint64_t* keys;
+  V* vals;
+  __device__ __forceinline__ void key(uint32_t g, uint64_t k) const { keys[g] = k; }
+  __device__ __forceinline__ void val(uint32_t g, V v) const { vals[g] = v; }
+};
+
 // a Source (see tilesort.cuh) with the position as payload
 template <class Source>
 struct SourceItems {
@@ -110,14 +134,14 @@ struct SourceItems {
   __device__ __forceinline__ void prepare(int64_t i) const { src.prepare(i); }
 };
 
-template <class V, class Items>
-__global__ void __launch_bounds__(kLsdThreads, 2)
-lsd_pass_kernel(Items items, int shift, int pass,
+template <class V, class Items, class Out>
+__global__ void __launch_bounds__(kLsdThreads, kLsdCtas)
+lsd_pass_kernel(Items items, Digit digit, int pass,
                 const unsigned long long* __restrict__ starts, unsigned int* __restrict__ ticket, uint64_t* __restrict__ state,
-                uint64_t* __restrict__ out_keys, V* __restrict__ out_vals, unsigned int* gave_up, int32_t* d_status) {
+                Out out, unsigned int* gave_up, int32_t* d_status) {
   extern __shared__ __align__(16) unsigned char smem[];
-  LsdSmem<V>& sm = *(LsdSmem<V>*)smem;
-  constexpr int kItems = kLsdItems<V>, kTile = kLsdTile<V>;
+  LsdSmem& sm = *(LsdSmem*)smem;
+  constexpr int kItems = kLsdItems, kTile = kLsdTile;
   const int64_t n = items.begin();
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   if (tid == 0) sm.ticket = (int)atomicAdd(ticket, 1u);
@@ -133,16 +157,10 @@ lsd_pass_kernel(Items items, int shift, int pass,
   // a warp owns consecutive keys of the tile, 32 at a time: (warp, round, lane) order = key order
   const int first = warp * (kItems * 32) + lane;
   uint64_t k[kItems];
-  V v[kItems];
 #pragma unroll
   for (int c = 0; c < kItems; ++c) {
     const int j = first + c * 32;
     k[c] = j < tile_n ? items.key(tile_base + j) : ~0ull;
-  }
-#pragma unroll
-  for (int c = 0; c < kItems; ++c) {
-    const int j = first + c * 32;
-    v[c] = j < tile_n ? items.val(tile_base + j) : (V)0;
   }
   // stable rank inside the warp: the lanes of a round that share a digit find each other through one word per digit
   uint16_t rank[kItems];
@@ -151,10 +169,11 @@ lsd_pass_kernel(Items items, int shift, int pass,
 #pragma unroll
   for (int c = 0; c < kItems; ++c) {
     const bool valid = first + c * 32 < tile_n;
-    const uint32_t d = digit_of(k[c], shift);
-    if (valid) atomicOr(&mask[d], 1u << lane);
+    const uint32_t d = digit.of(k[c]);
+    if (valid) atomicOr(&mask[d], 1u << lane);      // (ballots per digit bit and match_any were slower)
     __syncwarp();
-    const uint32_t peers = valid ? mask[d] : 0u, before = valid ? cnt[d] : 0u;
+    const uint32_t peers = valid ? mask[d] : 0u;
+    const uint32_t before = valid ? cnt[d] : 0u;
     __syncwarp();
     if (valid && (peers & below) == 0) {   // the lowest lane of the digit
       mask[d] = 0;
@@ -184,9 +203,8 @@ lsd_pass_kernel(Items items, int shift, int pass,
 #pragma unroll
   for (int c = 0; c < kItems; ++c) {
     if (first + c * 32 < tile_n) {
-      const uint32_t at = cnt[digit_of(k[c], shift)] + rank[c];
-      sm.keys[at] = k[c];
-      sm.vals[at] = v[c];
+      rank[c] += (uint16_t)cnt[digit.of(k[c])];      // place in the tile
+      sm.keys[rank[c]] = k[c];
     }
   }
   if (tid < kRadix) {
@@ -197,12 +215,12 @@ lsd_pass_kernel(Items items, int shift, int pass,
       const volatile uint64_t* st = state + tid;
       unsigned long long t0 = 0;
       for (int t = tile - 1; t >= 0;) {
-        uint64_t w[4];
+        uint64_t w[kLookWide];
 #pragma unroll
-        for (int u = 0; u < 4; ++u) w[u] = t - u >= 0 ? st[(size_t)(t - u) * kRadix] : 0;
+        for (int u = 0; u < kLookWide; ++u) w[u] = t - u >= 0 ? st[(size_t)(t - u) * kRadix] : 0;
         bool done = false, stalled = false;
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
+        for (int u = 0; u < kLookWide; ++u) {
           if (done || stalled || t < 0) continue;
           if ((w[u] & (0x3full << 56)) != tag) {
             stalled = true;
@@ -226,18 +244,39 @@ lsd_pass_kernel(Items items, int shift, int pass,
       }
       *(volatile uint64_t*)&state[(size_t)tile * kRadix + tid] = kAll | tag | (sum + total);
     }
-    sm.out[tid] = (int64_t)(starts[tid] + sum) - (int64_t)start;
+    sm.out[tid] = (uint32_t)(starts[tid] + sum) - start;
   }
   __syncthreads();
   // consecutive threads take consecutive tile positions, i.e. runs of one digit -> consecutive addresses
-  for (int j = tid; j < tile_n; j += kLsdThreads) {
-    const uint64_t key = sm.keys[j];
-    const int64_t g = sm.out[digit_of(key, shift)] + j;
-    if (g >= 0 && g < n) {                 // (always, unless a look-back gave up)
-      out_keys[g] = key;
-      out_vals[g] = sm.vals[j];
+  constexpr uint32_t kNone = ~0u;
+  uint32_t g[kItems];
+#pragma unroll
+  for (int c = 0; c < kItems; ++c) {
+    const int j = c * kLsdThreads + tid;
+    g[c] = kNone;
+    if (j < tile_n) {
+      const uint64_t key = sm.keys[j];
+      g[c] = sm.out[digit.of(key)] + j;
+      if (g[c] >= n) g[c] = kNone;       // (only where a look-back gave up)
+      if (g[c] != kNone) out.key(g[c], key);
     }
   }
+  // the payload follows through the same shared memory (loaded late: keys and payload do not fit the registers)
+  V v[kItems];
+#pragma unroll
+  for (int c = 0; c < kItems; ++c) {
+    const int j = first + c * 32;
+    v[c] = j < tile_n ? items.val(tile_base + j) : (V)0;
+  }
+  __syncthreads();
+  V* vals = (V*)sm.keys;
+#pragma unroll
+  for (int c = 0; c < kItems; ++c)
+    if (first + c * 32 < tile_n) vals[rank[c]] = v[c];
+  __syncthreads();
+#pragma unroll
+  for (int c = 0; c < kItems; ++c)
+    if (g[c] != kNone) out.val(g[c], vals[c * kLsdThreads + tid]);
 }
 
 // ---- delivery of a sorted list to a Sink (see tilesort.cuh) -------------------------------------------------------------
@@ -372,46 +411,49 @@ lsd_deliver_kernel(Sink sink, const uint64_t* __restrict__ keys, const uint32_t*
 template <class Source>
 __global__ void source_count_kernel(Source src, int64_t* d_count) { *d_count = src.begin(); }
 
-template <class V>
-inline int64_t lsd_tiles(int64_t n) { return (n + kLsdTile<V> - 1) / kLsdTile<V>; }
+inline int lsd_passes(int first_bit, int num_bits) { return num_bits <= first_bit + kBits ? 1 : (num_bits - first_bit + kBits - 1) / kBits; }
+inline int64_t lsd_tiles(int64_t n) { return (n + kLsdTile - 1) / kLsdTile; }
 
-template <class V>
 inline size_t lsd_ws_bytes(int64_t n) {
-  return align_up((kMaxPasses * kRadix + kMaxPasses) * 8) + align_up((size_t)lsd_tiles<V>(n < 1 ? 1 : n) * kRadix * 8);
+  return align_up((kMaxPasses * kRadix + kMaxPasses) * 8) + align_up((size_t)lsd_tiles(n < 1 ? 1 : n) * kRadix * 8);
 }
 
 // Sorts on key bits [first_bit, num_bits), at least one pass; the first pass reads from `items`, writes to (k1, v1), the next to
-// (k0, v0) and so on; *in_first says whether the result ends in (k1, v1).  **gave_up on the device: a look-back ran into its
-// time limit, the result is not to be used as positions.
-template <class V, class Items>
+// (k0, v0) and so on; *in_first says whether the result ends in (k1, v1).  With a `last` of another type than ArrayOut the last
+// pass writes there instead and its arrays stay free.  **gave_up on the device: a look-back ran into its time limit, the result
+// is not to be used as positions.
+template <class V, class Items, class Last>
 int lsd_sort(const Items& items, uint64_t* k1, V* v1, uint64_t* k0, V* v0, int64_t n, const int64_t* d_n, int first_bit, int num_bits,
-             bool* in_first, unsigned int** gave_up, WsCarver& c, int32_t* d_status, cudaStream_t stream) {
-  int passes = (num_bits - first_bit + kBits - 1) / kBits;
-  if (passes < 1) passes = 1;
-  const int64_t tiles = lsd_tiles<V>(n);
+             const Last& last, bool* in_first, unsigned int** gave_up, WsCarver& c, int32_t* d_status, cudaStream_t stream) {
+  using Array = ArrayOut<V>;
+  constexpr bool kArray = std::is_same<Last, Array>::value;
+  const int passes = lsd_passes(first_bit, num_bits);
+  const int bits = num_bits > first_bit ? (num_bits - first_bit + passes - 1) / passes : 1;     // an even share each
+  const int64_t tiles = lsd_tiles(n);
   unsigned long long* hist = c.take<unsigned long long>(kMaxPasses * kRadix + kMaxPasses);
   unsigned int* tickets = (unsigned int*)(hist + kMaxPasses * kRadix);
   *gave_up = tickets + kMaxPasses;
   uint64_t* state = c.take<uint64_t>((size_t)tiles * kRadix);
   SGL_REQUIRE(c.ok(), SGL_ERR_WORKSPACE, "radix sort: workspace too small for %lld keys", (long long)n);
-  static std::atomic<uint64_t> done0{0}, done1{0};
-  SGL_CUDA_CHECK(allow_smem((const void*)lsd_pass_kernel<V, Items>, done0, sizeof(LsdSmem<V>)));
-  SGL_CUDA_CHECK(allow_smem((const void*)lsd_pass_kernel<V, ArrayItems<V>>, done1, sizeof(LsdSmem<V>)));
   SGL_CHECK_RC(zero_async(hist, (kMaxPasses * kRadix + kMaxPasses) * 8, stream));
   SGL_CHECK_RC(zero_async(state, (size_t)tiles * kRadix * 8, stream));
-  SGL_CHECK_RC(launch(lsd_hist_kernel<Items>, stream_grid(n, kHistThreads * 16, 4), kHistThreads, 0, stream, items, first_bit, passes, hist));
+  SGL_CHECK_RC(launch(lsd_hist_kernel<Items>, stream_grid(n, kHistThreads * 16, 4), kHistThreads, 0, stream, items, Digit{first_bit, bits},
+                      passes, hist));
   SGL_CHECK_RC(launch(lsd_scan_kernel, passes, kRadix, 0, stream, hist));
   for (int p = 0; p < passes; ++p) {
-    uint64_t *kout = p & 1 ? k0 : k1, *kin = p & 1 ? k1 : k0;
-    V *vout = p & 1 ? v0 : v1, *vin = p & 1 ? v1 : v0;
-    const int shift = first_bit + p * kBits;
-    if (p == 0)
-      SGL_CHECK_RC(launch(lsd_pass_kernel<V, Items>, (unsigned)tiles, kLsdThreads, sizeof(LsdSmem<V>), stream, items, shift, p, hist, tickets,
-                          state, kout, vout, *gave_up, d_status));
-    else
-      SGL_CHECK_RC(launch(lsd_pass_kernel<V, ArrayItems<V>>, (unsigned)tiles, kLsdThreads, sizeof(LsdSmem<V>), stream,
-                          ArrayItems<V>{kin, vin, n, d_n}, shift, p, hist + p * kRadix, tickets + p, state, kout, vout, *gave_up,
-                          d_status));
+    const Array out{p & 1 ? k0 : k1, p & 1 ? v0 : v1};
+    const ArrayItems<V> in{p & 1 ? k1 : k0, p & 1 ? v1 : v0, n, d_n};
+    auto pass = [&](const auto& from, const auto& to) -> int {
+      using From = std::decay_t<decltype(from)>;
+      using To = std::decay_t<decltype(to)>;
+      static std::atomic<uint64_t> done{0};
+      SGL_CUDA_CHECK(allow_smem((const void*)lsd_pass_kernel<V, From, To>, done, sizeof(LsdSmem)));
+      return launch(lsd_pass_kernel<V, From, To>, (unsigned)tiles, kLsdThreads, sizeof(LsdSmem), stream, from, Digit{first_bit + p * bits, bits},
+                    p, hist + p * kRadix, tickets + p, state, to, *gave_up, d_status);
+    };
+    const bool to_last = !kArray && p == passes - 1;
+    if (p == 0) SGL_CHECK_RC(to_last ? pass(items, last) : pass(items, out));
+    else SGL_CHECK_RC(to_last ? pass(in, last) : pass(in, out));
   }
   *in_first = passes & 1;
   return SGL_OK;
@@ -420,7 +462,7 @@ int lsd_sort(const Items& items, uint64_t* k1, V* v1, uint64_t* k0, V* v0, int64
 inline size_t list_ws_bytes(int64_t n) {
   if (n < 1) n = 1;
   if (n <= tilesort::kMaxItems) return tilesort::ws_bytes(n);
-  return 2 * align_up((size_t)n * 8) + 2 * align_up((size_t)n * 4) + lsd_ws_bytes<uint32_t>(n) + align_up(8) +
+  return 2 * align_up((size_t)n * 8) + 2 * align_up((size_t)n * 4) + lsd_ws_bytes(n) + align_up(8) +
          align_up(((size_t)((n + kDeliverTile - 1) / kDeliverTile) + 2) * 8);
 }
 
@@ -446,8 +488,8 @@ int sort_list(const Source& src, const Sink& sink, int64_t n_cap, int key_bits, 
   SGL_CHECK_RC(zero_async(ctl, (size_t)(tiles + 2) * 8, stream));
   bool in_first;
   unsigned int* gave_up;
-  SGL_CHECK_RC((lsd_sort<uint32_t, SourceItems<Source>>(SourceItems<Source>{src}, k1, v1, k0, v0, n_cap, count, 0, key_bits, &in_first,
-                                                        &gave_up, c, d_status, stream)));
+  SGL_CHECK_RC((lsd_sort<uint32_t, SourceItems<Source>>(SourceItems<Source>{src}, k1, v1, k0, v0, n_cap, count, 0, key_bits,
+                                                        ArrayOut<uint32_t>{}, &in_first, &gave_up, c, d_status, stream)));
   return launch(lsd_deliver_kernel<Sink>, (unsigned)tiles, kDeliverThreads, 0, stream, sink, in_first ? k1 : k0, in_first ? v1 : v0, n_cap,
                 count, ctl, (uint64_t*)(ctl + 2), gave_up, d_status);
 }

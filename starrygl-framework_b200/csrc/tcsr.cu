@@ -9,8 +9,8 @@
 //                                          8-byte reads per edge took 2.6 of the 8.1 ms of a 50 M edge build.  Input in time
 //                                          order, as event streams are, is sorted on the node bits alone.
 //        node and timestamp bits above 64  by timestamp, then stably by node
-//   3. tcsr_emit_*_kernel reads the sorted keys sequentially, writes the edges and the row pointer from the row boundaries (no
-//                         atomics, no separate prefix sum)
+//   3. the last pass writes the edges to their places, tcsr_rows_kernel the row pointer from the row boundaries (no atomics, no
+//      prefix sum); with positions as payload tcsr_emit_gather_kernel does both
 //
 // 50 M edges, 1 M nodes in no particular order: bound by the radix passes' traffic, 264 B per edge.
 #include "chain.cuh"
@@ -162,22 +162,31 @@ struct EdgePositions {                // position as payload
   __device__ __forceinline__ void prepare(int64_t) const {}
 };
 
-__global__ void __launch_bounds__(256)
-tcsr_emit_pairs_kernel(const unsigned int* gave_up, const uint64_t* __restrict__ keys, const uint64_t* __restrict__ vals, EdgeKey k, int64_t m, int64_t num_nodes,
-                       int64_t* __restrict__ indptr, int64_t* __restrict__ out_nbr, int64_t* __restrict__ out_ts,
-                       int64_t* __restrict__ out_eid) {
-  if (*gave_up) return;
-  const int64_t stride = (int64_t)gridDim.x * 256;
-#pragma unroll 2
-  for (int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x; i < m; i += stride) {
-    const uint64_t key = keys[i], v = vals[i];
-    out_nbr[i] = (int64_t)(uint32_t)v;
-    out_eid[i] = (int64_t)(v >> 32);
-    out_ts[i] = k.time(key);
-    start_rows(indptr, i > 0 ? k.node(keys[i - 1]) : -1, k.node(key), i);
-    if (i == m - 1)
-      for (int64_t r = k.node(key) + 1; r <= num_nodes; ++r) indptr[r] = m;
+// The last radix pass writes the edges where they belong; the node of every edge stays for the row pointer.
+struct EdgeOut {
+  EdgeKey k;
+  uint32_t* node;
+  int64_t *nbr, *ts, *eid;
+  __device__ __forceinline__ void key(uint32_t g, uint64_t key) const {
+    node[g] = (uint32_t)k.node(key);
+    ts[g] = k.time(key);
   }
+  __device__ __forceinline__ void val(uint32_t g, uint64_t v) const {
+    nbr[g] = (int64_t)(uint32_t)v;
+    eid[g] = (int64_t)(v >> 32);
+  }
+};
+
+__global__ void __launch_bounds__(256)
+tcsr_rows_kernel(const unsigned int* gave_up, const uint32_t* __restrict__ node, int64_t m, int64_t num_nodes, int64_t* __restrict__ indptr) {
+  const int64_t stride = (int64_t)gridDim.x * 256;
+  if (*gave_up) {                          // (a look-back ran into its time limit: no rows rather than wrong ones)
+    for (int64_t v = (int64_t)blockIdx.x * 256 + threadIdx.x; v <= num_nodes; v += stride) indptr[v] = 0;
+    return;
+  }
+#pragma unroll 4
+  for (int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x; i <= m; i += stride)
+    start_rows(indptr, i > 0 ? (int64_t)node[i - 1] : -1, i < m ? (int64_t)node[i] : num_nodes, i);
 }
 
 // combined == 0: the keys are node ids and the timestamps are gathered too
@@ -222,7 +231,7 @@ using namespace sgl;
 extern "C" size_t sgl_tcsr_build_ws_bytes(int64_t num_nodes, int64_t m) {
   (void)num_nodes;
   if (m < 1) m = 1;
-  const size_t pairs = 4 * align_up((size_t)m * 8) + lsd_ws_bytes<uint64_t>(m);
+  const size_t pairs = 4 * align_up((size_t)m * 8) + lsd_ws_bytes(m);
   const size_t rounds = 2 * align_up((size_t)m * 8) + 2 * align_up((size_t)m * 4) + radix_sort_ws_bytes(m);
   size_t most = m <= tilesort::kMaxItems ? list_ws_bytes(m) : pairs;
   most = most > rounds ? most : rounds;
@@ -296,17 +305,18 @@ extern "C" int sgl_tcsr_build_fenced(int64_t num_nodes, int64_t m, const int64_t
     const int first_bit = flags & kUnordered ? 0 : (ts_bits < 56 ? ts_bits : 56);   // in time order: only the node bits are left
     bool in_first;
     unsigned int* gave_up;
-    if (!(flags & kWideIds) && out_perm == nullptr) {
+    if (!(flags & kWideIds) && out_perm == nullptr && num_nodes <= ((int64_t)1 << 32)) {
       uint64_t *k1 = c.take<uint64_t>(m), *k0 = c.take<uint64_t>(m), *v1 = c.take<uint64_t>(m), *v0 = c.take<uint64_t>(m);
-      SGL_CHECK_RC((lsd_sort<uint64_t, EdgePairs>(EdgePairs{k, nbr, eid, m}, k1, v1, k0, v0, m, nullptr, first_bit, ts_bits + id_bits,
+      uint32_t* node = (uint32_t*)(lsd_passes(first_bit, ts_bits + id_bits) & 1 ? k1 : k0);      // the last pass's own array
+      const EdgeOut out{k, node, out_nbr, out_ts, out_eid};
+      SGL_CHECK_RC((lsd_sort<uint64_t, EdgePairs>(EdgePairs{k, nbr, eid, m}, k1, v1, k0, v0, m, nullptr, first_bit, ts_bits + id_bits, out,
                                                   &in_first, &gave_up, c, nullptr, stream)));
-      SGL_CHECK_RC(launch(tcsr_emit_pairs_kernel, grid, 256, 0, stream, gave_up, in_first ? k1 : k0, in_first ? v1 : v0, k, m, num_nodes, indptr,
-                          out_nbr, out_ts, out_eid));
+      SGL_CHECK_RC(launch(tcsr_rows_kernel, grid, 256, 0, stream, gave_up, node, m, num_nodes, indptr));
     } else {
       uint64_t *k1 = c.take<uint64_t>(m), *k0 = c.take<uint64_t>(m);
       uint32_t *v1 = c.take<uint32_t>(m), *v0 = c.take<uint32_t>(m);
       SGL_CHECK_RC((lsd_sort<uint32_t, EdgePositions>(EdgePositions{k, m}, k1, v1, k0, v0, m, nullptr, first_bit, ts_bits + id_bits,
-                                                      &in_first, &gave_up, c, nullptr, stream)));
+                                                      ArrayOut<uint32_t>{}, &in_first, &gave_up, c, nullptr, stream)));
       SGL_CHECK_RC(launch(tcsr_emit_gather_kernel, grid, 256, 0, stream, in_first ? k1 : k0, in_first ? v1 : v0, 1, k, nbr, eid, m, num_nodes,
                           indptr, out_nbr, out_ts, out_eid, out_perm));
     }

@@ -15,6 +15,7 @@
 // word (used when the caller has none of its own).
 
 #include "chain.cuh"
+#include "rowcsc.cuh"
 #include "sampler.cuh"
 #include "sort.cuh"
 #include "tilesort.cuh"
@@ -79,12 +80,27 @@ size_t list_ws(int64_t n, const int32_t* fanouts, int hops) {
   return align_up(most);
 }
 
+// Edges of a hop go to their rows along the order of the layer list (rowcsc.cuh), but for lists that one CTA sorts.
+inline bool by_rows(int64_t edges) { return edges > tilesort::kSingleMax; }
+
+// orders of the layer lists that a CSC is made along: kept per hop, the next list is merged while it is read
+size_t order_ws(int64_t n, const int32_t* fanouts, int hops) {
+  size_t sum = 0;
+  int64_t t = n, c = n;
+  for (int l = 0; l + 1 < hops; ++l) {
+    t *= fanouts[l];
+    c += t;
+    if (by_rows(t * fanouts[l + 1])) sum += RowOrder::bytes(c);
+  }
+  return sum;
+}
+
 size_t csc_ws(int64_t n, const int32_t* fanouts, int hops) {
   size_t most = 0;
   int64_t t = n, c = n;
   for (int l = 0; l < hops; ++l) {
     const int64_t e = t * fanouts[l];
-    const size_t b = l > 0 ? sgl_build_csc_ws_bytes(e, c) : 0;
+    const size_t b = l > 0 ? (by_rows(e) ? build_csc_rows_ws_bytes(e, c) : sgl_build_csc_ws_bytes(e, c)) : 0;
     most = most > b ? most : b;
     t = e;
     c += e;
@@ -110,7 +126,8 @@ extern "C" int64_t sgl_build_batch_layout(int64_t n_roots, const int32_t* fanout
 }
 
 extern "C" size_t sgl_build_batch_ws_bytes(int64_t n_roots, const int32_t* fanouts, int n_hops) {
-  return sample_ws(n_roots, fanouts, n_hops) + list_ws(n_roots, fanouts, n_hops) + csc_ws(n_roots, fanouts, n_hops);
+  return sample_ws(n_roots, fanouts, n_hops) + list_ws(n_roots, fanouts, n_hops) + csc_ws(n_roots, fanouts, n_hops) +
+         order_ws(n_roots, fanouts, n_hops);
 }
 
 extern "C" int sgl_build_batch(const int64_t* indptr, const int64_t* nbr, const int64_t* ts, const int64_t* eid, const int64_t* fence,
@@ -139,6 +156,8 @@ extern "C" int sgl_build_batch(const int64_t* indptr, const int64_t* nbr, const 
   batch_sections(n_roots, fanouts, n_hops, size);
   const size_t swb = sample_ws(n_roots, fanouts, n_hops), lwb = list_ws(n_roots, fanouts, n_hops), cwb = csc_ws(n_roots, fanouts, n_hops);
   void *sws = ws, *lws = (char*)ws + swb, *cws = (char*)lws + lwb;
+  char* ows = (char*)cws + cwb;
+  RowOrder order_of{};                   // of the layer list merged last, where the next CSC goes along it
   int64_t* p = arena;
   int sec = 0;
   auto take = [&]() {
@@ -193,13 +212,21 @@ extern "C" int sgl_build_batch(const int64_t* indptr, const int64_t* nbr, const 
     }
     if (l > 0) {
       if (forked) SGL_CHECK_RC(order.wait(kRelabelled, side));
-      rc = sgl_build_csc(nullptr, h.dst, last_col, h.ts, h.dt, h.eid, e, d_edges, c, d_cur, bits_for((uint64_t)c), ts_bits, ts_base,
-                         h.indptr, h.indices, h.cts, h.cdt, h.ceid, 0, d_status, cws, cwb, side);
+      rc = by_rows(e) ? build_csc_rows(order_of, c, h.offs, fanouts[l], h.dst, last_col, h.ts, h.dt, h.eid, e, d_edges, c, d_cur,
+                                       bits_for((uint64_t)c), ts_bits, ts_base, h.indptr, h.indices, h.cts, h.cdt, h.ceid, d_status, cws, cwb,
+                                       side)
+                      : sgl_build_csc(nullptr, h.dst, last_col, h.ts, h.dt, h.eid, e, d_edges, c, d_cur, bits_for((uint64_t)c), ts_bits,
+                                      ts_base, h.indptr, h.indices, h.cts, h.cdt, h.ceid, 0, d_status, cws, cwb, side);
       if (rc) return rc;
       if (forked) SGL_CHECK_RC(order.mark(kCsc, side));
     }
-    rc = sgl_unique_pairs(cur_id, cur_ts, c, d_cur, h.nbr, h.ts, e, d_edges, id_bits, ts_bits, ts_base, h.gids, h.gts, nullptr, h.col,
-                          d_next, d_status, lws, lwb, stream);
+    order_of = RowOrder{};
+    if (l + 1 < n_hops && by_rows(e * fanouts[l + 1])) {
+      order_of = RowOrder::carve(ows, c + e);
+      ows += RowOrder::bytes(c + e);
+    }
+    rc = unique_pairs(cur_id, cur_ts, c, d_cur, h.nbr, h.ts, e, d_edges, id_bits, ts_bits, ts_base, h.gids, h.gts, nullptr, h.col, d_next,
+                      order_of, d_status, lws, lwb, stream);
     if (rc) return rc;
     if (forked && l + 1 < n_hops) SGL_CHECK_RC(order.mark(kRelabelled, stream));
     if (l > 0) {

@@ -37,10 +37,16 @@ struct PairSink {
   int ts_bits;
   int64_t ts_base;
   int64_t *out_id, *out_ts, *inv_a, *inv_b, *d_n_unique;
+  uint32_t *order, *row, *first;         // optional: see RowOrder
   __device__ __forceinline__ void begin() { n_a = eff_count(n_a, d_n_a); }
   __device__ __forceinline__ bool counted(uint64_t) const { return true; }
   __device__ __forceinline__ uint64_t group(uint64_t k) const { return k; }
-  __device__ __forceinline__ void item(int64_t, uint64_t k, uint32_t pos, bool head, int64_t u, bool, int64_t) const {
+  __device__ __forceinline__ void item(int64_t at, uint64_t k, uint32_t pos, bool head, int64_t u, bool, int64_t) const {
+    if (order) {
+      order[at] = (int64_t)pos < n_a ? ~0u : (uint32_t)(pos - n_a);
+      row[at] = (uint32_t)u;
+      if (head) first[u] = (uint32_t)at;
+    }
     if (head) {
       out_id[u] = ts_bits >= 64 ? 0 : (int64_t)(k >> ts_bits);
       out_ts[u] = (int64_t)(k & low_mask(ts_bits)) + ts_base;
@@ -51,8 +57,11 @@ struct PairSink {
       inv_b[(int64_t)pos - n_a] = u;
     }
   }
-  __device__ __forceinline__ void finish(int64_t, uint64_t, bool, int64_t groups, int64_t) const {
-    if (threadIdx.x == 0) *d_n_unique = groups;
+  __device__ __forceinline__ void finish(int64_t n, uint64_t, bool, int64_t groups, int64_t) const {
+    if (threadIdx.x == 0) {
+      *d_n_unique = groups;
+      if (order) first[groups] = (uint32_t)n;
+    }
   }
 };
 
@@ -61,8 +70,9 @@ struct CscSource {
   int64_t n_cap;
   int dst_bits, ts_bits;
   int64_t ts_base;
+  const int* gate;                       // optional: 0 = another kernel has done the work
   int32_t* d_status;
-  __device__ __forceinline__ int64_t begin() const { return eff_count(n_cap, d_n); }
+  __device__ __forceinline__ int64_t begin() const { return gate && *gate == 0 ? 0 : eff_count(n_cap, d_n); }
   __device__ __forceinline__ uint64_t key(int64_t e) const {
     int64_t d = dst[e];
     if (dst_map) d = dst_map[d];
@@ -86,7 +96,8 @@ struct CscSink {
   int64_t *indptr, *out_indices, *out_ts;
   float* out_dt;
   int64_t* out_eid;
-  __device__ __forceinline__ void begin() { num_dst = eff_count(num_dst, d_num_dst); }
+  const int* gate;                       // as in CscSource
+  __device__ __forceinline__ void begin() { num_dst = gate && *gate == 0 ? -1 : eff_count(num_dst, d_num_dst); }
   __device__ __forceinline__ int64_t row(uint64_t k) const { return ts_bits >= 64 ? 0 : (int64_t)(k >> ts_bits); }
   __device__ __forceinline__ void item(int64_t at, uint64_t k, uint32_t p, bool has_prev, uint64_t prev) const {
     out_indices[at] = src_local ? src_local[p] : (int64_t)p;

@@ -143,6 +143,7 @@ lsd_pass_kernel(Items items, Digit digit, int pass,
   LsdSmem& sm = *(LsdSmem*)smem;
   constexpr int kItems = kLsdItems, kTile = kLsdTile;
   const int64_t n = items.begin();
+  if ((int64_t)blockIdx.x * kTile >= n) return;            // (capacity beyond the count; the others share the tickets)
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   if (tid == 0) sm.ticket = (int)atomicAdd(ticket, 1u);
   for (int j = tid; j < kLsdWarps * kRadix; j += kLsdThreads) {
@@ -152,7 +153,6 @@ lsd_pass_kernel(Items items, Digit digit, int pass,
   __syncthreads();
   const int tile = sm.ticket;
   const int64_t tile_base = (int64_t)tile * kTile;
-  if (tile_base >= n) return;
   const int tile_n = (int)(n - tile_base < kTile ? n - tile_base : kTile);
   // a warp owns consecutive keys of the tile, 32 at a time: (warp, round, lane) order = key order
   const int first = warp * (kItems * 32) + lane;
@@ -350,11 +350,11 @@ lsd_deliver_kernel(Sink sink, const uint64_t* __restrict__ keys, const uint32_t*
     __shared__ int s_ticket;
     __shared__ uint64_t s_cnt[kDeliverItems * (kDeliverThreads / 32)], s_scan[kDeliverItems * (kDeliverThreads / 32)];
     __shared__ uint64_t s_base;
+    if ((int)blockIdx.x >= tiles) return;
     if (tid == 0) s_ticket = (int)atomicAdd(ctl, 1ull);
     __syncthreads();
     const int tile = s_ticket;
     const int64_t first = (int64_t)tile * kDeliverTile;
-    if (first >= n) return;
     uint64_t k[kDeliverItems];
     uint32_t p[kDeliverItems];
     unsigned h1 = 0, h2 = 0;             // bit c: item c of the thread starts a group / a coarser group

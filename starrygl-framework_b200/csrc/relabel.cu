@@ -10,6 +10,7 @@
 #include "sort.cuh"
 #include "lists.cuh"
 #include "lsd.cuh"
+#include "rowcsc.cuh"
 
 namespace sgl {
 namespace {
@@ -45,6 +46,141 @@ csc_emit_sorted_kernel(const int64_t* __restrict__ dst, int64_t n_cap, const int
   }
 }
 
+// CSC by sort; gate: see CscSource
+int csc_sort(const int64_t* src_local, const int64_t* dst, const int64_t* dst_map, const int64_t* ts, const float* dt, const int64_t* eid,
+             int64_t n_edges, const int64_t* d_n_edges, int64_t num_dst, const int64_t* d_num_dst, int dst_bits, int ts_bits, int64_t ts_base,
+             int64_t* out_indptr, int64_t* out_indices, int64_t* out_ts, float* out_dt, int64_t* out_eid, const int* gate, int32_t* d_status,
+             void* ws, size_t ws_bytes, cudaStream_t stream) {
+  return sort_list(CscSource{dst, dst_map, ts, d_n_edges, n_edges, dst_bits, ts_bits, ts_base, gate, d_status},
+                   CscSink{num_dst, d_num_dst, ts_bits, src_local, ts, dt, eid, out_indptr, out_indices, out_ts, out_dt, out_eid, gate},
+                   n_edges < 1 ? 1 : n_edges, dst_bits + ts_bits, ws, ws_bytes, d_status, stream);
+}
+
+// ---- CSC in list order (rowcsc.cuh) --------------------------------------------------------------------------------------
+constexpr int kRowItems = 8;             // list items per thread of the count kernel
+constexpr int kRowTile = kThreads * kRowItems;
+constexpr int64_t kMaxRowTargets = 128;
+constexpr int kMapFanout = 32;
+inline int64_t rows_ctas(int64_t cap) { return (cap + kRowTile - 1) / kRowTile < 1 ? 1 : (cap + kRowTile - 1) / kRowTile; }
+
+// start[at]: edges of the items before `at` in its tile; sums: edges before the tile
+__global__ void __launch_bounds__(kThreads)
+csc_rows_count_kernel(const RowOrder ro, const int64_t* d_rows, const int64_t* __restrict__ offsets, uint32_t* __restrict__ start,
+                      int64_t* sums, unsigned int* done, int* gate) {
+  __shared__ uint32_t s_w[kThreads / 32];
+  const int64_t n = ro.first[*d_rows];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int64_t first = (int64_t)blockIdx.x * kRowTile + warp * (32 * kRowItems) + lane;
+  uint32_t o[kRowItems], c[kRowItems];
+  bool crowded = false;
+#pragma unroll
+  for (int r = 0; r < kRowItems; ++r) {
+    const int64_t at = first + r * 32;
+    o[r] = at < n ? ro.order[at] : ~0u;
+    if (at + kMaxRowTargets < n) crowded |= ro.row[at] == ro.row[at + kMaxRowTargets];
+  }
+#pragma unroll
+  for (int r = 0; r < kRowItems; ++r) c[r] = o[r] != ~0u ? (uint32_t)(offsets[o[r] + 1] - offsets[o[r]]) : 0u;
+  uint32_t carry = 0;
+#pragma unroll
+  for (int r = 0; r < kRowItems; ++r) {
+    const uint32_t x = warp_inclusive_scan(c[r], lane), own = c[r];
+    c[r] = carry + x - own;
+    carry += __shfl_sync(0xffffffffu, x, 31);
+  }
+  if (lane == 0) s_w[warp] = carry;
+  if (crowded) *gate = 1;
+  __syncthreads();
+  uint32_t before = 0, total = 0;
+#pragma unroll
+  for (int w = 0; w < kThreads / 32; ++w) {
+    if (w < warp) before += s_w[w];
+    total += s_w[w];
+  }
+#pragma unroll
+  for (int r = 0; r < kRowItems; ++r)
+    if (first + r * 32 < n) start[first + r * 32] = before + c[r];
+  publish_and_scan_cta_totals<kThreads>((int64_t)total, sums, done, nullptr);
+}
+
+// Edges of kThreads list items; consecutive threads take consecutive edges.
+__global__ void __launch_bounds__(kThreads)
+csc_rows_copy_kernel(const RowOrder ro, const int64_t* d_rows, const int64_t* __restrict__ offsets, const int64_t* __restrict__ ts,
+                     const float* __restrict__ dt, const int64_t* __restrict__ eid, int fanout, const uint32_t* __restrict__ start,
+                     const int64_t* __restrict__ sums, const int* gate, int64_t* __restrict__ indptr, int64_t* __restrict__ indices,
+                     int64_t* __restrict__ out_ts, float* __restrict__ out_dt, int64_t* __restrict__ out_eid) {
+  extern __shared__ uint8_t s_map[];       // item of every edge (fan-outs up to kMapFanout)
+  __shared__ int s_ex[kThreads + 1];
+  __shared__ int64_t s_src[kThreads], s_to[kThreads];
+  __shared__ uint32_t s_q0[kThreads], s_q1[kThreads];
+  if (*gate) return;
+  const int64_t rows = *d_rows, n = ro.first[rows];
+  const int tid = threadIdx.x;
+  const int64_t first = (int64_t)blockIdx.x * kThreads, at = first + tid;
+  if (n == 0 && at == 0) indptr[0] = 0;
+  if (first >= n) return;
+  int c = 0;
+  if (at < n) {
+    const uint32_t o = ro.order[at], u = ro.row[at], q0 = ro.first[u], q1 = ro.first[u + 1];
+    const int64_t begin = sums[q0 / kRowTile] + start[q0];
+    int64_t src = 0;
+    if (o != ~0u) {
+      src = offsets[o];
+      c = (int)(offsets[o + 1] - src);
+    }
+    s_src[tid] = src;
+    s_to[tid] = begin;
+    s_q0[tid] = q0;
+    s_q1[tid] = q1;
+    if (q0 == at) indptr[u] = begin;
+    if (at == n - 1) indptr[rows] = sums[at / kRowTile] + start[at] + c;
+  }
+  int total;
+  const int ex = cta_exclusive_scan<kThreads, int>(c, &total);
+  const bool has_map = fanout <= kMapFanout;
+  s_ex[tid] = ex;
+  if (tid == kThreads - 1) s_ex[kThreads] = total;
+  if (has_map)
+    for (int j = 0; j < c; ++j) s_map[ex + j] = (uint8_t)tid;
+  __syncthreads();
+  for (int o = tid; o < total; o += kThreads) {
+    int k;
+    if (has_map) {
+      k = s_map[o];
+    } else {
+      int b = kThreads;                    // last item with s_ex[item] <= o
+      k = 0;
+      while (b - k > 1) {
+        const int m = (k + b) >> 1;
+        if (s_ex[m] <= o) k = m; else b = m;
+      }
+    }
+    const int j = o - s_ex[k];
+    const int64_t e = s_src[k] + j, t = ts[e];
+    const float d = dt[e];
+    const int64_t id = eid[e];
+    int64_t to = s_to[k] + j;
+    const uint32_t me = (uint32_t)(first + k), q1 = s_q1[k];
+    for (uint32_t q = s_q0[k]; q < q1; ++q) {
+      if (q == me) continue;
+      const uint32_t other = ro.order[q];
+      if (other == ~0u) continue;
+      // edges of the other target before this one: earlier ones, and equal ones of an earlier target
+      const int64_t s0 = __ldg(offsets + other);
+      int64_t a = s0, b = __ldg(offsets + other + 1);
+      while (a < b) {
+        const int64_t mid = (a + b) >> 1, x = __ldg(ts + mid);
+        if (x < t || (x == t && q < me)) a = mid + 1; else b = mid;
+      }
+      to += a - s0;
+    }
+    indices[to] = e;
+    out_ts[to] = t;
+    out_dt[to] = d;
+    out_eid[to] = id;
+  }
+}
+
 // first position with sorted[pos] >= value, one thread per value
 __global__ void lower_bound_kernel(const int64_t* __restrict__ sorted, int64_t n, const int64_t* __restrict__ values,
                                    int k, int64_t* __restrict__ out) {
@@ -66,10 +202,10 @@ using namespace sgl;
 
 extern "C" size_t sgl_unique_pairs_ws_bytes(int64_t n_total) { return list_ws_bytes(n_total); }
 
-extern "C" int sgl_unique_pairs(const int64_t* a_id, const int64_t* a_ts, int64_t n_a, const int64_t* d_n_a,
+int sgl::unique_pairs(const int64_t* a_id, const int64_t* a_ts, int64_t n_a, const int64_t* d_n_a,
                                 const int64_t* b_id, const int64_t* b_ts, int64_t n_b, const int64_t* d_n_b, int id_bits,
                                 int ts_bits, int64_t ts_base, int64_t* out_id, int64_t* out_ts, int64_t* inv_a,
-                                int64_t* inv_b, int64_t* d_n_unique, int32_t* d_status, void* ws, size_t ws_bytes,
+                                int64_t* inv_b, int64_t* d_n_unique, const RowOrder& ro, int32_t* d_status, void* ws, size_t ws_bytes,
                                 void* stream_) {
   SGL_NVTX("sgl_unique_pairs");
   cudaStream_t stream = (cudaStream_t)stream_;
@@ -80,15 +216,24 @@ extern "C" int sgl_unique_pairs(const int64_t* a_id, const int64_t* a_ts, int64_
   const int64_t n = n_a + n_b;
   if (n == 0) {
     SGL_CHECK_RC(zero_async(d_n_unique, sizeof(int64_t), stream));
+    if (ro.first) SGL_CHECK_RC(zero_async(ro.first, sizeof(uint32_t), stream));
     return SGL_OK;
   }
   SGL_REQUIRE((n_a == 0 || (a_id && a_ts)) && (n_b == 0 || (b_id && b_ts)) && out_id && out_ts, SGL_ERR_ARG,
               "unique_pairs: null array");
   LaunchScope scope(stream);
   SGL_CHECK_RC(sort_list(PairSource{a_id, a_ts, d_n_a, b_id, b_ts, d_n_b, n_a, n_b, id_bits, ts_bits, ts_base, d_status},
-                         PairSink{n_a, d_n_a, ts_bits, ts_base, out_id, out_ts, inv_a, inv_b, d_n_unique}, n, id_bits + ts_bits, ws,
-                         ws_bytes, d_status, stream));
+                         PairSink{n_a, d_n_a, ts_bits, ts_base, out_id, out_ts, inv_a, inv_b, d_n_unique, ro.order, ro.row, ro.first}, n,
+                         id_bits + ts_bits, ws, ws_bytes, d_status, stream));
   return scope.submit();
+}
+
+extern "C" int sgl_unique_pairs(const int64_t* a_id, const int64_t* a_ts, int64_t n_a, const int64_t* d_n_a, const int64_t* b_id,
+                                const int64_t* b_ts, int64_t n_b, const int64_t* d_n_b, int id_bits, int ts_bits, int64_t ts_base,
+                                int64_t* out_id, int64_t* out_ts, int64_t* inv_a, int64_t* inv_b, int64_t* d_n_unique, int32_t* d_status,
+                                void* ws, size_t ws_bytes, void* stream) {
+  return unique_pairs(a_id, a_ts, n_a, d_n_a, b_id, b_ts, n_b, d_n_b, id_bits, ts_bits, ts_base, out_id, out_ts, inv_a, inv_b, d_n_unique,
+                      RowOrder{}, d_status, ws, ws_bytes, stream);
 }
 
 extern "C" size_t sgl_build_csc_ws_bytes(int64_t n_edges, int64_t num_dst) {
@@ -118,14 +263,42 @@ extern "C" int sgl_build_csc(const int64_t* src_local, const int64_t* dst, const
   SGL_REQUIRE(dst_bits >= 0 && ts_bits >= 0 && dst_bits + ts_bits <= 64, SGL_ERR_UNSUPPORTED,
               "build_csc: dst_bits %d + ts_bits %d exceed the 64-bit sort key", dst_bits, ts_bits);
   SGL_REQUIRE(out_indptr, SGL_ERR_ARG, "build_csc: out_indptr is null");
-  const int64_t cap = n_edges < 1 ? 1 : n_edges;
   SGL_REQUIRE(n_edges == 0 || (dst && ts && dt && eid && out_indices && out_ts && out_dt && out_eid), SGL_ERR_ARG,
               "build_csc: null array");
   LaunchScope scope(stream);
-  SGL_CHECK_RC(sort_list(
-      CscSource{dst, dst_map, ts, d_n_edges, n_edges, dst_bits, ts_bits, ts_base, d_status},
-      CscSink{num_dst, d_num_dst, ts_bits, src_local, ts, dt, eid, out_indptr, out_indices, out_ts, out_dt, out_eid}, cap,
-      dst_bits + ts_bits, ws, ws_bytes, d_status, stream));
+  SGL_CHECK_RC(csc_sort(src_local, dst, dst_map, ts, dt, eid, n_edges, d_n_edges, num_dst, d_num_dst, dst_bits, ts_bits, ts_base, out_indptr,
+                        out_indices, out_ts, out_dt, out_eid, nullptr, d_status, ws, ws_bytes, stream));
+  return scope.submit();
+}
+
+size_t sgl::build_csc_rows_ws_bytes(int64_t n_edges, int64_t list_cap) {
+  return align_up((size_t)list_cap * 4) + align_up((size_t)rows_ctas(list_cap) * 8) + align_up(8) + list_ws_bytes(n_edges);
+}
+
+int sgl::build_csc_rows(const RowOrder& ro, int64_t list_cap, const int64_t* offsets, int fanout, const int64_t* dst, const int64_t* dst_map,
+                        const int64_t* ts, const float* dt, const int64_t* eid, int64_t n_edges, const int64_t* d_n_edges, int64_t num_dst,
+                        const int64_t* d_num_dst, int dst_bits, int ts_bits, int64_t ts_base, int64_t* out_indptr, int64_t* out_indices,
+                        int64_t* out_ts, float* out_dt, int64_t* out_eid, int32_t* d_status, void* ws, size_t ws_bytes, void* stream_) {
+  cudaStream_t stream = (cudaStream_t)stream_;
+  SGL_REQUIRE(dst_bits >= 0 && ts_bits >= 0 && dst_bits + ts_bits <= 64, SGL_ERR_UNSUPPORTED,
+              "build_csc: dst_bits %d + ts_bits %d exceed the 64-bit sort key", dst_bits, ts_bits);
+  LaunchScope scope(stream);
+  WsCarver c(ws, ws_bytes);
+  uint32_t* start = c.take<uint32_t>(list_cap);
+  const int64_t ctas = rows_ctas(list_cap);
+  int64_t* sums = c.take<int64_t>(ctas);
+  unsigned int* words = c.take<unsigned int>(2);           // arrivals, gate
+  const size_t sort_bytes = list_ws_bytes(n_edges);
+  char* sort_ws = c.take<char>(sort_bytes);
+  SGL_REQUIRE(c.ok(), SGL_ERR_WORKSPACE, "build_csc: workspace %zu < %zu bytes", ws_bytes, build_csc_rows_ws_bytes(n_edges, list_cap));
+  int* gate = (int*)(words + 1);
+  SGL_CHECK_RC(zero_async(words, 8, stream));
+  SGL_CHECK_RC(launch(csc_rows_count_kernel, (unsigned)ctas, kThreads, 0, stream, ro, d_num_dst, offsets, start, sums, words, gate));
+  SGL_CHECK_RC(launch(csc_rows_copy_kernel, (unsigned)((list_cap + kThreads - 1) / kThreads), kThreads,
+                      fanout <= kMapFanout ? (size_t)kThreads * fanout : 0, stream, ro, d_num_dst, offsets, ts, dt, eid, fanout, start, sums,
+                      gate, out_indptr, out_indices, out_ts, out_dt, out_eid));
+  SGL_CHECK_RC(csc_sort(nullptr, dst, dst_map, ts, dt, eid, n_edges, d_n_edges, num_dst, d_num_dst, dst_bits, ts_bits, ts_base, out_indptr,
+                        out_indices, out_ts, out_dt, out_eid, gate, d_status, sort_ws, sort_bytes, stream));
   return scope.submit();
 }
 

@@ -238,20 +238,20 @@ def build_batch(g, roots, root_ts, fanouts, policy="recent", **kw) -> List[dict]
 
 def batch_kernel_launches(num_nodes: int, num_roots: int, fanouts: Sequence[int], ts_span: int) -> int:
     """Kernels of this library that one mini-batch of :func:`build_batch_async` launches at the given capacities: count and
-    fill of every hop, the sort of every relabel and of every CSC after the first (with pack, head scan and emit kernels
-    around it only for lists above the mini-batch sort's limit)."""
+    fill of every hop, the sort of every relabel (above the mini-batch sort's limit with an item count and a delivery
+    kernel), and for every hop after the first the two CSC kernels, the sort behind them and the column map."""
     L = _C.lib()
     id_bits, ts_bits = ops.bits_for(num_nodes - 1), ops.bits_for(ts_span)
 
-    def sort(n, bits, around):
+    def sort(n, bits):
         k = L.sgl_radix_sort_launches(n, bits)
-        return k if k <= 2 else k + around
-    total = sort(num_roots, id_bits + ts_bits, 3)
+        return k if k <= 2 else k + 2
+    total = sort(num_roots, id_bits + ts_bits)
     cur, targets = num_roots, num_roots
     for l, k in enumerate(fanouts):
         edges = targets * k
-        total += 2 + sort(cur + edges, id_bits + ts_bits, 3)
-        total += 0 if l == 0 else 1 + sort(edges, ops.bits_for(cur) + ts_bits, 2)
+        total += 2 + sort(cur + edges, id_bits + ts_bits)
+        total += 0 if l == 0 else 1 + (2 if edges > 2048 else 0) + sort(edges, ops.bits_for(cur) + ts_bits)
         cur, targets = cur + edges, edges
     return int(total)
 

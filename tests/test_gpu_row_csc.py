@@ -1,0 +1,35 @@
+"""CSC of the later hops along the layer list's order: rows of one and of several targets, rows at and above the number of
+targets from which the sort takes over, fan-outs with and without the edge-to-item map, recent and uniform."""
+import numpy as np
+import pytest
+
+from oracle import oracle_np as O
+from gpu_util import cu, npy, build_graph
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("queries", [1, 127, 128, 129, 400])
+@pytest.mark.parametrize("fanouts", [[3, 4], [3, 40], [2, 3, 5]])
+@pytest.mark.parametrize("policy", ["recent", "uniform"])
+def test_rows_of_many_targets(queries, fanouts, policy):
+    from starrygl.graph.batch import build_batch
+    rng = np.random.default_rng(queries)
+    n, m = 200, 6000
+    # node 0 has three events, so every later query of it samples them all: one pair per event, `queries` targets each
+    src = np.concatenate([rng.integers(2, n, m), [1, 5, 1]]).astype(np.int64)
+    dst = np.concatenate([rng.integers(1, n, m), [0, 0, 0]]).astype(np.int64)
+    ts = np.concatenate([np.sort(rng.integers(0, 500, m)), [400, 420, 430]]).astype(np.int64)
+    z = {"n": n, "dst": dst, "src": src, "ts": ts, "eid": np.arange(m + 3, dtype=np.int64)}
+    g = build_graph(z)
+    indptr, nbr, tss, eid, _ = O.tcsr_build(dst, src, ts, z["eid"], n)
+    roots = np.concatenate([np.zeros(queries, np.int64), rng.integers(1, n, 250)])
+    rts = np.concatenate([600 + np.arange(queries), rng.integers(100, 500, 250)]).astype(np.int64)
+    pol = O.RECENT if policy == "recent" else O.UNIFORM
+    ref = O.build_batch(indptr, nbr, tss, eid, roots, rts, fanouts, pol, seed=3)
+    out = build_batch(g, cu(roots), cu(rts), fanouts, policy, seed=3, ts_range=(0, 1100))
+    assert len(out) == len(ref)
+    for i, (d, r) in enumerate(zip(out, ref)):
+        for k in r:
+            a = npy(d[k])
+            assert a.dtype == r[k].dtype and np.array_equal(a, r[k]), (i, k)

@@ -48,8 +48,8 @@ struct PairSink {
       if (head) first[u] = (uint32_t)at;
     }
     if (head) {
-      out_id[u] = ts_bits >= 64 ? 0 : (int64_t)(k >> ts_bits);
-      out_ts[u] = (int64_t)(k & low_mask(ts_bits)) + ts_base;
+      __stcs((long long*)out_id + u, ts_bits >= 64 ? 0ll : (long long)(k >> ts_bits));
+      __stcs((long long*)out_ts + u, (long long)((int64_t)(k & low_mask(ts_bits)) + ts_base));
     }
     if ((int64_t)pos < n_a) {
       if (inv_a) inv_a[pos] = u;

@@ -362,8 +362,8 @@ lsd_deliver_kernel(Sink sink, const uint64_t* __restrict__ keys, const uint32_t*
 #pragma unroll
     for (int c = 0; c < kDeliverItems; ++c) {
       const int64_t i = first + c * kDeliverThreads + tid;
-      k[c] = i < n ? keys[i] : 0;
-      p[c] = i < n ? pos[i] : 0u;
+      k[c] = i < n ? __ldcs(keys + i) : 0;     // (streamed: the cache is for what the sink scatters)
+      p[c] = i < n ? __ldcs(pos + i) : 0u;
     }
 #pragma unroll
     for (int c = 0; c < kDeliverItems; ++c) {

@@ -6,6 +6,8 @@
 //
 // Algorithmic HBM bytes: 16 read + 8 write per input pair, 16 per unique pair, plus the sort passes
 // (32 B per pair and populated key byte).
+#include <limits.h>
+
 #include "launch.cuh"
 #include "sort.cuh"
 #include "lists.cuh"
@@ -59,13 +61,14 @@ int csc_sort(const int64_t* src_local, const int64_t* dst, const int64_t* dst_ma
 // ---- CSC in list order (rowcsc.cuh) --------------------------------------------------------------------------------------
 constexpr int kRowItems = 8;             // list items per thread of the count kernel
 constexpr int kRowTile = kThreads * kRowItems;
-constexpr int64_t kMaxRowTargets = 128;
+constexpr int64_t kMaxRowTargets = 32;
 constexpr int kMapFanout = 32;
 inline int64_t rows_ctas(int64_t cap) { return (cap + kRowTile - 1) / kRowTile < 1 ? 1 : (cap + kRowTile - 1) / kRowTile; }
 
-// start[at]: edges of the items before `at` in its tile; sums: edges before the tile
+// start[at]: edges of the items before `at` in its tile; sums: edges before the tile.  Targets of `drawn` or more edges may have
+// drawn them.
 __global__ void __launch_bounds__(kThreads)
-csc_rows_count_kernel(const RowOrder ro, const int64_t* d_rows, const int64_t* __restrict__ offsets, uint32_t* __restrict__ start,
+csc_rows_count_kernel(const RowOrder ro, const int64_t* d_rows, const int64_t* __restrict__ offsets, int drawn, uint32_t* __restrict__ start,
                       int64_t* sums, unsigned int* done, int* gate) {
   __shared__ uint32_t s_w[kThreads / 32];
   const int64_t n = ro.first[*d_rows];
@@ -77,10 +80,14 @@ csc_rows_count_kernel(const RowOrder ro, const int64_t* d_rows, const int64_t* _
   for (int r = 0; r < kRowItems; ++r) {
     const int64_t at = first + r * 32;
     o[r] = at < n ? ro.order[at] : ~0u;
-    if (at + kMaxRowTargets < n) crowded |= ro.row[at] == ro.row[at + kMaxRowTargets];
   }
 #pragma unroll
   for (int r = 0; r < kRowItems; ++r) c[r] = o[r] != ~0u ? (uint32_t)(offsets[o[r] + 1] - offsets[o[r]]) : 0u;
+#pragma unroll
+  for (int r = 0; r < kRowItems; ++r) {
+    const int64_t at = first + r * 32;
+    if (c[r] >= (uint32_t)drawn && at + kMaxRowTargets < n) crowded |= ro.row[at] == ro.row[at + kMaxRowTargets];
+  }
   uint32_t carry = 0;
 #pragma unroll
   for (int r = 0; r < kRowItems; ++r) {
@@ -106,7 +113,7 @@ csc_rows_count_kernel(const RowOrder ro, const int64_t* d_rows, const int64_t* _
 // Edges of kThreads list items; consecutive threads take consecutive edges.
 __global__ void __launch_bounds__(kThreads)
 csc_rows_copy_kernel(const RowOrder ro, const int64_t* d_rows, const int64_t* __restrict__ offsets, const int64_t* __restrict__ ts,
-                     const float* __restrict__ dt, const int64_t* __restrict__ eid, int fanout, const uint32_t* __restrict__ start,
+                     const float* __restrict__ dt, const int64_t* __restrict__ eid, int fanout, int drawn, const uint32_t* __restrict__ start,
                      const int64_t* __restrict__ sums, const int* gate, int64_t* __restrict__ indptr, int64_t* __restrict__ indices,
                      int64_t* __restrict__ out_ts, float* __restrict__ out_dt, int64_t* __restrict__ out_eid) {
   extern __shared__ uint8_t s_map[];       // item of every edge (fan-outs up to kMapFanout)
@@ -160,8 +167,19 @@ csc_rows_copy_kernel(const RowOrder ro, const int64_t* d_rows, const int64_t* __
     const float d = dt[e];
     const int64_t id = eid[e];
     int64_t to = s_to[k] + j;
-    const uint32_t me = (uint32_t)(first + k), q1 = s_q1[k];
-    for (uint32_t q = s_q0[k]; q < q1; ++q) {
+    const uint32_t me = (uint32_t)(first + k), q0 = s_q0[k], q1 = s_q1[k];
+    if (s_ex[k + 1] - s_ex[k] < drawn) {
+      // the row's targets have this same list: before the edge come the earlier ones of every target, the equal ones of the targets
+      // before, and its own equal ones before it
+      const uint32_t others = ro.order[q0] == ~0u ? q0 + 1 : q0;         // the row's first target
+      if (q1 - others > 1) {
+        const int64_t end = s_src[k] + s_ex[k + 1] - s_ex[k];
+        int64_t lo = e, hi = e + 1;
+        while (lo > s_src[k] && __ldg(ts + lo - 1) == t) --lo;
+        while (hi < end && __ldg(ts + hi) == t) ++hi;
+        to += (lo - s_src[k]) * (int64_t)(q1 - others - 1) + (hi - lo) * (int64_t)(me - others);
+      }
+    } else for (uint32_t q = q0; q < q1; ++q) {
       if (q == me) continue;
       const uint32_t other = ro.order[q];
       if (other == ~0u) continue;
@@ -275,7 +293,7 @@ size_t sgl::build_csc_rows_ws_bytes(int64_t n_edges, int64_t list_cap) {
   return align_up((size_t)list_cap * 4) + align_up((size_t)rows_ctas(list_cap) * 8) + align_up(8) + list_ws_bytes(n_edges);
 }
 
-int sgl::build_csc_rows(const RowOrder& ro, int64_t list_cap, const int64_t* offsets, int fanout, const int64_t* dst, const int64_t* dst_map,
+int sgl::build_csc_rows(const RowOrder& ro, int64_t list_cap, const int64_t* offsets, int fanout, bool draws, const int64_t* dst, const int64_t* dst_map,
                         const int64_t* ts, const float* dt, const int64_t* eid, int64_t n_edges, const int64_t* d_n_edges, int64_t num_dst,
                         const int64_t* d_num_dst, int dst_bits, int ts_bits, int64_t ts_base, int64_t* out_indptr, int64_t* out_indices,
                         int64_t* out_ts, float* out_dt, int64_t* out_eid, int32_t* d_status, void* ws, size_t ws_bytes, void* stream_) {
@@ -293,10 +311,11 @@ int sgl::build_csc_rows(const RowOrder& ro, int64_t list_cap, const int64_t* off
   SGL_REQUIRE(c.ok(), SGL_ERR_WORKSPACE, "build_csc: workspace %zu < %zu bytes", ws_bytes, build_csc_rows_ws_bytes(n_edges, list_cap));
   int* gate = (int*)(words + 1);
   SGL_CHECK_RC(zero_async(words, 8, stream));
-  SGL_CHECK_RC(launch(csc_rows_count_kernel, (unsigned)ctas, kThreads, 0, stream, ro, d_num_dst, offsets, start, sums, words, gate));
+  SGL_CHECK_RC(launch(csc_rows_count_kernel, (unsigned)ctas, kThreads, 0, stream, ro, d_num_dst, offsets, draws ? fanout : INT_MAX, start,
+                      sums, words, gate));
   SGL_CHECK_RC(launch(csc_rows_copy_kernel, (unsigned)((list_cap + kThreads - 1) / kThreads), kThreads,
-                      fanout <= kMapFanout ? (size_t)kThreads * fanout : 0, stream, ro, d_num_dst, offsets, ts, dt, eid, fanout, start, sums,
-                      gate, out_indptr, out_indices, out_ts, out_dt, out_eid));
+                      fanout <= kMapFanout ? (size_t)kThreads * fanout : 0, stream, ro, d_num_dst, offsets, ts, dt, eid, fanout,
+                      draws ? fanout : INT_MAX, start, sums, gate, out_indptr, out_indices, out_ts, out_dt, out_eid));
   SGL_CHECK_RC(csc_sort(nullptr, dst, dst_map, ts, dt, eid, n_edges, d_n_edges, num_dst, d_num_dst, dst_bits, ts_bits, ts_base, out_indptr,
                         out_indices, out_ts, out_dt, out_eid, gate, d_status, sort_ws, sort_bytes, stream));
   return scope.submit();

@@ -161,6 +161,60 @@ __device__ __forceinline__ uint64_t draw_below(int64_t target, int d, uint32_t r
   return ((uint64_t)ph.c[0] | ((uint64_t)ph.c[1] << 32)) % bound;
 }
 
+// x mod b, exactly: a quotient estimate by reciprocal is off by at most one (its relative error is below 2^-45, the quotients
+// of the two 32-bit steps below 2^32), which the remainder's sign and size show.  The compiler's 64-bit remainder was a third of
+// the instructions of a launch that draws.
+__device__ __forceinline__ uint32_t remainder_step(uint32_t upper, uint32_t lower, uint32_t b, double db, double inv) {
+  const uint64_t y = ((uint64_t)upper << 32) | lower;      // upper < b
+  const uint32_t q = __double2uint_rz(fma((double)upper, 4294967296.0, (double)lower) * inv);     // (saturates)
+  int64_t r = (int64_t)(y - (uint64_t)q * b);
+  r += r < 0 ? (int64_t)b : 0;
+  r -= r >= (int64_t)b ? (int64_t)b : 0;
+  return (uint32_t)r;
+}
+__device__ __forceinline__ uint32_t remainder_u32(uint64_t x, uint32_t b) {
+  const double db = (double)b, guess = (double)__frcp_rn((float)b), inv = fma(guess, fma(-db, guess, 1.0), guess);   // one Newton step
+  return remainder_step(remainder_step(0u, (uint32_t)(x >> 32), b, db, inv), (uint32_t)x, b, db, inv);
+}
+
+__device__ __forceinline__ uint32_t draw_below_u32(int64_t target, int d, uint32_t rng_stream, uint64_t seed, uint32_t bound) {
+  Philox ph((uint32_t)target, (uint32_t)((uint64_t)target >> 32), (uint32_t)d, rng_stream, (uint32_t)seed, (uint32_t)(seed >> 32));
+  return remainder_u32((uint64_t)ph.c[0] | ((uint64_t)ph.c[1] << 32), bound);
+}
+
+// Floyd's subset selection of `fanout` <= kRegPicks out of cand > fanout positions by one lane: draw d picks uniformly in [0, cand -
+// fanout + d], a repeat is replaced by cand - fanout + d.  Everything in registers (unrolled: the round keys and a round of the
+// generator are shared by the draws); the picks are left in ascending order, FT words apart.
+constexpr int kRegPicks = 16;
+template <int FT>
+__device__ __forceinline__ void draw_sorted(int64_t target, uint32_t cand, int fanout, uint32_t rng_stream, uint64_t seed, uint32_t* picks) {
+  uint32_t pick[kRegPicks];
+  int rank[kRegPicks];
+#pragma unroll
+  for (int d = 0; d < kRegPicks; ++d) {
+    if (d < fanout) {
+      const uint32_t top = cand - (uint32_t)fanout + (uint32_t)d;
+      Philox ph((uint32_t)target, (uint32_t)((uint64_t)target >> 32), (uint32_t)d, rng_stream, (uint32_t)seed, (uint32_t)(seed >> 32));
+      uint32_t x = remainder_u32((uint64_t)ph.c[0] | ((uint64_t)ph.c[1] << 32), top + 1u);
+      bool clash = false;
+#pragma unroll
+      for (int q = 0; q < d; ++q) clash |= pick[q] == x;
+      x = clash ? top : x;
+      rank[d] = 0;
+#pragma unroll
+      for (int q = 0; q < d; ++q) {
+        const bool above = pick[q] < x;
+        rank[d] += above ? 1 : 0;
+        rank[q] += above ? 0 : 1;
+      }
+      pick[d] = x;
+    }
+  }
+#pragma unroll
+  for (int d = 0; d < kRegPicks; ++d)
+    if (d < fanout) picks[rank[d] * FT] = pick[d];
+}
+
 __device__ __forceinline__ void emit_edge(const SampleArgs& a, int64_t p, int64_t o, int64_t t, int64_t target) {
   const int64_t ets = __ldg(a.ts + p);
   a.out_nbr[o] = __ldg(a.nbr + p);
@@ -289,12 +343,13 @@ sample_fill_kernel(const SampleArgs a, int count_ctas) {
     if (has_map)
       for (int j = 0; j < c; ++j) s_map[ex - begin + j] = (uint8_t)slot;
     if (lane_draws) {
-      // Floyd's subset selection: draw d picks uniformly in [0, cand - k + d]; a repeat is replaced by cand - k + d
       const int64_t cand = cut - lo;
-      if (cand > fanout && cand <= 0xffffffffll) {
+      if (cand > fanout && cand <= 0xffffffffll && fanout <= kRegPicks) {
+        draw_sorted<FT>(i, (uint32_t)cand, fanout, a.rng_stream, a.seed, s_pick + slot);
+      } else if (cand > fanout && cand <= 0xffffffffll) {
         for (int d = 0; d < fanout; ++d) {
           const uint32_t top = (uint32_t)(cand - fanout + d);
-          uint32_t pick = (uint32_t)draw_below(i, d, a.rng_stream, a.seed, (uint64_t)top + 1);
+          uint32_t pick = draw_below_u32(i, d, a.rng_stream, a.seed, top + 1u);
           bool clash = false;
           for (int q = 0; q < d; ++q) clash |= s_pick[q * FT + slot] == pick;
           s_pick[d * FT + slot] = clash ? top : pick;
@@ -329,8 +384,11 @@ sample_fill_kernel(const SampleArgs a, int count_ctas) {
       if (draws && wcut - wlo > fanout) {
         if (!lane_draws || wcut - wlo > 0xffffffffll) continue;
         const uint32_t pick = s_pick[(o - s_ex[k]) * FT + k];
-        int rank = 0;
-        for (int q = 0; q < fanout; ++q) rank += s_pick[q * FT + k] < pick ? 1 : 0;
+        int rank = o - s_ex[k];
+        if (fanout > kRegPicks) {
+          rank = 0;
+          for (int q = 0; q < fanout; ++q) rank += s_pick[q * FT + k] < pick ? 1 : 0;
+        }
         p = wlo + pick;
         g[u] = base + s_ex[k] + rank;
       } else {

@@ -184,9 +184,24 @@ tcsr_rows_kernel(const unsigned int* gave_up, const uint32_t* __restrict__ node,
     for (int64_t v = (int64_t)blockIdx.x * 256 + threadIdx.x; v <= num_nodes; v += stride) indptr[v] = 0;
     return;
   }
-#pragma unroll 4
-  for (int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x; i <= m; i += stride)
-    start_rows(indptr, i > 0 ? (int64_t)node[i - 1] : -1, i < m ? (int64_t)node[i] : num_nodes, i);
+  for (int64_t i0 = ((int64_t)blockIdx.x * 256 + threadIdx.x) * 4; i0 <= m; i0 += stride * 4) {
+    uint32_t x[4] = {0, 0, 0, 0};
+    if (i0 + 4 <= m) {
+      const uint4 q = *(const uint4*)(node + i0);
+      x[0] = q.x; x[1] = q.y; x[2] = q.z; x[3] = q.w;
+    } else {
+      for (int u = 0; u < 4; ++u)
+        if (i0 + u < m) x[u] = node[i0 + u];
+    }
+    int64_t prev = i0 > 0 ? (int64_t)node[i0 - 1] : -1;
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      if (i0 + u > m) break;
+      const int64_t cur = i0 + u < m ? (int64_t)x[u] : num_nodes;
+      start_rows(indptr, prev, cur, i0 + u);
+      prev = cur;
+    }
+  }
 }
 
 // combined == 0: the keys are node ids and the timestamps are gathered too
@@ -311,7 +326,7 @@ extern "C" int sgl_tcsr_build_fenced(int64_t num_nodes, int64_t m, const int64_t
       const EdgeOut out{k, node, out_nbr, out_ts, out_eid};
       SGL_CHECK_RC((lsd_sort<uint64_t, EdgePairs>(EdgePairs{k, nbr, eid, m}, k1, v1, k0, v0, m, nullptr, first_bit, ts_bits + id_bits, out,
                                                   &in_first, &gave_up, c, nullptr, stream)));
-      SGL_CHECK_RC(launch(tcsr_rows_kernel, grid, 256, 0, stream, gave_up, node, m, num_nodes, indptr));
+      SGL_CHECK_RC(launch(tcsr_rows_kernel, stream_grid(m, 256 * 4, 8), 256, 0, stream, gave_up, node, m, num_nodes, indptr));
     } else {
       uint64_t *k1 = c.take<uint64_t>(m), *k0 = c.take<uint64_t>(m);
       uint32_t *v1 = c.take<uint32_t>(m), *v0 = c.take<uint32_t>(m);

@@ -226,3 +226,19 @@ def test_every_launch_shape_matches_oracle(n, policy):
     for nm, a, r in zip(NAMES, out, ref):
         assert np.array_equal(a, r), nm
     assert offs[0] == 0 and offs[-1] == len(out[0]) and (np.diff(offs) >= 0).all()
+
+
+@pytest.mark.parametrize("k", [1, 2, 15, 16, 17, 32])
+def test_lane_draws_match_oracle(k):
+    """Draws by a target's lane on both sides of the fan-out up to which the picks stay in registers."""
+    from oracle import oracle_c as OC
+    z = random_graph(8, 2000, 120000, 50000, hub=30000)
+    g = build_graph(z)
+    indptr, nbr, ts, eid, _ = OC.tcsr_build(z["dst"], z["src"], z["ts"], z["eid"], z["n"])
+    rng = np.random.default_rng(k)
+    q = rng.integers(0, z["n"], 17000).astype(np.int64)
+    qt = rng.integers(0, 50010, 17000).astype(np.int64)
+    out, offs = run(g, q, qt, k, "uniform", seed=2 ** 40 + k, rng_stream=2)
+    ref = OC.sample_layer(indptr, nbr, ts, eid, q, qt, k, O.UNIFORM, seed=2 ** 40 + k, stream=2)
+    for nm, a, r in zip(NAMES, out, ref):
+        assert np.array_equal(a, r), nm

@@ -280,7 +280,7 @@ lsd_pass_kernel(Items items, Digit digit, int pass,
 }
 
 // ---- delivery of a sorted list to a Sink (see tilesort.cuh) -------------------------------------------------------------
-constexpr int kDeliverThreads = 512;
+constexpr int kDeliverThreads = 256;
 constexpr int kDeliverItems = 8;
 constexpr int kDeliverTile = kDeliverThreads * kDeliverItems;
 
@@ -320,7 +320,7 @@ __device__ __forceinline__ uint64_t deliver_prefix(uint64_t* state, int tile, ui
 
 // ctl[0] ticket, ctl[1] arrivals; state: one word per tile, cleared
 template <class Sink>
-__global__ void __launch_bounds__(kDeliverThreads)
+__global__ void __launch_bounds__(kDeliverThreads, 4)
 lsd_deliver_kernel(Sink sink, const uint64_t* __restrict__ keys, const uint32_t* __restrict__ pos, int64_t n_cap, const int64_t* d_count,
                    unsigned long long* ctl, uint64_t* state, const unsigned int* gave_up, int32_t* d_status) {
   const int64_t n = *gave_up ? 0 : eff_count(n_cap, d_count);     // (a pass that gave up left places unwritten)

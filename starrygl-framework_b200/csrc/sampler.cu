@@ -184,9 +184,8 @@ __device__ __forceinline__ uint32_t draw_below_u32(int64_t target, int d, uint32
 
 // Floyd's subset selection of `fanout` <= kRegPicks out of cand > fanout positions by one lane: draw d picks uniformly in [0, cand -
 // fanout + d], a repeat is replaced by cand - fanout + d.  Everything in registers (unrolled: the round keys and a round of the
-// generator are shared by the draws); the picks are left in ascending order, FT words apart.
+// generator are shared by the draws); the picks are left in ascending order.
 constexpr int kRegPicks = 16;
-template <int FT>
 __device__ __forceinline__ void draw_sorted(int64_t target, uint32_t cand, int fanout, uint32_t rng_stream, uint64_t seed, uint32_t* picks) {
   uint32_t pick[kRegPicks];
   int rank[kRegPicks];
@@ -212,7 +211,7 @@ __device__ __forceinline__ void draw_sorted(int64_t target, uint32_t cand, int f
   }
 #pragma unroll
   for (int d = 0; d < kRegPicks; ++d)
-    if (d < fanout) picks[rank[d] * FT] = pick[d];
+    if (d < fanout) picks[rank[d]] = pick[d];
 }
 
 __device__ __forceinline__ void emit_edge(const SampleArgs& a, int64_t p, int64_t o, int64_t t, int64_t target) {
@@ -273,16 +272,21 @@ sample_count_kernel(const SampleArgs a) {
   }
 }
 
-// Edges of FT targets (FT divides CT, the targets per CTA of the count kernel).
+// Edges of FT targets (FT divides CT, the targets per CTA of the count kernel).  Up to kMapFanout edges per target, shared memory
+// says for every output element which target it belongs to and, where targets draw, which candidate it is, in output order: the
+// copy loop is then a handful of instructions around its three loads.  (It was issue bound: 100 - 170 instructions per edge,
+// 384,000 x 20 recent 101 us, a drawn hop of 4.2 M x 10 targets 458 us.)
+constexpr int kMapFanout = 32;
 template <int CT, int FT>
 __global__ void __launch_bounds__(kCtaThreads)
 sample_fill_kernel(const SampleArgs a, int count_ctas) {
   static_assert(CT % FT == 0 && CT <= kCtaThreads && FT % kWarpsPerCta == 0, "fill CTAs tile the count CTAs");
   constexpr bool kLaneDraws = CT != kWarpsPerCta;          // picks by the target's lane instead of its warp
-  extern __shared__ uint64_t s_dyn[];                      // picks of the targets that draw, target of every element
+  constexpr uint32_t kNotHere = ~0u;                       // (a candidate window this large is drawn from by a warp, below)
+  constexpr int64_t kDrawn = INT64_MIN;
+  extern __shared__ uint64_t s_dyn[];
   __shared__ int32_t s_ex[FT + 1];   // offset of the target's first element inside the CTA's output; [FT] = end
-  __shared__ int32_t s_cnt[FT];
-  __shared__ int64_t s_lo[FT], s_cut[FT], s_t[FT];
+  __shared__ int64_t s_src[FT], s_t[FT];                   // what a candidate number, or an output position, is added to
   __shared__ int64_t s_base[kWarpsPerCta];
   const int64_t n = eff_count(a.n_cap, a.d_n);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -293,7 +297,7 @@ sample_fill_kernel(const SampleArgs a, int count_ctas) {
   const bool direct = count_ctas <= kDirectCtas;
   const int slot = (int)threadIdx.x - sub;
   const int64_t i = count_cta * CT + threadIdx.x;
-  const bool in_ct = threadIdx.x < CT && i < n, mine = slot >= 0 && slot < FT;
+  const bool in_ct = threadIdx.x < CT && i < n, mine = slot >= 0 && slot < FT && threadIdx.x < CT;
   const int c = in_ct ? a.cnt[i] : 0;
   int64_t lo = 0, cut = 0, t = 0;
   if (mine && in_ct) {
@@ -322,16 +326,12 @@ sample_fill_kernel(const SampleArgs a, int count_ctas) {
     base = a.cta_sums[count_cta];
     if (threadIdx.x == 0 && first + FT >= a.n_cap && a.total_out) *a.total_out = a.out_offsets[a.n_cap];
   }
-  const bool draws = a.policy == SGL_POLICY_UNIFORM;
-  uint32_t* s_pick = (uint32_t*)s_dyn;     // [fanout][FT]
-  const bool lane_draws = kLaneDraws && draws && fanout <= 32;
-  const bool has_map = fanout <= 32;       // which target every output element belongs to, behind the picks
-  uint8_t* s_map = (uint8_t*)(s_pick + (lane_draws ? FT * fanout : 0));
-  if (mine && threadIdx.x < CT) {
+  const bool draws = a.policy == SGL_POLICY_UNIFORM, has_map = fanout <= kMapFanout;
+  const bool drawn = draws && cut - lo > fanout;           // (of this thread's target)
+  if (mine) {
     s_ex[slot] = ex;
-    s_cnt[slot] = c;
-    s_lo[slot] = lo;
-    s_cut[slot] = cut;
+    // recent: tail of the window; uniform with no more candidates than edges: the whole window
+    s_src[slot] = has_map && draws ? lo : (drawn ? kDrawn : cut - c - ex);
     s_t[slot] = t;
     if (slot == FT - 1) s_ex[FT] = ex + c;
     // offsets past the valid targets all equal the total, so out_offsets[n..n_cap] stays a valid prefix array
@@ -339,89 +339,109 @@ sample_fill_kernel(const SampleArgs a, int count_ctas) {
   }
   __syncthreads();
   const int begin = s_ex[0], end = s_ex[FT];
-  if (mine && threadIdx.x < CT) {
-    if (has_map)
-      for (int j = 0; j < c; ++j) s_map[ex - begin + j] = (uint8_t)slot;
-    if (lane_draws) {
-      const int64_t cand = cut - lo;
-      if (cand > fanout && cand <= 0xffffffffll && fanout <= kRegPicks) {
-        draw_sorted<FT>(i, (uint32_t)cand, fanout, a.rng_stream, a.seed, s_pick + slot);
-      } else if (cand > fanout && cand <= 0xffffffffll) {
-        for (int d = 0; d < fanout; ++d) {
-          const uint32_t top = (uint32_t)(cand - fanout + d);
-          uint32_t pick = draw_below_u32(i, d, a.rng_stream, a.seed, top + 1u);
-          bool clash = false;
-          for (int q = 0; q < d; ++q) clash |= s_pick[q * FT + slot] == pick;
-          s_pick[d * FT + slot] = clash ? top : pick;
+  const int64_t out0 = base + begin;
+  bool left = draws;                                       // targets that draw are left for the warps
+  if (has_map) {
+    uint32_t* s_pos = (uint32_t*)s_dyn;                    // [FT * fanout] candidate of every element, where targets draw
+    uint8_t* s_map = (uint8_t*)(s_pos + (draws ? FT * fanout : 0));
+    if (kLaneDraws) {
+      if (mine) {
+        const int e0 = ex - begin;
+        for (int j = 0; j < c; ++j) s_map[e0 + j] = (uint8_t)slot;
+        if (draws) {
+          const int64_t cand = cut - lo;
+          if (!drawn || cand > 0xffffffffll) {
+            for (int j = 0; j < c; ++j) s_pos[e0 + j] = drawn ? kNotHere : (uint32_t)j;
+          } else if (fanout <= kRegPicks) {
+            draw_sorted(i, (uint32_t)cand, fanout, a.rng_stream, a.seed, s_pos + e0);
+          } else {
+            for (int d = 0; d < fanout; ++d) {
+              const uint32_t top = (uint32_t)(cand - fanout + d);
+              uint32_t pick = draw_below_u32(i, d, a.rng_stream, a.seed, top + 1u);
+              bool clash = false;
+              for (int q = 0; q < d; ++q) clash |= s_pos[e0 + q] == pick;
+              if (clash) pick = top;
+              int q = d;                                   // ascending
+              for (; q > 0 && s_pos[e0 + q - 1] > pick; --q) s_pos[e0 + q] = s_pos[e0 + q - 1];
+              s_pos[e0 + q] = pick;
+            }
+          }
         }
       }
+    } else {
+      // one warp per target
+      const int e0 = s_ex[warp] - begin, cw = s_ex[warp + 1] - s_ex[warp];
+      if (lane < cw) s_map[e0 + lane] = (uint8_t)warp;
+      if (draws) {
+        const int64_t wcand = __shfl_sync(0xffffffffu, lane == 0 && first + warp < n ? a.win_cut[first + warp] - a.win_lo[first + warp] : 0, 0);
+        if (wcand <= fanout || wcand > 0xffffffffll) {
+          if (lane < cw) s_pos[e0 + lane] = wcand <= fanout ? (uint32_t)lane : kNotHere;
+        } else {
+          uint32_t pick = 0;
+          if (lane < fanout) pick = draw_below_u32(first + warp, lane, a.rng_stream, a.seed, (uint32_t)(wcand - fanout + lane) + 1u);
+          for (int d = 1; d < fanout; ++d) {
+            const uint32_t other = __shfl_sync(0xffffffffu, pick, d);
+            const bool clash = __any_sync(0xffffffffu, lane < d && pick == other);
+            if (clash && lane == d) pick = (uint32_t)(wcand - fanout + d);
+          }
+          int rank = 0;                                    // ascending
+          for (int d = 0; d < fanout; ++d) rank += __shfl_sync(0xffffffffu, pick, d) < pick ? 1 : 0;
+          if (lane < fanout) s_pos[e0 + rank] = pick;
+        }
+      }
+    }
+    left = __syncthreads_or(mine && drawn && cut - lo > 0xffffffffll);
+    // one output element per thread: all lanes busy, stores coalesced; the loads of kFillUnroll elements of a thread are in
+    // flight together
+    const int m = end - begin;
+    for (int o0 = (int)threadIdx.x; o0 < m; o0 += kCtaThreads * kFillUnroll) {
+      int at[kFillUnroll];
+      int64_t ets[kFillUnroll], nb[kFillUnroll], ei[kFillUnroll];
+#pragma unroll
+      for (int u = 0; u < kFillUnroll; ++u) {
+        const int o = o0 + u * kCtaThreads;
+        at[u] = -1;
+        if (o >= m) continue;
+        const int k = s_map[o];
+        uint32_t off = (uint32_t)(o + begin);
+        if (draws) off = s_pos[o];
+        if (draws && off == kNotHere) continue;
+        const int64_t p = s_src[k] + off;
+        at[u] = k;
+        ets[u] = __ldg(a.ts + p);
+        nb[u] = __ldg(a.nbr + p);
+        ei[u] = __ldg(a.eid + p);
+      }
+#pragma unroll
+      for (int u = 0; u < kFillUnroll; ++u) {
+        if (at[u] < 0) continue;
+        const int64_t g = out0 + (o0 + u * kCtaThreads), tt = s_t[at[u]];
+        a.out_nbr[g] = nb[u];
+        a.out_eid[g] = ei[u];
+        a.out_ts[g] = a.keep_root_time ? tt : ets[u];
+        a.out_dt[g] = (float)(tt - ets[u]);
+        if (a.out_dt_i64) a.out_dt_i64[g] = ets[u] - tt;
+        a.out_dst[g] = first + at[u];
+      }
+    }
+  } else {
+    for (int o = begin + (int)threadIdx.x; o < end; o += kCtaThreads) {
+      int k = 0, b = FT;                   // last slot with s_ex[slot] <= o (its next offset is > o, so it is not empty)
+      while (b - k > 1) {
+        const int m = (k + b) >> 1;
+        if (s_ex[m] <= o) k = m; else b = m;
+      }
+      if (s_src[k] != kDrawn) emit_edge(a, s_src[k] + o, base + o, s_t[k], first + k);
     }
   }
-  __syncthreads();
-  // one output element per thread: all lanes busy, stores coalesced; the loads of kFillUnroll elements of a thread are in
-  // flight together
-  for (int o0 = begin + (int)threadIdx.x; o0 < end; o0 += kCtaThreads * kFillUnroll) {
-    int at[kFillUnroll];
-    int64_t g[kFillUnroll], ets[kFillUnroll], nb[kFillUnroll], ei[kFillUnroll];
-#pragma unroll
-    for (int u = 0; u < kFillUnroll; ++u) {
-      const int o = o0 + u * kCtaThreads;
-      at[u] = -1;
-      if (o >= end) continue;
-      int k;
-      if (has_map) {
-        k = s_map[o - begin];
-      } else {
-        k = 0;
-        int b = FT;                      // last slot with s_ex[slot] <= o (its next offset is > o, so it is not empty)
-        while (b - k > 1) {
-          const int m = (k + b) >> 1;
-          if (s_ex[m] <= o) k = m; else b = m;
-        }
-      }
-      const int64_t wlo = s_lo[k], wcut = s_cut[k];
-      int64_t p;
-      if (draws && wcut - wlo > fanout) {
-        if (!lane_draws || wcut - wlo > 0xffffffffll) continue;
-        const uint32_t pick = s_pick[(o - s_ex[k]) * FT + k];
-        int rank = o - s_ex[k];
-        if (fanout > kRegPicks) {
-          rank = 0;
-          for (int q = 0; q < fanout; ++q) rank += s_pick[q * FT + k] < pick ? 1 : 0;
-        }
-        p = wlo + pick;
-        g[u] = base + s_ex[k] + rank;
-      } else {
-        // recent: tail of the window; uniform with cand <= k: the whole window
-        p = wcut - s_cnt[k] + (o - s_ex[k]);
-        g[u] = base + o;
-      }
-      at[u] = k;
-      ets[u] = __ldg(a.ts + p);
-      nb[u] = __ldg(a.nbr + p);
-      ei[u] = __ldg(a.eid + p);
-    }
-#pragma unroll
-    for (int u = 0; u < kFillUnroll; ++u) {
-      if (at[u] < 0) continue;
-      const int64_t tt = s_t[at[u]];
-      a.out_nbr[g[u]] = nb[u];
-      a.out_eid[g[u]] = ei[u];
-      a.out_ts[g[u]] = a.keep_root_time ? tt : ets[u];
-      a.out_dt[g[u]] = (float)(tt - ets[u]);
-      if (a.out_dt_i64) a.out_dt_i64[g[u]] = ets[u] - tt;
-      a.out_dst[g[u]] = first + at[u];
-    }
-  }
-  if (!draws) return;
+  if (!left) return;
   // targets that draw and were not served above: one warp per target
 #pragma unroll 1
   for (int wslot = warp; wslot < FT; wslot += kWarpsPerCta) {
     const int64_t i = first + wslot;
     if (i >= n) break;
-    const int64_t lo = s_lo[wslot], cut = s_cut[wslot];
-    const int64_t cand = cut - lo;
-    if (cand <= fanout || (lane_draws && cand <= 0xffffffffll)) continue;
+    const int64_t lo = a.win_lo[i], cand = a.win_cut[i] - lo;
+    if (cand <= fanout || (has_map && cand <= 0xffffffffll)) continue;
     const int64_t t = s_t[wslot];
     const int64_t off = base + s_ex[wslot];
     if (fanout > 32) {
@@ -498,10 +518,10 @@ static int launch_sample(const SampleArgs& a, cudaStream_t stream) {
   SGL_CHECK_RC(launch(sample_count_kernel<CT, WIDE>, ctas, kCtaThreads, 0, stream, a));
   size_t smem = 0;
   if (a.policy == SGL_POLICY_UNIFORM) {
-    if (a.fanout > 32) smem = (size_t)kWarpsPerCta * a.fanout * sizeof(uint64_t);
-    else if (CT != kWarpsPerCta) smem = (size_t)FT * a.fanout * sizeof(uint32_t);
+    if (a.fanout > kMapFanout) smem = (size_t)kWarpsPerCta * a.fanout * sizeof(uint64_t);
+    else smem = (size_t)FT * a.fanout * sizeof(uint32_t);
   }
-  if (a.fanout <= 32) smem += (size_t)FT * a.fanout;
+  if (a.fanout <= kMapFanout) smem += (size_t)FT * a.fanout;
   SGL_CHECK_RC(launch(sample_fill_kernel<CT, FT>, (unsigned)((a.n_cap + FT - 1) / FT), kCtaThreads, smem, stream, a,
                       (int)ctas));
   return SGL_OK;

@@ -126,6 +126,15 @@ int sgl_sample_layer_fenced(const int64_t* indptr, const int64_t* nbr, const int
                             int64_t allowed_offset, int keep_root_time, uint64_t seed, uint32_t rng_stream, int64_t* out_nbr,
                             int64_t* out_dst, int64_t* out_ts, float* out_dt, int64_t* out_dt_i64, int64_t* out_eid,
                             int64_t* out_offsets, int32_t* d_status, void* ws, size_t ws_bytes, void* stream);
+/* sgl_sample_layer_fenced; the number of sampled edges and behind it `seq` also go to host_total[0..1] (pinned; NULL or a
+ * capturing stream: not written, see sgl_wait_word) as soon as they are counted. */
+int sgl_sample_layer_counted(const int64_t* indptr, const int64_t* nbr, const int64_t* ts, const int64_t* eid,
+                             const int64_t* fence, int64_t num_nodes, const int64_t* targets, const int64_t* target_ts,
+                             int64_t n_targets, const int64_t* d_n, int fanout, int policy, int equal_root_time,
+                             int64_t allowed_offset, int keep_root_time, uint64_t seed, uint32_t rng_stream, int64_t* out_nbr,
+                             int64_t* out_dst, int64_t* out_ts, float* out_dt, int64_t* out_dt_i64, int64_t* out_eid,
+                             int64_t* out_offsets, int32_t* d_status, void* ws, size_t ws_bytes, int64_t* host_total,
+                             int64_t seq, void* stream);
 int sgl_sample_gather_fenced(const int64_t* indptr, const int64_t* nbr, const int64_t* ts, const int64_t* eid,
                              const int64_t* fence, int64_t num_nodes, const int64_t* targets, const int64_t* target_ts,
                              int64_t n_targets, int fanout, int policy, int equal_root_time, int64_t allowed_offset,

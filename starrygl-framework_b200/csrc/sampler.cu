@@ -484,6 +484,20 @@ sample_fill_kernel(const SampleArgs a, int count_ctas) {
   }
 }
 
+// number of sampled edges -> pinned host memory, then `seq` behind it; sums: one per count CTA
+__global__ void __launch_bounds__(kCtaThreads)
+export_total_kernel(const int64_t* __restrict__ sums, int count, int64_t* host, int64_t seq) {
+  int64_t x = 0;
+  for (int i = threadIdx.x; i < count; i += kCtaThreads) x += sums[i];
+  int64_t total;
+  cta_exclusive_scan<kCtaThreads, int64_t>(x, &total);
+  if (threadIdx.x == 0) {
+    *(volatile int64_t*)host = total;
+    __threadfence_system();
+    *(volatile int64_t*)(host + 1) = seq;
+  }
+}
+
 // roots and query times of a mini-batch out of pinned host memory
 __global__ void __launch_bounds__(256)
 stage_roots_kernel(const int64_t* __restrict__ roots, const int64_t* __restrict__ times, int64_t n, int64_t* __restrict__ d_roots,
@@ -512,10 +526,19 @@ extern "C" size_t sgl_sample_ws_bytes(int64_t n_targets) {
 }
 
 template <int CT, int FT, bool WIDE>
-static int launch_sample(const SampleArgs& a, cudaStream_t stream) {
+static int launch_sample(const SampleArgs& a, cudaStream_t stream, int64_t* host_total, int64_t seq) {
   const unsigned ctas = (unsigned)((a.n_cap + CT - 1) / CT);
   if (ctas > kDirectCtas) SGL_CHECK_RC(zero_async(a.done, sizeof(unsigned int), stream));
   SGL_CHECK_RC(launch(sample_count_kernel<CT, WIDE>, ctas, kCtaThreads, 0, stream, a));
+  LaunchScope* in = LaunchScope::current();
+  if (host_total && in) {
+    // on its way while the edges are copied (a second chain of the graph)
+    cudaStream_t side = (cudaStream_t)(uintptr_t)3;
+    in->wait(side, in->mark(stream));
+    const bool direct = ctas <= kDirectCtas;
+    SGL_CHECK_RC(launch(export_total_kernel, 1, kCtaThreads, 0, side, direct ? a.cta_sums : a.out_offsets + a.n_cap, direct ? (int)ctas : 1,
+                        host_total, seq));
+  }
   size_t smem = 0;
   if (a.policy == SGL_POLICY_UNIFORM) {
     if (a.fanout > kMapFanout) smem = (size_t)kWarpsPerCta * a.fanout * sizeof(uint64_t);
@@ -532,7 +555,7 @@ int sgl::sample_layer(const int64_t* indptr, const int64_t* nbr, const int64_t* 
                       int fanout, int policy, int equal_root_time, int64_t allowed_offset, int keep_root_time, uint64_t seed,
                       uint32_t rng_stream, int64_t* out_nbr, int64_t* out_dst, int64_t* out_ts, float* out_dt, int64_t* out_dt_i64,
                       int64_t* out_eid, int64_t* out_offsets, int64_t* total_out, int32_t* d_status, void* ws, size_t ws_bytes,
-                      void* stream_) {
+                      void* stream_, int64_t* host_total, int64_t seq) {
   SGL_NVTX("sgl_sample_layer");
   cudaStream_t stream = (cudaStream_t)stream_;
   SGL_REQUIRE(n_targets >= 0 && num_nodes >= 0, SGL_ERR_ARG, "sample_layer: negative size");
@@ -546,6 +569,10 @@ int sgl::sample_layer(const int64_t* indptr, const int64_t* nbr, const int64_t* 
   if (n_targets == 0) {
     SGL_CHECK_RC(zero_async(out_offsets, sizeof(int64_t), stream));
     if (total_out) SGL_CHECK_RC(zero_async(total_out, sizeof(int64_t), stream));
+    if (host_total) {
+      host_total[0] = 0;
+      host_total[1] = seq;
+    }
     return SGL_OK;
   }
   SGL_REQUIRE(indptr && nbr && ts && eid && targets && target_ts && out_nbr && out_dst && out_ts && out_dt && out_eid,
@@ -575,15 +602,15 @@ int sgl::sample_layer(const int64_t* indptr, const int64_t* nbr, const int64_t* 
               sgl_sample_ws_bytes(n_targets));
   LaunchScope scope(stream);
   if (n_targets <= kWarpTargets) {
-    SGL_CHECK_RC((launch_sample<kWarpsPerCta, kWarpsPerCta, true>(a, stream)));
+    SGL_CHECK_RC((launch_sample<kWarpsPerCta, kWarpsPerCta, true>(a, stream, host_total, seq)));
   } else if (policy == SGL_POLICY_UNIFORM) {
     // targets per fill CTA: a lane of the CTA draws for every target, so as many as there are threads once that leaves
     // several CTAs per SM; windows that are copied are spread thinner
-    if (n_targets < kManyTargets) SGL_CHECK_RC((launch_sample<kCtaThreads, 128, true>(a, stream)));
-    else SGL_CHECK_RC((launch_sample<kCtaThreads, 256, false>(a, stream)));
+    if (n_targets < kManyTargets) SGL_CHECK_RC((launch_sample<kCtaThreads, 128, true>(a, stream, host_total, seq)));
+    else SGL_CHECK_RC((launch_sample<kCtaThreads, 256, false>(a, stream, host_total, seq)));
   } else {
-    if (n_targets < kManyTargets) SGL_CHECK_RC((launch_sample<kCtaThreads, 64, true>(a, stream)));
-    else SGL_CHECK_RC((launch_sample<kCtaThreads, 64, false>(a, stream)));
+    if (n_targets < kManyTargets) SGL_CHECK_RC((launch_sample<kCtaThreads, 64, true>(a, stream, host_total, seq)));
+    else SGL_CHECK_RC((launch_sample<kCtaThreads, 64, false>(a, stream, host_total, seq)));
   }
   return scope.submit();
 }
@@ -598,6 +625,18 @@ extern "C" int sgl_sample_layer(const int64_t* indptr, const int64_t* nbr, const
   return sgl::sample_layer(indptr, nbr, ts, eid, nullptr, num_nodes, targets, target_ts, n_targets, d_n, fanout, policy,
                            equal_root_time, allowed_offset, keep_root_time, seed, rng_stream, out_nbr, out_dst, out_ts, out_dt,
                            out_dt_i64, out_eid, out_offsets, nullptr, d_status, ws, ws_bytes, stream);
+}
+
+extern "C" int sgl_sample_layer_counted(const int64_t* indptr, const int64_t* nbr, const int64_t* ts, const int64_t* eid,
+                                        const int64_t* fence, int64_t num_nodes, const int64_t* targets, const int64_t* target_ts,
+                                        int64_t n_targets, const int64_t* d_n, int fanout, int policy, int equal_root_time,
+                                        int64_t allowed_offset, int keep_root_time, uint64_t seed, uint32_t rng_stream,
+                                        int64_t* out_nbr, int64_t* out_dst, int64_t* out_ts, float* out_dt, int64_t* out_dt_i64,
+                                        int64_t* out_eid, int64_t* out_offsets, int32_t* d_status, void* ws, size_t ws_bytes,
+                                        int64_t* host_total, int64_t seq, void* stream) {
+  return sgl::sample_layer(indptr, nbr, ts, eid, fence, num_nodes, targets, target_ts, n_targets, d_n, fanout, policy,
+                           equal_root_time, allowed_offset, keep_root_time, seed, rng_stream, out_nbr, out_dst, out_ts, out_dt,
+                           out_dt_i64, out_eid, out_offsets, nullptr, d_status, ws, ws_bytes, stream, host_total, seq);
 }
 
 extern "C" int sgl_sample_layer_fenced(const int64_t* indptr, const int64_t* nbr, const int64_t* ts, const int64_t* eid,
@@ -659,12 +698,7 @@ extern "C" int sgl_prefetch_batch(const int64_t* host_roots, const int64_t* host
                         target_ts));
   SGL_CHECK_RC(sgl::sample_layer(indptr, nbr, ts, eid, fence, num_nodes, targets, target_ts, n_targets, nullptr, fanout, policy,
                                  equal_root_time, allowed_offset, keep_root_time, seed, rng_stream, out_nbr, out_dst, out_ts, out_dt,
-                                 nullptr, out_eid, out_offsets, nullptr, d_status, ws, ws_bytes, stream));
-  // the count is on its way while the rows are gathered (a second chain of the graph)
-  LaunchScope* in = LaunchScope::current();
-  cudaStream_t side = in ? (cudaStream_t)(uintptr_t)3 : stream;
-  if (in) in->wait(side, in->mark(stream));
-  SGL_CHECK_RC(launch(export_words_kernel, 1, 32, 0, side, out_offsets + n_targets, host_total, 1, seq));
+                                 nullptr, out_eid, out_offsets, nullptr, d_status, ws, ws_bytes, stream, host_total, seq));
   if (out_feats && n_targets > 0)
     SGL_CHECK_RC(sgl_gather_rows(feat_table, feat_rows, row_bytes, src_pitch, out_eid, nullptr, 0, n_targets * fanout,
                                  out_offsets + n_targets, out_feats, row_bytes, nullptr, nullptr, gather_mode, d_status, stream));

@@ -6,6 +6,7 @@ worker threads the way the reference's pybind module is (csrc/srcs/starrygl/expo
 ``py::gil_scoped_release`` on every heavy binding).
 """
 import ctypes as C
+import itertools
 import os
 import threading
 
@@ -42,6 +43,8 @@ _SIGNATURES = {
     "sgl_tcsr_fence": (_i32, [_vp, _vp, _i64, _i64, _vp, _vp]),
     "sgl_sample_layer_fenced": (_i32, [_vp, _vp, _vp, _vp, _vp, _i64, _vp, _vp, _i64, _vp, _i32, _i32, _i32, _i64, _i32, _u64, _u32,
                                        _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _sz, _vp]),
+    "sgl_sample_layer_counted": (_i32, [_vp, _vp, _vp, _vp, _vp, _i64, _vp, _vp, _i64, _vp, _i32, _i32, _i32, _i64, _i32, _u64,
+                                         _u32, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _sz, _vp, _i64, _vp]),
     "sgl_sample_layer_static": (_i32, [_vp, _vp, _vp, _vp, _i64, _vp, _vp, _i64, _i32, _i32, _i32, _i64, _i32, _u64, _u32,
                                        _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp]),
     "sgl_sample_gather": (_i32, [_vp, _vp, _vp, _vp, _i64, _vp, _vp, _i64, _i32, _i32, _i32, _i64, _i32, _u64, _u32,
@@ -188,6 +191,41 @@ def host_words():
         check(lib().sgl_host_words(C.byref(p)))
         h = _HOST.__dict__["words"] = (p.value, (C.c_int64 * 512).from_address(p.value))
     return h
+
+
+class CountRing:
+    """Pinned (value, sequence number) pairs that kernels fill in with a count the host may ask for later.  A pair is used
+    again after as many calls as there are pairs; who still wants the older count reads it from the device."""
+    SLOTS = 1024
+
+    def __init__(self):
+        self._seq = itertools.count(1)       # (one call of next() is atomic)
+        self._lock = threading.Lock()
+        self._buf = self._words = None
+
+    def take(self):
+        """(address, index of the value, sequence number)"""
+        if self._buf is None:
+            with self._lock:
+                if self._buf is None:
+                    buf = torch.zeros(2 * self.SLOTS, dtype=torch.int64).pin_memory()
+                    self._words = (C.c_int64 * (2 * self.SLOTS)).from_address(buf.data_ptr())
+                    self._base, self._buf = buf.data_ptr(), buf
+        seq = next(self._seq)
+        i = 2 * (seq % self.SLOTS)
+        return self._base + 8 * i, i, seq
+
+    def value(self, taken, stream):
+        """The count, or None when its pair was used again (or never filled in)."""
+        addr, i, seq = taken
+        w = self._words
+        if w[i + 1] < seq:
+            lib().sgl_wait_word(addr + 8, seq, stream)
+        v = w[i]
+        return v if w[i + 1] == seq else None
+
+
+COUNTS = CountRing()
 
 
 def read_words(t, count):

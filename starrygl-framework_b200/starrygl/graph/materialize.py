@@ -28,7 +28,10 @@ _PINNED_MOST, _PINNED_TOTAL = 256 << 20, 2 << 30
 
 def _pinned_now() -> int:
     """Bytes of pinned memory in use through torch's host allocator."""
-    return int(torch.cuda.host_memory_stats().get("allocated_bytes.current", 0))
+    try:
+        return int(torch._C._cuda_hostMemoryStats()["allocated_bytes"]["current"])      # (a tenth of the cost of the flat form)
+    except (AttributeError, KeyError, TypeError):
+        return int(torch.cuda.host_memory_stats().get("allocated_bytes.current", 0))
 
 
 def _dev_i64(x, dev):

@@ -86,7 +86,7 @@ class mailbox:
         its latest entry (reference: mailbox.py:56-84).  One host synchronisation, to size the results exactly."""
         index, mail, mail_ts, d_n = self.get_update_mail_async(src, dst, ts, edge_feats, mem_src, mem_dst, embedding,
                                                                use_src_emb, use_dst_emb)
-        u = int(d_n.item())
+        u = _C.read_words(d_n, 1)[0]
         return index[:u], mail[:u], mail_ts[:u]
 
     # ---- writes ------------------------------------------------------------------------------------------------
@@ -123,6 +123,9 @@ class mailbox:
         """(mailbox[idx], mailbox_ts[idx]) through the row-gather kernel."""
         idx = idx.to(self.device)
         n, s, w = self.shape
+        if s == 1:                      # one launch: the timestamps are a plain vector
+            rows, ts = ops.gather_rows(self.mailbox.view(n, w), idx, ts_table=self.mailbox_ts.view(n), status=self._status)
+            return rows.view(-1, 1, w), ts.view(-1, 1)
         rows = ops.gather_rows(self.mailbox.view(n, s * w), idx, status=self._status).view(-1, s, w)
         ts = ops.gather_rows(self.mailbox_ts, idx, status=self._status)
         return rows, ts

@@ -117,6 +117,7 @@ class Hop:
     offsets: torch.Tensor      # [n_targets + 1]
     capacity: int
     dt_i64: Optional[torch.Tensor] = None   # ts - t (int64), only when asked for
+    count: Optional[tuple] = None           # where the number of sampled edges reaches the host, and the stream
 
     @property
     def d_total(self):
@@ -124,7 +125,11 @@ class Hop:
         return self.offsets[-1:]
 
     def total(self) -> int:
-        """Number of sampled edges (synchronises)."""
+        """Number of sampled edges (waits until they are counted)."""
+        if self.count is not None:
+            v = _C.COUNTS.value(*self.count)
+            if v is not None:
+                return v
         return int(self.offsets[-1].item())
 
     def trimmed(self):
@@ -149,13 +154,14 @@ def sample_layer(g: TCSR, targets, target_ts, fanout: int, policy="recent", *, d
     o_dti = torch.empty(cap, dtype=I64, device=dev) if want_dt_i64 else None
     pol = _C.POLICY[policy] if isinstance(policy, str) else int(policy)
     _, wp, wn = _C.workspace(L.sgl_sample_ws_bytes(n), dev)
-    _C.check(L.sgl_sample_layer_fenced(_C.ptr(g.indptr), _C.ptr(g.nbr), _C.ptr(g.ts), _C.ptr(g.eid), _C.ptr(g.fence), g.num_nodes,
+    taken, stream = _C.COUNTS.take(), _C.stream_ptr()
+    _C.check(L.sgl_sample_layer_counted(_C.ptr(g.indptr), _C.ptr(g.nbr), _C.ptr(g.ts), _C.ptr(g.eid), _C.ptr(g.fence), g.num_nodes,
                                 _C.ptr(targets), _C.ptr(target_ts), n, _C.ptr(d_n), int(fanout), pol,
                                 int(bool(equal_root_time)), int(allowed_offset), int(bool(keep_root_time)),
                                 int(seed) & (2 ** 64 - 1), int(rng_stream) & 0xFFFFFFFF, _C.ptr(o_nbr), _C.ptr(o_dst),
                                 _C.ptr(o_ts), _C.ptr(o_dt), _C.ptr(o_dti), _C.ptr(o_eid), _C.ptr(offs),
-                                status.ptr() if status else None, wp, wn, _C.stream_ptr()))
-    return Hop(o_nbr, o_dst, o_ts, o_dt, o_eid, offs, cap, o_dti)
+                                status.ptr() if status else None, wp, wn, taken[0], taken[2], stream))
+    return Hop(o_nbr, o_dst, o_ts, o_dt, o_eid, offs, cap, o_dti, (taken, stream))
 
 
 # --------------------------------------------------------------------------------------------------------------

@@ -98,7 +98,7 @@ class MaterializedMultiLayerBuilder:
             return f(node_parts), f(ts_parts), None
         n, total = sum(len(x) for x in parts[:len(node_parts)]), sum(len(x) for x in parts)
         if self._stage is None or self._stage.numel() < total:
-            self._stage = torch.empty(max(2 * total, 1024), dtype=torch.int64).pin_memory()
+            self._stage = torch.empty(max(2 * total, 1024), dtype=torch.int64, pin_memory=True)
         st, at = self._stage.numpy(), 0
         for x in parts:
             st[at:at + len(x)] = x

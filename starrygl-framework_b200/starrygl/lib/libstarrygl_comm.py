@@ -16,6 +16,7 @@ ts >= t - allowed_offset when ``allowed_offset`` >= 0); "recent" keeps the last 
 k distinct ones in ascending position; ``neighbors_dt`` = ts - t as int64; hop l+1 queries every neighbour of
 hop l at the time of the edge that reached it (or at the root's time with ``keep_root_time``).
 """
+import ctypes as C
 import queue
 import threading
 from bisect import bisect_left
@@ -314,7 +315,7 @@ class _QueryFuture:
         n = 10 + 2 * hops
         _C.check(_C.lib().sgl_wait_word(addr + 8 * n, 1, g.stream.cuda_stream))
         meta = words[:n]
-        g._slots.append(self.slot)
+        _FREE_SLOTS.append(self.slot)
         bits = meta[5] & 0xFFFFFFFF
         if bits:
             raise _C.SglError(f"submit_query: device status {bits} ({_C.decode_status(bits)})")
@@ -356,6 +357,12 @@ def query_blocks(root, neg_roots, neighbors):
     return blocks
 
 
+# Free pinned result words of queries, (address, ctypes array); as many as queries were ever in flight together, kept for the next
+# graph (pinning memory takes a millisecond).
+_FREE_SLOTS: list = []
+_SLOT_BLOCKS: list = []
+
+
 class CUDAGraph:
     """Temporal graph on one GPU + an asynchronous sampling queue (FIFO results)."""
 
@@ -372,7 +379,6 @@ class CUDAGraph:
         self._worker = None               # started by the first task that has to wait for the GPU on the way
         self._pending = 0                 # tasks that the worker has not finished
         self._lock = threading.Lock()
-        self._slots = []                  # free pinned result words, (address, ctypes array)
         self._ev_index = None
         self._plans = {}
 
@@ -479,7 +485,7 @@ class CUDAGraph:
     def _window(self, t0, t1):
         """Host-known bounds of the window's events: (first, at most) from every 256th timestamp of the stream."""
         if self._ev_index is None:
-            self._ev_index = self.ev[1][::256].tolist()
+            self._ev_index = self.ev[1][::256].cpu().numpy()
         idx, m = self._ev_index, self.ev[1].numel()
         first = max(bisect_left(idx, t0) - 1, 0) * 256
         last = min(bisect_left(idx, t1) * 256, m)
@@ -487,15 +493,16 @@ class CUDAGraph:
             first, last = min(first, m - 1), min(first, m - 1) + 1
         return first, last - first
 
-    def _slot(self):
-        if not self._slots:
-            import ctypes as C
-            block = torch.empty(64 * 32, dtype=torch.int64).pin_memory()
-            self._slot_blocks = getattr(self, "_slot_blocks", []) + [block]
-            for i in range(64):
-                addr = block.data_ptr() + 256 * i
-                self._slots.append((addr, (C.c_int64 * 32).from_address(addr)))
-        return self._slots.pop()
+    @staticmethod
+    def _slot():
+        try:
+            return _FREE_SLOTS.pop()
+        except IndexError:
+            block = torch.zeros(64 * 32, dtype=torch.int64, pin_memory=True)
+            _SLOT_BLOCKS.append(block)
+            new = [(block.data_ptr() + 256 * i, (C.c_int64 * 32).from_address(block.data_ptr() + 256 * i)) for i in range(64)]
+            _FREE_SLOTS.extend(new[1:])
+            return new[0]
 
     def _enqueue(self, t0, t1, chunks, neg, stype, layers, fanout, off, eq, keep, op) -> Optional[_QueryFuture]:
         g = self.g

@@ -38,6 +38,7 @@ struct PairSink {
   int64_t ts_base;
   int64_t *out_id, *out_ts, *inv_a, *inv_b, *d_n_unique;
   uint32_t *order, *row, *first;         // optional: see RowOrder
+  uint32_t* inv_b32;                     // optional: in place of inv_b
   __device__ __forceinline__ void begin() { n_a = eff_count(n_a, d_n_a); }
   __device__ __forceinline__ bool counted(uint64_t) const { return true; }
   __device__ __forceinline__ uint64_t group(uint64_t k) const { return k; }
@@ -53,6 +54,8 @@ struct PairSink {
     }
     if ((int64_t)pos < n_a) {
       if (inv_a) inv_a[pos] = u;
+    } else if (inv_b32) {
+      inv_b32[(int64_t)pos - n_a] = (uint32_t)u;
     } else if (inv_b) {
       inv_b[(int64_t)pos - n_a] = u;
     }

@@ -21,14 +21,17 @@ namespace {
 constexpr int kBits = 9;
 constexpr int kRadix = 1 << kBits;
 constexpr int kMaxPasses = 8;
-// Measured (50 M and 4.2 M keys of 44 bits, 256 - 1,024 threads, 8 - 20 keys each, 8 and 9 bits a pass): what fills the LSU data
-// pipe with two CTAs per SM is the best of them; 9 bits take five passes instead of six.
+// Measured (50 M and 4.2 M keys of 44 bits, 256 - 1,024 threads, 8 - 20 keys each, 8 and 9 bits a pass): two CTAs of 512 threads per SM
+// are the best of them; 9 bits take five passes instead of six.  A pass of 50 M keys: 480 us with a 4-byte payload, 500 us with
+// 8 bytes, 2.4 - 3.2 TB/s; the load/store pipe is busy two thirds of the time (ranks, staging), HBM half.
 constexpr int kLsdThreads = 512;
 constexpr int kLsdCtas = 2;
 constexpr int kLsdWarps = kLsdThreads / 32;
-constexpr int kLsdItems = 14;            // keys per thread
-constexpr int kLsdTile = kLsdThreads * kLsdItems;
-constexpr int kLookWide = 16;            // tiles a look-back step reads: with 4 the chain of steps was slower than the tiles
+template <class V>
+constexpr int kLsdItems = sizeof(V) == 4 ? 14 : 12;      // keys per thread; more would spill
+template <class V>
+constexpr int kLsdTile = kLsdThreads * kLsdItems<V>;
+constexpr int kLookWide = 4;               // tiles a look-back step reads
 constexpr int kHistThreads = 512;
 
 // a pass: `bits` <= kBits bits from `shift` on
@@ -41,9 +44,10 @@ struct Digit {
 // same digit (high digits of a hub, ordered input) adds once.
 template <class Items>
 __global__ void __launch_bounds__(kHistThreads)
-lsd_hist_kernel(Items items, Digit first, int passes, unsigned long long* __restrict__ hist) {
+lsd_hist_kernel(Items items, Digit first, int passes, unsigned long long* __restrict__ hist, int64_t* d_count) {
   __shared__ uint32_t s_hist[kMaxPasses * kRadix];
   const int64_t n = items.begin();
+  if (d_count && blockIdx.x == 0 && threadIdx.x == 0) *d_count = n;      // for the kernels behind the first pass
   for (int j = threadIdx.x; j < passes * kRadix; j += kHistThreads) s_hist[j] = 0;
   __syncthreads();
   constexpr int kAhead = 4;              // keys in flight per thread
@@ -86,15 +90,16 @@ static __global__ void __launch_bounds__(kRadix) lsd_scan_kernel(unsigned long l
   h[threadIdx.x] = cta_exclusive_scan<kRadix, unsigned long long>(v, nullptr);
 }
 
-// Published by a tile per digit: value, pass number + 1, and whether the value is the tile's own count or includes all
+// Published by a tile per digit: value, pass number + 1, and whether the value is the tile's own or includes all
 // tiles before it.  Words of an earlier pass count as not published, so the array is cleared once per sort.
 constexpr uint64_t kOwn = 1ull << 62, kAll = 2ull << 62, kValue = (1ull << 56) - 1;
 __device__ __forceinline__ uint64_t pass_tag(int pass) { return (uint64_t)(pass + 1) << 56; }
 constexpr unsigned long long kLookLimitNs = 2000000000ull;
 
+template <class V>
 struct LsdSmem {
   union {
-    uint64_t keys[kLsdTile];               // the tile in digit order, and after that its payload
+    uint64_t keys[kLsdTile<V>];               // the tile in digit order, and after that its payload
     uint32_t mask[kLsdWarps][kRadix];      // before that: lanes of the warp's current round that hold the digit
   };
   uint32_t cnt[kLsdWarps][kRadix];         // keys of the digit in the warp so far, then where the warp's start in the tile
@@ -103,6 +108,45 @@ struct LsdSmem {
 };
 
 // where a pass reads its items from: the arrays of the pass before, or (first pass) the producer of the keys
+// Sum of what the tiles before this one hold of digit threadIdx.x; publishes it with the tile's own.
+__device__ __forceinline__ uint64_t look_back(uint64_t* state, int pass, int tile, uint32_t total, unsigned int* gave_up, int32_t* d_status) {
+  const uint64_t tag = pass_tag(pass);
+  volatile uint64_t* st = state + threadIdx.x;
+  uint64_t sum = 0;
+  unsigned long long t0 = 0;
+  // (tiles are taken in order: those before this one are running or done)
+  for (int t = tile - 1; t >= 0;) {
+    uint64_t w[kLookWide];
+#pragma unroll
+    for (int u = 0; u < kLookWide; ++u) w[u] = t - u >= 0 ? st[(size_t)(t - u) * kRadix] : 0;
+    bool done = false, stalled = false;
+#pragma unroll
+    for (int u = 0; u < kLookWide; ++u) {
+      if (done || stalled || t < 0) continue;
+      if ((w[u] & (0x3full << 56)) != tag) {
+        stalled = true;
+        continue;
+      }
+      sum += w[u] & kValue;
+      done = (w[u] & kAll) != 0;
+      --t;
+    }
+    if (done) break;
+    if (stalled) {
+      unsigned long long now;
+      asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(now));
+      if (t0 == 0) t0 = now;
+      if (now - t0 > kLookLimitNs) {
+        dev_flag(d_status, SGL_DEV_TIMEOUT);
+        *(volatile unsigned int*)gave_up = 1u;
+        break;
+      }
+    }
+  }
+  st[(size_t)tile * kRadix] = kAll | tag | (sum + total);
+  return sum;
+}
+
 template <class V>
 struct ArrayItems {
   const uint64_t* keys;
@@ -137,18 +181,18 @@ struct SourceItems {
 template <class V, class Items, class Out>
 __global__ void __launch_bounds__(kLsdThreads, kLsdCtas)
 lsd_pass_kernel(Items items, Digit digit, int pass,
-                const unsigned long long* __restrict__ starts, unsigned int* __restrict__ ticket, uint64_t* __restrict__ state,
+                const unsigned long long* __restrict__ starts, unsigned int* __restrict__ ticket, uint64_t* state,
                 Out out, unsigned int* gave_up, int32_t* d_status) {
   extern __shared__ __align__(16) unsigned char smem[];
-  LsdSmem& sm = *(LsdSmem*)smem;
-  constexpr int kItems = kLsdItems, kTile = kLsdTile;
+  LsdSmem<V>& sm = *(LsdSmem<V>*)smem;
+  constexpr int kItems = kLsdItems<V>, kTile = kLsdTile<V>;
   const int64_t n = items.begin();
   if ((int64_t)blockIdx.x * kTile >= n) return;            // (capacity beyond the count; the others share the tickets)
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   if (tid == 0) sm.ticket = (int)atomicAdd(ticket, 1u);
-  for (int j = tid; j < kLsdWarps * kRadix; j += kLsdThreads) {
-    (&sm.mask[0][0])[j] = 0;
-    (&sm.cnt[0][0])[j] = 0;
+  for (int j = tid; j < kLsdWarps * kRadix / 4; j += kLsdThreads) {
+    ((uint4*)&sm.mask[0][0])[j] = make_uint4(0, 0, 0, 0);
+    ((uint4*)&sm.cnt[0][0])[j] = make_uint4(0, 0, 0, 0);
   }
   __syncthreads();
   const int tile = sm.ticket;
@@ -170,13 +214,25 @@ lsd_pass_kernel(Items items, Digit digit, int pass,
   for (int c = 0; c < kItems; ++c) {
     const bool valid = first + c * 32 < tile_n;
     const uint32_t d = digit.of(k[c]);
-    if (valid) atomicOr(&mask[d], 1u << lane);      // (ballots per digit bit and match_any were slower)
-    __syncwarp();
-    const uint32_t peers = valid ? mask[d] : 0u;
+    // through shared memory, or by ballots: one kind of round fills the load/store pipe, the other the integer pipe
+    const bool by_ballot = c % 3 == 0;
+    uint32_t peers;
+    if (by_ballot) {
+      peers = __ballot_sync(0xffffffffu, valid);
+#pragma unroll
+      for (int b = 0; b < kBits; ++b) {
+        const uint32_t m = __ballot_sync(0xffffffffu, (d >> b) & 1u);
+        peers &= (d >> b) & 1u ? m : ~m;
+      }
+    } else {
+      if (valid) atomicOr(&mask[d], 1u << lane);
+      __syncwarp();
+      peers = valid ? mask[d] : 0u;
+    }
     const uint32_t before = valid ? cnt[d] : 0u;
     __syncwarp();
     if (valid && (peers & below) == 0) {   // the lowest lane of the digit
-      mask[d] = 0;
+      if (!by_ballot) mask[d] = 0;
       cnt[d] = before + __popc(peers);
     }
     __syncwarp();
@@ -184,20 +240,22 @@ lsd_pass_kernel(Items items, Digit digit, int pass,
   }
   __syncthreads();
   // per digit: counts of the warps -> starts of the warps; the tile's count is published, those of the tiles before added up
+  static_assert(kRadix <= kLsdThreads && kTile < (1 << 16), "a thread per digit, 16-bit places");
   uint32_t total = 0;
   if (tid < kRadix) {
 #pragma unroll
-    for (int w = 0; w < kLsdWarps; ++w) {
-      const uint32_t c = sm.cnt[w][tid];
-      sm.cnt[w][tid] = total;
-      total += c;
-    }
-    *(volatile uint64_t*)&state[(size_t)tile * kRadix + tid] = (tile == 0 ? kAll : kOwn) | pass_tag(pass) | total;
+    for (int w = 0; w < kLsdWarps; ++w) total += sm.cnt[w][tid];
+    ((volatile uint64_t*)state)[(size_t)tile * kRadix + tid] = (tile == 0 ? kAll : kOwn) | pass_tag(pass) | total;
   }
   const uint32_t start = cta_exclusive_scan<kLsdThreads, uint32_t>(total, nullptr);
   if (tid < kRadix) {
+    uint32_t at = start;
 #pragma unroll
-    for (int w = 0; w < kLsdWarps; ++w) sm.cnt[w][tid] += start;
+    for (int w = 0; w < kLsdWarps; ++w) {
+      const uint32_t c = sm.cnt[w][tid];
+      sm.cnt[w][tid] = at;
+      at += c;
+    }
   }
   __syncthreads();
 #pragma unroll
@@ -208,42 +266,7 @@ lsd_pass_kernel(Items items, Digit digit, int pass,
     }
   }
   if (tid < kRadix) {
-    uint64_t sum = 0;
-    if (tile > 0) {
-      // (tiles are taken in order: those before this one are running or done)
-      const uint64_t tag = pass_tag(pass);
-      const volatile uint64_t* st = state + tid;
-      unsigned long long t0 = 0;
-      for (int t = tile - 1; t >= 0;) {
-        uint64_t w[kLookWide];
-#pragma unroll
-        for (int u = 0; u < kLookWide; ++u) w[u] = t - u >= 0 ? st[(size_t)(t - u) * kRadix] : 0;
-        bool done = false, stalled = false;
-#pragma unroll
-        for (int u = 0; u < kLookWide; ++u) {
-          if (done || stalled || t < 0) continue;
-          if ((w[u] & (0x3full << 56)) != tag) {
-            stalled = true;
-            continue;
-          }
-          sum += w[u] & kValue;
-          done = (w[u] & kAll) != 0;
-          --t;
-        }
-        if (done) break;
-        if (stalled) {
-          unsigned long long now;
-          asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(now));
-          if (t0 == 0) t0 = now;
-          if (now - t0 > kLookLimitNs) {
-            dev_flag(d_status, SGL_DEV_TIMEOUT);
-            *(volatile unsigned int*)gave_up = 1u;
-            break;
-          }
-        }
-      }
-      *(volatile uint64_t*)&state[(size_t)tile * kRadix + tid] = kAll | tag | (sum + total);
-    }
+    const uint64_t sum = tile > 0 ? look_back(state, pass, tile, total, gave_up, d_status) : 0;
     sm.out[tid] = (uint32_t)(starts[tid] + sum) - start;
   }
   __syncthreads();
@@ -407,38 +430,35 @@ lsd_deliver_kernel(Sink sink, const uint64_t* __restrict__ keys, const uint32_t*
   }
 }
 
-// number of items of a Source, for the kernels behind the first pass
-template <class Source>
-__global__ void source_count_kernel(Source src, int64_t* d_count) { *d_count = src.begin(); }
-
 inline int lsd_passes(int first_bit, int num_bits) { return num_bits <= first_bit + kBits ? 1 : (num_bits - first_bit + kBits - 1) / kBits; }
-inline int64_t lsd_tiles(int64_t n) { return (n + kLsdTile - 1) / kLsdTile; }
+template <class V>
+inline int64_t lsd_tiles(int64_t n) { return (n + kLsdTile<V> - 1) / kLsdTile<V>; }
 
+template <class V>
 inline size_t lsd_ws_bytes(int64_t n) {
-  return align_up((kMaxPasses * kRadix + kMaxPasses) * 8) + align_up((size_t)lsd_tiles(n < 1 ? 1 : n) * kRadix * 8);
+  return align_up((kMaxPasses * kRadix + kMaxPasses) * 8) + align_up((size_t)lsd_tiles<V>(n < 1 ? 1 : n) * kRadix * 8);
 }
 
 // Sorts on key bits [first_bit, num_bits), at least one pass; the first pass reads from `items`, writes to (k1, v1), the next to
 // (k0, v0) and so on; *in_first says whether the result ends in (k1, v1).  With a `last` of another type than ArrayOut the last
 // pass writes there instead and its arrays stay free.  **gave_up on the device: a look-back ran into its time limit, the result
-// is not to be used as positions.
+// is not to be used as positions.  d_n: number of items on the device (<= n); d_count: the count kernel writes it there, from items.
 template <class V, class Items, class Last>
-int lsd_sort(const Items& items, uint64_t* k1, V* v1, uint64_t* k0, V* v0, int64_t n, const int64_t* d_n, int first_bit, int num_bits,
+int lsd_sort(const Items& items, uint64_t* k1, V* v1, uint64_t* k0, V* v0, int64_t n, const int64_t* d_n, int64_t* d_count, int first_bit, int num_bits,
              const Last& last, bool* in_first, unsigned int** gave_up, WsCarver& c, int32_t* d_status, cudaStream_t stream) {
   using Array = ArrayOut<V>;
   constexpr bool kArray = std::is_same<Last, Array>::value;
   const int passes = lsd_passes(first_bit, num_bits);
   const int bits = num_bits > first_bit ? (num_bits - first_bit + passes - 1) / passes : 1;     // an even share each
-  const int64_t tiles = lsd_tiles(n);
+  const int64_t tiles = lsd_tiles<V>(n);
   unsigned long long* hist = c.take<unsigned long long>(kMaxPasses * kRadix + kMaxPasses);
   unsigned int* tickets = (unsigned int*)(hist + kMaxPasses * kRadix);
   *gave_up = tickets + kMaxPasses;
   uint64_t* state = c.take<uint64_t>((size_t)tiles * kRadix);
   SGL_REQUIRE(c.ok(), SGL_ERR_WORKSPACE, "radix sort: workspace too small for %lld keys", (long long)n);
-  SGL_CHECK_RC(zero_async(hist, (kMaxPasses * kRadix + kMaxPasses) * 8, stream));
-  SGL_CHECK_RC(zero_async(state, (size_t)tiles * kRadix * 8, stream));
+  SGL_CHECK_RC(zero_async(hist, (size_t)((char*)(state + (size_t)tiles * kRadix) - (char*)hist), stream));     // (one behind the other)
   SGL_CHECK_RC(launch(lsd_hist_kernel<Items>, stream_grid(n, kHistThreads * 16, 4), kHistThreads, 0, stream, items, Digit{first_bit, bits},
-                      passes, hist));
+                      passes, hist, d_count));
   SGL_CHECK_RC(launch(lsd_scan_kernel, passes, kRadix, 0, stream, hist));
   for (int p = 0; p < passes; ++p) {
     const Array out{p & 1 ? k0 : k1, p & 1 ? v0 : v1};
@@ -447,8 +467,8 @@ int lsd_sort(const Items& items, uint64_t* k1, V* v1, uint64_t* k0, V* v0, int64
       using From = std::decay_t<decltype(from)>;
       using To = std::decay_t<decltype(to)>;
       static std::atomic<uint64_t> done{0};
-      SGL_CUDA_CHECK(allow_smem((const void*)lsd_pass_kernel<V, From, To>, done, sizeof(LsdSmem)));
-      return launch(lsd_pass_kernel<V, From, To>, (unsigned)tiles, kLsdThreads, sizeof(LsdSmem), stream, from, Digit{first_bit + p * bits, bits},
+      SGL_CUDA_CHECK(allow_smem((const void*)lsd_pass_kernel<V, From, To>, done, sizeof(LsdSmem<V>)));
+      return launch(lsd_pass_kernel<V, From, To>, (unsigned)tiles, kLsdThreads, sizeof(LsdSmem<V>), stream, from, Digit{first_bit + p * bits, bits},
                     p, hist + p * kRadix, tickets + p, state, to, *gave_up, d_status);
     };
     const bool to_last = !kArray && p == passes - 1;
@@ -462,7 +482,7 @@ int lsd_sort(const Items& items, uint64_t* k1, V* v1, uint64_t* k0, V* v0, int64
 inline size_t list_ws_bytes(int64_t n) {
   if (n < 1) n = 1;
   if (n <= tilesort::kMaxItems) return tilesort::ws_bytes(n);
-  return 2 * align_up((size_t)n * 8) + 2 * align_up((size_t)n * 4) + lsd_ws_bytes(n) + align_up(8) +
+  return 2 * align_up((size_t)n * 8) + 2 * align_up((size_t)n * 4) + lsd_ws_bytes<uint32_t>(n) + align_up(8) +
          align_up(((size_t)((n + kDeliverTile - 1) / kDeliverTile) + 2) * 8);
 }
 
@@ -484,11 +504,10 @@ int sort_list(const Source& src, const Sink& sink, int64_t n_cap, int key_bits, 
   const int64_t tiles = (n_cap + kDeliverTile - 1) / kDeliverTile;
   unsigned long long* ctl = c.take<unsigned long long>((size_t)tiles + 2);
   SGL_REQUIRE(c.ok(), SGL_ERR_WORKSPACE, "sort: workspace %zu < %zu bytes", ws_bytes, list_ws_bytes(n_cap));
-  SGL_CHECK_RC(launch(source_count_kernel<Source>, 1, 1, 0, stream, src, count));
   SGL_CHECK_RC(zero_async(ctl, (size_t)(tiles + 2) * 8, stream));
   bool in_first;
   unsigned int* gave_up;
-  SGL_CHECK_RC((lsd_sort<uint32_t, SourceItems<Source>>(SourceItems<Source>{src}, k1, v1, k0, v0, n_cap, count, 0, key_bits,
+  SGL_CHECK_RC((lsd_sort<uint32_t, SourceItems<Source>>(SourceItems<Source>{src}, k1, v1, k0, v0, n_cap, count, count, 0, key_bits,
                                                         ArrayOut<uint32_t>{}, &in_first, &gave_up, c, d_status, stream)));
   return launch(lsd_deliver_kernel<Sink>, (unsigned)tiles, kDeliverThreads, 0, stream, sink, in_first ? k1 : k0, in_first ? v1 : v0, n_cap,
                 count, ctl, (uint64_t*)(ctl + 2), gave_up, d_status);

@@ -223,8 +223,8 @@ extern "C" size_t sgl_unique_pairs_ws_bytes(int64_t n_total) { return list_ws_by
 int sgl::unique_pairs(const int64_t* a_id, const int64_t* a_ts, int64_t n_a, const int64_t* d_n_a,
                                 const int64_t* b_id, const int64_t* b_ts, int64_t n_b, const int64_t* d_n_b, int id_bits,
                                 int ts_bits, int64_t ts_base, int64_t* out_id, int64_t* out_ts, int64_t* inv_a,
-                                int64_t* inv_b, int64_t* d_n_unique, const RowOrder& ro, int32_t* d_status, void* ws, size_t ws_bytes,
-                                void* stream_) {
+                                int64_t* inv_b, uint32_t* inv_b32, int64_t* d_n_unique, const RowOrder& ro, int32_t* d_status, void* ws,
+                                size_t ws_bytes, void* stream_) {
   SGL_NVTX("sgl_unique_pairs");
   cudaStream_t stream = (cudaStream_t)stream_;
   SGL_REQUIRE(n_a >= 0 && n_b >= 0, SGL_ERR_ARG, "unique_pairs: negative size");
@@ -241,7 +241,7 @@ int sgl::unique_pairs(const int64_t* a_id, const int64_t* a_ts, int64_t n_a, con
               "unique_pairs: null array");
   LaunchScope scope(stream);
   SGL_CHECK_RC(sort_list(PairSource{a_id, a_ts, d_n_a, b_id, b_ts, d_n_b, n_a, n_b, id_bits, ts_bits, ts_base, d_status},
-                         PairSink{n_a, d_n_a, ts_bits, ts_base, out_id, out_ts, inv_a, inv_b, d_n_unique, ro.order, ro.row, ro.first}, n,
+                         PairSink{n_a, d_n_a, ts_bits, ts_base, out_id, out_ts, inv_a, inv_b, d_n_unique, ro.order, ro.row, ro.first, inv_b32}, n,
                          id_bits + ts_bits, ws, ws_bytes, d_status, stream));
   return scope.submit();
 }
@@ -250,8 +250,8 @@ extern "C" int sgl_unique_pairs(const int64_t* a_id, const int64_t* a_ts, int64_
                                 const int64_t* b_ts, int64_t n_b, const int64_t* d_n_b, int id_bits, int ts_bits, int64_t ts_base,
                                 int64_t* out_id, int64_t* out_ts, int64_t* inv_a, int64_t* inv_b, int64_t* d_n_unique, int32_t* d_status,
                                 void* ws, size_t ws_bytes, void* stream) {
-  return unique_pairs(a_id, a_ts, n_a, d_n_a, b_id, b_ts, n_b, d_n_b, id_bits, ts_bits, ts_base, out_id, out_ts, inv_a, inv_b, d_n_unique,
-                      RowOrder{}, d_status, ws, ws_bytes, stream);
+  return unique_pairs(a_id, a_ts, n_a, d_n_a, b_id, b_ts, n_b, d_n_b, id_bits, ts_bits, ts_base, out_id, out_ts, inv_a, inv_b, nullptr,
+                      d_n_unique, RowOrder{}, d_status, ws, ws_bytes, stream);
 }
 
 extern "C" size_t sgl_build_csc_ws_bytes(int64_t n_edges, int64_t num_dst) {

@@ -28,10 +28,12 @@ struct RowOrder {
   }
 };
 
-// sgl_unique_pairs that also leaves the order of its list
+// sgl_unique_pairs that also leaves the order of its list, and (inv_b32) the inverse of the second part in 32-bit words instead of
+// inv_b
 int unique_pairs(const int64_t* a_id, const int64_t* a_ts, int64_t n_a, const int64_t* d_n_a, const int64_t* b_id, const int64_t* b_ts,
                  int64_t n_b, const int64_t* d_n_b, int id_bits, int ts_bits, int64_t ts_base, int64_t* out_id, int64_t* out_ts, int64_t* inv_a,
-                 int64_t* inv_b, int64_t* d_n_unique, const RowOrder& ro, int32_t* d_status, void* ws, size_t ws_bytes, void* stream);
+                 int64_t* inv_b, uint32_t* inv_b32, int64_t* d_n_unique, const RowOrder& ro, int32_t* d_status, void* ws, size_t ws_bytes,
+                 void* stream);
 
 size_t build_csc_rows_ws_bytes(int64_t n_edges, int64_t list_cap);
 // `list_cap` / d_num_dst: capacity of the list's order and its number of rows; offsets[i]: first edge of target i

@@ -48,7 +48,7 @@ struct IotaItems {
 }  // namespace
 
 size_t radix_sort_ws_bytes(int64_t n) {
-  return n <= tilesort::kMaxItems ? tilesort::ws_bytes(n) : lsd_ws_bytes(n);
+  return n <= tilesort::kMaxItems ? tilesort::ws_bytes(n) : lsd_ws_bytes<uint32_t>(n);
 }
 
 int radix_sort_pairs(uint64_t* keys, uint32_t* vals, uint64_t* keys_alt, uint32_t* vals_alt, int64_t n,
@@ -73,11 +73,11 @@ int radix_sort_pairs(uint64_t* keys, uint32_t* vals, uint64_t* keys_alt, uint32_
   bool alt = false;
   unsigned int* gave_up;
   if (iota_vals)
-    SGL_CHECK_RC((lsd_sort<uint32_t, IotaItems>(IotaItems{keys, n, d_n}, keys_alt, vals_alt, keys, vals, n, d_n, 0, num_bits, ArrayOut<uint32_t>{}, &alt, &gave_up, c,
+    SGL_CHECK_RC((lsd_sort<uint32_t, IotaItems>(IotaItems{keys, n, d_n}, keys_alt, vals_alt, keys, vals, n, d_n, nullptr, 0, num_bits, ArrayOut<uint32_t>{}, &alt, &gave_up, c,
                                                 nullptr, stream)));
   else
     SGL_CHECK_RC((lsd_sort<uint32_t, ArrayItems<uint32_t>>(ArrayItems<uint32_t>{keys, vals, n, d_n}, keys_alt, vals_alt, keys, vals, n,
-                                                           d_n, 0, num_bits, ArrayOut<uint32_t>{}, &alt, &gave_up, c, nullptr, stream)));
+                                                           d_n, nullptr, 0, num_bits, ArrayOut<uint32_t>{}, &alt, &gave_up, c, nullptr, stream)));
   *result_in_alt = alt ? 1 : 0;
   return scope.submit();
 }

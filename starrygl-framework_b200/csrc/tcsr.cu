@@ -246,7 +246,7 @@ using namespace sgl;
 extern "C" size_t sgl_tcsr_build_ws_bytes(int64_t num_nodes, int64_t m) {
   (void)num_nodes;
   if (m < 1) m = 1;
-  const size_t pairs = 4 * align_up((size_t)m * 8) + lsd_ws_bytes(m);
+  const size_t pairs = 4 * align_up((size_t)m * 8) + lsd_ws_bytes<uint64_t>(m);
   const size_t rounds = 2 * align_up((size_t)m * 8) + 2 * align_up((size_t)m * 4) + radix_sort_ws_bytes(m);
   size_t most = m <= tilesort::kMaxItems ? list_ws_bytes(m) : pairs;
   most = most > rounds ? most : rounds;
@@ -324,13 +324,13 @@ extern "C" int sgl_tcsr_build_fenced(int64_t num_nodes, int64_t m, const int64_t
       uint64_t *k1 = c.take<uint64_t>(m), *k0 = c.take<uint64_t>(m), *v1 = c.take<uint64_t>(m), *v0 = c.take<uint64_t>(m);
       uint32_t* node = (uint32_t*)(lsd_passes(first_bit, ts_bits + id_bits) & 1 ? k1 : k0);      // the last pass's own array
       const EdgeOut out{k, node, out_nbr, out_ts, out_eid};
-      SGL_CHECK_RC((lsd_sort<uint64_t, EdgePairs>(EdgePairs{k, nbr, eid, m}, k1, v1, k0, v0, m, nullptr, first_bit, ts_bits + id_bits, out,
+      SGL_CHECK_RC((lsd_sort<uint64_t, EdgePairs>(EdgePairs{k, nbr, eid, m}, k1, v1, k0, v0, m, nullptr, nullptr, first_bit, ts_bits + id_bits, out,
                                                   &in_first, &gave_up, c, nullptr, stream)));
       SGL_CHECK_RC(launch(tcsr_rows_kernel, stream_grid(m, 256 * 4, 8), 256, 0, stream, gave_up, node, m, num_nodes, indptr));
     } else {
       uint64_t *k1 = c.take<uint64_t>(m), *k0 = c.take<uint64_t>(m);
       uint32_t *v1 = c.take<uint32_t>(m), *v0 = c.take<uint32_t>(m);
-      SGL_CHECK_RC((lsd_sort<uint32_t, EdgePositions>(EdgePositions{k, m}, k1, v1, k0, v0, m, nullptr, first_bit, ts_bits + id_bits,
+      SGL_CHECK_RC((lsd_sort<uint32_t, EdgePositions>(EdgePositions{k, m}, k1, v1, k0, v0, m, nullptr, nullptr, first_bit, ts_bits + id_bits,
                                                       ArrayOut<uint32_t>{}, &in_first, &gave_up, c, nullptr, stream)));
       SGL_CHECK_RC(launch(tcsr_emit_gather_kernel, grid, 256, 0, stream, in_first ? k1 : k0, in_first ? v1 : v0, 1, k, nbr, eid, m, num_nodes,
                           indptr, out_nbr, out_ts, out_eid, out_perm));

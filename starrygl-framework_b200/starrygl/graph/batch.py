@@ -238,14 +238,14 @@ def build_batch(g, roots, root_ts, fanouts, policy="recent", **kw) -> List[dict]
 
 def batch_kernel_launches(num_nodes: int, num_roots: int, fanouts: Sequence[int], ts_span: int) -> int:
     """Kernels of this library that one mini-batch of :func:`build_batch_async` launches at the given capacities: count and
-    fill of every hop, the sort of every relabel (above the mini-batch sort's limit with an item count and a delivery
-    kernel), and for every hop after the first the two CSC kernels, the sort behind them and the column map."""
+    fill of every hop, the sort of every relabel (above the mini-batch sort's limit with a delivery
+    kernel more), and for every hop after the first the two CSC kernels, the sort behind them and the column map."""
     L = _C.lib()
     id_bits, ts_bits = ops.bits_for(num_nodes - 1), ops.bits_for(ts_span)
 
     def sort(n, bits):
         k = L.sgl_radix_sort_launches(n, bits)
-        return k if k <= 2 else k + 2
+        return k if k <= 2 else k + 1
     total = sort(num_roots, id_bits + ts_bits)
     cur, targets = num_roots, num_roots
     for l, k in enumerate(fanouts):

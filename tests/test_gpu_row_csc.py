@@ -33,3 +33,24 @@ def test_rows_of_many_targets(queries, fanouts, policy):
         for k in r:
             a = npy(d[k])
             assert a.dtype == r[k].dtype and np.array_equal(a, r[k]), (i, k)
+
+
+@pytest.mark.parametrize("copies, fanouts", [(50, [20, 20]), (50, [20, 21]), (50, [20, 21, 2])])
+def test_narrow_columns(copies, fanouts):
+    """Both sides of the capacity from which the merge scatters 32-bit positions (8 Mi edges), and a hop behind it."""
+    from starrygl.graph.batch import build_batch
+    rng = np.random.default_rng(1)
+    n, m = 300, 2500
+    src, dst = rng.integers(0, n, m).astype(np.int64), rng.integers(0, n, m).astype(np.int64)
+    ts = np.sort(rng.integers(0, 900, m)).astype(np.int64)
+    z = {"n": n, "dst": dst, "src": src, "ts": ts, "eid": np.arange(m, dtype=np.int64)}
+    g = build_graph(z)
+    indptr, nbr, tss, eid, _ = O.tcsr_build(dst, src, ts, z["eid"], n)
+    roots = np.tile(rng.integers(0, n, 400), copies).astype(np.int64)
+    rts = np.tile(rng.integers(100, 1000, 400), copies).astype(np.int64)
+    ref = O.build_batch(indptr, nbr, tss, eid, roots, rts, fanouts, O.UNIFORM, seed=4)
+    out = build_batch(g, cu(roots), cu(rts), fanouts, "uniform", seed=4, ts_range=(0, 1000))
+    assert len(out) == len(ref)
+    for i, (d, r) in enumerate(zip(out, ref)):
+        for k in r:
+            assert np.array_equal(npy(d[k]), r[k]), (i, k)

@@ -517,6 +517,13 @@ int sgl_mail_reduce(const int64_t* ids_a, int64_t n_a, const int64_t* ids_b, int
                     int64_t ts_len, int ts_is_i64, int n_seg, const float* const* seg_a, const float* const* seg_b,
                     const int64_t* seg_dim, int64_t* out_index, int64_t* out_pos, float* out_ts, float* out_mail,
                     int64_t* d_num_unique, int32_t* d_status, void* ws, size_t ws_bytes, void* stream);
+/* The same; the number of distinct nodes and behind it `seq` also go to host_unique[0..1] (pinned; NULL or a capturing stream: not
+ * written, see sgl_wait_word) as soon as it is known. */
+int sgl_mail_reduce_counted(const int64_t* ids_a, int64_t n_a, const int64_t* ids_b, int64_t n_b, int64_t num_nodes,
+                            const void* ts, int64_t ts_len, int ts_is_i64, int n_seg, const float* const* seg_a,
+                            const float* const* seg_b, const int64_t* seg_dim, int64_t* out_index, int64_t* out_pos,
+                            float* out_ts, float* out_mail, int64_t* d_num_unique, int32_t* d_status, void* ws,
+                            size_t ws_bytes, int64_t* host_unique, int64_t seq, void* stream);
 int sgl_mailbox_write(const int64_t* index, int64_t n, const int64_t* d_n, const float* mail, const float* mail_ts,
                       int64_t width, float* mailbox, float* mailbox_ts, int64_t* next_mail_pos, int64_t num_nodes,
                       int64_t mailbox_size, int advance, int32_t* d_status, void* stream);

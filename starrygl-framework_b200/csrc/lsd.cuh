@@ -31,7 +31,8 @@ template <class V>
 constexpr int kLsdItems = sizeof(V) == 4 ? 14 : 12;      // keys per thread; more would spill
 template <class V>
 constexpr int kLsdTile = kLsdThreads * kLsdItems<V>;
-constexpr int kLookWide = 4;               // tiles a look-back step reads
+template <class V>
+constexpr int kLookWide = sizeof(V) == 4 ? 8 : 4;         // tiles a look-back step reads (measured: 2 - 16)
 constexpr int kHistThreads = 512;
 
 // a pass: `bits` <= kBits bits from `shift` on
@@ -109,6 +110,7 @@ struct LsdSmem {
 
 // where a pass reads its items from: the arrays of the pass before, or (first pass) the producer of the keys
 // Sum of what the tiles before this one hold of digit threadIdx.x; publishes it with the tile's own.
+template <int kWide>
 __device__ __forceinline__ uint64_t look_back(uint64_t* state, int pass, int tile, uint32_t total, unsigned int* gave_up, int32_t* d_status) {
   const uint64_t tag = pass_tag(pass);
   volatile uint64_t* st = state + threadIdx.x;
@@ -116,12 +118,12 @@ __device__ __forceinline__ uint64_t look_back(uint64_t* state, int pass, int til
   unsigned long long t0 = 0;
   // (tiles are taken in order: those before this one are running or done)
   for (int t = tile - 1; t >= 0;) {
-    uint64_t w[kLookWide];
+    uint64_t w[kWide];
 #pragma unroll
-    for (int u = 0; u < kLookWide; ++u) w[u] = t - u >= 0 ? st[(size_t)(t - u) * kRadix] : 0;
+    for (int u = 0; u < kWide; ++u) w[u] = t - u >= 0 ? st[(size_t)(t - u) * kRadix] : 0;
     bool done = false, stalled = false;
 #pragma unroll
-    for (int u = 0; u < kLookWide; ++u) {
+    for (int u = 0; u < kWide; ++u) {
       if (done || stalled || t < 0) continue;
       if ((w[u] & (0x3full << 56)) != tag) {
         stalled = true;
@@ -266,7 +268,7 @@ lsd_pass_kernel(Items items, Digit digit, int pass,
     }
   }
   if (tid < kRadix) {
-    const uint64_t sum = tile > 0 ? look_back(state, pass, tile, total, gave_up, d_status) : 0;
+    const uint64_t sum = tile > 0 ? look_back<kLookWide<V>>(state, pass, tile, total, gave_up, d_status) : 0;
     sm.out[tid] = (uint32_t)(starts[tid] + sum) - start;
   }
   __syncthreads();

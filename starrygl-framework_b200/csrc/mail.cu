@@ -10,7 +10,7 @@
 // Timestamps are compared as fp32, like the reference, which converts them to the mailbox dtype before the reduce.
 // Algorithmic HBM bytes: 8 + 4|8 read per entry + sort passes (32 B per entry and populated key byte), and per
 // unique node 2 * row bytes + 20 written / read.
-#include "launch.cuh"
+#include "chain.cuh"
 #include "lsd.cuh"
 
 namespace sgl {
@@ -193,11 +193,11 @@ extern "C" size_t sgl_mail_reduce_ws_bytes(int64_t n_entries) {
   return 2 * align_up((size_t)n * 4) + list_ws_bytes(n);
 }
 
-extern "C" int sgl_mail_reduce(const int64_t* ids_a, int64_t n_a, const int64_t* ids_b, int64_t n_b, int64_t num_nodes,
+extern "C" int sgl_mail_reduce_counted(const int64_t* ids_a, int64_t n_a, const int64_t* ids_b, int64_t n_b, int64_t num_nodes,
                                const void* ts, int64_t ts_len, int ts_is_i64, int n_seg, const float* const* seg_a,
                                const float* const* seg_b, const int64_t* seg_dim, int64_t* out_index, int64_t* out_pos,
                                float* out_ts, float* out_mail, int64_t* d_num_unique, int32_t* d_status, void* ws,
-                               size_t ws_bytes, void* stream_) {
+                               size_t ws_bytes, int64_t* host_unique, int64_t seq, void* stream_) {
   SGL_NVTX("sgl_mail_reduce");
   cudaStream_t stream = (cudaStream_t)stream_;
   const int64_t n = n_a + n_b;
@@ -206,6 +206,10 @@ extern "C" int sgl_mail_reduce(const int64_t* ids_a, int64_t n_a, const int64_t*
   SGL_REQUIRE(n_seg >= 0 && n_seg <= kMaxSeg, SGL_ERR_ARG, "mail_reduce: at most %d row segments", kMaxSeg);
   if (n == 0) {
     SGL_CHECK_RC(zero_async(d_num_unique, sizeof(int64_t), stream));
+    if (host_unique) {
+      host_unique[0] = 0;
+      host_unique[1] = seq;
+    }
     return SGL_OK;
   }
   SGL_REQUIRE((n_a == 0 || ids_a) && (n_b == 0 || ids_b) && ts && out_index, SGL_ERR_ARG, "mail_reduce: null array");
@@ -242,6 +246,12 @@ extern "C" int sgl_mail_reduce(const int64_t* ids_a, int64_t n_a, const int64_t*
     SGL_CHECK_RC(sort_list(MailNodes{entries, order}, MailSink{out_index, winner, d_num_unique, order, 0}, n, id_bits, sort_ws, sort_bytes,
                            d_status, stream));
   }
+  if (LaunchScope* in = host_unique ? LaunchScope::current() : nullptr) {
+    // the number of nodes is on its way while the rows are put together (a second chain of the graph)
+    cudaStream_t side = (cudaStream_t)(uintptr_t)3;
+    in->wait(side, in->mark(stream));
+    SGL_CHECK_RC(launch(export_words_kernel, 1, 32, 0, side, d_num_unique, host_unique, 1, seq));
+  }
   const int grid = stream_grid(n, kThreads / 32, 8);
   if (quads)
     SGL_CHECK_RC(launch(mail_emit_kernel<Words4>, grid, kThreads, 0, stream, winner, n, d_num_unique, n_a, ts, ts_len, ts_is_i64, segs,
@@ -250,6 +260,14 @@ extern "C" int sgl_mail_reduce(const int64_t* ids_a, int64_t n_a, const int64_t*
     SGL_CHECK_RC(launch(mail_emit_kernel<Words1>, grid, kThreads, 0, stream, winner, n, d_num_unique, n_a, ts, ts_len, ts_is_i64, segs,
                         width, out_pos, out_ts, out_mail));
   return scope.submit();
+}
+
+extern "C" int sgl_mail_reduce(const int64_t* ids_a, int64_t n_a, const int64_t* ids_b, int64_t n_b, int64_t num_nodes, const void* ts,
+                               int64_t ts_len, int ts_is_i64, int n_seg, const float* const* seg_a, const float* const* seg_b,
+                               const int64_t* seg_dim, int64_t* out_index, int64_t* out_pos, float* out_ts, float* out_mail,
+                               int64_t* d_num_unique, int32_t* d_status, void* ws, size_t ws_bytes, void* stream) {
+  return sgl_mail_reduce_counted(ids_a, n_a, ids_b, n_b, num_nodes, ts, ts_len, ts_is_i64, n_seg, seg_a, seg_b, seg_dim, out_index, out_pos,
+                                 out_ts, out_mail, d_num_unique, d_status, ws, ws_bytes, nullptr, 0, stream);
 }
 
 extern "C" int sgl_mailbox_write(const int64_t* index, int64_t n, const int64_t* d_n, const float* mail, const float* mail_ts,

@@ -110,6 +110,8 @@ _SIGNATURES = {
     "sgl_mail_reduce_ws_bytes": (_sz, [_i64]),
     "sgl_mail_reduce": (_i32, [_vp, _i64, _vp, _i64, _i64, _vp, _i64, _i32, _i32, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp,
                                _sz, _vp]),
+    "sgl_mail_reduce_counted": (_i32, [_vp, _i64, _vp, _i64, _i64, _vp, _i64, _i32, _i32, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp,
+                                       _vp, _sz, _vp, _i64, _vp]),
     "sgl_mailbox_write": (_i32, [_vp, _i64, _vp, _vp, _vp, _i64, _vp, _vp, _vp, _i64, _i64, _i32, _vp, _vp]),
     "sgl_build_batch_layout": (_i64, [_i64, _vp, _i32, _vp]),
     "sgl_build_batch_ws_bytes": (_sz, [_i64, _vp, _i32]),

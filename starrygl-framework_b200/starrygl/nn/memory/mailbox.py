@@ -58,7 +58,7 @@ class mailbox:
 
     # ---- latest message per node -------------------------------------------------------------------------------
     def get_update_mail_async(self, src, dst, ts, edge_feats, mem_src, mem_dst, embedding=None, use_src_emb=False,
-                              use_dst_emb=False):
+                              use_dst_emb=False, count=None):
         """``get_update_mail`` without the host synchronisation: returns ``(index, mail, mail_ts, d_n)`` where the
         tensors have capacity ``2 * len(src)`` and the device scalar ``d_n`` holds the number of distinct nodes."""
         src, dst = src.to(self.device), dst.to(self.device)
@@ -77,16 +77,19 @@ class mailbox:
         if ts.dtype not in (torch.int64, torch.float32):
             ts = ts.to(torch.float32)
         index, mail, mail_ts, _, d_n = ops.mail_reduce(src.reshape(-1), dst.reshape(-1), ts.reshape(-1), self.num_nodes, segs,
-                                                       status=self._status)
+                                                       status=self._status, count=count)
         return index, mail, mail_ts, d_n
 
     def get_update_mail(self, src, dst, ts, edge_feats, mem_src, mem_dst, embedding=None, use_src_emb=False,
                         use_dst_emb=False, block=None, Reduce_score=None):
         """(index, mail, mail_ts) of the batch: distinct nodes in ascending order, each with the row and timestamp of
         its latest entry (reference: mailbox.py:56-84).  One host synchronisation, to size the results exactly."""
+        count, stream = _C.COUNTS.take(), _C.stream_ptr()
         index, mail, mail_ts, d_n = self.get_update_mail_async(src, dst, ts, edge_feats, mem_src, mem_dst, embedding,
-                                                               use_src_emb, use_dst_emb)
-        u = _C.read_words(d_n, 1)[0]
+                                                               use_src_emb, use_dst_emb, count)
+        u = _C.COUNTS.value(count, stream)
+        if u is None:
+            u = int(d_n.item())
         return index[:u], mail[:u], mail_ts[:u]
 
     # ---- writes ------------------------------------------------------------------------------------------------

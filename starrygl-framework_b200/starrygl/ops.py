@@ -352,10 +352,11 @@ def _row_bytes(t):
         return t.element_size(), t.element_size()
     if t.stride(-1) != 1 and t.shape[-1] > 1:
         raise _C.SglError("rows must be contiguous")
-    inner = 1
+    size = t.element_size()
+    inner = size
     for s in t.shape[1:]:
         inner *= s
-    return inner * t.element_size(), t.stride(0) * t.element_size()
+    return inner, t.stride(0) * size
 
 
 def gather_rows(table, idx, *, map=None, d_n=None, ts_table=None, mode="auto", out=None,
@@ -366,9 +367,11 @@ def gather_rows(table, idx, *, map=None, d_n=None, ts_table=None, mode="auto", o
     idx = _i64(idx)
     n = idx.numel()
     row_bytes, src_pitch = _row_bytes(table)
+    dst_pitch = row_bytes
     if out is None:
-        out = torch.empty((n,) + tuple(table.shape[1:]), dtype=table.dtype, device=idx.device)
-    _, dst_pitch = _row_bytes(out) if n else (row_bytes, row_bytes)
+        out = torch.empty((n, *table.shape[1:]), dtype=table.dtype, device=idx.device)
+    elif n:
+        _, dst_pitch = _row_bytes(out)
     out_ts = torch.empty(n, dtype=torch.float32, device=idx.device) if ts_table is not None else None
     _C.check(L.sgl_gather_rows(_C.ptr(table) if table.numel() else None, table.shape[0], row_bytes, src_pitch,
                                _C.ptr(idx), _C.ptr(map), 0 if map is None else map.numel(), n, _C.ptr(d_n),
@@ -578,13 +581,17 @@ def plan_route(layer_ids, node_parts, pid: int, rep_indptr, rep_ranks, rep_locs,
 # mailbox update
 # --------------------------------------------------------------------------------------------------------------
 
+_SEG_ARRAYS = [C.c_int64 * max(k, 1) for k in range(5)]       # (making an array type takes longer than filling one in)
+
+
 def mail_reduce(ids_a, ids_b, ts, num_nodes: int, segments=(), *, want_pos: bool = False,
-                status: Optional[StatusWord] = None):
+                status: Optional[StatusWord] = None, count=None):
     """Latest message per node (see ``sgl_mail_reduce``).  ``ids_a`` / ``ids_b``: int64 node ids of the two entry lists
     (``ids_b`` may be None); ``ts``: int64 or fp32, one value per entry or one per event; ``segments``: list of
     ``(table_a, table_b)`` fp32 row tables whose rows are concatenated into the mail of the winning entry.
     Returns ``(index, mail, mail_ts, pos, d_num_unique)`` with capacity ``len(ids_a) + len(ids_b)``; the valid
-    length is the device scalar ``d_num_unique`` (no synchronisation here).  ``mail`` is None without segments."""
+    length is the device scalar ``d_num_unique`` (no synchronisation here).  ``mail`` is None without segments.
+    ``count``: a pair taken from ``_C.COUNTS`` that receives the number of nodes."""
     L = _C.lib()
     ids_a = _i64(ids_a)
     dev = ids_a.device
@@ -612,15 +619,16 @@ def mail_reduce(ids_a, ids_b, ts, num_nodes: int, segments=(), *, want_pos: bool
     mail = torch.empty((cap, width), dtype=torch.float32, device=dev) if segs else None
     d_u = torch.empty(1, dtype=I64, device=dev)
     k = len(segs)
-    arr_a = (C.c_void_p * max(k, 1))(*[a.data_ptr() for a, _ in segs])
-    arr_b = (C.c_void_p * max(k, 1))(*[b.data_ptr() for _, b in segs])
-    arr_d = (C.c_int64 * max(k, 1))(*[int(a.shape[1]) for a, _ in segs])
+    kind = _SEG_ARRAYS[k] if k < len(_SEG_ARRAYS) else C.c_int64 * k
+    arr_a = kind(*[a.data_ptr() for a, _ in segs])
+    arr_b = kind(*[b.data_ptr() for _, b in segs])
+    arr_d = kind(*[a.shape[1] for a, _ in segs])
     _, wp, wn = _C.workspace(L.sgl_mail_reduce_ws_bytes(n), dev)
-    _C.check(L.sgl_mail_reduce(_C.ptr(ids_a), n_a, _C.ptr(ids_b) if n_b else None, n_b, int(num_nodes), _C.ptr(ts), ts.numel(),
-                               1 if ts.dtype == torch.int64 else 0, k, C.cast(arr_a, C.c_void_p), C.cast(arr_b, C.c_void_p),
-                               C.cast(arr_d, C.c_void_p), _C.ptr(index), _C.ptr(pos) if want_pos else None, _C.ptr(out_ts),
+    _C.check(L.sgl_mail_reduce_counted(_C.ptr(ids_a), n_a, _C.ptr(ids_b) if n_b else None, n_b, int(num_nodes), _C.ptr(ts), ts.numel(),
+                               1 if ts.dtype == torch.int64 else 0, k, C.addressof(arr_a), C.addressof(arr_b),
+                               C.addressof(arr_d), _C.ptr(index), _C.ptr(pos) if want_pos else None, _C.ptr(out_ts),
                                _C.ptr(mail) if mail is not None else None, _C.ptr(d_u), status.ptr() if status else None,
-                               wp, wn, _C.stream_ptr()))
+                               wp, wn, None if count is None else count[0], 0 if count is None else count[2], _C.stream_ptr()))
     return index, mail, out_ts, pos, d_u
 
 

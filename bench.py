@@ -782,7 +782,7 @@ def run_single(args, dev, local, out_stream):
                             f"{len(e2e_times)} repeats of the K-step loop (wall clock around a device synchronisation)",
                     "edges_per_step": e2e_edges / K},
             "gpu_launches": R * K * pipe.kernel_launches_per_step,
-            "roofline": {"bound": "hbm", "kernel": "gather_bulk_kernel" if pipe.mode != 1 else "gather_lanes_kernel",
+            "roofline": {"bound": "hbm", "kernel": "bulk_rows_kernel" if pipe.mode != 1 else "gather_lanes_kernel",
                          "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                          "peak_source": peak_kind, "traffic": statistics.mean(edges) * GATHER_TRAFFIC_BYTES_PER_ROW,
                          "traffic_note": "ncu dram read+write of a 65 k-row launch scaled by rows; the output is still in L2 when "

@@ -543,6 +543,14 @@ int sgl_plan_route(const int64_t* layer_ids, int64_t n, const int64_t* d_n, cons
                    int64_t pid, const int64_t* rep_indptr, const int64_t* rep_ranks, const int64_t* rep_locs,
                    int64_t num_parts, int64_t cap, int64_t* out_ranks, int64_t* out_rows, int64_t* out_locs,
                    int64_t* d_send_sizes, int64_t* d_total, int32_t* d_status, void* ws, size_t ws_bytes, void* stream);
+/* Plans of several layer lists side by side (up to 9 in one set of launches; more, or more than 32 ranks, one after the other):
+ * list i has layer_ids[i], n[i], d_n[i], cap[i]; out[i] receives ranks, rows and slots, cap[i] words each; d_counts[i] the
+ * num_parts send sizes and the total.  The tables are host arrays. */
+size_t sgl_plan_routes_ws_bytes(int layers, const int64_t* n, const int64_t* cap);
+int sgl_plan_routes(int layers, const int64_t* const* layer_ids, const int64_t* n, const int64_t* const* d_n,
+                    const int64_t* node_parts, int64_t num_nodes, int64_t pid, const int64_t* rep_indptr, const int64_t* rep_ranks,
+                    const int64_t* rep_locs, int64_t num_parts, const int64_t* cap, int64_t* const* out, int64_t* const* d_counts,
+                    int32_t* d_status, void* ws, size_t ws_bytes, void* stream);
 
 /* ------------------------------------------------------------------------------------------------
  * Roots of a batch = the events of one time window.  Input: the window's slice of the time-ordered event
@@ -621,8 +629,8 @@ int sgl_query_blocks(int n_hops, const int64_t* const* node, const int64_t* cons
  * sgl_wait_word: waits until work on the stream has set *flag (pinned memory) to at_least or more.  sgl_read_back: copies up to 511 words of
  * device memory to the host through that buffer and waits for them. */
 /* Up to 96 device arrays (sizes multiples of 4 bytes) to the host in one copy: packed at the 16-byte aligned offsets at[]
- * of `staging` (device, total bytes) and copied to `host`, or, with host2, the bytes from `split` on to host2; waits for
- * the stream. */
+ * of `staging` (device, total bytes) and copied to `host`, or, with host2, the bytes from `split` on to host2; does not
+ * wait for the copies. */
 int sgl_export_arrays(int n, const void* const* src, const int64_t* bytes, const int64_t* at, void* staging, void* host,
                       int64_t total, void* host2, int64_t split, void* stream);
 int sgl_host_words(void** out);

@@ -315,7 +315,6 @@ extern "C" int sgl_export_arrays(int n, const void* const* src, const int64_t* b
   if (split > 0) SGL_CUDA_CHECK(cudaMemcpyAsync(host, staging, (size_t)split, cudaMemcpyDeviceToHost, stream));
   if (split < total)
     SGL_CUDA_CHECK(cudaMemcpyAsync(host2, (char*)staging + split, (size_t)(total - split), cudaMemcpyDeviceToHost, stream));
-  SGL_CUDA_CHECK(cudaStreamSynchronize(stream));
   return SGL_OK;
 }
 

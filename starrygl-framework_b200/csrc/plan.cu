@@ -98,6 +98,18 @@ plan_emit_kernel(const uint64_t* __restrict__ keys, const uint32_t* __restrict__
 
 // ---- up to kFewParts ranks: entries counted per (rank, CTA), placed by rank without a sort --------------------------------
 constexpr int kFewParts = 32;
+constexpr int kMaxLayers = 9;
+
+// Layer lists whose plans are made side by side (grid.y), one after the other a two-hop slot's three plans took 55 us of kernels.
+struct PlanLayer {
+  const int64_t *ids, *d_n;
+  int64_t n_cap, cap;
+  int32_t* tally;
+  int64_t *out_ranks, *out_rows, *out_locs, *send_sizes, *total;
+};
+struct PlanLayers {
+  PlanLayer l[kMaxLayers];
+};
 
 // does row i send its node's row, and to which copies?  [*s, *e) of the replica lists; false: nothing
 __device__ __forceinline__ bool plan_row(const int64_t* __restrict__ ids, int64_t n, int64_t i, const int64_t* __restrict__ node_parts,
@@ -120,11 +132,13 @@ __device__ __forceinline__ bool plan_row(const int64_t* __restrict__ ids, int64_
 }
 
 __global__ void __launch_bounds__(kThreads)
-plan_tally_kernel(const int64_t* __restrict__ ids, int64_t n_cap, const int64_t* d_n, const int64_t* __restrict__ node_parts,
-                  int64_t num_nodes, int64_t pid, const int64_t* __restrict__ indptr, const int64_t* __restrict__ ranks, int num_parts,
-                  int32_t* __restrict__ tally, int32_t* d_status) {
+plan_tally_kernel(const __grid_constant__ PlanLayers layers, const int64_t* __restrict__ node_parts, int64_t num_nodes, int64_t pid,
+                  const int64_t* __restrict__ indptr, const int64_t* __restrict__ ranks, int num_parts, int32_t* d_status) {
   __shared__ int s_cnt[kFewParts];
-  const int64_t n = eff_count(n_cap, d_n);
+  const PlanLayer& l = layers.l[blockIdx.y];
+  const int64_t* __restrict__ ids = l.ids;
+  int32_t* __restrict__ tally = l.tally;
+  const int64_t n = eff_count(l.n_cap, l.d_n);
   if ((int64_t)blockIdx.x * kThreads >= n) return;
   if (threadIdx.x < num_parts) s_cnt[threadIdx.x] = 0;
   __syncthreads();
@@ -140,11 +154,14 @@ plan_tally_kernel(const int64_t* __restrict__ ids, int64_t n_cap, const int64_t*
   if (threadIdx.x < num_parts) tally[threadIdx.x * ctas + blockIdx.x] = s_cnt[threadIdx.x];
 }
 
-// exclusive scan of the (rank, CTA) counts in place, rank by rank; sizes per rank and the total.  One CTA.
+// exclusive scan of the (rank, CTA) counts in place, rank by rank; sizes per rank and the total.  One CTA per layer.
 __global__ void __launch_bounds__(1024)
-plan_place_kernel(int64_t n_cap, const int64_t* d_n, int num_parts, int32_t* __restrict__ tally, int64_t* d_send_sizes, int64_t* d_total) {
+plan_place_kernel(const __grid_constant__ PlanLayers layers, int num_parts) {
   __shared__ int64_t s_carry;
-  const int64_t n = eff_count(n_cap, d_n), ctas = (n + kThreads - 1) / kThreads;
+  const PlanLayer& l = layers.l[blockIdx.x];
+  int32_t* __restrict__ tally = l.tally;
+  int64_t *d_send_sizes = l.send_sizes, *d_total = l.total;
+  const int64_t n = eff_count(l.n_cap, l.d_n), ctas = (n + kThreads - 1) / kThreads;
   if (threadIdx.x == 0) s_carry = 0;
   __syncthreads();
   int64_t begin = 0;
@@ -168,11 +185,15 @@ plan_place_kernel(int64_t n_cap, const int64_t* d_n, int num_parts, int32_t* __r
 }
 
 __global__ void __launch_bounds__(kThreads)
-plan_write_kernel(const int64_t* __restrict__ ids, int64_t n_cap, const int64_t* d_n, const int64_t* __restrict__ node_parts,
-                  int64_t num_nodes, int64_t pid, const int64_t* __restrict__ indptr, const int64_t* __restrict__ ranks,
-                  const int64_t* __restrict__ locs, int num_parts, const int32_t* __restrict__ tally, int64_t cap,
-                  int64_t* __restrict__ out_ranks, int64_t* __restrict__ out_rows, int64_t* __restrict__ out_locs, int32_t* d_status) {
-  const int64_t n = eff_count(n_cap, d_n);
+plan_write_kernel(const __grid_constant__ PlanLayers layers, const int64_t* __restrict__ node_parts, int64_t num_nodes, int64_t pid,
+                  const int64_t* __restrict__ indptr, const int64_t* __restrict__ ranks, const int64_t* __restrict__ locs, int num_parts,
+                  int32_t* d_status) {
+  const PlanLayer& l = layers.l[blockIdx.y];
+  const int64_t* __restrict__ ids = l.ids;
+  const int32_t* __restrict__ tally = l.tally;
+  const int64_t cap = l.cap;
+  int64_t *__restrict__ out_ranks = l.out_ranks, *__restrict__ out_rows = l.out_rows, *__restrict__ out_locs = l.out_locs;
+  const int64_t n = eff_count(l.n_cap, l.d_n);
   if ((int64_t)blockIdx.x * kThreads >= n) return;
   const int64_t ctas = (n + kThreads - 1) / kThreads;
   const int64_t i = (int64_t)blockIdx.x * kThreads + threadIdx.x;
@@ -200,6 +221,19 @@ plan_write_kernel(const int64_t* __restrict__ ids, int64_t n_cap, const int64_t*
 }
 
 inline int64_t ctas_for(int64_t n) { return (n + kThreads - 1) / kThreads < 1 ? 1 : (n + kThreads - 1) / kThreads; }
+
+bool few_parts(int64_t n, int64_t num_parts) { return num_parts <= kFewParts && n * num_parts < ((int64_t)1 << 31); }
+
+int plan_few(const PlanLayers& layers, int count, int64_t most_n, const int64_t* node_parts, int64_t num_nodes, int64_t pid,
+             const int64_t* rep_indptr, const int64_t* rep_ranks, const int64_t* rep_locs, int num_parts, int32_t* d_status,
+             cudaStream_t stream) {
+  const dim3 grid((unsigned)ctas_for(most_n), (unsigned)count);
+  SGL_CHECK_RC(launch(plan_tally_kernel, grid, kThreads, 0, stream, layers, node_parts, num_nodes, pid, rep_indptr, rep_ranks, num_parts,
+                      d_status));
+  SGL_CHECK_RC(launch(plan_place_kernel, (unsigned)count, 1024, 0, stream, layers, num_parts));
+  return launch(plan_write_kernel, grid, kThreads, 0, stream, layers, node_parts, num_nodes, pid, rep_indptr, rep_ranks, rep_locs, num_parts,
+                d_status);
+}
 
 }  // namespace
 }  // namespace sgl
@@ -232,16 +266,14 @@ extern "C" int sgl_plan_route(const int64_t* layer_ids, int64_t n, const int64_t
   SGL_REQUIRE(layer_ids && node_parts && rep_indptr && rep_ranks && rep_locs && out_ranks && out_rows && out_locs, SGL_ERR_ARG,
               "plan_route: null array");
   const int64_t capc = cap < 1 ? 1 : cap;
-  if (num_parts <= kFewParts && n * num_parts < ((int64_t)1 << 31)) {
+  if (few_parts(n, num_parts)) {
     WsCarver c(ws, ws_bytes);
     int32_t* tally = c.take<int32_t>((size_t)(num_parts * ctas_for(n)));
     SGL_REQUIRE(c.ok(), SGL_ERR_WORKSPACE, "plan_route: workspace %zu < %zu bytes", ws_bytes, sgl_plan_route_ws_bytes(n, cap));
-    const unsigned grid = (unsigned)ctas_for(n);
-    SGL_CHECK_RC(launch(plan_tally_kernel, grid, kThreads, 0, stream, layer_ids, n, d_n, node_parts, num_nodes, pid, rep_indptr, rep_ranks,
-                        (int)num_parts, tally, d_status));
-    SGL_CHECK_RC(launch(plan_place_kernel, 1, 1024, 0, stream, n, d_n, (int)num_parts, tally, d_send_sizes, d_total));
-    SGL_CHECK_RC(launch(plan_write_kernel, grid, kThreads, 0, stream, layer_ids, n, d_n, node_parts, num_nodes, pid, rep_indptr, rep_ranks,
-                        rep_locs, (int)num_parts, tally, cap, out_ranks, out_rows, out_locs, d_status));
+    PlanLayers layers;
+    memset(&layers, 0, sizeof(layers));
+    layers.l[0] = PlanLayer{layer_ids, d_n, n, cap, tally, out_ranks, out_rows, out_locs, d_send_sizes, d_total};
+    SGL_CHECK_RC(plan_few(layers, 1, n, node_parts, num_nodes, pid, rep_indptr, rep_ranks, rep_locs, (int)num_parts, d_status, stream));
     return scope.submit();
   }
   SGL_CHECK_RC(zero_async(d_send_sizes, (size_t)num_parts * sizeof(int64_t), stream));
@@ -272,5 +304,48 @@ extern "C" int sgl_plan_route(const int64_t* layer_ids, int64_t n, const int64_t
   if (rc) return rc;
   SGL_CHECK_RC(launch(plan_emit_kernel, stream_grid(capc, kThreads, 8), kThreads, 0, stream, in_alt ? k1 : k0, in_alt ? v1 :
                       v0, capc, d_total, tmp_rows, tmp_locs, out_ranks, out_rows, out_locs));
+  return scope.submit();
+}
+
+extern "C" size_t sgl_plan_routes_ws_bytes(int layers, const int64_t* n, const int64_t* cap) {
+  size_t sum = 0, most = 0;
+  for (int i = 0; i < layers; ++i) {
+    const size_t one = align_up(sgl_plan_route_ws_bytes(n[i], cap[i]));
+    most = one > most ? one : most;
+    sum += align_up((size_t)kFewParts * ctas_for(n[i]) * 4);
+  }
+  return sum > most ? sum : most;
+}
+
+extern "C" int sgl_plan_routes(int layers, const int64_t* const* layer_ids, const int64_t* n, const int64_t* const* d_n,
+                               const int64_t* node_parts, int64_t num_nodes, int64_t pid, const int64_t* rep_indptr,
+                               const int64_t* rep_ranks, const int64_t* rep_locs, int64_t num_parts, const int64_t* cap,
+                               int64_t* const* out, int64_t* const* d_counts, int32_t* d_status, void* ws, size_t ws_bytes, void* stream_) {
+  SGL_NVTX("sgl_plan_routes");
+  cudaStream_t stream = (cudaStream_t)stream_;
+  SGL_REQUIRE(layers >= 0 && (layers == 0 || (layer_ids && n && d_n && cap && out && d_counts)), SGL_ERR_ARG, "plan_routes: null table");
+  LaunchScope scope(stream);
+  bool few = layers <= kMaxLayers && num_parts >= 1 && pid >= 0 && pid < num_parts && num_nodes >= 0 && node_parts && rep_indptr && rep_ranks &&
+             rep_locs;
+  for (int i = 0; i < layers && few; ++i) few = n[i] > 0 && cap[i] > 0 && few_parts(n[i], num_parts) && layer_ids[i] && out[i] && d_counts[i];
+  if (few && layers > 0) {
+    WsCarver c(ws, ws_bytes);
+    PlanLayers l;
+    memset(&l, 0, sizeof(l));
+    int64_t most = 1;
+    for (int i = 0; i < layers; ++i) {
+      int32_t* tally = c.take<int32_t>((size_t)(num_parts * ctas_for(n[i])));
+      l.l[i] = PlanLayer{layer_ids[i], d_n[i], n[i], cap[i], tally, out[i], out[i] + cap[i], out[i] + 2 * cap[i], d_counts[i],
+                         d_counts[i] + num_parts};
+      most = n[i] > most ? n[i] : most;
+    }
+    SGL_REQUIRE(c.ok(), SGL_ERR_WORKSPACE, "plan_routes: workspace %zu < %zu bytes", ws_bytes, sgl_plan_routes_ws_bytes(layers, n, cap));
+    SGL_CHECK_RC(plan_few(l, layers, most, node_parts, num_nodes, pid, rep_indptr, rep_ranks, rep_locs, (int)num_parts, d_status, stream));
+  } else {
+    for (int i = 0; i < layers; ++i)
+      SGL_CHECK_RC(sgl_plan_route(layer_ids[i], n[i], d_n[i], node_parts, num_nodes, pid, rep_indptr, rep_ranks, rep_locs, num_parts, cap[i],
+                                  out[i], out[i] + cap[i], out[i] + 2 * cap[i], d_counts[i], d_counts[i] + num_parts, d_status, ws, ws_bytes,
+                                  stream_));
+  }
   return scope.submit();
 }

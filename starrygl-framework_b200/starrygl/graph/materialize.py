@@ -6,13 +6,14 @@ dictionaries -- layer 0: ``gids``, ``ts``, ``inv_map``, ``num_neg`` + the task t
 ``indptr``, ``indices``, ``eid``, ``edge_ts``, ``edge_dt``, ``gids``, ``ts`` -- and writes it with ``torch.save`` in the
 layout the reference's loader reads (all tensors on the CPU, ``comm_plan`` = one ``CommPlan`` or ``None`` per layer
 list).  Sampling, (node, ts) relabel, CSC and the route plans run through the library
-(``sgl_build_batch``, ``sgl_plan_route``); the T-CSR is built once per partition.
+(``sgl_build_batch``, ``sgl_plan_routes``); the T-CSR is built once per partition.
 
 Supported policy space = what the GPU sampler implements: continuous graphs (``graph_type == 'c'``), ``recent`` and
 ``uniform`` layers, ``end_offset`` 0 (strictly earlier edges) or 1 (edges at the query time included; integer
 timestamps).  ``cluster`` / ``full`` layers and discrete graphs raise ``NotImplementedError``.  Negative destinations
 of a ``'neg'`` task are drawn from a seeded torch generator (the reference draws from the unseeded global numpy state).
 """
+import ctypes as C
 from typing import List, Optional
 
 import numpy as np
@@ -132,14 +133,19 @@ class MaterializedMultiLayerBuilder:
             caps = [max(c * max(P - 1, 1), 1) for _, c in lists]
             room = torch.empty(3 * sum(caps), dtype=torch.int64, device=self.device)
             rt, sp, mp, at = self.rep_table, _C.stream_ptr(), meta.data_ptr(), room.data_ptr()
-            ws = _C.WORKSPACE.get(max(L.sgl_plan_route_ws_bytes(c, cap) for (_, c), cap in zip(lists, caps)), self.device, sp)
-            for i, ((ids, c), cap) in enumerate(zip(lists, caps)):
-                m = mp + 8 * (nb + i * (P + 1))
-                _C.check(L.sgl_plan_route(ids, c, mp + 8 * (2 * i), self.node_parts.data_ptr(), self.node_parts.numel(), self.pid,
-                                          rt.indptr.data_ptr(), rt.indices.data_ptr(), rt.locs.data_ptr(), P, cap, at, at + 8 * cap,
-                                          at + 16 * cap, m, m + 8 * P, mp + 8 * (nb - 1), ws.data_ptr(), ws.numel(), sp))
+            for cap in caps:
                 plans.append((at, cap))
                 at += 24 * cap
+            k = len(lists)
+            words = C.c_int64 * k
+            ids, ns, cp = words(*[a for a, _ in lists]), words(*[c for _, c in lists]), words(*caps)
+            d_ns, outs = words(*[mp + 16 * i for i in range(k)]), words(*[a for a, _ in plans])
+            cnts = words(*[mp + 8 * (nb + i * (P + 1)) for i in range(k)])
+            ref = C.addressof
+            ws = _C.WORKSPACE.get(L.sgl_plan_routes_ws_bytes(k, ref(ns), ref(cp)), self.device, sp)
+            _C.check(L.sgl_plan_routes(k, ref(ids), ref(ns), ref(d_ns), self.node_parts.data_ptr(), self.node_parts.numel(), self.pid,
+                                       rt.indptr.data_ptr(), rt.indices.data_ptr(), rt.locs.data_ptr(), P, ref(cp), ref(outs), ref(cnts),
+                                       mp + 8 * (nb - 1), ws.data_ptr(), ws.numel(), sp))
         host = _C.read_words(meta, meta.numel())    # the one synchronisation before the copy
         bits = host[nb - 1] & 0xFFFFFFFF
         if bits:
@@ -183,13 +189,13 @@ class MaterializedMultiLayerBuilder:
         if len(final) >= 2 and final[-1]["indptr"].numel() == 1:
             routes[-1] = None                       # the reference stops at an empty layer with no plan for it
         final[0]["comm_plan"] = routes
+        torch.cuda.current_stream(self.device).synchronize()       # the copies of _export
         return final
 
     def _export(self, picks):
         """Host tensors of device arrays (address, count, bytes per value): views of one buffer per type, filled by one copy
-        each.  The buffers are pinned (a copy to fresh pageable memory takes several times as long) as long as not too
-        much is."""
-        import ctypes as C
+        each -- which the caller waits for.  The buffers are pinned (a copy to fresh pageable memory takes several times as
+        long) as long as not too much is."""
         n, at, offs = len(picks), 0, [0] * len(picks)
         split = 0
         for want in (8, 4):                         # 8-byte values first

@@ -37,6 +37,19 @@ struct Order {
   }
 };
 
+// what `stream` is given from here on comes after everything `producer` has been given so far
+inline int order_after(cudaStream_t stream, cudaStream_t producer) {
+  if (producer == stream) return SGL_OK;
+  static thread_local cudaEvent_t ev[64];
+  int dev = 0;
+  SGL_CUDA_CHECK(cudaGetDevice(&dev));
+  cudaEvent_t& e = ev[dev & 63];
+  if (e == nullptr) SGL_CUDA_CHECK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+  SGL_CUDA_CHECK(cudaEventRecord(e, producer));
+  SGL_CUDA_CHECK(cudaStreamWaitEvent(stream, e, 0));
+  return SGL_OK;
+}
+
 // words of device memory -> pinned host memory, then the flag behind them
 static __global__ void export_words_kernel(const int64_t* __restrict__ src, int64_t* dst, int words, int64_t flag) {
   for (int i = threadIdx.x; i < words; i += blockDim.x) dst[i] = src[i];

@@ -121,7 +121,7 @@ extern "C" int sgl_query(const int64_t* indptr, const int64_t* nbr, const int64_
                          int64_t num_chunks, const int64_t* neg, const int64_t* neg_ts, int64_t n_neg, int fanout, int n_hops, int policy,
                          int equal_root_time, int64_t allowed_offset, int keep_root_time, int id_bits, int ts_bits, int64_t ts_base,
                          int64_t* mapper, int64_t* mask, int64_t epoch, int restart, int64_t* d_next_local, int64_t* arena, int64_t* meta,
-                         int64_t* host_meta, void* ws, size_t ws_bytes, void* stream_) {
+                         int64_t* host_meta, void* ws, size_t ws_bytes, void* producer, void* stream_) {
   SGL_NVTX("sgl_query");
   cudaStream_t stream = (cudaStream_t)stream_;
   SGL_REQUIRE(cap >= 1 && cap < ((int64_t)1 << 31) && n_neg >= 0 && n_hops >= 0 && n_hops <= kMaxHops, SGL_ERR_UNSUPPORTED,
@@ -132,6 +132,7 @@ extern "C" int sgl_query(const int64_t* indptr, const int64_t* nbr, const int64_
               SGL_ERR_ARG, "query: null array");
   SGL_REQUIRE(ws_bytes >= sgl_query_ws_bytes(cap, n_neg, fanout, n_hops), SGL_ERR_WORKSPACE, "query: workspace %zu < %zu bytes", ws_bytes,
               sgl_query_ws_bytes(cap, n_neg, fanout, n_hops));
+  SGL_CHECK_RC(order_after(stream, (cudaStream_t)producer));
   int64_t size[kHead + kMaxHops * kPerHop + 1];
   query_sections(cap, n_neg, fanout, n_hops, size);
   int64_t* p = arena;

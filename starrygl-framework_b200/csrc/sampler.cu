@@ -683,15 +683,7 @@ extern "C" int sgl_prefetch_batch(const int64_t* host_roots, const int64_t* host
   SGL_NVTX("sgl_prefetch_batch");
   cudaStream_t stream = (cudaStream_t)stream_;
   SGL_REQUIRE(n_targets >= 0 && host_total && (host_roots == nullptr) == (host_ts == nullptr), SGL_ERR_ARG, "prefetch_batch: bad argument");
-  if (consumer != stream_) {
-    static thread_local cudaEvent_t ev[64];
-    int dev = 0;
-    SGL_CUDA_CHECK(cudaGetDevice(&dev));
-    cudaEvent_t& e = ev[dev & 63];
-    if (e == nullptr) SGL_CUDA_CHECK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-    SGL_CUDA_CHECK(cudaEventRecord(e, (cudaStream_t)consumer));
-    SGL_CUDA_CHECK(cudaStreamWaitEvent(stream, e, 0));
-  }
+  SGL_CHECK_RC(order_after(stream, (cudaStream_t)consumer));
   LaunchScope scope(stream);
   if (host_roots && n_targets > 0)
     SGL_CHECK_RC(launch(stage_roots_kernel, (unsigned)((n_targets + 255) / 256), 256, 0, stream, host_roots, host_ts, n_targets, targets,

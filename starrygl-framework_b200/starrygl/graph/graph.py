@@ -48,9 +48,10 @@ class pyGraph:
         if op is not None and not isinstance(op, str):
             raise TypeError("op must be a str")
         ctx = DistributedContext.get_default_context()
-        empty = torch.tensor([], dtype=torch.long, device=ctx.device)
-        neg = test_generate_kwargs.get('test_generate_samples', empty)
-        neg_ts = test_generate_kwargs.get('test_generate_samples_ts', empty)
+        neg, neg_ts = test_generate_kwargs.get('test_generate_samples'), test_generate_kwargs.get('test_generate_samples_ts')
+        if neg is None or neg_ts is None:
+            empty = torch.empty(0, dtype=torch.long, device=ctx.device)
+            neg, neg_ts = empty if neg is None else neg, empty if neg_ts is None else neg_ts
         if policy['sample_type'] == 'cluster':
             return self.g.submit_query(time_start, time_end, chunk_list.to(ctx.device), neg.to(ctx.device),
                                        neg_ts.to(ctx.device), 'cluster', 1, 0, 0, 0, 0, op)

@@ -21,6 +21,7 @@ import queue
 import threading
 from bisect import bisect_left
 from collections import deque
+from functools import lru_cache
 from typing import List, Optional
 
 import torch
@@ -326,6 +327,11 @@ class _QueryFuture:
         return out
 
 
+@lru_cache(maxsize=16)
+def _hop_words(hops):
+    return C.c_int64 * hops               # (making an array type takes longer than filling one in)
+
+
 def query_blocks(root, neg_roots, neighbors):
     """Source nodes, source times and column indices of the blocks of a query's hops (self loops included) in one launch;
     None when the parts are not those of one query as ``CUDAGraph.get`` returned it.  Yields (dst count, nid, ts, indices)."""
@@ -337,17 +343,19 @@ def query_blocks(root, neg_roots, neighbors):
         return None
     n_neg = 0 if neg_roots is None else neg_roots.root_num
     # (roots whose tensors were handed out may have been replaced: then the general path takes what they hold now)
-    if n_neg != a.n_queries - a.n_pairs or any(root.__dict__.get(k, a.buf).untyped_storage().data_ptr() != a.buf.untyped_storage().data_ptr()
-                                               for k in ("roots", "ts", "ts_ptr")):
+    if n_neg != a.n_queries - a.n_pairs:
         return None
-    import ctypes as C
+    if any(k in root.__dict__ and root.__dict__[k].untyped_storage().data_ptr() != a.buf.untyped_storage().data_ptr()
+           for k in ("roots", "ts", "ts_ptr")):
+        return None
     hops = a.hops
     dst = [a.n_queries] + a.edges[:-1]
     total = sum(2 * (d + n) + n for d, n in zip(dst, a.edges))
     out = torch.empty(total, dtype=torch.int64, device=a.buf.device)
-    node = (C.c_void_p * hops)(*[a.ptr(7 + 8 * l + 6) for l in range(hops)])
-    ts = (C.c_void_p * hops)(*[a.ptr(7 + 8 * l + 2) for l in range(hops)])
-    cnt = (C.c_int64 * hops)(*a.edges)
+    kind, base, start = _hop_words(hops), a.buf.data_ptr(), a.start
+    node = kind(*[base + 8 * start[7 + 8 * l + 6] for l in range(hops)])
+    ts = kind(*[base + 8 * start[7 + 8 * l + 2] for l in range(hops)])
+    cnt = kind(*a.edges)
     _C.check(_C.lib().sgl_query_blocks(hops, node, ts, cnt, a.ptr(6), a.ptr(2), a.ptr(1), None if n_neg == 0 else neg_roots.roots.data_ptr(),
                                        a.n_roots, a.n_pairs, a.n_queries, out.data_ptr(), _C.stream_ptr()))
     blocks, at = [], 0
@@ -521,10 +529,12 @@ class CUDAGraph:
             if len(self._plans) > 64:
                 self._plans.clear()
             plan = self._plans[key] = _QueryPlan(*key)
-        self.stream.wait_stream(torch.cuda.current_stream(dev))
-        with torch.cuda.stream(self.stream):
+        producer = _C.stream_ptr() if torch._C._cuda_getDevice() == dev.index else torch.cuda.current_stream(dev).cuda_stream
+        neg_ids, neg_ts = neg.roots.contiguous(), neg.ts.contiguous()
+        if self.mapper is not None and chunks is not None and self.mapper.numel():
+            self.stream.wait_stream(torch.cuda.current_stream(dev))
+        with _C.on_stream(self.stream):
             mask, node_chunk, n_chunks = ops.chunk_mask(g, chunks, self.mapper)
-            neg_ids, neg_ts = neg.roots.contiguous(), neg.ts.contiguous()
             buf = torch.empty(plan.words + 10 + 2 * layers, dtype=torch.int64, device=dev)
             ws = _C.WORKSPACE.get(plan.ws_bytes, dev, sp)
         rl = self.relabel
@@ -540,7 +550,7 @@ class CUDAGraph:
             neg_ids.data_ptr() if n_neg else None, neg_ts.data_ptr() if n_neg else None, n_neg, fanout, layers, _C.POLICY[stype],
             int(eq), off, int(keep), ops.bits_for(g.num_nodes - 1), ops.bits_for(g.ts_max - g.ts_min), g.ts_min, rl.mapper.data_ptr(),
             rl.mask.data_ptr(), rl.epoch, int(op == "f"), rl.next_local.data_ptr(), base, base + 8 * plan.words, slot[0], ws.data_ptr(),
-            ws.numel(), sp))
+            ws.numel(), producer, sp))
         fut = _QueryFuture(self, slot, buf, plan, layers, neg)
         fut._keep = (neg_ids, neg_ts, mask)   # inputs of kernels that may still be queued
         return fut

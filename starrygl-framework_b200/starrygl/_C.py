@@ -184,6 +184,21 @@ def stream_ptr(stream=None):
     return torch.cuda.current_stream().cuda_stream
 
 
+_STREAMS = {}
+
+
+def current_stream(device=None):
+    """torch.cuda.current_stream(device) with the Stream objects kept (by stream, as many as a program has)."""
+    index = None if device is None else device.index
+    key = torch._C._cuda_getCurrentStream(torch._C._cuda_getDevice() if index is None else index)
+    s = _STREAMS.get(key)
+    if s is None:
+        if len(_STREAMS) >= 256:
+            _STREAMS.clear()
+        s = _STREAMS[key] = torch.cuda.Stream(stream_id=key[0], device_index=key[1], device_type=key[2])
+    return s
+
+
 class on_stream:
     """``with torch.cuda.stream(s)`` for a stream of the current device, at a fifth of its cost (other devices: that)."""
 

@@ -33,7 +33,7 @@ class PrefetchedBatch:
 
     def wait(self, stream: Optional[torch.cuda.Stream] = None):
         """Make ``stream`` (default: the current one) wait for this batch -- no host blocking."""
-        (stream or torch.cuda.current_stream()).wait_event(self.ready)
+        (stream or _C.current_stream()).wait_event(self.ready)
         return self
 
     def num_edges(self) -> int:

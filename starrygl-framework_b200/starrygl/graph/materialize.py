@@ -189,7 +189,7 @@ class MaterializedMultiLayerBuilder:
         if len(final) >= 2 and final[-1]["indptr"].numel() == 1:
             routes[-1] = None                       # the reference stops at an empty layer with no plan for it
         final[0]["comm_plan"] = routes
-        torch.cuda.current_stream(self.device).synchronize()       # the copies of _export
+        _C.current_stream(self.device).synchronize()               # the copies of _export
         return final
 
     def _export(self, picks):

@@ -413,9 +413,10 @@ ts_part_kernel(Source src, int pos_bits, Scratch sc) {
   const int buckets = tiles;             // one bucket per tile (two smaller ones were slower)
   if (tiles > 1) {
     // (more than one tile: n is above (tiles - 1) * 256, the sample is smaller than the list)
-    // 14 - 16 samples per bucket: the largest bucket is about 1.7 times the mean.  From 31 to 148 short tiles seven have to
-    // do: sorting twice as many costs more than the larger buckets do.
-    const int sb = tiles <= 16 ? 8 : (tiles <= 32 ? 9 : (n < 60000 ? 10 : 11)), s = 1 << sb;
+    // Samples: sorting more costs more, fewer leave larger buckets.  Measured with 148 buckets (512, 1,024, 2,048 samples): 60,000
+    // keys 29, 31, 35 us; 144,000 keys 41, 37, 41 us; 300,000 keys (57), 57, 53 us.  Buckets of 3.5 samples are at most about
+    // four times the mean, of 14 about 1.7 times.
+    const int sb = tiles <= 8 ? 8 : (n < 70000 ? 9 : (n < 220000 ? 10 : 11)), s = 1 << sb;
     for (int j = tid; j < s; j += kThreads) {
       const int i = sample_at(j, sb, (int)n);
       sm.v.set(j, make_item<WIDE>(src.key(i), (uint32_t)i, pos_bits));
@@ -580,9 +581,10 @@ int launch_as(const Source& src, const Sink& sink, int64_t n_cap, int pos_bits, 
   const int64_t min_tiles = (n_cap + kMinTile - 1) / kMinTile;
   const int ctas = (int)(min_tiles < kMaxCtas ? min_tiles : kMaxCtas);
   const int tile = tile_for(n_cap, ctas);
-  // a bucket is about a tile, up to twice that; what does not fit goes through global memory
+  // a bucket is about a tile, up to twice that, and with few samples per bucket (more than 64 of them) up to five times; what does
+  // not fit goes through global memory
   constexpr int kCapMost = WIDE ? 6912 : 9216;
-  const int cap = 4 * tile < kCapMost ? 4 * tile : kCapMost;
+  const int room = (ctas > 64 ? 8 : 4) * tile, cap = room < kCapMost ? room : kCapMost;
   SGL_CUDA_CHECK(allow_smem((const void*)ts_bucket_kernel<Source, Sink, WIDE>, bucket_done, Arrays<WIDE>::bytes(kCapMost)));
   SGL_CUDA_CHECK(allow_smem((const void*)ts_part_kernel<Source, WIDE, Sink::kPred>, part_done, Arrays<WIDE>::bytes(kMaxSamples)));
   SGL_CHECK_RC(launch(ts_part_kernel<Source, WIDE, Sink::kPred>, ctas, kThreads, Arrays<WIDE>::bytes(kMaxSamples), stream,

@@ -5,8 +5,8 @@ namespace sgl {
 
 __device__ __forceinline__ uint64_t low_mask(int bits) { return bits >= 64 ? ~0ull : ((1ull << bits) - 1ull); }
 
-// Producers and consumers for the mini-batch sort: the dedup / relabel operations on lists of at most tilesort::kMaxItems
-// entries, fused into its two kernels (pack, sort passes, head scan and emit were 8 - 9 kernels and a memset).
+// Producers and consumers of sorted lists: the dedup / relabel operations, fused into the sort's kernels (sort_list in lsd.cuh;
+// pack, sort passes, head scan and emit were 8 - 9 kernels and a memset).
 struct PairSource {
   const int64_t *a_id, *a_ts, *d_n_a, *b_id, *b_ts, *d_n_b;
   int64_t n_a, n_b;

@@ -493,7 +493,8 @@ class CUDAGraph:
     def _window(self, t0, t1):
         """Host-known bounds of the window's events: (first, at most) from every 256th timestamp of the stream."""
         if self._ev_index is None:
-            self._ev_index = self.ev[1][::256].cpu().numpy()
+            with torch.cuda.stream(self.stream):      # (events out of order are still being sorted there)
+                self._ev_index = self.ev[1][::256].cpu().numpy()
         idx, m = self._ev_index, self.ev[1].numel()
         first = max(bisect_left(idx, t0) - 1, 0) * 256
         last = min(bisect_left(idx, t1) * 256, m)

@@ -172,3 +172,27 @@ def test_slice_window_capacity_overflow_is_reported():
         ops.slice_window(g, None, None, 0, 100, 10, status=st)
     out = ops.slice_window(g, None, None, 0, 100, 2000, status=st)
     assert out[4].numel() == 2000
+
+
+def test_query_right_after_construction_of_unordered_events():
+    """Events out of time order are sorted on the graph's own stream; the first query's window is looked up behind that sort."""
+    from starrygl.lib import libstarrygl_comm as L
+    n, m = 1000, 24_000_000
+    gen = torch.Generator(device="cuda").manual_seed(5)
+    src, dst = (torch.randint(0, n, (m,), device="cuda", generator=gen) for _ in range(2))
+    ts = torch.randint(0, 10_000_000, (m,), device="cuda", generator=gen)
+    eid = torch.arange(m, device="cuda")
+    none = torch.empty(0, dtype=torch.int64, device="cuda")
+    t0, t1 = 5_000_000, 5_002_000
+    sel = ((ts >= t0) & (ts < t1)).nonzero().view(-1)
+    want = ref_seeds(npy(src[sel]), npy(ts[sel]), npy(sel), t0, t1)
+    assert len(want[4]) > 3000
+    for _ in range(2):              # (the first round loads kernels and allocates, which waits for the GPU)
+        torch.cuda.synchronize()
+        g = L.from_edge_index(n, 1, src, dst, ts, eid)
+        g.submit_query(t0, t1, None, none, none, "recent", 1, 5, -1, False, False, "f")
+        r = g.get().roots
+        assert np.array_equal(npy(r.q_eid), want[4]) and np.array_equal(npy(r.ts), want[2])
+        assert np.array_equal(npy(r.ts_ptr), want[1]) and np.array_equal(npy(r.q_ptr), want[3])
+        g.close()
+        del g, r

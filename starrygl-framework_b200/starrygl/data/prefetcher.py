@@ -54,7 +54,8 @@ class HostToDevicePrefetcher:
         self.streams = [torch.cuda.Stream(g.device) for _ in range(self.depth)]
         self.pipes = [SampleGatherPipeline(g, edge_feats, fanout, policy, max_roots, stream=s, **sampler_options)
                       for s in self.streams]
-        self.events = [torch.cuda.Event() for _ in range(self.depth)]
+        self._held = [deque() for _ in range(self.depth)]      # per slot: (event behind a batch, its inputs), oldest first
+        self._spare = [[] for _ in range(self.depth)]          # events of batches that are done
         self._totals = torch.zeros(2 * self.depth, dtype=torch.int64).pin_memory()   # per slot: edges, sequence number
         self._seq, self._fn = 0, _C.lib().sgl_prefetch_batch
         self._bound = [None] * self.depth
@@ -99,16 +100,21 @@ class HostToDevicePrefetcher:
             with torch.cuda.stream(st):
                 pipe.roots[:n].copy_(roots, non_blocking=True)
                 pipe.root_ts[:n].copy_(root_ts, non_blocking=True)
+        # The kernels read the inputs where they are, which no allocator knows: they are held until their batch is done,
+        # whatever becomes of the batch object.
+        held, spare = self._held[slot], self._spare[slot]
+        while held and held[0][0].query():
+            spare.append(held.popleft()[0])
+        ready = spare.pop() if spare else torch.cuda.Event()
         self._seq += 1
         c_n.value, c_seq.value, c_cons.value = n, self._seq, _C.stream_ptr()
         # The call orders the slot's reuse behind everything the consumer has enqueued so far on its stream: the work on the
         # batch that occupied this slot (handed out ``depth`` batches ago) and the kernels that produced ``roots``.
         # The batch submitted now is only needed ``depth`` requests later, so this does not stall the consumer.
         _C.check(self._fn(*args))
-        self.events[slot].record(st)
-        b = PrefetchedBatch(pipe, n, self.events[slot], (addr, words, self._seq))
-        b._keep = (roots, root_ts)        # inputs of kernels that may still be queued
-        return b
+        ready.record(st)
+        held.append((ready, (roots, root_ts)))
+        return PrefetchedBatch(pipe, n, ready, (addr, words, self._seq))
 
     def __iter__(self):
         it = iter(self.loader)
@@ -121,6 +127,14 @@ class HostToDevicePrefetcher:
             slot = (slot + 1) % self.depth
         while queue:
             yield queue.popleft().wait()
+
+    def __del__(self):
+        try:                              # the inputs and counts of batches that are still under way go with the object
+            for held in self._held:
+                if held:
+                    held[-1][0].synchronize()
+        except Exception:
+            pass
 
     def check(self):
         for p in self.pipes:

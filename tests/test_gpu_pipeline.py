@@ -158,3 +158,30 @@ def test_prefetcher_yields_every_batch_in_order(world):
         assert np.array_equal(np.diff(npy(offs)), counts)
         assert np.array_equal(npy(nbr[:tot]), src) and np.array_equal(npy(eid[:tot]), reid) and np.array_equal(npy(dt[:tot]), rdt)
         assert np.array_equal(npy(ef[:tot]), feats_np[reid])
+
+
+def test_prefetcher_holds_pinned_inputs_until_the_gpu_has_read_them(world):
+    """A loader that pins fresh tensors per batch, a GPU that is behind and a consumer that keeps nothing: the blocks of inputs
+    that are still to be read must not come back from the host allocator with the next batch's roots."""
+    from starrygl.data.prefetcher import HostToDevicePrefetcher
+    g, feats, feats_np, batches = world
+
+    def loader():
+        for i in range(12):
+            q, qt, _ = batches[i % len(batches)]
+            yield torch.from_numpy(q).pin_memory(), torch.from_numpy(qt).pin_memory()
+    for warm in (True, False):           # (the first round loads kernels, which waits for the GPU)
+        pf = HostToDevicePrefetcher(loader(), g, feats, K, "recent", B, depth=3)
+        torch.cuda.synchronize()
+        if not warm:
+            torch.cuda._sleep(400_000_000)
+        kept = []
+        for b in pf:
+            kept.append((b.offsets.clone(), b.nbr.clone(), b.eid.clone()))
+            del b
+        torch.cuda.synchronize()
+        pf.check()
+        for i, (offs, nbr, eid) in enumerate(kept):
+            src, dst, ts, rdt, reid, counts = batches[i % len(batches)][2][:6]
+            assert np.array_equal(np.diff(npy(offs)), counts), f"batch {i}"
+            assert np.array_equal(npy(nbr[:len(src)]), src) and np.array_equal(npy(eid[:len(src)]), reid), f"batch {i}"

@@ -26,7 +26,7 @@ class PrefetchedBatch:
 
     def __init__(self, pipe: SampleGatherPipeline, n_roots: int, ready: torch.cuda.Event, total=None):
         self.pipe, self.n_roots, self.ready = pipe, n_roots, ready
-        self._total = total               # (address, ctypes words, sequence number) of the pinned edge count
+        self._total = total               # (address, ctypes words, sequence number, their buffer) of the pinned edge count
         self.offsets, self.nbr, self.dst, self.ts, self.eid, self.dt = (pipe.offsets[:n_roots + 1], pipe.nbr, pipe.dst,
                                                                         pipe.ts, pipe.eid, pipe.dt)
         self.edge_feats = pipe.out_feats
@@ -38,7 +38,7 @@ class PrefetchedBatch:
 
     def num_edges(self) -> int:
         if self._total is not None:
-            addr, words, seq = self._total
+            addr, words, seq, _ = self._total
             if words[1] < seq:
                 _C.check(_C.lib().sgl_wait_word(addr + 8, seq, self.pipe.stream.cuda_stream))
             if words[1] == seq:           # (a later batch of the slot may have overwritten it)
@@ -114,7 +114,7 @@ class HostToDevicePrefetcher:
         _C.check(self._fn(*args))
         ready.record(st)
         held.append((ready, (roots, root_ts)))
-        return PrefetchedBatch(pipe, n, ready, (addr, words, self._seq))
+        return PrefetchedBatch(pipe, n, ready, (addr, words, self._seq, self._totals))
 
     def __iter__(self):
         it = iter(self.loader)

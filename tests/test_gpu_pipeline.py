@@ -185,3 +185,15 @@ def test_prefetcher_holds_pinned_inputs_until_the_gpu_has_read_them(world):
             src, dst, ts, rdt, reid, counts = batches[i % len(batches)][2][:6]
             assert np.array_equal(np.diff(npy(offs)), counts), f"batch {i}"
             assert np.array_equal(npy(nbr[:len(src)]), src) and np.array_equal(npy(eid[:len(src)]), reid), f"batch {i}"
+
+
+def test_edge_counts_of_batches_that_outlive_their_prefetcher(world):
+    from starrygl.data.prefetcher import HostToDevicePrefetcher
+    g, feats, _, batches = world
+    loader = [(cu(q), cu(qt)) for q, qt, _ in batches[:3]]
+    kept = list(HostToDevicePrefetcher(loader, g, feats, K, "recent", B, depth=3))
+    torch.cuda.synchronize()
+    other = [torch.zeros(6, dtype=torch.int64).pin_memory() for _ in range(64)]   # takes the counts' block if it was given back
+    for b, (_, _, want) in zip(kept, batches):
+        assert b.num_edges() == len(want[0])
+    del other

@@ -83,19 +83,20 @@ class HostToDevicePrefetcher:
         n = roots.numel()
         if n > pipe.max_roots:
             raise _C.SglError(f"batch of {n} roots exceeds max_roots={pipe.max_roots}")
-        if roots.dtype != torch.int64 or root_ts.dtype != torch.int64 or root_ts.numel() != n:
-            raise _C.SglError("prefetcher: the loader yields int64 roots and as many int64 query times")
+        as_is = roots.dtype == torch.int64 and root_ts.dtype == torch.int64 and root_ts.numel() == n
+        if roots.is_cuda and not as_is:
+            raise _C.SglError("prefetcher: roots on the GPU are int64 and come with as many int64 query times")
         if self._bound[slot] is None:
             self._bound[slot] = self._bind(slot)
         args, (h_r, h_t, d_r, d_t, c_n, c_seq, c_cons), addr, words = self._bound[slot]
         h_r.value = h_t.value = None
         d_r.value, d_t.value = pipe.roots.data_ptr(), pipe.root_ts.data_ptr()
         roots, root_ts = roots.contiguous(), root_ts.contiguous()
-        if roots.is_cuda:
+        if as_is and roots.is_cuda and root_ts.is_cuda:
             d_r.value, d_t.value = roots.data_ptr(), root_ts.data_ptr()
-        elif roots.is_pinned() and root_ts.is_pinned():
+        elif as_is and roots.is_pinned() and root_ts.is_pinned():
             h_r.value, h_t.value = roots.data_ptr(), root_ts.data_ptr()
-        else:                             # pageable: staged by a copy, behind what the consumer still does with the slot
+        else:                             # pageable, of another type, or one time for all: staged by a copy, behind what the consumer still does with the slot
             st.wait_stream(torch.cuda.current_stream())
             with torch.cuda.stream(st):
                 pipe.roots[:n].copy_(roots, non_blocking=True)

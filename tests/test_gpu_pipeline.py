@@ -197,3 +197,25 @@ def test_edge_counts_of_batches_that_outlive_their_prefetcher(world):
     for b, (_, _, want) in zip(kept, batches):
         assert b.num_edges() == len(want[0])
     del other
+
+
+@pytest.mark.parametrize("form", ["int32", "one time", "times on the host"])
+def test_prefetcher_stages_what_the_kernels_cannot_read(world, form):
+    from starrygl.data.prefetcher import HostToDevicePrefetcher
+    g, feats, _, batches = world
+    loader, want = [], []
+    for q, qt, _ in batches[:3]:
+        r, t = torch.from_numpy(q), torch.from_numpy(qt)
+        if form == "int32":
+            r, t = r.int(), t.int().pin_memory()
+        elif form == "one time":
+            t = torch.tensor([50000])
+        else:
+            r = r.cuda()
+        loader.append((r, t))
+        want.append((q, np.broadcast_to(npy(t).astype(np.int64), q.shape).copy()))
+    csr = [npy(x) for x in (g.indptr, g.nbr, g.ts, g.eid)]
+    for b, (q, qt) in zip(HostToDevicePrefetcher(loader, g, feats, K, "recent", B, depth=2), want):
+        src, dst, ts, dt, eid, counts = O.sample_layer(*csr, q, qt, K, O.RECENT)[:6]
+        assert b.num_edges() == len(src)
+        assert np.array_equal(np.diff(npy(b.offsets)), counts) and np.array_equal(npy(b.eid[:len(src)]), eid)

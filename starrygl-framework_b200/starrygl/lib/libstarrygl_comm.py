@@ -342,6 +342,7 @@ def query_blocks(root, neg_roots, neighbors):
                                        or nb._neighbors_override is not None for l, nb in enumerate(neighbors)):
         return None
     n_neg = 0 if neg_roots is None else neg_roots.root_num
+    neg = neg_roots.roots.contiguous() if n_neg else None          # (a column of a table, say)
     # (roots whose tensors were handed out may have been replaced: then the general path takes what they hold now)
     if n_neg != a.n_queries - a.n_pairs:
         return None
@@ -356,7 +357,7 @@ def query_blocks(root, neg_roots, neighbors):
     node = kind(*[base + 8 * start[7 + 8 * l + 6] for l in range(hops)])
     ts = kind(*[base + 8 * start[7 + 8 * l + 2] for l in range(hops)])
     cnt = kind(*a.edges)
-    _C.check(_C.lib().sgl_query_blocks(hops, node, ts, cnt, a.ptr(6), a.ptr(2), a.ptr(1), None if n_neg == 0 else neg_roots.roots.data_ptr(),
+    _C.check(_C.lib().sgl_query_blocks(hops, node, ts, cnt, a.ptr(6), a.ptr(2), a.ptr(1), None if neg is None else neg.data_ptr(),
                                        a.n_roots, a.n_pairs, a.n_queries, out.data_ptr(), _C.stream_ptr()))
     blocks, at = [], 0
     for d, n in zip(dst, a.edges):

@@ -196,3 +196,35 @@ def test_query_right_after_construction_of_unordered_events():
         assert np.array_equal(npy(r.ts_ptr), want[1]) and np.array_equal(npy(r.q_ptr), want[3])
         g.close()
         del g, r
+
+
+def _blocks_by_parts(res):
+    """to_block from tensors of the general types: the path that takes what the parts hold."""
+    from starrygl.graph.graph import AsyncBlock
+    from starrygl.lib.libstarrygl_comm import TemporalRoot
+    r = res.roots
+    return AsyncBlock.to_block(TemporalRoot(r.roots, r.ts_ptr, r.ts, r.q_ptr, r.q_eid), res.neg_roots, res.neighbors, res.nodes_remapper_id)
+
+
+def _same_blocks(a, b):
+    assert len(a[2]) == len(b[2])
+    for x, y in zip(a[2], b[2]):
+        assert torch.equal(x.indptr, y.indptr) and torch.equal(x.indices, y.indices)
+        for k in ("nid", "ts"):
+            assert torch.equal(x.srcdata[k], y.srcdata[k]), k
+
+
+def test_blocks_with_negatives_out_of_a_table():
+    from starrygl.graph.graph import AsyncBlock, pyGraph
+    n, src, dst, ts, eid = make_events()
+    g = pyGraph(cu(src), cu(dst), cu(ts), n, 1, eid=cu(eid))
+    table = torch.stack([torch.arange(60) * 3 % n, torch.full((60,), 2500), torch.arange(60)], 1).cuda()
+    g.async_sample(2000, 2300, torch.zeros(1, dtype=torch.int64).cuda(), {"sample_type": "recent", "layers": 2, "fanout": 5},
+                   {"test_generate_samples": table[:, 0], "test_generate_samples_ts": table[:, 1]}, op="f")
+    res = g.get_last_sample()
+    got = AsyncBlock.to_block(res.roots, res.neg_roots, res.neighbors, res.nodes_remapper_id)
+    _same_blocks(got, _blocks_by_parts(res))
+    nid = got[2][-1].srcdata["nid"]
+    at = res.roots.root_ts_num
+    assert torch.equal(nid[at:at + 60], table[:, 0])
+    g.g.close()

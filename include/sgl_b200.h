@@ -623,7 +623,7 @@ int sgl_query(const int64_t* indptr, const int64_t* nbr, const int64_t* ts, cons
               int64_t ts_base, int64_t* mapper, int64_t* mask, int64_t epoch, int restart, int64_t* d_next_local,
               int64_t* arena, int64_t* meta, int64_t* host_meta, void* ws, size_t ws_bytes, void* producer, void* stream);
 int sgl_query_blocks(int n_hops, const int64_t* const* node, const int64_t* const* ts, const int64_t* counts,
-                     const int64_t* q_ts, const int64_t* ts_ptr, const int64_t* roots_local, const int64_t* neg,
+                     const int64_t* q_ts, const int64_t* ts_ptr, const int64_t* roots_local, const int64_t* neg, const int64_t* neg_ts,
                      int64_t n_roots, int64_t n_pairs, int64_t n_queries, int64_t* out, void* stream);
 
 /* Small results for the host.  sgl_host_words: a pinned buffer of 512 words that belongs to the calling thread.

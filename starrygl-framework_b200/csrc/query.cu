@@ -213,7 +213,7 @@ struct BlockHop {
 };
 struct Blocks {
   BlockHop hop[kMaxHops];
-  const int64_t *ts_ptr, *roots_local, *neg;
+  const int64_t *ts_ptr, *roots_local, *neg, *neg_ts;
   int64_t n_roots, n_pairs;
 };
 
@@ -228,12 +228,14 @@ __global__ void __launch_bounds__(256) blocks_kernel(const __grid_constant__ Blo
       t = h.ts[j];
       h.out_index[j] = i;
     } else {
-      t = h.prev_ts[i];
       if (blockIdx.y > 0) {
         node = h.prev_node[i];
+        t = h.prev_ts[i];
       } else if (i >= b.n_pairs) {
         node = b.neg[i - b.n_pairs];
+        t = b.neg_ts[i - b.n_pairs];
       } else {
+        t = h.prev_ts[i];
         int64_t lo = 0, hi = b.n_roots;      // root whose pairs hold pair i
         while (hi - lo > 1) {
           const int64_t mid = (lo + hi) >> 1;
@@ -250,14 +252,16 @@ __global__ void __launch_bounds__(256) blocks_kernel(const __grid_constant__ Blo
 }  // namespace sgl
 
 extern "C" int sgl_query_blocks(int n_hops, const int64_t* const* node, const int64_t* const* ts, const int64_t* counts,
-                                const int64_t* q_ts, const int64_t* ts_ptr, const int64_t* roots_local, const int64_t* neg,
+                                const int64_t* q_ts, const int64_t* ts_ptr, const int64_t* roots_local, const int64_t* neg, const int64_t* neg_ts,
                                 int64_t n_roots, int64_t n_pairs, int64_t n_queries, int64_t* out, void* stream_) {
-  SGL_REQUIRE(n_hops >= 1 && n_hops <= kMaxHops && node && ts && counts && q_ts && ts_ptr && out, SGL_ERR_ARG, "query_blocks: bad argument");
+  SGL_REQUIRE(n_hops >= 1 && n_hops <= kMaxHops && node && ts && counts && q_ts && ts_ptr && out &&
+                  (n_queries <= n_pairs || (neg && neg_ts)), SGL_ERR_ARG, "query_blocks: bad argument");
   Blocks b;
   memset(&b, 0, sizeof(b));
   b.ts_ptr = ts_ptr;
   b.roots_local = roots_local;
   b.neg = neg;
+  b.neg_ts = neg_ts;
   b.n_roots = n_roots;
   b.n_pairs = n_pairs;
   int64_t d = n_queries, most = 1;

@@ -234,6 +234,12 @@ class _Arena:
     def ptr(self, section):
         return self.buf.data_ptr() + 8 * self.start[section]
 
+    def holds(self, t, name):
+        """Is ``t`` the root array ``name`` as the query left it?"""
+        section, count, extra = _ArenaRoot._SECTIONS[name]
+        return t.is_cuda and t.dtype == torch.int64 and t.is_contiguous() and t.data_ptr() == self.ptr(section) and \
+            t.numel() == getattr(self, count) + extra
+
 
 class _ArenaRoot(TemporalRoot):
     """Roots of a query under their local ids; the tensors are cut out of the query's arena on first use."""
@@ -254,11 +260,13 @@ class _ArenaRoot(TemporalRoot):
 
     @property
     def root_num(self):
-        return self._a.n_roots
+        t = self.__dict__.get("roots")
+        return self._a.n_roots if t is None else t.numel()
 
     @property
     def root_ts_num(self):
-        return self._a.n_pairs
+        t = self.__dict__.get("ts")
+        return self._a.n_pairs if t is None else t.numel()
 
 
 class _ArenaNeighbor(TemporalNeighbor):
@@ -342,13 +350,14 @@ def query_blocks(root, neg_roots, neighbors):
                                        or nb._neighbors_override is not None for l, nb in enumerate(neighbors)):
         return None
     n_neg = 0 if neg_roots is None else neg_roots.root_num
-    neg = neg_roots.roots.contiguous() if n_neg else None          # (a column of a table, say)
-    # (roots whose tensors were handed out may have been replaced: then the general path takes what they hold now)
-    if n_neg != a.n_queries - a.n_pairs:
+    # parts that were replaced since take the general path, which uses what they hold now
+    if n_neg != a.n_queries - a.n_pairs or any(k in root.__dict__ and not a.holds(root.__dict__[k], k) for k in ("roots", "ts", "ts_ptr")):
         return None
-    if any(k in root.__dict__ and root.__dict__[k].untyped_storage().data_ptr() != a.buf.untyped_storage().data_ptr()
-           for k in ("roots", "ts", "ts_ptr")):
-        return None
+    neg = neg_ts = None
+    if n_neg:
+        neg, neg_ts = neg_roots.roots.contiguous(), neg_roots.ts.contiguous()          # (a column of a table, say)
+        if any(not t.is_cuda or t.dtype != torch.int64 or t.numel() != n_neg for t in (neg, neg_ts)):
+            return None
     hops = a.hops
     dst = [a.n_queries] + a.edges[:-1]
     total = sum(2 * (d + n) + n for d, n in zip(dst, a.edges))
@@ -358,6 +367,7 @@ def query_blocks(root, neg_roots, neighbors):
     ts = kind(*[base + 8 * start[7 + 8 * l + 2] for l in range(hops)])
     cnt = kind(*a.edges)
     _C.check(_C.lib().sgl_query_blocks(hops, node, ts, cnt, a.ptr(6), a.ptr(2), a.ptr(1), None if neg is None else neg.data_ptr(),
+                                       None if neg is None else neg_ts.data_ptr(),
                                        a.n_roots, a.n_pairs, a.n_queries, out.data_ptr(), _C.stream_ptr()))
     blocks, at = [], 0
     for d, n in zip(dst, a.edges):

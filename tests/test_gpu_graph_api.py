@@ -228,3 +228,27 @@ def test_blocks_with_negatives_out_of_a_table():
     at = res.roots.root_ts_num
     assert torch.equal(nid[at:at + 60], table[:, 0])
     g.g.close()
+
+
+@pytest.mark.parametrize("change", ["fewer roots", "negative times", "negatives", "times in place"])
+def test_blocks_of_a_result_that_was_changed(change):
+    from starrygl.graph.graph import AsyncBlock, pyGraph
+    from starrygl.lib.libstarrygl_comm import NegativeRoot
+    n, src, dst, ts, eid = make_events()
+    g = pyGraph(cu(src), cu(dst), cu(ts), n, 1, eid=cu(eid))
+    neg, neg_ts = (torch.arange(40) * 7 % n).cuda(), torch.full((40,), 2500).cuda()
+    g.async_sample(2000, 2300, torch.zeros(1, dtype=torch.int64).cuda(), {"sample_type": "recent", "layers": 1, "fanout": 5},
+                   {"test_generate_samples": neg, "test_generate_samples_ts": neg_ts}, op="f")
+    res = g.get_last_sample()
+    r = res.roots
+    if change == "fewer roots":
+        r.roots, r.ts_ptr, r.ts = r.roots[:10], r.ts_ptr[:11], r.ts[:int(r.ts_ptr[10])]
+        assert r.root_num == 10 and r.root_ts_num == r.ts.numel()
+    elif change == "negative times":
+        res.neg_roots.ts = neg_ts + 1
+    elif change == "negatives":
+        res.neg_roots = NegativeRoot((neg + 1) % n, neg_ts - 5)
+    else:
+        neg_ts += 3
+    _same_blocks(AsyncBlock.to_block(r, res.neg_roots, res.neighbors, res.nodes_remapper_id), _blocks_by_parts(res))
+    g.g.close()

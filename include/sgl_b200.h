@@ -58,6 +58,9 @@ const char* sgl_build_info(void);
  * Stable LSD radix sort of 64-bit keys carrying a 32-bit payload (used by the T-CSR build and the
  * relabel; exported so it can be tested on its own).  Sorts on key bits [0, num_bits).  On return
  * *h_result_in_alt tells whether the sorted data are in (keys, vals) [0] or in (keys_alt, vals_alt) [1].
+ * Lists above 1,212,416 keys: the passes wait for each other's tiles, for 2 s at most; the call waits for their end and returns
+ * SGL_ERR_CUDA if one gave up (a capturing stream: not reported).  sgl_look_back_limit sets that limit, in nanoseconds, for the
+ * calls that the calling thread makes from then on (negative: unchanged) and returns the one before.
  * Replaces: thrust::sort calls in csrc/include/starrygl/sample.cu.hpp:1078, :1197, :1795.
  * ---------------------------------------------------------------------------------------------- */
 size_t sgl_radix_sort_ws_bytes(int64_t n);
@@ -65,13 +68,15 @@ size_t sgl_radix_sort_ws_bytes(int64_t n);
 int sgl_radix_sort_launches(int64_t n, int num_bits);
 int sgl_radix_sort_u64_u32(uint64_t* keys, uint32_t* vals, uint64_t* keys_alt, uint32_t* vals_alt, int64_t n,
                            int num_bits, int* h_result_in_alt, void* ws, size_t ws_bytes, void* stream);
+int64_t sgl_look_back_limit(int64_t ns);
 
 /* ------------------------------------------------------------------------------------------------
  * T-CSR construction.  Rows are keyed by `key` (node id in [0, num_nodes)); inside a row edges are in
  * ascending `ts`, ties in input order.  eid may be NULL (edge id = input position).
  * Outputs: indptr[num_nodes+1], nbr/ts/eid[m] in row order, perm[m] (optional) = input position of
  * every sorted edge.  h_ts_range[2] (optional, host) receives min and max timestamp.
- * Synchronises the stream once (the number of sort passes depends on the timestamp range).
+ * Waits for the stream once (the number of sort passes depends on the timestamp range), and above 1,212,416 edges for the end of
+ * the build: SGL_ERR_CUDA when a wait inside the sort gave up (see sgl_look_back_limit).
  * Replaces: Graph::Graph + build_graph_kernel (csrc/include/starrygl/sample.cu.hpp:985-1185, :83-114)
  * reached through from_edge_index (csrc/srcs/starrygl/export.cu:229-250); CPU twin
  * MaterializedMultiLayerBuilder.__init__ (prepare_sample.py:179-203).

@@ -96,7 +96,11 @@ __global__ void zero_words_kernel(uint32_t* p, size_t n) {
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) p[i] = 0;
 }
 
+thread_local int64_t t_look_back_ns = 2000000000;
+
 }  // namespace
+
+unsigned long long look_back_ns() { return (unsigned long long)t_look_back_ns; }
 
 int zero_async(void* p, size_t bytes, cudaStream_t stream) {
   if (LaunchScope::current() == nullptr) {
@@ -218,3 +222,9 @@ int LaunchScope::submit() {
 }
 
 }  // namespace sgl
+
+extern "C" int64_t sgl_look_back_limit(int64_t ns) {
+  const int64_t before = sgl::t_look_back_ns;
+  if (ns >= 0) sgl::t_look_back_ns = ns;
+  return before;
+}

@@ -85,6 +85,9 @@ int launch(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStr
 // Zero bytes (a multiple of four, four-byte aligned) in stream order, in a launch scope or not.
 int zero_async(void* p, size_t bytes, cudaStream_t stream);
 
+// How long the look-backs of lsd.cuh wait for the tiles before them, see sgl_look_back_limit.
+unsigned long long look_back_ns();
+
 // kernels that need more than 48 KB of shared memory say so once per device
 inline cudaError_t allow_smem(const void* kernel, std::atomic<uint64_t>& done, size_t bytes) {
   int dev = 0;

@@ -95,7 +95,6 @@ static __global__ void __launch_bounds__(kRadix) lsd_scan_kernel(unsigned long l
 // tiles before it.  Words of an earlier pass count as not published, so the array is cleared once per sort.
 constexpr uint64_t kOwn = 1ull << 62, kAll = 2ull << 62, kValue = (1ull << 56) - 1;
 __device__ __forceinline__ uint64_t pass_tag(int pass) { return (uint64_t)(pass + 1) << 56; }
-constexpr unsigned long long kLookLimitNs = 2000000000ull;
 
 template <class V>
 struct LsdSmem {
@@ -111,7 +110,8 @@ struct LsdSmem {
 // where a pass reads its items from: the arrays of the pass before, or (first pass) the producer of the keys
 // Sum of what the tiles before this one hold of digit threadIdx.x; publishes it with the tile's own.
 template <int kWide>
-__device__ __forceinline__ uint64_t look_back(uint64_t* state, int pass, int tile, uint32_t total, unsigned int* gave_up, int32_t* d_status) {
+__device__ __forceinline__ uint64_t look_back(uint64_t* state, int pass, int tile, uint32_t total, unsigned long long limit, unsigned int* gave_up,
+                                              int32_t* d_status) {
   const uint64_t tag = pass_tag(pass);
   volatile uint64_t* st = state + threadIdx.x;
   uint64_t sum = 0;
@@ -138,7 +138,7 @@ __device__ __forceinline__ uint64_t look_back(uint64_t* state, int pass, int til
       unsigned long long now;
       asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(now));
       if (t0 == 0) t0 = now;
-      if (now - t0 > kLookLimitNs) {
+      if (now - t0 > limit) {
         dev_flag(d_status, SGL_DEV_TIMEOUT);
         *(volatile unsigned int*)gave_up = 1u;
         break;
@@ -184,7 +184,7 @@ template <class V, class Items, class Out>
 __global__ void __launch_bounds__(kLsdThreads, kLsdCtas)
 lsd_pass_kernel(Items items, Digit digit, int pass,
                 const unsigned long long* __restrict__ starts, unsigned int* __restrict__ ticket, uint64_t* state,
-                Out out, unsigned int* gave_up, int32_t* d_status) {
+                Out out, unsigned long long limit, unsigned int* gave_up, int32_t* d_status) {
   extern __shared__ __align__(16) unsigned char smem[];
   LsdSmem<V>& sm = *(LsdSmem<V>*)smem;
   constexpr int kItems = kLsdItems<V>, kTile = kLsdTile<V>;
@@ -268,7 +268,7 @@ lsd_pass_kernel(Items items, Digit digit, int pass,
     }
   }
   if (tid < kRadix) {
-    const uint64_t sum = tile > 0 ? look_back<kLookWide<V>>(state, pass, tile, total, gave_up, d_status) : 0;
+    const uint64_t sum = tile > 0 ? look_back<kLookWide<V>>(state, pass, tile, total, limit, gave_up, d_status) : 0;
     sm.out[tid] = (uint32_t)(starts[tid] + sum) - start;
   }
   __syncthreads();
@@ -310,7 +310,7 @@ constexpr int kDeliverItems = 8;
 constexpr int kDeliverTile = kDeliverThreads * kDeliverItems;
 
 // Sum of what the CTAs before this one (by ticket: they all run already) published; called by one whole warp.
-__device__ __forceinline__ uint64_t deliver_prefix(uint64_t* state, int tile, uint64_t total, int lane, int32_t* d_status) {
+__device__ __forceinline__ uint64_t deliver_prefix(uint64_t* state, int tile, uint64_t total, int lane, unsigned long long limit, int32_t* d_status) {
   volatile uint64_t* st = state;
   if (lane == 0) st[tile] = tile == 0 ? (kAll | total) : (kOwn | total);
   constexpr uint64_t kSum = (1ull << 62) - 1;
@@ -324,7 +324,7 @@ __device__ __forceinline__ uint64_t deliver_prefix(uint64_t* state, int tile, ui
       unsigned long long now;
       asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(now));
       if (t0 == 0) t0 = now;
-      if (__any_sync(0xffffffffu, now - t0 > kLookLimitNs)) {
+      if (__any_sync(0xffffffffu, now - t0 > limit)) {
         if (lane == 0) dev_flag(d_status, SGL_DEV_TIMEOUT);
         break;
       }
@@ -347,7 +347,7 @@ __device__ __forceinline__ uint64_t deliver_prefix(uint64_t* state, int tile, ui
 template <class Sink>
 __global__ void __launch_bounds__(kDeliverThreads, 4)
 lsd_deliver_kernel(Sink sink, const uint64_t* __restrict__ keys, const uint32_t* __restrict__ pos, int64_t n_cap, const int64_t* d_count,
-                   unsigned long long* ctl, uint64_t* state, const unsigned int* gave_up, int32_t* d_status) {
+                   unsigned long long* ctl, uint64_t* state, unsigned long long limit, const unsigned int* gave_up, int32_t* d_status) {
   const int64_t n = *gave_up ? 0 : eff_count(n_cap, d_count);     // (a pass that gave up left places unwritten)
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   sink.begin();
@@ -414,7 +414,7 @@ lsd_deliver_kernel(Sink sink, const uint64_t* __restrict__ keys, const uint32_t*
     const uint64_t ex = cta_exclusive_scan<kDeliverThreads, uint64_t>(mine, &total);
     if (tid < kCells) s_scan[tid] = ex;
     if (warp == 0) {
-      const uint64_t base = deliver_prefix(state, tile, total, lane, d_status);
+      const uint64_t base = deliver_prefix(state, tile, total, lane, limit, d_status);
       if (lane == 0) s_base = base;
     }
     __syncthreads();
@@ -471,7 +471,7 @@ int lsd_sort(const Items& items, uint64_t* k1, V* v1, uint64_t* k0, V* v0, int64
       static std::atomic<uint64_t> done{0};
       SGL_CUDA_CHECK(allow_smem((const void*)lsd_pass_kernel<V, From, To>, done, sizeof(LsdSmem<V>)));
       return launch(lsd_pass_kernel<V, From, To>, (unsigned)tiles, kLsdThreads, sizeof(LsdSmem<V>), stream, from, Digit{first_bit + p * bits, bits},
-                    p, hist + p * kRadix, tickets + p, state, to, *gave_up, d_status);
+                    p, hist + p * kRadix, tickets + p, state, to, look_back_ns(), *gave_up, d_status);
     };
     const bool to_last = !kArray && p == passes - 1;
     if (p == 0) SGL_CHECK_RC(to_last ? pass(items, last) : pass(items, out));
@@ -512,7 +512,7 @@ int sort_list(const Source& src, const Sink& sink, int64_t n_cap, int key_bits, 
   SGL_CHECK_RC((lsd_sort<uint32_t, SourceItems<Source>>(SourceItems<Source>{src}, k1, v1, k0, v0, n_cap, count, count, 0, key_bits,
                                                         ArrayOut<uint32_t>{}, &in_first, &gave_up, c, d_status, stream)));
   return launch(lsd_deliver_kernel<Sink>, (unsigned)tiles, kDeliverThreads, 0, stream, sink, in_first ? k1 : k0, in_first ? v1 : v0, n_cap,
-                count, ctl, (uint64_t*)(ctl + 2), gave_up, d_status);
+                count, ctl, (uint64_t*)(ctl + 2), look_back_ns(), gave_up, d_status);
 }
 
 }  // namespace

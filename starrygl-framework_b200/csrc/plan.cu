@@ -299,7 +299,7 @@ extern "C" int sgl_plan_route(const int64_t* layer_ids, int64_t n, const int64_t
                       tmp_locs, d_status));
 
   int in_alt = 0;
-  int rc = radix_sort_pairs(k0, v0, k1, v1, capc, d_total, bits_for((uint64_t)(num_parts - 1)), true, &in_alt, sort_ws, sort_bytes,
+  int rc = radix_sort_pairs(k0, v0, k1, v1, capc, d_total, bits_for((uint64_t)(num_parts - 1)), true, &in_alt, d_status, sort_ws, sort_bytes,
                             stream);
   if (rc) return rc;
   SGL_CHECK_RC(launch(plan_emit_kernel, stream_grid(capc, kThreads, 8), kThreads, 0, stream, in_alt ? k1 : k0, in_alt ? v1 :

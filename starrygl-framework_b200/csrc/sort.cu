@@ -48,12 +48,12 @@ struct IotaItems {
 }  // namespace
 
 size_t radix_sort_ws_bytes(int64_t n) {
-  return n <= tilesort::kMaxItems ? tilesort::ws_bytes(n) : lsd_ws_bytes<uint32_t>(n);
+  return align_up(8) + (n <= tilesort::kMaxItems ? tilesort::ws_bytes(n) : lsd_ws_bytes<uint32_t>(n));     // (8: a status word)
 }
 
 int radix_sort_pairs(uint64_t* keys, uint32_t* vals, uint64_t* keys_alt, uint32_t* vals_alt, int64_t n,
-                     const int64_t* d_n, int num_bits, bool iota_vals, int* result_in_alt, void* ws, size_t ws_bytes,
-                     cudaStream_t stream) {
+                     const int64_t* d_n, int num_bits, bool iota_vals, int* result_in_alt, int32_t* d_status, void* ws,
+                     size_t ws_bytes, cudaStream_t stream) {
   SGL_REQUIRE(n >= 0 && n < ((int64_t)1 << 32), SGL_ERR_ARG, "radix sort: n=%lld outside [0, 2^32)", (long long)n);
   SGL_REQUIRE(num_bits >= 0 && num_bits <= 64, SGL_ERR_ARG, "radix sort: num_bits=%d", num_bits);
   *result_in_alt = 0;
@@ -67,17 +67,17 @@ int radix_sort_pairs(uint64_t* keys, uint32_t* vals, uint64_t* keys_alt, uint32_
     const uint64_t mask = num_bits >= 64 ? ~0ull : ((1ull << num_bits) - 1ull);
     *result_in_alt = 1;
     SGL_CHECK_RC(tilesort::launch(RawSource{keys, n, d_n, mask}, RawSink{keys, iota_vals ? nullptr : vals, keys_alt, vals_alt, mask}, n,
-                                  num_bits, sc, nullptr, stream));
+                                  num_bits, sc, d_status, stream));
     return scope.submit();
   }
   bool alt = false;
   unsigned int* gave_up;
   if (iota_vals)
     SGL_CHECK_RC((lsd_sort<uint32_t, IotaItems>(IotaItems{keys, n, d_n}, keys_alt, vals_alt, keys, vals, n, d_n, nullptr, 0, num_bits, ArrayOut<uint32_t>{}, &alt, &gave_up, c,
-                                                nullptr, stream)));
+                                                d_status, stream)));
   else
     SGL_CHECK_RC((lsd_sort<uint32_t, ArrayItems<uint32_t>>(ArrayItems<uint32_t>{keys, vals, n, d_n}, keys_alt, vals_alt, keys, vals, n,
-                                                           d_n, nullptr, 0, num_bits, ArrayOut<uint32_t>{}, &alt, &gave_up, c, nullptr, stream)));
+                                                           d_n, nullptr, 0, num_bits, ArrayOut<uint32_t>{}, &alt, &gave_up, c, d_status, stream)));
   *result_in_alt = alt ? 1 : 0;
   return scope.submit();
 }
@@ -96,6 +96,21 @@ extern "C" int sgl_radix_sort_launches(int64_t n, int num_bits) {
 extern "C" int sgl_radix_sort_u64_u32(uint64_t* keys, uint32_t* vals, uint64_t* keys_alt, uint32_t* vals_alt, int64_t n,
                                       int num_bits, int* h_result_in_alt, void* ws, size_t ws_bytes, void* stream) {
   int dummy = 0;
-  return sgl::radix_sort_pairs(keys, vals, keys_alt, vals_alt, n, nullptr, num_bits, false,
-                               h_result_in_alt ? h_result_in_alt : &dummy, ws, ws_bytes, (cudaStream_t)stream);
+  int* const in_alt = h_result_in_alt ? h_result_in_alt : &dummy;
+  if (n <= sgl::tilesort::kMaxItems)     // (nothing in it waits)
+    return sgl::radix_sort_pairs(keys, vals, keys_alt, vals_alt, n, nullptr, num_bits, false, in_alt, nullptr, ws, ws_bytes, (cudaStream_t)stream);
+  const size_t head = sgl::align_up(8);
+  SGL_REQUIRE(ws && ws_bytes >= sgl::radix_sort_ws_bytes(n), SGL_ERR_WORKSPACE, "radix sort: workspace %zu < %zu bytes", ws_bytes,
+              sgl::radix_sort_ws_bytes(n));
+  int64_t* status = (int64_t*)ws;
+  SGL_CUDA_CHECK(cudaMemsetAsync(status, 0, 8, (cudaStream_t)stream));
+  SGL_CHECK_RC(sgl::radix_sort_pairs(keys, vals, keys_alt, vals_alt, n, nullptr, num_bits, false, in_alt, (int32_t*)status, (char*)ws + head,
+                                     ws_bytes - head, (cudaStream_t)stream));
+  cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+  SGL_CUDA_CHECK(cudaStreamIsCapturing((cudaStream_t)stream, &st));
+  if (st != cudaStreamCaptureStatusNone) return SGL_OK;
+  int64_t bits = 0;
+  SGL_CHECK_RC(sgl_read_back(status, &bits, 8, stream));
+  SGL_REQUIRE(bits == 0, SGL_ERR_CUDA, "radix sort: a look-back over the tiles ran into its time limit");
+  return SGL_OK;
 }

@@ -25,6 +25,7 @@ struct InputScan {
   unsigned long long bad_keys;
   unsigned long long flags;          // kUnordered | kWideIds
   unsigned long long arrived;
+  long long status;                  // (low half) status word of the sort: a look-back that gave up
 };
 constexpr unsigned long long kUnordered = 1, kWideIds = 2, kSign = 1ull << 63;
 
@@ -178,9 +179,9 @@ struct EdgeOut {
 };
 
 __global__ void __launch_bounds__(256)
-tcsr_rows_kernel(const unsigned int* gave_up, const uint32_t* __restrict__ node, int64_t m, int64_t num_nodes, int64_t* __restrict__ indptr) {
+tcsr_rows_kernel(const InputScan* scan, const uint32_t* __restrict__ node, int64_t m, int64_t num_nodes, int64_t* __restrict__ indptr) {
   const int64_t stride = (int64_t)gridDim.x * 256;
-  if (*gave_up) {                          // (a look-back ran into its time limit: no rows rather than wrong ones)
+  if (scan->status) {                      // (the host reports it; no rows rather than wrong ones)
     for (int64_t v = (int64_t)blockIdx.x * 256 + threadIdx.x; v <= num_nodes; v += stride) indptr[v] = 0;
     return;
   }
@@ -206,19 +207,22 @@ tcsr_rows_kernel(const unsigned int* gave_up, const uint32_t* __restrict__ node,
 
 // combined == 0: the keys are node ids and the timestamps are gathered too
 __global__ void __launch_bounds__(256)
-tcsr_emit_gather_kernel(const uint64_t* __restrict__ keys, const uint32_t* __restrict__ perm, int combined, EdgeKey k,
+tcsr_emit_gather_kernel(const InputScan* scan, const uint64_t* __restrict__ keys, const uint32_t* __restrict__ perm, int combined, EdgeKey k,
                         const int64_t* __restrict__ nbr, const int64_t* __restrict__ eid, int64_t m, int64_t num_nodes,
                         int64_t* __restrict__ indptr, int64_t* __restrict__ out_nbr, int64_t* __restrict__ out_ts,
                         int64_t* __restrict__ out_eid, int64_t* __restrict__ out_perm) {
+  if (scan->status) {
+    for (int64_t v = (int64_t)blockIdx.x * 256 + threadIdx.x; v <= num_nodes; v += (int64_t)gridDim.x * 256) indptr[v] = 0;
+    return;
+  }
   for (int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x; i < m; i += (int64_t)gridDim.x * 256) {
-    const uint32_t p = perm[i] < m ? perm[i] : 0u;      // (a sort that ran into its time limit leaves any value)
+    const uint32_t p = perm[i];
     const uint64_t key = keys[i];
     out_nbr[i] = nbr[p];
     out_ts[i] = combined ? k.time(key) : k.ts[p];
     out_eid[i] = eid ? eid[p] : (int64_t)p;
     if (out_perm) out_perm[i] = (int64_t)p;
-    int64_t node = combined ? k.node(key) : (int64_t)key;
-    node = node < num_nodes ? node : num_nodes;
+    const int64_t node = combined ? k.node(key) : (int64_t)key;
     start_rows(indptr, i > 0 ? (combined ? k.node(keys[i - 1]) : (int64_t)keys[i - 1]) : -1, node, i);
     if (i == m - 1)
       for (int64_t r = node + 1; r <= num_nodes; ++r) indptr[r] = m;
@@ -275,6 +279,7 @@ extern "C" int sgl_tcsr_build_fenced(int64_t num_nodes, int64_t m, const int64_t
   void* rest = (char*)ws + align_up(sizeof(InputScan));
   const size_t rest_bytes = ws_bytes - align_up(sizeof(InputScan));
   const bool small = m <= tilesort::kMaxItems;
+  int32_t* const d_status = (int32_t*)&d_scan->status;
   void* words = nullptr;
   SGL_CHECK_RC(sgl_host_words(&words));
   int64_t* h = (int64_t*)words;
@@ -306,12 +311,12 @@ extern "C" int sgl_tcsr_build_fenced(int64_t num_nodes, int64_t m, const int64_t
     SGL_REQUIRE(c.ok(), SGL_ERR_WORKSPACE, "tcsr_build: workspace too small");
     SGL_CHECK_RC(launch(tcsr_round_keys_kernel, grid, 256, 0, stream, k, nullptr, m, k0));
     int in_alt = 0;
-    SGL_CHECK_RC(radix_sort_pairs(k0, v0, k1, v1, m, nullptr, ts_bits, true, &in_alt, sort_ws, sort_bytes, stream));
+    SGL_CHECK_RC(radix_sort_pairs(k0, v0, k1, v1, m, nullptr, ts_bits, true, &in_alt, d_status, sort_ws, sort_bytes, stream));
     uint32_t *perm = in_alt ? v1 : v0, *other = in_alt ? v0 : v1;
     uint64_t *kk = in_alt ? k1 : k0, *kk_alt = in_alt ? k0 : k1;     // (the sorted timestamps are no longer needed)
     SGL_CHECK_RC(launch(tcsr_round_keys_kernel, grid, 256, 0, stream, k, perm, m, kk));
-    SGL_CHECK_RC(radix_sort_pairs(kk, perm, kk_alt, other, m, nullptr, id_bits, false, &in_alt, sort_ws, sort_bytes, stream));
-    SGL_CHECK_RC(launch(tcsr_emit_gather_kernel, grid, 256, 0, stream, in_alt ? kk_alt : kk, in_alt ? other : perm, 0, k, nbr, eid, m,
+    SGL_CHECK_RC(radix_sort_pairs(kk, perm, kk_alt, other, m, nullptr, id_bits, false, &in_alt, d_status, sort_ws, sort_bytes, stream));
+    SGL_CHECK_RC(launch(tcsr_emit_gather_kernel, grid, 256, 0, stream, d_scan, in_alt ? kk_alt : kk, in_alt ? other : perm, 0, k, nbr, eid, m,
                         num_nodes, indptr, out_nbr, out_ts, out_eid, out_perm));
   } else if (small) {
     SGL_CHECK_RC(sort_list(EdgeSource{k, m}, EdgeSink{k, nbr, eid, num_nodes, indptr, out_nbr, out_ts, out_eid, out_perm}, m,
@@ -325,19 +330,26 @@ extern "C" int sgl_tcsr_build_fenced(int64_t num_nodes, int64_t m, const int64_t
       uint32_t* node = (uint32_t*)(lsd_passes(first_bit, ts_bits + id_bits) & 1 ? k1 : k0);      // the last pass's own array
       const EdgeOut out{k, node, out_nbr, out_ts, out_eid};
       SGL_CHECK_RC((lsd_sort<uint64_t, EdgePairs>(EdgePairs{k, nbr, eid, m}, k1, v1, k0, v0, m, nullptr, nullptr, first_bit, ts_bits + id_bits, out,
-                                                  &in_first, &gave_up, c, nullptr, stream)));
-      SGL_CHECK_RC(launch(tcsr_rows_kernel, stream_grid(m, 256 * 4, 8), 256, 0, stream, gave_up, node, m, num_nodes, indptr));
+                                                  &in_first, &gave_up, c, d_status, stream)));
+      SGL_CHECK_RC(launch(tcsr_rows_kernel, stream_grid(m, 256 * 4, 8), 256, 0, stream, d_scan, node, m, num_nodes, indptr));
     } else {
       uint64_t *k1 = c.take<uint64_t>(m), *k0 = c.take<uint64_t>(m);
       uint32_t *v1 = c.take<uint32_t>(m), *v0 = c.take<uint32_t>(m);
       SGL_CHECK_RC((lsd_sort<uint32_t, EdgePositions>(EdgePositions{k, m}, k1, v1, k0, v0, m, nullptr, nullptr, first_bit, ts_bits + id_bits,
-                                                      ArrayOut<uint32_t>{}, &in_first, &gave_up, c, nullptr, stream)));
-      SGL_CHECK_RC(launch(tcsr_emit_gather_kernel, grid, 256, 0, stream, in_first ? k1 : k0, in_first ? v1 : v0, 1, k, nbr, eid, m, num_nodes,
+                                                      ArrayOut<uint32_t>{}, &in_first, &gave_up, c, d_status, stream)));
+      SGL_CHECK_RC(launch(tcsr_emit_gather_kernel, grid, 256, 0, stream, d_scan, in_first ? k1 : k0, in_first ? v1 : v0, 1, k, nbr, eid, m, num_nodes,
                           indptr, out_nbr, out_ts, out_eid, out_perm));
     }
   }
   if (out_fence && num_nodes > 0) SGL_CHECK_RC(launch_fence(indptr, out_ts, num_nodes, m, out_fence, stream));
-  return scope.submit();
+  if (small) return scope.submit();
+  // The radix passes wait for each other's tiles, for a limited time: the graph is handed out once they are known to have come through.
+  int64_t* const result = h + 8;
+  SGL_CHECK_RC(export_words((const int64_t*)&d_scan->status, result, 1, stream));
+  SGL_CHECK_RC(scope.submit());
+  SGL_CHECK_RC(sgl_wait_word(result + 1, 1, stream));
+  SGL_REQUIRE(result[0] == 0, SGL_ERR_CUDA, "tcsr_build: a look-back over the tiles of the sort ran into its time limit");
+  return SGL_OK;
 }
 
 extern "C" int sgl_tcsr_build(int64_t num_nodes, int64_t m, const int64_t* key, const int64_t* nbr, const int64_t* ts, const int64_t* eid,

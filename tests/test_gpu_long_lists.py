@@ -113,3 +113,43 @@ def test_route_plan_ranks(ranks, n):
         return
     for a, b in zip((plan.send_ranks, plan.send_sizes, plan.send_indices, plan.send_remote_indices), ref):
         assert np.array_equal(npy(a), b)
+
+
+@pytest.fixture
+def no_patience():
+    """Look-backs of this thread's calls give up at once."""
+    from starrygl import _C
+    before = _C.lib().sgl_look_back_limit(0)
+    yield
+    _C.lib().sgl_look_back_limit(before)
+
+
+def _big_build(form, m=8_000_000):
+    from starrygl import ops
+    gen = torch.Generator(device="cuda").manual_seed(3)
+    wide = 2 ** 62 if form == "two rounds" else 100_000
+    key, nbr = (torch.randint(0, 50_000, (m,), device="cuda", generator=gen) for _ in range(2))
+    ts = torch.randint(0, wide, (m,), device="cuda", generator=gen)
+    return key, ops.tcsr_build(key, nbr, ts, None, 50_000, want_perm=form != "pairs")
+
+
+@pytest.mark.parametrize("form", ["pairs", "positions", "two rounds"])
+def test_build_whose_sort_gives_up_raises(form, no_patience):
+    from starrygl import _C
+    with pytest.raises(_C.SglError, match="time limit"):
+        _big_build(form)
+    _C.lib().sgl_look_back_limit(2_000_000_000)
+    key, g = _big_build(form)
+    assert torch.equal(g.indptr[1:] - g.indptr[:-1], torch.bincount(key, minlength=50_000))
+
+
+def test_sort_and_lists_that_give_up_say_so(no_patience):
+    from starrygl import _C, ops
+    n = 8_000_000
+    keys = torch.randint(0, 2 ** 40, (n,), device="cuda")
+    with pytest.raises(_C.SglError, match="time limit"):
+        ops.radix_sort_pairs(keys, torch.arange(n, dtype=torch.int32, device="cuda"), 40)
+    st = ops.StatusWord(keys.device)
+    ops.unique_pairs(keys, torch.zeros_like(keys), id_bits=40, ts_bits=0, ts_base=0, status=st)
+    with pytest.raises(_C.SglError, match="device status"):
+        st.check("lists")

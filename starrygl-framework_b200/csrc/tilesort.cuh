@@ -338,7 +338,7 @@ struct Scratch {
   uint64_t* tile_k;     // [n] items grouped by bucket inside every tile
   uint32_t* tile_p;     // [n] (WIDE)
   int32_t* start;       // [bucket][tile] where the bucket's piece starts inside the tile; row `tiles` = the tile's end
-  uint64_t* top;        // [bucket][tile] largest key of the piece plus one, 0 = no item
+  uint64_t* top;        // [bucket][tile] largest key of the piece (0 where it is empty)
   uint64_t* over_k;     // [2][n] buckets that do not fit shared memory
   uint32_t* over_p;     // [2][n] (WIDE)
   uint32_t* over_a;     // [n]
@@ -437,7 +437,7 @@ ts_part_kernel(Source src, int pos_bits, Scratch sc) {
     if (tid + r * kThreads < m) {
       bucket[r] = not_above<WIDE>(split, buckets - 1, step, x[r]);
       at[r] = atomicAdd(&s_cnt[bucket[r]], 1);
-      if (TOP) atomicMax(&s_top[bucket[r]], (unsigned long long)key_of<WIDE>(x[r], pos_bits) + 1ull);
+      if (TOP) atomicMax(&s_top[bucket[r]], (unsigned long long)key_of<WIDE>(x[r], pos_bits));
     }
   }
   __syncthreads();
@@ -470,6 +470,7 @@ ts_bucket_kernel(Source src, Sink sink, int pos_bits, int64_t n_cap, Scratch sc,
   __shared__ int s_w[kWarps];
   __shared__ long long s_sum[kWarps];
   __shared__ unsigned long long s_top;
+  __shared__ int s_pred;
   const int64_t n = src.begin();
   sink.begin();
   if (n <= 0) {
@@ -487,6 +488,7 @@ ts_bucket_kernel(Source src, Sink sink, int pos_bits, int64_t n_cap, Scratch sc,
   if (tid == 0) {
     s_ticket = Sink::kUnique ? (int)atomicAdd(sc.ctl, 1ull) : (int)blockIdx.x;
     s_top = 0;
+    s_pred = 0;
   }
   __syncthreads();
   const int b = s_ticket;
@@ -500,7 +502,10 @@ ts_bucket_kernel(Source src, Sink sink, int pos_bits, int64_t n_cap, Scratch sc,
     if (Sink::kPred && b > 0) {
       // (a bucket after the first holds at least its splitter, so only bucket 0 can be an empty predecessor)
       const unsigned long long top = sc.top[(b - 1) * tiles + tid];
-      if (top) atomicMax(&s_top, top);
+      if (lo > sc.start[(b - 1) * tiles + tid]) {
+        s_pred = 1;
+        atomicMax(&s_top, top);
+      }
     }
   }
   const int off = warp_inclusive_scan(len, lane);
@@ -522,8 +527,8 @@ ts_bucket_kernel(Source src, Sink sink, int pos_bits, int64_t n_cap, Scratch sc,
     s_from[tid] = tid * tile + lo - (woff + off - len);
   }
   if (tid == 0) s_at[tiles] = m;
-  const bool has_pred = s_top != 0;
-  const uint64_t pred_key = has_pred ? s_top - 1ull : 0ull;
+  const bool has_pred = s_pred != 0;
+  const uint64_t pred_key = s_top;
   __syncthreads();
   const View<WIDE> from{sc.tile_k, sc.tile_p};
   // four lanes copy one piece (about seven items at 148 tiles of 1,000)

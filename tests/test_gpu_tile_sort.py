@@ -1,7 +1,10 @@
 """The two-kernel sort of mini-batch sized lists at the edges of its forms: one CTA (up to 2,048 items), 256-item tiles, the
 largest list, and key widths with which key and position share a word or do not."""
+import numpy as np
 import pytest
 import torch
+
+from gpu_util import cu, npy
 
 pytestmark = pytest.mark.gpu
 
@@ -23,3 +26,22 @@ def test_stable_at_every_form(n, bits, pattern):
     ks, vs = ops.radix_sort_pairs(k, v, bits)
     order = torch.sort(k if bits < 64 else k ^ (-1 << 63), stable=True).indices
     assert torch.equal(ks, k[order]) and torch.equal(vs, v[order])
+
+
+@pytest.mark.parametrize("n", [2049, 5000, 60000])
+def test_equal_keys_of_all_ones_across_buckets(n):
+    """64-bit keys whose largest value, all ones, fills several buckets."""
+    from starrygl import ops
+    top = 2 ** 63 - 1
+    rng = np.random.default_rng(n)
+    ids = np.where(rng.random(n) < 0.9, 1, rng.integers(0, 2, n)).astype(np.int64)
+    ts = np.where(rng.random(n) < 0.95, top, rng.integers(0, 2, n) * top).astype(np.int64)
+    st = ops.StatusWord(torch.device("cuda"))
+    out_id, out_ts, inv, _, d_n = ops.unique_pairs(cu(ids), cu(ts), id_bits=1, ts_bits=63, ts_base=0, status=st)[:5]
+    uniq, want = np.unique(np.stack([ids, ts], 1), axis=0, return_inverse=True)
+    assert int(d_n) == len(uniq) and np.array_equal(npy(inv[:n]), want.reshape(-1))
+    assert np.array_equal(npy(out_id[:len(uniq)]), uniq[:, 0]) and np.array_equal(npy(out_ts[:len(uniq)]), uniq[:, 1])
+    st.check("unique_pairs")
+    g = ops.tcsr_build(cu(ids), cu(np.arange(n, dtype=np.int64)), cu(ts), None, 2)
+    order = np.lexsort((ts, ids))
+    assert np.array_equal(npy(g.indptr), np.searchsorted(ids[order], [0, 1, 2])) and np.array_equal(npy(g.nbr), order)

@@ -108,20 +108,28 @@ size_t csc_ws(int64_t n, const int32_t* fanouts, int hops) {
   return align_up(most);
 }
 
-// indices[j] = col[indices[j]]: edge numbers -> positions in the merged list
+// indices[j] = col[indices[j]]: edge numbers -> positions in the merged list.  A batch with ids or times that were flagged and
+// replaced can leave entries of `indices` unwritten (targets of one list entry then have different edges, which build_csc_rows
+// rules out): they are not followed.
 __global__ void __launch_bounds__(256)
-map_columns_kernel(int64_t* __restrict__ indices, const int64_t* __restrict__ col, int64_t n_cap, const int64_t* d_n) {
+map_columns_kernel(int64_t* __restrict__ indices, const int64_t* __restrict__ col, int64_t n_cap, const int64_t* d_n, int32_t* d_status) {
   const int64_t n = eff_count(n_cap, d_n), stride = (int64_t)gridDim.x * 256;
-  for (int64_t j = (int64_t)blockIdx.x * 256 + threadIdx.x; j < n; j += stride) indices[j] = __ldg(col + indices[j]);
+  for (int64_t j = (int64_t)blockIdx.x * 256 + threadIdx.x; j < n; j += stride) {
+    const int64_t e = indices[j];
+    if ((uint64_t)e < (uint64_t)n) indices[j] = __ldg(col + e);
+    else dev_flag(d_status, SGL_DEV_BAD_INDEX);
+  }
 }
 
 // The same from 32-bit positions, which also become the list's 64-bit ones.
 __global__ void __launch_bounds__(256)
 map_columns_narrow_kernel(int64_t* __restrict__ indices, const uint32_t* __restrict__ narrow, int64_t* __restrict__ col, int64_t n_cap,
-                          const int64_t* d_n) {
+                          const int64_t* d_n, int32_t* d_status) {
   const int64_t n = eff_count(n_cap, d_n), stride = (int64_t)gridDim.x * 256;
   for (int64_t j = (int64_t)blockIdx.x * 256 + threadIdx.x; j < n; j += stride) {
-    indices[j] = (int64_t)__ldg(narrow + indices[j]);
+    const int64_t e = indices[j];
+    if ((uint64_t)e < (uint64_t)n) indices[j] = (int64_t)__ldg(narrow + e);
+    else dev_flag(d_status, SGL_DEV_BAD_INDEX);
     __stcs((long long*)col + j, (long long)__ldg(narrow + j));
   }
 }
@@ -258,8 +266,9 @@ extern "C" int sgl_build_batch(const int64_t* indptr, const int64_t* nbr, const 
     if (forked && l + 1 < n_hops && !narrow) SGL_CHECK_RC(order.mark(kRelabelled, stream));
     if (l > 0) {
       if (forked) SGL_CHECK_RC(order.wait(kCsc, stream));
-      if (narrow) SGL_CHECK_RC(launch(map_columns_narrow_kernel, stream_grid(e, 256 * 4, 8), 256, 0, stream, h.indices, cols32, h.col, e, d_edges));
-      else SGL_CHECK_RC(launch(map_columns_kernel, stream_grid(e, 256 * 4, 8), 256, 0, stream, h.indices, h.col, e, d_edges));
+      if (narrow) SGL_CHECK_RC(launch(map_columns_narrow_kernel, stream_grid(e, 256 * 4, 8), 256, 0, stream, h.indices, cols32, h.col, e, d_edges,
+                                       d_status));
+      else SGL_CHECK_RC(launch(map_columns_kernel, stream_grid(e, 256 * 4, 8), 256, 0, stream, h.indices, h.col, e, d_edges, d_status));
     }
     if (forked && l + 1 < n_hops && narrow) SGL_CHECK_RC(order.mark(kRelabelled, stream));     // (the next CSC may read h.col)
     cur_id = h.gids;

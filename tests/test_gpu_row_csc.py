@@ -2,6 +2,7 @@
 targets from which the sort takes over, fan-outs with and without the edge-to-item map, recent and uniform."""
 import numpy as np
 import pytest
+import torch
 
 from oracle import oracle_np as O
 from gpu_util import cu, npy, build_graph
@@ -54,3 +55,25 @@ def test_narrow_columns(copies, fanouts):
     for i, (d, r) in enumerate(zip(out, ref)):
         for k in r:
             assert np.array_equal(npy(d[k]), r[k]), (i, k)
+
+
+def test_neighbours_outside_the_graph_are_an_error():
+    """A list entry of replaced ids has targets with different edges: rows of the CSC stay partly unwritten, the call raises."""
+    from starrygl import _C, ops
+    from starrygl.graph.batch import build_batch
+    n, per = 256, 40
+    rng = np.random.default_rng(0)
+    key = np.repeat(np.arange(n), per)
+    ts = np.tile(np.arange(per) // 4, n)                       # four edges of every node at each time
+    good = rng.integers(0, n, n * per)
+    bad = np.where(np.arange(n * per) % 2 == 0, 0, 2 ** 30)   # node 0 and an id that becomes node 0, at the same times
+    q, qt = torch.arange(n).cuda().repeat(4), torch.full((4 * n,), per).cuda()
+    for nbr in (bad, good):
+        g = ops.tcsr_build(cu(key), cu(nbr.astype(np.int64)), cu(ts), None, n)
+        junk = [torch.full((1 << k,), 2 ** 61, device="cuda") for k in range(15, 25) for _ in range(4)]   # what memory holds before
+        del junk
+        if nbr is bad:
+            with pytest.raises(_C.SglError, match="node id out of range, row index out of range"):
+                build_batch(g, q, qt, [10, 10], "recent")
+        else:
+            assert len(build_batch(g, q, qt, [10, 10], "recent")) == 3

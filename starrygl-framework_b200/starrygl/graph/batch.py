@@ -216,21 +216,24 @@ def build_batch(g, roots, root_ts, fanouts, policy="recent", **kw) -> List[dict]
     """Synchronous form of :func:`build_batch_async`."""
     if kw.get("ts_range") is not None or not _SYNC_OPTIONS.issuperset(kw):
         return build_batch_async(g, roots, root_ts, fanouts, policy, **kw).finish()
-    # Query times nearly always lie in the graph's own time range (events of the stream): the batch is enqueued with the
-    # range known so far instead of waiting for the smallest and largest query time.  The kernels flag a time outside of
-    # it; then the range is read, kept on the graph, and the batch built again.
-    lo, hi = g.__dict__.get("_query_range", (g.ts_min, g.ts_max))
+    # Query times nearly always lie in the graph's own time range (events of the stream): the batch is enqueued with that range
+    # instead of waiting for the smallest and largest query time.  The kernels flag a time outside of it; then the range is read
+    # and the batch built again, and while a graph's queries stay outside they are read first.  Only that is remembered: the
+    # width of the sort keys is always that of the batch at hand.
     fanouts = list(fanouts)
+    if g.__dict__.get("_queried_outside", False):
+        a, b = _root_range(g, root_ts)
+        g.__dict__["_queried_outside"] = a < g.ts_min or b > g.ts_max
+        return build_batch_async(g, roots, root_ts, fanouts, policy, **{**kw, "ts_range": (a, b)}).finish()
     addr, words = _C.host_words()
     last = 1 + 2 * len(fanouts)
-    db = _enqueue(g, roots, root_ts, fanouts, policy, lo, hi, kw.get("equal_root_time", False), kw.get("allowed_offset", -1),
+    db = _enqueue(g, roots, root_ts, fanouts, policy, g.ts_min, g.ts_max, kw.get("equal_root_time", False), kw.get("allowed_offset", -1),
                   kw.get("seed", 0), None, None, addr)
     _C.check(_C.lib().sgl_wait_word(addr + 8 * (last + 1), 1, _C.stream_ptr()))
     host, bits = words[:last], words[last] & 0xFFFFFFFF
     if bits & 2:
-        a, b = _root_range(g, root_ts)
-        g.__dict__["_query_range"] = (min(lo, a), max(hi, b))
-        return build_batch_async(g, roots, root_ts, fanouts, policy, **{**kw, "ts_range": (a, b)}).finish()
+        g.__dict__["_queried_outside"] = True
+        return build_batch(g, roots, root_ts, fanouts, policy, **kw)
     if bits:
         raise _C.SglError(f"build_batch: device status {bits} ({_C.decode_status(bits)})")
     return db._trim(host)

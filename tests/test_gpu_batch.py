@@ -114,3 +114,35 @@ def test_batch_graph_replay_matches_eager():
         for d, r in zip(got, ref):
             for k in r:
                 assert torch.equal(d[k], r[k]), (trial, k)
+
+
+def test_query_times_outside_the_graph_leave_later_batches_alone():
+    """An extreme query time fails (or is served) by itself; batches of the same graph before and behind it are the same."""
+    from starrygl import _C
+    from starrygl.graph.batch import build_batch
+    rng = np.random.default_rng(6)
+    n, m = 1 << 20, 200000
+    z = {"n": n, "dst": rng.integers(0, n, m).astype(np.int64) // 1000, "src": rng.integers(0, n, m).astype(np.int64),
+         "ts": np.sort(rng.integers(0, 10 ** 6, m)).astype(np.int64), "eid": np.arange(m, dtype=np.int64)}
+    g = build_graph(z)
+    csr = O.tcsr_build(z["dst"], z["src"], z["ts"], z["eid"], n)[:4]
+    roots = z["dst"][rng.integers(0, m, 300)]
+    inside = rng.integers(1, 10 ** 6, 300).astype(np.int64)
+
+    def check(times):
+        out, ref = build_batch(g, cu(roots), cu(times), [5, 5]), O.build_batch(*csr, roots, times, [5, 5])
+        assert len(out) == len(ref)
+        for d, r in zip(out, ref):
+            for k in r:
+                assert np.array_equal(npy(d[k]), r[k]), k
+    check(inside)
+    for late in (2 ** 62, -2 ** 62):
+        far = inside.copy()
+        far[7] = late                                 # with 20 bits of node id the key has no room for it
+        with pytest.raises(_C.SglError):
+            build_batch(g, cu(roots), cu(far), [5, 5])
+        check(inside)
+        check(inside)
+    far[7] = 2 ** 40
+    for times in (far, far, inside, inside + 2 * 10 ** 6, inside):
+        check(times)

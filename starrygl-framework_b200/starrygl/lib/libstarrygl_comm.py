@@ -322,9 +322,11 @@ class _QueryFuture:
         g, hops = self.graph, self.hops
         addr, words = self.slot
         n = 10 + 2 * hops
-        _C.check(_C.lib().sgl_wait_word(addr + 8 * n, 1, g.stream.cuda_stream))
-        meta = words[:n]
-        _FREE_SLOTS.append(self.slot)
+        try:
+            _C.check(_C.lib().sgl_wait_word(addr + 8 * n, 1, g.stream.cuda_stream))
+            meta = words[:n]
+        finally:                          # (the stream has come to its end either way)
+            _FREE_SLOTS.append(self.slot)
         bits = meta[5] & 0xFFFFFFFF
         if bits:
             raise _C.SglError(f"submit_query: device status {bits} ({_C.decode_status(bits)})")
@@ -550,19 +552,22 @@ class CUDAGraph:
             buf = torch.empty(plan.words + 10 + 2 * layers, dtype=torch.int64, device=dev)
             ws = _C.WORKSPACE.get(plan.ws_bytes, dev, sp)
         rl = self.relabel
-        if op == "f":                     # the reference restarts the numbering on "f"
-            rl.epoch += 1
+        epoch = rl.epoch + (1 if op == "f" else 0)       # the reference restarts the numbering on "f"
         slot = self._slot()
         slot[1][10 + 2 * layers] = 0
         base = buf.data_ptr()
-        _C.check(_C.lib().sgl_query(
+        rc = _C.lib().sgl_query(
             g.indptr.data_ptr(), g.nbr.data_ptr(), g.ts.data_ptr(), g.eid.data_ptr(), None if g.fence is None else g.fence.data_ptr(),
             g.num_nodes, self.ev[0].data_ptr(), self.ev[1].data_ptr(), self.ev[2].data_ptr(), first, cap, t0, t1,
             None if node_chunk is None else node_chunk.data_ptr(), None if mask is None else mask.data_ptr(), n_chunks,
             neg_ids.data_ptr() if n_neg else None, neg_ts.data_ptr() if n_neg else None, n_neg, fanout, layers, _C.POLICY[stype],
             int(eq), off, int(keep), ops.bits_for(g.num_nodes - 1), ops.bits_for(g.ts_max - g.ts_min), g.ts_min, rl.mapper.data_ptr(),
-            rl.mask.data_ptr(), rl.epoch, int(op == "f"), rl.next_local.data_ptr(), base, base + 8 * plan.words, slot[0], ws.data_ptr(),
-            ws.numel(), producer, sp))
+            rl.mask.data_ptr(), epoch, int(op == "f"), rl.next_local.data_ptr(), base, base + 8 * plan.words, slot[0], ws.data_ptr(),
+            ws.numel(), producer, sp)
+        if rc:                            # nothing was enqueued: the numbering goes on as it was
+            _FREE_SLOTS.append(slot)
+            _C.check(rc)
+        rl.epoch = epoch
         fut = _QueryFuture(self, slot, buf, plan, layers, neg)
         fut._keep = (neg_ids, neg_ts, mask)   # inputs of kernels that may still be queued
         return fut

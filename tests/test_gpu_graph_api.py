@@ -252,3 +252,30 @@ def test_blocks_of_a_result_that_was_changed(change):
         neg_ts += 3
     _same_blocks(AsyncBlock.to_block(r, res.neg_roots, res.neighbors, res.nodes_remapper_id), _blocks_by_parts(res))
     g.g.close()
+
+
+def test_a_query_that_is_refused_leaves_no_trace():
+    """A refused "f" query neither restarts the numbering nor keeps its result words."""
+    from starrygl import _C
+    from starrygl.lib import libstarrygl_comm as L
+    n, src, dst, ts, eid = make_events()
+    none = torch.empty(0, dtype=torch.int64, device="cuda")
+    ids = []
+    for refused in (False, True):
+        g = L.from_edge_index(n, 1, cu(src), cu(dst), cu(ts), cu(eid))
+        got = []
+        for t0, op in ((2000, "f"), (2050, "r"), (2100, "r")):
+            if refused and t0 == 2050:
+                free = len(L._FREE_SLOTS)
+                for _ in range(3):
+                    g.submit_query(t0, t0 + 40, None, none, none, "uniform", 1, 600, -1, False, False, "f")   # at most 512
+                    with pytest.raises(_C.SglError, match="fanout"):
+                        g.get()
+                assert len(L._FREE_SLOTS) == free
+            g.submit_query(t0, t0 + 40, None, none, none, "recent", 1, 5, -1, False, False, op)
+            r = g.get()
+            got += [npy(r.nodes_remapper_id), npy(r.roots.roots), npy(r.neighbors[0].neighbors)]
+        ids.append(got)
+        g.close()
+    for a, b in zip(*ids):
+        assert np.array_equal(a, b)

@@ -495,7 +495,9 @@ class CUDAGraph:
                 if fut is not None:
                     self._results.append(fut)
                     return
-            fut = {"event": threading.Event(), "value": None, "error": None}
+            made = torch.cuda.Event()            # the caller's tensors are ready behind it
+            made.record(torch.cuda.current_stream(self.g.device))
+            fut = {"event": threading.Event(), "value": None, "error": None, "made": made}
             self._pending += 1
             if self._worker is None:
                 self._worker = threading.Thread(target=_serve, args=(self._tasks, self.g.device), daemon=True)
@@ -589,6 +591,7 @@ class CUDAGraph:
         """One task on the worker thread."""
         t0, t1, chunks, neg, stype, layers, fanout, off, eq, keep, op = task
         try:
+            self.stream.wait_event(fut["made"])
             nat = self._enqueue(*task)
             if nat is not None:
                 fut["value"] = nat.wait()

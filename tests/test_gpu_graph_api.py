@@ -279,3 +279,34 @@ def test_a_query_that_is_refused_leaves_no_trace():
         g.close()
     for a, b in zip(*ids):
         assert np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("width", [40, 3000])
+def test_negatives_made_on_a_stream_of_their_own(width):
+    """A query that goes through the worker thread waits for the stream on which its negatives are made, as others do; also
+    a window above the mini-batch limit, which is sampled step by step there."""
+    from starrygl.lib import libstarrygl_comm as L
+    n, src, dst, ts, eid = make_events(m=20000 if width == 40 else 2_000_000)
+    g = L.from_edge_index(n, 1, cu(src), cu(dst), cu(ts), cu(eid))
+    none = torch.empty(0, dtype=torch.int64, device="cuda")
+    want = (np.arange(64) * 5 % n).astype(np.int64)
+    t0, t1 = (5000, 5040) if width == 40 else (1000, 9000)
+    true, neg_ts = cu(want), torch.full((64,), 4000, device="cuda")
+    side = torch.cuda.Stream()
+    for warm in (True, False):                 # (the first round loads kernels)
+        neg = torch.zeros(64, dtype=torch.int64, device="cuda")
+        torch.cuda.synchronize()
+        with torch.cuda.stream(side):
+            if not warm:
+                torch.cuda._sleep(400_000_000)
+            neg.copy_(true)
+            g.submit_query(3000, 3100, None, none, none, "cluster", 1, 0, 0, False, False, "f")     # keeps the worker busy
+            g.submit_query(t0, t1, None, neg, neg_ts, "recent", 1, 5, -1, False, False, "f")
+        g.get()
+        r = g.get()
+    indptr, nbr, tss, eids, _ = O.tcsr_build(src, dst, ts, eid, n)
+    h = O.sample_layer(indptr, nbr, tss, eids, want, np.full(64, 4000, np.int64), 5)
+    nb, at = r.neighbors[0], r.roots.root_ts_num
+    start = npy(nb.root_start_ptr)
+    assert np.array_equal(np.diff(start[at:]), h[5]) and np.array_equal(npy(nb.neighbors_eid)[start[at]:], h[4])
+    g.close()

@@ -315,15 +315,15 @@ class _ArenaNeighbor(TemporalNeighbor):
 class _QueryFuture:
     """A query whose kernels are enqueued; ``wait()`` reads its sizes and builds the result."""
 
-    def __init__(self, graph, slot, buf, plan, hops, neg):
-        self.graph, self.slot, self.buf, self.plan, self.hops, self.neg = graph, slot, buf, plan, hops, neg
+    def __init__(self, stream, slot, buf, plan, hops, neg):
+        self.stream, self.slot, self.buf, self.plan, self.hops, self.neg = stream, slot, buf, plan, hops, neg
 
     def wait(self):
-        g, hops = self.graph, self.hops
+        hops = self.hops
         addr, words = self.slot
         n = 10 + 2 * hops
         try:
-            _C.check(_C.lib().sgl_wait_word(addr + 8 * n, 1, g.stream.cuda_stream))
+            _C.check(_C.lib().sgl_wait_word(addr + 8 * n, 1, self.stream.cuda_stream))
             meta = words[:n]
         finally:                          # (the stream has come to its end either way)
             _FREE_SLOTS.append(self.slot)
@@ -570,7 +570,7 @@ class CUDAGraph:
             _FREE_SLOTS.append(slot)
             _C.check(rc)
         rl.epoch = epoch
-        fut = _QueryFuture(self, slot, buf, plan, layers, neg)
+        fut = _QueryFuture(self.stream, slot, buf, plan, layers, neg)
         fut._keep = (neg_ids, neg_ts, mask)   # inputs of kernels that may still be queued
         return fut
 
@@ -623,6 +623,11 @@ class CUDAGraph:
     def __del__(self):
         try:
             self.close()
+            # queries that nobody fetched: their kernels still use the graph's arrays, their negatives and result words
+            left = [f for f in self._results if isinstance(f, _QueryFuture)]
+            if left:
+                self.stream.synchronize()
+                _FREE_SLOTS.extend(f.slot for f in left)
         except Exception:
             pass
 

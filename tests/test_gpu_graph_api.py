@@ -310,3 +310,24 @@ def test_negatives_made_on_a_stream_of_their_own(width):
     start = npy(nb.root_start_ptr)
     assert np.array_equal(np.diff(start[at:]), h[5]) and np.array_equal(npy(nb.neighbors_eid)[start[at]:], h[4])
     g.close()
+
+
+def test_a_dropped_graph_waits_for_queries_that_nobody_fetched():
+    import weakref
+    from starrygl.lib import libstarrygl_comm as L
+    n, src, dst, ts, eid = make_events()
+    own = torch.cuda.Stream()
+    for warm in (True, False):
+        g = L.from_edge_index(n, 1, cu(src), cu(dst), cu(ts), cu(eid), stream=own)
+        neg = torch.arange(64, device="cuda")
+        g.submit_query(2000, 2100, None, neg, neg + 2500, "recent", 2, 5, -1, False, False, "f")
+        g.get()
+        free = len(L._FREE_SLOTS)
+        torch.cuda.synchronize()
+        torch.cuda._sleep(200_000_000)              # the queries wait for the caller's stream
+        for op in ("f", "r"):
+            g.submit_query(2000, 2100, None, neg, neg + 2500, "recent", 2, 5, -1, False, False, op)
+        assert warm or not own.query()
+        gone = weakref.ref(g)
+        del g
+        assert gone() is None and own.query() and len(L._FREE_SLOTS) == free

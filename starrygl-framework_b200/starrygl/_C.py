@@ -6,7 +6,6 @@ worker threads the way the reference's pybind module is (csrc/srcs/starrygl/expo
 ``py::gil_scoped_release`` on every heavy binding).
 """
 import ctypes as C
-import itertools
 import os
 import threading
 
@@ -236,34 +235,45 @@ def host_words():
 
 class CountRing:
     """Pinned (value, sequence number) pairs that kernels fill in with a count the host may ask for later.  A pair is used
-    again after as many calls as there are pairs; who still wants the older count reads it from the device."""
+    again after as many calls as there are pairs, once its count has arrived -- so that one kernel at a time may write to it;
+    who still wants the older count reads it from the device."""
     SLOTS = 1024
 
     def __init__(self):
-        self._seq = itertools.count(1)       # (one call of next() is atomic)
+        self._seq = 0
         self._lock = threading.Lock()
         self._buf = self._words = None
+        self._owner = [0] * self.SLOTS       # sequence number the pair was last given out for
 
     def take(self):
-        """(address, index of the value, sequence number)"""
-        if self._buf is None:
-            with self._lock:
-                if self._buf is None:
-                    buf = torch.zeros(2 * self.SLOTS, dtype=torch.int64).pin_memory()
-                    self._words = (C.c_int64 * (2 * self.SLOTS)).from_address(buf.data_ptr())
-                    self._base, self._buf = buf.data_ptr(), buf
-        seq = next(self._seq)
-        i = 2 * (seq % self.SLOTS)
-        return self._base + 8 * i, i, seq
+        """(address, index of the value, sequence number); None while the pair's last count is still on its way."""
+        with self._lock:
+            if self._buf is None:
+                buf = torch.zeros(2 * self.SLOTS, dtype=torch.int64).pin_memory()
+                self._words = (C.c_int64 * (2 * self.SLOTS)).from_address(buf.data_ptr())
+                self._base, self._buf = buf.data_ptr(), buf
+            seq = self._seq = self._seq + 1
+            k = seq % self.SLOTS
+            if self._words[2 * k + 1] != self._owner[k]:
+                return None
+            self._owner[k] = seq
+        return self._base + 16 * k, 2 * k, seq
+
+    def give_back(self, taken):
+        """The pair of a call that failed: nothing is going to arrive."""
+        if taken is not None:
+            self._words[taken[1] + 1] = taken[2]
 
     def value(self, taken, stream):
         """The count, or None when its pair was used again (or never filled in)."""
         addr, i, seq = taken
         w = self._words
+        if self._owner[i // 2] != seq:
+            return None
         if w[i + 1] < seq:
             lib().sgl_wait_word(addr + 8, seq, stream)
-        v = w[i]
-        return v if w[i + 1] == seq else None
+        arrived, v = w[i + 1] == seq, w[i]
+        return v if arrived and self._owner[i // 2] == seq else None     # (given out again meanwhile: v may be the next one's)
 
 
 COUNTS = CountRing()

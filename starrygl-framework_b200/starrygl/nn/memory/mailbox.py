@@ -85,9 +85,13 @@ class mailbox:
         """(index, mail, mail_ts) of the batch: distinct nodes in ascending order, each with the row and timestamp of
         its latest entry (reference: mailbox.py:56-84).  One host synchronisation, to size the results exactly."""
         count, stream = _C.COUNTS.take(), _C.stream_ptr()
-        index, mail, mail_ts, d_n = self.get_update_mail_async(src, dst, ts, edge_feats, mem_src, mem_dst, embedding,
-                                                               use_src_emb, use_dst_emb, count)
-        u = _C.COUNTS.value(count, stream)
+        try:
+            index, mail, mail_ts, d_n = self.get_update_mail_async(src, dst, ts, edge_feats, mem_src, mem_dst, embedding,
+                                                                   use_src_emb, use_dst_emb, count)
+        except BaseException:
+            _C.COUNTS.give_back(count)
+            raise
+        u = None if count is None else _C.COUNTS.value(count, stream)
         if u is None:
             u = int(d_n.item())
         return index[:u], mail[:u], mail_ts[:u]

@@ -156,12 +156,16 @@ def sample_layer(g: TCSR, targets, target_ts, fanout: int, policy="recent", *, d
     _, wp, wn = _C.workspace(L.sgl_sample_ws_bytes(n), dev)
     # (a captured launch does not hand its count over)
     taken, stream = None if torch._C._cuda_isCurrentStreamCapturing() else _C.COUNTS.take(), _C.stream_ptr()
-    _C.check(L.sgl_sample_layer_counted(_C.ptr(g.indptr), _C.ptr(g.nbr), _C.ptr(g.ts), _C.ptr(g.eid), _C.ptr(g.fence), g.num_nodes,
-                                _C.ptr(targets), _C.ptr(target_ts), n, _C.ptr(d_n), int(fanout), pol,
-                                int(bool(equal_root_time)), int(allowed_offset), int(bool(keep_root_time)),
-                                int(seed) & (2 ** 64 - 1), int(rng_stream) & 0xFFFFFFFF, _C.ptr(o_nbr), _C.ptr(o_dst),
-                                _C.ptr(o_ts), _C.ptr(o_dt), _C.ptr(o_dti), _C.ptr(o_eid), _C.ptr(offs),
-                                status.ptr() if status else None, wp, wn, taken and taken[0], taken[2] if taken else 0, stream))
+    try:
+        _C.check(L.sgl_sample_layer_counted(_C.ptr(g.indptr), _C.ptr(g.nbr), _C.ptr(g.ts), _C.ptr(g.eid), _C.ptr(g.fence), g.num_nodes,
+                                    _C.ptr(targets), _C.ptr(target_ts), n, _C.ptr(d_n), int(fanout), pol,
+                                    int(bool(equal_root_time)), int(allowed_offset), int(bool(keep_root_time)),
+                                    int(seed) & (2 ** 64 - 1), int(rng_stream) & 0xFFFFFFFF, _C.ptr(o_nbr), _C.ptr(o_dst),
+                                    _C.ptr(o_ts), _C.ptr(o_dt), _C.ptr(o_dti), _C.ptr(o_eid), _C.ptr(offs),
+                                    status.ptr() if status else None, wp, wn, taken and taken[0], taken[2] if taken else 0, stream))
+    except BaseException:
+        _C.COUNTS.give_back(taken)
+        raise
     return Hop(o_nbr, o_dst, o_ts, o_dt, o_eid, offs, cap, o_dti, taken and (taken, stream))
 
 

@@ -242,3 +242,16 @@ def test_lane_draws_match_oracle(k):
     ref = OC.sample_layer(indptr, nbr, ts, eid, q, qt, k, O.UNIFORM, seed=2 ** 40 + k, stream=2)
     for nm, a, r in zip(NAMES, out, ref):
         assert np.array_equal(a, r), nm
+
+
+def test_counts_of_more_hops_than_the_ring_holds():
+    """1,100 hops enqueued before any count is asked for: first, last and every one between have their own."""
+    from starrygl import ops
+    z = random_graph(4, 300, 20000, 1000)
+    g = build_graph(z)
+    hops = []
+    for i in range(1100):
+        q = torch.full((1 + i % 50,), i % 300, device="cuda")
+        hops.append((q, ops.sample_layer(g, q, torch.full_like(q, 500 + i % 400), 7, "recent")))
+    for q, h in hops:
+        assert h.total() == int(h.offsets[-1].item())

@@ -593,6 +593,8 @@ int sgl_lower_bound_i64(const int64_t* sorted, int64_t n, const int64_t* values,
  * status word is used when d_status is NULL.  host_meta (optional, pinned, 3 + 2 * n_hops words): receives meta when the
  * batch is done and then a 1 behind it (see sgl_wait_word).  side_stream (optional): hops after the first and their CSC run there,
  * next to the relabels; everything is joined into `stream`.
+ * sgl_build_batch_at: the same with a place of its own for every section: section s is at base + section_at[s] words, or, where
+ * that is negative, at other_base + (-1 - section_at[s]) words.
  * Replaces: build_aligned_batch's per-layer loop (prepare_sample.py:313-377).
  * ---------------------------------------------------------------------------------------------- */
 int64_t sgl_build_batch_layout(int64_t n_roots, const int32_t* fanouts, int n_hops, int64_t* section_words);
@@ -602,6 +604,11 @@ int sgl_build_batch(const int64_t* indptr, const int64_t* nbr, const int64_t* ts
                     const int32_t* fanouts, int n_hops, int policy, int equal_root_time, int64_t allowed_offset,
                     uint64_t seed, int id_bits, int ts_bits, int64_t ts_base, int64_t* arena, int64_t* meta,
                     int32_t* d_status, int64_t* host_meta, void* ws, size_t ws_bytes, void* side_stream, void* stream);
+int sgl_build_batch_at(const int64_t* indptr, const int64_t* nbr, const int64_t* ts, const int64_t* eid, const int64_t* fence,
+                    int64_t num_nodes, const int64_t* roots, const int64_t* root_ts, int64_t n_roots,
+                    const int32_t* fanouts, int n_hops, int policy, int equal_root_time, int64_t allowed_offset,
+                    uint64_t seed, int id_bits, int ts_bits, int64_t ts_base, const int64_t* section_at,
+                    int64_t* base, int64_t* other_base, int64_t* meta, int32_t* d_status, int64_t* host_meta, void* ws, size_t ws_bytes, void* side_stream, void* stream);
 
 /* ------------------------------------------------------------------------------------------------
  * One query of the graph API in one call: roots of the window [t_begin, t_end) (sgl_seeds_in_window), the negatives

@@ -4,7 +4,8 @@
 // What this replaces is host time: driven entry point by entry point from Python a two-hop batch of 4,096 roots cost 37
 // allocations and 20 foreign calls, and its 200 us of kernels took 490 us to issue.
 //
-// Arena (8-byte words, sections in the order of batch_sections(), each rounded up to 32 words):
+// Results: sections of 8-byte words in the order of batch_sections(), each rounded up to 32 words, one behind the other in an
+// arena or (sgl_build_batch_at) wherever the caller wants each to lie:
 //   roots            gids[n], ts[n], inverse map[n]
 //   hop l            nbr, dst, ts, dt (fp32), eid [T_l k_l], offsets[T_l + 1]; merged list gids, ts [C_l + T_l k_l], column
 //                    indices of the hop's edges in it [T_l k_l]; from the second hop on: CSC row pointer [C_l + 1], indices,
@@ -163,11 +164,12 @@ extern "C" size_t sgl_build_batch_ws_bytes(int64_t n_roots, const int32_t* fanou
          order_ws(n_roots, fanouts, n_hops) + narrow_ws(n_roots, fanouts, n_hops);
 }
 
-extern "C" int sgl_build_batch(const int64_t* indptr, const int64_t* nbr, const int64_t* ts, const int64_t* eid, const int64_t* fence,
-                               int64_t num_nodes, const int64_t* roots, const int64_t* root_ts, int64_t n_roots,
-                               const int32_t* fanouts, int n_hops, int policy, int equal_root_time, int64_t allowed_offset,
-                               uint64_t seed, int id_bits, int ts_bits, int64_t ts_base, int64_t* arena, int64_t* meta,
-                               int32_t* d_status, int64_t* host_meta, void* ws, size_t ws_bytes, void* side_stream, void* stream_) {
+extern "C" int sgl_build_batch_at(const int64_t* indptr, const int64_t* nbr, const int64_t* ts, const int64_t* eid, const int64_t* fence,
+                                  int64_t num_nodes, const int64_t* roots, const int64_t* root_ts, int64_t n_roots,
+                                  const int32_t* fanouts, int n_hops, int policy, int equal_root_time, int64_t allowed_offset,
+                                  uint64_t seed, int id_bits, int ts_bits, int64_t ts_base, const int64_t* section_at, int64_t* base,
+                                  int64_t* other_base, int64_t* meta, int32_t* d_status, int64_t* host_meta, void* ws, size_t ws_bytes,
+                                  void* side_stream, void* stream_) {
   SGL_NVTX("sgl_build_batch");
   cudaStream_t stream = (cudaStream_t)stream_;
   SGL_REQUIRE(n_roots >= 0 && n_hops >= 0 && n_hops <= kMaxHops && (n_hops == 0 || fanouts), SGL_ERR_ARG,
@@ -181,23 +183,19 @@ extern "C" int sgl_build_batch(const int64_t* indptr, const int64_t* nbr, const 
     return scope.submit();
   };
   if (n_roots == 0) return done();
-  SGL_REQUIRE(arena && roots && root_ts, SGL_ERR_ARG, "build_batch: null array");
+  SGL_REQUIRE(section_at && roots && root_ts, SGL_ERR_ARG, "build_batch: null array");
   SGL_REQUIRE(ws_bytes >= sgl_build_batch_ws_bytes(n_roots, fanouts, n_hops), SGL_ERR_WORKSPACE, "build_batch: workspace %zu < %zu bytes",
               ws_bytes, sgl_build_batch_ws_bytes(n_roots, fanouts, n_hops));
   if (d_status == nullptr) d_status = (int32_t*)(meta + 1 + 2 * n_hops);
-  int64_t size[kRootSections + kMaxHops * kHopSections];
-  batch_sections(n_roots, fanouts, n_hops, size);
   const size_t swb = sample_ws(n_roots, fanouts, n_hops), lwb = list_ws(n_roots, fanouts, n_hops), cwb = csc_ws(n_roots, fanouts, n_hops);
   void *sws = ws, *lws = (char*)ws + swb, *cws = (char*)lws + lwb;
   char* ows = (char*)cws + cwb;
   uint32_t* const cols32 = (uint32_t*)(ows + order_ws(n_roots, fanouts, n_hops));
   RowOrder order_of{};                   // of the layer list merged last, where the next CSC goes along it
-  int64_t* p = arena;
   int sec = 0;
-  auto take = [&]() {
-    int64_t* q = p;
-    p += size[sec++];
-    return q;
+  auto take = [&]() -> int64_t* {
+    const int64_t at = section_at[sec++];
+    return (int64_t*)(at >= 0 ? (uintptr_t)base + (uintptr_t)at * 8 : (uintptr_t)other_base + (uintptr_t)(-1 - at) * 8);
   };
   int64_t *cur_id = take(), *cur_ts = take(), *inv = take();
   int rc = sgl_unique_pairs(roots, root_ts, n_roots, nullptr, nullptr, nullptr, 0, nullptr, id_bits, ts_bits, ts_base, cur_id, cur_ts, inv,
@@ -279,6 +277,25 @@ extern "C" int sgl_build_batch(const int64_t* indptr, const int64_t* nbr, const 
     c += e;
   }
   return done();
+}
+
+extern "C" int sgl_build_batch(const int64_t* indptr, const int64_t* nbr, const int64_t* ts, const int64_t* eid, const int64_t* fence,
+                               int64_t num_nodes, const int64_t* roots, const int64_t* root_ts, int64_t n_roots,
+                               const int32_t* fanouts, int n_hops, int policy, int equal_root_time, int64_t allowed_offset,
+                               uint64_t seed, int id_bits, int ts_bits, int64_t ts_base, int64_t* arena, int64_t* meta,
+                               int32_t* d_status, int64_t* host_meta, void* ws, size_t ws_bytes, void* side_stream, void* stream) {
+  int64_t at[kRootSections + kMaxHops * kHopSections];
+  SGL_REQUIRE(sgl_build_batch_layout(n_roots, fanouts, n_hops, at) >= 0, SGL_ERR_ARG, "build_batch: bad size (at most %d hops)", kMaxHops);
+  SGL_REQUIRE(arena || n_roots == 0, SGL_ERR_ARG, "build_batch: null array");
+  int64_t next = 0;
+  for (int s = 0; s < kRootSections + n_hops * kHopSections; ++s) {
+    const int64_t size = at[s];
+    at[s] = next;
+    next += size;
+  }
+  return sgl_build_batch_at(indptr, nbr, ts, eid, fence, num_nodes, roots, root_ts, n_roots, fanouts, n_hops, policy, equal_root_time,
+                            allowed_offset, seed, id_bits, ts_bits, ts_base, at, arena, nullptr, meta, d_status, host_meta, ws, ws_bytes,
+                            side_stream, stream);
 }
 
 // Up to kMaxExport arrays packed one behind the other (16-byte aligned offsets) and copied to the host in one go, or in two

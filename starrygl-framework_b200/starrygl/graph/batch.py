@@ -8,6 +8,7 @@ previous list (``indptr``, ``indices``, ``eid``, ``edge_ts``, ``edge_dt``) + the
 synchronisation: the number of edges a hop produced is handed to the next kernels as a device count.
 ``finish()`` performs the single synchronisation that is needed to give the tensors their final shapes.
 """
+import ctypes as C
 from collections import OrderedDict
 from typing import List, Optional, Sequence
 
@@ -16,25 +17,40 @@ import torch
 from .. import _C, ops
 
 
+# Results up to this size share one allocation (a tensor that is kept keeps the others' memory); larger ones have one each.
+_SHARED_MOST = 32 << 20
+
+
 class _Plan:
-    """What a batch of one shape (number of roots, fan-outs) needs: the arena's sections, the scratch size and the fan-outs as
-    the library reads them."""
+    """What a batch of one shape (number of roots, fan-outs) needs: the size of every section and where it goes, the scratch
+    size and the fan-outs as the library reads them.  Sections that :meth:`DeviceBatch.finish` returns are kept apart from the
+    raw arrays of the hops, which go with the :class:`DeviceBatch`."""
 
     def __init__(self, n: int, fanouts: Sequence[int]):
-        import ctypes as C
         L = _C.lib()
-        if len(fanouts) > 8:
+        hops = len(fanouts)
+        if hops > 8:
             raise _C.SglError("build_batch: at most 8 hops")
-        self.fan = (C.c_int32 * max(len(fanouts), 1))(*[int(k) for k in fanouts])
-        sec = (C.c_int64 * (3 + 14 * len(fanouts)))()
-        self.words = int(L.sgl_build_batch_layout(n, self.fan, len(fanouts), sec))
-        if self.words < 0:
+        self.fan = (C.c_int32 * max(hops, 1))(*[int(k) for k in fanouts])
+        self.places = C.c_int64 * (3 + 14 * hops)
+        sec = self.places()
+        if int(L.sgl_build_batch_layout(n, self.fan, hops, sec)) < 0:
             raise _C.SglError("build_batch: bad batch shape")
-        self.ws_bytes = int(L.sgl_build_batch_ws_bytes(n, self.fan, len(fanouts)))
-        self.start, at = [], 0
-        for w in sec:
-            self.start.append(at)
-            at += int(w)
+        self.ws_bytes = int(L.sgl_build_batch_ws_bytes(n, self.fan, hops))
+        self.size = [int(w) for w in sec]
+        kept = [0, 1, 2]
+        for l in range(hops):
+            kept += [3 + 14 * l + i for i in ((2, 3, 4, 5, 6, 7, 8) if l == 0 else (6, 7, 9, 10, 11, 12, 13))]
+        self.kept = kept
+        at, words, raw = self.places(), 0, 0
+        for s in kept:
+            at[s] = words
+            words += self.size[s]
+        for s in sorted(set(range(len(self.size))) - set(kept)):
+            at[s] = -1 - raw
+            raw += self.size[s]
+        self.at, self.words, self.raw_words = at, words, raw
+        self.shared = 8 * words <= _SHARED_MOST
 
 
 _PLANS: "OrderedDict" = OrderedDict()
@@ -58,11 +74,12 @@ class _MetaStatus(ops.StatusWord):
 
 
 class DeviceBatch:
-    """Un-trimmed result of :func:`build_batch_async`: one arena with every array at capacity, the counts on the device."""
+    """Un-trimmed result of :func:`build_batch_async`: every array at capacity, the counts on the device.  ``results``: one tensor
+    for all sections that a caller gets to keep, or a dictionary of one each; ``raw``: the others."""
 
-    def __init__(self, g, n, fanouts, plan, arena, meta, status):
+    def __init__(self, g, n, fanouts, plan, results, raw, meta, status):
         self.g, self.n, self.fanouts = g, n, list(fanouts)
-        self._plan, self._arena, self._meta, self._status = plan, arena, meta, status
+        self._plan, self._results, self._raw, self._meta, self._status = plan, results, raw, meta, status
         self._layers = None
 
     @property
@@ -76,15 +93,26 @@ class DeviceBatch:
         """Device int64 scalars (1-element tensors): root list, then per hop sampled edges and merged list."""
         return [self._meta[i:i + 1] for i in range(1 + 2 * len(self.fanouts))]
 
+    def _place(self, section):
+        """(tensor, offset) of a section."""
+        s = self._plan.at[section]
+        if s < 0:
+            return self._raw, -1 - s
+        return (self._results, s) if self._plan.shared else (self._results[section], 0)
+
     def _view(self, section, count, floats=False):
-        s = self._plan.start[section]
+        t, s = self._place(section)
         if floats:
-            return self._arena[s:s + (count + 1) // 2].view(torch.float32)[:count]
-        return self._arena[s:s + count]
+            return t[s:s + (count + 1) // 2].view(torch.float32)[:count]
+        return t[s:s + count]
+
+    def address(self, section):
+        t, s = self._place(section)
+        return t.data_ptr() + 8 * s
 
     @property
     def layers(self):
-        """Capacity-sized tensors per layer (views into the arena)."""
+        """Capacity-sized tensors per layer."""
         if self._layers is None:
             v, n = self._view, self.n
             out = [{"gids": v(0, n), "ts": v(1, n), "inv_map": v(2, n)}]
@@ -153,26 +181,33 @@ class DeviceBatch:
 def _enqueue(g, roots, root_ts, fanouts, policy, lo, hi, equal_root_time, allowed_offset, seed, status, side, host=None,
              meta=None) -> DeviceBatch:
     """``lo`` / ``hi``: lowest and highest timestamp that can occur; ``host``: pinned address that receives the counts;
-    ``meta``: block of 2 + 2 * hops device words for the counts and the status (default: behind the arena)."""
+    ``meta``: block of 2 + 2 * hops device words for the counts and the status (default: behind the raw arrays)."""
     roots, root_ts = ops._i64(roots), ops._i64(root_ts)
     n = roots.numel()
     if root_ts.numel() != n:
         raise _C.SglError("build_batch: roots and root_ts differ in length")
     plan = _plan(n, fanouts)
     dev = g.device
-    arena = torch.empty(plan.words + (2 + 2 * len(fanouts) if meta is None else 0), dtype=torch.int64, device=dev)
+    raw = torch.empty(plan.raw_words + (2 + 2 * len(fanouts) if meta is None else 0), dtype=torch.int64, device=dev)
     if meta is None:
-        meta = arena[plan.words:]
+        meta = raw[plan.raw_words:]
+    if plan.shared:
+        results = torch.empty(plan.words, dtype=torch.int64, device=dev)
+        at, base = plan.at, results.data_ptr()
+    else:
+        results = {s: torch.empty(plan.size[s], dtype=torch.int64, device=dev) for s in plan.kept}
+        at, base = plan.places(*plan.at), None
+        for s, t in results.items():
+            at[s] = t.data_ptr() // 8
     sp = _C.stream_ptr()
     ws = _C.WORKSPACE.get(plan.ws_bytes, dev, sp)
-    base = arena.data_ptr()
-    _C.check(_C.lib().sgl_build_batch(
+    _C.check(_C.lib().sgl_build_batch_at(
         g.indptr.data_ptr(), g.nbr.data_ptr(), g.ts.data_ptr(), g.eid.data_ptr(), None if g.fence is None else g.fence.data_ptr(),
         g.num_nodes, _C.ptr(roots), _C.ptr(root_ts), n, plan.fan, len(fanouts),
         _C.POLICY[policy] if isinstance(policy, str) else int(policy), int(bool(equal_root_time)), int(allowed_offset),
-        int(seed) & (2 ** 64 - 1), ops.bits_for(g.num_nodes - 1), ops.bits_for(hi - lo), lo, base, meta.data_ptr(),
+        int(seed) & (2 ** 64 - 1), ops.bits_for(g.num_nodes - 1), ops.bits_for(hi - lo), lo, at, base, raw.data_ptr(), meta.data_ptr(),
         None if status is None else status.ptr(), host, ws.data_ptr(), ws.numel(), None if side is None else side.cuda_stream, sp))
-    return DeviceBatch(g, n, fanouts, plan, arena, meta, status)
+    return DeviceBatch(g, n, fanouts, plan, results, raw, meta, status)
 
 
 def _graph_range(g, lo, hi):
@@ -184,7 +219,7 @@ def build_batch_async(g: ops.TCSR, roots: torch.Tensor, root_ts: torch.Tensor, f
                       policy: str = "recent", *, ts_range: Optional[Sequence[int]] = None, equal_root_time=False,
                       allowed_offset=-1, seed=0, status: Optional[ops.StatusWord] = None,
                       side_streams: Optional[Sequence[torch.cuda.Stream]] = None) -> DeviceBatch:
-    """Enqueue the whole batch construction on the current stream: one foreign call, one allocation.
+    """Enqueue the whole batch construction on the current stream, in one foreign call.
 
     ``ts_range`` = (lowest, highest) timestamp that can occur among the roots' query times; together with the
     graph's own timestamp range it fixes the width of the (id, ts) sort key.  When omitted it is read from

@@ -122,12 +122,11 @@ class MaterializedMultiLayerBuilder:
         db = _enqueue(g, roots, root_ts, fanouts, policy, lo, hi, inclusive, -1, seed, None, None, None, meta[:nb])
         lists = []                                  # (address of the ids, capacity) of every layer list
         n = c = t = roots.numel()
-        base = db._arena.data_ptr()
-        lists.append((base + 8 * db._plan.start[0], c))
+        lists.append((db.address(0), c))
         for l, k in enumerate(fanouts):
             t *= k
             c += t
-            lists.append((base + 8 * db._plan.start[3 + 14 * l + 6], c))
+            lists.append((db.address(3 + 14 * l + 6), c))
         plans = []
         if planned:
             caps = [max(c * max(P - 1, 1), 1) for _, c in lists]
@@ -158,8 +157,7 @@ class MaterializedMultiLayerBuilder:
                 layers = None
         picks = []                                  # (address, count, bytes per value) in the order of the result
         if layers is None:
-            starts = db._plan.start
-            sec = lambda i, count, size=8: picks.append((base + 8 * starts[i], count, size))
+            sec = lambda i, count, size=8: picks.append((db.address(i), count, size))
             sec(0, host[0]); sec(1, host[0]); sec(2, n)
             prev = host[0]
             for l in range(hops):

@@ -146,3 +146,25 @@ def test_query_times_outside_the_graph_leave_later_batches_alone():
     far[7] = 2 ** 40
     for times in (far, far, inside, inside + 2 * 10 ** 6, inside):
         check(times)
+
+
+@pytest.mark.parametrize("roots", [4096, 60000])
+def test_a_kept_tensor_keeps_little_else(roots):
+    """What one tensor of a batch's result holds in memory: nothing of the raw hops, and itself alone in a large batch."""
+    from starrygl import ops
+    from starrygl.graph.batch import build_batch
+    n, m = 50000, 2_000_000
+    gen = torch.Generator(device="cuda").manual_seed(1)
+    src, dst = (torch.randint(0, n, (m,), device="cuda", generator=gen) for _ in range(2))
+    g = ops.tcsr_build(src, dst, torch.randint(0, 10 ** 6, (m,), device="cuda", generator=gen), None, n)
+    q, qt = src[:roots].contiguous(), torch.full((roots,), 900_000, device="cuda")
+    build_batch(g, q, qt, [10, 10])                       # (scratch that stays)
+    torch.cuda.synchronize()
+    before = torch.cuda.memory_allocated()
+    out = build_batch(g, q, qt, [10, 10])
+    capacity = 8 * (3 * roots + roots * (1 + 10 * (2 + 1.5 + 1 + 2)) + 10 * roots * (1 + 10 * (2 + 2.5 + 2)) + 22 * roots)
+    assert torch.cuda.memory_allocated() - before <= 1.05 * capacity       # the results' own capacities
+    keep = out[0]["gids"]
+    del out
+    assert torch.cuda.memory_allocated() - before <= max(8 * roots + 4096, 0 if roots > 4096 else 33 << 20)
+    assert int(keep.max()) < n

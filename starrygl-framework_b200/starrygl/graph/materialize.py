@@ -88,7 +88,6 @@ class MaterializedMultiLayerBuilder:
         self.pid, self.num_parts = int(pid), int(num_parts)
         self.gen = torch.Generator(device="cpu")
         self.gen.manual_seed(0)
-        self._stage = None                # pinned buffer for the tasks' roots
 
     def _roots(self, node_parts, ts_parts):
         """(nodes, times, (lowest, highest time)) of a task on the GPU: host arrays go through one pinned buffer and one copy,
@@ -98,13 +97,13 @@ class MaterializedMultiLayerBuilder:
             f = lambda xs: torch.cat([_dev_i64(x, self.device) for x in xs])
             return f(node_parts), f(ts_parts), None
         n, total = sum(len(x) for x in parts[:len(node_parts)]), sum(len(x) for x in parts)
-        if self._stage is None or self._stage.numel() < total:
-            self._stage = torch.empty(max(2 * total, 1024), dtype=torch.int64, pin_memory=True)
-        st, at = self._stage.numpy(), 0
+        # (a buffer of this call's own: several threads may build slots with one builder)
+        stage = torch.empty(total, dtype=torch.int64, pin_memory=True)
+        st, at = stage.numpy(), 0
         for x in parts:
             st[at:at + len(x)] = x
             at += len(x)
-        d = self._stage[:total].to(self.device, non_blocking=True)     # (the slot's end waits for the stream)
+        d = stage.to(self.device, non_blocking=True)
         t = parts[len(node_parts)]
         return d[:n], d[n:], (int(t.min()), int(t.max())) if len(t) else None
 

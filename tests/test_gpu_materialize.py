@@ -67,3 +67,32 @@ def test_unsupported_policies_raise():
             b.build_aligned_batch(task, None, cfg)
     out = b.build_aligned_batch(task, None, {'meta': {}, 'layer': [{'type': 'uniform', 'fanout': 2}]}, seed=3)
     assert out[0]["comm_plan"] == [None, None] and out[1]["indptr"].numel() == out[0]["gids"].numel() + 1
+
+
+def test_one_builder_in_two_threads():
+    """Slots built side by side with one builder, each thread on a stream of its own, are those of one thread."""
+    import threading
+    from starrygl.graph.materialize import MaterializedMultiLayerBuilder
+    rng = np.random.default_rng(0)
+    n, m = 5000, 100000
+    z = {k: rng.integers(0, n, m).astype(np.int64) for k in ("src", "dst")}
+    z["ts"] = np.sort(rng.integers(0, 10 ** 6, m)).astype(np.int64)
+    b = MaterializedMultiLayerBuilder(z, n, None, None, 0, 1)
+    cfg = {'meta': {}, 'layer': [{'type': 'recent', 'fanout': 5}]}
+
+    def slot(i):
+        at = slice(50000 + 100 * i, 50000 + 100 * i + 3000)
+        return b.build_aligned_batch(('node', (z["src"][at], z["ts"][at], np.zeros(3000))), None, cfg)
+    want = [slot(i) for i in range(100)]
+    wrong = []
+
+    def work(first):
+        with torch.cuda.stream(torch.cuda.Stream()):
+            for i in range(first, 100, 2):
+                got = slot(i)
+                if not all(torch.equal(got[l][k], want[i][l][k]) for l in range(2) for k in ("gids", "ts")):
+                    wrong.append(i)
+    threads = [threading.Thread(target=work, args=(t,)) for t in range(2)]
+    [t.start() for t in threads]
+    [t.join() for t in threads]
+    assert not wrong

@@ -646,6 +646,8 @@ int sgl_query_blocks(int n_hops, const int64_t* const* node, const int64_t* cons
  * wait for the copies. */
 int sgl_export_arrays(int n, const void* const* src, const int64_t* bytes, const int64_t* at, void* staging, void* host,
                       int64_t total, void* host2, int64_t split, void* stream);
+/* Device arrays to the host, one copy each; does not wait for the copies. */
+int sgl_copy_arrays(int n, const void* const* src, const int64_t* bytes, void* const* dst, void* stream);
 int sgl_host_words(void** out);
 int sgl_wait_word(const int64_t* flag, int64_t at_least, void* stream);
 int sgl_read_back(const void* src, void* dst, size_t bytes, void* stream);

@@ -344,6 +344,16 @@ extern "C" int sgl_export_arrays(int n, const void* const* src, const int64_t* b
   return SGL_OK;
 }
 
+// One copy per array.
+extern "C" int sgl_copy_arrays(int n, const void* const* src, const int64_t* bytes, void* const* dst, void* stream) {
+  SGL_REQUIRE(n >= 0 && (n == 0 || (src && bytes && dst)), SGL_ERR_ARG, "copy_arrays: null table");
+  for (int i = 0; i < n; ++i) {
+    SGL_REQUIRE(bytes[i] >= 0 && (bytes[i] == 0 || (src[i] && dst[i])), SGL_ERR_ARG, "copy_arrays: bad array %d", i);
+    if (bytes[i] > 0) SGL_CUDA_CHECK(cudaMemcpyAsync(dst[i], src[i], (size_t)bytes[i], cudaMemcpyDeviceToHost, (cudaStream_t)stream));
+  }
+  return SGL_OK;
+}
+
 // Pinned buffer of the calling thread (4,096 bytes) for results that the host waits for.
 extern "C" int sgl_host_words(void** out) {
   SGL_REQUIRE(out, SGL_ERR_ARG, "host_words: out is null");

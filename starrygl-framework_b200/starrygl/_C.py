@@ -127,6 +127,7 @@ _SIGNATURES = {
                          _i32, _i32, _i64, _i32, _i32, _i32, _i64, _vp, _vp, _i64, _i32, _vp, _vp, _vp, _vp, _vp, _sz, _vp, _vp]),
     "sgl_query_blocks": (_i32, [_i32, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i64, _i64, _i64, _vp, _vp]),
     "sgl_export_arrays": (_i32, [_i32, _vp, _vp, _vp, _vp, _vp, _i64, _vp, _i64, _vp]),
+    "sgl_copy_arrays": (_i32, [_i32, _vp, _vp, _vp, _vp]),
     "sgl_host_words": (_i32, [C.POINTER(C.c_void_p)]),
     "sgl_wait_word": (_i32, [_vp, _i64, _vp]),
     "sgl_read_back": (_i32, [_vp, _vp, _sz, _vp]),

@@ -25,6 +25,7 @@ from .batch import _enqueue, _graph_range, _root_range
 
 
 _PINNED_MOST, _PINNED_TOTAL = 256 << 20, 2 << 30
+_SHARED_MOST = 32 << 20
 
 
 def _pinned_now() -> int:
@@ -190,28 +191,28 @@ class MaterializedMultiLayerBuilder:
         return final
 
     def _export(self, picks):
-        """Host tensors of device arrays (address, count, bytes per value): views of one buffer per type, filled by one copy
-        each -- which the caller waits for.  The buffers are pinned (a copy to fresh pageable memory takes several times as
-        long) as long as not too much is."""
-        n, at, offs = len(picks), 0, [0] * len(picks)
-        split = 0
-        for want in (8, 4):                         # 8-byte values first
-            for i, (_, count, size) in enumerate(picks):
-                if size == want:
-                    offs[i] = at
-                    at += (count * size + 15) & ~15
-            if want == 8:
-                split = at
-        total = at
-        pin = total <= _PINNED_MOST and _pinned_now() + total <= _PINNED_TOTAL
-        h = torch.empty(split // 8, dtype=torch.int64, pin_memory=pin)
-        f = torch.empty((total - split) // 4, dtype=torch.float32, pin_memory=pin)
-        d = torch.empty(max(total, 16) // 8, dtype=torch.int64, device=self.device)
-        src = (C.c_void_p * max(n, 1))(*[p[0] for p in picks])
-        size = (C.c_int64 * max(n, 1))(*[p[1] * p[2] for p in picks])
-        _C.check(_C.lib().sgl_export_arrays(n, src, size, (C.c_int64 * max(n, 1))(*offs), d.data_ptr(), h.data_ptr(), total, f.data_ptr(),
-                                            split, _C.stream_ptr()))
-        return [h[o // 8:o // 8 + count] if s == 8 else f[(o - split) // 4:(o - split) // 4 + count] for o, (_, count, s) in zip(offs, picks)]
+        """Host tensors of device arrays (address, count, bytes per value), on their way: the caller waits for the copies.  Up to
+        32 MiB in all they are pieces of one buffer, packed by a kernel and filled by one copy, above that each has its own.
+        The memory is pinned (a copy to fresh pageable memory takes several times as long) as long as not too much is."""
+        n, at, offs = len(picks), 0, []
+        for _, count, size in picks:
+            offs.append(at)
+            at += (count * size + 15) & ~15
+        pin = at <= _PINNED_MOST and _pinned_now() + at <= _PINNED_TOTAL
+        src, size = (C.c_void_p * max(n, 1))(*[p[0] for p in picks]), (C.c_int64 * max(n, 1))(*[p[1] * p[2] for p in picks])
+        types = {8: torch.int64, 4: torch.float32}
+        if at > _SHARED_MOST:
+            out = [torch.empty(count, dtype=types[s], pin_memory=pin) for _, count, s in picks]
+            _C.check(_C.lib().sgl_copy_arrays(n, src, size, (C.c_void_p * n)(*[t.data_ptr() for t in out]), _C.stream_ptr()))
+            return out
+        h = torch.empty(at // 8, dtype=torch.int64, pin_memory=pin)
+        d = torch.empty(max(at, 16) // 8, dtype=torch.int64, device=self.device)
+        _C.check(_C.lib().sgl_export_arrays(n, src, size, (C.c_int64 * max(n, 1))(*offs), d.data_ptr(), h.data_ptr(), at, None, at,
+                                            _C.stream_ptr()))
+        # (pieces with a storage of their own size: what saves or shares one does not take the others along)
+        buf = h.numpy()
+        return [torch.frombuffer(buf, dtype=types[s], count=count, offset=o) if count else torch.empty(0, dtype=types[s])
+                for o, (_, count, s) in zip(offs, picks)]
 
     # ---- one slot ------------------------------------------------------------------------------------------------
     def build_aligned_batch(self, task_param, save_path, layer_configs, num_neg=1, global_dst_pool=None, cluster_ids=None,

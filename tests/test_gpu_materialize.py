@@ -96,3 +96,30 @@ def test_one_builder_in_two_threads():
     [t.start() for t in threads]
     [t.join() for t in threads]
     assert not wrong
+
+
+@pytest.mark.parametrize("events", [500, 60000])
+def test_one_tensor_of_a_slot_stands_for_itself(events, tmp_path):
+    """Saved alone it is a file of its own size; in a large slot it holds no other's memory.  Both forms of the copy."""
+    from starrygl.graph.materialize import MaterializedMultiLayerBuilder
+    rng = np.random.default_rng(0)
+    n, m = 50000, 400000
+    z = {k: rng.integers(0, n, m).astype(np.int64) for k in ("src", "dst")}
+    z["ts"] = np.sort(rng.integers(0, 10 ** 6, m)).astype(np.int64)
+    b = MaterializedMultiLayerBuilder(z, n, None, None, 0, 1)
+    at = slice(300000, 300000 + events)
+    out = b.build_aligned_batch(('node', (z["src"][at], z["ts"][at], np.zeros(events))), None,
+                                {'meta': {}, 'layer': [{'type': 'recent', 'fanout': 5}] * 2})
+    from oracle import oracle_np as O
+    csr = O.tcsr_build(z["dst"], z["src"], z["ts"], np.arange(m), n)[:4]
+    ref = O.build_batch(*csr, z["src"][at], z["ts"][at], [5, 5])
+    total = 0
+    for d, r in zip(out, ref):
+        for k in r:
+            assert np.array_equal(d[k].numpy(), r[k]), k
+            assert d[k].untyped_storage().nbytes() == d[k].numel() * d[k].element_size(), k
+            total += d[k].untyped_storage().nbytes()
+    assert (total > 32 << 20) == (events == 60000)
+    path = os.path.join(tmp_path, "one.pt")
+    torch.save(out[1]["indptr"], path)
+    assert os.path.getsize(path) < out[1]["indptr"].numel() * 8 + 4096

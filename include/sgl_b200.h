@@ -622,6 +622,7 @@ int sgl_build_batch_at(const int64_t* indptr, const int64_t* nbr, const int64_t*
  * new ids per list; host_meta (pinned, one word more): receives meta and then a 1 (see sgl_wait_word).  The query comes after
  * everything `producer` (a stream) has been given so far.
  * Replaces: submit_query's worker (csrc/include/starrygl/sample.cu.hpp:1932-1990).
+ * sgl_query_at: the same with a place of its own for every section, section_at[s] words behind base.
  * sgl_query_blocks: source nodes, source times and column indices of the hops' message-flow blocks (self loops
  * included) into `out`: per hop (d + n) nodes, (d + n) times, n indices, with d = queries and n = counts[l].
  * ---------------------------------------------------------------------------------------------- */
@@ -634,6 +635,13 @@ int sgl_query(const int64_t* indptr, const int64_t* nbr, const int64_t* ts, cons
               int policy, int equal_root_time, int64_t allowed_offset, int keep_root_time, int id_bits, int ts_bits,
               int64_t ts_base, int64_t* mapper, int64_t* mask, int64_t epoch, int restart, int64_t* d_next_local,
               int64_t* arena, int64_t* meta, int64_t* host_meta, void* ws, size_t ws_bytes, void* producer, void* stream);
+int sgl_query_at(const int64_t* indptr, const int64_t* nbr, const int64_t* ts, const int64_t* eid, const int64_t* fence,
+              int64_t num_nodes, const int64_t* ev_src, const int64_t* ev_ts, const int64_t* ev_eid, int64_t ev_from,
+              int64_t cap, int64_t t_begin, int64_t t_end, const int64_t* node_chunk, const uint8_t* chunk_mask,
+              int64_t num_chunks, const int64_t* neg, const int64_t* neg_ts, int64_t n_neg, int fanout, int n_hops,
+              int policy, int equal_root_time, int64_t allowed_offset, int keep_root_time, int id_bits, int ts_bits,
+              int64_t ts_base, int64_t* mapper, int64_t* mask, int64_t epoch, int restart, int64_t* d_next_local,
+              const int64_t* section_at, int64_t* base, int64_t* meta, int64_t* host_meta, void* ws, size_t ws_bytes, void* producer, void* stream);
 int sgl_query_blocks(int n_hops, const int64_t* const* node, const int64_t* const* ts, const int64_t* counts,
                      const int64_t* q_ts, const int64_t* ts_ptr, const int64_t* roots_local, const int64_t* neg, const int64_t* neg_ts,
                      int64_t n_roots, int64_t n_pairs, int64_t n_queries, int64_t* out, void* stream);

@@ -115,12 +115,13 @@ extern "C" size_t sgl_query_ws_bytes(int64_t cap, int64_t n_neg, int fanout, int
   return seeds + sample + nodes;
 }
 
-extern "C" int sgl_query(const int64_t* indptr, const int64_t* nbr, const int64_t* ts, const int64_t* eid, const int64_t* fence,
+extern "C" int sgl_query_at(const int64_t* indptr, const int64_t* nbr, const int64_t* ts, const int64_t* eid, const int64_t* fence,
                          int64_t num_nodes, const int64_t* ev_src, const int64_t* ev_ts, const int64_t* ev_eid, int64_t ev_from,
                          int64_t cap, int64_t t_begin, int64_t t_end, const int64_t* node_chunk, const uint8_t* chunk_mask,
                          int64_t num_chunks, const int64_t* neg, const int64_t* neg_ts, int64_t n_neg, int fanout, int n_hops, int policy,
                          int equal_root_time, int64_t allowed_offset, int keep_root_time, int id_bits, int ts_bits, int64_t ts_base,
-                         int64_t* mapper, int64_t* mask, int64_t epoch, int restart, int64_t* d_next_local, int64_t* arena, int64_t* meta,
+                         int64_t* mapper, int64_t* mask, int64_t epoch, int restart, int64_t* d_next_local,
+                            const int64_t* section_at, int64_t* base, int64_t* meta,
                          int64_t* host_meta, void* ws, size_t ws_bytes, void* producer, void* stream_) {
   SGL_NVTX("sgl_query");
   cudaStream_t stream = (cudaStream_t)stream_;
@@ -128,20 +129,13 @@ extern "C" int sgl_query(const int64_t* indptr, const int64_t* nbr, const int64_
               "query: at most 2^31 events and %d hops", kMaxHops);
   SGL_REQUIRE(id_bits >= 0 && ts_bits >= 0 && id_bits + ts_bits < 64, SGL_ERR_UNSUPPORTED,
               "query: id_bits %d + ts_bits %d leave no room for the sentinel key", id_bits, ts_bits);
-  SGL_REQUIRE(ev_src && ev_ts && ev_eid && mapper && mask && d_next_local && arena && meta && host_meta && (n_neg == 0 || (neg && neg_ts)),
+  SGL_REQUIRE(ev_src && ev_ts && ev_eid && mapper && mask && d_next_local && section_at && meta && host_meta && (n_neg == 0 || (neg && neg_ts)),
               SGL_ERR_ARG, "query: null array");
   SGL_REQUIRE(ws_bytes >= sgl_query_ws_bytes(cap, n_neg, fanout, n_hops), SGL_ERR_WORKSPACE, "query: workspace %zu < %zu bytes", ws_bytes,
               sgl_query_ws_bytes(cap, n_neg, fanout, n_hops));
   SGL_CHECK_RC(order_after(stream, (cudaStream_t)producer));
-  int64_t size[kHead + kMaxHops * kPerHop + 1];
-  query_sections(cap, n_neg, fanout, n_hops, size);
-  int64_t* p = arena;
   int sec = 0;
-  auto take = [&]() {
-    int64_t* q = p;
-    p += size[sec++];
-    return q;
-  };
+  auto take = [&]() -> int64_t* { return (int64_t*)((uintptr_t)base + (uintptr_t)section_at[sec++] * 8); };
   int64_t *roots = take(), *roots_local = take(), *ts_ptr = take(), *q_ptr = take(), *q_eid = take(), *q_node = take(), *q_ts = take();
   struct Hop {
     int64_t *nbr, *dst, *ts, *dti, *eid, *local, *offs;
@@ -199,6 +193,25 @@ extern "C" int sgl_query(const int64_t* indptr, const int64_t* nbr, const int64_
   if (in) in->wait(stream, in->mark(side));
   SGL_CHECK_RC(export_words(meta, host_meta, kMetaHead + 2 * n_hops + 1, stream));
   return scope.submit();
+}
+
+extern "C" int sgl_query(const int64_t* indptr, const int64_t* nbr, const int64_t* ts, const int64_t* eid, const int64_t* fence,
+                         int64_t num_nodes, const int64_t* ev_src, const int64_t* ev_ts, const int64_t* ev_eid, int64_t ev_from,
+                         int64_t cap, int64_t t_begin, int64_t t_end, const int64_t* node_chunk, const uint8_t* chunk_mask,
+                         int64_t num_chunks, const int64_t* neg, const int64_t* neg_ts, int64_t n_neg, int fanout, int n_hops, int policy,
+                         int equal_root_time, int64_t allowed_offset, int keep_root_time, int id_bits, int ts_bits, int64_t ts_base,
+                         int64_t* mapper, int64_t* mask, int64_t epoch, int restart, int64_t* d_next_local, int64_t* arena, int64_t* meta,
+                         int64_t* host_meta, void* ws, size_t ws_bytes, void* producer, void* stream) {
+  int64_t at[kHead + kMaxHops * kPerHop + 1], next = 0;
+  SGL_REQUIRE(arena && sgl_query_layout(cap, n_neg, fanout, n_hops, at) >= 0, SGL_ERR_ARG, "query: bad shape or null arena");
+  for (int s = 0; s < kHead + n_hops * kPerHop + 1; ++s) {
+    const int64_t size = at[s];
+    at[s] = next;
+    next += size;
+  }
+  return sgl_query_at(indptr, nbr, ts, eid, fence, num_nodes, ev_src, ev_ts, ev_eid, ev_from, cap, t_begin, t_end, node_chunk, chunk_mask,
+                      num_chunks, neg, neg_ts, n_neg, fanout, n_hops, policy, equal_root_time, allowed_offset, keep_root_time, id_bits, ts_bits,
+                      ts_base, mapper, mask, epoch, restart, d_next_local, at, arena, meta, host_meta, ws, ws_bytes, producer, stream);
 }
 
 // Source side of message-flow blocks for the hops of a query: block l has the D_l destinations (queries of the hop) followed

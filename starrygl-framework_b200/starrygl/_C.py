@@ -125,6 +125,8 @@ _SIGNATURES = {
     "sgl_query_ws_bytes": (_sz, [_i64, _i64, _i32, _i32]),
     "sgl_query": (_i32, [_vp, _vp, _vp, _vp, _vp, _i64, _vp, _vp, _vp, _i64, _i64, _i64, _i64, _vp, _vp, _i64, _vp, _vp, _i64, _i32, _i32,
                          _i32, _i32, _i64, _i32, _i32, _i32, _i64, _vp, _vp, _i64, _i32, _vp, _vp, _vp, _vp, _vp, _sz, _vp, _vp]),
+    "sgl_query_at": (_i32, [_vp, _vp, _vp, _vp, _vp, _i64, _vp, _vp, _vp, _i64, _i64, _i64, _i64, _vp, _vp, _i64, _vp, _vp, _i64, _i32, _i32,
+                         _i32, _i32, _i64, _i32, _i32, _i32, _i64, _vp, _vp, _i64, _i32, _vp, _vp, _vp, _vp, _vp, _vp, _sz, _vp, _vp]),
     "sgl_query_blocks": (_i32, [_i32, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i64, _i64, _i64, _vp, _vp]),
     "sgl_export_arrays": (_i32, [_i32, _vp, _vp, _vp, _vp, _vp, _i64, _vp, _i64, _vp]),
     "sgl_copy_arrays": (_i32, [_i32, _vp, _vp, _vp, _vp]),

@@ -199,40 +199,49 @@ class TemporalResult:
         return f"<TemporalResult with {len(self.neighbors_list)} neighbor layers>"
 
 
+# Arrays of a query up to this size share one allocation (what keeps one keeps the others' memory); larger ones have one each.
+_SHARED_MOST = 32 << 20
+
+
 class _QueryPlan:
-    """Arena layout of a query of one shape (events at most, negatives, fan-out, hops)."""
+    """Layout of the arrays of a query of one shape (events at most, negatives, fan-out, hops)."""
 
     def __init__(self, cap, n_neg, fanout, hops):
-        import ctypes as C
         L = _C.lib()
-        sec = (C.c_int64 * (8 + 8 * hops))()
+        self.places = C.c_int64 * (8 + 8 * hops)
+        sec = self.places()
         self.words = int(L.sgl_query_layout(cap, n_neg, fanout, hops, sec))
         if self.words < 0:
             raise _C.SglError("query: bad shape")
         self.ws_bytes = int(L.sgl_query_ws_bytes(cap, n_neg, fanout, hops))
-        self.start, at = [], 0
-        for w in sec:
-            self.start.append(at)
-            at += int(w)
+        self.size = [int(w) for w in sec]
+        self.at, at = self.places(), 0
+        for s, w in enumerate(self.size):
+            self.at[s] = at
+            at += w
+        self.shared = 8 * self.words <= _SHARED_MOST
 
 
 class _Arena:
-    """All arrays of one query (see ``sgl_query``) with their sizes known on the host: ``cut(section, n)`` is a view."""
+    """All arrays of one query (see ``sgl_query``) with their sizes known on the host: ``cut(section, n)`` is a view.  ``buf``: one
+    tensor, or a list of one per section."""
 
     def __init__(self, buf, plan, hops, meta):
-        self.buf, self.start, self.hops = buf, plan.start, hops
+        self.buf, self.hops = buf, hops
+        self.device = buf.device if plan.shared else buf[0].device
+        self._at = plan.at if plan.shared else None
         self.n_roots, self.n_pairs, self.n_events, self.n_queries = meta[:4]
         self.edges = meta[9:9 + hops]
         self.n_new = sum(meta[9 + hops:10 + 2 * hops])
 
     def cut(self, section, n, floats=False):
-        s = self.start[section]
+        t, s = (self.buf, self._at[section]) if self._at is not None else (self.buf[section], 0)
         if floats:
-            return self.buf[s:s + (n + 1) // 2].view(torch.float32)[:n]
-        return self.buf[s:s + n]
+            return t[s:s + (n + 1) // 2].view(torch.float32)[:n]
+        return t[s:s + n]
 
     def ptr(self, section):
-        return self.buf.data_ptr() + 8 * self.start[section]
+        return self.buf.data_ptr() + 8 * self._at[section] if self._at is not None else self.buf[section].data_ptr()
 
     def holds(self, t, name):
         """Is ``t`` the root array ``name`` as the query left it?"""
@@ -363,10 +372,10 @@ def query_blocks(root, neg_roots, neighbors):
     hops = a.hops
     dst = [a.n_queries] + a.edges[:-1]
     total = sum(2 * (d + n) + n for d, n in zip(dst, a.edges))
-    out = torch.empty(total, dtype=torch.int64, device=a.buf.device)
-    kind, base, start = _hop_words(hops), a.buf.data_ptr(), a.start
-    node = kind(*[base + 8 * start[7 + 8 * l + 6] for l in range(hops)])
-    ts = kind(*[base + 8 * start[7 + 8 * l + 2] for l in range(hops)])
+    out = torch.empty(total, dtype=torch.int64, device=a.device)
+    kind = _hop_words(hops)
+    node = kind(*[a.ptr(7 + 8 * l + 6) for l in range(hops)])
+    ts = kind(*[a.ptr(7 + 8 * l + 2) for l in range(hops)])
     cnt = kind(*a.edges)
     _C.check(_C.lib().sgl_query_blocks(hops, node, ts, cnt, a.ptr(6), a.ptr(2), a.ptr(1), None if neg is None else neg.data_ptr(),
                                        None if neg is None else neg_ts.data_ptr(),
@@ -551,20 +560,24 @@ class CUDAGraph:
             self.stream.wait_stream(torch.cuda.current_stream(dev))
         with _C.on_stream(self.stream):
             mask, node_chunk, n_chunks = ops.chunk_mask(g, chunks, self.mapper)
-            buf = torch.empty(plan.words + 10 + 2 * layers, dtype=torch.int64, device=dev)
+            if plan.shared:
+                buf = torch.empty(plan.words + 10 + 2 * layers, dtype=torch.int64, device=dev)
+                at, base, meta = plan.at, buf.data_ptr(), buf.data_ptr() + 8 * plan.words
+            else:
+                buf = [torch.empty(w, dtype=torch.int64, device=dev) for w in (*plan.size, 10 + 2 * layers)]
+                at, base, meta = plan.places(*[t.data_ptr() // 8 for t in buf[:-1]]), None, buf[-1].data_ptr()
             ws = _C.WORKSPACE.get(plan.ws_bytes, dev, sp)
         rl = self.relabel
         epoch = rl.epoch + (1 if op == "f" else 0)       # the reference restarts the numbering on "f"
         slot = self._slot()
         slot[1][10 + 2 * layers] = 0
-        base = buf.data_ptr()
-        rc = _C.lib().sgl_query(
+        rc = _C.lib().sgl_query_at(
             g.indptr.data_ptr(), g.nbr.data_ptr(), g.ts.data_ptr(), g.eid.data_ptr(), None if g.fence is None else g.fence.data_ptr(),
             g.num_nodes, self.ev[0].data_ptr(), self.ev[1].data_ptr(), self.ev[2].data_ptr(), first, cap, t0, t1,
             None if node_chunk is None else node_chunk.data_ptr(), None if mask is None else mask.data_ptr(), n_chunks,
             neg_ids.data_ptr() if n_neg else None, neg_ts.data_ptr() if n_neg else None, n_neg, fanout, layers, _C.POLICY[stype],
             int(eq), off, int(keep), ops.bits_for(g.num_nodes - 1), ops.bits_for(g.ts_max - g.ts_min), g.ts_min, rl.mapper.data_ptr(),
-            rl.mask.data_ptr(), epoch, int(op == "f"), rl.next_local.data_ptr(), base, base + 8 * plan.words, slot[0], ws.data_ptr(),
+            rl.mask.data_ptr(), epoch, int(op == "f"), rl.next_local.data_ptr(), at, base, meta, slot[0], ws.data_ptr(),
             ws.numel(), producer, sp)
         if rc:                            # nothing was enqueued: the numbering goes on as it was
             _FREE_SLOTS.append(slot)

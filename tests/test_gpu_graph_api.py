@@ -331,3 +331,31 @@ def test_a_dropped_graph_waits_for_queries_that_nobody_fetched():
         gone = weakref.ref(g)
         del g
         assert gone() is None and own.query() and len(L._FREE_SLOTS) == free
+
+
+def test_large_query_and_what_one_of_its_tensors_holds():
+    """A query above the size up to which its arrays share an allocation: the arrays, the blocks, and the memory of a kept one."""
+    from starrygl.graph.graph import AsyncBlock
+    from starrygl.lib import libstarrygl_comm as L
+    n, src, dst, ts, eid = make_events(n=5000, m=400_000, tmax=10 ** 6)
+    g = L.from_edge_index(n, 1, cu(src), cu(dst), cu(ts), cu(eid))
+    none = torch.empty(0, dtype=torch.int64, device="cuda")
+    ask = lambda: (g.submit_query(500_000, 560_000, None, none, none, "recent", 2, 10, -1, False, False, "f"), g.get())[1]
+    ask()
+    step = g.sample_src_in_chunks_khop(g.get_seeds_in_chunks(None, 500_000, 560_000), None, 10, 2, -1, False, False, "recent")
+    step.materialize()
+    torch.cuda.synchronize()
+    before = torch.cuda.memory_allocated()
+    r = ask()
+    assert torch.cuda.memory_allocated() - before > 64 << 20
+    _same_blocks(AsyncBlock.to_block(r.roots, r.neg_roots, r.neighbors, r.nodes_remapper_id), _blocks_by_parts(r))
+    for a, b in zip(r.neighbors, step.neighbors):
+        for k in ("root_start_ptr", "neighbors_ts", "neighbors_eid", "neighbors_dt"):
+            assert torch.equal(getattr(a, k), getattr(b, k)), k
+        assert torch.equal(r.nodes_remapper_id[a.neighbors], b.hop.nbr[:b.neighbor_num])
+    eids = r.neighbors[0].neighbors_eid
+    keep = eids.numel()
+    del a, r
+    torch.cuda.synchronize()
+    assert torch.cuda.memory_allocated() - before < 4 * 8 * keep
+    g.close()

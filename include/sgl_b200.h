@@ -584,7 +584,7 @@ int sgl_lower_bound_i64(const int64_t* sorted, int64_t n, const int64_t* values,
  * hop l at that edge's time), merged list and CSC per hop -- sgl_unique_pairs, sgl_sample_layer_fenced and sgl_build_csc
  * enqueued back to back with all sizes on the device.  All results lie in one caller-allocated arena of
  * sgl_build_batch_layout(...) 64-bit words, as consecutive sections whose sizes that function writes to section_words
- * (room for 3 + 14 * n_hops entries; at most 8 hops; returns -1 on a bad argument):
+ * (room for 3 + 14 * n_hops entries; returns -1 on a bad argument):
  *   3 for the roots   gids[n], ts[n], inverse map[n]
  *   14 per hop        nbr, dst, ts, dt (fp32), eid, offsets of the sampled edges; merged gids, ts; the edges' positions in the
  *                     merged list; CSC indptr, indices, ts, dt (fp32), eid (absent for the first hop: its edges are in

@@ -15,6 +15,9 @@
 // Meta (8-byte words): entries of the root list, then per hop sampled edges and entries of the merged list, then a status
 // word (used when the caller has none of its own).
 
+#include <memory>
+#include <new>
+
 #include "chain.cuh"
 #include "rowcsc.cuh"
 #include "sampler.cuh"
@@ -25,7 +28,6 @@ using namespace sgl;
 
 namespace {
 
-constexpr int kMaxHops = 8;
 constexpr int kHostWords = 512;   // of sgl_host_words
 constexpr int kRootSections = 3, kHopSections = 14;
 
@@ -152,7 +154,7 @@ size_t narrow_ws(int64_t n, const int32_t* fanouts, int hops) {
 }  // namespace
 
 extern "C" int64_t sgl_build_batch_layout(int64_t n_roots, const int32_t* fanouts, int n_hops, int64_t* section_words) {
-  if (n_roots < 0 || n_hops < 0 || n_hops > kMaxHops || (n_hops && !fanouts) || !section_words) return -1;
+  if (n_roots < 0 || n_hops < 0 || (n_hops && !fanouts) || !section_words) return -1;
   const int s = batch_sections(n_roots, fanouts, n_hops, section_words);
   int64_t total = 0;
   for (int i = 0; i < s; ++i) total += section_words[i];
@@ -172,8 +174,7 @@ extern "C" int sgl_build_batch_at(const int64_t* indptr, const int64_t* nbr, con
                                   void* side_stream, void* stream_) {
   SGL_NVTX("sgl_build_batch");
   cudaStream_t stream = (cudaStream_t)stream_;
-  SGL_REQUIRE(n_roots >= 0 && n_hops >= 0 && n_hops <= kMaxHops && (n_hops == 0 || fanouts), SGL_ERR_ARG,
-              "build_batch: bad size (at most %d hops)", kMaxHops);
+  SGL_REQUIRE(n_roots >= 0 && n_hops >= 0 && (n_hops == 0 || fanouts), SGL_ERR_ARG, "build_batch: bad size");
   for (int l = 0; l < n_hops; ++l) SGL_REQUIRE(fanouts[l] >= 1, SGL_ERR_ARG, "build_batch: fanout=%d must be >= 1", fanouts[l]);
   SGL_REQUIRE(meta, SGL_ERR_ARG, "build_batch: meta is null");
   LaunchScope scope(stream);
@@ -204,7 +205,9 @@ extern "C" int sgl_build_batch_at(const int64_t* indptr, const int64_t* nbr, con
   struct Hop {
     int64_t *nbr, *dst, *ts, *eid, *offs, *gids, *gts, *col, *indptr, *indices, *cts, *ceid;
     float *dt, *cdt;
-  } hop[kMaxHops];
+  };
+  const std::unique_ptr<Hop[]> hop(new (std::nothrow) Hop[n_hops + 1]);
+  SGL_REQUIRE(hop, SGL_ERR_ARG, "build_batch: no host memory for %d hops", n_hops);
   for (int l = 0; l < n_hops; ++l) {
     Hop& h = hop[l];
     h.nbr = take(); h.dst = take(); h.ts = take(); h.dt = (float*)take(); h.eid = take(); h.offs = take();
@@ -284,8 +287,8 @@ extern "C" int sgl_build_batch(const int64_t* indptr, const int64_t* nbr, const 
                                const int32_t* fanouts, int n_hops, int policy, int equal_root_time, int64_t allowed_offset,
                                uint64_t seed, int id_bits, int ts_bits, int64_t ts_base, int64_t* arena, int64_t* meta,
                                int32_t* d_status, int64_t* host_meta, void* ws, size_t ws_bytes, void* side_stream, void* stream) {
-  int64_t at[kRootSections + kMaxHops * kHopSections];
-  SGL_REQUIRE(sgl_build_batch_layout(n_roots, fanouts, n_hops, at) >= 0, SGL_ERR_ARG, "build_batch: bad size (at most %d hops)", kMaxHops);
+  const std::unique_ptr<int64_t[]> at(n_hops >= 0 ? new (std::nothrow) int64_t[kRootSections + (size_t)n_hops * kHopSections] : nullptr);
+  SGL_REQUIRE(at && sgl_build_batch_layout(n_roots, fanouts, n_hops, at.get()) >= 0, SGL_ERR_ARG, "build_batch: bad size");
   SGL_REQUIRE(arena || n_roots == 0, SGL_ERR_ARG, "build_batch: null array");
   int64_t next = 0;
   for (int s = 0; s < kRootSections + n_hops * kHopSections; ++s) {
@@ -294,7 +297,7 @@ extern "C" int sgl_build_batch(const int64_t* indptr, const int64_t* nbr, const 
     next += size;
   }
   return sgl_build_batch_at(indptr, nbr, ts, eid, fence, num_nodes, roots, root_ts, n_roots, fanouts, n_hops, policy, equal_root_time,
-                            allowed_offset, seed, id_bits, ts_bits, ts_base, at, arena, nullptr, meta, d_status, host_meta, ws, ws_bytes,
+                            allowed_offset, seed, id_bits, ts_bits, ts_base, at.get(), arena, nullptr, meta, d_status, host_meta, ws, ws_bytes,
                             side_stream, stream);
 }
 

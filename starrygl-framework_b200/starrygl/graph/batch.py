@@ -29,8 +29,6 @@ class _Plan:
     def __init__(self, n: int, fanouts: Sequence[int]):
         L = _C.lib()
         hops = len(fanouts)
-        if hops > 8:
-            raise _C.SglError("build_batch: at most 8 hops")
         self.fan = (C.c_int32 * max(hops, 1))(*[int(k) for k in fanouts])
         self.places = C.c_int64 * (3 + 14 * hops)
         sec = self.places()
@@ -133,7 +131,8 @@ class DeviceBatch:
 
     def _read(self):
         """The one read-back: every count and, when the batch owns it, the status word."""
-        host = _C.read_words(self._meta, 2 + 2 * len(self.fanouts))
+        n = 2 + 2 * len(self.fanouts)
+        host = _C.read_words(self._meta, n) if n < 512 else self._meta.tolist()
         return host[:-1], host[-1] & 0xFFFFFFFF
 
     def finish(self) -> List[dict]:
@@ -262,6 +261,8 @@ def build_batch(g, roots, root_ts, fanouts, policy="recent", **kw) -> List[dict]
         return build_batch_async(g, roots, root_ts, fanouts, policy, **{**kw, "ts_range": (a, b)}).finish()
     addr, words = _C.host_words()
     last = 1 + 2 * len(fanouts)
+    if last + 2 > len(words):
+        return build_batch_async(g, roots, root_ts, fanouts, policy, **kw).finish()
     db = _enqueue(g, roots, root_ts, fanouts, policy, g.ts_min, g.ts_max, kw.get("equal_root_time", False), kw.get("allowed_offset", -1),
                   kw.get("seed", 0), None, None, addr)
     _C.check(_C.lib().sgl_wait_word(addr + 8 * (last + 1), 1, _C.stream_ptr()))

@@ -145,7 +145,7 @@ class MaterializedMultiLayerBuilder:
             _C.check(L.sgl_plan_routes(k, ref(ids), ref(ns), ref(d_ns), self.node_parts.data_ptr(), self.node_parts.numel(), self.pid,
                                        rt.indptr.data_ptr(), rt.indices.data_ptr(), rt.locs.data_ptr(), P, ref(cp), ref(outs), ref(cnts),
                                        mp + 8 * (nb - 1), ws.data_ptr(), ws.numel(), sp))
-        host = _C.read_words(meta, meta.numel())    # the one synchronisation before the copy
+        host = _C.read_words(meta, meta.numel()) if meta.numel() < 512 else meta.tolist()    # the one synchronisation before the copy
         bits = host[nb - 1] & 0xFFFFFFFF
         if bits:
             raise _C.SglError(f"build_batch: device status {bits} ({_C.decode_status(bits)})")
@@ -192,7 +192,8 @@ class MaterializedMultiLayerBuilder:
 
     def _export(self, picks):
         """Host tensors of device arrays (address, count, bytes per value), on their way: the caller waits for the copies.  Up to
-        32 MiB in all they are pieces of one buffer, packed by a kernel and filled by one copy, above that each has its own.
+        32 MiB in all they are pieces of one buffer, packed by a kernel and filled by one copy, above that (and above the kernel's
+        96 arrays, nine hops) each has its own.
         The memory is pinned (a copy to fresh pageable memory takes several times as long) as long as not too much is."""
         n, at, offs = len(picks), 0, []
         for _, count, size in picks:
@@ -201,7 +202,7 @@ class MaterializedMultiLayerBuilder:
         pin = at <= _PINNED_MOST and _pinned_now() + at <= _PINNED_TOTAL
         src, size = (C.c_void_p * max(n, 1))(*[p[0] for p in picks]), (C.c_int64 * max(n, 1))(*[p[1] * p[2] for p in picks])
         types = {8: torch.int64, 4: torch.float32}
-        if at > _SHARED_MOST:
+        if at > _SHARED_MOST or n > 96:
             out = [torch.empty(count, dtype=types[s], pin_memory=pin) for _, count, s in picks]
             _C.check(_C.lib().sgl_copy_arrays(n, src, size, (C.c_void_p * n)(*[t.data_ptr() for t in out]), _C.stream_ptr()))
             return out

@@ -168,3 +168,22 @@ def test_a_kept_tensor_keeps_little_else(roots):
     del out
     assert torch.cuda.memory_allocated() - before <= max(8 * roots + 4096, 0 if roots > 4096 else 33 << 20)
     assert int(keep.max()) < n
+
+
+@pytest.mark.parametrize("hops", [9, 12, 260])
+def test_as_many_hops_as_asked_for(hops):
+    from starrygl.graph.batch import build_batch
+    rng = np.random.default_rng(7)
+    n, m = 300, 40000
+    z = {"n": n, "dst": rng.integers(0, n, m).astype(np.int64), "src": rng.integers(0, n, m).astype(np.int64),
+         "ts": np.sort(rng.integers(0, 10 ** 6, m)).astype(np.int64), "eid": np.arange(m, dtype=np.int64)}
+    g = build_graph(z)
+    csr = O.tcsr_build(z["dst"], z["src"], z["ts"], z["eid"], n)[:4]
+    roots, rts = rng.integers(0, n, 20).astype(np.int64), np.full(20, 10 ** 6 - 1, np.int64)
+    fanouts = [2, 2] + [1] * (hops - 2)
+    ref = O.build_batch(*csr, roots, rts, fanouts)
+    for out in (build_batch(g, cu(roots), cu(rts), fanouts), build_batch(g, cu(roots), cu(rts), fanouts, ts_range=(0, 10 ** 6))):
+        assert len(out) == len(ref)
+        for i, (d, r) in enumerate(zip(out, ref)):
+            for k in r:
+                assert np.array_equal(npy(d[k]), r[k]), (i, k)

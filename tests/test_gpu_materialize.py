@@ -123,3 +123,28 @@ def test_one_tensor_of_a_slot_stands_for_itself(events, tmp_path):
     path = os.path.join(tmp_path, "one.pt")
     torch.save(out[1]["indptr"], path)
     assert os.path.getsize(path) < out[1]["indptr"].numel() * 8 + 4096
+
+
+@pytest.mark.parametrize("hops", [9, 10, 12])
+def test_slots_of_many_hops(hops):
+    from oracle import oracle_np as O
+    from starrygl.cache.replica_table import CSRReplicaTable
+    from starrygl.graph.materialize import MaterializedMultiLayerBuilder
+    rng = np.random.default_rng(0)
+    n, m, parts = 300, 40000, 3
+    z = {k: rng.integers(0, n, m).astype(np.int64) for k in ("src", "dst")}
+    z["ts"] = np.sort(rng.integers(0, 10 ** 6, m)).astype(np.int64)
+    ranks = torch.arange(parts).repeat(n)                 # every node on every partition
+    table = CSRReplicaTable(torch.arange(n + 1) * parts, ranks, torch.arange(n).repeat_interleave(parts))
+    node_parts = torch.arange(n) % parts
+    b = MaterializedMultiLayerBuilder(z, n, node_parts, table, 0, parts)
+    roots, rts = rng.integers(0, n, 50).astype(np.int64), np.full(50, 10 ** 6 - 1, np.int64)
+    out = b.build_aligned_batch(('node', (roots, rts, np.zeros(50))), None, {'meta': {}, 'layer': [{'type': 'recent', 'fanout': 1}] * hops})
+    ref = O.build_batch(*O.tcsr_build(z["dst"], z["src"], z["ts"], np.arange(m), n)[:4], roots, rts, [1] * hops)
+    assert len(out) == len(ref) == hops + 1 and len(out[0]["comm_plan"]) == hops + 1
+    for d, r, p in zip(out, ref, out[0]["comm_plan"]):
+        for k in r:
+            assert np.array_equal(d[k].numpy(), r[k]), k
+        gids = r["gids"]
+        last = np.append(gids[1:] != gids[:-1], True) & (gids % parts == 0)
+        assert np.array_equal(p.send_indices.numpy(), np.tile(last.nonzero()[0], 2)) and p.send_sizes.tolist() == [0, last.sum(), last.sum()]

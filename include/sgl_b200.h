@@ -69,6 +69,9 @@ int sgl_radix_sort_launches(int64_t n, int num_bits);
 int sgl_radix_sort_u64_u32(uint64_t* keys, uint32_t* vals, uint64_t* keys_alt, uint32_t* vals_alt, int64_t n,
                            int num_bits, int* h_result_in_alt, void* ws, size_t ws_bytes, void* stream);
 int64_t sgl_look_back_limit(int64_t ns);
+/* Composite entry points are submitted as one executable graph from the second call of a sequence of kernels on a stream on;
+ * how many of them the calling thread holds (at most 32). */
+int sgl_launch_graphs(void);
 
 /* ------------------------------------------------------------------------------------------------
  * T-CSR construction.  Rows are keyed by `key` (node id in [0, num_nodes)); inside a row edges are in

@@ -18,10 +18,12 @@ struct Cached {
   }
   std::vector<cudaGraphNode_t> nodes;
   uint64_t last_use = 0;
+  bool refused = false;               // no graph could be made of it (no memory, say): launched one by one
 };
 
 struct Thread {
   LaunchScope* open = nullptr;
+  int plain = 0;
   LaunchList list;
   std::vector<Cached*> graphs;
   uint64_t clock = 0;
@@ -83,8 +85,9 @@ int build(Cached& c) {
   if (e == cudaSuccess) e = cudaGraphInstantiate(&exec, graph, 0);
   if (e != cudaSuccess) {
     cudaGraphDestroy(graph);
-    set_error("building a launch graph failed: %s", cudaGetErrorString(e));
-    return SGL_ERR_CUDA;
+    cudaGetLastError();
+    c.refused = true;
+    return SGL_OK;
   }
   c.graph = graph;
   c.exec = exec;
@@ -110,11 +113,14 @@ int zero_async(void* p, size_t bytes, cudaStream_t stream) {
   return launch(zero_words_kernel, stream_grid((int64_t)(bytes / 4), 256, 8), 256, 0, stream, (uint32_t*)p, bytes / 4);
 }
 
+PlainLaunches::PlainLaunches() { ++t_state.plain; }
+PlainLaunches::~PlainLaunches() { --t_state.plain; }
+
 LaunchScope* LaunchScope::current() { return t_state.open; }
 
 LaunchScope::LaunchScope(cudaStream_t main) : owner_(false), main_(main) {
   Thread& t = t_state;
-  if (t.open != nullptr) return;
+  if (t.open != nullptr || t.plain > 0) return;
   cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
   if (cudaStreamIsCapturing(main, &st) != cudaSuccess) {
     cudaGetLastError();
@@ -209,19 +215,25 @@ int LaunchScope::submit() {
     return one_by_one(main_);
   }
   c->last_use = t.clock;
-  if (c->exec == nullptr) {
-    SGL_CHECK_RC(build(*c));
-  } else {
+  if (c->exec == nullptr && !c->refused) SGL_CHECK_RC(build(*c));
+  else if (!c->refused) {
     for (size_t i = 0; i < l.used; ++i) {
       const cudaKernelNodeParams p = node_params(l.nodes[i]);
       SGL_CUDA_CHECK(cudaGraphExecKernelNodeSetParams(c->exec, c->nodes[i], &p));
     }
   }
+  if (c->refused) return one_by_one(main_);
   SGL_CUDA_CHECK(cudaGraphLaunch(c->exec, main_));
   return SGL_OK;
 }
 
 }  // namespace sgl
+
+extern "C" int sgl_launch_graphs(void) {
+  int n = 0;
+  for (const sgl::Cached* c : sgl::t_state.graphs) n += c->exec != nullptr ? 1 : 0;
+  return n;
+}
 
 extern "C" int64_t sgl_look_back_limit(int64_t ns) {
   const int64_t before = sgl::t_look_back_ns;

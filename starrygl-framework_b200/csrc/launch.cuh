@@ -43,6 +43,14 @@ struct LaunchList {
   }
 };
 
+// While one exists, the calling thread launches its kernels one by one: for calls that must not make the driver allocate, as an
+// executable graph does.
+class PlainLaunches {
+ public:
+  PlainLaunches();
+  ~PlainLaunches();
+};
+
 class LaunchScope {
  public:
   explicit LaunchScope(cudaStream_t main);

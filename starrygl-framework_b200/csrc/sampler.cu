@@ -756,7 +756,8 @@ extern "C" int sgl_sample_layer_static(const int64_t* indptr, const int64_t* nbr
     SGL_REQUIRE(p != nullptr, SGL_ERR_CUDA, "sample_layer_static: no device address for the built-in scratch");
     g_static_scratch_addr[dev] = p;
   }
-  // sgl_sample_layer clears the part of the scratch it uses on the stream before its kernel.
+  // (no clearing: launches of this size leave the only word of the scratch that would need it alone)
+  const PlainLaunches plain;
   return sgl_sample_layer(indptr, nbr, ts, eid, num_nodes, targets, target_ts, n_targets, nullptr, fanout, policy,
                           equal_root_time, allowed_offset, keep_root_time, seed, rng_stream, out_nbr, out_dst, out_ts,
                           out_dt, nullptr, out_eid, out_offsets, d_status, g_static_scratch_addr[dev], kStaticScratchBytes,

@@ -81,3 +81,24 @@ def test_static_scratch_entry_point_rejects_oversized_batches():
     rc, out, _ = _call_static(L, g, e, e, 3, 0, seed=0)
     torch.cuda.synchronize()
     assert rc == 0 and out[5].tolist() == [0]
+
+
+def test_static_scratch_entry_point_makes_no_graph():
+    """Called again and again it makes no executable graph (which takes device memory), and its results stay the same."""
+    from starrygl import _C, ops
+    L = _C.lib()
+    g, rng = _graph(2)
+    q = torch.from_numpy(rng.integers(0, g.num_nodes, 3000).astype(np.int64)).cuda()
+    qt = torch.from_numpy(rng.integers(0, 100001, 3000).astype(np.int64)).cuda()
+    stream = torch.cuda.Stream()
+    with torch.cuda.stream(stream):
+        held = L.sgl_launch_graphs()
+        outs = [_call_static(L, g, q, qt, 11, 0, seed=0)[1] for _ in range(4)]
+        assert L.sgl_launch_graphs() == held
+        ops.sample_layer(g, q, qt, 11, "recent")
+        ref = ops.sample_layer(g, q, qt, 11, "recent")
+        assert L.sgl_launch_graphs() == held + 1
+    torch.cuda.synchronize()
+    tot = int(ref.offsets[-1].item())
+    for out in outs:
+        assert torch.equal(out[5], ref.offsets) and torch.equal(out[0][:tot], ref.nbr[:tot]) and torch.equal(out[4][:tot], ref.eid[:tot])

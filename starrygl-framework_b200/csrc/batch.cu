@@ -360,9 +360,15 @@ extern "C" int sgl_copy_arrays(int n, const void* const* src, const int64_t* byt
 // Pinned buffer of the calling thread (4,096 bytes) for results that the host waits for.
 extern "C" int sgl_host_words(void** out) {
   SGL_REQUIRE(out, SGL_ERR_ARG, "host_words: out is null");
-  static thread_local void* pinned = nullptr;
-  if (pinned == nullptr) SGL_CUDA_CHECK(cudaHostAlloc(&pinned, kHostWords * 8, cudaHostAllocPortable));
-  *out = pinned;
+  struct Pinned {
+    void* p = nullptr;
+    ~Pinned() {                          // (with the thread; at the end of the process the driver may be gone already)
+      if (p) cudaFreeHost(p);
+    }
+  };
+  static thread_local Pinned words;
+  if (words.p == nullptr) SGL_CUDA_CHECK(cudaHostAlloc(&words.p, kHostWords * 8, cudaHostAllocPortable));
+  *out = words.p;
   return SGL_OK;
 }
 

@@ -4,26 +4,38 @@
 
 namespace sgl {
 
+// N events per device of the calling thread, made on first use and given back when the thread ends.
+template <int N>
+struct ThreadEvents {
+  cudaEvent_t ev[64][N] = {};
+  ~ThreadEvents() {
+    for (auto& d : ev)
+      for (cudaEvent_t e : d)
+        if (e) cudaEventDestroy(e);
+  }
+  int of_device(cudaEvent_t** out) {
+    int dev = 0;
+    SGL_CUDA_CHECK(cudaGetDevice(&dev));
+    for (cudaEvent_t& e : ev[dev & 63])
+      if (e == nullptr) SGL_CUDA_CHECK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+    *out = ev[dev & 63];
+    return SGL_OK;
+  }
+};
+
 // Order between the two streams of an entry point: nodes of the launch scope, or (captured calls) events of this thread, recorded
 // and waited for at once and so reusable.
 struct Order {
   static constexpr int kMarks = 4;
   LaunchScope* scope;
   std::vector<int> nodes[kMarks];
-  cudaEvent_t ev[kMarks];
+  cudaEvent_t* ev;
 
   int init(LaunchScope* s) {
     scope = s;
     if (scope) return SGL_OK;
-    static thread_local cudaEvent_t pool[64][kMarks];
-    int dev = 0;
-    SGL_CUDA_CHECK(cudaGetDevice(&dev));
-    for (int i = 0; i < kMarks; ++i) {
-      cudaEvent_t& e = pool[dev & 63][i];
-      if (e == nullptr) SGL_CUDA_CHECK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-      ev[i] = e;
-    }
-    return SGL_OK;
+    static thread_local ThreadEvents<kMarks> pool;
+    return pool.of_device(&ev);
   }
   int mark(int i, cudaStream_t s) {
     if (scope) nodes[i] = scope->mark(s);
@@ -40,13 +52,12 @@ struct Order {
 // what `stream` is given from here on comes after everything `producer` has been given so far
 inline int order_after(cudaStream_t stream, cudaStream_t producer) {
   if (producer == stream) return SGL_OK;
-  static thread_local cudaEvent_t ev[64];
-  int dev = 0;
-  SGL_CUDA_CHECK(cudaGetDevice(&dev));
-  cudaEvent_t& e = ev[dev & 63];
-  if (e == nullptr) SGL_CUDA_CHECK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-  SGL_CUDA_CHECK(cudaEventRecord(e, producer));
-  SGL_CUDA_CHECK(cudaStreamWaitEvent(stream, e, 0));
+  static thread_local ThreadEvents<1> pool;
+  cudaEvent_t* e = nullptr;
+  const int rc = pool.of_device(&e);
+  if (rc != SGL_OK) return rc;
+  SGL_CUDA_CHECK(cudaEventRecord(*e, producer));
+  SGL_CUDA_CHECK(cudaStreamWaitEvent(stream, *e, 0));
   return SGL_OK;
 }
 

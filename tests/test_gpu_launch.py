@@ -57,3 +57,18 @@ def test_threads_side_by_side():
         th.start()
         th.join()
         assert done == [[True] * 4]
+
+
+def test_a_thread_that_ends_gives_its_result_words_back():
+    from starrygl import _C
+    t = torch.arange(8, device="cuda")
+    used, ok = set(), []
+
+    def once():
+        used.add(_C.host_words()[0])
+        ok.append(_C.read_words(t, 8) == list(range(8)))
+    for _ in range(64):
+        th = threading.Thread(target=once)
+        th.start()
+        th.join()
+    assert all(ok) and len(ok) == 64 and len(used) < 16        # the driver hands freed words out again

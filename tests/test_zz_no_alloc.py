@@ -8,6 +8,7 @@ caller-provided workspace.  It also checks the size limit.  Collected last on pu
 failure has then already run every other test.
 """
 import ctypes as C
+import threading
 
 import numpy as np
 import pytest
@@ -90,14 +91,20 @@ def test_static_scratch_entry_point_makes_no_graph():
     g, rng = _graph(2)
     q = torch.from_numpy(rng.integers(0, g.num_nodes, 3000).astype(np.int64)).cuda()
     qt = torch.from_numpy(rng.integers(0, 100001, 3000).astype(np.int64)).cuda()
-    stream = torch.cuda.Stream()
-    with torch.cuda.stream(stream):
-        held = L.sgl_launch_graphs()
-        outs = [_call_static(L, g, q, qt, 11, 0, seed=0)[1] for _ in range(4)]
-        assert L.sgl_launch_graphs() == held
-        ops.sample_layer(g, q, qt, 11, "recent")
-        ref = ops.sample_layer(g, q, qt, 11, "recent")
-        assert L.sgl_launch_graphs() == held + 1
+    got = []
+
+    def work():                          # (a thread of its own: it holds no graphs yet)
+        with torch.cuda.stream(torch.cuda.Stream()):
+            outs = [_call_static(L, g, q, qt, 11, 0, seed=0)[1] for _ in range(4)]
+            got.append(L.sgl_launch_graphs())
+            ops.sample_layer(g, q, qt, 11, "recent")
+            ref = ops.sample_layer(g, q, qt, 11, "recent")
+            got.extend([L.sgl_launch_graphs(), outs, ref])
+    th = threading.Thread(target=work)
+    th.start()
+    th.join()
+    none, one, outs, ref = got
+    assert none == 0 and one == 1
     torch.cuda.synchronize()
     tot = int(ref.offsets[-1].item())
     for out in outs:

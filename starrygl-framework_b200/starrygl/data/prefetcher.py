@@ -104,8 +104,12 @@ class HostToDevicePrefetcher:
         # The kernels read the inputs where they are, which no allocator knows: they are held until their batch is done,
         # whatever becomes of the batch object.
         held, spare = self._held[slot], self._spare[slot]
-        while held and held[0][0].query():
-            spare.append(held.popleft()[0])
+        if len(held) >= 8:               # (not for every batch: asking costs as much as recording)
+            if held[-1][0].query():
+                spare.extend(e for e, _ in held)
+                held.clear()
+            while held and held[0][0].query():
+                spare.append(held.popleft()[0])
         ready = spare.pop() if spare else torch.cuda.Event()
         self._seq += 1
         c_n.value, c_seq.value, c_cons.value = n, self._seq, _C.stream_ptr()

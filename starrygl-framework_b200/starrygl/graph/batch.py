@@ -17,8 +17,9 @@ import torch
 from .. import _C, ops
 
 
-# Results up to this size share one allocation (a tensor that is kept keeps the others' memory); larger ones have one each.
-_SHARED_MOST = 32 << 20
+# Results up to this size share one allocation (a tensor that is kept keeps the others' memory), together with the raw arrays when
+# they are small; larger ones have an allocation each.
+_SHARED_MOST, _WHOLE_MOST = 32 << 20, 2 << 20
 
 
 class _Plan:
@@ -40,14 +41,19 @@ class _Plan:
         for l in range(hops):
             kept += [3 + 14 * l + i for i in ((2, 3, 4, 5, 6, 7, 8) if l == 0 else (6, 7, 9, 10, 11, 12, 13))]
         self.kept = kept
-        at, words, raw = self.places(), 0, 0
+        self.whole = 8 * sum(self.size) <= _WHOLE_MOST
+        start, words, raw = [0] * len(self.size), 0, 0       # place in the results, or -1 - place in the raw arrays
         for s in kept:
-            at[s] = words
+            start[s] = words
             words += self.size[s]
         for s in sorted(set(range(len(self.size))) - set(kept)):
-            at[s] = -1 - raw
-            raw += self.size[s]
-        self.at, self.words, self.raw_words = at, words, raw
+            if self.whole:
+                start[s] = words
+                words += self.size[s]
+            else:
+                start[s] = -1 - raw
+                raw += self.size[s]
+        self.start, self.at, self.words, self.raw_words = start, self.places(*start), words, raw
         self.shared = 8 * words <= _SHARED_MOST
 
 
@@ -78,6 +84,7 @@ class DeviceBatch:
     def __init__(self, g, n, fanouts, plan, results, raw, meta, status):
         self.g, self.n, self.fanouts = g, n, list(fanouts)
         self._plan, self._results, self._raw, self._meta, self._status = plan, results, raw, meta, status
+        self._shared = not isinstance(results, dict)
         self._layers = None
 
     @property
@@ -93,10 +100,10 @@ class DeviceBatch:
 
     def _place(self, section):
         """(tensor, offset) of a section."""
-        s = self._plan.at[section]
+        s = self._plan.start[section]
         if s < 0:
             return self._raw, -1 - s
-        return (self._results, s) if self._plan.shared else (self._results[section], 0)
+        return (self._results, s) if self._shared else (self._results[section], 0)
 
     def _view(self, section, count, floats=False):
         t, s = self._place(section)
@@ -104,9 +111,13 @@ class DeviceBatch:
             return t[s:s + (count + 1) // 2].view(torch.float32)[:count]
         return t[s:s + count]
 
-    def address(self, section):
-        t, s = self._place(section)
-        return t.data_ptr() + 8 * s
+    def addresses(self):
+        """Address of every section (0: a raw array)."""
+        start = self._plan.start
+        if not self._shared:
+            return [0 if s < 0 else self._results[i].data_ptr() for i, s in enumerate(start)]
+        base = self._results.data_ptr()
+        return [0 if s < 0 else base + 8 * s for s in start]
 
     @property
     def layers(self):
@@ -147,6 +158,12 @@ class DeviceBatch:
     def _trim(self, host):
         self._host = host
         v, n = self._view, self.n
+        if self._shared:
+            t, at = self._results, self._plan.start
+
+            def v(section, count, floats=False):
+                s = at[section]
+                return t[s:s + (count + 1) // 2].view(torch.float32)[:count] if floats else t[s:s + count]
         n_list = host[0]
         out = [{"gids": v(0, n_list), "ts": v(1, n_list), "inv_map": v(2, n)}]
         prev_n = n_list
@@ -178,20 +195,26 @@ class DeviceBatch:
 
 
 def _enqueue(g, roots, root_ts, fanouts, policy, lo, hi, equal_root_time, allowed_offset, seed, status, side, host=None,
-             meta=None) -> DeviceBatch:
+             meta=None, together=False) -> DeviceBatch:
     """``lo`` / ``hi``: lowest and highest timestamp that can occur; ``host``: pinned address that receives the counts;
-    ``meta``: block of 2 + 2 * hops device words for the counts and the status (default: behind the raw arrays)."""
+    ``meta``: block of 2 + 2 * hops device words for the counts and the status (default: behind the raw arrays);
+    ``together``: one allocation for the results whatever their size (for callers that keep none of them)."""
     roots, root_ts = ops._i64(roots), ops._i64(root_ts)
     n = roots.numel()
     if root_ts.numel() != n:
         raise _C.SglError("build_batch: roots and root_ts differ in length")
     plan = _plan(n, fanouts)
     dev = g.device
-    raw = torch.empty(plan.raw_words + (2 + 2 * len(fanouts) if meta is None else 0), dtype=torch.int64, device=dev)
+    extra = 2 + 2 * len(fanouts) if meta is None else 0
+    if plan.whole:
+        results = raw = torch.empty(plan.words + extra, dtype=torch.int64, device=dev)
+    else:
+        results, raw = None, torch.empty(plan.raw_words + extra, dtype=torch.int64, device=dev)
     if meta is None:
-        meta = raw[plan.raw_words:]
-    if plan.shared:
-        results = torch.empty(plan.words, dtype=torch.int64, device=dev)
+        meta = raw[raw.numel() - extra:]
+    if plan.shared or together:
+        if results is None:
+            results = torch.empty(plan.words, dtype=torch.int64, device=dev)
         at, base = plan.at, results.data_ptr()
     else:
         results = {s: torch.empty(plan.size[s], dtype=torch.int64, device=dev) for s in plan.kept}

@@ -14,6 +14,7 @@ timestamps).  ``cluster`` / ``full`` layers and discrete graphs raise ``NotImple
 of a ``'neg'`` task are drawn from a seeded torch generator (the reference draws from the unseeded global numpy state).
 """
 import ctypes as C
+import threading
 from typing import List, Optional
 
 import numpy as np
@@ -26,6 +27,7 @@ from .batch import _enqueue, _graph_range, _root_range
 
 _PINNED_MOST, _PINNED_TOTAL = 256 << 20, 2 << 30
 _SHARED_MOST = 32 << 20
+_STAGE = threading.local()                # pinned buffer for the roots of a thread's tasks
 
 
 def _pinned_now() -> int:
@@ -98,13 +100,14 @@ class MaterializedMultiLayerBuilder:
             f = lambda xs: torch.cat([_dev_i64(x, self.device) for x in xs])
             return f(node_parts), f(ts_parts), None
         n, total = sum(len(x) for x in parts[:len(node_parts)]), sum(len(x) for x in parts)
-        # (a buffer of this call's own: several threads may build slots with one builder)
-        stage = torch.empty(total, dtype=torch.int64, pin_memory=True)
-        st, at = stage.numpy(), 0
+        # (a buffer of this thread's own: several may build slots with one builder)
+        if getattr(_STAGE, "buf", None) is None or _STAGE.buf.numel() < total:
+            _STAGE.buf = torch.empty(max(2 * total, 1024), dtype=torch.int64, pin_memory=True)
+        st, at = _STAGE.buf.numpy(), 0
         for x in parts:
             st[at:at + len(x)] = x
             at += len(x)
-        d = stage.to(self.device, non_blocking=True)
+        d = _STAGE.buf[:total].to(self.device, non_blocking=True)     # (the slot's end waits for the stream)
         t = parts[len(node_parts)]
         return d[:n], d[n:], (int(t.min()), int(t.max())) if len(t) else None
 
@@ -119,14 +122,15 @@ class MaterializedMultiLayerBuilder:
         nb = 2 + 2 * hops
         meta = torch.empty(nb + ((hops + 1) * (P + 1) if planned else 0), dtype=torch.int64, device=self.device)
         lo, hi = _graph_range(g, *ts_range)
-        db = _enqueue(g, roots, root_ts, fanouts, policy, lo, hi, inclusive, -1, seed, None, None, None, meta[:nb])
+        db = _enqueue(g, roots, root_ts, fanouts, policy, lo, hi, inclusive, -1, seed, None, None, None, meta[:nb], True)
         lists = []                                  # (address of the ids, capacity) of every layer list
         n = c = t = roots.numel()
-        lists.append((db.address(0), c))
+        place = db.addresses()
+        lists.append((place[0], c))
         for l, k in enumerate(fanouts):
             t *= k
             c += t
-            lists.append((db.address(3 + 14 * l + 6), c))
+            lists.append((place[3 + 14 * l + 6], c))
         plans = []
         if planned:
             caps = [max(c * max(P - 1, 1), 1) for _, c in lists]
@@ -157,7 +161,7 @@ class MaterializedMultiLayerBuilder:
                 layers = None
         picks = []                                  # (address, count, bytes per value) in the order of the result
         if layers is None:
-            sec = lambda i, count, size=8: picks.append((db.address(i), count, size))
+            sec = lambda i, count, size=8: picks.append((place[i], count, size))
             sec(0, host[0]); sec(1, host[0]); sec(2, n)
             prev = host[0]
             for l in range(hops):

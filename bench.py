@@ -541,15 +541,17 @@ def sampler_roofline(g, pipes, b_roots, b_ts, dev, peak):
         pipes[0].replay_sample(ptrs[it[0] % NUM_BATCHES])
     ms_alone = _time_ms(alone, pipes[0].stream, 400, warm=20)
     main = torch.cuda.Stream(dev)
-    times = []
+    times, issue = [], []
     for rep in range(30):
         e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
         e0.record(main)
+        t0 = time.perf_counter()
         for p_ in pipes:
             p_.stream.wait_stream(main)
         for r in range(16):
             for j, p_ in enumerate(pipes):
                 p_.replay_sample(ptrs[(rep * 16 * S + r * S + j) % NUM_BATCHES])
+        issue.append((time.perf_counter() - t0) * 1e3 / (16 * S))
         for p_ in pipes:
             main.wait_stream(p_.stream)
         e1.record(main)
@@ -567,7 +569,7 @@ def sampler_roofline(g, pipes, b_roots, b_ts, dev, peak):
                              "frac": alg_big / ms_big / 1e6 / peak},
             "unit": "GB/s", "peak": peak,
             "alone": {"ms_per_batch": ms_alone, "achieved": alg_mean / ms_alone / 1e6, "frac": alg_mean / ms_alone / 1e6 / peak},
-            "in_flight": {"batches": S, "ms_per_batch": ms_fly, "achieved": alg_mean / ms_fly / 1e6,
+            "in_flight": {"batches": S, "ms_per_batch": ms_fly, "host_issue_ms_per_batch": statistics.median(issue), "achieved": alg_mean / ms_fly / 1e6,
                           "frac": alg_mean / ms_fly / 1e6 / peak},
             "note": "4,096 roots per batch is a latency-bound size; the in-flight figure is the aggregate of one batch per stream "
                     "and is bound by the host's launch rate (one copy + one graph launch per batch from one thread)"}
@@ -642,7 +644,7 @@ def main():
 
 def run_single(args, dev, local, out_stream):
     """N = 1: the sampler microbenchmark graph, recent-20 + gather of the sampled edges' feature rows."""
-    from starrygl import ops
+    from starrygl import _C, ops
     from starrygl.graph.pipeline import SampleGatherPipeline
     # ---- set-up (untimed): graph, T-CSR, feature table, batches -------------------------------------------
     src, dst, ts, gen = make_graph(dev, seed=0)
@@ -657,7 +659,9 @@ def run_single(args, dev, local, out_stream):
         e1_.record()
         torch.cuda.synchronize(dev)
         ms_ = e0_.elapsed_time(e1_) / reps
-        alg_ = NUM_EDGES * 56 + (NUM_NODES + 1) * 8 + 6 * 2 * NUM_EDGES * 12
+        # inputs and outputs once, and per radix pass 16 bytes read and written (key, neighbour and edge id)
+        passes = _C.lib().sgl_radix_sort_launches(NUM_EDGES, ops.bits_for(NUM_NODES - 1) + ops.bits_for(TS_MAX - 1)) - 2
+        alg_ = NUM_EDGES * 56 + (NUM_NODES + 1) * 8 + passes * 32 * NUM_EDGES
         print(json.dumps({"tcsr_build_ms": ms_, "edges": NUM_EDGES, "nodes": NUM_NODES, "algorithmic_bytes": alg_,
                           "algorithmic_GBps": alg_ / ms_ / 1e6}), file=out_stream, flush=True)
         return
@@ -728,7 +732,10 @@ def run_single(args, dev, local, out_stream):
         p_.status.check("bench")
 
     # the step is one graph replay, so its kernels cannot be bracketed individually: the dominant kernel is timed in a
-    # second pass over K batches, kernel by kernel on one stream
+    # second pass over K batches, kernel by kernel on one stream -- all enqueued while the stream is held back, so that the
+    # events bracket the kernel and not the host's next call
+    with torch.cuda.stream(pipe.stream):
+        torch.cuda._sleep(40_000_000)
     gev = [(torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)) for _ in range(max(K, 50))]
     for i, ev in enumerate(gev):
         pipe.run_device(b_roots[(W + i) % NUM_BATCHES], b_ts[(W + i) % NUM_BATCHES], 0, ev)

@@ -55,9 +55,9 @@ TS_MAX = 10_000_000
 NUM_BATCHES = 64          # distinct pre-generated batches cycled through the steps
 STREAMS = 6
 REGION_REPEATS = 200      # the K-step timed region is repeated this often; the median is reported
-# DRAM bytes per gathered row measured with ncu on a small case (61.2 MB for 68.2 k rows of 688 bytes);
+# DRAM bytes per gathered row measured with ncu on a small case (61.1 MB for 68.2 k rows of 688 bytes);
 # roofline.traffic scales it by the rows of a full-size launch
-GATHER_TRAFFIC_BYTES_PER_ROW = 897.0
+GATHER_TRAFFIC_BYTES_PER_ROW = 895.0
 
 
 def peaks():

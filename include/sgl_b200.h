@@ -127,6 +127,12 @@ int sgl_sample_layer(const int64_t* indptr, const int64_t* nbr, const int64_t* t
                      int64_t* out_ts, float* out_dt, int64_t* out_dt_i64, int64_t* out_eid, int64_t* out_offsets,
                      int32_t* d_status, void* ws, size_t ws_bytes, void* stream);
 
+/* The uniform policy's draws, exported so that they can be tested on their own: out[i] = draw number `draw` of target
+ * first_target + i, uniform in [0, bounds[i]) (bounds >= 1): Philox4x32-10 of (target, draw, rng_stream) under the key `seed`, the
+ * 64 low bits modulo the bound. */
+int sgl_draws_below(int64_t first_target, int draw, uint32_t rng_stream, uint64_t seed, const uint32_t* bounds, int64_t n,
+                    uint32_t* out, void* stream);
+
 /* sgl_sample_layer / sgl_sample_gather with the rows' fence (sgl_tcsr_fence; NULL = search the rows directly). */
 int sgl_sample_layer_fenced(const int64_t* indptr, const int64_t* nbr, const int64_t* ts, const int64_t* eid,
                             const int64_t* fence, int64_t num_nodes, const int64_t* targets, const int64_t* target_ts,
@@ -649,9 +655,6 @@ int sgl_query_blocks(int n_hops, const int64_t* const* node, const int64_t* cons
                      const int64_t* q_ts, const int64_t* ts_ptr, const int64_t* roots_local, const int64_t* neg, const int64_t* neg_ts,
                      int64_t n_roots, int64_t n_pairs, int64_t n_queries, int64_t* out, void* stream);
 
-/* Small results for the host.  sgl_host_words: a pinned buffer of 512 words that belongs to the calling thread.
- * sgl_wait_word: waits until work on the stream has set *flag (pinned memory) to at_least or more.  sgl_read_back: copies up to 511 words of
- * device memory to the host through that buffer and waits for them. */
 /* Up to 96 device arrays (sizes multiples of 4 bytes) to the host in one copy: packed at the 16-byte aligned offsets at[]
  * of `staging` (device, total bytes) and copied to `host`, or, with host2, the bytes from `split` on to host2; does not
  * wait for the copies. */
@@ -659,6 +662,10 @@ int sgl_export_arrays(int n, const void* const* src, const int64_t* bytes, const
                       int64_t total, void* host2, int64_t split, void* stream);
 /* Device arrays to the host, one copy each; does not wait for the copies. */
 int sgl_copy_arrays(int n, const void* const* src, const int64_t* bytes, void* const* dst, void* stream);
+
+/* Small results for the host.  sgl_host_words: a pinned buffer of 512 words that belongs to the calling thread.
+ * sgl_wait_word: waits until work on the stream has set *flag (pinned memory) to at_least or more.  sgl_read_back: copies up to 511 words of
+ * device memory to the host through that buffer and waits for them. */
 int sgl_host_words(void** out);
 int sgl_wait_word(const int64_t* flag, int64_t at_least, void* stream);
 int sgl_read_back(const void* src, void* dst, size_t bytes, void* stream);

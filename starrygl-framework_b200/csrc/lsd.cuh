@@ -22,8 +22,9 @@ constexpr int kBits = 9;
 constexpr int kRadix = 1 << kBits;
 constexpr int kMaxPasses = 8;
 // Measured (50 M and 4.2 M keys of 44 bits, 256 - 1,024 threads, 8 - 20 keys each, 8 and 9 bits a pass): two CTAs of 512 threads per SM
-// are the best of them; 9 bits take five passes instead of six.  A pass of 50 M keys: 480 us with a 4-byte payload, 500 us with
-// 8 bytes, 2.4 - 3.2 TB/s; the load/store pipe is busy two thirds of the time (ranks, staging), HBM half.
+// are the best of them; 9 bits take five passes instead of six.  A pass of 50 M keys with an 8-byte payload: 481 - 490 us, 3.3 TB/s;
+// the first and the last of a T-CSR build, which read and write four arrays, 597 and 566 us.  The load/store pipe is busy two
+// thirds of the time (ranks, staging), HBM half.
 constexpr int kLsdThreads = 512;
 constexpr int kLsdCtas = 2;
 constexpr int kLsdWarps = kLsdThreads / 32;
@@ -41,7 +42,7 @@ struct Digit {
   __device__ __forceinline__ uint32_t of(uint64_t key) const { return (uint32_t)(key >> shift) & ((1u << bits) - 1u); }
 };
 
-// Digit totals of passes shift0, shift0 + 8, ...: one shared-memory counter table per pass.  A warp whose keys all carry the
+// Digit totals of every pass, each first.bits further up: one shared-memory counter table per pass.  A warp whose keys all carry the
 // same digit (high digits of a hub, ordered input) adds once.
 template <class Items>
 __global__ void __launch_bounds__(kHistThreads)
@@ -107,7 +108,6 @@ struct LsdSmem {
   int ticket;
 };
 
-// where a pass reads its items from: the arrays of the pass before, or (first pass) the producer of the keys
 // Sum of what the tiles before this one hold of digit threadIdx.x; publishes it with the tile's own.
 template <int kWide>
 __device__ __forceinline__ uint64_t look_back(uint64_t* state, int pass, int tile, uint32_t total, unsigned long long limit, unsigned int* gave_up,
@@ -149,6 +149,7 @@ __device__ __forceinline__ uint64_t look_back(uint64_t* state, int pass, int til
   return sum;
 }
 
+// where a pass reads its items from: the arrays of the pass before, or (first pass) the producer of the keys
 template <class V>
 struct ArrayItems {
   const uint64_t* keys;

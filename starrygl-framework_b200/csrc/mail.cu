@@ -136,7 +136,6 @@ struct MailSource {
 // Node ids beyond 32 bits leave no room for the time in the key: sorted by time first, then stably by node.
 struct MailTimes {
   MailSource m;
-  uint32_t* order;
   __device__ __forceinline__ int64_t begin() const { return m.n; }
   __device__ __forceinline__ uint64_t key(int64_t j) const { return m.late_first(j); }
   __device__ __forceinline__ void prepare(int64_t) const {}
@@ -242,7 +241,7 @@ extern "C" int sgl_mail_reduce_counted(const int64_t* ids_a, int64_t n_a, const 
     SGL_CHECK_RC(sort_list(entries, MailSink{out_index, winner, d_num_unique, nullptr, 32}, n, id_bits + 32, sort_ws, sort_bytes, d_status,
                            stream));
   } else {
-    SGL_CHECK_RC(sort_list(MailTimes{entries, order}, OrderSink{order}, n, 32, sort_ws, sort_bytes, d_status, stream));
+    SGL_CHECK_RC(sort_list(MailTimes{entries}, OrderSink{order}, n, 32, sort_ws, sort_bytes, d_status, stream));
     SGL_CHECK_RC(sort_list(MailNodes{entries, order}, MailSink{out_index, winner, d_num_unique, order, 0}, n, id_bits, sort_ws, sort_bytes,
                            d_status, stream));
   }

@@ -7,9 +7,10 @@
 //                        with Philox4x32-10, ranked ascending) are written one OUTPUT ELEMENT per thread -- every lane
 //                        busy, stores coalesced, all loads of a thread independent of each other.
 //
-// Large launches are bound by sectors: 384,000 recent-20 targets take 155 us (180 with 8-ary searches and one element per
-// thread in flight), uniform-10 235 us (300 with a warp drawing for one target after the other); small ones by the chain
-// of dependent loads: 4,096 recent-20 targets 17.4 us (20.5 with an arrival counter to clear and a last-CTA scan).
+// Large launches are bound by sectors: 384,000 recent-20 targets take 140 us (180 with 8-ary searches and one element per
+// thread in flight, 155 before the copy loop was driven from shared memory), uniform-10 217 us (300 with a warp drawing for one
+// target after the other, 235 before the draws were kept in registers); small ones by the chain of dependent loads: 4,096
+// recent-20 targets 15 us as a graph of their own (20.5 with an arrival counter to clear and a last-CTA scan).
 // One fused kernel (offsets by a look-back over the CTAs) was slower from 16,000 targets on: the look-back has to wait for
 // the slowest search before it.
 //
@@ -161,9 +162,10 @@ __device__ __forceinline__ uint64_t draw_below(int64_t target, int d, uint32_t r
   return ((uint64_t)ph.c[0] | ((uint64_t)ph.c[1] << 32)) % bound;
 }
 
-// x mod b, exactly: a quotient estimate by reciprocal is off by at most one (its relative error is below 2^-45, the quotients
-// of the two 32-bit steps below 2^32), which the remainder's sign and size show.  The compiler's 64-bit remainder was a third of
-// the instructions of a launch that draws.
+// x mod b, exactly, by reciprocal estimate and correction (Barrett's method in two 32-bit steps, the reciprocal of a Newton step in
+// double precision): the quotient estimate is off by at most one -- the reciprocal's relative error is below 2^-45, a step's quotient
+// below 2^32 --, which the remainder's sign and size show.  The compiler's 64-bit remainder was a third of the instructions of a
+// launch that draws.
 __device__ __forceinline__ uint32_t remainder_step(uint32_t upper, uint32_t lower, uint32_t b, double db, double inv) {
   const uint64_t y = ((uint64_t)upper << 32) | lower;      // upper < b
   const uint32_t q = __double2uint_rz(fma((double)upper, 4294967296.0, (double)lower) * inv);     // (saturates)
@@ -484,6 +486,13 @@ sample_fill_kernel(const SampleArgs a, int count_ctas) {
   }
 }
 
+__global__ void __launch_bounds__(kCtaThreads)
+draws_below_kernel(int64_t first_target, int draw, uint32_t rng_stream, uint64_t seed, const uint32_t* __restrict__ bounds, int64_t n,
+                   uint32_t* __restrict__ out) {
+  const int64_t i = (int64_t)blockIdx.x * kCtaThreads + threadIdx.x;
+  if (i < n) out[i] = draw_below_u32(first_target + i, draw, rng_stream, seed, bounds[i]);
+}
+
 // number of sampled edges -> pinned host memory, then `seq` behind it; sums: one per count CTA
 __global__ void __launch_bounds__(kCtaThreads)
 export_total_kernel(const int64_t* __restrict__ sums, int count, int64_t* host, int64_t seq) {
@@ -714,6 +723,14 @@ extern "C" int sgl_sample_gather(const int64_t* indptr, const int64_t* nbr, cons
   SGL_CHECK_RC(sgl_gather_rows(feat_table, feat_rows, row_bytes, src_pitch, out_eid, nullptr, 0, n_targets * fanout,
                          out_offsets + n_targets, out_feats, row_bytes, nullptr, nullptr, gather_mode, d_status, stream));
   return scope.submit();
+}
+
+extern "C" int sgl_draws_below(int64_t first_target, int draw, uint32_t rng_stream, uint64_t seed, const uint32_t* bounds, int64_t n,
+                               uint32_t* out, void* stream) {
+  SGL_REQUIRE(n >= 0 && n < ((int64_t)1 << 38) && (n == 0 || (bounds && out)), SGL_ERR_ARG, "draws_below: bad argument");
+  if (n == 0) return SGL_OK;
+  return launch(draws_below_kernel, (unsigned)((n + kCtaThreads - 1) / kCtaThreads), kCtaThreads, 0, (cudaStream_t)stream, first_target, draw,
+                rng_stream, seed, bounds, n, out);
 }
 
 // ---------------------------------------------------------------------------------------------------------------

@@ -46,6 +46,7 @@ _SIGNATURES = {
                                        _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _sz, _vp]),
     "sgl_sample_layer_counted": (_i32, [_vp, _vp, _vp, _vp, _vp, _i64, _vp, _vp, _i64, _vp, _i32, _i32, _i32, _i64, _i32, _u64,
                                          _u32, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _sz, _vp, _i64, _vp]),
+    "sgl_draws_below": (_i32, [_i64, _i32, _u32, _u64, _vp, _i64, _vp, _vp]),
     "sgl_sample_layer_static": (_i32, [_vp, _vp, _vp, _vp, _i64, _vp, _vp, _i64, _i32, _i32, _i32, _i64, _i32, _u64, _u32,
                                        _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp]),
     "sgl_sample_gather": (_i32, [_vp, _vp, _vp, _vp, _i64, _vp, _vp, _i64, _i32, _i32, _i32, _i64, _i32, _u64, _u32,

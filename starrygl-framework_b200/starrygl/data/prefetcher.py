@@ -8,7 +8,7 @@ reference tree; its job -- hide the data path behind the model -- is done here w
 of one mini-batch as ``(roots, query_times)`` int64 tensors (CUDA, or pinned host memory) of at most ``max_roots``
 entries.  Iterating yields :class:`PrefetchedBatch` objects in loader order, already ordered into the consumer's
 current stream; a batch's tensors alias the buffers of its pipeline object and may be read by kernels enqueued on that
-stream until ``depth`` further batches have been requested.
+stream until the next batch is requested, which hands the pipeline object to the batch ``depth`` places on.
 """
 import ctypes as C
 from collections import deque
@@ -114,8 +114,8 @@ class HostToDevicePrefetcher:
         self._seq += 1
         c_n.value, c_seq.value, c_cons.value = n, self._seq, _C.stream_ptr()
         # The call orders the slot's reuse behind everything the consumer has enqueued so far on its stream: the work on the
-        # batch that occupied this slot (handed out ``depth`` batches ago) and the kernels that produced ``roots``.
-        # The batch submitted now is only needed ``depth`` requests later, so this does not stall the consumer.
+        # batch that occupied this slot (handed out just before) and the kernels that produced ``roots``.  The batch submitted
+        # now is only needed ``depth`` requests later, so this does not stall the consumer.
         _C.check(self._fn(*args))
         ready.record(st)
         held.append((ready, (roots, root_ts)))

@@ -106,3 +106,22 @@ def test_set_mailbox_local_with_max_reduce():
     O.mailbox_write(r_mb, r_ts, r_pos, *O.reduce_max_rows(index, rows, ts))
     assert np.array_equal(npy(mb.mailbox), r_mb) and np.array_equal(npy(mb.mailbox_ts), r_ts)
     assert np.array_equal(npy(mb.next_mail_pos), r_pos)
+
+
+@pytest.mark.parametrize("n", [700, 50000])
+def test_reduce_over_more_nodes_than_32_bits_count(n):
+    """Node ids that leave no room for the time in the sort key: sorted by time first, then by node."""
+    from starrygl import ops
+    rng = np.random.default_rng(n)
+    nodes = np.concatenate([rng.integers(0, 2 ** 33, 300), [0, 2 ** 32 - 1, 2 ** 32, 2 ** 33 - 1]])
+    ids = nodes[rng.integers(0, len(nodes), n)]
+    ts = rng.integers(-30, 30, n).astype(np.float32)
+    cut = n // 3
+    st = ops.StatusWord(torch.device("cuda"))
+    index, _, out_ts, pos, d_u = ops.mail_reduce(cu(ids[:cut]), cu(ids[cut:]), cu(ts), 2 ** 33, want_pos=True, status=st)
+    order = np.lexsort((np.arange(n), -ts, ids))
+    first = order[np.unique(ids[order], return_index=True)[1]]
+    u = int(d_u)
+    st.check("mail")
+    assert u == len(first) and np.array_equal(npy(index[:u]), ids[first])
+    assert np.array_equal(npy(pos[:u]), first) and np.array_equal(npy(out_ts[:u]), ts[first])

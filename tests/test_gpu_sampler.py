@@ -255,3 +255,23 @@ def test_counts_of_more_hops_than_the_ring_holds():
         hops.append((q, ops.sample_layer(g, q, torch.full_like(q, 500 + i % 400), 7, "recent")))
     for q, h in hops:
         assert h.total() == int(h.offsets[-1].item())
+
+
+@pytest.mark.parametrize("seed", [0, 2 ** 63 + 12345])
+def test_draws_below_bounds_of_up_to_32_bits(seed):
+    """The remainder by reciprocal is exact: every power of two and its neighbours, bounds next to 2^32 and random ones."""
+    from starrygl import _C
+    edges = {1, 2, 3, 2 ** 32 - 1, 2 ** 32 - 2, 2 ** 32 - 3} | {2 ** k + d for k in range(1, 32) for d in (-1, 0, 1)}
+    rng = np.random.default_rng(seed % 1000)
+    n = 2_000_000
+    bounds = np.exp2(rng.random(n) * 32).astype(np.uint64).clip(1, 2 ** 32 - 1)
+    bounds[:len(edges) * 1000] = np.repeat(np.array(sorted(b for b in edges if b >= 1), np.uint64), 1000)
+    first = 2 ** 32 - 1000                               # target numbers on both sides of 32 bits
+    out = torch.empty(n, dtype=torch.int32, device="cuda")
+    d_b = cu(bounds.astype(np.uint32).view(np.int32))
+    _C.check(_C.lib().sgl_draws_below(first, 7, 3, seed, d_b.data_ptr(), n, out.data_ptr(), _C.stream_ptr()))
+    t = first + np.arange(n, dtype=np.uint64)
+    c = O.philox4x32_10((t & 0xFFFFFFFF, t >> np.uint64(32), np.full(n, 7, np.uint64), np.full(n, 3, np.uint64)),
+                        (seed & 0xFFFFFFFF, seed >> 32))
+    u = c[0] | (c[1] << np.uint64(32))
+    assert np.array_equal(npy(out).view(np.uint32).astype(np.uint64), u % bounds)

@@ -38,13 +38,13 @@ struct Order {
     return pool.of_device(&ev);
   }
   int mark(int i, cudaStream_t s) {
-    if (scope) nodes[i] = scope->mark(s);
-    else SGL_CUDA_CHECK(cudaEventRecord(ev[i], s));
+    if (scope) return scope->mark(s, &nodes[i]);
+    SGL_CUDA_CHECK(cudaEventRecord(ev[i], s));
     return SGL_OK;
   }
   int wait(int i, cudaStream_t s) {
-    if (scope) scope->wait(s, nodes[i]);
-    else SGL_CUDA_CHECK(cudaStreamWaitEvent(s, ev[i], 0));
+    if (scope) return scope->wait(s, nodes[i]);
+    SGL_CUDA_CHECK(cudaStreamWaitEvent(s, ev[i], 0));
     return SGL_OK;
   }
 };

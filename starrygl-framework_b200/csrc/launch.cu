@@ -145,43 +145,52 @@ LaunchScope::Tail& LaunchScope::tail(cudaStream_t s) {
 
 int LaunchScope::add(const void* func, dim3 grid, dim3 block, size_t smem, cudaStream_t on, const void* const* args,
                      const size_t* sizes, int n) {
-  LaunchList& l = t_state.list;
-  if (l.used == l.nodes.size()) l.nodes.emplace_back();
-  LaunchNode& node = l.nodes[l.used];
-  node.func = func;
-  node.grid = grid;
-  node.block = block;
-  node.smem = (unsigned)smem;
-  node.on = on;
-  node.arg_first = (uint32_t)l.arg_at.size();
-  node.arg_count = (uint32_t)n;
-  for (int i = 0; i < n; ++i) {
-    const size_t at = (l.bytes.size() + 15) & ~(size_t)15;
-    l.bytes.resize(at + sizes[i]);
-    memcpy(l.bytes.data() + at, args[i], sizes[i]);
-    l.arg_at.push_back((uint32_t)at);
-  }
-  Tail& t = tail(on);
-  node.deps = t.nodes;
-  t.nodes.assign(1, (int)l.used);
-  ++l.used;
-  return SGL_OK;
+  return no_throw([&] {
+    LaunchList& l = t_state.list;
+    if (l.used == l.nodes.size()) l.nodes.emplace_back();
+    LaunchNode& node = l.nodes[l.used];
+    node.func = func;
+    node.grid = grid;
+    node.block = block;
+    node.smem = (unsigned)smem;
+    node.on = on;
+    node.arg_first = (uint32_t)l.arg_at.size();
+    node.arg_count = (uint32_t)n;
+    for (int i = 0; i < n; ++i) {
+      const size_t at = (l.bytes.size() + 15) & ~(size_t)15;
+      l.bytes.resize(at + sizes[i]);
+      memcpy(l.bytes.data() + at, args[i], sizes[i]);
+      l.arg_at.push_back((uint32_t)at);
+    }
+    Tail& t = tail(on);
+    node.deps = t.nodes;
+    t.nodes.assign(1, (int)l.used);
+    ++l.used;
+    return SGL_OK;
+  });
 }
 
-void LaunchScope::wait(cudaStream_t s, const std::vector<int>& nodes) {
-  Tail& t = tail(s);
-  for (int d : nodes) {
-    bool known = false;
-    for (int k : t.nodes) known = known || k == d;
-    if (!known) t.nodes.push_back(d);
-  }
+int LaunchScope::wait(cudaStream_t s, const std::vector<int>& nodes) {
+  return no_throw([&] {
+    Tail& t = tail(s);
+    for (int d : nodes) {
+      bool known = false;
+      for (int k : t.nodes) known = known || k == d;
+      if (!known) t.nodes.push_back(d);
+    }
+    return SGL_OK;
+  });
 }
 
 int LaunchScope::submit() {
   if (!owner_) return SGL_OK;
   owner_ = false;
+  t_state.open = nullptr;
+  return no_throw([&] { return submit_list(); });
+}
+
+int LaunchScope::submit_list() {
   Thread& t = t_state;
-  t.open = nullptr;
   LaunchList& l = t.list;
   if (l.used == 0) return SGL_OK;
   if (l.used == 1) return one_by_one(main_);

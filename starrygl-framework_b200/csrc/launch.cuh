@@ -16,11 +16,23 @@
 #include <string.h>
 
 #include <atomic>
+#include <new>
 #include <vector>
 
 #include "common.cuh"
 
 namespace sgl {
+
+// Nothing may throw across the library's C functions: what allocates host memory on the way runs in here.
+template <class F>
+int no_throw(F&& f) {
+  try {
+    return f();
+  } catch (const std::bad_alloc&) {
+    set_error("out of host memory");
+    return SGL_ERR_CUDA;
+  }
+}
 
 struct LaunchNode {
   const void* func;
@@ -58,12 +70,24 @@ class LaunchScope {
   // Adds a kernel to the scope that is open on this thread; false when there is none (or it launches one by one).
   static LaunchScope* current();
   int add(const void* func, dim3 grid, dim3 block, size_t smem, cudaStream_t on, const void* const* args, const size_t* sizes, int n);
-  // what is added to stream s after wait(s, m) comes after everything that was on the marked stream at m = mark(...)
-  std::vector<int> mark(cudaStream_t s) { return tail(s).nodes; }
-  void wait(cudaStream_t s, const std::vector<int>& nodes);
+  // what is added to stream s after wait(s, m) comes after everything that was on the marked stream at mark(marked, &m)
+  int mark(cudaStream_t s, std::vector<int>* nodes) {
+    return no_throw([&] {
+      *nodes = tail(s).nodes;
+      return SGL_OK;
+    });
+  }
+  int wait(cudaStream_t s, const std::vector<int>& nodes);
+  // ... after everything that is on the other stream by now
+  int follow(cudaStream_t s, cudaStream_t other) {
+    std::vector<int> nodes;
+    const int rc = mark(other, &nodes);
+    return rc != SGL_OK ? rc : wait(s, nodes);
+  }
   int submit();
 
  private:
+  int submit_list();
   bool owner_;
   cudaStream_t main_;
   struct Tail {

@@ -248,7 +248,7 @@ extern "C" int sgl_mail_reduce_counted(const int64_t* ids_a, int64_t n_a, const 
   if (LaunchScope* in = host_unique ? LaunchScope::current() : nullptr) {
     // the number of nodes is on its way while the rows are put together (a second chain of the graph)
     cudaStream_t side = (cudaStream_t)(uintptr_t)3;
-    in->wait(side, in->mark(stream));
+    SGL_CHECK_RC(in->follow(side, stream));
     SGL_CHECK_RC(launch(export_words_kernel, 1, 32, 0, side, d_num_unique, host_unique, 1, seq));
   }
   const int grid = stream_grid(n, kThreads / 32, 8);

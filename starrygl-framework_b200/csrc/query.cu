@@ -169,7 +169,7 @@ extern "C" int sgl_query_at(const int64_t* indptr, const int64_t* nbr, const int
   // the hops next to the relabels: hop l + 1 needs the raw neighbours of hop l, their relabel comes whenever it comes
   LaunchScope* in = LaunchScope::current();
   cudaStream_t side = in ? (cudaStream_t)(uintptr_t)3 : stream;      // (a second chain of the graph)
-  if (in) in->wait(side, in->mark(stream));
+  if (in) SGL_CHECK_RC(in->follow(side, stream));
   auto relabel = [&](const int64_t* ids, int64_t n, const int64_t* d_ids, int64_t* local, int64_t* d_new) -> int {
     return relabel_nodes(ids, n, d_ids, num_nodes, mapper, mask, epoch, d_next_local, local, new_ids, d_new, meta + 4, d_status, nodes_ws,
                          nodes_b, stream);
@@ -182,7 +182,7 @@ extern "C" int sgl_query_at(const int64_t* indptr, const int64_t* nbr, const int
     SGL_CHECK_RC(sample_layer(indptr, nbr, ts, eid, fence, num_nodes, tgt, tgt_ts, t, d_n, fanout, policy, equal_root_time, allowed_offset,
                               keep_root_time, 0, (uint32_t)l, h.nbr, h.dst, h.ts, h.dt, h.dti, h.eid, h.offs, meta + kMetaHead + l,
                               d_status, sample_ws, sample_b, side));
-    if (in) in->wait(stream, in->mark(side));
+    if (in) SGL_CHECK_RC(in->follow(stream, side));
     const int64_t e = t * fanout;
     SGL_CHECK_RC(relabel(h.nbr, e, meta + kMetaHead + l, h.local, meta + kMetaHead + n_hops + 1 + l));
     tgt = h.nbr;
@@ -190,7 +190,7 @@ extern "C" int sgl_query_at(const int64_t* indptr, const int64_t* nbr, const int
     d_n = meta + kMetaHead + l;
     t = e;
   }
-  if (in) in->wait(stream, in->mark(side));
+  if (in) SGL_CHECK_RC(in->follow(stream, side));
   SGL_CHECK_RC(export_words(meta, host_meta, kMetaHead + 2 * n_hops + 1, stream));
   return scope.submit();
 }

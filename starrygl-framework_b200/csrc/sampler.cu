@@ -543,7 +543,7 @@ static int launch_sample(const SampleArgs& a, cudaStream_t stream, int64_t* host
   if (host_total && in) {
     // on its way while the edges are copied (a second chain of the graph)
     cudaStream_t side = (cudaStream_t)(uintptr_t)3;
-    in->wait(side, in->mark(stream));
+    SGL_CHECK_RC(in->follow(side, stream));
     const bool direct = ctas <= kDirectCtas;
     SGL_CHECK_RC(launch(export_total_kernel, 1, kCtaThreads, 0, side, direct ? a.cta_sums : a.out_offsets + a.n_cap, direct ? (int)ctas : 1,
                         host_total, seq));

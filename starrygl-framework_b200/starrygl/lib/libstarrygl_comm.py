@@ -542,6 +542,8 @@ class CUDAGraph:
         m = self.ev[1].numel()
         if stype not in ("recent", "uniform") or m == 0 or not 0 <= layers <= 8 or fanout < 1:
             return None
+        if not (-2 ** 63 <= t0 < 2 ** 63 and -2 ** 63 <= t1 < 2 ** 63):
+            return None                     # (refused there; the foreign call would take the low 64 bits)
         first, cap = self._window(t0, t1)
         if cap > 1_200_000:                 # above the mini-batch sort's limit
             return None

@@ -359,3 +359,17 @@ def test_large_query_and_what_one_of_its_tensors_holds():
     torch.cuda.synchronize()
     assert torch.cuda.memory_allocated() - before < 4 * 8 * keep
     g.close()
+
+
+def test_window_bounds_beyond_64_bits_are_refused():
+    from starrygl.lib import libstarrygl_comm as L
+    n, src, dst, ts, eid = make_events(m=500)
+    g = L.from_edge_index(n, 1, cu(src), cu(dst), cu(ts), cu(eid))
+    none = torch.empty(0, dtype=torch.int64, device="cuda")
+    for t0, t1 in ((0, 2 ** 63), (-2 ** 63 - 1, 100)):
+        g.submit_query(t0, t1, None, none, none, "recent", 1, 5, -1, False, False, "f")
+        with pytest.raises((RuntimeError, OverflowError, ValueError)):
+            g.get()
+    g.submit_query(-2 ** 63, 2 ** 63 - 1, None, none, none, "recent", 1, 5, -1, False, False, "f")
+    assert g.get().roots.q_eid.numel() == 500
+    g.close()

@@ -37,6 +37,8 @@ class PrefetchedBatch:
         return self
 
     def num_edges(self) -> int:
+        if self.n_roots == 0:             # (its count would race with that of the slot's batch before)
+            return 0
         if self._total is not None:
             addr, words, seq, _ = self._total
             if words[1] < seq:

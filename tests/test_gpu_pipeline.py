@@ -219,3 +219,23 @@ def test_prefetcher_stages_what_the_kernels_cannot_read(world, form):
         src, dst, ts, dt, eid, counts = O.sample_layer(*csr, q, qt, K, O.RECENT)[:6]
         assert b.num_edges() == len(src)
         assert np.array_equal(np.diff(npy(b.offsets)), counts) and np.array_equal(npy(b.eid[:len(src)]), eid)
+
+
+def test_a_batch_without_roots_behind_one_that_is_still_queued(world):
+    from starrygl.data.prefetcher import HostToDevicePrefetcher
+    g, feats, _, batches = world
+    none = torch.empty(0, dtype=torch.int64).pin_memory()
+    q, qt, want = batches[0]
+    loader = [(torch.from_numpy(q).pin_memory(), torch.from_numpy(qt).pin_memory()), (none, none)] * 2
+    for warm in (True, False):
+        pf = HostToDevicePrefetcher(loader, g, feats, K, "recent", B, depth=1)
+        torch.cuda.synchronize()
+        if not warm:
+            torch.cuda._sleep(100_000_000)
+        it = iter(pf)
+        next(it)
+        b = next(it)
+        torch.cuda.synchronize()              # (the first batch's count arrives after the second was submitted)
+        assert b.num_edges() == 0
+        assert next(it).num_edges() == len(want[0])
+        assert next(it).num_edges() == 0

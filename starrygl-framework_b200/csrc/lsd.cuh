@@ -138,7 +138,7 @@ __device__ __forceinline__ uint64_t look_back(uint64_t* state, int pass, int til
       unsigned long long now;
       asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(now));
       if (t0 == 0) t0 = now;
-      if (now - t0 > limit) {
+      if (now - t0 >= limit) {
         dev_flag(d_status, SGL_DEV_TIMEOUT);
         *(volatile unsigned int*)gave_up = 1u;
         break;
@@ -325,7 +325,7 @@ __device__ __forceinline__ uint64_t deliver_prefix(uint64_t* state, int tile, ui
       unsigned long long now;
       asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(now));
       if (t0 == 0) t0 = now;
-      if (__any_sync(0xffffffffu, now - t0 > limit)) {
+      if (__any_sync(0xffffffffu, now - t0 >= limit)) {
         if (lane == 0) dev_flag(d_status, SGL_DEV_TIMEOUT);
         break;
       }

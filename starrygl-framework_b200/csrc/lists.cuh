@@ -18,19 +18,24 @@ struct PairSource {
     n_b = eff_count(n_b, d_n_b);
     return n_a + n_b;
   }
-  __device__ __forceinline__ uint64_t key(int64_t i) const {
-    int64_t id = i < n_a ? a_id[i] : b_id[i - n_a];
-    const int64_t t = i < n_a ? a_ts[i] : b_ts[i - n_a];
+  using Raw = longlong2;
+  __device__ __forceinline__ Raw load(int64_t i) const {
+    const bool a = i < n_a;              // (selects addresses, not values: loads without branches overlap)
+    const int64_t j = a ? i : i - n_a;
+    return {(a ? a_id : b_id)[j], (a ? a_ts : b_ts)[j]};
+  }
+  __device__ __forceinline__ uint64_t key(const Raw& x) const {
+    int64_t id = x.x;
+    const int64_t t = x.y;
     uint64_t dt = (uint64_t)t - (uint64_t)ts_base;
     if (id < 0 || ((uint64_t)id & ~low_mask(id_bits))) { dev_flag(d_status, SGL_DEV_BAD_NODE); id = 0; }
     if (t < ts_base || (dt & ~low_mask(ts_bits))) { dev_flag(d_status, SGL_DEV_BAD_TS); dt = 0; }
     return ts_bits >= 64 ? dt : (((uint64_t)id << ts_bits) | dt);
   }
-  __device__ __forceinline__ void prepare(int64_t) const {}
 };
 
 struct PairSink {
-  static constexpr bool kUnique = true, kPred = true, kAfter = false;
+  static constexpr bool kUnique = true, kAfter = false;
   static constexpr int kLevels = 1;
   int64_t n_a;
   const int64_t* d_n_a;
@@ -76,20 +81,20 @@ struct CscSource {
   const int* gate;                       // optional: 0 = another kernel has done the work
   int32_t* d_status;
   __device__ __forceinline__ int64_t begin() const { return gate && *gate == 0 ? 0 : eff_count(n_cap, d_n); }
-  __device__ __forceinline__ uint64_t key(int64_t e) const {
-    int64_t d = dst[e];
-    if (dst_map) d = dst_map[d];
-    const int64_t t = ts[e];
+  using Raw = longlong2;
+  __device__ __forceinline__ Raw load(int64_t e) const { return {dst_map ? dst_map[dst[e]] : dst[e], ts[e]}; }
+  __device__ __forceinline__ uint64_t key(const Raw& x) const {
+    int64_t d = x.x;
+    const int64_t t = x.y;
     uint64_t dt = (uint64_t)t - (uint64_t)ts_base;
     if (d < 0 || ((uint64_t)d & ~low_mask(dst_bits))) { dev_flag(d_status, SGL_DEV_BAD_NODE); d = 0; }
     if (t < ts_base || (dt & ~low_mask(ts_bits))) { dev_flag(d_status, SGL_DEV_BAD_TS); dt = 0; }
     return ts_bits >= 64 ? dt : (((uint64_t)d << ts_bits) | dt);
   }
-  __device__ __forceinline__ void prepare(int64_t) const {}
 };
 
 struct CscSink {
-  static constexpr bool kUnique = false, kPred = true, kAfter = false;
+  static constexpr bool kUnique = false, kAfter = false;
   int64_t num_dst;
   const int64_t* d_num_dst;
   int ts_bits;
@@ -102,11 +107,13 @@ struct CscSink {
   const int* gate;                       // as in CscSource
   __device__ __forceinline__ void begin() { num_dst = gate && *gate == 0 ? -1 : eff_count(num_dst, d_num_dst); }
   __device__ __forceinline__ int64_t row(uint64_t k) const { return ts_bits >= 64 ? 0 : (int64_t)(k >> ts_bits); }
-  __device__ __forceinline__ void item(int64_t at, uint64_t k, uint32_t p, bool has_prev, uint64_t prev) const {
+  __device__ __forceinline__ void item(int64_t at, uint64_t, uint32_t p) const {
     out_indices[at] = src_local ? src_local[p] : (int64_t)p;
     out_ts[at] = ts[p];
     out_dt[at] = dt[p];
     out_eid[at] = eid[p];
+  }
+  __device__ __forceinline__ void between(int64_t at, uint64_t k, bool has_prev, uint64_t prev) const {
     const int64_t d = row(k);
     for (int64_t v = has_prev ? row(prev) + 1 : 0; v <= d && v <= num_dst; ++v) indptr[v] = at;
   }
@@ -123,19 +130,23 @@ struct NodesSource {
   int id_bits;
   int32_t* d_status;
   __device__ __forceinline__ int64_t begin() const { return eff_count(n_cap, d_n); }
-  __device__ __forceinline__ uint64_t key(int64_t i) const {
+  using Raw = longlong2;                 // id, epoch of the node
+  __device__ __forceinline__ Raw load(int64_t i) const {
     const int64_t g = ids[i];
+    return {g, g >= 0 && g < num_nodes ? mask[g] : 0};
+  }
+  __device__ __forceinline__ uint64_t key(const Raw& x) const {
+    const int64_t g = x.x;
     if (g < 0 || g >= num_nodes) {
       dev_flag(d_status, SGL_DEV_BAD_NODE);
       return 1ull << id_bits;            // invalid and already known ids sort behind every new id
     }
-    return mask[g] != epoch ? (uint64_t)g : 1ull << id_bits;
+    return x.y != epoch ? (uint64_t)g : 1ull << id_bits;
   }
-  __device__ __forceinline__ void prepare(int64_t) const {}
 };
 
 struct NodesSink {
-  static constexpr bool kUnique = true, kPred = true, kAfter = true;
+  static constexpr bool kUnique = true, kAfter = true;
   static constexpr int kLevels = 1;
   const int64_t* ids;
   int64_t num_nodes;
@@ -190,28 +201,34 @@ struct SeedsSource {
     }
     return n;
   }
-  __device__ __forceinline__ uint64_t key(int64_t j) const {
-    const int64_t s = ev_src[j], t = ev_ts[j];
+  struct Raw {
+    int64_t s, t;
+    bool take;
+  };
+  __device__ __forceinline__ Raw load(int64_t j) const {
+    Raw x{ev_src[j], ev_ts[j], true};
+    if (chunk_mask && x.s >= 0 && x.s < num_nodes) {
+      const int64_t c = node_chunk ? node_chunk[x.s] : 0;
+      x.take = c >= 0 && c < num_chunks && chunk_mask[c];
+    }
+    return x;
+  }
+  __device__ __forceinline__ uint64_t key(const Raw& x) const {
+    const int64_t s = x.s, t = x.t;
     const uint64_t dt = (uint64_t)t - (uint64_t)ts_base;
     if (s < 0 || s >= num_nodes) {
       dev_flag(d_status, SGL_DEV_BAD_NODE);
     } else if (t < ts_base || (dt & ~low_mask(ts_bits))) {
       dev_flag(d_status, SGL_DEV_BAD_TS);
     } else {
-      bool take = true;
-      if (chunk_mask) {
-        const int64_t c = node_chunk ? node_chunk[s] : 0;
-        take = c >= 0 && c < num_chunks && chunk_mask[c];
-      }
-      if (take) return ((uint64_t)s << ts_bits) | dt;
+      if (x.take) return ((uint64_t)s << ts_bits) | dt;
     }
     return 1ull << (id_bits + ts_bits);
   }
-  __device__ __forceinline__ void prepare(int64_t) const {}
 };
 
 struct SeedsSink {
-  static constexpr bool kUnique = true, kPred = true, kAfter = true;
+  static constexpr bool kUnique = true, kAfter = true;
   static constexpr int kLevels = 2;
   const int64_t* win;        // as in SeedsSource
   int key_bits, ts_bits;

@@ -66,7 +66,6 @@ lsd_hist_kernel(Items items, Digit first, int passes, unsigned long long* __rest
     for (int u = 0; u < kAhead; ++u) {
       const int64_t i = i0 + u * kHistThreads + threadIdx.x;
       const bool valid = i < n;
-      if (valid) items.prepare(i);
       const unsigned act = __ballot_sync(0xffffffffu, valid);
       if (act == 0) continue;
       for (int p = 0; p < passes; ++p) {
@@ -159,7 +158,6 @@ struct ArrayItems {
   __device__ __forceinline__ int64_t begin() const { return eff_count(n_cap, d_n); }
   __device__ __forceinline__ uint64_t key(int64_t i) const { return keys[i]; }
   __device__ __forceinline__ V val(int64_t i) const { return vals[i]; }
-  __device__ __forceinline__ void prepare(int64_t) const {}
 };
 
 // where a pass writes them: the arrays of the next one, or (last pass, optionally) what the caller makes of sorted items
@@ -176,9 +174,8 @@ template <class Source>
 struct SourceItems {
   Source src;
   __device__ __forceinline__ int64_t begin() { return src.begin(); }
-  __device__ __forceinline__ uint64_t key(int64_t i) const { return src.key(i); }
+  __device__ __forceinline__ uint64_t key(int64_t i) const { return src.key(src.load(i)); }
   __device__ __forceinline__ uint32_t val(int64_t i) const { return (uint32_t)i; }
-  __device__ __forceinline__ void prepare(int64_t i) const { src.prepare(i); }
 };
 
 template <class V, class Items, class Out>
@@ -366,7 +363,10 @@ lsd_deliver_kernel(Sink sink, const uint64_t* __restrict__ keys, const uint32_t*
 #pragma unroll
     for (int c = 0; c < kDeliverItems; ++c) {
       const int64_t i = base + c * kDeliverThreads + tid;
-      if (i < n) sink.item(i, keys[i], pos[i], i > 0, i > 0 ? keys[i - 1] : 0ull);
+      if (i < n) {
+        sink.item(i, keys[i], pos[i]);
+        sink.between(i, keys[i], i > 0, i > 0 ? keys[i - 1] : 0ull);
+      }
     }
     if ((int)blockIdx.x == tiles - 1) sink.finish(n, keys[n - 1], true, 0, 0);
     tilesort::arrive(sink, ctl + 1, tiles);

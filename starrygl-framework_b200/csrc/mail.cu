@@ -121,47 +121,56 @@ struct MailSource {
   int ts_is_i64;
   int32_t* d_status;
   __device__ __forceinline__ int64_t begin() const { return n; }
-  __device__ __forceinline__ uint64_t key(int64_t j) const {
-    int64_t g = j < n_a ? ids_a[j] : ids_b[j - n_a];
+  struct Raw {
+    int64_t g;
+    uint32_t late;
+  };
+  __device__ __forceinline__ Raw load(int64_t j) const { return {j < n_a ? ids_a[j] : ids_b[j - n_a], late_first(j)}; }
+  __device__ __forceinline__ uint64_t key(const Raw& x) const {
+    int64_t g = x.g;
     if (g < 0 || g >= num_nodes) {
       dev_flag(d_status, SGL_DEV_BAD_NODE);
       g = 0;
     }
-    return ((uint64_t)g << 32) | late_first(j);
+    return ((uint64_t)g << 32) | x.late;
   }
   __device__ __forceinline__ uint32_t late_first(int64_t j) const { return ~orderable(ts_at(ts, ts_len, ts_is_i64, j)); }
-  __device__ __forceinline__ void prepare(int64_t) const {}
 };
 
 // Node ids beyond 32 bits leave no room for the time in the key: sorted by time first, then stably by node.
 struct MailTimes {
   MailSource m;
   __device__ __forceinline__ int64_t begin() const { return m.n; }
-  __device__ __forceinline__ uint64_t key(int64_t j) const { return m.late_first(j); }
-  __device__ __forceinline__ void prepare(int64_t) const {}
+  using Raw = uint32_t;
+  __device__ __forceinline__ Raw load(int64_t j) const { return m.late_first(j); }
+  __device__ __forceinline__ uint64_t key(Raw x) const { return x; }
 };
 struct OrderSink {
-  static constexpr bool kUnique = false, kPred = false, kAfter = false;
+  static constexpr bool kUnique = false, kAfter = false;
   uint32_t* order;
   __device__ __forceinline__ void begin() const {}
-  __device__ __forceinline__ void item(int64_t at, uint64_t, uint32_t pos, bool, uint64_t) const { order[at] = pos; }
+  __device__ __forceinline__ void item(int64_t at, uint64_t, uint32_t pos) const { order[at] = pos; }
+  __device__ __forceinline__ void between(int64_t, uint64_t, bool, uint64_t) const {}
   __device__ __forceinline__ void finish(int64_t, uint64_t, bool, int64_t, int64_t) const {}
 };
 struct MailNodes {
   MailSource m;
   const uint32_t* order;
   __device__ __forceinline__ int64_t begin() const { return m.n; }
-  __device__ __forceinline__ uint64_t key(int64_t i) const {
-    const int64_t j = order[i], g = j < m.n_a ? m.ids_a[j] : m.ids_b[j - m.n_a];
+  using Raw = int64_t;
+  __device__ __forceinline__ Raw load(int64_t i) const {
+    const int64_t j = order[i];
+    return j < m.n_a ? m.ids_a[j] : m.ids_b[j - m.n_a];
+  }
+  __device__ __forceinline__ uint64_t key(Raw g) const {
     if (g >= 0 && g < m.num_nodes) return (uint64_t)g;
     dev_flag(m.d_status, SGL_DEV_BAD_NODE);
     return 0;
   }
-  __device__ __forceinline__ void prepare(int64_t) const {}
 };
 
 struct MailSink {
-  static constexpr bool kUnique = true, kPred = true, kAfter = false;
+  static constexpr bool kUnique = true, kAfter = false;
   static constexpr int kLevels = 1;
   int64_t* out_index;
   uint32_t* winner;

@@ -15,22 +15,24 @@ struct RawSource {
   const int64_t* d_n;
   uint64_t mask;        // only the sorted bits take part
   __device__ __forceinline__ int64_t begin() const { return eff_count(n_cap, d_n); }
-  __device__ __forceinline__ void prepare(int64_t) const {}
-  __device__ __forceinline__ uint64_t key(int64_t i) const { return keys[i] & mask; }
+  using Raw = uint64_t;
+  __device__ __forceinline__ Raw load(int64_t i) const { return keys[i]; }
+  __device__ __forceinline__ uint64_t key(Raw x) const { return x & mask; }
 };
 
 struct RawSink {
-  static constexpr bool kUnique = false, kPred = false, kAfter = false;
+  static constexpr bool kUnique = false, kAfter = false;
   __device__ __forceinline__ void begin() const {}
   const uint64_t* keys;
   const uint32_t* vals;  // nullptr: the payload is the input position
   uint64_t* out_keys;
   uint32_t* out_vals;
   uint64_t mask;
-  __device__ __forceinline__ void item(int64_t at, uint64_t key, uint32_t pos, bool, uint64_t) const {
+  __device__ __forceinline__ void item(int64_t at, uint64_t key, uint32_t pos) const {
     out_keys[at] = mask == ~0ull ? key : keys[pos];
     out_vals[at] = vals ? vals[pos] : pos;
   }
+  __device__ __forceinline__ void between(int64_t, uint64_t, bool, uint64_t) const {}
   __device__ __forceinline__ void finish(int64_t, uint64_t, bool, int64_t, int64_t) const {}
 };
 
@@ -42,7 +44,6 @@ struct IotaItems {
   __device__ __forceinline__ int64_t begin() const { return eff_count(n_cap, d_n); }
   __device__ __forceinline__ uint64_t key(int64_t i) const { return keys[i]; }
   __device__ __forceinline__ uint32_t val(int64_t i) const { return (uint32_t)i; }
-  __device__ __forceinline__ void prepare(int64_t) const {}
 };
 
 }  // namespace

@@ -98,9 +98,10 @@ struct EdgeKey {
   const int64_t *key, *ts;
   long long ts_min;
   int ts_bits;
-  __device__ __forceinline__ uint64_t of(int64_t i) const {
-    const uint64_t dt = (uint64_t)ts[i] - (uint64_t)ts_min;
-    return ts_bits >= 64 ? dt : (((uint64_t)key[i] << ts_bits) | dt);
+  __device__ __forceinline__ uint64_t of(int64_t i) const { return make({key[i], ts[i]}); }
+  __device__ __forceinline__ uint64_t make(const longlong2& x) const {
+    const uint64_t dt = (uint64_t)x.y - (uint64_t)ts_min;
+    return ts_bits >= 64 ? dt : (((uint64_t)x.x << ts_bits) | dt);
   }
   __device__ __forceinline__ int64_t node(uint64_t k) const { return ts_bits >= 64 ? 0 : (int64_t)(k >> ts_bits); }
   __device__ __forceinline__ int64_t time(uint64_t k) const {
@@ -117,23 +118,26 @@ __device__ __forceinline__ void start_rows(int64_t* __restrict__ indptr, int64_t
 struct EdgeSource {
   EdgeKey k;
   int64_t m;
+  using Raw = longlong2;
   __device__ __forceinline__ int64_t begin() const { return m; }
-  __device__ __forceinline__ uint64_t key(int64_t i) const { return k.of(i); }
-  __device__ __forceinline__ void prepare(int64_t) const {}
+  __device__ __forceinline__ Raw load(int64_t i) const { return {k.key[i], k.ts[i]}; }
+  __device__ __forceinline__ uint64_t key(const Raw& x) const { return k.make(x); }
 };
 
 struct EdgeSink {
-  static constexpr bool kUnique = false, kPred = true, kAfter = false;
+  static constexpr bool kUnique = false, kAfter = false;
   EdgeKey k;
   const int64_t *nbr, *eid;
   int64_t num_nodes;
   int64_t *indptr, *out_nbr, *out_ts, *out_eid, *out_perm;
   __device__ __forceinline__ void begin() const {}
-  __device__ __forceinline__ void item(int64_t at, uint64_t key, uint32_t p, bool has_prev, uint64_t prev) const {
+  __device__ __forceinline__ void item(int64_t at, uint64_t key, uint32_t p) const {
     out_nbr[at] = nbr[p];
     out_ts[at] = k.time(key);
     out_eid[at] = eid ? eid[p] : (int64_t)p;
     if (out_perm) out_perm[at] = p;
+  }
+  __device__ __forceinline__ void between(int64_t at, uint64_t key, bool has_prev, uint64_t prev) const {
     start_rows(indptr, has_prev ? k.node(prev) : -1, k.node(key), at);
   }
   __device__ __forceinline__ void finish(int64_t m, uint64_t last, bool has_last, int64_t, int64_t) const {
@@ -151,7 +155,6 @@ struct EdgePairs {                    // neighbour and edge id as payload
   __device__ __forceinline__ uint64_t val(int64_t i) const {
     return (uint64_t)(uint32_t)nbr[i] | ((uint64_t)(uint32_t)(eid ? eid[i] : i) << 32);
   }
-  __device__ __forceinline__ void prepare(int64_t) const {}
 };
 
 struct EdgePositions {                // position as payload
@@ -160,7 +163,6 @@ struct EdgePositions {                // position as payload
   __device__ __forceinline__ int64_t begin() const { return m; }
   __device__ __forceinline__ uint64_t key(int64_t i) const { return k.of(i); }
   __device__ __forceinline__ uint32_t val(int64_t i) const { return (uint32_t)i; }
-  __device__ __forceinline__ void prepare(int64_t) const {}
 };
 
 // The last radix pass writes the edges where they belong; the node of every edge stays for the row pointer.

@@ -15,8 +15,13 @@
 // What bounds it: latency.  A list of 40 k - 300 k keys is 0.3 - 2 MB, a microsecond of bandwidth; the chain is two
 // launches, a sample sort and an in-CTA sort.  The tile size is picked ON THE DEVICE from the item count, so that a
 // list spreads over all 148 SMs even when the launch capacity is several times the actual count (multi-hop batches).
-// Measured (44-bit keys): 4,096 keys 14 us, 41,000 20 us, 160,000 29 us, 480,000 61 us; an LSD radix sort with one kernel
-// per 11 key bits took 25, 84, 95 and 140 us: few CTAs with large digit tables, and a dependent kernel per digit.
+// Every instruction here is fetched once or twice per CTA, and that, not memory, was half of the time: loops over the item slots of a
+// thread jump over the slots that the CTA's items do not reach, sums over warps are warp reductions instead of unrolled loads, and
+// splitters are searched by one rolled loop for all items of a thread.  Both kernels together, unique (id, time) pairs of 44 bits:
+// 4,096 pairs 12.3 us (17.9 before), 41,000 17.6 (23.1), 144,000 23.5 (32.6), 300,000 34.2 (50.5); with a power-law share of the ids
+// 14.1 (18.4), 17.8 (22.9), 26.5 (32.2), 43.5 (50.1).  One CTA, 600 / 1,500 pairs: 5.4 / 7.2 us (7.3 / 10.9), power law 8.3 / 11.5
+// (7.4 / 10.6), thirty copies of every pair 9.3 / 11.8 (7.2 / 10.9): cut into bins once or twice before they go by pivots.  An LSD radix sort with one kernel per 11 key bits
+// took 25, 84 and 95 us for 4,096, 41,000 and 160,000: few CTAs with large digit tables, and a dependent kernel per digit.
 #pragma once
 #include "common.cuh"
 #include "launch.cuh"
@@ -29,6 +34,9 @@ constexpr int kMaxCtas = kNumSM;        // tiles, and buckets: one CTA per SM
 constexpr int kThreadBits = 9;
 constexpr int kThreads = 1 << kThreadBits;   // threads of every kernel here; at least kMaxCtas (1,024 were no faster)
 constexpr int kWarps = kThreads / 32;
+// The kernels' registers are bounded as if they had more threads: the whole register file of an SM would keep everything else off it
+// (the CSC of a hop next to the merge of the next list: 11 us, 40 us when it had to wait for the merge's CTAs).
+constexpr int kRegThreads = 640;
 constexpr int kMinTile = 256;
 constexpr int kMaxTile = 8192;
 constexpr int kTileItems = kMaxTile / kThreads;
@@ -70,29 +78,6 @@ __device__ __forceinline__ uint64_t key_of(const Item& x, int pos_bits) {
 template <bool WIDE>
 __device__ __forceinline__ uint32_t pos_of(const Item& x, int pos_bits) {
   return WIDE ? x.p : (uint32_t)(x.k & ((1ull << pos_bits) - 1ull));
-}
-
-// Number of the `cnt` ascending items of v that are not greater than x.  The first step counts against every 2^step-th item,
-// which all lanes read at the same address; only the last few probes differ between lanes (a plain binary search is bound
-// by the bank conflicts of its middle levels).  1 << step = about cnt / 16.
-template <bool WIDE>
-__device__ __forceinline__ int not_above(const View<WIDE>& v, int cnt, int step, const Item& x) {
-  int lo = 0;
-#pragma unroll 4
-  for (int i = (1 << step) - 1; i < cnt; i += 1 << step) lo += less<WIDE>(x, v.get(i)) ? 0 : 1;
-  lo <<= step;
-  int hi = lo + (1 << step) - 1;         // item hi is greater than x, or does not exist
-  if (hi > cnt) hi = cnt;
-  while (lo < hi) {
-    const int mid = (lo + hi) >> 1;
-    if (less<WIDE>(x, v.get(mid))) hi = mid; else lo = mid + 1;
-  }
-  return lo;
-}
-__device__ __forceinline__ int step_for(int cnt) {
-  int s = 0;
-  while ((16 << s) < cnt) ++s;
-  return s;
 }
 
 // one position out of the j-th of 2^sb equal parts of [0, m), m >= 2^sb
@@ -151,9 +136,7 @@ __device__ __forceinline__ void group_sort(const View<WIDE>& v, const View<WIDE>
     int x = warp_inclusive_scan(c, lane);
     if (lane == 31) s_wsum[warp] = x;
     __syncthreads();
-#pragma unroll
-    for (int w = 0; w < (Q + 32) / 32; ++w)
-      if (w < warp) x += s_wsum[w];
+    x += __reduce_add_sync(0xffffffffu, lane < warp && lane < kWarps ? s_wsum[lane] : 0);
     if (tid <= Q) s_start[tid + 1] = x;
     if (tid == 0) s_start[0] = 0;
     __syncthreads();
@@ -195,120 +178,338 @@ __device__ __forceinline__ void rank_sort(const View<WIDE>& v, const View<WIDE>&
   __syncthreads();
 }
 
-// q grows with m so that ordering q pivots and ranking inside groups of m / q cost about the same (measured at 300, 600,
-// 1,600, 2,200 and 7,000 items).
-template <bool WIDE>
-__device__ __forceinline__ void block_sort(const View<WIDE>& v, const View<WIDE>& tmp, uint32_t* aux, uint16_t* grp, int m) {
+// smallest and largest of a warp's words, by halves (64-bit shuffles would be 20 dependent steps)
+__device__ __forceinline__ uint64_t warp_min(uint64_t x) {
+  const uint32_t hi = __reduce_min_sync(0xffffffffu, (uint32_t)(x >> 32));
+  return ((uint64_t)hi << 32) | __reduce_min_sync(0xffffffffu, (uint32_t)(x >> 32) == hi ? (uint32_t)x : ~0u);
+}
+__device__ __forceinline__ uint64_t warp_max(uint64_t x) {
+  const uint32_t hi = __reduce_max_sync(0xffffffffu, (uint32_t)(x >> 32));
+  return ((uint64_t)hi << 32) | __reduce_max_sync(0xffffffffu, (uint32_t)(x >> 32) == hi ? (uint32_t)x : 0u);
+}
+
+// Sort of up to K * kThreads items inside a CTA by counting: the range of the items is cut into 2^b >= m equal bins; while a bin
+// holds more than a few of its c items it is cut again, into 2^b >= c; inside a bin an item's place is the number of smaller
+// ones.  A uniform list is done after one level, a list with a few ids that hold a large part of it after two or three.  One atomic
+// and two loads of shared memory per item and level, and a scan of at most 2 m counters.  Copies of one key stay together until bins
+// are as narrow as positions: where crowded bins are full of them (recent neighbours of the same few nodes), or after kSpreadLevels
+// levels, it gives up and leaves the items as they were; returns whether they are sorted.
+// cnt: scratch of 2 m words, 16-byte aligned, and 16 bytes that may be written behind them; some: 2 m half words.
+constexpr int kSpreadFew = 32, kSpreadLevels = 3;         // (32, 128, 512 items of a bin are left to comparisons at levels 1, 2, 3)
+constexpr int kSpreadCopies = 32;                         // threads that may hold a copy of a crowded bin's first key
+template <bool WIDE, int K>
+__device__ __forceinline__ bool spread_sort(const View<WIDE>& v, uint32_t* cnt, uint16_t* some, int m, int pos_bits) {
+  constexpr int R = K / 2;               // rounds of a scan: four counters per thread and round, 2 m counters
+  static_assert(K % 2 == 0 && 2 * K * kThreads < (1 << 16), "items and bins are counted in 16 bits each");
+  __shared__ uint64_t s_lo[kWarps], s_hi[kWarps];
+  __shared__ uint32_t s_sum[R][kWarps], s_end;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  Item x[K];
+  uint32_t bin[K], in[K];                // bin of the item (upper half: bits of the key below what the bin says), its number in it
+  __syncthreads();
+  uint64_t lo = ~0ull, hi = 0;
+#pragma unroll
+  for (int c = 0; c < K; ++c) {
+    if (c * kThreads >= m) break;
+    const int i = tid + c * kThreads;
+    if (i < m) {
+      x[c] = v.get(i);
+      lo = x[c].k < lo ? x[c].k : lo;
+      hi = x[c].k > hi ? x[c].k : hi;
+    }
+  }
+  lo = warp_min(lo);
+  hi = warp_max(hi);
+  if (lane == 0) {
+    s_lo[warp] = lo;
+    s_hi[warp] = hi;
+  }
+  const int first_bits = m > 1 ? 32 - __clz(m - 1) : 0;
+  int bins = 1 << first_bits;
+  for (int i = tid * 4; i < bins; i += kThreads * 4) *(uint4*)(cnt + i) = make_uint4(0, 0, 0, 0);
+  __syncthreads();
+  lo = warp_min(s_lo[lane & (kWarps - 1)]);
+  hi = warp_max(s_hi[lane & (kWarps - 1)]);
+  {
+    const int bits = 64 - __clzll((long long)(hi - lo)), below = bits > first_bits ? bits - first_bits : 0;
+#pragma unroll
+    for (int c = 0; c < K; ++c) {
+      if (c * kThreads >= m) break;
+      bin[c] = tid + c * kThreads < m ? (uint32_t)((x[c].k - lo) >> below) | (uint32_t)below << 16 : 0u;
+    }
+  }
+  uint32_t few = kSpreadFew;
+  for (int level = 1;; ++level, few *= 4) {
+#pragma unroll
+    for (int c = 0; c < K; ++c) {
+      if (c * kThreads >= m) break;
+      if (tid + c * kThreads < m) in[c] = atomicAdd(&cnt[bin[c] & 0xffffu], 1u);
+    }
+    __syncthreads();
+    // items before every bin (upper half), and bins of the next level before its own (lower half)
+    uint4 own[R];
+    uint32_t upto[R];
+    bool many = false;
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      if (r * kThreads * 4 >= bins) break;
+      const int i = (r * kThreads + tid) * 4;
+      uint4 w = make_uint4(0, 0, 0, 0);
+      if (i < bins) {
+        w = *(const uint4*)(cnt + i);
+        uint32_t* const p = &w.x;
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const uint32_t n = i + u < bins ? p[u] : 0u;
+          many |= n > few;
+          p[u] = (n << 16) | (n > 1 ? 1u << (32 - __clz(n - 1)) : n);
+        }
+      }
+      own[r] = w;
+      upto[r] = warp_inclusive_scan(w.x + w.y + w.z + w.w, lane);
+      if (lane == 31) s_sum[r][warp] = upto[r];
+    }
+    many = __syncthreads_or(many);
+    if (many) {
+      // (the counters are as they were: the starts are written below)
+      if (level == kSpreadLevels) return false;
+#pragma unroll
+      for (int c = 0; c < K; ++c) {
+        if (c * kThreads >= m) break;
+        if (tid + c * kThreads < m && in[c] == 0) some[bin[c] & 0xffffu] = (uint16_t)(tid + c * kThreads);
+      }
+      __syncthreads();
+      bool copy = false;
+#pragma unroll
+      for (int c = 0; c < K; ++c) {
+        if (c * kThreads >= m) break;
+        if (tid + c * kThreads < m && in[c] > 0 && cnt[bin[c] & 0xffffu] > few)
+          copy |= key_of<WIDE>(x[c], pos_bits) == key_of<WIDE>(v.get(some[bin[c] & 0xffffu]), pos_bits);
+      }
+      if (__syncthreads_count(copy) > kSpreadCopies) return false;
+    }
+    uint32_t base = 0;
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      if (r * kThreads * 4 >= bins) break;
+      const uint32_t n = lane < kWarps ? s_sum[r][lane] : 0u, before = base + __reduce_add_sync(0xffffffffu, lane < warp ? n : 0u);
+      base += __reduce_add_sync(0xffffffffu, n);
+      const int i = (r * kThreads + tid) * 4;
+      if (i < bins) {
+        uint4 s;
+        s.x = before + upto[r] - (own[r].x + own[r].y + own[r].z + own[r].w);
+        s.y = s.x + own[r].x;
+        s.z = s.y + own[r].y;
+        s.w = s.z + own[r].z;
+        *(uint4*)(cnt + i) = s;
+      }
+    }
+    if (tid == 0) s_end = base;
+    __syncthreads();
+    const uint32_t end = s_end;
+    if (!many) {
+      uint32_t at[K], e[K];
+#pragma unroll
+      for (int c = 0; c < K; ++c) {
+        if (c * kThreads >= m) break;
+        if (tid + c * kThreads < m) {
+          const int j = (int)(bin[c] & 0xffffu);
+          at[c] = cnt[j] >> 16;
+          e[c] = (j + 1 < bins ? cnt[j + 1] : end) >> 16;
+          v.set(at[c] + in[c], x[c]);
+        }
+      }
+      __syncthreads();
+#pragma unroll
+      for (int c = 0; c < K; ++c) {
+        if (c * kThreads >= m) break;
+        if (tid + c * kThreads < m) {
+          uint32_t to = at[c];
+#pragma unroll 4
+          for (uint32_t j = at[c]; j < e[c]; ++j) to += less<WIDE>(v.get(j), x[c]) ? 1u : 0u;
+          at[c] = to;
+        }
+      }
+      __syncthreads();
+#pragma unroll
+      for (int c = 0; c < K; ++c) {
+        if (c * kThreads >= m) break;
+        if (tid + c * kThreads < m) v.set(at[c], x[c]);
+      }
+      __syncthreads();
+      return true;
+    }
+#pragma unroll
+    for (int c = 0; c < K; ++c) {
+      if (c * kThreads >= m) break;
+      if (tid + c * kThreads < m) {
+        const int j = (int)(bin[c] & 0xffffu), left = (int)(bin[c] >> 16);
+        const uint32_t s = cnt[j], n = ((j + 1 < bins ? cnt[j + 1] : end) >> 16) - (s >> 16);
+        const int want = n > 1 ? 32 - __clz(n - 1) : 0, take = want < left ? want : left;
+        bin[c] = ((s & 0xffffu) + ((uint32_t)((x[c].k - lo) >> (left - take)) & ((1u << take) - 1u))) | (uint32_t)(left - take) << 16;
+      }
+    }
+    bins = (int)(end & 0xffffu);
+    __syncthreads();
+    for (int i = tid * 4; i < bins; i += kThreads * 4) *(uint4*)(cnt + i) = make_uint4(0, 0, 0, 0);
+    __syncthreads();
+  }
+}
+
+// By counting up to MOST * kThreads items (0: not at all), otherwise, or where that gave up, by pivots: q grows with m so that ordering
+// q pivots and ranking inside groups of m / q cost about the same (measured at 300, 600, 1,600, 2,200 and 7,000 items).
+template <bool WIDE, int MOST>
+__device__ __forceinline__ void block_sort(const View<WIDE>& v, const View<WIDE>& tmp, uint32_t* aux, uint16_t* grp, int m, int pos_bits) {
+  if (m < 64) {
+    rank_sort<WIDE>(v, tmp, m);
+    return;
+  }
+  if constexpr (MOST > 0) {
+    if (m <= 4 * kThreads) {
+      if (spread_sort<WIDE, 4>(v, (uint32_t*)tmp.k, (uint16_t*)aux, m, pos_bits)) return;
+    } else if (m <= MOST * kThreads) {
+      if (spread_sort<WIDE, MOST>(v, (uint32_t*)tmp.k, (uint16_t*)aux, m, pos_bits)) return;
+    }
+  }
   if (m >= 3072) group_sort<WIDE, 8>(v, tmp, aux, grp, m);
   else if (m >= 768) group_sort<WIDE, 7>(v, tmp, aux, grp, m);
-  else if (m >= 64) group_sort<WIDE, 5>(v, tmp, aux, grp, m);
-  else rank_sort<WIDE>(v, tmp, m);
+  else group_sort<WIDE, 5>(v, tmp, aux, grp, m);
 }
 static_assert(kMaxItems < (1 << 21), "rank inside a group: 21 bits");
 
 // What a Sink is:
-//   kUnique = false   item(at, key, pos, has_prev, prev_key): the item at global position `at`, and the key before it
+//   kUnique = false   item(at, key, pos): the item at global position `at`
+//                     between(at, key, has_prev, prev_key): `key` is the first at or behind position `at`, `prev_key` the last before
+//                     it; called once per item, not always by the item's own CTA
 //   kUnique = true    item(at, key, pos, head, u, head2, u2): `head` = first item of its group (equal sink.group(key)), `u` =
 //                     number of the group; with kLevels = 2 the same for sink.group2(key), coarser than group.  Items with
 //                     counted(key) = false (sorted behind the others) belong to no group.
-//   kPred             needs the key before a bucket's first item (prev_key, head)
 //   begin()           called once per thread before the rest (loads device-side counts)
 //   finish(n, last_key, has_last, groups, groups2)   once, by all threads of the CTA of the last bucket
 //   kAfter / after()  by one thread after every CTA has delivered its items
-// A Source: begin() loads device-side counts and returns the number of items; key(i); prepare(i) is called for every i in
-// [0, n) before any item is delivered.
+// A Source: begin() loads device-side counts and returns the number of items; key(load(i)) is the key of item i.  load() only reads,
+// so that the loads of several items are in flight together; what is wrong with an item is flagged by key().
 
-// The items of one CTA in sorted order -> the sink.  `base` = global position of the first, `pred_key` = the key before it
-// (when has_pred), `b` / `last` = which bucket this is and whether it is the last one.
+// What a bucket publishes for a sink that numbers groups, in ctl[1 + b] (0: not known yet): whether the item behind it starts a group
+// / a coarser group, and the groups that start in it, its own first item aside (that is for the bucket before to say).
+constexpr unsigned long long kKnown = 1, kNext1 = 2, kNext2 = 4;
+__device__ __forceinline__ unsigned long long groups_of(unsigned long long pub) {      // coarser groups in the upper half
+  return ((pub >> 8) & 0xffffffull) + (pub & kNext1 ? 1ull : 0ull) + ((pub >> 32) << 32) + (pub & kNext2 ? 1ull << 32 : 0ull);
+}
+static_assert(kMaxItems < (1 << 24), "groups of a bucket: 24 bits");
+
+// The items of one CTA in sorted order -> the sink.  `base` = global position of the first; `b` / `last` = which bucket this is and
+// whether it is the last one; `next_key` (not the last): the first key of the bucket behind it.  A bucket but the first begins with
+// its splitter, so only the first can be empty.
 template <class Sink, bool WIDE>
-__device__ __forceinline__ void deliver(const Sink& sink, const View<WIDE>& v, int m, int64_t n, int64_t base, uint64_t pred_key,
-                                        bool has_pred, int pos_bits, int b, bool last, unsigned long long* ctl, int32_t* d_status) {
+__device__ __forceinline__ void deliver(const Sink& sink, const View<WIDE>& v, int m, int64_t n, int64_t base, uint64_t next_key,
+                                        int pos_bits, int b, bool last, unsigned long long* ctl, int32_t* d_status) {
+  auto key_at = [&](int i) { return key_of<WIDE>(v.get(i), pos_bits); };
   if constexpr (!Sink::kUnique) {
     for (int i = threadIdx.x; i < m; i += kThreads) {
       const Item x = v.get(i);
-      const bool hp = i > 0 || has_pred;
-      const uint64_t pk = i > 0 ? key_of<WIDE>(v.get(i - 1), pos_bits) : pred_key;
-      sink.item(base + i, key_of<WIDE>(x, pos_bits), pos_of<WIDE>(x, pos_bits), hp, pk);
+      const uint64_t k = key_of<WIDE>(x, pos_bits);
+      sink.item(base + i, k, pos_of<WIDE>(x, pos_bits));
+      if (i > 0 || b == 0) sink.between(base + i, k, i > 0, i > 0 ? key_at(i - 1) : 0);
     }
-    if (last) sink.finish(n, m > 0 ? key_of<WIDE>(v.get(m - 1), pos_bits) : pred_key, m > 0 || has_pred, 0, 0);
+    if (!last && threadIdx.x == 0) sink.between(base + m, next_key, m > 0, m > 0 ? key_at(m - 1) : 0);
+    if (last) sink.finish(n, m > 0 ? key_at(m - 1) : 0, m > 0, 0, 0);
   } else {
     constexpr bool kTwo = Sink::kLevels == 2;
-    __shared__ unsigned long long s_warp[kWarps];
-    __shared__ unsigned long long s_base;
-    // heads of item i: bit 0 of its group, bit 32 of its coarser group
-    auto heads_of = [&](int i) -> unsigned long long {
-      const uint64_t k = key_of<WIDE>(v.get(i), pos_bits);
+    __shared__ unsigned long long s_warp[kWarps], s_before[kWarps];
+    __shared__ int s_head;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    // groups that start between two neighbours: bit 0, coarser groups: bit 1
+    auto heads = [&](uint64_t p, uint64_t k) -> int {
       if (!sink.counted(k)) return 0;
-      if (i == 0 && !has_pred) return kTwo ? 0x100000001ull : 1ull;
-      const uint64_t p = i > 0 ? key_of<WIDE>(v.get(i - 1), pos_bits) : pred_key;
-      unsigned long long h = sink.group(p) != sink.group(k) ? 1ull : 0ull;
-      if constexpr (kTwo) h |= sink.group2(p) != sink.group2(k) ? 0x100000000ull : 0ull;
+      int h = sink.group(p) != sink.group(k) ? 1 : 0;
+      if constexpr (kTwo) h |= sink.group2(p) != sink.group2(k) ? 2 : 0;
       return h;
     };
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    auto cta_sum = [&](unsigned long long x) {
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
-      __syncthreads();
-      if (lane == 0) s_warp[warp] = x;
-      __syncthreads();
-      x = 0;
-#pragma unroll
-      for (int w = 0; w < kWarps; ++w) x += s_warp[w];
-      return x;
+    auto first_heads = [&](uint64_t k) -> int { return sink.counted(k) ? (kTwo ? 3 : 1) : 0; };
+    // a warp takes consecutive items; their groups are counted, published, and those of the buckets before added up
+    const int span = ((m + kWarps * 32 - 1) / (kWarps * 32)) * 32, from = warp * span, to = from + span < m ? from + span : m;
+    unsigned long long own = 0;
+    for (int i0 = from; i0 < to; i0 += 32) {
+      const int i = i0 + lane, h = i > 0 && i < to ? heads(key_at(i - 1), key_at(i)) : 0;
+      own += (unsigned long long)__popc(__ballot_sync(0xffffffffu, h & 1));
+      if (kTwo) own += (unsigned long long)__popc(__ballot_sync(0xffffffffu, h & 2)) << 32;
+    }
+    if (lane == 0) s_warp[warp] = own;
+    if (threadIdx.x == 0) s_head = b == 0 && m > 0 ? first_heads(key_at(0)) : 0;
+    __syncthreads();
+    // (two counts below 2^32 each, summed apart)
+    auto sum = [](unsigned long long x) -> unsigned long long {
+      const unsigned lower = __reduce_add_sync(0xffffffffu, (unsigned)x);
+      return (unsigned long long)lower | (kTwo ? (unsigned long long)__reduce_add_sync(0xffffffffu, (unsigned)(x >> 32)) << 32 : 0ull);
     };
-    // heads of the bucket -> published; the numbers of the earlier buckets are summed up by one thread each
-    unsigned long long heads = 0, before = 0;
-    for (int i = threadIdx.x; i < m; i += kThreads) heads += heads_of(i);
-    heads = cta_sum(heads);
+    const unsigned long long share = lane < kWarps ? s_warp[lane] : 0;
+    const unsigned long long total = sum(share);
+    unsigned long long off = sum(lane < warp ? share : 0), others = 0;
     if (ctl != nullptr) {
       volatile unsigned long long* pub = ctl + 1;
-      if (threadIdx.x == 0) pub[b] = heads + 1ull;
+      if (threadIdx.x == 0) {
+        const int next = last ? 0 : (m > 0 ? heads(key_at(m - 1), next_key) : first_heads(next_key));
+        const int first = b == 0 ? s_head : 0;       // (nobody before bucket 0 counts its first item)
+        pub[b] = kKnown | (next & 1 ? kNext1 : 0) | (next & 2 ? kNext2 : 0) | (((total & 0xffffffffull) + (first & 1)) << 8) |
+                 ((total >> 32) + (unsigned long long)(first >> 1)) << 32;
+      }
       // lower buckets have taken their ticket before this one: their CTAs are running and wait only for still lower ones
+      unsigned long long before = 0;
       for (int t = threadIdx.x; t < b; t += kThreads) {
         unsigned long long c = pub[t];
-        if (c == 0) {
-          unsigned long long t0, t1;
-          asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t0));
-          do {
-            c = pub[t];
-            asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t1));
-          } while (c == 0 && t1 - t0 < kWaitNs);
-          if (c == 0) {
+        // (the clock is read now and then only: a read takes longer than a poll)
+        unsigned long long t0 = 0;
+        for (unsigned spin = 1; c == 0; ++spin) {
+          c = pub[t];
+          if ((spin & 63u) != 0 || c != 0) continue;
+          unsigned long long now;
+          asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(now));
+          if (t0 == 0) t0 = now;
+          if (now - t0 > kWaitNs) {
             dev_flag(d_status, SGL_DEV_TIMEOUT);
-            c = 1;
+            break;
           }
         }
-        before += c - 1ull;
+        before += groups_of(c);
+        if (t == b - 1) s_head = (c & kNext1 ? 1 : 0) | (c & kNext2 ? 2 : 0);
       }
-      before = cta_sum(before);
+      before = sum(before);
+      if (lane == 0) s_before[warp] = before;
+      __syncthreads();
+      others = sum(lane < kWarps ? s_before[lane] : 0);
+      off += others;
     }
-    if (threadIdx.x == 0) s_base = before;
-    __syncthreads();
-    for (int i0 = 0; i0 < m; i0 += kThreads) {
-      const int i = i0 + threadIdx.x;
-      const unsigned long long h = i < m ? heads_of(i) : 0ull;
-      const unsigned b1 = __ballot_sync(0xffffffffu, (h & 1ull) != 0), b2 = kTwo ? __ballot_sync(0xffffffffu, (h >> 32) != 0) : 0u;
-      if (lane == 0) s_warp[warp] = (unsigned long long)__popc(b1) | ((unsigned long long)__popc(b2) << 32);
-      __syncthreads();
-      unsigned long long off = s_base, tot = 0;
-#pragma unroll
-      for (int w = 0; w < kWarps; ++w) {
-        const unsigned long long c = s_warp[w];
-        if (w < warp) off += c;
-        tot += c;
+    // groups that start before the warp's first item: the bucket's first item is counted with the buckets before (b > 0)
+    const int head0 = s_head;
+    if (b == 0 ? warp > 0 : warp == 0) {
+      const unsigned long long h = (unsigned long long)(head0 & 1) | ((unsigned long long)(head0 >> 1) << 32);
+      if (b == 0) off += h; else off -= h;
+    }
+    for (int i0 = from; i0 < to; i0 += 32) {
+      const int i = i0 + lane;
+      int h = 0;
+      Item x{0, 0};
+      uint64_t k = 0;
+      if (i < to) {
+        x = v.get(i);
+        k = key_of<WIDE>(x, pos_bits);
+        h = i > 0 ? heads(key_at(i - 1), k) : head0;
       }
-      __syncthreads();
-      if (threadIdx.x == 0) s_base += tot;
-      if (i < m) {
-        const Item x = v.get(i);
+      const unsigned b1 = __ballot_sync(0xffffffffu, h & 1), b2 = kTwo ? __ballot_sync(0xffffffffu, h & 2) : 0u;
+      if (i < to) {
         const unsigned upto = (2u << lane) - 1u;
         const int64_t u = (int64_t)(off & 0xffffffffull) + __popc(b1 & upto) - 1, u2 = (int64_t)(off >> 32) + __popc(b2 & upto) - 1;
-        sink.item(base + i, key_of<WIDE>(x, pos_bits), pos_of<WIDE>(x, pos_bits), (h & 1ull) != 0, u, (h >> 32) != 0, u2);
+        sink.item(base + i, k, pos_of<WIDE>(x, pos_bits), h & 1, u, h >> 1, u2);
       }
-      __syncthreads();
+      off += (unsigned long long)__popc(b1) | ((unsigned long long)__popc(b2) << 32);
     }
-    if (last) sink.finish(n, 0, false, (int64_t)((before + heads) & 0xffffffffull), (int64_t)((before + heads) >> 32));
+    if (last) {
+      // all groups: those before the bucket, and its own
+      unsigned long long all = total + others;
+      if (b == 0) all += (unsigned long long)(head0 & 1) | ((unsigned long long)(head0 >> 1) << 32);
+      sink.finish(n, 0, false, (int64_t)(all & 0xffffffffull), (int64_t)(all >> 32));
+    }
   }
 }
 
@@ -329,7 +530,7 @@ __device__ __forceinline__ void arrive(const Sink& sink, unsigned long long* cou
 
 // Tile size for n items on at most `ctas` CTAs: an even share, so that the list spreads over all SMs.
 __host__ __device__ inline int tile_for(int64_t n, int ctas) {
-  const int t = (int)((n + ctas - 1) / ctas);
+  const int t = (int)(((uint32_t)n + (uint32_t)ctas - 1u) / (uint32_t)ctas);       // (lists are below 2^21)
   return t < kMinTile ? kMinTile : (t + 31) & ~31;
 }
 
@@ -338,12 +539,12 @@ struct Scratch {
   uint64_t* tile_k;     // [n] items grouped by bucket inside every tile
   uint32_t* tile_p;     // [n] (WIDE)
   int32_t* start;       // [bucket][tile] where the bucket's piece starts inside the tile; row `tiles` = the tile's end
-  uint64_t* top;        // [bucket][tile] largest key of the piece (0 where it is empty)
+  uint64_t* split;      // [bucket] smallest key of the bucket (of all but the first)
   uint64_t* over_k;     // [2][n] buckets that do not fit shared memory
   uint32_t* over_p;     // [2][n] (WIDE)
   uint32_t* over_a;     // [n]
   uint16_t* over_g;     // [n]
-  unsigned long long* ctl;   // [0] ticket, [1 + b] groups of bucket b plus one (0 = not known yet), [kCtlWords - 1] arrivals
+  unsigned long long* ctl;   // [0] ticket, [1 + b] what bucket b has published, [kCtlWords - 1] arrivals
 };
 
 constexpr int kCtlWords = kMaxCtas + 3;
@@ -351,7 +552,7 @@ constexpr int kMatrix = (kMaxCtas + 1) * kMaxCtas;
 
 inline size_t ws_bytes(int64_t n) {
   if (n < 1) n = 1;
-  return align_up((size_t)n * 8) + align_up((size_t)n * 4) + align_up(kMatrix * 4) + align_up(kMatrix * 8) + align_up((size_t)n * 16) +
+  return align_up((size_t)n * 8) + align_up((size_t)n * 4) + align_up(kMatrix * 4) + align_up(kMaxCtas * 8) + align_up((size_t)n * 16) +
          align_up((size_t)n * 8) + align_up((size_t)n * 4) + align_up((size_t)n * 2) + align_up(kCtlWords * 8);
 }
 
@@ -360,7 +561,7 @@ inline Scratch carve(WsCarver& c, int64_t n) {
   s.tile_k = c.take<uint64_t>(n);
   s.tile_p = c.take<uint32_t>(n);
   s.start = c.take<int32_t>(kMatrix);
-  s.top = c.take<uint64_t>(kMatrix);
+  s.split = c.take<uint64_t>(kMaxCtas);
   s.over_k = c.take<uint64_t>(2 * (size_t)n);
   s.over_p = c.take<uint32_t>(2 * (size_t)n);
   s.over_a = c.take<uint32_t>(n);
@@ -386,58 +587,90 @@ struct Arrays {
   }
 };
 
-template <class Source, bool WIDE, bool TOP>
-__global__ void __launch_bounds__(kThreads)
-ts_part_kernel(Source src, int pos_bits, Scratch sc) {
-  extern __shared__ __align__(16) unsigned char smem_ts[];
+// Tile [first, first + m) of K * kThreads items at most.  What a part costs is largely its instructions, fetched once each: those of
+// item slots that no thread of a mini-batch has are jumped over.
+template <class Source, bool WIDE, int K>
+__device__ __forceinline__ void part_tile(const Source& src, int pos_bits, const Scratch& sc, int64_t n, int64_t first, int m, int tiles,
+                                          const Arrays<WIDE>& sm) {
+  constexpr int kBatch = 4;              // items of a thread whose loads, and searches, run side by side
+  constexpr int kSplit = 256;            // splitters, filled up with largest words
+  static_assert(kMaxCtas <= kSplit && K % kBatch == 0, "eight steps of the search");
   __shared__ int s_cnt[kMaxCtas], s_w[kWarps];
-  __shared__ unsigned long long s_top[kMaxCtas];
-  const int64_t n = src.begin();
-  const int tile = tile_for(n, (int)gridDim.x);
-  const int tiles = (int)((n + tile - 1) / tile);
+  __shared__ uint64_t s_split_k[kSplit];
+  __shared__ uint32_t s_split_p[WIDE ? kSplit : 1];
+  const View<WIDE> split{s_split_k, s_split_p};      // splitter b (b = 1 .. tiles - 1) at split[b - 1]
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  if (blockIdx.x == 0)
-    for (int t = tid; t < kCtlWords; t += kThreads) sc.ctl[t] = 0;
-  const int64_t first = (int64_t)blockIdx.x * tile;
-  if (first >= n) return;
-  const int m = (int)(n - first < tile ? n - first : tile);
-  Item x[kTileItems];
-#pragma unroll
-  for (int r = 0; r < kTileItems; ++r) {
-    const int i = tid + r * kThreads;
-    x[r] = i < m ? make_item<WIDE>(src.key(first + i), (uint32_t)(first + i), pos_bits) : Item{0, 0};
-    if (i < m) src.prepare(first + i);
-  }
-  const Arrays<WIDE> sm(smem_ts, kMaxSamples);
-  const View<WIDE> split = sm.tmp;       // splitter b (b = 1 .. tiles - 1) at split[b - 1]
   const int buckets = tiles;             // one bucket per tile (two smaller ones were slower)
-  if (tiles > 1) {
-    // (more than one tile: n is above (tiles - 1) * 256, the sample is smaller than the list)
-    // Samples: sorting more costs more, fewer leave larger buckets.  Measured with 148 buckets (512, 1,024, 2,048 samples): 60,000
-    // keys 29, 31, 35 us; 144,000 keys 41, 37, 41 us; 300,000 keys (57), 57, 53 us.  Buckets of 3.5 samples are at most about
-    // four times the mean, of 14 about 1.7 times.
-    const int sb = tiles <= 8 ? 8 : (n < 70000 ? 9 : (n < 220000 ? 10 : 11)), s = 1 << sb;
-    for (int j = tid; j < s; j += kThreads) {
-      const int i = sample_at(j, sb, (int)n);
-      sm.v.set(j, make_item<WIDE>(src.key(i), (uint32_t)i, pos_bits));
-    }
-    block_sort<WIDE>(sm.v, sm.tmp, sm.aux, sm.grp, s);
-    for (int b = 1 + tid; b < buckets; b += kThreads) split.set(b - 1, sm.v.get(b * s / buckets));
+  // Samples: sorting more costs more, fewer leave larger buckets.  Measured with 148 buckets (512, 1,024, 2,048 samples): 41,000 pairs
+  // 17, 20, - us; 100,000 19.5, 21.6, -; 144,000 24.4, 23.6, 30; 200,000 -, 26.3, 26.7 - 34; 300,000 -, 41, 34.6.  Buckets of 3.5 samples
+  // are at most about four times the mean, of 14 about 1.7 times.  (With more than one tile the sample is smaller than the list.)
+  const int sb = tiles <= 8 ? 8 : (n < 100000 ? 9 : (n < 220000 ? 10 : 11)), s = tiles > 1 ? 1 << sb : 0;
+  typename Source::Raw sample[kMaxSamples / kThreads];
+#pragma unroll
+  for (int r = 0; r < kMaxSamples / kThreads; ++r) {
+    if (r * kThreads >= s) break;        // (s is at least half the number of threads)
+    sample[r] = src.load(sample_at((tid + r * kThreads) & (s - 1), sb, (int)n));
   }
-  const int step = step_for(buckets - 1);
-  for (int b = tid; b < buckets; b += kThreads) {
-    s_cnt[b] = 0;
-    s_top[b] = 0;
+  Item x[K];
+#pragma unroll
+  for (int r0 = 0; r0 < K; r0 += kBatch) {
+    if (r0 * kThreads >= m) break;
+    typename Source::Raw raw[kBatch];
+#pragma unroll
+    for (int r = 0; r < kBatch; ++r) {
+      if ((r0 + r) * kThreads >= m) break;
+      const int i = tid + (r0 + r) * kThreads;
+      raw[r] = src.load(first + (i < m ? i : m - 1));      // (no branch around a load)
+    }
+#pragma unroll
+    for (int r = 0; r < kBatch; ++r) {
+      if ((r0 + r) * kThreads >= m) break;
+      const int i = tid + (r0 + r) * kThreads;
+      if (i < m) x[r0 + r] = make_item<WIDE>(src.key(raw[r]), (uint32_t)(first + i), pos_bits);
+    }
+  }
+#pragma unroll
+  for (int r = 0; r < kMaxSamples / kThreads; ++r) {
+    if (r * kThreads >= s) break;
+    const int j = tid + r * kThreads;
+    if (j < s) sm.v.set(j, make_item<WIDE>(src.key(sample[r]), (uint32_t)sample_at(j, sb, (int)n), pos_bits));
+  }
+  if (tid < buckets) s_cnt[tid] = 0;
+  if (tiles > 1) {
+    block_sort<WIDE, 0>(sm.v, sm.tmp, sm.aux, sm.grp, s, pos_bits);
+    if (tid < kSplit) {
+      const Item none{~0ull, ~0u};
+      split.set(tid, tid + 1 < buckets ? sm.v.get((int)((uint32_t)((tid + 1) * s) / (uint32_t)buckets)) : none);
+      if (blockIdx.x == 0 && tid + 1 < buckets) sc.split[tid + 1] = key_of<WIDE>(split.get(tid), pos_bits);
+    }
   }
   __syncthreads();
-  int bucket[kTileItems], at[kTileItems];
+  int bucket[K], at[K];
 #pragma unroll
-  for (int r = 0; r < kTileItems; ++r) {
-    bucket[r] = at[r] = 0;
-    if (tid + r * kThreads < m) {
-      bucket[r] = not_above<WIDE>(split, buckets - 1, step, x[r]);
-      at[r] = atomicAdd(&s_cnt[bucket[r]], 1);
-      if (TOP) atomicMax(&s_top[bucket[r]], (unsigned long long)key_of<WIDE>(x[r], pos_bits));
+  for (int r0 = 0; r0 < K; r0 += kBatch) {
+    if (r0 * kThreads >= m) break;
+    int lo[kBatch];
+#pragma unroll
+    for (int r = 0; r < kBatch; ++r) lo[r] = 0;
+    if (tiles > 1) {
+      // number of splitters that are not greater (the words that fill up count where an item is all ones: none of them is a bucket)
+#pragma unroll 1
+      for (int h = kSplit / 2; h >= 1; h >>= 1) {
+#pragma unroll
+        for (int r = 0; r < kBatch; ++r) {
+          if ((r0 + r) * kThreads >= m) break;
+          lo[r] += less<WIDE>(x[r0 + r], split.get(lo[r] + h - 1)) ? 0 : h;
+        }
+      }
+    }
+#pragma unroll
+    for (int r = 0; r < kBatch; ++r) {
+      if ((r0 + r) * kThreads >= m) break;
+      if (tid + (r0 + r) * kThreads < m) {
+        const int bk = lo[r] < buckets ? lo[r] : buckets - 1;
+        bucket[r0 + r] = bk;
+        at[r0 + r] = atomicAdd(&s_cnt[bk], 1);
+      }
     }
   }
   __syncthreads();
@@ -445,129 +678,125 @@ ts_part_kernel(Source src, int pos_bits, Scratch sc) {
   int off = warp_inclusive_scan(c, lane);
   if (lane == 31) s_w[warp] = off;
   __syncthreads();
-  for (int w = 0; w < warp; ++w) off += s_w[w];
-  off -= c;
+  off += __reduce_add_sync(0xffffffffu, lane < warp && lane < kWarps ? s_w[lane] : 0) - c;
   if (tid < buckets) {
     s_cnt[tid] = off;
     sc.start[tid * tiles + blockIdx.x] = off;
-    if (TOP) sc.top[tid * tiles + blockIdx.x] = s_top[tid];
   }
   if (tid == 0) sc.start[buckets * tiles + blockIdx.x] = m;
   __syncthreads();
 #pragma unroll
-  for (int r = 0; r < kTileItems; ++r)
+  for (int r = 0; r < K; ++r) {
+    if (r * kThreads >= m) break;
     if (tid + r * kThreads < m) View<WIDE>{sc.tile_k, sc.tile_p}.set((int)first + s_cnt[bucket[r]] + at[r], x[r]);
+  }
+}
+
+template <class Source, bool WIDE>
+__global__ void __launch_bounds__(kRegThreads)
+ts_part_kernel(Source src, int pos_bits, Scratch sc) {
+  extern __shared__ __align__(16) unsigned char smem_ts[];
+  const int64_t n = src.begin();
+  const int tile = tile_for(n, (int)gridDim.x);
+  const int tiles = (int)(((uint32_t)n + (uint32_t)tile - 1u) / (uint32_t)tile);
+  if (blockIdx.x == 0)
+    for (int t = threadIdx.x; t < kCtlWords; t += kThreads) sc.ctl[t] = 0;
+  const int64_t first = (int64_t)blockIdx.x * tile;
+  if (first >= n) return;
+  const int m = (int)(n - first < tile ? n - first : tile);
+  const Arrays<WIDE> sm(smem_ts, kMaxSamples);
+  if (m <= 4 * kThreads) part_tile<Source, WIDE, 4>(src, pos_bits, sc, n, first, m, tiles, sm);
+  else part_tile<Source, WIDE, kTileItems>(src, pos_bits, sc, n, first, m, tiles, sm);
 }
 
 // cap = items that fit this launch's shared memory
 template <class Source, class Sink, bool WIDE>
-__global__ void __launch_bounds__(kThreads)
+__global__ void __launch_bounds__(kRegThreads)
 ts_bucket_kernel(Source src, Sink sink, int pos_bits, int64_t n_cap, Scratch sc, int cap, int32_t* d_status) {
   extern __shared__ __align__(16) unsigned char smem_ts[];
   __shared__ int s_ticket;
   __shared__ int s_at[kMaxCtas + 1];
   __shared__ int s_from[kMaxCtas];
   __shared__ int s_w[kWarps];
-  __shared__ long long s_sum[kWarps];
-  __shared__ unsigned long long s_top;
-  __shared__ int s_pred;
+  __shared__ int s_sum[kWarps];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  // (every CTA takes a ticket, next to the loads of begin(); those beyond the number of buckets leave)
+  if (tid == 0) s_ticket = Sink::kUnique ? (int)atomicAdd(sc.ctl, 1ull) : (int)blockIdx.x;
   const int64_t n = src.begin();
   sink.begin();
+  __syncthreads();
+  const int b = s_ticket;
   if (n <= 0) {
-    if (blockIdx.x == 0) {
+    if (b == 0) {
       sink.finish(0, 0, false, 0, 0);
       arrive(sink, nullptr, 1);
     }
     return;
   }
   const int tile = tile_for(n, (int)gridDim.x);
-  const int tiles = (int)((n + tile - 1) / tile);
+  const int tiles = (int)(((uint32_t)n + (uint32_t)tile - 1u) / (uint32_t)tile);
   const int buckets = tiles;             // one bucket per tile (two smaller ones were slower)
-  if ((int)blockIdx.x >= buckets) return;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  if (tid == 0) {
-    s_ticket = Sink::kUnique ? (int)atomicAdd(sc.ctl, 1ull) : (int)blockIdx.x;
-    s_top = 0;
-    s_pred = 0;
-  }
-  __syncthreads();
-  const int b = s_ticket;
+  if (b >= buckets) return;
+  const uint64_t next_key = b + 1 < buckets ? sc.split[b + 1] : 0;
   // thread t: the bucket's piece of tile t
-  long long before = 0;
   int lo = 0, len = 0;
   if (tid < tiles) {
     lo = sc.start[b * tiles + tid];
     len = sc.start[(b + 1) * tiles + tid] - lo;
-    before = lo;
-    if (Sink::kPred && b > 0) {
-      // (a bucket after the first holds at least its splitter, so only bucket 0 can be an empty predecessor)
-      const unsigned long long top = sc.top[(b - 1) * tiles + tid];
-      if (lo > sc.start[(b - 1) * tiles + tid]) {
-        s_pred = 1;
-        atomicMax(&s_top, top);
-      }
-    }
   }
   const int off = warp_inclusive_scan(len, lane);
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) before += __shfl_xor_sync(0xffffffffu, before, o);
+  const int before = (int)__reduce_add_sync(0xffffffffu, (unsigned)lo);
   if (lane == 31) s_w[warp] = off;
   if (lane == 0) s_sum[warp] = before;
   __syncthreads();
-  int woff = 0, m = 0;
-  int64_t base = 0;
-#pragma unroll
-  for (int w = 0; w < kWarps; ++w) {
-    if (w < warp) woff += s_w[w];
-    m += s_w[w];
-    base += s_sum[w];
-  }
+  const int share_w = lane < kWarps ? s_w[lane] : 0, woff = __reduce_add_sync(0xffffffffu, lane < warp ? share_w : 0);
+  const int m = __reduce_add_sync(0xffffffffu, share_w);
+  const int64_t base = __reduce_add_sync(0xffffffffu, lane < kWarps ? s_sum[lane] : 0);
   if (tid < tiles) {
     s_at[tid] = woff + off - len;
     s_from[tid] = tid * tile + lo - (woff + off - len);
   }
   if (tid == 0) s_at[tiles] = m;
-  const bool has_pred = s_pred != 0;
-  const uint64_t pred_key = s_top;
   __syncthreads();
   const View<WIDE> from{sc.tile_k, sc.tile_p};
-  // four lanes copy one piece (about seven items at 148 tiles of 1,000)
+  // a few lanes copy one piece, all pieces at once (148 tiles of 1,000: about seven items a piece, two lanes)
+  const int share = tiles > kThreads / 4 ? 1 : (tiles > kThreads / 8 ? 2 : (tiles > kThreads / 16 ? 3 : 4));
   auto collect = [&](const View<WIDE>& v) {
-    for (int a = tid >> 2; a < tiles; a += kThreads / 4) {
+    const int a = tid >> share;
+    if (a < tiles) {
       const int e = s_at[a + 1], f = s_from[a];
-#pragma unroll 4
-      for (int i = s_at[a] + (tid & 3); i < e; i += 4) v.set(i, from.get(f + i));
+#pragma unroll 8
+      for (int i = s_at[a] + (tid & ((1 << share) - 1)); i < e; i += 1 << share) v.set(i, from.get(f + i));
     }
   };
   const bool last = b == buckets - 1;
   if (m <= cap) {
     const Arrays<WIDE> sm(smem_ts, cap);
     collect(sm.v);
-    block_sort<WIDE>(sm.v, sm.tmp, sm.aux, sm.grp, m);
-    deliver<Sink, WIDE>(sink, sm.v, m, n, base, pred_key, has_pred, pos_bits, b, last, sc.ctl, d_status);
+    block_sort<WIDE, 8>(sm.v, sm.tmp, sm.aux, sm.grp, m, pos_bits);
+    deliver<Sink, WIDE>(sink, sm.v, m, n, base, next_key, pos_bits, b, last, sc.ctl, d_status);
   } else {
     // a bucket that shared memory does not hold (unevenly spread sample) is sorted in global memory
     const View<WIDE> v{sc.over_k + base, sc.over_p + base}, tmp{sc.over_k + n_cap + base, sc.over_p + n_cap + base};
     collect(v);
-    block_sort<WIDE>(v, tmp, sc.over_a + base, sc.over_g + base, m);
-    deliver<Sink, WIDE>(sink, v, m, n, base, pred_key, has_pred, pos_bits, b, last, sc.ctl, d_status);
+    block_sort<WIDE, 0>(v, tmp, sc.over_a + base, sc.over_g + base, m, pos_bits);
+    deliver<Sink, WIDE>(sink, v, m, n, base, next_key, pos_bits, b, last, sc.ctl, d_status);
   }
   arrive(sink, sc.ctl + kCtlWords - 1, buckets);
 }
 
 template <class Source, class Sink, bool WIDE>
-__global__ void __launch_bounds__(kThreads)
+__global__ void __launch_bounds__(kRegThreads)
 ts_single_kernel(Source src, Sink sink, int pos_bits, int32_t* d_status) {
   extern __shared__ __align__(16) unsigned char smem_ts[];
   const int m = (int)src.begin();
   sink.begin();
   const Arrays<WIDE> sm(smem_ts, kSingleMax);
   for (int i = threadIdx.x; i < m; i += kThreads) {
-    sm.v.set(i, make_item<WIDE>(src.key(i), (uint32_t)i, pos_bits));
-    src.prepare(i);
+    sm.v.set(i, make_item<WIDE>(src.key(src.load(i)), (uint32_t)i, pos_bits));
   }
-  block_sort<WIDE>(sm.v, sm.tmp, sm.aux, sm.grp, m);
-  deliver<Sink, WIDE>(sink, sm.v, m, m, 0, 0, false, pos_bits, 0, true, nullptr, d_status);
+  block_sort<WIDE, kSingleMax / kThreads>(sm.v, sm.tmp, sm.aux, sm.grp, m, pos_bits);
+  deliver<Sink, WIDE>(sink, sm.v, m, m, 0, 0, pos_bits, 0, true, nullptr, d_status);
   arrive(sink, nullptr, 1);
 }
 
@@ -591,8 +820,8 @@ int launch_as(const Source& src, const Sink& sink, int64_t n_cap, int pos_bits, 
   constexpr int kCapMost = WIDE ? 6912 : 9216;
   const int room = (ctas > 64 ? 8 : 4) * tile, cap = room < kCapMost ? room : kCapMost;
   SGL_CUDA_CHECK(allow_smem((const void*)ts_bucket_kernel<Source, Sink, WIDE>, bucket_done, Arrays<WIDE>::bytes(kCapMost)));
-  SGL_CUDA_CHECK(allow_smem((const void*)ts_part_kernel<Source, WIDE, Sink::kPred>, part_done, Arrays<WIDE>::bytes(kMaxSamples)));
-  SGL_CHECK_RC(launch(ts_part_kernel<Source, WIDE, Sink::kPred>, ctas, kThreads, Arrays<WIDE>::bytes(kMaxSamples), stream,
+  SGL_CUDA_CHECK(allow_smem((const void*)ts_part_kernel<Source, WIDE>, part_done, Arrays<WIDE>::bytes(kMaxSamples)));
+  SGL_CHECK_RC(launch(ts_part_kernel<Source, WIDE>, ctas, kThreads, Arrays<WIDE>::bytes(kMaxSamples), stream,
                       src, pos_bits, sc));
   SGL_CHECK_RC(launch(ts_bucket_kernel<Source, Sink, WIDE>, ctas, kThreads, Arrays<WIDE>::bytes(cap), stream, src, sink,
                       pos_bits, n_cap, sc, cap, d_status));

@@ -45,3 +45,24 @@ def test_equal_keys_of_all_ones_across_buckets(n):
     g = ops.tcsr_build(cu(ids), cu(np.arange(n, dtype=np.int64)), cu(ts), None, 2)
     order = np.lexsort((ts, ids))
     assert np.array_equal(npy(g.indptr), np.searchsorted(ids[order], [0, 1, 2])) and np.array_equal(npy(g.nbr), order)
+
+
+@pytest.mark.parametrize("n", [600, 2048, 2049, 41000, 300000, 610000])
+@pytest.mark.parametrize("copies", [1, 30])
+def test_pairs_of_a_power_law(n, copies):
+    """A few ids hold a large part of the list, all within a short time: bins are cut again, or given up for pivots."""
+    from starrygl import ops
+    rng = np.random.default_rng(n + copies)
+    m = max(n // copies, 1)
+    pick = rng.integers(0, m, n) if copies > 1 else np.arange(n)
+    ids = np.minimum((rng.random(m) + 1e-9) ** -1.1, 799999).astype(np.int64)[pick]
+    ts = rng.integers(5_000_000, 5_000_000 + max(m // 50, 3), m).astype(np.int64)[pick]
+    cut = n // 3
+    st = ops.StatusWord(torch.device("cuda"))
+    out_id, out_ts, inv_a, inv_b, d_n = ops.unique_pairs(cu(ids[:cut]), cu(ts[:cut]), cu(ids[cut:]), cu(ts[cut:]), id_bits=20, ts_bits=24,
+                                                         ts_base=0, status=st)[:5]
+    uniq, inv = np.unique((ids << 24) | ts, return_inverse=True)
+    assert int(d_n) == len(uniq)
+    assert np.array_equal(npy(out_id[:len(uniq)]), uniq >> 24) and np.array_equal(npy(out_ts[:len(uniq)]), uniq & (2 ** 24 - 1))
+    assert np.array_equal(npy(inv_a[:cut]), inv[:cut]) and np.array_equal(npy(inv_b[:n - cut]), inv[cut:])
+    st.check("unique_pairs")

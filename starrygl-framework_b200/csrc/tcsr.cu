@@ -115,11 +115,27 @@ __device__ __forceinline__ void start_rows(int64_t* __restrict__ indptr, int64_t
 }
 
 // ---- up to the mini-batch limit -----------------------------------------------------------------------------------------
+// The sort is enqueued together with the scan and reads the time range where the scan leaves it; node, time and position share a word of
+// 64 bits then, or there is nothing to sort and the host, which learns the same a little later, starts over with what it knows.
+struct ScannedRange {
+  const InputScan* scan;                 // nullptr: the key is complete
+  int id_bits, pos_bits;
+  // false: node ids out of range, or key and position need more than a word
+  __device__ __forceinline__ bool read(EdgeKey& k) const {
+    if (scan == nullptr) return true;
+    const unsigned long long early = scan->early, late = scan->late;
+    k.ts_min = (long long)(~early ^ kSign);
+    k.ts_bits = 64 - __clzll((long long)(late - ~early));
+    return scan->bad_keys == 0 && k.ts_bits + id_bits + pos_bits <= 64;
+  }
+};
+
 struct EdgeSource {
   EdgeKey k;
   int64_t m;
+  ScannedRange range;
   using Raw = longlong2;
-  __device__ __forceinline__ int64_t begin() const { return m; }
+  __device__ __forceinline__ int64_t begin() { return range.read(k) ? m : 0; }
   __device__ __forceinline__ Raw load(int64_t i) const { return {k.key[i], k.ts[i]}; }
   __device__ __forceinline__ uint64_t key(const Raw& x) const { return k.make(x); }
 };
@@ -130,7 +146,8 @@ struct EdgeSink {
   const int64_t *nbr, *eid;
   int64_t num_nodes;
   int64_t *indptr, *out_nbr, *out_ts, *out_eid, *out_perm;
-  __device__ __forceinline__ void begin() const {}
+  ScannedRange range;
+  __device__ __forceinline__ void begin() { range.read(k); }
   __device__ __forceinline__ void item(int64_t at, uint64_t key, uint32_t p) const {
     out_nbr[at] = nbr[p];
     out_ts[at] = k.time(key);
@@ -286,10 +303,25 @@ extern "C" int sgl_tcsr_build_fenced(int64_t num_nodes, int64_t m, const int64_t
   SGL_CHECK_RC(sgl_host_words(&words));
   int64_t* h = (int64_t*)words;
   h[4] = 0;
-  SGL_CUDA_CHECK(cudaMemsetAsync(d_scan, 0, sizeof(InputScan), stream));
-  // (the mini-batch sort gathers through the position anyway: its scan leaves the ids alone)
-  tcsr_scan_kernel<<<stream_grid(m, kScanThreads * 4, 8), kScanThreads, 0, stream>>>(key, nbr, ts, eid, m, num_nodes, small ? 0 : 1, d_scan, h);
-  SGL_LAUNCH_CHECK();
+  const int id_bits = bits_for(num_nodes > 0 ? (uint64_t)(num_nodes - 1) : 0);
+  int pos_bits = 0;
+  while (((m - 1) >> pos_bits) != 0) ++pos_bits;
+  {
+    LaunchScope scope(stream);
+    SGL_CHECK_RC(zero_async(d_scan, sizeof(InputScan), stream));
+    // (the mini-batch sort gathers through the position anyway: its scan leaves the ids alone)
+    SGL_CHECK_RC(launch(tcsr_scan_kernel, stream_grid(m, kScanThreads * 4, 8), kScanThreads, 0, stream, key, nbr, ts, eid, m, num_nodes, small ? 0 : 1,
+                        d_scan, h));
+    // 160,000 edges: 14 of 49 us passed between the scan and a sort that waited for the host to know its result.
+    if (small) {
+      const EdgeKey k{key, ts, 0, 0};
+      const ScannedRange range{d_scan, id_bits, pos_bits};
+      SGL_CHECK_RC(sort_list(EdgeSource{k, m, range}, EdgeSink{k, nbr, eid, num_nodes, indptr, out_nbr, out_ts, out_eid, out_perm, range}, m,
+                             64 - pos_bits, rest, rest_bytes, nullptr, stream));
+      if (out_fence && num_nodes > 0) SGL_CHECK_RC(launch_fence(indptr, out_ts, num_nodes, m, out_fence, stream));
+    }
+    SGL_CHECK_RC(scope.submit());
+  }
   SGL_CHECK_RC(sgl_wait_word(h + 4, 1, stream));
   const long long ts_min = h[0], ts_max = h[1];
   const unsigned long long bad = (unsigned long long)h[2], flags = (unsigned long long)h[3];
@@ -299,7 +331,7 @@ extern "C" int sgl_tcsr_build_fenced(int64_t num_nodes, int64_t m, const int64_t
     h_ts_range[1] = ts_max;
   }
   const int ts_bits = bits_for((uint64_t)ts_max - (uint64_t)ts_min);
-  const int id_bits = bits_for(num_nodes > 0 ? (uint64_t)(num_nodes - 1) : 0);
+  if (small && ts_bits + id_bits + pos_bits <= 64) return SGL_OK;
   const EdgeKey k{key, ts, ts_min, ts_bits};
   const int grid = stream_grid(m, 256 * 4, 8);
   LaunchScope scope(stream);
@@ -321,7 +353,8 @@ extern "C" int sgl_tcsr_build_fenced(int64_t num_nodes, int64_t m, const int64_t
     SGL_CHECK_RC(launch(tcsr_emit_gather_kernel, grid, 256, 0, stream, d_scan, in_alt ? kk_alt : kk, in_alt ? other : perm, 0, k, nbr, eid, m,
                         num_nodes, indptr, out_nbr, out_ts, out_eid, out_perm));
   } else if (small) {
-    SGL_CHECK_RC(sort_list(EdgeSource{k, m}, EdgeSink{k, nbr, eid, num_nodes, indptr, out_nbr, out_ts, out_eid, out_perm}, m,
+    const ScannedRange known{nullptr, 0, 0};
+    SGL_CHECK_RC(sort_list(EdgeSource{k, m, known}, EdgeSink{k, nbr, eid, num_nodes, indptr, out_nbr, out_ts, out_eid, out_perm, known}, m,
                            ts_bits + id_bits, rest, rest_bytes, nullptr, stream));
   } else {
     const int first_bit = flags & kUnordered ? 0 : (ts_bits < 56 ? ts_bits : 56);   // in time order: only the node bits are left

@@ -166,12 +166,13 @@ extern "C" size_t sgl_build_batch_ws_bytes(int64_t n_roots, const int32_t* fanou
          order_ws(n_roots, fanouts, n_hops) + narrow_ws(n_roots, fanouts, n_hops);
 }
 
-extern "C" int sgl_build_batch_at(const int64_t* indptr, const int64_t* nbr, const int64_t* ts, const int64_t* eid, const int64_t* fence,
+// host_early: see sgl_build_batch_staged
+static int build_batch(const int64_t* indptr, const int64_t* nbr, const int64_t* ts, const int64_t* eid, const int64_t* fence,
                                   int64_t num_nodes, const int64_t* roots, const int64_t* root_ts, int64_t n_roots,
                                   const int32_t* fanouts, int n_hops, int policy, int equal_root_time, int64_t allowed_offset,
                                   uint64_t seed, int id_bits, int ts_bits, int64_t ts_base, const int64_t* section_at, int64_t* base,
-                                  int64_t* other_base, int64_t* meta, int32_t* d_status, int64_t* host_meta, void* ws, size_t ws_bytes,
-                                  void* side_stream, void* stream_) {
+                                  int64_t* other_base, int64_t* meta, int32_t* d_status, int64_t* host_meta, int64_t* host_early, void* ws,
+                                  size_t ws_bytes, void* side_stream, void* stream_) {
   SGL_NVTX("sgl_build_batch");
   cudaStream_t stream = (cudaStream_t)stream_;
   SGL_REQUIRE(n_roots >= 0 && n_hops >= 0 && (n_hops == 0 || fanouts), SGL_ERR_ARG, "build_batch: bad size");
@@ -183,6 +184,7 @@ extern "C" int sgl_build_batch_at(const int64_t* indptr, const int64_t* nbr, con
     if (host_meta) SGL_CHECK_RC(export_words(meta, host_meta, 2 + 2 * n_hops, stream));
     return scope.submit();
   };
+  if (host_early) *(volatile int64_t*)(host_early + 1 + 2 * n_hops) = 0;
   if (n_roots == 0) return done();
   SGL_REQUIRE(section_at && roots && root_ts, SGL_ERR_ARG, "build_batch: null array");
   SGL_REQUIRE(ws_bytes >= sgl_build_batch_ws_bytes(n_roots, fanouts, n_hops), SGL_ERR_WORKSPACE, "build_batch: workspace %zu < %zu bytes",
@@ -260,6 +262,12 @@ extern "C" int sgl_build_batch_at(const int64_t* indptr, const int64_t* nbr, con
       order_of = RowOrder::carve(ows, c + e);
       ows += RowOrder::bytes(c + e);
     }
+    if (host_early && l + 1 == n_hops && LaunchScope::current() != nullptr) {
+      // (a third chain of the graph, next to the last merge)
+      cudaStream_t third = (cudaStream_t)(uintptr_t)5;
+      SGL_CHECK_RC(LaunchScope::current()->follow(third, stream));
+      SGL_CHECK_RC(export_words(meta, host_early, 1 + 2 * n_hops, third));
+    }
     rc = unique_pairs(cur_id, cur_ts, c, d_cur, h.nbr, h.ts, e, d_edges, id_bits, ts_bits, ts_base, h.gids, h.gts, nullptr, h.col,
                       l > 0 && narrow_columns(e) ? cols32 : nullptr, d_next, order_of, d_status, lws, lwb, stream);
     if (rc) return rc;
@@ -280,6 +288,27 @@ extern "C" int sgl_build_batch_at(const int64_t* indptr, const int64_t* nbr, con
     c += e;
   }
   return done();
+}
+
+extern "C" int sgl_build_batch_at(const int64_t* indptr, const int64_t* nbr, const int64_t* ts, const int64_t* eid, const int64_t* fence,
+                                  int64_t num_nodes, const int64_t* roots, const int64_t* root_ts, int64_t n_roots,
+                                  const int32_t* fanouts, int n_hops, int policy, int equal_root_time, int64_t allowed_offset,
+                                  uint64_t seed, int id_bits, int ts_bits, int64_t ts_base, const int64_t* section_at, int64_t* base,
+                                  int64_t* other_base, int64_t* meta, int32_t* d_status, int64_t* host_meta, void* ws, size_t ws_bytes,
+                                  void* side_stream, void* stream) {
+  return build_batch(indptr, nbr, ts, eid, fence, num_nodes, roots, root_ts, n_roots, fanouts, n_hops, policy, equal_root_time, allowed_offset, seed,
+                     id_bits, ts_bits, ts_base, section_at, base, other_base, meta, d_status, host_meta, nullptr, ws, ws_bytes, side_stream, stream);
+}
+
+extern "C" int sgl_build_batch_staged(const int64_t* indptr, const int64_t* nbr, const int64_t* ts, const int64_t* eid, const int64_t* fence,
+                                      int64_t num_nodes, const int64_t* roots, const int64_t* root_ts, int64_t n_roots,
+                                      const int32_t* fanouts, int n_hops, int policy, int equal_root_time, int64_t allowed_offset,
+                                      uint64_t seed, int id_bits, int ts_bits, int64_t ts_base, const int64_t* section_at, int64_t* base,
+                                      int64_t* other_base, int64_t* meta, int32_t* d_status, int64_t* host_meta, int64_t* host_early,
+                                      void* ws, size_t ws_bytes, void* side_stream, void* stream) {
+  return build_batch(indptr, nbr, ts, eid, fence, num_nodes, roots, root_ts, n_roots, fanouts, n_hops, policy, equal_root_time, allowed_offset, seed,
+                     id_bits, ts_bits, ts_base, section_at, base, other_base, meta, d_status, host_meta, host_early, ws, ws_bytes, side_stream,
+                     stream);
 }
 
 extern "C" int sgl_build_batch(const int64_t* indptr, const int64_t* nbr, const int64_t* ts, const int64_t* eid, const int64_t* fence,

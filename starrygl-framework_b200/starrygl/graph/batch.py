@@ -155,18 +155,22 @@ class DeviceBatch:
             raise _C.SglError(f"build_batch: device status {bits} ({_C.decode_status(bits)})")
         return self._trim(host)
 
+    def _cut(self):
+        """View of the first ``count`` values of a section, as a function."""
+        if not self._shared:
+            return self._view
+        # (a strided view of the whole costs half of a slice, and its float form one conversion instead of two views each)
+        t, at, cut = self._results, self._plan.start, torch.as_strided
+        f = t.view(torch.float32)
+
+        def v(section, count, floats=False):
+            return cut(f, (count,), (1,), 2 * at[section]) if floats else cut(t, (count,), (1,), at[section])
+        return v
+
     def _trim(self, host):
         self._host = host
-        v, n = self._view, self.n
-        if self._shared:
-            t, at = self._results, self._plan.start
-
-            def v(section, count, floats=False):
-                s = at[section]
-                return t[s:s + (count + 1) // 2].view(torch.float32)[:count] if floats else t[s:s + count]
-        n_list = host[0]
-        out = [{"gids": v(0, n_list), "ts": v(1, n_list), "inv_map": v(2, n)}]
-        prev_n = n_list
+        v = self._cut()
+        out, prev_n = [{"gids": v(0, host[0]), "ts": v(1, host[0]), "inv_map": v(2, self.n)}], host[0]
         for l in range(len(self.fanouts)):
             n_edges, n_next = host[1 + 2 * l], host[2 + 2 * l]
             if n_edges == 0 and not self._any_target_has_edges(l, out):
@@ -177,14 +181,33 @@ class DeviceBatch:
                             "eid": z, "edge_ts": z, "edge_dt": torch.zeros(0, dtype=torch.float32, device=self.g.device),
                             "gids": z, "ts": z})
                 break
-            b = 3 + 14 * l
-            # (the first hop's edges are in CSC order as they were sampled, see sgl_build_batch)
-            ip, ix, ts, dt, ei = (5, 8, 2, 3, 4) if l == 0 else (9, 10, 11, 12, 13)
-            out.append({"indptr": v(b + ip, prev_n + 1), "indices": v(b + ix, n_edges), "eid": v(b + ei, n_edges),
-                        "edge_ts": v(b + ts, n_edges), "edge_dt": v(b + dt, n_edges, True),
-                        "gids": v(b + 6, n_next), "ts": v(b + 7, n_next)})
+            out.append(self._hop(v, l, prev_n, n_edges))
+            out[-1]["gids"], out[-1]["ts"] = v(3 + 14 * l + 6, n_next), v(3 + 14 * l + 7, n_next)
             prev_n = n_next
         return out
+
+    @staticmethod
+    def _hop(v, l, prev_n, n_edges):
+        b = 3 + 14 * l
+        # (the first hop's edges are in CSC order as they were sampled, see sgl_build_batch)
+        ip, ix, ts, dt, ei = (5, 8, 2, 3, 4) if l == 0 else (9, 10, 11, 12, 13)
+        return {"indptr": v(b + ip, prev_n + 1), "indices": v(b + ix, n_edges), "eid": v(b + ei, n_edges), "edge_ts": v(b + ts, n_edges),
+                "edge_dt": v(b + dt, n_edges, True)}
+
+    def _trim_but_last(self, host):
+        """The layers as :meth:`_trim` returns them without the last list, whose length ``host`` does not say yet, and how to cut that;
+        None where a hop has no edges."""
+        hops = len(self.fanouts)
+        if 0 in host[1:2 * hops:2]:
+            return None
+        v = self._cut()
+        out, prev_n = [{"gids": v(0, host[0]), "ts": v(1, host[0]), "inv_map": v(2, self.n)}], host[0]
+        for l in range(hops):
+            out.append(self._hop(v, l, prev_n, host[1 + 2 * l]))
+            if l + 1 < hops:
+                prev_n = host[2 + 2 * l]
+                out[-1]["gids"], out[-1]["ts"] = v(3 + 14 * l + 6, prev_n), v(3 + 14 * l + 7, prev_n)
+        return out, v
 
     def _any_target_has_edges(self, l, out):
         tgt = out[0]["gids"] if l == 0 else self._view(3 + 14 * (l - 1), self._host[1 + 2 * (l - 1)])
@@ -195,8 +218,9 @@ class DeviceBatch:
 
 
 def _enqueue(g, roots, root_ts, fanouts, policy, lo, hi, equal_root_time, allowed_offset, seed, status, side, host=None,
-             meta=None, together=False) -> DeviceBatch:
-    """``lo`` / ``hi``: lowest and highest timestamp that can occur; ``host``: pinned address that receives the counts;
+             meta=None, together=False, early=None) -> DeviceBatch:
+    """``lo`` / ``hi``: lowest and highest timestamp that can occur; ``host``: pinned address that receives the counts, ``early`` one
+    that receives all but the last while the last list is merged;
     ``meta``: block of 2 + 2 * hops device words for the counts and the status (default: behind the raw arrays);
     ``together``: one allocation for the results whatever their size (for callers that keep none of them)."""
     roots, root_ts = ops._i64(roots), ops._i64(root_ts)
@@ -223,12 +247,12 @@ def _enqueue(g, roots, root_ts, fanouts, policy, lo, hi, equal_root_time, allowe
             at[s] = t.data_ptr() // 8
     sp = _C.stream_ptr()
     ws = _C.WORKSPACE.get(plan.ws_bytes, dev, sp)
-    _C.check(_C.lib().sgl_build_batch_at(
+    _C.check(_C.lib().sgl_build_batch_staged(
         g.indptr.data_ptr(), g.nbr.data_ptr(), g.ts.data_ptr(), g.eid.data_ptr(), None if g.fence is None else g.fence.data_ptr(),
         g.num_nodes, _C.ptr(roots), _C.ptr(root_ts), n, plan.fan, len(fanouts),
         _C.POLICY[policy] if isinstance(policy, str) else int(policy), int(bool(equal_root_time)), int(allowed_offset),
         int(seed) & (2 ** 64 - 1), ops.bits_for(g.num_nodes - 1), ops.bits_for(hi - lo), lo, at, base, raw.data_ptr(), meta.data_ptr(),
-        None if status is None else status.ptr(), host, ws.data_ptr(), ws.numel(), None if side is None else side.cuda_stream, sp))
+        None if status is None else status.ptr(), host, early, ws.data_ptr(), ws.numel(), None if side is None else side.cuda_stream, sp))
     return DeviceBatch(g, n, fanouts, plan, results, raw, meta, status)
 
 
@@ -266,6 +290,7 @@ def _root_range(g, root_ts):
     return lo, hi
 
 
+_EARLY = 256                 # place of the early counts among the thread's result words
 _SYNC_OPTIONS = {"ts_range", "equal_root_time", "allowed_offset", "seed"}
 
 
@@ -286,16 +311,27 @@ def build_batch(g, roots, root_ts, fanouts, policy="recent", **kw) -> List[dict]
     last = 1 + 2 * len(fanouts)
     if last + 2 > len(words):
         return build_batch_async(g, roots, root_ts, fanouts, policy, **kw).finish()
+    staged = bool(fanouts) and roots.numel() > 0 and last + 2 <= _EARLY
     db = _enqueue(g, roots, root_ts, fanouts, policy, g.ts_min, g.ts_max, kw.get("equal_root_time", False), kw.get("allowed_offset", -1),
-                  kw.get("seed", 0), None, None, addr)
-    _C.check(_C.lib().sgl_wait_word(addr + 8 * (last + 1), 1, _C.stream_ptr()))
+                  kw.get("seed", 0), None, None, addr, early=addr + 8 * _EARLY if staged else None)
+    wait, sp, laid = _C.lib().sgl_wait_word, _C.stream_ptr(), None
+    if staged:
+        # laid out while the device merges the last list: a fifth of a small batch's time is the making of tensors
+        _C.check(wait(addr + 8 * (_EARLY + last), 1, sp))
+        laid = db._trim_but_last(words[_EARLY:_EARLY + last])
+    _C.check(wait(addr + 8 * (last + 1), 1, sp))
     host, bits = words[:last], words[last] & 0xFFFFFFFF
     if bits & 2:
         g.__dict__["_queried_outside"] = True
         return build_batch(g, roots, root_ts, fanouts, policy, **kw)
     if bits:
         raise _C.SglError(f"build_batch: device status {bits} ({_C.decode_status(bits)})")
-    return db._trim(host)
+    if laid is None:
+        return db._trim(host)
+    out, v = laid
+    b = 3 + 14 * (len(fanouts) - 1)
+    out[-1]["gids"], out[-1]["ts"] = v(b + 6, host[-1]), v(b + 7, host[-1])
+    return out
 
 
 def batch_kernel_launches(num_nodes: int, num_roots: int, fanouts: Sequence[int], ts_span: int) -> int:

@@ -236,9 +236,10 @@ class _Arena:
 
     def cut(self, section, n, floats=False):
         t, s = (self.buf, self._at[section]) if self._at is not None else (self.buf[section], 0)
+        # (a strided view of the whole costs half of a slice)
         if floats:
-            return t[s:s + (n + 1) // 2].view(torch.float32)[:n]
-        return t[s:s + n]
+            return torch.as_strided(t.view(torch.float32), (n,), (1,), 2 * s)
+        return torch.as_strided(t, (n,), (1,), s)
 
     def ptr(self, section):
         return self.buf.data_ptr() + 8 * self._at[section] if self._at is not None else self.buf[section].data_ptr()
@@ -380,9 +381,9 @@ def query_blocks(root, neg_roots, neighbors):
     _C.check(_C.lib().sgl_query_blocks(hops, node, ts, cnt, a.ptr(6), a.ptr(2), a.ptr(1), None if neg is None else neg.data_ptr(),
                                        None if neg is None else neg_ts.data_ptr(),
                                        a.n_roots, a.n_pairs, a.n_queries, out.data_ptr(), _C.stream_ptr()))
-    blocks, at = [], 0
+    blocks, at, cut = [], 0, torch.as_strided
     for d, n in zip(dst, a.edges):
-        blocks.append((d, out[at:at + d + n], out[at + d + n:at + 2 * (d + n)], out[at + 2 * (d + n):at + 2 * (d + n) + n]))
+        blocks.append((d, cut(out, (d + n,), (1,), at), cut(out, (d + n,), (1,), at + d + n), cut(out, (n,), (1,), at + 2 * (d + n))))
         at += 2 * (d + n) + n
     return blocks
 

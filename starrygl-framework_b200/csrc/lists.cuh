@@ -8,6 +8,7 @@ __device__ __forceinline__ uint64_t low_mask(int bits) { return bits >= 64 ? ~0u
 // Producers and consumers of sorted lists: the dedup / relabel operations, fused into the sort's kernels (sort_list in lsd.cuh;
 // pack, sort passes, head scan and emit were 8 - 9 kernels and a memset).
 struct PairSource {
+  static constexpr bool kOnDemand = false;
   const int64_t *a_id, *a_ts, *d_n_a, *b_id, *b_ts, *d_n_b;
   int64_t n_a, n_b;
   int id_bits, ts_bits;
@@ -74,6 +75,7 @@ struct PairSink {
 };
 
 struct CscSource {
+  static constexpr bool kOnDemand = true;
   const int64_t *dst, *dst_map, *ts, *d_n;
   int64_t n_cap;
   int dst_bits, ts_bits;
@@ -123,6 +125,7 @@ struct CscSink {
 };
 
 struct NodesSource {
+  static constexpr bool kOnDemand = false;
   const int64_t *ids, *d_n;
   int64_t n_cap, num_nodes;
   const int64_t* mask;
@@ -184,6 +187,7 @@ struct NodesSink {
 // Events of the window by (source, time); events outside the chosen chunks sort behind.  Groups: (source, time) pairs;
 // coarser groups: sources.
 struct SeedsSource {
+  static constexpr bool kOnDemand = false;
   const int64_t *ev_src, *ev_ts;
   int64_t n;
   const int64_t* win;        // optional: {first event, number of events} on the device; n is the capacity then

@@ -178,7 +178,9 @@ struct SourceItems {
   __device__ __forceinline__ uint32_t val(int64_t i) const { return (uint32_t)i; }
 };
 
-template <class V, class Items, class Out>
+// kLoop: a CTA takes tile after tile instead of one, for sorts that mostly turn out not to be needed (a CTA per tile of 38 M entries that
+// are not there took 8 us a pass, 38 us behind the last merge of a batch; a list that is there is 6 % faster without the loop).
+template <class V, class Items, class Out, bool kLoop>
 __global__ void __launch_bounds__(kLsdThreads, kLsdCtas)
 lsd_pass_kernel(Items items, Digit digit, int pass,
                 const unsigned long long* __restrict__ starts, unsigned int* __restrict__ ticket, uint64_t* state,
@@ -190,121 +192,128 @@ lsd_pass_kernel(Items items, Digit digit, int pass,
   if ((int64_t)blockIdx.x * kTile >= n) return;            // (capacity beyond the count; the others share the tickets)
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   if (tid == 0) sm.ticket = (int)atomicAdd(ticket, 1u);
-  for (int j = tid; j < kLsdWarps * kRadix / 4; j += kLsdThreads) {
-    ((uint4*)&sm.mask[0][0])[j] = make_uint4(0, 0, 0, 0);
-    ((uint4*)&sm.cnt[0][0])[j] = make_uint4(0, 0, 0, 0);
-  }
-  __syncthreads();
-  const int tile = sm.ticket;
-  const int64_t tile_base = (int64_t)tile * kTile;
-  const int tile_n = (int)(n - tile_base < kTile ? n - tile_base : kTile);
-  // a warp owns consecutive keys of the tile, 32 at a time: (warp, round, lane) order = key order
-  const int first = warp * (kItems * 32) + lane;
-  uint64_t k[kItems];
+  do {
+    for (int j = tid; j < kLsdWarps * kRadix / 4; j += kLsdThreads) {
+      ((uint4*)&sm.mask[0][0])[j] = make_uint4(0, 0, 0, 0);
+      ((uint4*)&sm.cnt[0][0])[j] = make_uint4(0, 0, 0, 0);
+    }
+    __syncthreads();
+    const int tile = sm.ticket;
+    const int64_t tile_base = (int64_t)tile * kTile;
+    if (kLoop && tile_base >= n) break;
+    const int tile_n = (int)(n - tile_base < kTile ? n - tile_base : kTile);
+    // a warp owns consecutive keys of the tile, 32 at a time: (warp, round, lane) order = key order
+    const int first = warp * (kItems * 32) + lane;
+    uint64_t k[kItems];
 #pragma unroll
-  for (int c = 0; c < kItems; ++c) {
-    const int j = first + c * 32;
-    k[c] = j < tile_n ? items.key(tile_base + j) : ~0ull;
-  }
-  // stable rank inside the warp: the lanes of a round that share a digit find each other through one word per digit
-  uint16_t rank[kItems];
-  uint32_t *mask = sm.mask[warp], *cnt = sm.cnt[warp];
-  const uint32_t below = (1u << lane) - 1u;
+    for (int c = 0; c < kItems; ++c) {
+      const int j = first + c * 32;
+      k[c] = j < tile_n ? items.key(tile_base + j) : ~0ull;
+    }
+    // stable rank inside the warp: the lanes of a round that share a digit find each other through one word per digit
+    uint16_t rank[kItems];
+    uint32_t *mask = sm.mask[warp], *cnt = sm.cnt[warp];
+    const uint32_t below = (1u << lane) - 1u;
 #pragma unroll
-  for (int c = 0; c < kItems; ++c) {
-    const bool valid = first + c * 32 < tile_n;
-    const uint32_t d = digit.of(k[c]);
-    // through shared memory, or by ballots: one kind of round fills the load/store pipe, the other the integer pipe
-    const bool by_ballot = c % 3 == 0;
-    uint32_t peers;
-    if (by_ballot) {
-      peers = __ballot_sync(0xffffffffu, valid);
+    for (int c = 0; c < kItems; ++c) {
+      const bool valid = first + c * 32 < tile_n;
+      const uint32_t d = digit.of(k[c]);
+      // through shared memory, or by ballots: one kind of round fills the load/store pipe, the other the integer pipe
+      const bool by_ballot = c % 3 == 0;
+      uint32_t peers;
+      if (by_ballot) {
+        peers = __ballot_sync(0xffffffffu, valid);
 #pragma unroll
-      for (int b = 0; b < kBits; ++b) {
-        const uint32_t m = __ballot_sync(0xffffffffu, (d >> b) & 1u);
-        peers &= (d >> b) & 1u ? m : ~m;
+        for (int b = 0; b < kBits; ++b) {
+          const uint32_t m = __ballot_sync(0xffffffffu, (d >> b) & 1u);
+          peers &= (d >> b) & 1u ? m : ~m;
+        }
+      } else {
+        if (valid) atomicOr(&mask[d], 1u << lane);
+        __syncwarp();
+        peers = valid ? mask[d] : 0u;
       }
-    } else {
-      if (valid) atomicOr(&mask[d], 1u << lane);
+      const uint32_t before = valid ? cnt[d] : 0u;
       __syncwarp();
-      peers = valid ? mask[d] : 0u;
+      if (valid && (peers & below) == 0) {   // the lowest lane of the digit
+        if (!by_ballot) mask[d] = 0;
+        cnt[d] = before + __popc(peers);
+      }
+      __syncwarp();
+      rank[c] = (uint16_t)(before + __popc(peers & below));
     }
-    const uint32_t before = valid ? cnt[d] : 0u;
-    __syncwarp();
-    if (valid && (peers & below) == 0) {   // the lowest lane of the digit
-      if (!by_ballot) mask[d] = 0;
-      cnt[d] = before + __popc(peers);
+    __syncthreads();
+    // per digit: counts of the warps -> starts of the warps; the tile's count is published, those of the tiles before added up
+    static_assert(kRadix <= kLsdThreads && kTile < (1 << 16), "a thread per digit, 16-bit places");
+    uint32_t total = 0;
+    if (tid < kRadix) {
+#pragma unroll
+      for (int w = 0; w < kLsdWarps; ++w) total += sm.cnt[w][tid];
+      ((volatile uint64_t*)state)[(size_t)tile * kRadix + tid] = (tile == 0 ? kAll : kOwn) | pass_tag(pass) | total;
     }
-    __syncwarp();
-    rank[c] = (uint16_t)(before + __popc(peers & below));
-  }
-  __syncthreads();
-  // per digit: counts of the warps -> starts of the warps; the tile's count is published, those of the tiles before added up
-  static_assert(kRadix <= kLsdThreads && kTile < (1 << 16), "a thread per digit, 16-bit places");
-  uint32_t total = 0;
-  if (tid < kRadix) {
+    const uint32_t start = cta_exclusive_scan<kLsdThreads, uint32_t>(total, nullptr);
+    if (tid < kRadix) {
+      uint32_t at = start;
 #pragma unroll
-    for (int w = 0; w < kLsdWarps; ++w) total += sm.cnt[w][tid];
-    ((volatile uint64_t*)state)[(size_t)tile * kRadix + tid] = (tile == 0 ? kAll : kOwn) | pass_tag(pass) | total;
-  }
-  const uint32_t start = cta_exclusive_scan<kLsdThreads, uint32_t>(total, nullptr);
-  if (tid < kRadix) {
-    uint32_t at = start;
-#pragma unroll
-    for (int w = 0; w < kLsdWarps; ++w) {
-      const uint32_t c = sm.cnt[w][tid];
-      sm.cnt[w][tid] = at;
-      at += c;
+      for (int w = 0; w < kLsdWarps; ++w) {
+        const uint32_t c = sm.cnt[w][tid];
+        sm.cnt[w][tid] = at;
+        at += c;
+      }
     }
-  }
-  __syncthreads();
+    __syncthreads();
 #pragma unroll
-  for (int c = 0; c < kItems; ++c) {
-    if (first + c * 32 < tile_n) {
-      rank[c] += (uint16_t)cnt[digit.of(k[c])];      // place in the tile
-      sm.keys[rank[c]] = k[c];
+    for (int c = 0; c < kItems; ++c) {
+      if (first + c * 32 < tile_n) {
+        rank[c] += (uint16_t)cnt[digit.of(k[c])];      // place in the tile
+        sm.keys[rank[c]] = k[c];
+      }
     }
-  }
-  if (tid < kRadix) {
-    const uint64_t sum = tile > 0 ? look_back<kLookWide<V>>(state, pass, tile, total, limit, gave_up, d_status) : 0;
-    sm.out[tid] = (uint32_t)(starts[tid] + sum) - start;
-  }
-  __syncthreads();
-  // consecutive threads take consecutive tile positions, i.e. runs of one digit -> consecutive addresses
-  constexpr uint32_t kNone = ~0u;
-  uint32_t g[kItems];
-#pragma unroll
-  for (int c = 0; c < kItems; ++c) {
-    const int j = c * kLsdThreads + tid;
-    g[c] = kNone;
-    if (j < tile_n) {
-      const uint64_t key = sm.keys[j];
-      g[c] = sm.out[digit.of(key)] + j;
-      if (g[c] >= n) g[c] = kNone;       // (only where a look-back gave up)
-      if (g[c] != kNone) out.key(g[c], key);
+    if (tid < kRadix) {
+      const uint64_t sum = tile > 0 ? look_back<kLookWide<V>>(state, pass, tile, total, limit, gave_up, d_status) : 0;
+      sm.out[tid] = (uint32_t)(starts[tid] + sum) - start;
     }
-  }
-  // the payload follows through the same shared memory (loaded late: keys and payload do not fit the registers)
-  V v[kItems];
+    __syncthreads();
+    // (everybody has read the ticket; its tile has published what others wait for)
+    if (kLoop && tid == 0) sm.ticket = (int)atomicAdd(ticket, 1u);
+    // consecutive threads take consecutive tile positions, i.e. runs of one digit -> consecutive addresses
+    constexpr uint32_t kNone = ~0u;
+    uint32_t g[kItems];
 #pragma unroll
-  for (int c = 0; c < kItems; ++c) {
-    const int j = first + c * 32;
-    v[c] = j < tile_n ? items.val(tile_base + j) : (V)0;
-  }
-  __syncthreads();
-  V* vals = (V*)sm.keys;
+    for (int c = 0; c < kItems; ++c) {
+      const int j = c * kLsdThreads + tid;
+      g[c] = kNone;
+      if (j < tile_n) {
+        const uint64_t key = sm.keys[j];
+        g[c] = sm.out[digit.of(key)] + j;
+        if (g[c] >= n) g[c] = kNone;       // (only where a look-back gave up)
+        if (g[c] != kNone) out.key(g[c], key);
+      }
+    }
+    // the payload follows through the same shared memory (loaded late: keys and payload do not fit the registers)
+    V v[kItems];
 #pragma unroll
-  for (int c = 0; c < kItems; ++c)
-    if (first + c * 32 < tile_n) vals[rank[c]] = v[c];
-  __syncthreads();
+    for (int c = 0; c < kItems; ++c) {
+      const int j = first + c * 32;
+      v[c] = j < tile_n ? items.val(tile_base + j) : (V)0;
+    }
+    __syncthreads();
+    V* vals = (V*)sm.keys;
 #pragma unroll
-  for (int c = 0; c < kItems; ++c)
-    if (g[c] != kNone) out.val(g[c], vals[c * kLsdThreads + tid]);
+    for (int c = 0; c < kItems; ++c)
+      if (first + c * 32 < tile_n) vals[rank[c]] = v[c];
+    __syncthreads();
+#pragma unroll
+    for (int c = 0; c < kItems; ++c)
+      if (g[c] != kNone) out.val(g[c], vals[c * kLsdThreads + tid]);
+    if (kLoop) __syncthreads();
+  } while (kLoop);
 }
 
 // ---- delivery of a sorted list to a Sink (see tilesort.cuh) -------------------------------------------------------------
 constexpr int kDeliverThreads = 256;
 constexpr int kDeliverItems = 8;
+constexpr int kDeliverCtas = 4;           // per SM
 constexpr int kDeliverTile = kDeliverThreads * kDeliverItems;
 
 // Sum of what the CTAs before this one (by ticket: they all run already) published; called by one whole warp.
@@ -343,7 +352,7 @@ __device__ __forceinline__ uint64_t deliver_prefix(uint64_t* state, int tile, ui
 
 // ctl[0] ticket, ctl[1] arrivals; state: one word per tile, cleared
 template <class Sink>
-__global__ void __launch_bounds__(kDeliverThreads, 4)
+__global__ void __launch_bounds__(kDeliverThreads, kDeliverCtas)
 lsd_deliver_kernel(Sink sink, const uint64_t* __restrict__ keys, const uint32_t* __restrict__ pos, int64_t n_cap, const int64_t* d_count,
                    unsigned long long* ctl, uint64_t* state, unsigned long long limit, const unsigned int* gave_up, int32_t* d_status) {
   const int64_t n = *gave_up ? 0 : eff_count(n_cap, d_count);     // (a pass that gave up left places unwritten)
@@ -358,18 +367,19 @@ lsd_deliver_kernel(Sink sink, const uint64_t* __restrict__ keys, const uint32_t*
   }
   const int tiles = (int)((n + kDeliverTile - 1) / kDeliverTile);
   if constexpr (!Sink::kUnique) {
-    const int64_t base = (int64_t)blockIdx.x * kDeliverTile;
-    if (base >= n) return;
+    for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+      const int64_t base = (int64_t)tile * kDeliverTile;
 #pragma unroll
-    for (int c = 0; c < kDeliverItems; ++c) {
-      const int64_t i = base + c * kDeliverThreads + tid;
-      if (i < n) {
-        sink.item(i, keys[i], pos[i]);
-        sink.between(i, keys[i], i > 0, i > 0 ? keys[i - 1] : 0ull);
+      for (int c = 0; c < kDeliverItems; ++c) {
+        const int64_t i = base + c * kDeliverThreads + tid;
+        if (i < n) {
+          sink.item(i, keys[i], pos[i]);
+          sink.between(i, keys[i], i > 0, i > 0 ? keys[i - 1] : 0ull);
+        }
       }
+      if (tile == tiles - 1) sink.finish(n, keys[n - 1], true, 0, 0);
+      tilesort::arrive(sink, ctl + 1, tiles);
     }
-    if ((int)blockIdx.x == tiles - 1) sink.finish(n, keys[n - 1], true, 0, 0);
-    tilesort::arrive(sink, ctl + 1, tiles);
   } else {
     constexpr bool kTwo = Sink::kLevels == 2;
     constexpr int kShift = 31;           // two counts share the word: 31 bits each
@@ -377,59 +387,63 @@ lsd_deliver_kernel(Sink sink, const uint64_t* __restrict__ keys, const uint32_t*
     __shared__ uint64_t s_cnt[kDeliverItems * (kDeliverThreads / 32)], s_scan[kDeliverItems * (kDeliverThreads / 32)];
     __shared__ uint64_t s_base;
     if ((int)blockIdx.x >= tiles) return;
-    if (tid == 0) s_ticket = (int)atomicAdd(ctl, 1ull);
-    __syncthreads();
-    const int tile = s_ticket;
-    const int64_t first = (int64_t)tile * kDeliverTile;
-    uint64_t k[kDeliverItems];
-    uint32_t p[kDeliverItems];
-    unsigned h1 = 0, h2 = 0;             // bit c: item c of the thread starts a group / a coarser group
-    unsigned up1[kDeliverItems], up2[kDeliverItems];
+    for (;;) {                           // tile after tile (14 M entries of 42 M at most: 252 us, with a CTA per tile of the capacity 284)
+      if (tid == 0) s_ticket = (int)atomicAdd(ctl, 1ull);
+      __syncthreads();
+      const int tile = s_ticket;
+      if (tile >= tiles) break;
+      const int64_t first = (int64_t)tile * kDeliverTile;
+      uint64_t k[kDeliverItems];
+      uint32_t p[kDeliverItems];
+      unsigned h1 = 0, h2 = 0;             // bit c: item c of the thread starts a group / a coarser group
+      unsigned up1[kDeliverItems], up2[kDeliverItems];
 #pragma unroll
-    for (int c = 0; c < kDeliverItems; ++c) {
-      const int64_t i = first + c * kDeliverThreads + tid;
-      k[c] = i < n ? __ldcs(keys + i) : 0;     // (streamed: the cache is for what the sink scatters)
-      p[c] = i < n ? __ldcs(pos + i) : 0u;
-    }
-#pragma unroll
-    for (int c = 0; c < kDeliverItems; ++c) {
-      const int64_t i = first + c * kDeliverThreads + tid;
-      bool a = false, b = false;
-      if (i < n && sink.counted(k[c])) {
-        const uint64_t q = i > 0 ? keys[i - 1] : 0ull;
-        a = i == 0 || sink.group(q) != sink.group(k[c]);
-        if constexpr (kTwo) b = i == 0 || sink.group2(q) != sink.group2(k[c]);
+      for (int c = 0; c < kDeliverItems; ++c) {
+        const int64_t i = first + c * kDeliverThreads + tid;
+        k[c] = i < n ? __ldcs(keys + i) : 0;     // (streamed: the cache is for what the sink scatters)
+        p[c] = i < n ? __ldcs(pos + i) : 0u;
       }
-      const unsigned ba = __ballot_sync(0xffffffffu, a), bb = kTwo ? __ballot_sync(0xffffffffu, b) : 0u;
-      h1 |= (a ? 1u : 0u) << c;
-      h2 |= (b ? 1u : 0u) << c;
-      const unsigned upto = (2u << lane) - 1u;
-      up1[c] = __popc(ba & upto);
-      up2[c] = __popc(bb & upto);
-      if (lane == 0) s_cnt[c * (kDeliverThreads / 32) + warp] = (uint64_t)__popc(ba) | ((uint64_t)__popc(bb) << kShift);
-    }
-    __syncthreads();
-    constexpr int kCells = kDeliverItems * (kDeliverThreads / 32);
-    const uint64_t mine = tid < kCells ? s_cnt[tid] : 0;
-    uint64_t total;
-    const uint64_t ex = cta_exclusive_scan<kDeliverThreads, uint64_t>(mine, &total);
-    if (tid < kCells) s_scan[tid] = ex;
-    if (warp == 0) {
-      const uint64_t base = deliver_prefix(state, tile, total, lane, limit, d_status);
-      if (lane == 0) s_base = base;
-    }
-    __syncthreads();
-    const uint64_t base = s_base, low = kTwo ? (1ull << kShift) - 1 : ~0ull;
 #pragma unroll
-    for (int c = 0; c < kDeliverItems; ++c) {
-      const int64_t i = first + c * kDeliverThreads + tid;
-      if (i >= n) continue;
-      const uint64_t off = base + s_scan[c * (kDeliverThreads / 32) + warp];
-      const int64_t u = (int64_t)(off & low) + up1[c] - 1, u2 = kTwo ? (int64_t)(off >> kShift) + up2[c] - 1 : 0;
-      sink.item(i, k[c], p[c], (h1 >> c) & 1u, u, (h2 >> c) & 1u, u2);
+      for (int c = 0; c < kDeliverItems; ++c) {
+        const int64_t i = first + c * kDeliverThreads + tid;
+        bool a = false, b = false;
+        if (i < n && sink.counted(k[c])) {
+          const uint64_t q = i > 0 ? keys[i - 1] : 0ull;
+          a = i == 0 || sink.group(q) != sink.group(k[c]);
+          if constexpr (kTwo) b = i == 0 || sink.group2(q) != sink.group2(k[c]);
+        }
+        const unsigned ba = __ballot_sync(0xffffffffu, a), bb = kTwo ? __ballot_sync(0xffffffffu, b) : 0u;
+        h1 |= (a ? 1u : 0u) << c;
+        h2 |= (b ? 1u : 0u) << c;
+        const unsigned upto = (2u << lane) - 1u;
+        up1[c] = __popc(ba & upto);
+        up2[c] = __popc(bb & upto);
+        if (lane == 0) s_cnt[c * (kDeliverThreads / 32) + warp] = (uint64_t)__popc(ba) | ((uint64_t)__popc(bb) << kShift);
+      }
+      __syncthreads();
+      constexpr int kCells = kDeliverItems * (kDeliverThreads / 32);
+      const uint64_t mine = tid < kCells ? s_cnt[tid] : 0;
+      uint64_t total;
+      const uint64_t ex = cta_exclusive_scan<kDeliverThreads, uint64_t>(mine, &total);
+      if (tid < kCells) s_scan[tid] = ex;
+      if (warp == 0) {
+        const uint64_t base = deliver_prefix(state, tile, total, lane, limit, d_status);
+        if (lane == 0) s_base = base;
+      }
+      __syncthreads();
+      const uint64_t base = s_base, low = kTwo ? (1ull << kShift) - 1 : ~0ull;
+#pragma unroll
+      for (int c = 0; c < kDeliverItems; ++c) {
+        const int64_t i = first + c * kDeliverThreads + tid;
+        if (i >= n) continue;
+        const uint64_t off = base + s_scan[c * (kDeliverThreads / 32) + warp];
+        const int64_t u = (int64_t)(off & low) + up1[c] - 1, u2 = kTwo ? (int64_t)(off >> kShift) + up2[c] - 1 : 0;
+        sink.item(i, k[c], p[c], (h1 >> c) & 1u, u, (h2 >> c) & 1u, u2);
+      }
+      if (tile == tiles - 1) sink.finish(n, 0, false, (int64_t)((base + total) & low), kTwo ? (int64_t)((base + total) >> kShift) : 0);
+      tilesort::arrive(sink, ctl + 1, tiles);
+      __syncthreads();
     }
-    if (tile == tiles - 1) sink.finish(n, 0, false, (int64_t)((base + total) & low), kTwo ? (int64_t)((base + total) >> kShift) : 0);
-    tilesort::arrive(sink, ctl + 1, tiles);
   }
 }
 
@@ -446,7 +460,7 @@ inline size_t lsd_ws_bytes(int64_t n) {
 // (k0, v0) and so on; *in_first says whether the result ends in (k1, v1).  With a `last` of another type than ArrayOut the last
 // pass writes there instead and its arrays stay free.  **gave_up on the device: a look-back ran into its time limit, the result
 // is not to be used as positions.  d_n: number of items on the device (<= n); d_count: the count kernel writes it there, from items.
-template <class V, class Items, class Last>
+template <class V, class Items, class Last, bool kLoop = false>
 int lsd_sort(const Items& items, uint64_t* k1, V* v1, uint64_t* k0, V* v0, int64_t n, const int64_t* d_n, int64_t* d_count, int first_bit, int num_bits,
              const Last& last, bool* in_first, unsigned int** gave_up, WsCarver& c, int32_t* d_status, cudaStream_t stream) {
   using Array = ArrayOut<V>;
@@ -470,9 +484,10 @@ int lsd_sort(const Items& items, uint64_t* k1, V* v1, uint64_t* k0, V* v0, int64
       using From = std::decay_t<decltype(from)>;
       using To = std::decay_t<decltype(to)>;
       static std::atomic<uint64_t> done{0};
-      SGL_CUDA_CHECK(allow_smem((const void*)lsd_pass_kernel<V, From, To>, done, sizeof(LsdSmem<V>)));
-      return launch(lsd_pass_kernel<V, From, To>, (unsigned)tiles, kLsdThreads, sizeof(LsdSmem<V>), stream, from, Digit{first_bit + p * bits, bits},
-                    p, hist + p * kRadix, tickets + p, state, to, look_back_ns(), *gave_up, d_status);
+      SGL_CUDA_CHECK(allow_smem((const void*)lsd_pass_kernel<V, From, To, kLoop>, done, sizeof(LsdSmem<V>)));
+      const unsigned ctas = (unsigned)(kLoop && tiles > kNumSM * kLsdCtas ? kNumSM * kLsdCtas : tiles);
+      return launch(lsd_pass_kernel<V, From, To, kLoop>, ctas, kLsdThreads, sizeof(LsdSmem<V>), stream, from, Digit{first_bit + p * bits, bits}, p,
+                    hist + p * kRadix, tickets + p, state, to, look_back_ns(), *gave_up, d_status);
     };
     const bool to_last = !kArray && p == passes - 1;
     if (p == 0) SGL_CHECK_RC(to_last ? pass(items, last) : pass(items, out));
@@ -510,10 +525,11 @@ int sort_list(const Source& src, const Sink& sink, int64_t n_cap, int key_bits, 
   SGL_CHECK_RC(zero_async(ctl, (size_t)(tiles + 2) * 8, stream));
   bool in_first;
   unsigned int* gave_up;
-  SGL_CHECK_RC((lsd_sort<uint32_t, SourceItems<Source>>(SourceItems<Source>{src}, k1, v1, k0, v0, n_cap, count, count, 0, key_bits,
-                                                        ArrayOut<uint32_t>{}, &in_first, &gave_up, c, d_status, stream)));
-  return launch(lsd_deliver_kernel<Sink>, (unsigned)tiles, kDeliverThreads, 0, stream, sink, in_first ? k1 : k0, in_first ? v1 : v0, n_cap,
-                count, ctl, (uint64_t*)(ctl + 2), look_back_ns(), gave_up, d_status);
+  SGL_CHECK_RC((lsd_sort<uint32_t, SourceItems<Source>, ArrayOut<uint32_t>, Source::kOnDemand>(
+      SourceItems<Source>{src}, k1, v1, k0, v0, n_cap, count, count, 0, key_bits, ArrayOut<uint32_t>{}, &in_first, &gave_up, c, d_status, stream)));
+  const unsigned ctas = (unsigned)(tiles < kNumSM * kDeliverCtas ? tiles : kNumSM * kDeliverCtas);
+  return launch(lsd_deliver_kernel<Sink>, ctas, kDeliverThreads, 0, stream, sink, in_first ? k1 : k0, in_first ? v1 : v0, n_cap, count, ctl,
+                (uint64_t*)(ctl + 2), look_back_ns(), gave_up, d_status);
 }
 
 }  // namespace

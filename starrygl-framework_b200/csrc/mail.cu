@@ -114,6 +114,7 @@ mailbox_write_kernel(const int64_t* __restrict__ index, int64_t n_cap, const int
 inline bool aligned16(const void* p) { return ((uintptr_t)p & 15) == 0; }
 
 struct MailSource {
+  static constexpr bool kOnDemand = false;
   const int64_t *ids_a, *ids_b;
   int64_t n_a, n, num_nodes;
   const void* ts;
@@ -139,6 +140,7 @@ struct MailSource {
 
 // Node ids beyond 32 bits leave no room for the time in the key: sorted by time first, then stably by node.
 struct MailTimes {
+  static constexpr bool kOnDemand = false;
   MailSource m;
   __device__ __forceinline__ int64_t begin() const { return m.n; }
   using Raw = uint32_t;
@@ -154,6 +156,7 @@ struct OrderSink {
   __device__ __forceinline__ void finish(int64_t, uint64_t, bool, int64_t, int64_t) const {}
 };
 struct MailNodes {
+  static constexpr bool kOnDemand = false;
   MailSource m;
   const uint32_t* order;
   __device__ __forceinline__ int64_t begin() const { return m.n; }

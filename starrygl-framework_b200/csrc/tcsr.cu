@@ -131,6 +131,7 @@ struct ScannedRange {
 };
 
 struct EdgeSource {
+  static constexpr bool kOnDemand = false;
   EdgeKey k;
   int64_t m;
   ScannedRange range;

@@ -19,9 +19,10 @@
 // thread jump over the slots that the CTA's items do not reach, sums over warps are warp reductions instead of unrolled loads, and
 // splitters are searched by one rolled loop for all items of a thread.  Both kernels together, unique (id, time) pairs of 44 bits:
 // 4,096 pairs 12.3 us (17.9 before), 41,000 17.6 (23.1), 144,000 23.5 (32.6), 300,000 34.2 (50.5); with a power-law share of the ids
-// 14.1 (18.4), 17.8 (22.9), 26.5 (32.2), 43.5 (50.1).  One CTA, 600 / 1,500 pairs: 5.4 / 7.2 us (7.3 / 10.9), power law 8.3 / 11.5
-// (7.4 / 10.6), thirty copies of every pair 9.3 / 11.8 (7.2 / 10.9): cut into bins once or twice before they go by pivots.  An LSD radix sort with one kernel per 11 key bits
-// took 25, 84 and 95 us for 4,096, 41,000 and 160,000: few CTAs with large digit tables, and a dependent kernel per digit.
+// 14.9 (18.4), 17.2 (22.9), 25.8 (32.2), 39.5 (50.1).  One CTA, 600 / 1,500 pairs: 5.4 / 7.2 us (7.3 / 10.9), power law 8.3 / 11.5
+// (7.4 / 10.6), thirty copies of every pair 8.0 / 12.0 (7.2 / 10.9): cut into bins once or twice before they go by pivots.
+// An LSD radix sort with one kernel per 11 key bits took 25, 84 and 95 us for 4,096, 41,000 and 160,000 pairs: few CTAs with large
+// digit tables, and a dependent kernel per digit.
 #pragma once
 #include "common.cuh"
 #include "launch.cuh"
@@ -195,7 +196,7 @@ __device__ __forceinline__ uint64_t warp_max(uint64_t x) {
 // are as narrow as positions: where crowded bins are full of them (recent neighbours of the same few nodes), or after kSpreadLevels
 // levels, it gives up and leaves the items as they were; returns whether they are sorted.
 // cnt: scratch of 2 m words, 16-byte aligned, and 16 bytes that may be written behind them; some: 2 m half words.
-constexpr int kSpreadFew = 32, kSpreadLevels = 3;         // (32, 128, 512 items of a bin are left to comparisons at levels 1, 2, 3)
+constexpr int kSpreadFew = 16, kSpreadLevels = 4;         // (16, 32, 64, 128 items of a bin are left to comparisons at levels 1 - 4)
 constexpr int kSpreadCopies = 32;                         // threads that may hold a copy of a crowded bin's first key
 template <bool WIDE, int K>
 __device__ __forceinline__ bool spread_sort(const View<WIDE>& v, uint32_t* cnt, uint16_t* some, int m, int pos_bits) {
@@ -239,7 +240,7 @@ __device__ __forceinline__ bool spread_sort(const View<WIDE>& v, uint32_t* cnt, 
     }
   }
   uint32_t few = kSpreadFew;
-  for (int level = 1;; ++level, few *= 4) {
+  for (int level = 1;; ++level, few *= 2) {
 #pragma unroll
     for (int c = 0; c < K; ++c) {
       if (c * kThreads >= m) break;
@@ -388,7 +389,8 @@ static_assert(kMaxItems < (1 << 21), "rank inside a group: 21 bits");
 //   finish(n, last_key, has_last, groups, groups2)   once, by all threads of the CTA of the last bucket
 //   kAfter / after()  by one thread after every CTA has delivered its items
 // A Source: begin() loads device-side counts and returns the number of items; key(load(i)) is the key of item i.  load() only reads,
-// so that the loads of several items are in flight together; what is wrong with an item is flagged by key().
+// so that the loads of several items are in flight together; what is wrong with an item is flagged by key().  kOnDemand: the list mostly
+// turns out to be empty.
 
 // What a bucket publishes for a sink that numbers groups, in ctl[1 + b] (0: not known yet): whether the item behind it starts a group
 // / a coarser group, and the groups that start in it, its own first item aside (that is for the bucket before to say).

@@ -549,7 +549,8 @@ int sgl_mailbox_write(const int64_t* index, int64_t n, const int64_t* d_n, const
  * is sent to every replica on another rank (replica table: CSR rep_indptr / rep_ranks / rep_locs over node id).
  * Outputs, grouped by destination rank, ascending row inside a rank: out_ranks, out_rows (row of the layer list
  * to read), out_locs (slot on the receiver); d_send_sizes[num_parts]; *d_total entries (capacity cap, overflow
- * raises SGL_DEV_OVERFLOW).  These are the four arrays of a CommPlan.
+ * raises SGL_DEV_OVERFLOW, sizes and total are those of the whole plan even so; up to 32 ranks entries from place 2^31 - 1 on are an
+ * overflow too).  These are the four arrays of a CommPlan.
  * Replaces: MaterializedMultiLayerBuilder._compute_layer_route (prepare_sample.py:266-310).
  * ---------------------------------------------------------------------------------------------- */
 size_t sgl_plan_route_ws_bytes(int64_t n, int64_t cap);

@@ -155,42 +155,48 @@ plan_tally_kernel(const __grid_constant__ PlanLayers layers, const int64_t* __re
 }
 
 // exclusive scan of the (rank, CTA) counts in place, rank by rank; sizes per rank and the total.  One CTA per layer.  The counts of a rank
-// lie behind those of the rank before: one scan of all of them, four to a thread (7.4 us with a scan per rank for 4 ranks, 3.6 now).
+// lie behind those of the rank before: one scan of all of them, four to a thread (7.4 us with a scan per rank for 4 ranks, 3.9 now).
+// Sizes and total are exact whatever they are; a place beyond kLastPlace is kept as kLastPlace, and nothing is written there.
+constexpr int32_t kLastPlace = INT32_MAX;
 __global__ void __launch_bounds__(1024)
 plan_place_kernel(const __grid_constant__ PlanLayers layers, int num_parts) {
-  __shared__ int s_carry;
+  __shared__ int64_t s_carry, s_begin[kFewParts + 1];
   const PlanLayer& l = layers.l[blockIdx.x];
   int32_t* tally = l.tally;
   int64_t *d_send_sizes = l.send_sizes, *d_total = l.total;
-  const int64_t n = eff_count(l.n_cap, l.d_n), ctas = (n + kThreads - 1) / kThreads, all = ctas * num_parts;
+  const int64_t n = eff_count(l.n_cap, l.d_n);
+  const uint32_t ctas = (uint32_t)((n + kThreads - 1) / kThreads), all = ctas * (uint32_t)num_parts;      // (below 2^24, see few_parts)
   if (threadIdx.x == 0) s_carry = 0;
+  if (threadIdx.x <= num_parts) s_begin[threadIdx.x] = 0;
   __syncthreads();
-  for (int64_t b = 0; b < all; b += 4 * 1024) {
-    const int64_t j = b + 4 * threadIdx.x;
-    int v[4], sum = 0;
+  for (uint32_t b = 0; b < all; b += 4 * 1024) {
+    const uint32_t j = b + 4 * threadIdx.x;
+    int64_t v[4], sum = 0;
 #pragma unroll
     for (int u = 0; u < 4; ++u) v[u] = j + u < all ? tally[j + u] : 0;
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
-      const int x = v[u];
+      const int64_t x = v[u];
       v[u] = sum;
       sum += x;
     }
-    const int carry = s_carry;           // (the barriers of the scan lie between this read and the write below)
-    int tot;
-    const int at = carry + cta_exclusive_scan<1024, int>(sum, &tot);
+    const int64_t carry = s_carry;       // (the barriers of the scan lie between this read and the write below)
+    int64_t tot;
+    const int64_t at = carry + cta_exclusive_scan<1024, int64_t>(sum, &tot);
 #pragma unroll
-    for (int u = 0; u < 4; ++u)
-      if (j + u < all) tally[j + u] = at + v[u];
+    for (int u = 0; u < 4; ++u) {
+      if (j + u >= all) break;
+      const int64_t place = at + v[u];
+      tally[j + u] = place < kLastPlace ? (int32_t)place : kLastPlace;
+      const uint32_t r = (j + u) / ctas;
+      if (r * ctas == j + u) s_begin[r] = place;
+    }
     if (threadIdx.x == 0) s_carry = carry + tot;
     __syncthreads();
   }
-  const int64_t total = s_carry;
-  for (int r = threadIdx.x; r < num_parts; r += 1024) {
-    const int64_t begin = ctas ? tally[r * ctas] : 0, end = r + 1 < num_parts && ctas ? (int64_t)tally[(r + 1) * ctas] : total;
-    d_send_sizes[r] = end - begin;
-  }
-  if (threadIdx.x == 0) *d_total = total;
+  if (threadIdx.x == 0) *d_total = s_begin[num_parts] = s_carry;
+  __syncthreads();
+  if (threadIdx.x < num_parts) d_send_sizes[threadIdx.x] = s_begin[threadIdx.x + 1] - s_begin[threadIdx.x];
 }
 
 // Four ranks at a time share a scan, 16 bits each (three layers, 4 ranks: 11.4 -> 10.9 us), unless a node has more copies than that allows.
@@ -223,6 +229,7 @@ plan_write_kernel(const __grid_constant__ PlanLayers layers, const int64_t* __re
     }
     uint64_t at = cta_exclusive_scan<kThreads, uint64_t>(mine, nullptr);
     if (mine == 0) continue;
+    bool over = false;
     const uint64_t low = width == 1 ? ~0ull : 0xffffull;
     for (int64_t p = s; p < e; ++p) {
       const int64_t r = ranks[p];
@@ -231,14 +238,15 @@ plan_write_kernel(const __grid_constant__ PlanLayers layers, const int64_t* __re
       const int64_t first = u == 0 ? before[0] : (u == 1 ? before[1] : (u == 2 ? before[2] : before[3]));
       const int64_t to = first + (int64_t)((at >> (u * bits)) & low);
       at += 1ull << (u * bits);
-      if (to >= cap) {
-        dev_flag(d_status, SGL_DEV_OVERFLOW);
+      if (first == kLastPlace || to >= cap) {
+        over = true;
         continue;
       }
       out_ranks[to] = r;
       out_rows[to] = i;
       out_locs[to] = locs[p];
     }
+    if (over) dev_flag(d_status, SGL_DEV_OVERFLOW);
   }
 }
 

@@ -71,6 +71,23 @@ def test_route_plan_of_nodes_with_many_copies(num_parts, copies):
         assert np.array_equal(npy(a), b)
 
 
+def test_route_plan_of_more_entries_than_32_bits_count():
+    """Every second node's copies are the same 2^20 table entries: 2^31 + 2^20 places in a plan with room for 1,000 of each rank's."""
+    from starrygl import ops
+    copies, rows, cap = 1 << 20, 2 * 2049, 1000
+    indptr = torch.arange(rows + 1, device="cuda") % 2 * copies
+    ranks = (torch.arange(copies, device="cuda") % 4 == 0).long() + 1                  # three quarters on rank 1, the others on rank 2
+    locs = torch.arange(copies, device="cuda")
+    st = ops.StatusWord(torch.device("cuda"))
+    out_ranks, out_rows, out_locs, sizes, total = ops.plan_route(torch.arange(rows, device="cuda"), torch.zeros(rows, dtype=torch.int64, device="cuda"),
+                                                                 0, indptr, ranks, locs, 3, cap, status=st)
+    assert int(total) == 2049 * copies > 2 ** 31 and sizes.tolist() == [0, 2049 * copies // 4 * 3, 2049 * copies // 4]
+    assert torch.equal(out_ranks, torch.ones_like(out_ranks)) and not out_rows.any()
+    assert torch.equal(out_locs, locs[ranks == 1][:cap])
+    with pytest.raises(Exception, match="capacity"):
+        st.check("plan")
+
+
 @pytest.mark.parametrize("fanouts", [[3], [10, 10], [4, 3, 2]])
 @pytest.mark.parametrize("roots", [1, 700, 5000])
 def test_layout_of_a_batch_next_to_its_last_merge(fanouts, roots):

@@ -71,6 +71,25 @@ def test_route_plan_of_nodes_with_many_copies(num_parts, copies):
         assert np.array_equal(npy(a), b)
 
 
+@pytest.mark.parametrize("rank", [0, 3])
+@pytest.mark.parametrize("copies", [255, 256, 257, 1000])
+def test_route_plan_whose_ranks_fill_their_part_of_a_scan(copies, rank):
+    """256 rows of one CTA with all copies on one rank: 65,280 places of a field of 16 bits, and more than it holds."""
+    from starrygl.cache.cache_route import compute_layer_route
+    from starrygl.cache.replica_table import CSRReplicaTable
+    nodes = 600
+    ids, parts = np.arange(nodes), np.ones(nodes, np.int64)
+    indptr = np.concatenate([[0], np.cumsum(np.full(nodes, copies))]).astype(np.int64)
+    ranks = np.full(indptr[-1], rank, np.int64)
+    ranks[indptr[255]:indptr[256]:5] = 2                       # (the field behind the one that is full, or before it)
+    ranks[indptr[255] + 1] = 4
+    locs = np.arange(indptr[-1], dtype=np.int64)
+    plan = compute_layer_route(cu(ids), cu(parts), 1, CSRReplicaTable(cu(indptr), cu(ranks), cu(locs)), 5, max_replicas_per_node=copies)
+    ref = O.compute_layer_route(ids, np.arange(nodes), parts, 1, indptr, ranks, locs, 5)
+    for a, b in zip((plan.send_ranks, plan.send_sizes, plan.send_indices, plan.send_remote_indices), ref):
+        assert np.array_equal(npy(a), b)
+
+
 def test_route_plan_of_more_entries_than_32_bits_count():
     """Every second node's copies are the same 2^20 table entries: 2^31 + 2^20 places in a plan with room for 1,000 of each rank's."""
     from starrygl import ops

@@ -620,8 +620,8 @@ int sgl_build_batch_at(const int64_t* indptr, const int64_t* nbr, const int64_t*
                     uint64_t seed, int id_bits, int ts_bits, int64_t ts_base, const int64_t* section_at,
                     int64_t* base, int64_t* other_base, int64_t* meta, int32_t* d_status, int64_t* host_meta, void* ws, size_t ws_bytes, void* side_stream, void* stream);
 /* sgl_build_batch_at that also writes the counts to host_early (pinned, 1 + 2 * n_hops words, then a flag word that becomes 1) as soon as
- * all of them but the last are known, next to the merge of the last list: a host that waits for that flag (which may also stay 0,
- * outside of a launch graph) lays out everything but the last list while the device still merges it. */
+ * all of them but the last are known, before or next to the merge of the last list: a host that waits for that flag lays out everything
+ * but the last list while the device still merges it.  The flag comes with every call that succeeds. */
 int sgl_build_batch_staged(const int64_t* indptr, const int64_t* nbr, const int64_t* ts, const int64_t* eid, const int64_t* fence,
                     int64_t num_nodes, const int64_t* roots, const int64_t* root_ts, int64_t n_roots,
                     const int32_t* fanouts, int n_hops, int policy, int equal_root_time, int64_t allowed_offset,

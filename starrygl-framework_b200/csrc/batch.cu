@@ -181,10 +181,10 @@ static int build_batch(const int64_t* indptr, const int64_t* nbr, const int64_t*
   LaunchScope scope(stream);
   SGL_CHECK_RC(zero_async(meta, (size_t)(2 + 2 * n_hops) * sizeof(int64_t), stream));
   auto done = [&]() -> int {
+    if (host_early) SGL_CHECK_RC(export_words(meta, host_early, 1 + 2 * n_hops, stream));      // (no roots, or no hops)
     if (host_meta) SGL_CHECK_RC(export_words(meta, host_meta, 2 + 2 * n_hops, stream));
     return scope.submit();
   };
-  if (host_early) *(volatile int64_t*)(host_early + 1 + 2 * n_hops) = 0;
   if (n_roots == 0) return done();
   SGL_REQUIRE(section_at && roots && root_ts, SGL_ERR_ARG, "build_batch: null array");
   SGL_REQUIRE(ws_bytes >= sgl_build_batch_ws_bytes(n_roots, fanouts, n_hops), SGL_ERR_WORKSPACE, "build_batch: workspace %zu < %zu bytes",
@@ -262,11 +262,14 @@ static int build_batch(const int64_t* indptr, const int64_t* nbr, const int64_t*
       order_of = RowOrder::carve(ows, c + e);
       ows += RowOrder::bytes(c + e);
     }
-    if (host_early && l + 1 == n_hops && LaunchScope::current() != nullptr) {
-      // (a third chain of the graph, next to the last merge)
-      cudaStream_t third = (cudaStream_t)(uintptr_t)5;
-      SGL_CHECK_RC(LaunchScope::current()->follow(third, stream));
-      SGL_CHECK_RC(export_words(meta, host_early, 1 + 2 * n_hops, third));
+    if (host_early && l + 1 == n_hops) {
+      cudaStream_t on = stream;
+      if (LaunchScope::current() != nullptr) {
+        on = (cudaStream_t)(uintptr_t)5;       // a third chain of the graph, next to the last merge
+        SGL_CHECK_RC(LaunchScope::current()->follow(on, stream));
+      }
+      SGL_CHECK_RC(export_words(meta, host_early, 1 + 2 * n_hops, on));
+      host_early = nullptr;
     }
     rc = unique_pairs(cur_id, cur_ts, c, d_cur, h.nbr, h.ts, e, d_edges, id_bits, ts_bits, ts_base, h.gids, h.gts, nullptr, h.col,
                       l > 0 && narrow_columns(e) ? cols32 : nullptr, d_next, order_of, d_status, lws, lwb, stream);

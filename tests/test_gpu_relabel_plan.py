@@ -125,3 +125,35 @@ def test_layout_of_a_batch_next_to_its_last_merge(fanouts, roots):
             assert list(x) == list(y)
             for k in x:
                 assert x[k].dtype == y[k].dtype and torch.equal(x[k], y[k]), k
+
+
+@pytest.mark.parametrize("fanouts", [[], [3], [4, 2]])
+@pytest.mark.parametrize("roots", [0, 500])
+@pytest.mark.parametrize("captured", [False, True])
+def test_early_counts_come_with_every_batch(fanouts, roots, captured):
+    """Also where the batch has no last merge, and where its kernels are captured instead of collected into a launch graph."""
+    from starrygl import ops
+    from starrygl.graph.batch import _enqueue
+    rng = np.random.default_rng(roots)
+    n, m = 300, 4000
+    src, dst, ts = rng.integers(0, n, m), rng.integers(0, n, m), np.sort(rng.integers(0, 10 ** 6, m))
+    g = ops.tcsr_build(cu(src), cu(dst), cu(ts), None, n)
+    pick = rng.integers(0, m, roots)
+    q, t = cu(src[pick]), cu(ts[pick])
+    words, last = torch.zeros(64, dtype=torch.int64).pin_memory(), 1 + 2 * len(fanouts)
+
+    def call():
+        return _enqueue(g, q, t, fanouts, "recent", g.ts_min, g.ts_max, False, -1, 0, None, None, words.data_ptr(), early=words[32:].data_ptr())
+    kept = call()
+    if captured:
+        torch.cuda.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            kept = call()
+        words.fill_(-1)
+        graph.replay()
+    torch.cuda.synchronize()
+    all_counts, early = words[:last + 2].tolist(), words[32:33 + last].tolist()
+    assert all_counts[last:] == [0, 1] and early[last] == 1 and kept.n == roots
+    known = last if not fanouts else last - 1
+    assert early[:known] == all_counts[:known] and (roots == 0 or all_counts[0] > 0)

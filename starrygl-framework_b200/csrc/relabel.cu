@@ -201,20 +201,54 @@ csc_rows_copy_kernel(const RowOrder ro, const int64_t* d_rows, const int64_t* __
 
 // ---- node relabel by bitmap ----------------------------------------------------------------------------------------------
 // Ids without a time need no sort: the new ones of a list are marked in a bitmap of the nodes, their ascending order is the bitmap's, and
-// an entry's local id is its node's.  Three kernels of 2 - 4 us: 20,000 and 80,000 entries over 50,000 nodes 10 and 11 us, the two kernels
-// of the sort 16 and 27.  A CTA of the middle kernel counts the marks before its own by itself, so the bitmap is bounded: 2^19 nodes,
-// 64 KB, an eighth of that a thread's loads each; up to 2,048 entries one CTA sorts faster.
+// an entry's local id is its node's.  Three kernels of 2 - 5 us; kernels of a list, the sort -> the bitmap (entries over 50,000 nodes, all
+// nodes alike / a power law with its hubs next to each other / one node): 2,049 entries 21 -> 11 us; 20,000 24 / 24 / 26 -> 12 / 13 / 10;
+// 80,000 31 / 31 / 38 -> 17 / 20 / 12; 300,000 54 / 56 / 75 -> 30 / 43 / 17; 1.2 M 250 / 234 / 224 -> 78 / 107 / 37; 4 M 208 / 198 / 161 ->
+// 145 / 223 / 62.  Over 2^19 nodes: 2,049 entries 21 -> 13, 80,000 33 / 32 / 38 -> 15 / 22 / 14, 4 M 250 / 238 / 201 -> 95 / 218 / 64.
+// A CTA of the middle kernel counts the marks before its own by itself, so the bitmap is bounded: 2^19 nodes are 64 KB, at most 64 loads a
+// thread; up to 2,048 entries one CTA sorts in a single launch.
 constexpr int64_t kBitmapNodes = 1 << 19;
+static_assert(kBitmapNodes / 8 <= tilesort::kMatrix * 4, "the bitmap lies in the scratch of a sort");
 inline bool by_bitmap(int64_t n, int64_t num_nodes) { return n > tilesort::kSingleMax && num_nodes > 0 && num_nodes <= kBitmapNodes; }
 
+// Lists have hubs, and an atomic on a hot word takes 0.65 ns: lanes of a warp that share a word set their marks together (looked for only
+// where some of 48 pairs of lanes do), and a mark that is there already is not set again (one atomic per entry: 300,000 entries 133 us with
+// a power law, 202 us of one node; 4 M entries 1.6 and 2.6 ms).
 __global__ void __launch_bounds__(kThreads)
 nodes_mark_kernel(const int64_t* __restrict__ ids, int64_t n_cap, const int64_t* d_n, int64_t num_nodes, const int64_t* __restrict__ mask,
                   int64_t epoch, uint32_t* bits, int32_t* d_status) {
+  __shared__ uint32_t s_marks[kThreads];   // of the lanes that share a word, at the first of them
   const int64_t n = eff_count(n_cap, d_n), stride = (int64_t)gridDim.x * kThreads;
-  for (int64_t i = (int64_t)blockIdx.x * kThreads + threadIdx.x; i < n; i += stride) {
-    const int64_t g = ids[i];
-    if (g < 0 || g >= num_nodes) dev_flag(d_status, SGL_DEV_BAD_NODE);
-    else if (mask[g] != epoch) atomicOr(bits + (g >> 5), 1u << (g & 31));
+  const int lane = threadIdx.x & 31;
+  uint32_t* const marks = s_marks + (threadIdx.x & ~31);
+  for (int64_t i = (int64_t)blockIdx.x * kThreads + threadIdx.x; i - lane < n; i += stride) {
+    int word = -1;
+    uint32_t mark = 0;
+    if (i < n) {
+      const int64_t g = ids[i];
+      if (g < 0 || g >= num_nodes) {
+        dev_flag(d_status, SGL_DEV_BAD_NODE);
+      } else {
+        // (not in the first round: there is nothing to find, and reading behind everybody's marks took 2 of 7 us)
+        const uint32_t there = i >= stride ? __ldcg(bits + (g >> 5)) : 0u, own = 1u << (g & 31);
+        if (mask[g] != epoch && !(there & own)) {
+          word = (int)(g >> 5);
+          mark = own;
+        }
+      }
+    }
+    const int w16 = __shfl_xor_sync(0xffffffffu, word, 16), w8 = __shfl_xor_sync(0xffffffffu, word, 8), w4 = __shfl_xor_sync(0xffffffffu, word, 4);
+    if (__any_sync(0xffffffffu, word >= 0 && (word == w16 || word == w8 || word == w4))) {
+      const int first = __ffs(__match_any_sync(0xffffffffu, word)) - 1;
+      marks[lane] = 0;
+      __syncwarp();
+      if (word >= 0) atomicOr(marks + first, mark);
+      __syncwarp();
+      mark = marks[lane];
+      if (lane != first) word = -1;
+      __syncwarp();
+    }
+    if (word >= 0) atomicOr(bits + word, mark);
   }
 }
 

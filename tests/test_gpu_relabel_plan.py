@@ -34,6 +34,26 @@ def test_relabel_of_lists_that_continue_each_other(num_nodes, n):
     st.check("relabel")
 
 
+@pytest.mark.parametrize("num_nodes", [32, 50000])
+@pytest.mark.parametrize("share", [0.5, 0.99, 1.0])
+def test_relabel_of_lists_with_hubs(num_nodes, share):
+    """Nodes that a large part of the list is copies of: all lanes of a warp, and all warps, mark the same word."""
+    from starrygl import ops
+    rng = np.random.default_rng(num_nodes)
+    n = 1_300_000
+    rl, st = ops.NodeRelabeler(num_nodes, torch.device("cuda")), ops.StatusWord(torch.device("cuda"))
+    table, base = np.full(num_nodes, -1, np.int64), 0
+    for hubs in ([7], [0, 31, num_nodes - 1]):
+        ids = np.where(rng.random(n) < share, rng.choice(hubs, n), rng.integers(0, num_nodes, n)).astype(np.int64)
+        local, new, d_new = rl.insert(cu(ids), status=st)
+        fresh = np.unique(ids)
+        fresh = fresh[table[fresh] < 0]
+        table[fresh] = base + np.arange(len(fresh))
+        base += len(fresh)
+        assert int(d_new) == len(fresh) and np.array_equal(npy(new[:len(fresh)]), fresh) and np.array_equal(npy(local), table[ids])
+    st.check("relabel")
+
+
 def test_relabel_flags_ids_out_of_range():
     from starrygl import ops
     n, num_nodes = 5000, 1000

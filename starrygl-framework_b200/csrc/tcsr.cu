@@ -116,7 +116,8 @@ __device__ __forceinline__ void start_rows(int64_t* __restrict__ indptr, int64_t
 
 // ---- up to the mini-batch limit -----------------------------------------------------------------------------------------
 // The sort is enqueued together with the scan and reads the time range where the scan leaves it; node, time and position share a word of
-// 64 bits then, or there is nothing to sort and the host, which learns the same a little later, starts over with what it knows.
+// 64 bits then, or there is nothing to sort, nothing is written, and the host, which learns the same a little later, raises or starts over
+// with what it knows.
 struct ScannedRange {
   const InputScan* scan;                 // nullptr: the key is complete
   int id_bits, pos_bits;
@@ -148,7 +149,8 @@ struct EdgeSink {
   int64_t num_nodes;
   int64_t *indptr, *out_nbr, *out_ts, *out_eid, *out_perm;
   ScannedRange range;
-  __device__ __forceinline__ void begin() { range.read(k); }
+  bool sorted;
+  __device__ __forceinline__ void begin() { sorted = range.read(k); }
   __device__ __forceinline__ void item(int64_t at, uint64_t key, uint32_t p) const {
     out_nbr[at] = nbr[p];
     out_ts[at] = k.time(key);
@@ -159,6 +161,7 @@ struct EdgeSink {
     start_rows(indptr, has_prev ? k.node(prev) : -1, k.node(key), at);
   }
   __device__ __forceinline__ void finish(int64_t m, uint64_t last, bool has_last, int64_t, int64_t) const {
+    if (!sorted) return;
     for (int64_t v = (has_last ? k.node(last) + 1 : 0) + threadIdx.x; v <= num_nodes; v += blockDim.x) indptr[v] = m;
   }
 };
@@ -260,7 +263,8 @@ __global__ void fill_i64_kernel(int64_t* p, int64_t n, int64_t v) {
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) p[i] = v;
 }
 
-int launch_fence(const int64_t* indptr, const int64_t* ts, int64_t num_nodes, int64_t m, int64_t* out_fence, cudaStream_t stream);
+int launch_fence(const int64_t* indptr, const int64_t* ts, int64_t num_nodes, int64_t m, int64_t* out_fence, const ScannedRange& range,
+                 cudaStream_t stream);
 
 }  // namespace
 }  // namespace sgl
@@ -317,9 +321,9 @@ extern "C" int sgl_tcsr_build_fenced(int64_t num_nodes, int64_t m, const int64_t
     if (small) {
       const EdgeKey k{key, ts, 0, 0};
       const ScannedRange range{d_scan, id_bits, pos_bits};
-      SGL_CHECK_RC(sort_list(EdgeSource{k, m, range}, EdgeSink{k, nbr, eid, num_nodes, indptr, out_nbr, out_ts, out_eid, out_perm, range}, m,
+      SGL_CHECK_RC(sort_list(EdgeSource{k, m, range}, EdgeSink{k, nbr, eid, num_nodes, indptr, out_nbr, out_ts, out_eid, out_perm, range, false}, m,
                              64 - pos_bits, rest, rest_bytes, nullptr, stream));
-      if (out_fence && num_nodes > 0) SGL_CHECK_RC(launch_fence(indptr, out_ts, num_nodes, m, out_fence, stream));
+      if (out_fence && num_nodes > 0) SGL_CHECK_RC(launch_fence(indptr, out_ts, num_nodes, m, out_fence, range, stream));
     }
     SGL_CHECK_RC(scope.submit());
   }
@@ -355,7 +359,7 @@ extern "C" int sgl_tcsr_build_fenced(int64_t num_nodes, int64_t m, const int64_t
                         num_nodes, indptr, out_nbr, out_ts, out_eid, out_perm));
   } else if (small) {
     const ScannedRange known{nullptr, 0, 0};
-    SGL_CHECK_RC(sort_list(EdgeSource{k, m, known}, EdgeSink{k, nbr, eid, num_nodes, indptr, out_nbr, out_ts, out_eid, out_perm, known}, m,
+    SGL_CHECK_RC(sort_list(EdgeSource{k, m, known}, EdgeSink{k, nbr, eid, num_nodes, indptr, out_nbr, out_ts, out_eid, out_perm, known, false}, m,
                            ts_bits + id_bits, rest, rest_bytes, nullptr, stream));
   } else {
     const int first_bit = flags & kUnordered ? 0 : (ts_bits < 56 ? ts_bits : 56);   // in time order: only the node bits are left
@@ -377,7 +381,7 @@ extern "C" int sgl_tcsr_build_fenced(int64_t num_nodes, int64_t m, const int64_t
                           indptr, out_nbr, out_ts, out_eid, out_perm));
     }
   }
-  if (out_fence && num_nodes > 0) SGL_CHECK_RC(launch_fence(indptr, out_ts, num_nodes, m, out_fence, stream));
+  if (out_fence && num_nodes > 0) SGL_CHECK_RC(launch_fence(indptr, out_ts, num_nodes, m, out_fence, {nullptr, 0, 0}, stream));
   if (small) return scope.submit();
   // The radix passes wait for each other's tiles, for a limited time: the graph is handed out once they are known to have come through.
   int64_t* const result = h + 8;
@@ -410,7 +414,9 @@ namespace {
 // written by as many threads, not by one warp.
 __global__ void __launch_bounds__(256)
 tcsr_fence_kernel(const int64_t* __restrict__ indptr, const int64_t* __restrict__ ts, int64_t num_nodes, int64_t len,
-                  int64_t* __restrict__ fence) {
+                  int64_t* __restrict__ fence, const ScannedRange range) {
+  EdgeKey unused{};
+  if (!range.read(unused)) return;
   const int64_t stride = (int64_t)gridDim.x * 256;
   for (int64_t x = (int64_t)blockIdx.x * 256 + threadIdx.x; x < len; x += stride) {
     int64_t lo = 0, hi = num_nodes;          // invariant: start(lo) <= x; rows >= hi start after x
@@ -427,9 +433,10 @@ tcsr_fence_kernel(const int64_t* __restrict__ indptr, const int64_t* __restrict_
   }
 }
 
-int launch_fence(const int64_t* indptr, const int64_t* ts, int64_t num_nodes, int64_t m, int64_t* out_fence, cudaStream_t stream) {
+int launch_fence(const int64_t* indptr, const int64_t* ts, int64_t num_nodes, int64_t m, int64_t* out_fence, const ScannedRange& range,
+                 cudaStream_t stream) {
   const int64_t len = sgl_tcsr_fence_len(num_nodes, m);
-  return launch(tcsr_fence_kernel, stream_grid(len, 256, 16), 256, 0, stream, indptr, ts, num_nodes, len, out_fence);
+  return launch(tcsr_fence_kernel, stream_grid(len, 256, 16), 256, 0, stream, indptr, ts, num_nodes, len, out_fence, range);
 }
 }  // namespace
 }  // namespace sgl
@@ -441,5 +448,5 @@ extern "C" int sgl_tcsr_fence(const int64_t* indptr, const int64_t* ts, int64_t 
   SGL_REQUIRE(num_nodes >= 0 && m >= 0, SGL_ERR_ARG, "tcsr_fence: negative size");
   if (num_nodes == 0 || m == 0) return SGL_OK;
   SGL_REQUIRE(indptr && ts && out_fence, SGL_ERR_ARG, "tcsr_fence: null array");
-  return launch_fence(indptr, ts, num_nodes, m, out_fence, (cudaStream_t)stream_);
+  return launch_fence(indptr, ts, num_nodes, m, out_fence, {nullptr, 0, 0}, (cudaStream_t)stream_);
 }

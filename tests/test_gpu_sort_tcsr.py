@@ -78,3 +78,21 @@ def test_tcsr_rejects_out_of_range_ids():
         ops.tcsr_build(key, key, key, None, 5)
     with pytest.raises(_C.SglError):
         ops.tcsr_build(cu(np.array([-1], dtype=np.int64)), key[:1], key[:1], None, 5)
+
+
+@pytest.mark.parametrize("m", [1500, 160000])
+def test_build_that_is_refused_writes_nothing(m):
+    """The sort of a small build is enqueued before the host knows that a node id is out of range."""
+    from starrygl import _C
+    lib, n = _C.lib(), 5000
+    key = torch.randint(0, n, (m,), device="cuda")
+    key[m // 2] = n
+    ts = torch.arange(m, device="cuda")
+    out = [torch.full((k,), -7, dtype=torch.int64, device="cuda") for k in (n + 1, m, m, m, int(lib.sgl_tcsr_fence_len(n, m)))]
+    ws = torch.empty(int(lib.sgl_tcsr_build_ws_bytes(n, m)), dtype=torch.uint8, device="cuda")
+    with pytest.raises(_C.SglError, match="1 edge keys outside"):
+        _C.check(lib.sgl_tcsr_build_fenced(n, m, key.data_ptr(), key.data_ptr(), ts.data_ptr(), None, out[0].data_ptr(), out[1].data_ptr(),
+                                           out[2].data_ptr(), out[3].data_ptr(), None, out[4].data_ptr(), None, ws.data_ptr(), ws.numel(),
+                                           _C.stream_ptr()))
+    torch.cuda.synchronize()
+    assert all(bool((t == -7).all()) for t in out)

@@ -82,6 +82,7 @@ struct CscSource {
   int64_t ts_base;
   const int* gate;                       // optional: 0 = another kernel has done the work
   int32_t* d_status;
+  bool on_demand() const { return gate != nullptr; }
   __device__ __forceinline__ int64_t begin() const { return gate && *gate == 0 ? 0 : eff_count(n_cap, d_n); }
   using Raw = longlong2;
   __device__ __forceinline__ Raw load(int64_t e) const { return {dst_map ? dst_map[dst[e]] : dst[e], ts[e]}; }

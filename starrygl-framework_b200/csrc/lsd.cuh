@@ -179,7 +179,8 @@ struct SourceItems {
 };
 
 // kLoop: a CTA takes tile after tile instead of one, for sorts that mostly turn out not to be needed (a CTA per tile of 38 M entries that
-// are not there took 8 us a pass, 38 us behind the last merge of a batch; a list that is there is 6 % faster without the loop).
+// are not there took 8 us a pass, 38 us behind the last merge of a batch; a list that is there is faster without the loop, passes of a
+// CSC of 1.3 M edges 84 and 80 us, 16 M 793 and 756).
 template <class V, class Items, class Out, bool kLoop>
 __global__ void __launch_bounds__(kLsdThreads, kLsdCtas)
 lsd_pass_kernel(Items items, Digit digit, int pass,
@@ -313,7 +314,8 @@ lsd_pass_kernel(Items items, Digit digit, int pass,
 // ---- delivery of a sorted list to a Sink (see tilesort.cuh) -------------------------------------------------------------
 constexpr int kDeliverThreads = 256;
 constexpr int kDeliverItems = 8;
-constexpr int kDeliverCtas = 4;           // per SM
+template <class Sink>
+constexpr int kDeliverCtas = Sink::kUnique ? 4 : 6;       // per SM (without numbering 32 registers, with the 56 of 4 CTAs 1.3 M edges took 44 us, not 33)
 constexpr int kDeliverTile = kDeliverThreads * kDeliverItems;
 
 // Sum of what the CTAs before this one (by ticket: they all run already) published; called by one whole warp.
@@ -352,7 +354,7 @@ __device__ __forceinline__ uint64_t deliver_prefix(uint64_t* state, int tile, ui
 
 // ctl[0] ticket, ctl[1] arrivals; state: one word per tile, cleared
 template <class Sink>
-__global__ void __launch_bounds__(kDeliverThreads, kDeliverCtas)
+__global__ void __launch_bounds__(kDeliverThreads, kDeliverCtas<Sink>)
 lsd_deliver_kernel(Sink sink, const uint64_t* __restrict__ keys, const uint32_t* __restrict__ pos, int64_t n_cap, const int64_t* d_count,
                    unsigned long long* ctl, uint64_t* state, unsigned long long limit, const unsigned int* gave_up, int32_t* d_status) {
   const int64_t n = *gave_up ? 0 : eff_count(n_cap, d_count);     // (a pass that gave up left places unwritten)
@@ -525,9 +527,20 @@ int sort_list(const Source& src, const Sink& sink, int64_t n_cap, int key_bits, 
   SGL_CHECK_RC(zero_async(ctl, (size_t)(tiles + 2) * 8, stream));
   bool in_first;
   unsigned int* gave_up;
-  SGL_CHECK_RC((lsd_sort<uint32_t, SourceItems<Source>, ArrayOut<uint32_t>, Source::kOnDemand>(
-      SourceItems<Source>{src}, k1, v1, k0, v0, n_cap, count, count, 0, key_bits, ArrayOut<uint32_t>{}, &in_first, &gave_up, c, d_status, stream)));
-  const unsigned ctas = (unsigned)(tiles < kNumSM * kDeliverCtas ? tiles : kNumSM * kDeliverCtas);
+  auto sort = [&](auto loop) -> int {
+    return lsd_sort<uint32_t, SourceItems<Source>, ArrayOut<uint32_t>, decltype(loop)::value>(
+        SourceItems<Source>{src}, k1, v1, k0, v0, n_cap, count, count, 0, key_bits, ArrayOut<uint32_t>{}, &in_first, &gave_up, c, d_status, stream);
+  };
+  bool loop = Sink::kUnique;             // (delivery without numbering, as many CTAs as there is room for or one per tile: CSC of 16 M edges
+                                         // 1,301, 1,208 us)
+  if constexpr (Source::kOnDemand) {
+    SGL_CHECK_RC(src.on_demand() ? sort(std::true_type{}) : sort(std::false_type{}));
+    loop = loop || src.on_demand();
+  } else {
+    SGL_CHECK_RC(sort(std::false_type{}));
+  }
+  constexpr int kRoom = kNumSM * kDeliverCtas<Sink>;
+  const unsigned ctas = (unsigned)(loop && tiles > kRoom ? kRoom : tiles);
   return launch(lsd_deliver_kernel<Sink>, ctas, kDeliverThreads, 0, stream, sink, in_first ? k1 : k0, in_first ? v1 : v0, n_cap, count, ctl,
                 (uint64_t*)(ctl + 2), look_back_ns(), gave_up, d_status);
 }

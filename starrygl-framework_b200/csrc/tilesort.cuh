@@ -389,8 +389,8 @@ static_assert(kMaxItems < (1 << 21), "rank inside a group: 21 bits");
 //   finish(n, last_key, has_last, groups, groups2)   once, by all threads of the CTA of the last bucket
 //   kAfter / after()  by one thread after every CTA has delivered its items
 // A Source: begin() loads device-side counts and returns the number of items; key(load(i)) is the key of item i.  load() only reads,
-// so that the loads of several items are in flight together; what is wrong with an item is flagged by key().  kOnDemand: the list mostly
-// turns out to be empty.
+// so that the loads of several items are in flight together; what is wrong with an item is flagged by key().  kOnDemand: where on_demand()
+// says so the list mostly turns out to be empty.
 
 // What a bucket publishes for a sink that numbers groups, in ctl[1 + b] (0: not known yet): whether the item behind it starts a group
 // / a coarser group, and the groups that start in it, its own first item aside (that is for the bucket before to say).

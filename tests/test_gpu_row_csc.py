@@ -57,6 +57,31 @@ def test_narrow_columns(copies, fanouts):
             assert np.array_equal(npy(d[k]), r[k]), (i, k)
 
 
+def test_sort_that_is_needed_after_all_of_millions_of_edges():
+    """Rows of more targets than the rows kernel takes, in a hop of more edges than the sort's passes have CTAs for at a time (2,121,728):
+    its CTAs take a second tile, and what the first one left in shared memory is gone."""
+    from starrygl import ops
+    from starrygl.graph.batch import build_batch_async
+    gen = torch.Generator(device="cuda").manual_seed(2)
+    n, m, roots, fanouts = 1000, 300_000, 4000, [30, 50]
+    src, dst = (torch.randint(0, n, (m,), device="cuda", generator=gen) for _ in range(2))
+    g = ops.tcsr_build(src, dst, torch.randint(0, 4, (m,), device="cuda", generator=gen), None, n)
+    db = build_batch_async(g, torch.arange(roots, device="cuda") % n, 4 + torch.arange(roots, device="cuda"), fanouts, "uniform",
+                           ts_range=(0, 4 + roots))
+    out = db.finish()
+    first, hop = db.layers[1], db.layers[2]["hop"]
+    k, targets = int(db.counts[3]), int(db.counts[1])
+    assert k > 2 * 2_121_728
+    per_target = hop.offsets[1:targets + 1] - hop.offsets[:targets]
+    assert int(torch.bincount(first["inv"][:targets][per_target == fanouts[1]]).max()) > 33
+    row, ts = first["inv"][hop.dst[:k]], hop.ts[:k]
+    order = torch.sort(row * 8 + ts, stable=True).indices
+    rows = out[1]["gids"].numel()
+    assert torch.equal(out[2]["indptr"], torch.cat([row.new_zeros(1), torch.bincount(row, minlength=rows).cumsum(0)]))
+    for name, raw in (("indices", db.layers[2]["inv"]), ("eid", hop.eid), ("edge_ts", hop.ts), ("edge_dt", hop.dt)):
+        assert torch.equal(out[2][name], raw[:k][order]), name
+
+
 def test_neighbours_outside_the_graph_are_an_error():
     """A list entry of replaced ids has targets with different edges: rows of the CSC stay partly unwritten, the call raises."""
     from starrygl import _C, ops

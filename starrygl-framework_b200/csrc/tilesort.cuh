@@ -19,8 +19,9 @@
 // thread jump over the slots that the CTA's items do not reach, sums over warps are warp reductions instead of unrolled loads, and
 // splitters are searched by one rolled loop for all items of a thread.  Both kernels together, unique (id, time) pairs of 44 bits:
 // 4,096 pairs 12.3 us (17.9 before), 41,000 17.6 (23.1), 144,000 23.5 (32.6), 300,000 34.2 (50.5); with a power-law share of the ids
-// 14.9 (18.4), 17.2 (22.9), 25.8 (32.2), 39.5 (50.1).  One CTA, 600 / 1,500 pairs: 5.4 / 7.2 us (7.3 / 10.9), power law 8.3 / 11.5
-// (7.4 / 10.6), thirty copies of every pair 8.0 / 12.0 (7.2 / 10.9): cut into bins once or twice before they go by pivots.
+// 14.9 (18.4), 17.2 (22.9), 25.8 (32.2), 39.5 (50.1).  One CTA, 100 / 600 / 1,500 / 2,048 pairs: 4.2 / 5.6 / 7.4 / 8.5 us (4.5 / 7.3 /
+// 10.9 / 13.5); power law 4.5 / 6.9 / 10.5 / 12.8 (4.5 / 7.2 / 11.0 / 13.5), thirty copies of every pair 4.5 / 7.1 / 10.4 / 12.1 (4.5 / 7.4 /
+// 11.0 / 12.9): these go to the pivots at once (cut into bins two to four times they took 6.1 / 8.1 / 10.9 / 13.3 and 5.2 / 8.2 / 12.1 / 13.9).
 // An LSD radix sort with one kernel per 11 key bits took 25, 84 and 95 us for 4,096, 41,000 and 160,000 pairs: few CTAs with large
 // digit tables, and a dependent kernel per digit.
 #pragma once
@@ -195,10 +196,13 @@ __device__ __forceinline__ uint64_t warp_max(uint64_t x) {
 // and two loads of shared memory per item and level, and a scan of at most 2 m counters.  Copies of one key stay together until bins
 // are as narrow as positions: where crowded bins are full of them (recent neighbours of the same few nodes), or after kSpreadLevels
 // levels, it gives up and leaves the items as they were; returns whether they are sorted.
+// ALONE (a list that one CTA sorts; buckets of a longer one are cut by its splitters already): a list whose items crowd is left to the
+// pivots before anything is counted.  It shows in pairs of lanes that are close to each other: 3 % of the threads see one among five
+// others if an id holds 8 % of the list or a pair has thirty copies of 1,500, and 0.2 % of them where all are alike.
 // cnt: scratch of 2 m words, 16-byte aligned, and 16 bytes that may be written behind them; some: 2 m half words.
 constexpr int kSpreadFew = 16, kSpreadLevels = 4;         // (16, 32, 64, 128 items of a bin are left to comparisons at levels 1 - 4)
 constexpr int kSpreadCopies = 32;                         // threads that may hold a copy of a crowded bin's first key
-template <bool WIDE, int K>
+template <bool WIDE, int K, bool ALONE>
 __device__ __forceinline__ bool spread_sort(const View<WIDE>& v, uint32_t* cnt, uint16_t* some, int m, int pos_bits) {
   constexpr int R = K / 2;               // rounds of a scan: four counters per thread and round, 2 m counters
   static_assert(K % 2 == 0 && 2 * K * kThreads < (1 << 16), "items and bins are counted in 16 bits each");
@@ -221,6 +225,13 @@ __device__ __forceinline__ bool spread_sort(const View<WIDE>& v, uint32_t* cnt, 
   }
   lo = warp_min(lo);
   hi = warp_max(hi);
+  bool near = false;                     // does one of five other lanes have its first item within 1 / 4,096 of the warp's range?
+  if (ALONE) {
+    const int bits = 64 - __clzll((long long)(hi - lo));
+    const uint32_t part = tid < m ? (uint32_t)((x[0].k - lo) >> (bits > 12 ? bits - 12 : 0)) : 1u << 31 | lane;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) near |= __shfl_xor_sync(0xffffffffu, part, o) == part;
+  }
   if (lane == 0) {
     s_lo[warp] = lo;
     s_hi[warp] = hi;
@@ -228,7 +239,11 @@ __device__ __forceinline__ bool spread_sort(const View<WIDE>& v, uint32_t* cnt, 
   const int first_bits = m > 1 ? 32 - __clz(m - 1) : 0;
   int bins = 1 << first_bits;
   for (int i = tid * 4; i < bins; i += kThreads * 4) *(uint4*)(cnt + i) = make_uint4(0, 0, 0, 0);
-  __syncthreads();
+  if (ALONE) {
+    if (__syncthreads_count(near) * 32 > (m < kThreads ? m : kThreads)) return false;
+  } else {
+    __syncthreads();
+  }
   lo = warp_min(s_lo[lane & (kWarps - 1)]);
   hi = warp_max(s_hi[lane & (kWarps - 1)]);
   {
@@ -359,7 +374,7 @@ __device__ __forceinline__ bool spread_sort(const View<WIDE>& v, uint32_t* cnt, 
 
 // By counting up to MOST * kThreads items (0: not at all), otherwise, or where that gave up, by pivots: q grows with m so that ordering
 // q pivots and ranking inside groups of m / q cost about the same (measured at 300, 600, 1,600, 2,200 and 7,000 items).
-template <bool WIDE, int MOST>
+template <bool WIDE, int MOST, bool ALONE = false>
 __device__ __forceinline__ void block_sort(const View<WIDE>& v, const View<WIDE>& tmp, uint32_t* aux, uint16_t* grp, int m, int pos_bits) {
   if (m < 64) {
     rank_sort<WIDE>(v, tmp, m);
@@ -367,9 +382,9 @@ __device__ __forceinline__ void block_sort(const View<WIDE>& v, const View<WIDE>
   }
   if constexpr (MOST > 0) {
     if (m <= 4 * kThreads) {
-      if (spread_sort<WIDE, 4>(v, (uint32_t*)tmp.k, (uint16_t*)aux, m, pos_bits)) return;
+      if (spread_sort<WIDE, 4, ALONE>(v, (uint32_t*)tmp.k, (uint16_t*)aux, m, pos_bits)) return;
     } else if (m <= MOST * kThreads) {
-      if (spread_sort<WIDE, MOST>(v, (uint32_t*)tmp.k, (uint16_t*)aux, m, pos_bits)) return;
+      if (spread_sort<WIDE, MOST, ALONE>(v, (uint32_t*)tmp.k, (uint16_t*)aux, m, pos_bits)) return;
     }
   }
   if (m >= 3072) group_sort<WIDE, 8>(v, tmp, aux, grp, m);
@@ -797,7 +812,7 @@ ts_single_kernel(Source src, Sink sink, int pos_bits, int32_t* d_status) {
   for (int i = threadIdx.x; i < m; i += kThreads) {
     sm.v.set(i, make_item<WIDE>(src.key(src.load(i)), (uint32_t)i, pos_bits));
   }
-  block_sort<WIDE, kSingleMax / kThreads>(sm.v, sm.tmp, sm.aux, sm.grp, m, pos_bits);
+  block_sort<WIDE, kSingleMax / kThreads, true>(sm.v, sm.tmp, sm.aux, sm.grp, m, pos_bits);
   deliver<Sink, WIDE>(sink, sm.v, m, m, 0, 0, pos_bits, 0, true, nullptr, d_status);
   arrive(sink, nullptr, 1);
 }

@@ -66,3 +66,20 @@ def test_pairs_of_a_power_law(n, copies):
     assert np.array_equal(npy(out_id[:len(uniq)]), uniq >> 24) and np.array_equal(npy(out_ts[:len(uniq)]), uniq & (2 ** 24 - 1))
     assert np.array_equal(npy(inv_a[:cut]), inv[:cut]) and np.array_equal(npy(inv_b[:n - cut]), inv[cut:])
     st.check("unique_pairs")
+
+
+@pytest.mark.parametrize("n", [64, 65, 511, 512, 513, 1537, 2048])
+@pytest.mark.parametrize("ts_bits", [24, 40])
+@pytest.mark.parametrize("share", [0, 0.05, 0.1, 0.6, 1])
+def test_one_cta_with_items_close_to_each_other(n, ts_bits, share):
+    """A list of one CTA by counting and by pivots, on both sides of the share of one id at which it changes; keys of one word and of two."""
+    from starrygl import ops
+    rng = np.random.default_rng(n)
+    ids = np.where(rng.random(n) < share, 777, rng.integers(0, 800000, n)).astype(np.int64)
+    ts = rng.integers(0, 2 ** ts_bits if n % 2 else 50, n).astype(np.int64)
+    st = ops.StatusWord(torch.device("cuda"))
+    out_id, out_ts, inv, _, d_n = ops.unique_pairs(cu(ids), cu(ts), None, None, id_bits=20, ts_bits=ts_bits, ts_base=0, status=st)[:5]
+    uniq, want = np.unique((ids << ts_bits) | ts, return_inverse=True)
+    assert int(d_n) == len(uniq) and np.array_equal(npy(inv[:n]), want)
+    assert np.array_equal(npy(out_id[:len(uniq)]), uniq >> ts_bits) and np.array_equal(npy(out_ts[:len(uniq)]), uniq & (2 ** ts_bits - 1))
+    st.check("unique_pairs")

@@ -357,8 +357,8 @@ def batch_kernel_launches(num_nodes: int, num_roots: int, fanouts: Sequence[int]
 class BatchGraph:
     """The whole multi-hop batch construction of :func:`build_batch_async` captured once as a CUDA graph for a fixed
     number of roots, and replayed per mini-batch.  The plain call is submitted as one graph launch too and on a stream of its
-    own is the faster of the two (4,096 roots uniform [10, 10]: 0.120 ms a batch, 0.130 as a replay); a replay costs the host one
-    launch and two copies and is for callers that drive several batches side by side (four in flight: 0.079 ms a batch).
+    own is the faster of the two (4,096 roots uniform [10, 10]: 0.103 ms a batch, 0.111 as a replay); a replay costs the host one
+    launch and two copies and is for callers that drive several batches side by side (four in flight: 0.068 ms a batch).
 
     The result tensors are the same objects for every batch: consume (or copy) a result before the next ``run``.
     """

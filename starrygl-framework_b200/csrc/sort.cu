@@ -38,6 +38,7 @@ struct RawSink {
 
 // first pass over pairs without a payload of their own
 struct IotaItems {
+  static constexpr bool kChecked = false;
   const uint64_t* keys;
   int64_t n_cap;
   const int64_t* d_n;

@@ -1,7 +1,8 @@
 // T-CSR construction: rows keyed by node id, inside a row ascending timestamp, ties in input order.
 //
-//   1. tcsr_scan_kernel   one pass over the input: timestamp range, keys out of range, is it in time order already, do
-//                         neighbour and edge id fit 32 bits each; the last CTA hands the answer to the host
+//   1. tcsr_scan_kernel   one pass over keys and times: timestamp range, keys out of range, is it in time order already, do the
+//                         first neighbour and edge ids fit 32 bits each (the sort's counts look at all of them); the last CTA
+//                         hands the answer to the host
 //   2. stable sort by (node << ts_bits) | (ts - ts_min), only the populated bits:
 //        up to tilesort::kMaxItems edges   the mini-batch sort, whose sink writes the rows
 //        more                              radix passes (lsd.cuh).  Neighbour and edge id travel as the payload (8 bytes) when
@@ -13,6 +14,8 @@
 //      prefix sum); with positions as payload tcsr_emit_gather_kernel does both
 //
 // 50 M edges, 1 M nodes in no particular order: bound by the radix passes' traffic, 264 B per edge.
+#include <stddef.h>
+
 #include "chain.cuh"
 #include "lsd.cuh"
 
@@ -45,7 +48,7 @@ tcsr_scan_kernel(const int64_t* __restrict__ key, const int64_t* __restrict__ nb
     early = ~u > early ? ~u : early;
     if (i + 1 < m) unordered |= ts[i + 1] < t ? 1u : 0u;
     bad += (k < 0 || k >= num_nodes) ? 1u : 0u;
-    if (check_ids) {
+    if (check_ids && i < stride) {       // (a look at some; the counts of the sort see all of them)
       wide |= (unsigned long long)nbr[i];
       if (eid) wide |= (unsigned long long)eid[i];
     }
@@ -168,9 +171,15 @@ struct EdgeSink {
 
 // ---- above: items of the first radix pass ---------------------------------------------------------------------------------
 struct EdgePairs {                    // neighbour and edge id as payload
+  static constexpr bool kChecked = true;
   EdgeKey k;
   const int64_t *nbr, *eid;
   int64_t m;
+  InputScan* scan;
+  __device__ __forceinline__ unsigned long long check(int64_t i) const { return (unsigned long long)nbr[i] | (unsigned long long)(eid ? eid[i] : 0); }
+  __device__ __forceinline__ void checked(unsigned long long bits) const {
+    if ((bits >> 32) != 0) atomicOr(&scan->flags, kWideIds);
+  }
   __device__ __forceinline__ int64_t begin() const { return m; }
   __device__ __forceinline__ uint64_t key(int64_t i) const { return k.of(i); }
   __device__ __forceinline__ uint64_t val(int64_t i) const {
@@ -179,6 +188,7 @@ struct EdgePairs {                    // neighbour and edge id as payload
 };
 
 struct EdgePositions {                // position as payload
+  static constexpr bool kChecked = false;
   EdgeKey k;
   int64_t m;
   __device__ __forceinline__ int64_t begin() const { return m; }
@@ -339,57 +349,63 @@ extern "C" int sgl_tcsr_build_fenced(int64_t num_nodes, int64_t m, const int64_t
   if (small && ts_bits + id_bits + pos_bits <= 64) return SGL_OK;
   const EdgeKey k{key, ts, ts_min, ts_bits};
   const int grid = stream_grid(m, 256 * 4, 8);
-  LaunchScope scope(stream);
-  WsCarver c(rest, rest_bytes);
-  if (ts_bits + id_bits > 64) {
-    // two stable rounds: by timestamp, then by node id
-    uint64_t *k0 = c.take<uint64_t>(m), *k1 = c.take<uint64_t>(m);
-    uint32_t *v0 = c.take<uint32_t>(m), *v1 = c.take<uint32_t>(m);
-    const size_t sort_bytes = radix_sort_ws_bytes(m);
-    char* sort_ws = c.take<char>(sort_bytes);
-    SGL_REQUIRE(c.ok(), SGL_ERR_WORKSPACE, "tcsr_build: workspace too small");
-    SGL_CHECK_RC(launch(tcsr_round_keys_kernel, grid, 256, 0, stream, k, nullptr, m, k0));
-    int in_alt = 0;
-    SGL_CHECK_RC(radix_sort_pairs(k0, v0, k1, v1, m, nullptr, ts_bits, true, &in_alt, d_status, sort_ws, sort_bytes, stream));
-    uint32_t *perm = in_alt ? v1 : v0, *other = in_alt ? v0 : v1;
-    uint64_t *kk = in_alt ? k1 : k0, *kk_alt = in_alt ? k0 : k1;     // (the sorted timestamps are no longer needed)
-    SGL_CHECK_RC(launch(tcsr_round_keys_kernel, grid, 256, 0, stream, k, perm, m, kk));
-    SGL_CHECK_RC(radix_sort_pairs(kk, perm, kk_alt, other, m, nullptr, id_bits, false, &in_alt, d_status, sort_ws, sort_bytes, stream));
-    SGL_CHECK_RC(launch(tcsr_emit_gather_kernel, grid, 256, 0, stream, d_scan, in_alt ? kk_alt : kk, in_alt ? other : perm, 0, k, nbr, eid, m,
-                        num_nodes, indptr, out_nbr, out_ts, out_eid, out_perm));
-  } else if (small) {
-    const ScannedRange known{nullptr, 0, 0};
-    SGL_CHECK_RC(sort_list(EdgeSource{k, m, known}, EdgeSink{k, nbr, eid, num_nodes, indptr, out_nbr, out_ts, out_eid, out_perm, known, false}, m,
-                           ts_bits + id_bits, rest, rest_bytes, nullptr, stream));
-  } else {
-    const int first_bit = flags & kUnordered ? 0 : (ts_bits < 56 ? ts_bits : 56);   // in time order: only the node bits are left
-    bool in_first;
-    unsigned int* gave_up;
-    if (!(flags & kWideIds) && out_perm == nullptr && num_nodes <= ((int64_t)1 << 32)) {
-      uint64_t *k1 = c.take<uint64_t>(m), *k0 = c.take<uint64_t>(m), *v1 = c.take<uint64_t>(m), *v0 = c.take<uint64_t>(m);
-      uint32_t* node = (uint32_t*)(lsd_passes(first_bit, ts_bits + id_bits) & 1 ? k1 : k0);      // the last pass's own array
-      const EdgeOut out{k, node, out_nbr, out_ts, out_eid};
-      SGL_CHECK_RC((lsd_sort<uint64_t, EdgePairs>(EdgePairs{k, nbr, eid, m}, k1, v1, k0, v0, m, nullptr, nullptr, first_bit, ts_bits + id_bits, out,
-                                                  &in_first, &gave_up, c, d_status, stream)));
-      SGL_CHECK_RC(launch(tcsr_rows_kernel, stream_grid(m, 256 * 4, 8), 256, 0, stream, d_scan, node, m, num_nodes, indptr));
+  // neighbour and edge id as payload, as far as the scan saw; the sort's counts see all ids, and where some do not fit everything is done again
+  bool narrow = !small && ts_bits + id_bits <= 64 && !(flags & kWideIds) && out_perm == nullptr && num_nodes <= ((int64_t)1 << 32);
+  for (;;) {
+    LaunchScope scope(stream);
+    WsCarver c(rest, rest_bytes);
+    if (ts_bits + id_bits > 64) {
+      // two stable rounds: by timestamp, then by node id
+      uint64_t *k0 = c.take<uint64_t>(m), *k1 = c.take<uint64_t>(m);
+      uint32_t *v0 = c.take<uint32_t>(m), *v1 = c.take<uint32_t>(m);
+      const size_t sort_bytes = radix_sort_ws_bytes(m);
+      char* sort_ws = c.take<char>(sort_bytes);
+      SGL_REQUIRE(c.ok(), SGL_ERR_WORKSPACE, "tcsr_build: workspace too small");
+      SGL_CHECK_RC(launch(tcsr_round_keys_kernel, grid, 256, 0, stream, k, nullptr, m, k0));
+      int in_alt = 0;
+      SGL_CHECK_RC(radix_sort_pairs(k0, v0, k1, v1, m, nullptr, ts_bits, true, &in_alt, d_status, sort_ws, sort_bytes, stream));
+      uint32_t *perm = in_alt ? v1 : v0, *other = in_alt ? v0 : v1;
+      uint64_t *kk = in_alt ? k1 : k0, *kk_alt = in_alt ? k0 : k1;     // (the sorted timestamps are no longer needed)
+      SGL_CHECK_RC(launch(tcsr_round_keys_kernel, grid, 256, 0, stream, k, perm, m, kk));
+      SGL_CHECK_RC(radix_sort_pairs(kk, perm, kk_alt, other, m, nullptr, id_bits, false, &in_alt, d_status, sort_ws, sort_bytes, stream));
+      SGL_CHECK_RC(launch(tcsr_emit_gather_kernel, grid, 256, 0, stream, d_scan, in_alt ? kk_alt : kk, in_alt ? other : perm, 0, k, nbr, eid, m,
+                          num_nodes, indptr, out_nbr, out_ts, out_eid, out_perm));
+    } else if (small) {
+      const ScannedRange known{nullptr, 0, 0};
+      SGL_CHECK_RC(sort_list(EdgeSource{k, m, known}, EdgeSink{k, nbr, eid, num_nodes, indptr, out_nbr, out_ts, out_eid, out_perm, known, false}, m,
+                             ts_bits + id_bits, rest, rest_bytes, nullptr, stream));
     } else {
-      uint64_t *k1 = c.take<uint64_t>(m), *k0 = c.take<uint64_t>(m);
-      uint32_t *v1 = c.take<uint32_t>(m), *v0 = c.take<uint32_t>(m);
-      SGL_CHECK_RC((lsd_sort<uint32_t, EdgePositions>(EdgePositions{k, m}, k1, v1, k0, v0, m, nullptr, nullptr, first_bit, ts_bits + id_bits,
-                                                      ArrayOut<uint32_t>{}, &in_first, &gave_up, c, d_status, stream)));
-      SGL_CHECK_RC(launch(tcsr_emit_gather_kernel, grid, 256, 0, stream, d_scan, in_first ? k1 : k0, in_first ? v1 : v0, 1, k, nbr, eid, m, num_nodes,
-                          indptr, out_nbr, out_ts, out_eid, out_perm));
+      const int first_bit = flags & kUnordered ? 0 : (ts_bits < 56 ? ts_bits : 56);   // in time order: only the node bits are left
+      bool in_first;
+      unsigned int* gave_up;
+      if (narrow) {
+        uint64_t *k1 = c.take<uint64_t>(m), *k0 = c.take<uint64_t>(m), *v1 = c.take<uint64_t>(m), *v0 = c.take<uint64_t>(m);
+        uint32_t* node = (uint32_t*)(lsd_passes(first_bit, ts_bits + id_bits) & 1 ? k1 : k0);      // the last pass's own array
+        const EdgeOut out{k, node, out_nbr, out_ts, out_eid};
+        SGL_CHECK_RC((lsd_sort<uint64_t, EdgePairs>(EdgePairs{k, nbr, eid, m, d_scan}, k1, v1, k0, v0, m, nullptr, nullptr, first_bit, ts_bits + id_bits, out,
+                                                    &in_first, &gave_up, c, d_status, stream)));
+        SGL_CHECK_RC(launch(tcsr_rows_kernel, stream_grid(m, 256 * 4, 8), 256, 0, stream, d_scan, node, m, num_nodes, indptr));
+      } else {
+        uint64_t *k1 = c.take<uint64_t>(m), *k0 = c.take<uint64_t>(m);
+        uint32_t *v1 = c.take<uint32_t>(m), *v0 = c.take<uint32_t>(m);
+        SGL_CHECK_RC((lsd_sort<uint32_t, EdgePositions>(EdgePositions{k, m}, k1, v1, k0, v0, m, nullptr, nullptr, first_bit, ts_bits + id_bits,
+                                                        ArrayOut<uint32_t>{}, &in_first, &gave_up, c, d_status, stream)));
+        SGL_CHECK_RC(launch(tcsr_emit_gather_kernel, grid, 256, 0, stream, d_scan, in_first ? k1 : k0, in_first ? v1 : v0, 1, k, nbr, eid, m, num_nodes,
+                            indptr, out_nbr, out_ts, out_eid, out_perm));
+      }
     }
+    if (out_fence && num_nodes > 0) SGL_CHECK_RC(launch_fence(indptr, out_ts, num_nodes, m, out_fence, {nullptr, 0, 0}, stream));
+    if (small) return scope.submit();
+    // The radix passes wait for each other's tiles, for a limited time: the graph is handed out once they are known to have come through.
+    int64_t* const result = h + 8;
+    constexpr int kStatus = (offsetof(InputScan, status) - offsetof(InputScan, flags)) / 8;
+    SGL_CHECK_RC(export_words((const int64_t*)&d_scan->flags, result, kStatus + 1, stream));
+    SGL_CHECK_RC(scope.submit());
+    SGL_CHECK_RC(sgl_wait_word(result + kStatus + 1, 1, stream));
+    SGL_REQUIRE(result[kStatus] == 0, SGL_ERR_CUDA, "tcsr_build: a look-back over the tiles of the sort ran into its time limit");
+    if (!narrow || !(result[0] & (int64_t)kWideIds)) return SGL_OK;
+    narrow = false;
   }
-  if (out_fence && num_nodes > 0) SGL_CHECK_RC(launch_fence(indptr, out_ts, num_nodes, m, out_fence, {nullptr, 0, 0}, stream));
-  if (small) return scope.submit();
-  // The radix passes wait for each other's tiles, for a limited time: the graph is handed out once they are known to have come through.
-  int64_t* const result = h + 8;
-  SGL_CHECK_RC(export_words((const int64_t*)&d_scan->status, result, 1, stream));
-  SGL_CHECK_RC(scope.submit());
-  SGL_CHECK_RC(sgl_wait_word(result + 1, 1, stream));
-  SGL_REQUIRE(result[0] == 0, SGL_ERR_CUDA, "tcsr_build: a look-back over the tiles of the sort ran into its time limit");
-  return SGL_OK;
 }
 
 extern "C" int sgl_tcsr_build(int64_t num_nodes, int64_t m, const int64_t* key, const int64_t* nbr, const int64_t* ts, const int64_t* eid,

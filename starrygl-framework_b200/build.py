@@ -1,4 +1,5 @@
-"""Build libsgl_b200.so (the C-ABI CUDA library) in-tree with nvcc for sm_100a.
+"""Build libsgl_b200.so (the C-ABI CUDA library) in-tree with nvcc for sm_100a, and _sgl_host.so (the Python side of its hot calls)
+with g++ against the installed torch.
 
     python starrygl-framework_b200/build.py [--force] [--verbose]
 
@@ -7,35 +8,49 @@ The shared object lands in starrygl-framework_b200/lib/.  nvcc cross-compiles, s
 import os
 import subprocess
 import sys
+import sysconfig
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 SRC = os.path.join(HERE, "csrc")
 OUT_DIR = os.path.join(HERE, "lib")
 OUT = os.path.join(OUT_DIR, "libsgl_b200.so")
+HOST = os.path.join(OUT_DIR, "_sgl_host.so")
 SOURCES = ["api.cu", "sort.cu", "tcsr.cu", "sampler.cu", "relabel.cu", "gather.cu", "comm.cu", "p2p_route.cu", "plan.cu", "mail.cu", "slice.cu", "batch.cu", "launch.cu", "query.cu"]
 FLAGS = ["-O3", "--threads", "0", "-std=c++17", "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "--expt-relaxed-constexpr",
          "-Xcompiler", "-fPIC", "-shared", "-cudart", "shared"]
 
 
-def _stale():
-    if not os.path.exists(OUT):
+def _stale(out, deps):
+    if not os.path.exists(out):
         return True
-    t = os.path.getmtime(OUT)
-    deps = [os.path.join(SRC, f) for f in os.listdir(SRC)] + [os.path.join(HERE, "..", "include", "sgl_b200.h"), __file__]
-    return any(os.path.getmtime(d) > t for d in deps)
+    t = os.path.getmtime(out)
+    return any(os.path.getmtime(d) > t for d in (*deps, os.path.join(HERE, "..", "include", "sgl_b200.h"), __file__))
 
 
-def build(force=False, verbose=False):
-    if not force and not _stale():
-        return OUT
-    os.makedirs(OUT_DIR, exist_ok=True)
-    nvcc = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
-    cmd = [nvcc] + FLAGS + (["-Xptxas", "-v"] if verbose else []) + [os.path.join(SRC, s) for s in SOURCES] + ["-ldl", "-o", OUT]
+def _run(cmd, what, verbose):
     r = subprocess.run(cmd, capture_output=True, text=True)
     if verbose or r.returncode != 0:
         sys.stderr.write(r.stdout + r.stderr)
     if r.returncode != 0:
-        raise RuntimeError("nvcc failed building libsgl_b200.so")
+        raise RuntimeError(f"building {what} failed")
+
+
+def build(force=False, verbose=False):
+    os.makedirs(OUT_DIR, exist_ok=True)
+    kernels = [os.path.join(SRC, f) for f in os.listdir(SRC) if f.endswith((".cu", ".cuh"))]
+    if force or _stale(OUT, kernels):
+        nvcc = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
+        _run([nvcc] + FLAGS + (["-Xptxas", "-v"] if verbose else []) + [os.path.join(SRC, s) for s in SOURCES] + ["-ldl", "-o", OUT],
+             "libsgl_b200.so", verbose)
+    host = os.path.join(SRC, "host.cpp")
+    if force or _stale(HOST, [host]):
+        import torch
+        at = os.path.dirname(torch.__file__)
+        inc = [os.path.join(at, "include"), os.path.join(at, "include", "torch", "csrc", "api", "include"), "/usr/local/cuda/include"]
+        _run([os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden",
+              f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", *[x for i in inc for x in ("-isystem", i)],
+              "-I", sysconfig.get_paths()["include"], host, "-o", HOST, "-L", OUT_DIR, "-lsgl_b200", "-L", os.path.join(at, "lib"),
+              "-ltorch_python", "-ltorch", "-ltorch_cpu", "-lc10", "-lc10_cuda", "-Wl,-rpath,$ORIGIN"], "_sgl_host.so", verbose)
     return OUT
 
 

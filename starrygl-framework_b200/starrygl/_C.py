@@ -6,13 +6,16 @@ worker threads the way the reference's pybind module is (csrc/srcs/starrygl/expo
 ``py::gil_scoped_release`` on every heavy binding).
 """
 import ctypes as C
+import importlib.util
 import os
+import sys
 import threading
 
 import torch
 
 _PKG_ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 LIB_PATH = os.path.join(_PKG_ROOT, "lib", "libsgl_b200.so")
+HOST_PATH = os.path.join(_PKG_ROOT, "lib", "_sgl_host.so")
 
 SGL_DEV_BITS = {1: "node id out of range", 2: "timestamp outside the declared window", 4: "row index out of range",
                 8: "output capacity exceeded", 16: "device-side wait timed out",
@@ -20,8 +23,8 @@ SGL_DEV_BITS = {1: "node id out of range", 2: "timestamp outside the declared wi
 POLICY = {"recent": 0, "uniform": 1}
 GATHER_MODE = {"auto": 0, "vec": 1, "bulk": 2}
 
-_lib = None
-_lock = threading.Lock()
+_lib = _host = None
+_lock = threading.RLock()
 
 _vp, _i64, _i32, _u64, _u32, _sz = C.c_void_p, C.c_int64, C.c_int, C.c_uint64, C.c_uint32, C.c_size_t
 
@@ -168,6 +171,24 @@ class SglError(RuntimeError):
     pass
 
 
+def host():
+    """The extension module over the same library (csrc/host.cpp) for the calls that every mini-batch makes: its functions take tensors
+    and integers, raise by themselves, and cost a fraction of a ctypes call."""
+    global _host
+    if _host is None:
+        with _lock:
+            if _host is None:
+                lib()
+                if not os.path.exists(HOST_PATH):
+                    raise RuntimeError(f"{HOST_PATH} is missing: build it with `python starrygl-framework_b200/build.py`")
+                spec = importlib.util.spec_from_file_location("_sgl_host", HOST_PATH)
+                m = importlib.util.module_from_spec(spec)
+                spec.loader.exec_module(m)
+                m.bind(SglError, sys.modules[__name__])
+                _host = m
+    return _host
+
+
 def check(rc):
     if rc != 0:
         raise SglError(f"libsgl_b200 error {rc}: {lib().sgl_last_error().decode()}")
@@ -291,7 +312,7 @@ COUNTS = CountRing()
 def read_words(t, count):
     """The first ``count`` int64 words of a device tensor, as a list (waits for the current stream's work on them)."""
     buf = (C.c_int64 * count)()
-    check(lib().sgl_read_back(t.data_ptr(), buf, 8 * count, stream_ptr()))
+    host().sgl_read_back(t.data_ptr(), C.addressof(buf), 8 * count, stream_ptr())
     return list(buf)
 
 

@@ -49,6 +49,10 @@ class PrefetchedBatch:
         return int(self.offsets[self.n_roots].item())
 
 
+# places among the arguments of sgl_prefetch_batch
+_HOST, _DEVICE, _COUNT, _SEQ = slice(0, 2), slice(8, 10), 10, slice(34, 36)
+
+
 class HostToDevicePrefetcher:
     def __init__(self, loader: Iterable, g: ops.TCSR, edge_feats: Optional[torch.Tensor], fanout: int,
                  policy: str = "recent", max_roots: int = 4096, depth: int = 4, device=None, **sampler_options):
@@ -59,26 +63,22 @@ class HostToDevicePrefetcher:
         self._held = [deque() for _ in range(self.depth)]      # per slot: (event behind a batch, its inputs), oldest first
         self._spare = [[] for _ in range(self.depth)]          # events of batches that are done
         self._totals = torch.zeros(2 * self.depth, dtype=torch.int64).pin_memory()   # per slot: edges, sequence number
-        self._seq, self._fn = 0, _C.lib().sgl_prefetch_batch
+        self._seq, self._fn = 0, _C.host().sgl_prefetch_batch
         self._bound = [None] * self.depth
 
     def _bind(self, slot):
-        """Everything of a slot's foreign call that does not change from batch to batch."""
-        v, p, g = C.c_void_p, self.pipes[slot], self.pipes[slot].g
-        a = p.args
+        """The arguments of a slot's foreign call, those that change from batch to batch at their places (_HOST, _DEVICE, _COUNT, _SEQ)."""
+        p, g = self.pipes[slot], self.pipes[slot].g
+        a, table = p.args, p.feats
         addr = self._totals.data_ptr() + 16 * slot
         words = (C.c_int64 * 2).from_address(addr)
-        var = v(0), v(0), v(0), v(0), C.c_int64(0), C.c_int64(0), v(0)       # host roots / times, targets / times, n, seq, consumer
-        table = p.feats
-        args = [var[0], var[1], v(g.indptr.data_ptr()), v(g.nbr.data_ptr()), v(g.ts.data_ptr()), v(g.eid.data_ptr()),
-                v(g.fence.data_ptr() if g.fence is not None else 0), C.c_int64(g.num_nodes), var[2], var[3], var[4], C.c_int(p.k),
-                C.c_int(a["pol"]), C.c_int(a["eq"]), C.c_int64(a["off"]), C.c_int(a["keep"]), C.c_uint64(a["seed"]), C.c_uint32(0),
-                v(p.nbr.data_ptr()), v(p.dst.data_ptr()), v(p.ts.data_ptr()), v(p.dt.data_ptr()), v(p.eid.data_ptr()),
-                v(p.offsets.data_ptr()), v(0 if table is None else table.data_ptr()), C.c_int64(0 if table is None else table.shape[0]),
-                C.c_int64(0 if table is None else p.row_bytes), C.c_int64(0 if table is None else p.src_pitch),
-                v(0 if table is None else p.out_feats.data_ptr()), C.c_int(p.mode), v(p.status.ptr()), v(p.ws.data_ptr()),
-                C.c_size_t(p.ws.numel()), v(addr), var[5], var[6], v(p.stream.cuda_stream)]
-        return args, var, addr, words
+        args = [0, 0, g.indptr.data_ptr(), g.nbr.data_ptr(), g.ts.data_ptr(), g.eid.data_ptr(), g.fence.data_ptr() if g.fence is not None else 0,
+                g.num_nodes, 0, 0, 0, p.k, a["pol"], a["eq"], a["off"], a["keep"], a["seed"], 0, p.nbr.data_ptr(), p.dst.data_ptr(),
+                p.ts.data_ptr(), p.dt.data_ptr(), p.eid.data_ptr(), p.offsets.data_ptr(), 0 if table is None else table.data_ptr(),
+                0 if table is None else table.shape[0], 0 if table is None else p.row_bytes, 0 if table is None else p.src_pitch,
+                0 if table is None else p.out_feats.data_ptr(), p.mode, p.status.ptr(), p.ws.data_ptr(), p.ws.numel(), addr, 0, 0,
+                p.stream.cuda_stream]
+        return args, addr, words
 
     def _submit(self, slot, roots, root_ts):
         pipe, st = self.pipes[slot], self.streams[slot]
@@ -90,14 +90,13 @@ class HostToDevicePrefetcher:
             raise _C.SglError("prefetcher: roots on the GPU are int64 and come with as many int64 query times")
         if self._bound[slot] is None:
             self._bound[slot] = self._bind(slot)
-        args, (h_r, h_t, d_r, d_t, c_n, c_seq, c_cons), addr, words = self._bound[slot]
-        h_r.value = h_t.value = None
-        d_r.value, d_t.value = pipe.roots.data_ptr(), pipe.root_ts.data_ptr()
+        args, addr, words = self._bound[slot]
+        on_host, on_device = (0, 0), (pipe.roots.data_ptr(), pipe.root_ts.data_ptr())
         roots, root_ts = roots.contiguous(), root_ts.contiguous()
         if as_is and roots.is_cuda and root_ts.is_cuda:
-            d_r.value, d_t.value = roots.data_ptr(), root_ts.data_ptr()
+            on_device = roots.data_ptr(), root_ts.data_ptr()
         elif as_is and roots.is_pinned() and root_ts.is_pinned():
-            h_r.value, h_t.value = roots.data_ptr(), root_ts.data_ptr()
+            on_host = roots.data_ptr(), root_ts.data_ptr()
         else:                             # pageable, of another type, or one time for all: staged by a copy, behind what the consumer still does with the slot
             st.wait_stream(torch.cuda.current_stream())
             with torch.cuda.stream(st):
@@ -114,11 +113,11 @@ class HostToDevicePrefetcher:
                 spare.append(held.popleft()[0])
         ready = spare.pop() if spare else torch.cuda.Event()
         self._seq += 1
-        c_n.value, c_seq.value, c_cons.value = n, self._seq, _C.stream_ptr()
+        args[_HOST], args[_DEVICE], args[_COUNT], args[_SEQ] = on_host, on_device, n, (self._seq, _C.stream_ptr())
         # The call orders the slot's reuse behind everything the consumer has enqueued so far on its stream: the work on the
         # batch that occupied this slot (handed out just before) and the kernels that produced ``roots``.  The batch submitted
         # now is only needed ``depth`` requests later, so this does not stall the consumer.
-        _C.check(self._fn(*args))
+        self._fn(*args)
         ready.record(st)
         held.append((ready, (roots, root_ts)))
         return PrefetchedBatch(pipe, n, ready, (addr, words, self._seq, self._totals))

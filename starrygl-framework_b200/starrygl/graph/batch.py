@@ -54,6 +54,7 @@ class _Plan:
                 start[s] = -1 - raw
                 raw += self.size[s]
         self.start, self.at, self.words, self.raw_words = start, self.places(*start), words, raw
+        self.fan_at, self.at_at = C.addressof(self.fan), C.addressof(self.at)
         self.shared = 8 * words <= _SHARED_MOST
 
 
@@ -70,6 +71,9 @@ def _plan(n, fanouts) -> _Plan:
     return p
 
 
+_HOP = ("indptr", "indices", "eid", "edge_ts", "edge_dt", "gids", "ts")     # of a layer behind the roots
+
+
 class _MetaStatus(ops.StatusWord):
     """The status word of a batch that came without one: the last word of its meta block."""
 
@@ -83,9 +87,16 @@ class DeviceBatch:
 
     def __init__(self, g, n, fanouts, plan, results, raw, meta, status):
         self.g, self.n, self.fanouts = g, n, list(fanouts)
-        self._plan, self._results, self._raw, self._meta, self._status = plan, results, raw, meta, status
+        self._plan, self._results, self._raw, self._own_meta, self._status = plan, results, raw, meta, status
         self._shared = not isinstance(results, dict)
         self._layers = None
+
+    @property
+    def _meta(self):
+        """Counts and status word: the block that was given, or the end of the raw arrays."""
+        if self._own_meta is None:
+            self._own_meta = self._raw[self._raw.numel() - (2 + 2 * len(self.fanouts)):]
+        return self._own_meta
 
     @property
     def status(self):
@@ -155,23 +166,24 @@ class DeviceBatch:
             raise _C.SglError(f"build_batch: device status {bits} ({_C.decode_status(bits)})")
         return self._trim(host)
 
-    def _cut(self):
-        """View of the first ``count`` values of a section, as a function."""
+    def _cuts(self, pieces):
+        """Views of the first ``count`` values of sections, (section, count, fp32?) thrice each."""
         if not self._shared:
-            return self._view
-        # (a strided view of the whole costs half of a slice, and its float form one conversion instead of two views each)
-        t, at, cut = self._results, self._plan.start, torch.as_strided
-        f = t.view(torch.float32)
-
-        def v(section, count, floats=False):
-            return cut(f, (count,), (1,), 2 * at[section]) if floats else cut(t, (count,), (1,), at[section])
-        return v
+            return [self._view(*pieces[i:i + 3]) for i in range(0, len(pieces), 3)]
+        at = self._plan.start
+        return _C.host().cuts(self._results, *[at[x] if i % 3 == 0 else x for i, x in enumerate(pieces)])
 
     def _trim(self, host):
         self._host = host
-        v = self._cut()
-        out, prev_n = [{"gids": v(0, host[0]), "ts": v(1, host[0]), "inv_map": v(2, self.n)}], host[0]
-        for l in range(len(self.fanouts)):
+        hops = len(self.fanouts)
+        if 0 not in host[1:2 * hops + 1:2]:
+            out, last = self._trim_but_last(host)
+            if hops:
+                out[-1]["gids"], out[-1]["ts"] = last(host[-1])
+            return out
+        first = self._cuts((0, host[0], 0, 1, host[0], 0, 2, self.n, 0))
+        out, prev_n = [dict(zip(("gids", "ts", "inv_map"), first))], host[0]
+        for l in range(hops):
             n_edges, n_next = host[1 + 2 * l], host[2 + 2 * l]
             if n_edges == 0 and not self._any_target_has_edges(l, out):
                 # the reference emits an empty layer and stops when no target has any edge at all
@@ -181,33 +193,35 @@ class DeviceBatch:
                             "eid": z, "edge_ts": z, "edge_dt": torch.zeros(0, dtype=torch.float32, device=self.g.device),
                             "gids": z, "ts": z})
                 break
-            out.append(self._hop(v, l, prev_n, n_edges))
-            out[-1]["gids"], out[-1]["ts"] = v(3 + 14 * l + 6, n_next), v(3 + 14 * l + 7, n_next)
+            out.append(dict(zip(_HOP, self._cuts(self._hop(l, prev_n, n_edges) + (3 + 14 * l + 6, n_next, 0, 3 + 14 * l + 7, n_next, 0)))))
             prev_n = n_next
         return out
 
     @staticmethod
-    def _hop(v, l, prev_n, n_edges):
+    def _hop(l, prev_n, n_edges):
         b = 3 + 14 * l
         # (the first hop's edges are in CSC order as they were sampled, see sgl_build_batch)
-        ip, ix, ts, dt, ei = (5, 8, 2, 3, 4) if l == 0 else (9, 10, 11, 12, 13)
-        return {"indptr": v(b + ip, prev_n + 1), "indices": v(b + ix, n_edges), "eid": v(b + ei, n_edges), "edge_ts": v(b + ts, n_edges),
-                "edge_dt": v(b + dt, n_edges, True)}
+        ip, ix, ts, dt, ei = (b + 5, b + 8, b + 2, b + 3, b + 4) if l == 0 else (b + 9, b + 10, b + 11, b + 12, b + 13)
+        return ip, prev_n + 1, 0, ix, n_edges, 0, ei, n_edges, 0, ts, n_edges, 0, dt, n_edges, 1
 
     def _trim_but_last(self, host):
-        """The layers as :meth:`_trim` returns them without the last list, whose length ``host`` does not say yet, and how to cut that;
-        None where a hop has no edges."""
+        """The layers as :meth:`_trim` returns them without the last list, whose length ``host`` does not say yet, and a function of
+        that length for its two arrays; None where a hop has no edges."""
         hops = len(self.fanouts)
         if 0 in host[1:2 * hops:2]:
             return None
-        v = self._cut()
-        out, prev_n = [{"gids": v(0, host[0]), "ts": v(1, host[0]), "inv_map": v(2, self.n)}], host[0]
+        pieces, prev_n = (0, host[0], 0, 1, host[0], 0, 2, self.n, 0), host[0]
         for l in range(hops):
-            out.append(self._hop(v, l, prev_n, host[1 + 2 * l]))
+            pieces += self._hop(l, prev_n, host[1 + 2 * l])
             if l + 1 < hops:
                 prev_n = host[2 + 2 * l]
-                out[-1]["gids"], out[-1]["ts"] = v(3 + 14 * l + 6, prev_n), v(3 + 14 * l + 7, prev_n)
-        return out, v
+                pieces += (3 + 14 * l + 6, prev_n, 0, 3 + 14 * l + 7, prev_n, 0)
+        got = self._cuts(pieces)
+        out = [dict(zip(("gids", "ts", "inv_map"), got))]
+        for l in range(hops):
+            out.append(dict(zip(_HOP if l + 1 < hops else _HOP[:5], got[3 + 7 * l:10 + 7 * l])))
+        b = 3 + 14 * (hops - 1)
+        return out, lambda n: self._cuts((b + 6, n, 0, b + 7, n, 0))
 
     def _any_target_has_edges(self, l, out):
         tgt = out[0]["gids"] if l == 0 else self._view(3 + 14 * (l - 1), self._host[1 + 2 * (l - 1)])
@@ -223,37 +237,22 @@ def _enqueue(g, roots, root_ts, fanouts, policy, lo, hi, equal_root_time, allowe
     that receives all but the last while the last list is merged;
     ``meta``: block of 2 + 2 * hops device words for the counts and the status (default: behind the raw arrays);
     ``together``: one allocation for the results whatever their size (for callers that keep none of them)."""
-    roots, root_ts = ops._i64(roots), ops._i64(root_ts)
-    n = roots.numel()
-    if root_ts.numel() != n:
-        raise _C.SglError("build_batch: roots and root_ts differ in length")
+    n, hops = roots.numel(), len(fanouts)
     plan = _plan(n, fanouts)
-    dev = g.device
-    extra = 2 + 2 * len(fanouts) if meta is None else 0
-    if plan.whole:
-        results = raw = torch.empty(plan.words + extra, dtype=torch.int64, device=dev)
-    else:
-        results, raw = None, torch.empty(plan.raw_words + extra, dtype=torch.int64, device=dev)
-    if meta is None:
-        meta = raw[raw.numel() - extra:]
-    if plan.shared or together:
-        if results is None:
-            results = torch.empty(plan.words, dtype=torch.int64, device=dev)
-        at, base = plan.at, results.data_ptr()
-    else:
-        results = {s: torch.empty(plan.size[s], dtype=torch.int64, device=dev) for s in plan.kept}
-        at, base = plan.places(*plan.at), None
-        for s, t in results.items():
-            at[s] = t.data_ptr() // 8
-    sp = _C.stream_ptr()
-    ws = _C.WORKSPACE.get(plan.ws_bytes, dev, sp)
-    _C.check(_C.lib().sgl_build_batch_staged(
-        g.indptr.data_ptr(), g.nbr.data_ptr(), g.ts.data_ptr(), g.eid.data_ptr(), None if g.fence is None else g.fence.data_ptr(),
-        g.num_nodes, _C.ptr(roots), _C.ptr(root_ts), n, plan.fan, len(fanouts),
-        _C.POLICY[policy] if isinstance(policy, str) else int(policy), int(bool(equal_root_time)), int(allowed_offset),
-        int(seed) & (2 ** 64 - 1), ops.bits_for(g.num_nodes - 1), ops.bits_for(hi - lo), lo, at, base, raw.data_ptr(), meta.data_ptr(),
-        None if status is None else status.ptr(), host, early, ws.data_ptr(), ws.numel(), None if side is None else side.cuda_stream, sp))
-    return DeviceBatch(g, n, fanouts, plan, results, raw, meta, status)
+    at, words, kept = plan.at_at, plan.words, None
+    if not (plan.whole or plan.shared or together):
+        kept = {s: torch.empty(plan.size[s], dtype=torch.int64, device=g.device) for s in plan.kept}
+        places, words = plan.places(*plan.at), 0
+        for s, t in kept.items():
+            places[s] = t.data_ptr() // 8
+        at = C.addressof(places)
+    results, raw = _C.host().build_batch(
+        g.indptr, g.nbr, g.ts, g.eid, g.fence, g.num_nodes, roots, root_ts, plan.fan_at, hops,
+        _C.POLICY[policy] if isinstance(policy, str) else int(policy), bool(equal_root_time), int(allowed_offset), int(seed),
+        ops.bits_for(g.num_nodes - 1), ops.bits_for(hi - lo), lo, at, words, -1 if plan.whole else plan.raw_words,
+        2 + 2 * hops if meta is None else 0, meta, plan.ws_bytes, None if status is None else status.ptr(), host, early,
+        None if side is None else side.cuda_stream)
+    return DeviceBatch(g, n, fanouts, plan, results if kept is None else kept, raw, meta, status)
 
 
 def _graph_range(g, lo, hi):
@@ -314,12 +313,12 @@ def build_batch(g, roots, root_ts, fanouts, policy="recent", **kw) -> List[dict]
     staged = bool(fanouts) and roots.numel() > 0 and last + 2 <= _EARLY
     db = _enqueue(g, roots, root_ts, fanouts, policy, g.ts_min, g.ts_max, kw.get("equal_root_time", False), kw.get("allowed_offset", -1),
                   kw.get("seed", 0), None, None, addr, early=addr + 8 * _EARLY if staged else None)
-    wait, sp, laid = _C.lib().sgl_wait_word, _C.stream_ptr(), None
+    wait, sp, laid = _C.host().sgl_wait_word, _C.stream_ptr(), None
     if staged:
         # laid out while the device merges the last list: a fifth of a small batch's time is the making of tensors
-        _C.check(wait(addr + 8 * (_EARLY + last), 1, sp))
+        wait(addr + 8 * (_EARLY + last), 1, sp)
         laid = db._trim_but_last(words[_EARLY:_EARLY + last])
-    _C.check(wait(addr + 8 * (last + 1), 1, sp))
+    wait(addr + 8 * (last + 1), 1, sp)
     host, bits = words[:last], words[last] & 0xFFFFFFFF
     if bits & 2:
         g.__dict__["_queried_outside"] = True
@@ -328,9 +327,8 @@ def build_batch(g, roots, root_ts, fanouts, policy="recent", **kw) -> List[dict]
         raise _C.SglError(f"build_batch: device status {bits} ({_C.decode_status(bits)})")
     if laid is None:
         return db._trim(host)
-    out, v = laid
-    b = 3 + 14 * (len(fanouts) - 1)
-    out[-1]["gids"], out[-1]["ts"] = v(b + 6, host[-1]), v(b + 7, host[-1])
+    out, last_list = laid
+    out[-1]["gids"], out[-1]["ts"] = last_list(host[-1])
     return out
 
 

@@ -145,10 +145,10 @@ class MaterializedMultiLayerBuilder:
             d_ns, outs = words(*[mp + 16 * i for i in range(k)]), words(*[a for a, _ in plans])
             cnts = words(*[mp + 8 * (nb + i * (P + 1)) for i in range(k)])
             ref = C.addressof
-            ws = _C.WORKSPACE.get(L.sgl_plan_routes_ws_bytes(k, ref(ns), ref(cp)), self.device, sp)
-            _C.check(L.sgl_plan_routes(k, ref(ids), ref(ns), ref(d_ns), self.node_parts.data_ptr(), self.node_parts.numel(), self.pid,
-                                       rt.indptr.data_ptr(), rt.indices.data_ptr(), rt.locs.data_ptr(), P, ref(cp), ref(outs), ref(cnts),
-                                       mp + 8 * (nb - 1), ws.data_ptr(), ws.numel(), sp))
+            ws = _C.WORKSPACE.get(_C.host().sgl_plan_routes_ws_bytes(k, ref(ns), ref(cp)), self.device, sp)
+            _C.host().sgl_plan_routes(k, ref(ids), ref(ns), ref(d_ns), self.node_parts.data_ptr(), self.node_parts.numel(), self.pid,
+                                      rt.indptr.data_ptr(), rt.indices.data_ptr(), rt.locs.data_ptr(), P, ref(cp), ref(outs), ref(cnts),
+                                      mp + 8 * (nb - 1), ws.data_ptr(), ws.numel(), sp)
         host = _C.read_words(meta, meta.numel()) if meta.numel() < 512 else meta.tolist()    # the one synchronisation before the copy
         bits = host[nb - 1] & 0xFFFFFFFF
         if bits:
@@ -212,8 +212,8 @@ class MaterializedMultiLayerBuilder:
             return out
         h = torch.empty(at // 8, dtype=torch.int64, pin_memory=pin)
         d = torch.empty(max(at, 16) // 8, dtype=torch.int64, device=self.device)
-        _C.check(_C.lib().sgl_export_arrays(n, src, size, (C.c_int64 * max(n, 1))(*offs), d.data_ptr(), h.data_ptr(), at, None, at,
-                                            _C.stream_ptr()))
+        places, ref = (C.c_int64 * max(n, 1))(*offs), C.addressof
+        _C.host().sgl_export_arrays(n, ref(src), ref(size), ref(places), d.data_ptr(), h.data_ptr(), at, None, at, _C.stream_ptr())
         # (pieces with a storage of their own size: what saves or shares one does not take the others along)
         buf = h.numpy()
         return [torch.frombuffer(buf, dtype=types[s], count=count, offset=o) if count else torch.empty(0, dtype=types[s])

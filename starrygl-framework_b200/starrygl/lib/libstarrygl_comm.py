@@ -21,7 +21,6 @@ import queue
 import threading
 from bisect import bisect_left
 from collections import deque
-from functools import lru_cache
 from typing import List, Optional
 
 import torch
@@ -173,7 +172,7 @@ class TemporalResult:
                 self._status.t.zero_()
                 raise _C.SglError(f"sampling: device status {bits} ({_C.decode_status(bits)})")
         for nb, n in zip(hops, host):
-            nb._n = int(n)
+            nb._n, nb._owner = int(n), None     # (nothing else needs the owner: hops and result no longer hold each other)
         prev = None
         for nb in self.neighbors_list:      # queries of hop l+1 = neighbours of hop l
             if nb._nq is None and prev is not None:
@@ -236,10 +235,7 @@ class _Arena:
 
     def cut(self, section, n, floats=False):
         t, s = (self.buf, self._at[section]) if self._at is not None else (self.buf[section], 0)
-        # (a strided view of the whole costs half of a slice)
-        if floats:
-            return torch.as_strided(t.view(torch.float32), (n,), (1,), 2 * s)
-        return torch.as_strided(t, (n,), (1,), s)
+        return _C.host().cut(t, s, n, floats)
 
     def ptr(self, section):
         return self.buf.data_ptr() + 8 * self._at[section] if self._at is not None else self.buf[section].data_ptr()
@@ -333,7 +329,7 @@ class _QueryFuture:
         addr, words = self.slot
         n = 10 + 2 * hops
         try:
-            _C.check(_C.lib().sgl_wait_word(addr + 8 * n, 1, self.stream.cuda_stream))
+            _C.host().sgl_wait_word(addr + 8 * n, 1, self.stream.cuda_stream)
             meta = words[:n]
         finally:                          # (the stream has come to its end either way)
             _FREE_SLOTS.append(self.slot)
@@ -345,11 +341,6 @@ class _QueryFuture:
         out.neighbors_list = [_ArenaNeighbor(arena, l) for l in range(hops)]
         out._remapper = arena.cut(7 + 8 * hops, arena.n_new)
         return out
-
-
-@lru_cache(maxsize=16)
-def _hop_words(hops):
-    return C.c_int64 * hops               # (making an array type takes longer than filling one in)
 
 
 def query_blocks(root, neg_roots, neighbors):
@@ -370,22 +361,11 @@ def query_blocks(root, neg_roots, neighbors):
         neg, neg_ts = neg_roots.roots.contiguous(), neg_roots.ts.contiguous()          # (a column of a table, say)
         if any(not t.is_cuda or t.dtype != torch.int64 or t.numel() != n_neg for t in (neg, neg_ts)):
             return None
-    hops = a.hops
-    dst = [a.n_queries] + a.edges[:-1]
-    total = sum(2 * (d + n) + n for d, n in zip(dst, a.edges))
-    out = torch.empty(total, dtype=torch.int64, device=a.device)
-    kind = _hop_words(hops)
-    node = kind(*[a.ptr(7 + 8 * l + 6) for l in range(hops)])
-    ts = kind(*[a.ptr(7 + 8 * l + 2) for l in range(hops)])
-    cnt = kind(*a.edges)
-    _C.check(_C.lib().sgl_query_blocks(hops, node, ts, cnt, a.ptr(6), a.ptr(2), a.ptr(1), None if neg is None else neg.data_ptr(),
-                                       None if neg is None else neg_ts.data_ptr(),
-                                       a.n_roots, a.n_pairs, a.n_queries, out.data_ptr(), _C.stream_ptr()))
-    blocks, at, cut = [], 0, torch.as_strided
-    for d, n in zip(dst, a.edges):
-        blocks.append((d, cut(out, (d + n,), (1,), at), cut(out, (d + n,), (1,), at + d + n), cut(out, (n,), (1,), at + 2 * (d + n))))
-        at += 2 * (d + n) + n
-    return blocks
+    parts = []
+    for l, n in enumerate(a.edges):
+        parts += (a.ptr(7 + 8 * l + 6), a.ptr(7 + 8 * l + 2), n)
+    blocks = _C.host().query_blocks(a.device.index, a.ptr(6), a.ptr(2), a.ptr(1), neg, neg_ts, a.n_roots, a.n_pairs, a.n_queries, *parts)
+    return [(d, *arrays) for d, arrays in blocks]
 
 
 # Free pinned result words of queries, (address, ctypes array); as many as queries were ever in flight together, kept for the next
@@ -519,7 +499,7 @@ class CUDAGraph:
         """Host-known bounds of the window's events: (first, at most) from every 256th timestamp of the stream."""
         if self._ev_index is None:
             with torch.cuda.stream(self.stream):      # (events out of order are still being sorted there)
-                self._ev_index = self.ev[1][::256].cpu().numpy()
+                self._ev_index = self.ev[1][::256].tolist()      # (a list: what is looked up in an array is made an object first)
         idx, m = self._ev_index, self.ev[1].numel()
         first = max(bisect_left(idx, t0) - 1, 0) * 256
         last = min(bisect_left(idx, t1) * 256, m)
@@ -561,30 +541,29 @@ class CUDAGraph:
         neg_ids, neg_ts = neg.roots.contiguous(), neg.ts.contiguous()
         if self.mapper is not None and chunks is not None and self.mapper.numel():
             self.stream.wait_stream(torch.cuda.current_stream(dev))
-        with _C.on_stream(self.stream):
-            mask, node_chunk, n_chunks = ops.chunk_mask(g, chunks, self.mapper)
-            if plan.shared:
-                buf = torch.empty(plan.words + 10 + 2 * layers, dtype=torch.int64, device=dev)
-                at, base, meta = plan.at, buf.data_ptr(), buf.data_ptr() + 8 * plan.words
-            else:
-                buf = [torch.empty(w, dtype=torch.int64, device=dev) for w in (*plan.size, 10 + 2 * layers)]
-                at, base, meta = plan.places(*[t.data_ptr() // 8 for t in buf[:-1]]), None, buf[-1].data_ptr()
-            ws = _C.WORKSPACE.get(plan.ws_bytes, dev, sp)
-        rl = self.relabel
+        rl, st, extra = self.relabel, self.stream, 10 + 2 * layers
+        mask, node_chunk, n_chunks, buf = None, None, 0, None
+        at, words, meta = C.addressof(plan.at), plan.words, extra
+        if self.mapper is not None or not plan.shared:
+            with _C.on_stream(st):
+                mask, node_chunk, n_chunks = ops.chunk_mask(g, chunks, self.mapper)
+                if not plan.shared:
+                    buf = [torch.empty(w, dtype=torch.int64, device=dev) for w in (*plan.size, extra)]
+                    places = plan.places(*[t.data_ptr() // 8 for t in buf[:-1]])
+                    at, words, meta = C.addressof(places), 0, buf[-1].data_ptr()
         epoch = rl.epoch + (1 if op == "f" else 0)       # the reference restarts the numbering on "f"
         slot = self._slot()
-        slot[1][10 + 2 * layers] = 0
-        rc = _C.lib().sgl_query_at(
-            g.indptr.data_ptr(), g.nbr.data_ptr(), g.ts.data_ptr(), g.eid.data_ptr(), None if g.fence is None else g.fence.data_ptr(),
-            g.num_nodes, self.ev[0].data_ptr(), self.ev[1].data_ptr(), self.ev[2].data_ptr(), first, cap, t0, t1,
-            None if node_chunk is None else node_chunk.data_ptr(), None if mask is None else mask.data_ptr(), n_chunks,
-            neg_ids.data_ptr() if n_neg else None, neg_ts.data_ptr() if n_neg else None, n_neg, fanout, layers, _C.POLICY[stype],
-            int(eq), off, int(keep), ops.bits_for(g.num_nodes - 1), ops.bits_for(g.ts_max - g.ts_min), g.ts_min, rl.mapper.data_ptr(),
-            rl.mask.data_ptr(), epoch, int(op == "f"), rl.next_local.data_ptr(), at, base, meta, slot[0], ws.data_ptr(),
-            ws.numel(), producer, sp)
-        if rc:                            # nothing was enqueued: the numbering goes on as it was
+        slot[1][extra] = 0
+        try:
+            own, = _C.host().query(
+                g.indptr, g.nbr, g.ts, g.eid, g.fence, g.num_nodes, *self.ev, first, cap, t0, t1, node_chunk, mask, n_chunks, neg_ids, neg_ts,
+                fanout, layers, _C.POLICY[stype], eq, off, keep, ops.bits_for(g.num_nodes - 1), ops.bits_for(g.ts_max - g.ts_min), g.ts_min,
+                rl.mapper, rl.mask, epoch, op == "f", rl.next_local, at, words, meta, slot[0], plan.ws_bytes, producer, st.stream_id,
+                st.device_index, st.device_type, sp)
+        except BaseException:             # nothing was enqueued: the numbering goes on as it was
             _FREE_SLOTS.append(slot)
-            _C.check(rc)
+            raise
+        buf = own if buf is None else buf
         rl.epoch = epoch
         fut = _QueryFuture(self.stream, slot, buf, plan, layers, neg)
         fut._keep = (neg_ids, neg_ts, mask)   # inputs of kernels that may still be queued

@@ -83,23 +83,8 @@ class TCSR:
 def tcsr_build(key, nbr, ts, eid, num_nodes: int, want_perm: bool = False, want_fence: bool = True) -> TCSR:
     """Build the T-CSR keyed by ``key`` (and, unless ``want_fence`` is off, the search index the sampler walks before it
     touches a row).  Synchronises the stream once.  Raises on out-of-range keys."""
-    L = _C.lib()
-    key, nbr, ts = _i64(key), _i64(nbr), _i64(ts)
-    eid = None if eid is None else _i64(eid)
-    m = key.numel()
-    if not (nbr.numel() == m and ts.numel() == m and (eid is None or eid.numel() == m)):
-        raise _C.SglError("tcsr_build: edge arrays differ in length")
-    dev = key.device
-    indptr = torch.empty(num_nodes + 1, dtype=I64, device=dev)
-    o_nbr, o_ts, o_eid = (torch.empty(m, dtype=I64, device=dev) for _ in range(3))
-    perm = torch.empty(m, dtype=I64, device=dev) if want_perm else None
-    rng = (C.c_int64 * 2)(0, 0)
-    fence = torch.empty(L.sgl_tcsr_fence_len(num_nodes, m), dtype=I64, device=dev) if want_fence and m and num_nodes else None
-    _, wp, wn = _C.workspace(L.sgl_tcsr_build_ws_bytes(num_nodes, m), dev)
-    _C.check(L.sgl_tcsr_build_fenced(num_nodes, m, _C.ptr(key), _C.ptr(nbr), _C.ptr(ts), _C.ptr(eid), _C.ptr(indptr),
-                                     _C.ptr(o_nbr), _C.ptr(o_ts), _C.ptr(o_eid), _C.ptr(perm), _C.ptr(fence), rng, wp, wn,
-                                     _C.stream_ptr()))
-    return TCSR(num_nodes, indptr, o_nbr, o_ts, o_eid, perm, int(rng[0]), int(rng[1]), fence)
+    (indptr, o_nbr, o_ts, o_eid, perm, fence), lo, hi = _C.host().tcsr_build(key, nbr, ts, eid, num_nodes, want_perm, want_fence)
+    return TCSR(num_nodes, indptr, o_nbr, o_ts, o_eid, perm, lo, hi, fence)
 
 
 # --------------------------------------------------------------------------------------------------------------
@@ -141,32 +126,18 @@ class Hop:
 def sample_layer(g: TCSR, targets, target_ts, fanout: int, policy="recent", *, d_n=None, equal_root_time=False,
                  allowed_offset=-1, keep_root_time=False, seed=0, rng_stream=0, want_dt_i64=False,
                  status: Optional[StatusWord] = None) -> Hop:
-    L = _C.lib()
-    targets, target_ts = _i64(targets), _i64(target_ts)
-    n = targets.numel()
-    if target_ts.numel() != n:
-        raise _C.SglError("sample_layer: targets and target_ts differ in length")
-    dev = g.device
-    cap = max(n * fanout, 1)
-    o_nbr, o_dst, o_ts, o_eid = (torch.empty(cap, dtype=I64, device=dev) for _ in range(4))
-    o_dt = torch.empty(cap, dtype=torch.float32, device=dev)
-    offs = torch.empty(n + 1, dtype=I64, device=dev)
-    o_dti = torch.empty(cap, dtype=I64, device=dev) if want_dt_i64 else None
     pol = _C.POLICY[policy] if isinstance(policy, str) else int(policy)
-    _, wp, wn = _C.workspace(L.sgl_sample_ws_bytes(n), dev)
     # (a captured launch does not hand its count over)
-    taken, stream = None if torch._C._cuda_isCurrentStreamCapturing() else _C.COUNTS.take(), _C.stream_ptr()
+    taken = None if torch._C._cuda_isCurrentStreamCapturing() else _C.COUNTS.take()
     try:
-        _C.check(L.sgl_sample_layer_counted(_C.ptr(g.indptr), _C.ptr(g.nbr), _C.ptr(g.ts), _C.ptr(g.eid), _C.ptr(g.fence), g.num_nodes,
-                                    _C.ptr(targets), _C.ptr(target_ts), n, _C.ptr(d_n), int(fanout), pol,
-                                    int(bool(equal_root_time)), int(allowed_offset), int(bool(keep_root_time)),
-                                    int(seed) & (2 ** 64 - 1), int(rng_stream) & 0xFFFFFFFF, _C.ptr(o_nbr), _C.ptr(o_dst),
-                                    _C.ptr(o_ts), _C.ptr(o_dt), _C.ptr(o_dti), _C.ptr(o_eid), _C.ptr(offs),
-                                    status.ptr() if status else None, wp, wn, taken and taken[0], taken[2] if taken else 0, stream))
+        o_nbr, o_dst, o_ts, o_dt, o_eid, offs, o_dti = _C.host().sample_layer(
+            g.indptr, g.nbr, g.ts, g.eid, g.fence, g.num_nodes, targets, target_ts, int(fanout), pol, d_n, bool(equal_root_time),
+            int(allowed_offset), bool(keep_root_time), int(seed), int(rng_stream), want_dt_i64, status.ptr() if status else None,
+            taken and taken[0], taken[2] if taken else 0)
     except BaseException:
         _C.COUNTS.give_back(taken)
         raise
-    return Hop(o_nbr, o_dst, o_ts, o_dt, o_eid, offs, cap, o_dti, taken and (taken, stream))
+    return Hop(o_nbr, o_dst, o_ts, o_dt, o_eid, offs, o_nbr.numel(), o_dti, taken and (taken, _C.stream_ptr()))
 
 
 # --------------------------------------------------------------------------------------------------------------
@@ -368,59 +339,19 @@ def gather_rows(table, idx, *, map=None, d_n=None, ts_table=None, mode="auto", o
                 status: Optional[StatusWord] = None):
     """out[i] = table[row(i)] (row(i) = map[idx[i]] when map is given; negative rows count from the end).
     With ts_table also returns ts_table[row(i)]."""
-    L = _C.lib()
-    idx = _i64(idx)
-    n = idx.numel()
-    row_bytes, src_pitch = _row_bytes(table)
-    dst_pitch = row_bytes
-    if out is None:
-        out = torch.empty((n, *table.shape[1:]), dtype=table.dtype, device=idx.device)
-    elif n:
-        _, dst_pitch = _row_bytes(out)
-    out_ts = torch.empty(n, dtype=torch.float32, device=idx.device) if ts_table is not None else None
-    _C.check(L.sgl_gather_rows(_C.ptr(table) if table.numel() else None, table.shape[0], row_bytes, src_pitch,
-                               _C.ptr(idx), _C.ptr(map), 0 if map is None else map.numel(), n, _C.ptr(d_n),
-                               out.data_ptr() if out.numel() else None, dst_pitch, _C.ptr(ts_table), _C.ptr(out_ts),
-                               _C.GATHER_MODE[mode], status.ptr() if status else None, _C.stream_ptr()))
-    return (out, out_ts) if ts_table is not None else out
+    return _C.host().gather_rows(table, idx, map, d_n, ts_table, _C.GATHER_MODE[mode], out, status.ptr() if status else None)
 
 
 def scatter_rows(table, idx, rows, *, map=None, d_n=None, ts_table=None, ts=None, split_last_col=False,
                  status: Optional[StatusWord] = None):
     """table[row(i)] = rows[i] for row(i) >= 0; optionally ts_table[row(i)] = ts[i] (or the trailing column)."""
-    L = _C.lib()
-    idx = _i64(idx)
-    n = idx.numel()
-    row_bytes, dst_pitch = _row_bytes(table)
-    _, src_pitch = _row_bytes(rows) if n else (0, row_bytes + (4 if split_last_col else 0))
-    _C.check(L.sgl_scatter_rows(_C.ptr(table) if table.numel() else None, table.shape[0], row_bytes, dst_pitch,
-                                _C.ptr(idx), _C.ptr(map), 0 if map is None else map.numel(), n, _C.ptr(d_n),
-                                rows.data_ptr() if rows.numel() else None, src_pitch, _C.ptr(ts_table), _C.ptr(ts),
-                                int(bool(split_last_col)), status.ptr() if status else None, _C.stream_ptr()))
+    _C.host().scatter_rows(table, idx, rows, map, d_n, ts_table, ts, bool(split_last_col), status.ptr() if status else None)
 
 
 def cache_gather(cache_rows, hitmap, backing, ids, *, status: Optional[StatusWord] = None):
     """Gather through the device cache.  Returns (out, miss_pos, miss_ids, counts) where counts = [hits, misses]
     (device int64) and the miss lists have capacity len(ids)."""
-    L = _C.lib()
-    ids = _i64(ids)
-    n = ids.numel()
-    if hitmap.dtype != torch.int32:
-        raise _C.SglError("hitmap must be int32")
-    row_bytes, pitch = _row_bytes(cache_rows)
-    if pitch != row_bytes or (backing is not None and _row_bytes(backing) != (row_bytes, row_bytes)):
-        raise _C.SglError("cache and backing rows must be dense and of equal size")
-    dev = ids.device
-    out = torch.empty((n,) + tuple(cache_rows.shape[1:]), dtype=cache_rows.dtype, device=dev)
-    miss_pos = torch.empty(max(n, 1), dtype=I64, device=dev)
-    miss_ids = torch.empty(max(n, 1), dtype=I64, device=dev)
-    counts = torch.empty(2, dtype=I64, device=dev)
-    _, wp, wn = _C.workspace(L.sgl_cache_gather_ws_bytes(n), dev)
-    _C.check(L.sgl_cache_gather(_C.ptr(cache_rows), cache_rows.shape[0], _C.ptr(hitmap), hitmap.numel(),
-                                _C.ptr(backing), row_bytes, _C.ptr(ids), n,
-                                out.data_ptr() if n else None, _C.ptr(miss_pos), _C.ptr(miss_ids), _C.ptr(counts),
-                                status.ptr() if status else None, wp, wn, _C.stream_ptr()))
-    return out, miss_pos, miss_ids, counts
+    return _C.host().cache_gather(cache_rows, hitmap, backing, ids, status.ptr() if status else None)
 
 
 # --------------------------------------------------------------------------------------------------------------
@@ -586,9 +517,6 @@ def plan_route(layer_ids, node_parts, pid: int, rep_indptr, rep_ranks, rep_locs,
 # mailbox update
 # --------------------------------------------------------------------------------------------------------------
 
-_SEG_ARRAYS = [C.c_int64 * max(k, 1) for k in range(5)]       # (making an array type takes longer than filling one in)
-
-
 def mail_reduce(ids_a, ids_b, ts, num_nodes: int, segments=(), *, want_pos: bool = False,
                 status: Optional[StatusWord] = None, count=None):
     """Latest message per node (see ``sgl_mail_reduce``).  ``ids_a`` / ``ids_b``: int64 node ids of the two entry lists
@@ -597,60 +525,12 @@ def mail_reduce(ids_a, ids_b, ts, num_nodes: int, segments=(), *, want_pos: bool
     Returns ``(index, mail, mail_ts, pos, d_num_unique)`` with capacity ``len(ids_a) + len(ids_b)``; the valid
     length is the device scalar ``d_num_unique`` (no synchronisation here).  ``mail`` is None without segments.
     ``count``: a pair taken from ``_C.COUNTS`` that receives the number of nodes."""
-    L = _C.lib()
-    ids_a = _i64(ids_a)
-    dev = ids_a.device
-    n_a = ids_a.numel()
-    ids_b = _i64(ids_b) if ids_b is not None else None
-    n_b = ids_b.numel() if ids_b is not None else 0
-    n = n_a + n_b
-    if ts.dtype not in (torch.int64, torch.float32):
-        raise _C.SglError(f"mail_reduce: timestamps must be int64 or float32, got {ts.dtype}")
-    ts = ts.contiguous()
-    segs = []
-    for ta, tb in segments:
-        ta = ta.contiguous()
-        tb = ta if tb is None else tb.contiguous()
-        if ta.dtype != torch.float32 or tb.dtype != torch.float32 or ta.dim() != 2 or tb.shape[1:] != ta.shape[1:]:
-            raise _C.SglError("mail_reduce: segments are pairs of fp32 [rows, dim] tables of equal width")
-        if ta.shape[0] < n_a or (n_b and tb.shape[0] < n_b):
-            raise _C.SglError("mail_reduce: a segment table has fewer rows than its entry list")
-        segs.append((ta, tb))
-    width = sum(int(a.shape[1]) for a, _ in segs)
-    cap = max(n, 1)
-    index = torch.empty(cap, dtype=I64, device=dev)
-    pos = torch.empty(cap, dtype=I64, device=dev) if want_pos else None
-    out_ts = torch.empty(cap, dtype=torch.float32, device=dev)
-    mail = torch.empty((cap, width), dtype=torch.float32, device=dev) if segs else None
-    d_u = torch.empty(1, dtype=I64, device=dev)
-    k = len(segs)
-    kind = _SEG_ARRAYS[k] if k < len(_SEG_ARRAYS) else C.c_int64 * k
-    arr_a = kind(*[a.data_ptr() for a, _ in segs])
-    arr_b = kind(*[b.data_ptr() for _, b in segs])
-    arr_d = kind(*[a.shape[1] for a, _ in segs])
-    _, wp, wn = _C.workspace(L.sgl_mail_reduce_ws_bytes(n), dev)
-    _C.check(L.sgl_mail_reduce_counted(_C.ptr(ids_a), n_a, _C.ptr(ids_b) if n_b else None, n_b, int(num_nodes), _C.ptr(ts), ts.numel(),
-                               1 if ts.dtype == torch.int64 else 0, k, C.addressof(arr_a), C.addressof(arr_b),
-                               C.addressof(arr_d), _C.ptr(index), _C.ptr(pos) if want_pos else None, _C.ptr(out_ts),
-                               _C.ptr(mail) if mail is not None else None, _C.ptr(d_u), status.ptr() if status else None,
-                               wp, wn, None if count is None else count[0], 0 if count is None else count[2], _C.stream_ptr()))
-    return index, mail, out_ts, pos, d_u
+    return _C.host().mail_reduce(ids_a, ids_b, ts, int(num_nodes), segments, want_pos, status.ptr() if status else None,
+                                 None if count is None else count[0], 0 if count is None else count[2])
 
 
 def mailbox_write(index, mail, mail_ts, mailbox, mailbox_ts, next_mail_pos, *, d_n=None, advance: bool = True,
                   status: Optional[StatusWord] = None):
     """``mailbox[index, next_mail_pos[index]] = mail`` (+ timestamps, + ring position), see ``sgl_mailbox_write``.
     ``index`` must hold distinct nodes.  With ``d_n`` (device int64) only the first ``*d_n`` rows are written."""
-    L = _C.lib()
-    index = _i64(index)
-    if mailbox.dim() != 3 or not mailbox.is_contiguous() or not mailbox_ts.is_contiguous():
-        raise _C.SglError("mailbox_write: mailbox must be a contiguous [nodes, slots, width] tensor")
-    nodes, slots, width = mailbox.shape
-    if mail.dim() != 2 or mail.shape[1] != width or mail.dtype != torch.float32 or mail_ts.dtype != torch.float32:
-        raise _C.SglError("mailbox_write: mail rows must be fp32 of the mailbox's width")
-    if next_mail_pos is not None:
-        next_mail_pos = _i64(next_mail_pos)
-    n = min(index.numel(), mail.shape[0])
-    _C.check(L.sgl_mailbox_write(_C.ptr(index), n, _C.ptr(d_n), _C.ptr(mail.contiguous()), _C.ptr(mail_ts.contiguous()), width,
-                                 _C.ptr(mailbox), _C.ptr(mailbox_ts), _C.ptr(next_mail_pos) if next_mail_pos is not None else None,
-                                 nodes, slots, 1 if advance else 0, status.ptr() if status else None, _C.stream_ptr()))
+    _C.host().mailbox_write(index, mail, mail_ts, mailbox, mailbox_ts, next_mail_pos, d_n, advance, status.ptr() if status else None)

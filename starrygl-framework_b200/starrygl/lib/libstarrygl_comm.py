@@ -19,6 +19,7 @@ hop l at the time of the edge that reached it (or at the root's time with ``keep
 import ctypes as C
 import queue
 import threading
+import weakref
 from bisect import bisect_left
 from collections import deque
 from typing import List, Optional
@@ -79,16 +80,24 @@ class TemporalNeighbor:
 
     def __init__(self, hop: ops.Hop, owner: "TemporalResult" = None, n_queries: Optional[int] = None):
         self.hop = hop
-        self._owner = owner
+        # (not the result itself: the two would hold each other, and with them the arrays of every hop, until a garbage collection)
+        self._owner = None if owner is None else weakref.ref(owner)
+        self._status = None if owner is None else owner._status
+        self._before = owner.neighbors_list[-1] if owner is not None and owner.neighbors_list else None
         self._n = None                  # number of sampled neighbours, once known on the host
         self._nq = n_queries            # number of queries (None: known only once the previous hop has been cut)
         self._neighbors_override = None
 
     def _cut(self) -> int:
         if self._n is None:
-            if self._owner is not None:
-                self._owner.materialize()
+            owner = None if self._owner is None else self._owner()
+            if owner is not None:
+                owner.materialize()
             else:
+                if self._status is not None:
+                    self._status.check("sampling")
+                if self._nq is None and self._before is not None:
+                    self._nq = self._before._cut()
                 self._n = self.hop.total()
         return self._n
 
@@ -172,7 +181,7 @@ class TemporalResult:
                 self._status.t.zero_()
                 raise _C.SglError(f"sampling: device status {bits} ({_C.decode_status(bits)})")
         for nb, n in zip(hops, host):
-            nb._n, nb._owner = int(n), None     # (nothing else needs the owner: hops and result no longer hold each other)
+            nb._n = int(n)
         prev = None
         for nb in self.neighbors_list:      # queries of hop l+1 = neighbours of hop l
             if nb._nq is None and prev is not None:
@@ -282,7 +291,7 @@ class _ArenaNeighbor(TemporalNeighbor):
         self._a, self._l, self._b = arena, level, 7 + 8 * level
         self._n = arena.edges[level]
         self._nq = arena.n_queries if level == 0 else arena.edges[level - 1]
-        self._owner, self._neighbors_override = None, None
+        self._neighbors_override = None
 
     def _cut(self):
         return self._n

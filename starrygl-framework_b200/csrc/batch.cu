@@ -204,6 +204,7 @@ static int build_batch(const int64_t* indptr, const int64_t* nbr, const int64_t*
   int rc = sgl_unique_pairs(roots, root_ts, n_roots, nullptr, nullptr, nullptr, 0, nullptr, id_bits, ts_bits, ts_base, cur_id, cur_ts, inv,
                             nullptr, meta, d_status, lws, lwb, stream);
   if (rc) return rc;
+  if (n_hops > 0) SGL_CHECK_RC(scope.flush());             // (600 roots 50.3 -> 46.5 us a batch, 4,096 roots two hops 143 -> 134)
   struct Hop {
     int64_t *nbr, *dst, *ts, *eid, *offs, *gids, *gts, *col, *indptr, *indices, *cts, *ceid;
     float *dt, *cdt;

@@ -189,6 +189,16 @@ int LaunchScope::submit() {
   return no_throw([&] { return submit_list(); });
 }
 
+int LaunchScope::flush() {
+  if (!owner_) return SGL_OK;
+  return no_throw([&] {
+    const int rc = submit_list();
+    t_state.list.clear();
+    tails_.clear();                      // (what follows comes after all of it, in stream order)
+    return rc;
+  });
+}
+
 int LaunchScope::submit_list() {
   Thread& t = t_state;
   LaunchList& l = t.list;

@@ -85,6 +85,10 @@ class LaunchScope {
     return rc != SGL_OK ? rc : wait(s, nodes);
   }
   int submit();
+  // Submits what was collected so far and goes on collecting (nothing in an inner scope): the device starts on it while the host
+  // still adds and sets up the rest, which takes 0.6 us a kernel and 5 us a launch.  For a beginning of 10 - 15 us that everything else
+  // waits for; all refusals that must leave no trace come before it.
+  int flush();
 
  private:
   int submit_list();

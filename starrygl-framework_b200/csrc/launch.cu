@@ -17,6 +17,7 @@ struct Cached {
     if (graph) cudaGraphDestroy(graph);
   }
   std::vector<cudaGraphNode_t> nodes;
+  std::vector<std::vector<unsigned char>> set;     // grid, block, shared memory and arguments that a node has
   uint64_t last_use = 0;
   bool refused = false;               // no graph could be made of it (no memory, say): launched one by one
 };
@@ -60,6 +61,23 @@ cudaKernelNodeParams node_params(const LaunchNode& n) {
   return p;
 }
 
+// Notes what node i of the list is given; false: its node in the graph has just that.
+bool changed(Cached& c, size_t i) {
+  const LaunchList& l = t_state.list;
+  const LaunchNode& n = l.nodes[i];
+  const size_t from = n.arg_count ? l.arg_at[n.arg_first] : 0,
+               to = n.arg_count ? (i + 1 < l.used && l.nodes[i + 1].arg_count ? l.arg_at[l.nodes[i + 1].arg_first] : l.bytes.size()) : 0;
+  const unsigned shape[] = {n.grid.x, n.grid.y, n.grid.z, n.block.x, n.block.y, n.block.z, n.smem};
+  std::vector<unsigned char>& set = c.set[i];
+  if (set.size() == sizeof(shape) + (to - from) && memcmp(set.data(), shape, sizeof(shape)) == 0 &&
+      memcmp(set.data() + sizeof(shape), l.bytes.data() + from, to - from) == 0)
+    return false;
+  set.resize(sizeof(shape) + (to - from));
+  memcpy(set.data(), shape, sizeof(shape));
+  memcpy(set.data() + sizeof(shape), l.bytes.data() + from, to - from);
+  return true;
+}
+
 int one_by_one(cudaStream_t stream) {
   const LaunchList& l = t_state.list;
   for (size_t i = 0; i < l.used; ++i) {
@@ -92,6 +110,8 @@ int build(Cached& c) {
   c.graph = graph;
   c.exec = exec;
   c.nodes = std::move(nodes);
+  c.set.resize(l.used);
+  for (size_t i = 0; i < l.used; ++i) changed(c, i);
   return SGL_OK;
 }
 
@@ -237,8 +257,11 @@ int LaunchScope::submit_list() {
   if (c->exec == nullptr && !c->refused) SGL_CHECK_RC(build(*c));
   else if (!c->refused) {
     for (size_t i = 0; i < l.used; ++i) {
+      if (!changed(*c, i)) continue;
       const cudaKernelNodeParams p = node_params(l.nodes[i]);
-      SGL_CUDA_CHECK(cudaGraphExecKernelNodeSetParams(c->exec, c->nodes[i], &p));
+      const cudaError_t e = cudaGraphExecKernelNodeSetParams(c->exec, c->nodes[i], &p);
+      if (e != cudaSuccess) c->set[i].clear();         // (who knows what it has)
+      SGL_CUDA_CHECK(e);
     }
   }
   if (c->refused) return one_by_one(main_);

@@ -33,6 +33,17 @@ __device__ __forceinline__ uint32_t ld_stream(const uint32_t* p) {
   asm volatile("ld.global.nc.L1::no_allocate.u32 %0, [%1];" : "=r"(v) : "l"(p));
   return v;
 }
+// the same through the path that sees what was written since the kernel was set up (see launch_early)
+__device__ __forceinline__ uint4 ld_current(const uint4* p) {
+  uint4 v;
+  asm volatile("ld.global.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ uint32_t ld_current(const uint32_t* p) {
+  uint32_t v;
+  asm volatile("ld.global.L1::no_allocate.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  return v;
+}
 __device__ __forceinline__ void st_stream(uint4* p, uint4 v) {
   asm volatile("st.global.cs.v4.u32 [%0], {%1,%2,%3,%4};" ::"l"(p), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
 }
@@ -69,16 +80,15 @@ struct LaneSplit {
 };
 
 // resolve the source/destination row of item i; returns false when the row must be skipped
-__device__ __forceinline__ bool resolve_row(const int64_t* __restrict__ idx, const int64_t* __restrict__ map,
-                                            int64_t map_len, int64_t table_rows, int64_t i, bool wrap_negative,
-                                            int32_t* d_status, int64_t* row) {
-  int64_t r = __ldg(idx + i);
+__device__ __forceinline__ bool resolve_row(const int64_t* idx, const int64_t* map, int64_t map_len, int64_t table_rows, int64_t i,
+                                            bool wrap_negative, int32_t* d_status, int64_t* row) {
+  int64_t r = idx[i];
   if (map) {
     if (r < 0 || r >= map_len) {
       dev_flag(d_status, SGL_DEV_BAD_INDEX);
       return false;
     }
-    r = __ldg(map + r);
+    r = map[r];
   }
   if (r < 0) {
     if (!wrap_negative) return false;  // "not stored here": skipped silently
@@ -94,35 +104,45 @@ __device__ __forceinline__ bool resolve_row(const int64_t* __restrict__ idx, con
 
 template <typename V>
 __global__ void __launch_bounds__(kLaneThreads)
-gather_lanes_kernel(const char* __restrict__ table, int64_t table_rows, LaneSplit split, int64_t src_pitch,
-                    const int64_t* __restrict__ idx, const int64_t* __restrict__ map, int64_t map_len, int64_t n_cap,
-                    const int64_t* d_n, char* __restrict__ out, int64_t dst_pitch, const float* __restrict__ ts_table,
-                    float* __restrict__ out_ts, int32_t* d_status) {
-  const int64_t n = eff_count(n_cap, d_n);
+gather_lanes_kernel(const char* table, int64_t table_rows, LaneSplit split, int64_t src_pitch, const int64_t* idx, const int64_t* map,
+                    int64_t map_len, int64_t n_cap, const int64_t* d_n, char* out, int64_t dst_pitch, const float* ts_table,
+                    float* out_ts, int32_t* d_status) {
+  after_predecessor();
+  idx = current(idx);
+  map = current(map);
+  ts_table = current(ts_table);
+  const int64_t n = eff_count(n_cap, current(d_n));
   const int64_t total = n * split.lanes;
   const int64_t stride = (int64_t)gridDim.x * kLaneThreads;
   for (int64_t q0 = (int64_t)blockIdx.x * kLaneThreads + threadIdx.x; q0 < total; q0 += stride * kLaneUnroll) {
+    // (every step for all of a thread's pieces before the next one: the loads of one do not wait for the others')
     V v[kLaneUnroll];
     V* dst[kLaneUnroll];
+    int64_t row[kLaneUnroll], at[kLaneUnroll];
+    uint32_t lane[kLaneUnroll];
 #pragma unroll
     for (int u = 0; u < kLaneUnroll; ++u) {
-      int64_t q = q0 + u * stride;
+      const int64_t q = q0 + u * stride;
       dst[u] = nullptr;
+      at[u] = -1;
       if (q < total) {
         int64_t i;
-        uint32_t l;
-        split(q, &i, &l);
-        int64_t r;
-        if (resolve_row(idx, map, map_len, table_rows, i, true, d_status, &r)) {
-          v[u] = ld_stream((const V*)(table + r * src_pitch) + l);
-          dst[u] = (V*)(out + i * dst_pitch) + l;
-          if (l == 0 && ts_table) out_ts[i] = __ldg(ts_table + r);
-        }
+        split(q, &i, &lane[u]);
+        if (resolve_row(idx, map, map_len, table_rows, i, true, d_status, &row[u])) at[u] = i;
       }
     }
 #pragma unroll
-    for (int u = 0; u < kLaneUnroll; ++u)
-      if (dst[u]) st_stream(dst[u], v[u]);
+    for (int u = 0; u < kLaneUnroll; ++u) {
+      if (at[u] < 0) continue;
+      v[u] = ld_current((const V*)(table + row[u] * src_pitch) + lane[u]);
+      dst[u] = (V*)(out + at[u] * dst_pitch) + lane[u];
+    }
+#pragma unroll
+    for (int u = 0; u < kLaneUnroll; ++u) {
+      if (dst[u] == nullptr) continue;
+      if (lane[u] == 0 && ts_table) out_ts[at[u]] = ts_table[row[u]];
+      st_stream(dst[u], v[u]);
+    }
   }
 }
 
@@ -178,7 +198,7 @@ __device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.a
 
 // Where row i of a bulk copy comes from, in three steps that depend on each other and that the pipeline keeps apart, so that
 // their latencies overlap the copies: first(i) and second(first) are loads, source() turns the result into an address
-// (nullptr: the output row is left as it is).
+// (nullptr: the output row is left as it is).  kEarly, begin(): see launch_early.
 struct TableRows {
   const char* table;
   int64_t table_rows, src_pitch;
@@ -188,11 +208,17 @@ struct TableRows {
   float* out_ts;
   int32_t* d_status;
   using Key = int64_t;
+  static constexpr bool kEarly = true;
   static constexpr int64_t kBad = INT64_MIN;
-  __device__ __forceinline__ Key first(int64_t i) const { return __ldg(idx + i); }
+  __device__ __forceinline__ void begin() {
+    idx = current(idx);
+    map = current(map);
+    ts_table = current(ts_table);
+  }
+  __device__ __forceinline__ Key first(int64_t i) const { return idx[i]; }
   __device__ __forceinline__ Key second(Key r) const {
     if (map == nullptr) return r;
-    return r >= 0 && r < map_len ? __ldg(map + r) : kBad;
+    return r >= 0 && r < map_len ? map[r] : kBad;
   }
   __device__ __forceinline__ const char* source(int64_t i, Key r, float* ts, int64_t* ts_row) const {
     if (r != kBad && r < 0) r += table_rows;
@@ -201,7 +227,7 @@ struct TableRows {
       return nullptr;
     }
     if (ts_table) {
-      *ts = __ldg(ts_table + r);
+      *ts = ts_table[r];
       *ts_row = i;
     }
     return table + r * src_pitch;
@@ -212,19 +238,14 @@ struct TableRows {
 // Output rows must be contiguous (dst_pitch == row_bytes); row_bytes multiple of 16; rows_per_stage <= 32.
 template <class Rows, int WARPS, int STAGES>
 __global__ void __launch_bounds__(WARPS * 32)
-bulk_rows_kernel(const Rows src, uint32_t row_bytes, int64_t n_cap, const int64_t* d_n, char* __restrict__ out, int rows_per_stage,
+bulk_rows_kernel(Rows src, uint32_t row_bytes, int64_t n_cap, const int64_t* d_n, char* __restrict__ out, int rows_per_stage,
                  int32_t* d_status) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
   __shared__ __align__(8) uint64_t bars[WARPS][STAGES];
   __shared__ uint32_t s_have[WARPS][STAGES];             // rows of the stage that have a source
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int64_t n = eff_count(n_cap, d_n);
   const uint32_t stage_bytes = (uint32_t)rows_per_stage * row_bytes;
   unsigned char* my_smem = smem_raw + (size_t)warp * STAGES * stage_bytes;
-  const int64_t num_chunks = (n + rows_per_stage - 1) / rows_per_stage;
-  const int64_t warps_total = (int64_t)gridDim.x * WARPS;
-  const int64_t gwarp = (int64_t)blockIdx.x * WARPS + warp;
-
   if (lane == 0) {
 #pragma unroll
     for (int s = 0; s < STAGES; ++s) mbar_init(smem_u32(&bars[warp][s]), 1);
@@ -232,6 +253,12 @@ bulk_rows_kernel(const Rows src, uint32_t row_bytes, int64_t n_cap, const int64_
     fence_async_smem();
   }
   __syncwarp();
+  after_predecessor();
+  src.begin();
+  const int64_t n = eff_count(n_cap, current(d_n));
+  const int64_t num_chunks = (n + rows_per_stage - 1) / rows_per_stage;
+  const int64_t warps_total = (int64_t)gridDim.x * WARPS;
+  const int64_t gwarp = (int64_t)blockIdx.x * WARPS + warp;
 
   // this lane's row of the warp's k-th chunk, -1 when there is none
   auto row_of = [&](int64_t k) -> int64_t {
@@ -343,38 +370,51 @@ int launch_bulk(const Rows& src, int64_t row_bytes, int64_t n, const int64_t* d_
   if (ctas > (int64_t)kNumSM * 2) ctas = (int64_t)kNumSM * 2;  // persistent CTAs
   static std::atomic<uint64_t> done{0};
   SGL_CUDA_CHECK(allow_smem((const void*)bulk_rows_kernel<Rows, kBulkWarps, kBulkStages>, done, 200 * 1024));
-  return launch(bulk_rows_kernel<Rows, kBulkWarps, kBulkStages>, (unsigned)ctas, kBulkWarps * 32, smem, stream, src, (uint32_t)row_bytes, n,
-                d_n, (char*)out, rows_per_stage, d_status);
+  auto go = [&](auto how) -> int {
+    return how(bulk_rows_kernel<Rows, kBulkWarps, kBulkStages>, dim3((unsigned)ctas), dim3(kBulkWarps * 32), smem, stream, src, (uint32_t)row_bytes, n, d_n,
+               (char*)out, rows_per_stage, d_status);
+  };
+  if constexpr (Rows::kEarly) return go([](const auto&... a) { return launch_early(a...); });
+  else return go([](const auto&... a) { return launch(a...); });
 }
 
 // ---------------------------------------------------------------------------------------------------------------
 // cache
 // ---------------------------------------------------------------------------------------------------------------
 constexpr int kCacheThreads = 256;
+constexpr int kCachePer = 4;             // ids a thread takes, one behind the other (200,000 ids, one a thread 7.2 us, so 6.2: fewer totals for the last CTA)
+constexpr int kCacheTile = kCacheThreads * kCachePer;
 
 __global__ void __launch_bounds__(kCacheThreads)
 cache_lookup_kernel(const int32_t* __restrict__ hitmap, int64_t num_ids, const int64_t* __restrict__ ids, int64_t n,
                     int32_t* __restrict__ slot_ws, int32_t* __restrict__ rank_ws, int64_t* __restrict__ cta_miss,
                     unsigned int* done_counter, int64_t* d_counts, int32_t* d_status) {
-  const int64_t i = (int64_t)blockIdx.x * kCacheThreads + threadIdx.x;
-  int32_t slot = -1;
-  int miss = 0;
-  if (i < n) {
-    int64_t id = __ldg(ids + i);
-    if (id < 0 || id >= num_ids) {
+  const int64_t first = (int64_t)blockIdx.x * kCacheTile + threadIdx.x * kCachePer;
+  int64_t id[kCachePer];
+  int32_t slot[kCachePer];               // -2: neither hit nor reportable miss, the row is left untouched
+  int misses = 0;
+#pragma unroll
+  for (int u = 0; u < kCachePer; ++u) id[u] = first + u < n ? __ldg(ids + first + u) : 0;
+#pragma unroll
+  for (int u = 0; u < kCachePer; ++u) slot[u] = id[u] >= 0 && id[u] < num_ids ? __ldg(hitmap + id[u]) : -2;
+#pragma unroll
+  for (int u = 0; u < kCachePer; ++u) {
+    if (first + u >= n) continue;
+    if (id[u] < 0 || id[u] >= num_ids) {
       dev_flag(d_status, SGL_DEV_BAD_INDEX);
-      slot = -2;  // neither hit nor reportable miss: row is left untouched
-    } else {
-      slot = __ldg(hitmap + id);
-      miss = slot < 0 ? 1 : 0;
-      if (slot < 0) slot = -1;
+    } else if (slot[u] < 0) {
+      slot[u] = -1;
+      ++misses;
     }
   }
   int total;
-  int rank = cta_exclusive_scan<kCacheThreads, int>(miss, &total);
-  if (i < n) {
-    slot_ws[i] = slot;
-    rank_ws[i] = rank;
+  int rank = cta_exclusive_scan<kCacheThreads, int>(misses, &total);
+#pragma unroll
+  for (int u = 0; u < kCachePer; ++u) {
+    if (first + u >= n) continue;
+    slot_ws[first + u] = slot[u];
+    rank_ws[first + u] = rank;
+    rank += slot[u] == -1 ? 1 : 0;
   }
   if (publish_and_scan_cta_totals<kCacheThreads>((int64_t)total, cta_miss, done_counter, d_counts + 1) && threadIdx.x == 0)
     d_counts[0] = n - d_counts[1];
@@ -395,6 +435,8 @@ struct CachedRows {
     int64_t id;
     int32_t slot, rank;
   };
+  static constexpr bool kEarly = false;  // (reads what the lookup wrote through the read-only path)
+  __device__ __forceinline__ void begin() const {}
   __device__ __forceinline__ Key first(int64_t i) const { return {__ldg(ids + i), __ldg(slot_ws + i), __ldg(rank_ws + i)}; }
   __device__ __forceinline__ Key second(Key k) const { return k; }
   __device__ __forceinline__ const char* source(int64_t i, Key k, float*, int64_t*) const {
@@ -404,7 +446,7 @@ struct CachedRows {
       return nullptr;
     }
     if (k.slot != -1) return nullptr;
-    const int64_t p = __ldg(cta_miss + i / kCacheThreads) + k.rank;
+    const int64_t p = __ldg(cta_miss + i / kCacheTile) + k.rank;
     miss_pos[p] = i;
     miss_ids[p] = k.id;
     return backing + k.id * row_bytes;
@@ -440,7 +482,7 @@ cache_copy_kernel(const char* __restrict__ cache_rows, int64_t cache_slots, cons
         } else if (slot == -1) {
           int64_t id = __ldg(ids + i);
           if (l == 0) {
-            int64_t p = cta_miss[i / kCacheThreads] + rank_ws[i];
+            int64_t p = cta_miss[i / kCacheTile] + rank_ws[i];
             miss_pos[p] = i;
             miss_ids[p] = id;
           }
@@ -463,20 +505,24 @@ cache_copy_kernel(const char* __restrict__ cache_rows, int64_t cache_slots, cons
 // ---------------------------------------------------------------------------------------------------------------
 template <typename V>
 __global__ void __launch_bounds__(kLaneThreads)
-scatter_lanes_kernel(char* __restrict__ table, int64_t table_rows, uint32_t lanes_per_row, int64_t row_bytes,
-                     int64_t dst_pitch,
-                     const int64_t* __restrict__ idx, const int64_t* __restrict__ map, int64_t map_len, int64_t n_cap,
-                     const int64_t* d_n, const char* __restrict__ rows, int64_t src_pitch, float* __restrict__ ts_table,
-                     const float* __restrict__ ts, int split_last_col, int32_t* d_status) {
-  const int64_t n = eff_count(n_cap, d_n);
-  const int64_t total = n * lanes_per_row;
+scatter_lanes_kernel(char* table, int64_t table_rows, LaneSplit split, int64_t row_bytes, int64_t dst_pitch, const int64_t* idx,
+                     const int64_t* map, int64_t map_len, int64_t n_cap, const int64_t* d_n, const char* rows, int64_t src_pitch,
+                     float* ts_table, const float* ts, int split_last_col, int32_t* d_status) {
+  after_predecessor();
+  idx = current(idx);
+  map = current(map);
+  ts = current(ts);
+  const int64_t n = eff_count(n_cap, current(d_n));
+  const int64_t total = n * split.lanes;
   const int64_t stride = (int64_t)gridDim.x * kLaneThreads;
   for (int64_t q = (int64_t)blockIdx.x * kLaneThreads + threadIdx.x; q < total; q += stride) {
-    int64_t i = q / lanes_per_row;
-    uint32_t l = (uint32_t)(q - i * lanes_per_row);
+    int64_t i;
+    uint32_t l;
+    split(q, &i, &l);
+    const V v = ld_current((const V*)(rows + i * src_pitch) + l);        // (does not depend on where it goes)
     int64_t r;
     if (!resolve_row(idx, map, map_len, table_rows, i, false, d_status, &r)) continue;
-    ((V*)(table + r * dst_pitch))[l] = ((const V*)(rows + i * src_pitch))[l];
+    ((V*)(table + r * dst_pitch))[l] = v;
     if (l == 0 && ts_table) {
       if (split_last_col) ts_table[r] = *(const float*)(rows + i * src_pitch + row_bytes);
       else if (ts) ts_table[r] = ts[i];
@@ -777,13 +823,13 @@ extern "C" int sgl_gather_rows(const void* table, int64_t table_rows, int64_t ro
     SGL_REQUIRE(vec_ok, SGL_ERR_UNSUPPORTED, "gather_rows: 128-bit mode needs 16-byte aligned rows");
     const uint32_t lanes = (uint32_t)(row_bytes / 16);
     const int grid = stream_grid(n * lanes, kLaneThreads * kLaneUnroll, 8);
-    SGL_CHECK_RC(launch(gather_lanes_kernel<uint4>, grid, kLaneThreads, 0, stream, (const char*)table, table_rows,
+    SGL_CHECK_RC(launch_early(gather_lanes_kernel<uint4>, grid, kLaneThreads, 0, stream, (const char*)table, table_rows,
                         LaneSplit(lanes, n * lanes), src_pitch, idx, map, map_len, n, d_n, (char*)out, dst_pitch, ts_table,
                         out_ts, d_status));
   } else {
     const uint32_t lanes = (uint32_t)(row_bytes / 4);
     const int grid = stream_grid(n * lanes, kLaneThreads * kLaneUnroll, 8);
-    SGL_CHECK_RC(launch(gather_lanes_kernel<uint32_t>, grid, kLaneThreads, 0, stream, (const char*)table, table_rows,
+    SGL_CHECK_RC(launch_early(gather_lanes_kernel<uint32_t>, grid, kLaneThreads, 0, stream, (const char*)table, table_rows,
                         LaneSplit(lanes, n * lanes), src_pitch, idx, map, map_len, n, d_n, (char*)out, dst_pitch, ts_table,
                         out_ts, d_status));
   }
@@ -814,7 +860,7 @@ extern "C" int sgl_copy_prefix(int n_arrays, const void* const* src, void* const
 
 extern "C" size_t sgl_cache_gather_ws_bytes(int64_t n) {
   if (n < 1) n = 1;
-  int64_t ctas = (n + kCacheThreads - 1) / kCacheThreads;
+  int64_t ctas = (n + kCacheTile - 1) / kCacheTile;
   return 2 * align_up((size_t)n * 4) + align_up((size_t)ctas * 8) + align_up(sizeof(unsigned int));
 }
 
@@ -835,7 +881,7 @@ extern "C" int sgl_cache_gather(const void* cache_rows, int64_t cache_slots, con
   WsCarver c(ws, ws_bytes);
   int32_t* slot_ws = c.take<int32_t>(n);
   int32_t* rank_ws = c.take<int32_t>(n);
-  const int64_t ctas = (n + kCacheThreads - 1) / kCacheThreads;
+  const int64_t ctas = (n + kCacheTile - 1) / kCacheTile;
   int64_t* cta_miss = c.take<int64_t>(ctas);
   unsigned int* done = c.take<unsigned int>(1);
   SGL_REQUIRE(c.ok(), SGL_ERR_WORKSPACE, "cache_gather: workspace %zu < %zu bytes", ws_bytes, sgl_cache_gather_ws_bytes(n));
@@ -879,13 +925,13 @@ extern "C" int sgl_scatter_rows(void* table, int64_t table_rows, int64_t row_byt
   if (vec_ok) {
     const uint32_t lanes = (uint32_t)(row_bytes / 16);
     const int grid = stream_grid(n * lanes, kLaneThreads, 16);
-    SGL_CHECK_RC(launch(scatter_lanes_kernel<uint4>, grid, kLaneThreads, 0, stream, (char*)table, table_rows, lanes,
+    SGL_CHECK_RC(launch_early(scatter_lanes_kernel<uint4>, grid, kLaneThreads, 0, stream, (char*)table, table_rows, LaneSplit(lanes, n * lanes),
                         row_bytes, dst_pitch, idx, map, map_len, n, d_n, (const char*)rows, src_pitch, ts_table, ts,
                         split_last_col, d_status));
   } else {
     const uint32_t lanes = (uint32_t)(row_bytes / 4);
     const int grid = stream_grid(n * lanes, kLaneThreads, 16);
-    SGL_CHECK_RC(launch(scatter_lanes_kernel<uint32_t>, grid, kLaneThreads, 0, stream, (char*)table, table_rows, lanes,
+    SGL_CHECK_RC(launch_early(scatter_lanes_kernel<uint32_t>, grid, kLaneThreads, 0, stream, (char*)table, table_rows, LaneSplit(lanes, n * lanes),
                         row_bytes, dst_pitch, idx, map, map_len, n, d_n, (const char*)rows, src_pitch, ts_table, ts,
                         split_last_col, d_status));
   }

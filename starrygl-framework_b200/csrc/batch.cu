@@ -250,8 +250,8 @@ static int build_batch(const int64_t* indptr, const int64_t* nbr, const int64_t*
     }
     if (l > 0) {
       if (forked) SGL_CHECK_RC(order.wait(kRelabelled, side));
-      rc = by_rows(e) ? build_csc_rows(order_of, c, h.offs, fanouts[l], policy == SGL_POLICY_UNIFORM, h.dst, last_col, h.ts, h.dt, h.eid, e, d_edges, c, d_cur,
-                                       bits_for((uint64_t)c), ts_bits, ts_base, h.indptr, h.indices, h.cts, h.cdt, h.ceid, d_status, cws, cwb,
+      rc = by_rows(e) ? build_csc_rows(order_of, c, cur_ts, h.offs, fanouts[l], policy == SGL_POLICY_UNIFORM, h.dst, last_col, h.ts, h.dt, h.eid, e,
+                                       d_edges, c, d_cur, bits_for((uint64_t)c), ts_bits, ts_base, h.indptr, h.indices, h.cts, h.cdt, h.ceid, d_status, cws, cwb,
                                        side)
                       : sgl_build_csc(nullptr, h.dst, last_col, h.ts, h.dt, h.eid, e, d_edges, c, d_cur, bits_for((uint64_t)c), ts_bits,
                                       ts_base, h.indptr, h.indices, h.cts, h.cdt, h.ceid, 0, d_status, cws, cwb, side);

@@ -36,9 +36,10 @@ int unique_pairs(const int64_t* a_id, const int64_t* a_ts, int64_t n_a, const in
                  void* stream);
 
 size_t build_csc_rows_ws_bytes(int64_t n_edges, int64_t list_cap);
-// `list_cap` / d_num_dst: capacity of the list's order and its number of rows; offsets[i]: first edge of target i
-int build_csc_rows(const RowOrder& ro, int64_t list_cap, const int64_t* offsets, int fanout, bool draws, const int64_t* dst, const int64_t* dst_map,
-                   const int64_t* ts, const float* dt, const int64_t* eid, int64_t n_edges, const int64_t* d_n_edges, int64_t num_dst,
+// `list_cap` / d_num_dst: capacity of the list's order and its number of rows; row_ts: time of every row; offsets[i]: first edge of target
+// i; dt: the row's time minus the edge's, as the sampler writes it
+int build_csc_rows(const RowOrder& ro, int64_t list_cap, const int64_t* row_ts, const int64_t* offsets, int fanout, bool draws,
+                   const int64_t* dst, const int64_t* dst_map, const int64_t* ts, const float* dt, const int64_t* eid, int64_t n_edges, const int64_t* d_n_edges, int64_t num_dst,
                    const int64_t* d_num_dst, int dst_bits, int ts_bits, int64_t ts_base, int64_t* out_indptr, int64_t* out_indices,
                    int64_t* out_ts, float* out_dt, int64_t* out_eid, int32_t* d_status, void* ws, size_t ws_bytes, void* stream);
 

@@ -627,6 +627,14 @@ int sgl_build_batch_staged(const int64_t* indptr, const int64_t* nbr, const int6
                     const int32_t* fanouts, int n_hops, int policy, int equal_root_time, int64_t allowed_offset,
                     uint64_t seed, int id_bits, int ts_bits, int64_t ts_base, const int64_t* section_at,
                     int64_t* base, int64_t* other_base, int64_t* meta, int32_t* d_status, int64_t* host_meta, int64_t* host_early, void* ws, size_t ws_bytes, void* side_stream, void* stream);
+/* The same; host_ready (optional, one pinned word) becomes 1 when the CSC of the last hop is there as well: once both flags are set, all
+ * arrays but the last list, the columns of the last hop's edges and the last of the counts are what they will be, and may be read by other
+ * streams next to the merge of the last list. */
+int sgl_build_batch_ready(const int64_t* indptr, const int64_t* nbr, const int64_t* ts, const int64_t* eid, const int64_t* fence,
+                    int64_t num_nodes, const int64_t* roots, const int64_t* root_ts, int64_t n_roots,
+                    const int32_t* fanouts, int n_hops, int policy, int equal_root_time, int64_t allowed_offset,
+                    uint64_t seed, int id_bits, int ts_bits, int64_t ts_base, const int64_t* section_at,
+                    int64_t* base, int64_t* other_base, int64_t* meta, int32_t* d_status, int64_t* host_meta, int64_t* host_early, int64_t* host_ready, void* ws, size_t ws_bytes, void* side_stream, void* stream);
 
 /* ------------------------------------------------------------------------------------------------
  * One query of the graph API in one call: roots of the window [t_begin, t_end) (sgl_seeds_in_window), the negatives

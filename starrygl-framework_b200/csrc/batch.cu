@@ -166,13 +166,13 @@ extern "C" size_t sgl_build_batch_ws_bytes(int64_t n_roots, const int32_t* fanou
          order_ws(n_roots, fanouts, n_hops) + narrow_ws(n_roots, fanouts, n_hops);
 }
 
-// host_early: see sgl_build_batch_staged
+// host_early, host_ready: see sgl_build_batch_staged, sgl_build_batch_ready
 static int build_batch(const int64_t* indptr, const int64_t* nbr, const int64_t* ts, const int64_t* eid, const int64_t* fence,
                                   int64_t num_nodes, const int64_t* roots, const int64_t* root_ts, int64_t n_roots,
                                   const int32_t* fanouts, int n_hops, int policy, int equal_root_time, int64_t allowed_offset,
                                   uint64_t seed, int id_bits, int ts_bits, int64_t ts_base, const int64_t* section_at, int64_t* base,
-                                  int64_t* other_base, int64_t* meta, int32_t* d_status, int64_t* host_meta, int64_t* host_early, void* ws,
-                                  size_t ws_bytes, void* side_stream, void* stream_) {
+                                  int64_t* other_base, int64_t* meta, int32_t* d_status, int64_t* host_meta, int64_t* host_early,
+                                  int64_t* host_ready, void* ws, size_t ws_bytes, void* side_stream, void* stream_) {
   SGL_NVTX("sgl_build_batch");
   cudaStream_t stream = (cudaStream_t)stream_;
   SGL_REQUIRE(n_roots >= 0 && n_hops >= 0 && (n_hops == 0 || fanouts), SGL_ERR_ARG, "build_batch: bad size");
@@ -182,6 +182,7 @@ static int build_batch(const int64_t* indptr, const int64_t* nbr, const int64_t*
   SGL_CHECK_RC(zero_async(meta, (size_t)(2 + 2 * n_hops) * sizeof(int64_t), stream));
   auto done = [&]() -> int {
     if (host_early) SGL_CHECK_RC(export_words(meta, host_early, 1 + 2 * n_hops, stream));      // (no roots, or no hops)
+    if (host_ready) SGL_CHECK_RC(export_words(meta, host_ready, 0, stream));
     if (host_meta) SGL_CHECK_RC(export_words(meta, host_meta, 2 + 2 * n_hops, stream));
     return scope.submit();
   };
@@ -258,6 +259,10 @@ static int build_batch(const int64_t* indptr, const int64_t* nbr, const int64_t*
       if (rc) return rc;
       if (forked) SGL_CHECK_RC(order.mark(kCsc, side));
     }
+    if (host_ready && l + 1 == n_hops) {
+      SGL_CHECK_RC(export_words(meta, host_ready, 0, l > 0 ? side : stream));
+      host_ready = nullptr;
+    }
     order_of = RowOrder{};
     if (l + 1 < n_hops && by_rows(e * fanouts[l + 1])) {
       order_of = RowOrder::carve(ows, c + e);
@@ -301,7 +306,8 @@ extern "C" int sgl_build_batch_at(const int64_t* indptr, const int64_t* nbr, con
                                   int64_t* other_base, int64_t* meta, int32_t* d_status, int64_t* host_meta, void* ws, size_t ws_bytes,
                                   void* side_stream, void* stream) {
   return build_batch(indptr, nbr, ts, eid, fence, num_nodes, roots, root_ts, n_roots, fanouts, n_hops, policy, equal_root_time, allowed_offset, seed,
-                     id_bits, ts_bits, ts_base, section_at, base, other_base, meta, d_status, host_meta, nullptr, ws, ws_bytes, side_stream, stream);
+                     id_bits, ts_bits, ts_base, section_at, base, other_base, meta, d_status, host_meta, nullptr, nullptr, ws, ws_bytes, side_stream,
+                     stream);
 }
 
 extern "C" int sgl_build_batch_staged(const int64_t* indptr, const int64_t* nbr, const int64_t* ts, const int64_t* eid, const int64_t* fence,
@@ -311,8 +317,19 @@ extern "C" int sgl_build_batch_staged(const int64_t* indptr, const int64_t* nbr,
                                       int64_t* other_base, int64_t* meta, int32_t* d_status, int64_t* host_meta, int64_t* host_early,
                                       void* ws, size_t ws_bytes, void* side_stream, void* stream) {
   return build_batch(indptr, nbr, ts, eid, fence, num_nodes, roots, root_ts, n_roots, fanouts, n_hops, policy, equal_root_time, allowed_offset, seed,
-                     id_bits, ts_bits, ts_base, section_at, base, other_base, meta, d_status, host_meta, host_early, ws, ws_bytes, side_stream,
-                     stream);
+                     id_bits, ts_bits, ts_base, section_at, base, other_base, meta, d_status, host_meta, host_early, nullptr, ws, ws_bytes,
+                     side_stream, stream);
+}
+
+extern "C" int sgl_build_batch_ready(const int64_t* indptr, const int64_t* nbr, const int64_t* ts, const int64_t* eid, const int64_t* fence,
+                                      int64_t num_nodes, const int64_t* roots, const int64_t* root_ts, int64_t n_roots,
+                                      const int32_t* fanouts, int n_hops, int policy, int equal_root_time, int64_t allowed_offset,
+                                      uint64_t seed, int id_bits, int ts_bits, int64_t ts_base, const int64_t* section_at, int64_t* base,
+                                      int64_t* other_base, int64_t* meta, int32_t* d_status, int64_t* host_meta, int64_t* host_early,
+                                      int64_t* host_ready, void* ws, size_t ws_bytes, void* side_stream, void* stream) {
+  return build_batch(indptr, nbr, ts, eid, fence, num_nodes, roots, root_ts, n_roots, fanouts, n_hops, policy, equal_root_time, allowed_offset, seed,
+                     id_bits, ts_bits, ts_base, section_at, base, other_base, meta, d_status, host_meta, host_early, host_ready, ws, ws_bytes,
+                     side_stream, stream);
 }
 
 extern "C" int sgl_build_batch(const int64_t* indptr, const int64_t* nbr, const int64_t* ts, const int64_t* eid, const int64_t* fence,

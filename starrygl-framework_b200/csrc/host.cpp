@@ -515,11 +515,11 @@ int64_t* at_graph(PyObject* o) { return o == Py_None ? nullptr : (int64_t*)tenso
 
 // (indptr, nbr, ts, eid, fence, num_nodes, roots, root_ts, fan-outs, hops, policy, equal_root_time, allowed_offset, seed, id_bits, ts_bits,
 //  lowest time, places, words of the results (0: the places are addresses), words of the raw arrays (-1: they lie behind the results),
-//  words of meta behind the raw arrays (0: meta is given), meta, bytes of scratch, status, host words, early host words, side stream)
+//  words of meta behind the raw arrays (0: meta is given), meta, bytes of scratch, status, host words, early ones, ready one, side stream)
 // -> (results or None, raw arrays)
 PyObject* build_batch(PyObject*, Args a, Py_ssize_t n_args) {
   return guarded([&]() -> PyObject* {
-    count("build_batch", n_args, 27);
+    count("build_batch", n_args, 28);
     const at::Device dev = tensor(a[0]).device();
     const at::Tensor roots = i64(a[6]), root_ts = i64(a[7]);
     const int64_t n = roots.numel();
@@ -545,14 +545,14 @@ PyObject* build_batch(PyObject*, Args a, Py_ssize_t n_args) {
     const uint64_t seed = argument<uint64_t>(a[13]);
     const int64_t* const places = argument<const int64_t*>(a[17]);
     int32_t* const status = argument<int32_t*>(a[23]);
-    int64_t *const host = argument<int64_t*>(a[24]), *const early = argument<int64_t*>(a[25]);
-    void *const side = argument<void*>(a[26]), *const on = stream();
+    int64_t *const host = argument<int64_t*>(a[24]), *const early = argument<int64_t*>(a[25]), *const ready = argument<int64_t*>(a[26]);
+    void *const side = argument<void*>(a[27]), *const on = stream();
     const Scratch ws(argument<size_t>(a[22]), dev, on);
     int rc;
     {
       Unlocked u;
-      rc = sgl_build_batch_staged(g_ptr, g_nbr, g_ts, g_eid, g_fence, num_nodes, p_roots, p_times, n, fan, hops, policy, equal, offset, seed, id_bits,
-                                  ts_bits, lowest, places, base, other, meta, status, host, early, ws.p, ws.n, side, on);
+      rc = sgl_build_batch_ready(g_ptr, g_nbr, g_ts, g_eid, g_fence, num_nodes, p_roots, p_times, n, fan, hops, policy, equal, offset, seed, id_bits,
+                                 ts_bits, lowest, places, base, other, meta, status, host, early, ready, ws.p, ws.n, side, on);
     }
     check(rc);
     return tuple({results, raw});

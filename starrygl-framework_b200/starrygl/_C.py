@@ -128,6 +128,8 @@ _SIGNATURES = {
                                   _vp, _vp, _vp, _vp, _vp, _vp, _vp, _sz, _vp, _vp]),
     "sgl_build_batch_staged": (_i32, [_vp, _vp, _vp, _vp, _vp, _i64, _vp, _vp, _i64, _vp, _i32, _i32, _i32, _i64, _u64, _i32, _i32, _i64,
                                       _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _sz, _vp, _vp]),
+    "sgl_build_batch_ready": (_i32, [_vp, _vp, _vp, _vp, _vp, _i64, _vp, _vp, _i64, _vp, _i32, _i32, _i32, _i64, _u64, _i32, _i32, _i64,
+                                     _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _sz, _vp, _vp]),
     "sgl_query_layout": (_i64, [_i64, _i64, _i32, _i32, _vp]),
     "sgl_query_ws_bytes": (_sz, [_i64, _i64, _i32, _i32]),
     "sgl_query": (_i32, [_vp, _vp, _vp, _vp, _vp, _i64, _vp, _vp, _vp, _i64, _i64, _i64, _i64, _vp, _vp, _i64, _vp, _vp, _i64, _i32, _i32,

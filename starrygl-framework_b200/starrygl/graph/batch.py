@@ -232,9 +232,9 @@ class DeviceBatch:
 
 
 def _enqueue(g, roots, root_ts, fanouts, policy, lo, hi, equal_root_time, allowed_offset, seed, status, side, host=None,
-             meta=None, together=False, early=None) -> DeviceBatch:
+             meta=None, together=False, early=None, ready=None) -> DeviceBatch:
     """``lo`` / ``hi``: lowest and highest timestamp that can occur; ``host``: pinned address that receives the counts, ``early`` one
-    that receives all but the last while the last list is merged;
+    that receives all but the last while the last list is merged, ``ready`` that of a word that becomes 1 when everything else is there;
     ``meta``: block of 2 + 2 * hops device words for the counts and the status (default: behind the raw arrays);
     ``together``: one allocation for the results whatever their size (for callers that keep none of them)."""
     n, hops = roots.numel(), len(fanouts)
@@ -250,7 +250,7 @@ def _enqueue(g, roots, root_ts, fanouts, policy, lo, hi, equal_root_time, allowe
         g.indptr, g.nbr, g.ts, g.eid, g.fence, g.num_nodes, roots, root_ts, plan.fan_at, hops,
         _C.POLICY[policy] if isinstance(policy, str) else int(policy), bool(equal_root_time), int(allowed_offset), int(seed),
         ops.bits_for(g.num_nodes - 1), ops.bits_for(hi - lo), lo, at, words, -1 if plan.whole else plan.raw_words,
-        2 + 2 * hops if meta is None else 0, meta, plan.ws_bytes, None if status is None else status.ptr(), host, early,
+        2 + 2 * hops if meta is None else 0, meta, plan.ws_bytes, None if status is None else status.ptr(), host, early, ready,
         None if side is None else side.cuda_stream)
     return DeviceBatch(g, n, fanouts, plan, results if kept is None else kept, raw, meta, status)
 

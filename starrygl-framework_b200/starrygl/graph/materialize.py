@@ -22,12 +22,13 @@ import torch
 
 from .. import _C, ops
 from ..cache.cache_route import CommPlan
-from .batch import _enqueue, _graph_range, _root_range
+from .batch import _EARLY, _HOP, _enqueue, _graph_range, _root_range
 
 
 _PINNED_MOST, _PINNED_TOTAL = 256 << 20, 2 << 30
 _SHARED_MOST = 32 << 20
-_STAGE = threading.local()                # pinned buffer for the roots of a thread's tasks
+_STAGE = threading.local()                # of a thread: pinned buffer for the roots of its tasks, a stream per device for early copies
+_READY = 511                              # place of the word that says so among the thread's result words
 
 
 def _pinned_now() -> int:
@@ -113,8 +114,9 @@ class MaterializedMultiLayerBuilder:
 
     # ---- layers and route plans of one slot on the host (prepare_sample.py:266-310) -------------------------------
     def _build(self, roots, root_ts, ts_range, fanouts, policy, inclusive, seed) -> List[dict]:
-        """Batch, then the plan of every layer list, all enqueued without a host round trip; one read-back of every size;
-        one copy of every array."""
+        """Batch, then the plan of every layer list, all enqueued without a host round trip; the arrays that are there before the last list
+        is merged cross PCIe next to that merge and the plans (8,000 roots, two hops, 8 MB: 437 us, so 390 - 407), the others after one
+        read-back of every size."""
         g, L, P, hops = self.g, _C.lib(), self.num_parts, len(fanouts)
         if ts_range is None:
             ts_range = _root_range(g, root_ts)
@@ -122,7 +124,10 @@ class MaterializedMultiLayerBuilder:
         nb = 2 + 2 * hops
         meta = torch.empty(nb + ((hops + 1) * (P + 1) if planned else 0), dtype=torch.int64, device=self.device)
         lo, hi = _graph_range(g, *ts_range)
-        db = _enqueue(g, roots, root_ts, fanouts, policy, lo, hi, inclusive, -1, seed, None, None, None, meta[:nb], True)
+        addr, result = _C.host_words()
+        staged = hops > 0 and roots.numel() > 0 and meta.numel() < _EARLY and _EARLY + nb < _READY
+        db = _enqueue(g, roots, root_ts, fanouts, policy, lo, hi, inclusive, -1, seed, None, None, None, meta[:nb], True,
+                      addr + 8 * _EARLY if staged else None, addr + 8 * _READY if staged else None)
         lists = []                                  # (address of the ids, capacity) of every layer list
         n = c = t = roots.numel()
         place = db.addresses()
@@ -149,6 +154,51 @@ class MaterializedMultiLayerBuilder:
             _C.host().sgl_plan_routes(k, ref(ids), ref(ns), ref(d_ns), self.node_parts.data_ptr(), self.node_parts.numel(), self.pid,
                                       rt.indptr.data_ptr(), rt.indices.data_ptr(), rt.locs.data_ptr(), P, ref(cp), ref(outs), ref(cnts),
                                       mp + 8 * (nb - 1), ws.data_ptr(), ws.numel(), sp)
+        early = copies = None
+        try:
+            if staged:
+                sp, wait = _C.stream_ptr(), _C.host().sgl_wait_word
+                wait(addr + 8 * (_EARLY + nb - 1), 1, sp)
+                counts = result[_EARLY:_EARLY + nb - 1]
+                if 0 not in counts[1::2]:
+                    picks = self._picks(place, counts, n, hops, "early")
+                    copies = self._copies()
+                    with _C.on_stream(copies):
+                        early = list(zip(picks, self._export([p[2:] for p in picks], lambda: wait(addr + 8 * _READY, 1, sp))))
+            return self._finish(db, meta, place, n, hops, plans, early)
+        finally:
+            if copies is not None:                  # (whatever becomes of the slot: they write to memory of its own)
+                copies.synchronize()
+
+    def _copies(self):
+        """The calling thread's stream for copies next to what its current stream does."""
+        streams = _STAGE.__dict__.setdefault("streams", {})
+        s = streams.get(self.device.index)
+        if s is None:
+            s = streams[self.device.index] = torch.cuda.Stream(self.device)
+        return s
+
+    @staticmethod
+    def _picks(place, host, n, hops, part):
+        """(layer, name, address, count, bytes per value) of the layers' arrays: those that are there before the last list is merged
+        ("early"; the last of the counts is not looked at), the others ("late"), or all."""
+        out = []
+
+        def sec(layer, name, section, count, size=8, late=False):
+            if part == "all" or late == (part == "late"):
+                out.append((layer, name, place[section], count, size))
+        sec(0, "gids", 0, host[0]); sec(0, "ts", 1, host[0]); sec(0, "inv_map", 2, n)
+        for l in range(hops):
+            e, b, last = host[1 + 2 * l], 3 + 14 * l, l + 1 == hops
+            ip, ix, ts, dt, ei = (5, 8, 2, 3, 4) if l == 0 else (9, 10, 11, 12, 13)
+            sec(l + 1, "indptr", b + ip, host[2 * l] + 1); sec(l + 1, "indices", b + ix, e, 8, last); sec(l + 1, "eid", b + ei, e)
+            sec(l + 1, "edge_ts", b + ts, e); sec(l + 1, "edge_dt", b + dt, e, 4)
+            sec(l + 1, "gids", b + 6, host[2 + 2 * l], 8, last); sec(l + 1, "ts", b + 7, host[2 + 2 * l], 8, last)
+        return out
+
+    def _finish(self, db, meta, place, n, hops, plans, early) -> List[dict]:
+        """``early``: the early arrays of the layers on the host, on their way; None: nothing is."""
+        P, nb = self.num_parts, 2 + 2 * hops
         host = _C.read_words(meta, meta.numel()) if meta.numel() < 512 else meta.tolist()    # the one synchronisation before the copy
         bits = host[nb - 1] & 0xFFFFFFFF
         if bits:
@@ -159,26 +209,15 @@ class MaterializedMultiLayerBuilder:
             layers = db._trim(host[:nb - 1])
             if len(layers) == hops + 1 and layers[-1]["indptr"].numel() > 1:
                 layers = None
-        picks = []                                  # (address, count, bytes per value) in the order of the result
-        if layers is None:
-            sec = lambda i, count, size=8: picks.append((place[i], count, size))
-            sec(0, host[0]); sec(1, host[0]); sec(2, n)
-            prev = host[0]
-            for l in range(hops):
-                e, nxt, b = host[1 + 2 * l], host[2 + 2 * l], 3 + 14 * l
-                ip, ix, ts, dt, ei = (5, 8, 2, 3, 4) if l == 0 else (9, 10, 11, 12, 13)
-                sec(b + ip, prev + 1); sec(b + ix, e); sec(b + ei, e); sec(b + ts, e); sec(b + dt, e, 4); sec(b + 6, nxt); sec(b + 7, nxt)
-                prev = nxt
+        picks = self._picks(place, host, n, hops, "all" if early is None else "late") if layers is None else []
         sizes = [host[nb + i * (P + 1):nb + (i + 1) * (P + 1)] for i in range(len(plans))]
-        for (at, cap), s in zip(plans, sizes):
-            for j in range(3):
-                picks.append((at + 8 * j * cap, s[P], 8))
-        got = self._export(picks)
+        routed = [(at + 8 * j * cap, s[P], 8) for (at, cap), s in zip(plans, sizes) for j in range(3)]
+        got = self._export([p[2:] for p in picks] + routed)
         if layers is None:
-            names = ("indptr", "indices", "eid", "edge_ts", "edge_dt", "gids", "ts")
-            final = [dict(zip(("gids", "ts", "inv_map"), got[:3]))]
-            final += [dict(zip(names, got[3 + 7 * l:10 + 7 * l])) for l in range(hops)]
-            got = got[3 + 7 * hops:]
+            arrays = {p[:2]: t for p, t in [*(early or ()), *zip(picks, got)]}
+            final = [{k: arrays[0, k] for k in ("gids", "ts", "inv_map")}]
+            final += [{k: arrays[l, k] for k in _HOP} for l in range(1, hops + 1)]
+            got = got[len(picks):]
         else:
             final = [{k: v.cpu() for k, v in d.items()} for d in layers]
         routes = []
@@ -194,10 +233,10 @@ class MaterializedMultiLayerBuilder:
         _C.current_stream(self.device).synchronize()               # the copies of _export
         return final
 
-    def _export(self, picks):
-        """Host tensors of device arrays (address, count, bytes per value), on their way: the caller waits for the copies.  Up to
-        32 MiB in all they are pieces of one buffer, packed by a kernel and filled by one copy, above that (and above the kernel's
-        96 arrays, nine hops) each has its own.
+    def _export(self, picks, ready=None):
+        """Host tensors of device arrays (address, count, bytes per value), on their way: the caller waits for the copies.  ``ready``
+        returns once the arrays may be read.  Up to 32 MiB in all they are pieces of one buffer, packed by a kernel and filled by one
+        copy, above that (and above the kernel's 96 arrays, nine hops) each has its own.
         The memory is pinned (a copy to fresh pageable memory takes several times as long) as long as not too much is."""
         n, at, offs = len(picks), 0, []
         for _, count, size in picks:
@@ -208,11 +247,15 @@ class MaterializedMultiLayerBuilder:
         types = {8: torch.int64, 4: torch.float32}
         if at > _SHARED_MOST or n > 96:
             out = [torch.empty(count, dtype=types[s], pin_memory=pin) for _, count, s in picks]
+            if ready is not None:
+                ready()
             _C.check(_C.lib().sgl_copy_arrays(n, src, size, (C.c_void_p * n)(*[t.data_ptr() for t in out]), _C.stream_ptr()))
             return out
         h = torch.empty(at // 8, dtype=torch.int64, pin_memory=pin)
         d = torch.empty(max(at, 16) // 8, dtype=torch.int64, device=self.device)
         places, ref = (C.c_int64 * max(n, 1))(*offs), C.addressof
+        if ready is not None:
+            ready()
         _C.host().sgl_export_arrays(n, ref(src), ref(size), ref(places), d.data_ptr(), h.data_ptr(), at, None, at, _C.stream_ptr())
         # (pieces with a storage of their own size: what saves or shares one does not take the others along)
         buf = h.numpy()

@@ -141,7 +141,7 @@ __device__ __forceinline__ uint64_t look_back(uint64_t* state, int pass, int til
     uint64_t w[kWide];
 #pragma unroll
     for (int u = 0; u < kWide; ++u) w[u] = t - u >= 0 ? st[(size_t)(t - u) * kRadix] : 0;
-    bool done = false, stalled = false;
+    bool done = false, stalled = limit == 0;       // (no patience: given up whether it would have waited or not)
 #pragma unroll
     for (int u = 0; u < kWide; ++u) {
       if (done || stalled || t < 0) continue;

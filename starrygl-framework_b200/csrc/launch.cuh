@@ -120,7 +120,7 @@ int launch(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStr
 
 // A kernel that a call launches by itself may be set up while the one before it on the stream still runs (programmatic stream
 // serialization): a gather of 22 us and a scatter of 6 were 1.8 us apart, and
-// a pass of both took 32.8 us, 31.7 so.  Such a kernel calls after_predecessor()
+// a pass of both took 32.8 us, 27.1 so (31.7 when a kernel let the next one in at its start: it holds what the running one needs).  Such a kernel calls after_predecessor()
 // before it touches memory, reads what others may have written through pointers that current() has handed out behind that, and not
 // through the read-only path, which may be served from before.  In a scope the launch is an ordinary one.
 template <class... KArgs, class... Args>
@@ -141,10 +141,7 @@ int launch_early(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, c
 }
 
 #ifdef __CUDACC__
-__device__ __forceinline__ void after_predecessor() {
-  asm volatile("griddepcontrol.wait;" ::: "memory");
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");        // (the next one waits for this one's end as well)
-}
+__device__ __forceinline__ void after_predecessor() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 // p, in a form that the compiler knows only from here on
 template <class T>
 __device__ __forceinline__ T* current(T* p) {

@@ -136,12 +136,18 @@ __device__ __forceinline__ uint64_t look_back(uint64_t* state, int pass, int til
   volatile uint64_t* st = state + threadIdx.x;
   uint64_t sum = 0;
   unsigned long long t0 = 0;
+  if (limit == 0) {                      // (no patience: given up whether it would have waited or not; not in the loop, where it cost 3 %)
+    dev_flag(d_status, SGL_DEV_TIMEOUT);
+    *(volatile unsigned int*)gave_up = 1u;
+    st[(size_t)tile * kRadix] = kAll | tag | total;
+    return 0;
+  }
   // (tiles are taken in order: those before this one are running or done)
   for (int t = tile - 1; t >= 0;) {
     uint64_t w[kWide];
 #pragma unroll
     for (int u = 0; u < kWide; ++u) w[u] = t - u >= 0 ? st[(size_t)(t - u) * kRadix] : 0;
-    bool done = false, stalled = limit == 0;       // (no patience: given up whether it would have waited or not)
+    bool done = false, stalled = false;
 #pragma unroll
     for (int u = 0; u < kWide; ++u) {
       if (done || stalled || t < 0) continue;

@@ -79,29 +79,9 @@ struct LaneSplit {
   }
 };
 
-// resolve the source/destination row of item i; returns false when the row must be skipped
-__device__ __forceinline__ bool resolve_row(const int64_t* idx, const int64_t* map, int64_t map_len, int64_t table_rows, int64_t i,
-                                            bool wrap_negative, int32_t* d_status, int64_t* row) {
-  int64_t r = idx[i];
-  if (map) {
-    if (r < 0 || r >= map_len) {
-      dev_flag(d_status, SGL_DEV_BAD_INDEX);
-      return false;
-    }
-    r = map[r];
-  }
-  if (r < 0) {
-    if (!wrap_negative) return false;  // "not stored here": skipped silently
-    r += table_rows;
-  }
-  if (r < 0 || r >= table_rows) {
-    dev_flag(d_status, SGL_DEV_BAD_INDEX);
-    return false;
-  }
-  *row = r;
-  return true;
-}
-
+// Rows through 16- or 4-byte lanes; rows below 0 count from the end.  Every step for all of a thread's pieces before the next one, so that
+// the loads of one do not wait for the others', and what is out of range is flagged at the end: an atomic in between keeps them apart
+// (90,000 rows of 1,544 bytes with their times, many of them twice: 166 us with the flags and the times in between, 135 so).
 template <typename V>
 __global__ void __launch_bounds__(kLaneThreads)
 gather_lanes_kernel(const char* table, int64_t table_rows, LaneSplit split, int64_t src_pitch, const int64_t* idx, const int64_t* map,
@@ -115,34 +95,47 @@ gather_lanes_kernel(const char* table, int64_t table_rows, LaneSplit split, int6
   const int64_t total = n * split.lanes;
   const int64_t stride = (int64_t)gridDim.x * kLaneThreads;
   for (int64_t q0 = (int64_t)blockIdx.x * kLaneThreads + threadIdx.x; q0 < total; q0 += stride * kLaneUnroll) {
-    // (every step for all of a thread's pieces before the next one: the loads of one do not wait for the others')
     V v[kLaneUnroll];
-    V* dst[kLaneUnroll];
     int64_t row[kLaneUnroll], at[kLaneUnroll];
     uint32_t lane[kLaneUnroll];
+    float t[kLaneUnroll];
+    bool bad = false;
 #pragma unroll
     for (int u = 0; u < kLaneUnroll; ++u) {
       const int64_t q = q0 + u * stride;
-      dst[u] = nullptr;
-      at[u] = -1;
+      at[u] = -1;                        // (nothing to copy)
+      row[u] = 0;
       if (q < total) {
-        int64_t i;
-        split(q, &i, &lane[u]);
-        if (resolve_row(idx, map, map_len, table_rows, i, true, d_status, &row[u])) at[u] = i;
+        split(q, &at[u], &lane[u]);
+        row[u] = idx[at[u]];
       }
+    }
+    if (map) {
+#pragma unroll
+      for (int u = 0; u < kLaneUnroll; ++u) {
+        if (at[u] < 0) continue;
+        if (row[u] >= 0 && row[u] < map_len) row[u] = map[row[u]];
+        else bad = true, at[u] = -1;
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < kLaneUnroll; ++u) {
+      if (row[u] < 0) row[u] += table_rows;
+      if (at[u] >= 0 && (row[u] < 0 || row[u] >= table_rows)) bad = true, at[u] = -1;
     }
 #pragma unroll
     for (int u = 0; u < kLaneUnroll; ++u) {
       if (at[u] < 0) continue;
       v[u] = ld_current((const V*)(table + row[u] * src_pitch) + lane[u]);
-      dst[u] = (V*)(out + at[u] * dst_pitch) + lane[u];
+      if (lane[u] == 0 && ts_table) t[u] = ts_table[row[u]];
     }
 #pragma unroll
     for (int u = 0; u < kLaneUnroll; ++u) {
-      if (dst[u] == nullptr) continue;
-      if (lane[u] == 0 && ts_table) out_ts[at[u]] = ts_table[row[u]];
-      st_stream(dst[u], v[u]);
+      if (at[u] < 0) continue;
+      st_stream((V*)(out + at[u] * dst_pitch) + lane[u], v[u]);
+      if (lane[u] == 0 && ts_table) out_ts[at[u]] = t[u];
     }
+    if (bad) dev_flag(d_status, SGL_DEV_BAD_INDEX);
   }
 }
 
@@ -503,6 +496,22 @@ cache_copy_kernel(const char* __restrict__ cache_rows, int64_t cache_slots, cons
 // ---------------------------------------------------------------------------------------------------------------
 // scatter / route helpers
 // ---------------------------------------------------------------------------------------------------------------
+// destination row of item i; false when there is none: below 0 ("not stored here", skipped silently) or out of range
+__device__ __forceinline__ bool resolve_row(const int64_t* idx, const int64_t* map, int64_t map_len, int64_t table_rows, int64_t i,
+                                            int32_t* d_status, int64_t* row) {
+  int64_t r = idx[i];
+  if (map) {
+    if (r < 0 || r >= map_len) {
+      dev_flag(d_status, SGL_DEV_BAD_INDEX);
+      return false;
+    }
+    r = map[r];
+  }
+  if (r >= table_rows) dev_flag(d_status, SGL_DEV_BAD_INDEX);
+  *row = r;
+  return r >= 0 && r < table_rows;
+}
+
 // A piece is read once its destination is known: source rows of items without one need not exist.  (Reading it first was no gain where
 // it counts: 400,000 rows of 400 bytes 90 us, so 79; two or four pieces of a thread side by side 87, 88.)
 template <typename V>
@@ -523,7 +532,7 @@ scatter_lanes_kernel(char* table, int64_t table_rows, LaneSplit split, int64_t r
     uint32_t l;
     split(q, &i, &l);
     int64_t r;
-    if (!resolve_row(idx, map, map_len, table_rows, i, false, d_status, &r)) continue;
+    if (!resolve_row(idx, map, map_len, table_rows, i, d_status, &r)) continue;
     ((V*)(table + r * dst_pitch))[l] = ((const V*)(rows + i * src_pitch))[l];
     if (l == 0 && ts_table) {
       if (split_last_col) ts_table[r] = *(const float*)(rows + i * src_pitch + row_bytes);

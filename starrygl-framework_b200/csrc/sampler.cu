@@ -279,11 +279,13 @@ sample_count_kernel(const SampleArgs a) {
 // copy loop is then a handful of instructions around its three loads.  (It was issue bound: 100 - 170 instructions per edge,
 // 384,000 x 20 recent 101 us, a drawn hop of 4.2 M x 10 targets 458 us.)
 constexpr int kMapFanout = 32;
-// Without draws the kernel needs few registers, and the copy wants CTAs (384,000 x 20 recent: one kernel for both, 62 registers, 90.6 us;
-// bounded to six CTAs per SM 84.7, to eight 84.5, four elements in flight per thread 86 - 111; 32, 128 and 256 targets per CTA 85, 86, 90).
-// Targets that draw were no faster with more CTAs and spills.
-template <int CT, int FT, bool DRAWS>
-__global__ void __launch_bounds__(kCtaThreads, DRAWS ? 4 : 6)
+// COPY: windows that are copied, up to kMapFanout edges each.  Without draws the kernel needs few registers, and the copy wants CTAs
+// (384,000 x 20 recent: one kernel for both, 62 registers, 90.6 us; bounded to six CTAs per SM 84.7, to eight 84.5, four elements in flight
+// per thread 86 - 111; 32, 128 and 256 targets per CTA 85, 86, 90).  Everything else keeps the kernel for both: one for draws alone was
+// slower (uniform, 16,384 targets: fan-out 33 53.2 -> 59.4 us, 100 158 -> 175), and so were six CTAs where there is no map (recent, 65,536
+// targets, fan-out 100: 70.3 -> 71.8).
+template <int CT, int FT, bool COPY>
+__global__ void __launch_bounds__(kCtaThreads, COPY ? 6 : 0)
 sample_fill_kernel(const SampleArgs a, int count_ctas) {
   static_assert(CT % FT == 0 && CT <= kCtaThreads && FT % kWarpsPerCta == 0, "fill CTAs tile the count CTAs");
   constexpr bool kLaneDraws = CT != kWarpsPerCta;          // picks by the target's lane instead of its warp
@@ -331,8 +333,7 @@ sample_fill_kernel(const SampleArgs a, int count_ctas) {
     base = a.cta_sums[count_cta];
     if (threadIdx.x == 0 && first + FT >= a.n_cap && a.total_out) *a.total_out = a.out_offsets[a.n_cap];
   }
-  constexpr bool draws = DRAWS;
-  const bool has_map = fanout <= kMapFanout;
+  const bool draws = !COPY && a.policy == SGL_POLICY_UNIFORM, has_map = COPY || fanout <= kMapFanout;
   const bool drawn = draws && cut - lo > fanout;           // (of this thread's target)
   if (mine) {
     s_ex[slot] = ex;
@@ -559,8 +560,9 @@ static int launch_sample(const SampleArgs& a, cudaStream_t stream, int64_t* host
   }
   if (a.fanout <= kMapFanout) smem += (size_t)FT * a.fanout;
   const unsigned fill_ctas = (unsigned)((a.n_cap + FT - 1) / FT);
-  return a.policy == SGL_POLICY_UNIFORM ? launch(sample_fill_kernel<CT, FT, true>, fill_ctas, kCtaThreads, smem, stream, a, (int)ctas)
-                                        : launch(sample_fill_kernel<CT, FT, false>, fill_ctas, kCtaThreads, smem, stream, a, (int)ctas);
+  return a.policy != SGL_POLICY_UNIFORM && a.fanout <= kMapFanout
+             ? launch(sample_fill_kernel<CT, FT, true>, fill_ctas, kCtaThreads, smem, stream, a, (int)ctas)
+             : launch(sample_fill_kernel<CT, FT, false>, fill_ctas, kCtaThreads, smem, stream, a, (int)ctas);
 }
 
 int sgl::sample_layer(const int64_t* indptr, const int64_t* nbr, const int64_t* ts, const int64_t* eid, const int64_t* fence,

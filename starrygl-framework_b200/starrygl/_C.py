@@ -265,6 +265,16 @@ def host_words():
     return h
 
 
+def abandon():
+    """A call that fails behind its launches waits for the current stream: what is still running writes to the thread's result words, and the
+    thread's next call would take it for its own.  (A capturing stream runs nothing.)"""
+    try:
+        if not torch._C._cuda_isCurrentStreamCapturing():
+            current_stream().synchronize()
+    except RuntimeError:
+        pass                             # (the call's own error says more)
+
+
 class CountRing:
     """Pinned (value, sequence number) pairs that kernels fill in with a count the host may ask for later.  A pair is used
     again after as many calls as there are pairs, once its count has arrived -- so that one kernel at a time may write to it;

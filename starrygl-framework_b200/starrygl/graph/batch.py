@@ -311,14 +311,18 @@ def build_batch(g, roots, root_ts, fanouts, policy="recent", **kw) -> List[dict]
     if last + 2 > len(words):
         return build_batch_async(g, roots, root_ts, fanouts, policy, **kw).finish()
     staged = bool(fanouts) and roots.numel() > 0 and last + 2 <= _EARLY
-    db = _enqueue(g, roots, root_ts, fanouts, policy, g.ts_min, g.ts_max, kw.get("equal_root_time", False), kw.get("allowed_offset", -1),
-                  kw.get("seed", 0), None, None, addr, early=addr + 8 * _EARLY if staged else None)
     wait, sp, laid = _C.host().sgl_wait_word, _C.stream_ptr(), None
-    if staged:
-        # laid out while the device merges the last list: a fifth of a small batch's time is the making of tensors
-        wait(addr + 8 * (_EARLY + last), 1, sp)
-        laid = db._trim_but_last(words[_EARLY:_EARLY + last])
-    wait(addr + 8 * (last + 1), 1, sp)
+    try:
+        db = _enqueue(g, roots, root_ts, fanouts, policy, g.ts_min, g.ts_max, kw.get("equal_root_time", False), kw.get("allowed_offset", -1),
+                      kw.get("seed", 0), None, None, addr, early=addr + 8 * _EARLY if staged else None)
+        if staged:
+            # laid out while the device merges the last list: a fifth of a small batch's time is the making of tensors
+            wait(addr + 8 * (_EARLY + last), 1, sp)
+            laid = db._trim_but_last(words[_EARLY:_EARLY + last])
+        wait(addr + 8 * (last + 1), 1, sp)
+    except BaseException:
+        _C.abandon()
+        raise
     host, bits = words[:last], words[last] & 0xFFFFFFFF
     if bits & 2:
         g.__dict__["_queried_outside"] = True

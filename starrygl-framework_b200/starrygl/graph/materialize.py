@@ -117,7 +117,7 @@ class MaterializedMultiLayerBuilder:
         """Batch, then the plan of every layer list, all enqueued without a host round trip; the arrays that are there before the last list
         is merged cross PCIe next to that merge and the plans (8,000 roots, two hops, 8 MB: 437 us, so 390 - 407), the others after one
         read-back of every size."""
-        g, L, P, hops = self.g, _C.lib(), self.num_parts, len(fanouts)
+        g, P, hops = self.g, self.num_parts, len(fanouts)
         if ts_range is None:
             ts_range = _root_range(g, root_ts)
         planned = self.rep_table is not None and self.node_parts is not None and P > 1
@@ -126,36 +126,12 @@ class MaterializedMultiLayerBuilder:
         lo, hi = _graph_range(g, *ts_range)
         addr, result = _C.host_words()
         staged = hops > 0 and roots.numel() > 0 and meta.numel() < _EARLY and _EARLY + nb < _READY
-        db = _enqueue(g, roots, root_ts, fanouts, policy, lo, hi, inclusive, -1, seed, None, None, None, meta[:nb], True,
-                      addr + 8 * _EARLY if staged else None, addr + 8 * _READY if staged else None)
-        lists = []                                  # (address of the ids, capacity) of every layer list
-        n = c = t = roots.numel()
-        place = db.addresses()
-        lists.append((place[0], c))
-        for l, k in enumerate(fanouts):
-            t *= k
-            c += t
-            lists.append((place[3 + 14 * l + 6], c))
-        plans = []
-        if planned:
-            caps = [max(c * max(P - 1, 1), 1) for _, c in lists]
-            room = torch.empty(3 * sum(caps), dtype=torch.int64, device=self.device)
-            rt, sp, mp, at = self.rep_table, _C.stream_ptr(), meta.data_ptr(), room.data_ptr()
-            for cap in caps:
-                plans.append((at, cap))
-                at += 24 * cap
-            k = len(lists)
-            words = C.c_int64 * k
-            ids, ns, cp = words(*[a for a, _ in lists]), words(*[c for _, c in lists]), words(*caps)
-            d_ns, outs = words(*[mp + 16 * i for i in range(k)]), words(*[a for a, _ in plans])
-            cnts = words(*[mp + 8 * (nb + i * (P + 1)) for i in range(k)])
-            ref = C.addressof
-            ws = _C.WORKSPACE.get(_C.host().sgl_plan_routes_ws_bytes(k, ref(ns), ref(cp)), self.device, sp)
-            _C.host().sgl_plan_routes(k, ref(ids), ref(ns), ref(d_ns), self.node_parts.data_ptr(), self.node_parts.numel(), self.pid,
-                                      rt.indptr.data_ptr(), rt.indices.data_ptr(), rt.locs.data_ptr(), P, ref(cp), ref(outs), ref(cnts),
-                                      mp + 8 * (nb - 1), ws.data_ptr(), ws.numel(), sp)
         early = copies = None
         try:
+            db = _enqueue(g, roots, root_ts, fanouts, policy, lo, hi, inclusive, -1, seed, None, None, None, meta[:nb], True,
+                          addr + 8 * _EARLY if staged else None, addr + 8 * _READY if staged else None)
+            n, place = roots.numel(), db.addresses()
+            plans, room = self._plan(place, n, fanouts, meta) if planned else ([], None)
             if staged:
                 sp, wait = _C.stream_ptr(), _C.host().sgl_wait_word
                 wait(addr + 8 * (_EARLY + nb - 1), 1, sp)
@@ -166,9 +142,39 @@ class MaterializedMultiLayerBuilder:
                     with _C.on_stream(copies):
                         early = list(zip(picks, self._export([p[2:] for p in picks], lambda: wait(addr + 8 * _READY, 1, sp))))
             return self._finish(db, meta, place, n, hops, plans, early)
+        except BaseException:
+            _C.abandon()
+            raise
         finally:
             if copies is not None:                  # (whatever becomes of the slot: they write to memory of its own)
                 copies.synchronize()
+
+    def _plan(self, place, n, fanouts, meta):
+        """Enqueues the route plan of every layer list; sizes go behind the batch's counts in ``meta``.  Returns (address, capacity) of
+        every plan's arrays and the tensor that holds them."""
+        P, nb = self.num_parts, 2 + 2 * len(fanouts)
+        lists, c, t = [(place[0], n)], n, n         # (address of the ids, capacity) of every layer list
+        for l, k in enumerate(fanouts):
+            t *= k
+            c += t
+            lists.append((place[3 + 14 * l + 6], c))
+        caps = [max(c * max(P - 1, 1), 1) for _, c in lists]
+        room = torch.empty(3 * sum(caps), dtype=torch.int64, device=self.device)
+        rt, sp, mp, at, plans = self.rep_table, _C.stream_ptr(), meta.data_ptr(), room.data_ptr(), []
+        for cap in caps:
+            plans.append((at, cap))
+            at += 24 * cap
+        k = len(lists)
+        words = C.c_int64 * k
+        ids, ns, cp = words(*[a for a, _ in lists]), words(*[c for _, c in lists]), words(*caps)
+        d_ns, outs = words(*[mp + 16 * i for i in range(k)]), words(*[a for a, _ in plans])
+        cnts = words(*[mp + 8 * (nb + i * (P + 1)) for i in range(k)])
+        ref = C.addressof
+        ws = _C.WORKSPACE.get(_C.host().sgl_plan_routes_ws_bytes(k, ref(ns), ref(cp)), self.device, sp)
+        _C.host().sgl_plan_routes(k, ref(ids), ref(ns), ref(d_ns), self.node_parts.data_ptr(), self.node_parts.numel(), self.pid,
+                                  rt.indptr.data_ptr(), rt.indices.data_ptr(), rt.locs.data_ptr(), P, ref(cp), ref(outs), ref(cnts),
+                                  mp + 8 * (nb - 1), ws.data_ptr(), ws.numel(), sp)
+        return plans, room
 
     def _copies(self):
         """The calling thread's stream for copies next to what its current stream does."""

@@ -260,6 +260,11 @@ static int build_batch(const int64_t* indptr, const int64_t* nbr, const int64_t*
       if (forked) SGL_CHECK_RC(order.mark(kCsc, side));
     }
     if (host_ready && l + 1 == n_hops) {
+      // (behind the columns of the hop before too: they are translated on the main stream, next to this hop's CSC)
+      if (forked && l > 0) {
+        SGL_CHECK_RC(order.mark(kFork, stream));
+        SGL_CHECK_RC(order.wait(kFork, side));
+      }
       SGL_CHECK_RC(export_words(meta, host_ready, 0, l > 0 ? side : stream));
       host_ready = nullptr;
     }

@@ -16,6 +16,8 @@
  *   - Counts that are only known on the device (the number of edges a hop produced) can be chained to
  *     the next call through `d_n` parameters: a device int64 that overrides the host count, which then
  *     only acts as the capacity the launch is sized for.
+ *   - sgl_build_batch*, sgl_query*: refused with SGL_ERR_ARG, _WORKSPACE or _UNSUPPORTED they have started nothing.  After
+ *     SGL_ERR_CUDA, of any entry point, work may be running: its arrays may be freed or reused once the stream has been waited for.
  *   - Callable from any host thread (no Python, no global locks); the device of the pointers must be
  *     current on the calling thread.
  *

@@ -178,6 +178,46 @@ static int build_batch(const int64_t* indptr, const int64_t* nbr, const int64_t*
   SGL_REQUIRE(n_roots >= 0 && n_hops >= 0 && (n_hops == 0 || fanouts), SGL_ERR_ARG, "build_batch: bad size");
   for (int l = 0; l < n_hops; ++l) SGL_REQUIRE(fanouts[l] >= 1, SGL_ERR_ARG, "build_batch: fanout=%d must be >= 1", fanouts[l]);
   SGL_REQUIRE(meta, SGL_ERR_ARG, "build_batch: meta is null");
+  // The root list starts before the hops are set up (flush, below): what a hop refuses is refused here, before anything runs.
+  struct Hop {
+    int64_t *nbr, *dst, *ts, *eid, *offs, *gids, *gts, *col, *indptr, *indices, *cts, *ceid;
+    float *dt, *cdt;
+  };
+  const std::unique_ptr<Hop[]> hop(new (std::nothrow) Hop[n_hops + 1]);
+  SGL_REQUIRE(hop, SGL_ERR_ARG, "build_batch: no host memory for %d hops", n_hops);
+  int64_t *cur_id = nullptr, *cur_ts = nullptr, *inv = nullptr;
+  if (n_roots > 0) {
+    SGL_REQUIRE(section_at && roots && root_ts && (n_hops == 0 || (indptr && nbr && ts && eid)), SGL_ERR_ARG, "build_batch: null array");
+    constexpr int64_t kMost = (int64_t)1 << 32;
+    int64_t t = n_roots, c = n_roots;
+    for (int l = 0; l < n_hops; ++l) {
+      SGL_CHECK_RC(check_sampling(fanouts[l], policy, t));
+      SGL_REQUIRE(t < kMost && fanouts[l] <= kMost / t && c + t * fanouts[l] < kMost, SGL_ERR_UNSUPPORTED,
+                  "build_batch: hop %d: edges and list entries need 64-bit positions", l);
+      SGL_REQUIRE(l == 0 || bits_for((uint64_t)c) + ts_bits <= 64, SGL_ERR_UNSUPPORTED,
+                  "build_batch: hop %d: rows and times (%d bits) exceed the 64-bit sort key", l, ts_bits);
+      t *= fanouts[l];
+      c += t;
+    }
+    SGL_REQUIRE(ws_bytes >= sgl_build_batch_ws_bytes(n_roots, fanouts, n_hops), SGL_ERR_WORKSPACE, "build_batch: workspace %zu < %zu bytes",
+                ws_bytes, sgl_build_batch_ws_bytes(n_roots, fanouts, n_hops));
+    int sec = 0;
+    auto take = [&]() -> int64_t* {
+      const int64_t at = section_at[sec++];
+      return (int64_t*)(at >= 0 ? (uintptr_t)base + (uintptr_t)at * 8 : (uintptr_t)other_base + (uintptr_t)(-1 - at) * 8);
+    };
+    cur_id = take(); cur_ts = take(); inv = take();
+    bool all = cur_id && cur_ts;
+    for (int l = 0; l < n_hops; ++l) {
+      Hop& h = hop[l];
+      h.nbr = take(); h.dst = take(); h.ts = take(); h.dt = (float*)take(); h.eid = take(); h.offs = take();
+      h.gids = take(); h.gts = take(); h.col = take();
+      h.indptr = take(); h.indices = take(); h.cts = take(); h.cdt = (float*)take(); h.ceid = take();
+      all = all && h.nbr && h.dst && h.ts && h.dt && h.eid && h.offs && h.gids && h.gts && (h.col || n_hops == 1) &&
+            (l == 0 || (h.indptr && h.indices && h.cts && h.cdt && h.ceid));
+    }
+    SGL_REQUIRE(all, SGL_ERR_ARG, "build_batch: null section");
+  }
   LaunchScope scope(stream);
   SGL_CHECK_RC(zero_async(meta, (size_t)(2 + 2 * n_hops) * sizeof(int64_t), stream));
   auto done = [&]() -> int {
@@ -187,37 +227,16 @@ static int build_batch(const int64_t* indptr, const int64_t* nbr, const int64_t*
     return scope.submit();
   };
   if (n_roots == 0) return done();
-  SGL_REQUIRE(section_at && roots && root_ts, SGL_ERR_ARG, "build_batch: null array");
-  SGL_REQUIRE(ws_bytes >= sgl_build_batch_ws_bytes(n_roots, fanouts, n_hops), SGL_ERR_WORKSPACE, "build_batch: workspace %zu < %zu bytes",
-              ws_bytes, sgl_build_batch_ws_bytes(n_roots, fanouts, n_hops));
   if (d_status == nullptr) d_status = (int32_t*)(meta + 1 + 2 * n_hops);
   const size_t swb = sample_ws(n_roots, fanouts, n_hops), lwb = list_ws(n_roots, fanouts, n_hops), cwb = csc_ws(n_roots, fanouts, n_hops);
   void *sws = ws, *lws = (char*)ws + swb, *cws = (char*)lws + lwb;
   char* ows = (char*)cws + cwb;
   uint32_t* const cols32 = (uint32_t*)(ows + order_ws(n_roots, fanouts, n_hops));
   RowOrder order_of{};                   // of the layer list merged last, where the next CSC goes along it
-  int sec = 0;
-  auto take = [&]() -> int64_t* {
-    const int64_t at = section_at[sec++];
-    return (int64_t*)(at >= 0 ? (uintptr_t)base + (uintptr_t)at * 8 : (uintptr_t)other_base + (uintptr_t)(-1 - at) * 8);
-  };
-  int64_t *cur_id = take(), *cur_ts = take(), *inv = take();
   int rc = sgl_unique_pairs(roots, root_ts, n_roots, nullptr, nullptr, nullptr, 0, nullptr, id_bits, ts_bits, ts_base, cur_id, cur_ts, inv,
                             nullptr, meta, d_status, lws, lwb, stream);
   if (rc) return rc;
   if (n_hops > 0) SGL_CHECK_RC(scope.flush());             // (600 roots 50.3 -> 46.5 us a batch, 4,096 roots two hops 143 -> 134)
-  struct Hop {
-    int64_t *nbr, *dst, *ts, *eid, *offs, *gids, *gts, *col, *indptr, *indices, *cts, *ceid;
-    float *dt, *cdt;
-  };
-  const std::unique_ptr<Hop[]> hop(new (std::nothrow) Hop[n_hops + 1]);
-  SGL_REQUIRE(hop, SGL_ERR_ARG, "build_batch: no host memory for %d hops", n_hops);
-  for (int l = 0; l < n_hops; ++l) {
-    Hop& h = hop[l];
-    h.nbr = take(); h.dst = take(); h.ts = take(); h.dt = (float*)take(); h.eid = take(); h.offs = take();
-    h.gids = take(); h.gts = take(); h.col = take();
-    h.indptr = take(); h.indices = take(); h.cts = take(); h.cdt = (float*)take(); h.ceid = take();
-  }
   auto sample = [&](int l, const int64_t* tgt, const int64_t* tgt_ts, int64_t n, const int64_t* d_n, cudaStream_t on) {
     const Hop& h = hop[l];
     return sample_layer(indptr, nbr, ts, eid, fence, num_nodes, tgt, tgt_ts, n, d_n, fanouts[l], policy, equal_root_time, allowed_offset, 0,

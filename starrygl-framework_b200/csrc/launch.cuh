@@ -87,7 +87,7 @@ class LaunchScope {
   int submit();
   // Submits what was collected so far and goes on collecting (nothing in an inner scope): the device starts on it while the host
   // still adds and sets up the rest, which takes 0.6 us a kernel and 5 us a launch.  For a beginning of 10 - 15 us that everything else
-  // waits for; all refusals that must leave no trace come before it.
+  // waits for.  Arguments are checked before it, those of what follows too: a call that is refused has started nothing.
   int flush();
 
  private:

@@ -279,6 +279,9 @@ struct SeedsSink {
   }
 };
 
+// What relabel_nodes refuses whatever its arrays: for entry points that start work before they set up the relabels.
+int check_relabel(int64_t n, int64_t num_nodes);
+
 // sgl_relabel_nodes for lists that continue each other: with d_start, out_new_ids[0] is the id of local number *d_start.
 int relabel_nodes(const int64_t* ids, int64_t n, const int64_t* d_n, int64_t num_nodes, int64_t* mapper, int64_t* mask, int64_t epoch,
                   int64_t* d_next_local, int64_t* out_local, int64_t* out_new_ids, int64_t* d_n_new, const int64_t* d_start,

@@ -133,6 +133,14 @@ extern "C" int sgl_query_at(const int64_t* indptr, const int64_t* nbr, const int
               SGL_ERR_ARG, "query: null array");
   SGL_REQUIRE(ws_bytes >= sgl_query_ws_bytes(cap, n_neg, fanout, n_hops), SGL_ERR_WORKSPACE, "query: workspace %zu < %zu bytes", ws_bytes,
               sgl_query_ws_bytes(cap, n_neg, fanout, n_hops));
+  // The seeds start before the hops are set up (flush, below): what a hop refuses is refused here, before anything runs.
+  SGL_REQUIRE(n_hops == 0 || (indptr && nbr && ts && eid), SGL_ERR_ARG, "query: null array");
+  SGL_CHECK_RC(check_relabel(cap, num_nodes));
+  for (int64_t l = 0, q = cap + n_neg; l < n_hops; ++l, q *= fanout) {
+    SGL_CHECK_RC(check_sampling(fanout, policy, q));
+    SGL_REQUIRE(fanout <= INT64_MAX / (q > 0 ? q : 1), SGL_ERR_UNSUPPORTED, "query: too many edges");
+    SGL_CHECK_RC(check_relabel(q * fanout, num_nodes));
+  }
   SGL_CHECK_RC(order_after(stream, (cudaStream_t)producer));
   int sec = 0;
   auto take = [&]() -> int64_t* { return (int64_t*)((uintptr_t)base + (uintptr_t)section_at[sec++] * 8); };

@@ -429,13 +429,20 @@ int sgl::build_csc_rows(const RowOrder& ro, int64_t list_cap, const int64_t* row
 
 extern "C" size_t sgl_relabel_nodes_ws_bytes(int64_t n) { return list_ws_bytes(n); }
 
+int sgl::check_relabel(int64_t n, int64_t num_nodes) {
+  SGL_REQUIRE(n >= 0 && num_nodes >= 0, SGL_ERR_ARG, "relabel_nodes: negative size");
+  SGL_REQUIRE(bits_for(num_nodes > 0 ? (uint64_t)(num_nodes - 1) : 0) < 63, SGL_ERR_UNSUPPORTED, "relabel_nodes: num_nodes too large");
+  SGL_REQUIRE(by_bitmap(n, num_nodes) || n < ((int64_t)1 << 32), SGL_ERR_UNSUPPORTED, "relabel_nodes: %lld entries need a 64-bit position", (long long)n);
+  return SGL_OK;
+}
+
 int sgl::relabel_nodes(const int64_t* ids, int64_t n, const int64_t* d_n, int64_t num_nodes, int64_t* mapper,
                                  int64_t* mask, int64_t epoch, int64_t* d_next_local, int64_t* out_local,
                                  int64_t* out_new_ids, int64_t* d_n_new, const int64_t* d_start, int32_t* d_status, void* ws, size_t ws_bytes,
                                  void* stream_) {
   SGL_NVTX("sgl_relabel_nodes");
   cudaStream_t stream = (cudaStream_t)stream_;
-  SGL_REQUIRE(n >= 0 && num_nodes >= 0, SGL_ERR_ARG, "relabel_nodes: negative size");
+  SGL_CHECK_RC(check_relabel(n, num_nodes));
   SGL_REQUIRE(d_next_local && d_n_new, SGL_ERR_ARG, "relabel_nodes: null counter");
   if (n == 0) {
     SGL_CHECK_RC(zero_async(d_n_new, sizeof(int64_t), stream));
@@ -443,7 +450,6 @@ int sgl::relabel_nodes(const int64_t* ids, int64_t n, const int64_t* d_n, int64_
   }
   SGL_REQUIRE(ids && mapper && mask && out_local && out_new_ids, SGL_ERR_ARG, "relabel_nodes: null array");
   const int id_bits = bits_for(num_nodes > 0 ? (uint64_t)(num_nodes - 1) : 0);
-  SGL_REQUIRE(id_bits < 63, SGL_ERR_UNSUPPORTED, "relabel_nodes: num_nodes too large");
   LaunchScope scope(stream);
   if (by_bitmap(n, num_nodes)) {
     WsCarver c(ws, ws_bytes);

@@ -565,6 +565,15 @@ static int launch_sample(const SampleArgs& a, cudaStream_t stream, int64_t* host
              : launch(sample_fill_kernel<CT, FT, false>, fill_ctas, kCtaThreads, smem, stream, a, (int)ctas);
 }
 
+int sgl::check_sampling(int fanout, int policy, int64_t n_targets) {
+  SGL_REQUIRE(fanout >= 1, SGL_ERR_ARG, "sample_layer: fanout=%d must be >= 1", fanout);
+  SGL_REQUIRE(policy == SGL_POLICY_RECENT || policy == SGL_POLICY_UNIFORM, SGL_ERR_ARG, "sample_layer: unknown policy %d", policy);
+  SGL_REQUIRE(policy != SGL_POLICY_UNIFORM || fanout <= SGL_MAX_UNIFORM_FANOUT, SGL_ERR_UNSUPPORTED, "sample_layer: uniform fanout %d > %d", fanout,
+              SGL_MAX_UNIFORM_FANOUT);
+  SGL_REQUIRE(n_targets < ((int64_t)1 << 34), SGL_ERR_UNSUPPORTED, "sample_layer: too many targets");
+  return SGL_OK;
+}
+
 int sgl::sample_layer(const int64_t* indptr, const int64_t* nbr, const int64_t* ts, const int64_t* eid, const int64_t* fence,
                       int64_t num_nodes, const int64_t* targets, const int64_t* target_ts, int64_t n_targets, const int64_t* d_n,
                       int fanout, int policy, int equal_root_time, int64_t allowed_offset, int keep_root_time, uint64_t seed,
@@ -574,13 +583,8 @@ int sgl::sample_layer(const int64_t* indptr, const int64_t* nbr, const int64_t* 
   SGL_NVTX("sgl_sample_layer");
   cudaStream_t stream = (cudaStream_t)stream_;
   SGL_REQUIRE(n_targets >= 0 && num_nodes >= 0, SGL_ERR_ARG, "sample_layer: negative size");
-  SGL_REQUIRE(fanout >= 1, SGL_ERR_ARG, "sample_layer: fanout=%d must be >= 1", fanout);
-  SGL_REQUIRE(policy == SGL_POLICY_RECENT || policy == SGL_POLICY_UNIFORM, SGL_ERR_ARG,
-              "sample_layer: unknown policy %d", policy);
-  SGL_REQUIRE(policy != SGL_POLICY_UNIFORM || fanout <= SGL_MAX_UNIFORM_FANOUT, SGL_ERR_UNSUPPORTED,
-              "sample_layer: uniform fanout %d > %d", fanout, SGL_MAX_UNIFORM_FANOUT);
+  SGL_CHECK_RC(check_sampling(fanout, policy, n_targets));
   SGL_REQUIRE(out_offsets, SGL_ERR_ARG, "sample_layer: out_offsets is null");
-  SGL_REQUIRE(n_targets < ((int64_t)1 << 34), SGL_ERR_UNSUPPORTED, "sample_layer: too many targets");
   if (n_targets == 0) {
     SGL_CHECK_RC(zero_async(out_offsets, sizeof(int64_t), stream));
     if (total_out) SGL_CHECK_RC(zero_async(total_out, sizeof(int64_t), stream));

@@ -4,6 +4,9 @@
 #include "common.cuh"
 
 namespace sgl {
+// What sample_layer refuses whatever its arrays: for entry points that start work before they set up the hops.
+int check_sampling(int fanout, int policy, int64_t n_targets);
+
 int sample_layer(const int64_t* indptr, const int64_t* nbr, const int64_t* ts, const int64_t* eid, const int64_t* fence,
                  int64_t num_nodes, const int64_t* targets, const int64_t* target_ts, int64_t n_targets, const int64_t* d_n, int fanout,
                  int policy, int equal_root_time, int64_t allowed_offset, int keep_root_time, uint64_t seed, uint32_t rng_stream,

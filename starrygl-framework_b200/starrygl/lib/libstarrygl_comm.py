@@ -569,7 +569,7 @@ class CUDAGraph:
                 fanout, layers, _C.POLICY[stype], eq, off, keep, ops.bits_for(g.num_nodes - 1), ops.bits_for(g.ts_max - g.ts_min), g.ts_min,
                 rl.mapper, rl.mask, epoch, op == "f", rl.next_local, at, words, meta, slot[0], plan.ws_bytes, producer, st.stream_id,
                 st.device_index, st.device_type, sp)
-        except BaseException:             # nothing was enqueued: the numbering goes on as it was
+        except BaseException:             # refused before anything ran: the numbering goes on as it was
             _FREE_SLOTS.append(slot)
             raise
         buf = own if buf is None else buf

@@ -101,6 +101,31 @@ uint64_t integer(PyObject* o) {
   return v;
 }
 
+// a size: beyond 64 bits it is refused, where an argument of the C functions is taken modulo 2^64 (as ctypes does)
+int64_t size(PyObject* o) {
+  PyObject* const n = must(PyNumber_Index(o));
+  const long long v = PyLong_AsLongLong(n);
+  Py_DECREF(n);
+  if (v == -1 && PyErr_Occurred()) throw Raised();
+  return v;
+}
+
+bool truth(PyObject* o) {
+  const int v = PyObject_IsTrue(o);
+  if (v < 0) throw Raised();
+  return v != 0;
+}
+
+int64_t sum(int64_t a, int64_t b) {
+  if (__builtin_add_overflow(a, b, &a)) throw Refused("a size beyond 64 bits");
+  return a;
+}
+
+int64_t product(int64_t a, int64_t b) {
+  if (__builtin_mul_overflow(a, b, &a)) throw Refused("a size beyond 64 bits");
+  return a;
+}
+
 template <class T>
 T argument(PyObject* o) {
   if constexpr (std::is_pointer_v<T>) {
@@ -389,7 +414,7 @@ PyObject* mail_reduce(PyObject*, Args a, Py_ssize_t n_args) {
     }
     Py_DECREF(seq);
     at::Tensor index = fresh(cap, at::kLong, dev), out_ts = fresh(cap, at::kFloat, dev), d_u = fresh(1, at::kLong, dev), pos, mail;
-    if (argument<int>(a[5])) pos = fresh(cap, at::kLong, dev);
+    if (truth(a[5])) pos = fresh(cap, at::kLong, dev);
     if (!dims.empty()) mail = at::empty({cap, width}, at::TensorOptions().dtype(at::kFloat).device(dev));
     const int64_t *const pa = (const int64_t*)ptr(ids_a), *const pb = n_b ? (const int64_t*)ptr(ids_b) : nullptr;
     const void* const times = ptr(ts);
@@ -427,7 +452,7 @@ PyObject* mailbox_write(PyObject*, Args a, Py_ssize_t n_args) {
     const float *const p_rows = (const float*)ptr(rows), *const p_times = (const float*)ptr(times);
     float *const p_box = (float*)ptr(box), *const p_box_ts = (float*)ptr(box_ts);
     int64_t* const p_next = next.defined() ? (int64_t*)ptr(next) : nullptr;
-    const int advance = argument<int>(a[7]);
+    const bool advance = truth(a[7]);
     int32_t* const status = argument<int32_t*>(a[8]);
     void* const on = stream();
     int rc;
@@ -447,14 +472,14 @@ PyObject* sample_layer(PyObject*, Args a, Py_ssize_t n_args) {
   return guarded([&]() -> PyObject* {
     count("sample_layer", n_args, 20);
     const at::Tensor targets = i64(a[6]), target_ts = i64(a[7]);
-    const int64_t n = targets.numel(), fanout = argument<int64_t>(a[8]);
+    const int64_t n = targets.numel(), fanout = size(a[8]);
     if (target_ts.numel() != n) throw Refused("sample_layer: targets and target_ts differ in length");
     const at::Tensor& indptr = tensor(a[0]);
     const at::Device dev = indptr.device();
-    const int64_t cap = n * fanout > 1 ? n * fanout : 1;
+    const int64_t edges = product(n, fanout), cap = edges > 1 ? edges : 1;
     at::Tensor nbr = fresh(cap, at::kLong, dev), dst = fresh(cap, at::kLong, dev), ts = fresh(cap, at::kLong, dev), eid = fresh(cap, at::kLong, dev),
                dt = fresh(cap, at::kFloat, dev), offs = fresh(n + 1, at::kLong, dev), dti;
-    if (argument<int>(a[16])) dti = fresh(cap, at::kLong, dev);
+    if (truth(a[16])) dti = fresh(cap, at::kLong, dev);
     const int64_t *const g_ptr = (const int64_t*)ptr(indptr), *const g_nbr = optional<int64_t>(a[1]), *const g_ts = optional<int64_t>(a[2]),
                   *const g_eid = optional<int64_t>(a[3]), *const g_fence = optional<int64_t>(a[4]);
     const int64_t *const t = (const int64_t*)ptr(targets), *const tt = (const int64_t*)ptr(target_ts), *const d_n = optional<int64_t>(a[10]);
@@ -484,13 +509,13 @@ PyObject* tcsr_build(PyObject*, Args a, Py_ssize_t n_args) {
   return guarded([&]() -> PyObject* {
     count("tcsr_build", n_args, 7);
     const at::Tensor key = i64(a[0]), nbr = i64(a[1]), ts = i64(a[2]), eid = a[3] == Py_None ? at::Tensor() : i64(a[3]);
-    const int64_t m = key.numel(), num_nodes = argument<int64_t>(a[4]);
+    const int64_t m = key.numel(), num_nodes = size(a[4]);
     if (nbr.numel() != m || ts.numel() != m || (eid.defined() && eid.numel() != m)) throw Refused("tcsr_build: edge arrays differ in length");
     const at::Device dev = key.device();
-    at::Tensor indptr = fresh(num_nodes + 1, at::kLong, dev), o_nbr = fresh(m, at::kLong, dev), o_ts = fresh(m, at::kLong, dev),
+    at::Tensor indptr = fresh(sum(num_nodes, 1), at::kLong, dev), o_nbr = fresh(m, at::kLong, dev), o_ts = fresh(m, at::kLong, dev),
                o_eid = fresh(m, at::kLong, dev), perm, fence;
-    if (argument<int>(a[5])) perm = fresh(m, at::kLong, dev);
-    if (argument<int>(a[6]) && m && num_nodes) fence = fresh(sgl_tcsr_fence_len(num_nodes, m), at::kLong, dev);
+    if (truth(a[5])) perm = fresh(m, at::kLong, dev);
+    if (truth(a[6]) && m && num_nodes) fence = fresh(sgl_tcsr_fence_len(num_nodes, m), at::kLong, dev);
     auto words = [](const at::Tensor& t) { return t.defined() ? (int64_t*)ptr(t) : nullptr; };
     const int64_t *const k = words(key), *const p_nbr = words(nbr), *const p_ts = words(ts), *const p_eid = words(eid);
     int64_t *const p_ptr = words(indptr), *const q_nbr = words(o_nbr), *const q_ts = words(o_ts), *const q_eid = words(o_eid), *const q_perm = words(perm),

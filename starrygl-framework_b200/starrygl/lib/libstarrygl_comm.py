@@ -508,7 +508,8 @@ class CUDAGraph:
         """Host-known bounds of the window's events: (first, at most) from every 256th timestamp of the stream."""
         if self._ev_index is None:
             with torch.cuda.stream(self.stream):      # (events out of order are still being sorted there)
-                self._ev_index = self.ev[1][::256].tolist()      # (a list: what is looked up in an array is made an object first)
+                # (a view of the copy: a look-up costs 0.3 us, in an array 1.0; a list is made in 0.14 ms for 2 M events, in 5 for 50 M)
+                self._ev_index = memoryview(self.ev[1][::256].cpu().numpy())
         idx, m = self._ev_index, self.ev[1].numel()
         first = max(bisect_left(idx, t0) - 1, 0) * 256
         last = min(bisect_left(idx, t1) * 256, m)

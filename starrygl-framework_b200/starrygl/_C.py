@@ -15,7 +15,7 @@ import torch
 
 _PKG_ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 LIB_PATH = os.path.join(_PKG_ROOT, "lib", "libsgl_b200.so")
-HOST_PATH = os.path.join(_PKG_ROOT, "lib", "_sgl_host.so")
+HOST_PATH = os.path.join(_PKG_ROOT, "lib", f"_sgl_host.{torch.__version__}.{sys.implementation.cache_tag}.so")     # (as build.host_path)
 
 SGL_DEV_BITS = {1: "node id out of range", 2: "timestamp outside the declared window", 4: "row index out of range",
                 8: "output capacity exceeded", 16: "device-side wait timed out",
@@ -182,7 +182,7 @@ def host():
             if _host is None:
                 lib()
                 if not os.path.exists(HOST_PATH):
-                    raise RuntimeError(f"{HOST_PATH} is missing: build it with `python starrygl-framework_b200/build.py`")
+                    raise RuntimeError(f"{HOST_PATH} is missing: build it for this torch with `python starrygl-framework_b200/build.py`")
                 spec = importlib.util.spec_from_file_location("_sgl_host", HOST_PATH)
                 m = importlib.util.module_from_spec(spec)
                 spec.loader.exec_module(m)

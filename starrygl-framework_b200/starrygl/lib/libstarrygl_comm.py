@@ -19,7 +19,6 @@ hop l at the time of the edge that reached it (or at the root's time with ``keep
 import ctypes as C
 import queue
 import threading
-import weakref
 from bisect import bisect_left
 from collections import deque
 from typing import List, Optional
@@ -68,6 +67,37 @@ class NegativeRoot:
         return f"<NegativeRoot with {self.root_num} roots>"
 
 
+class _Sizes:
+    """What a result and its hops share: where the sizes (of the hops, of the pieces of the id map) are on the device, and not the arrays --
+    a result holds its hops, and a hop that held the result would keep both, and the arrays of every other hop, until a garbage collection."""
+
+    def __init__(self):
+        self.status = None               # device status word of the graph that produced the result
+        self.counts, self.known = [], []           # device counts (until they are read), and sizes (None: not read yet)
+
+    def add(self, d_total) -> int:
+        self.counts.append(d_total)
+        self.known.append(None)
+        return len(self.known) - 1
+
+    def read(self):
+        """One read-back of all sizes that are not known yet."""
+        counts = [d for d in self.counts if d is not None]
+        if not counts:
+            return
+        if self.status is not None:      # the kernels' error bits ride along in the same copy
+            counts.append(self.status.t.to(torch.int64))
+        host = torch.cat(counts).tolist()
+        if self.status is not None:
+            bits = int(host.pop())
+            if bits:
+                self.status.t.zero_()
+                raise _C.SglError(f"sampling: device status {bits} ({_C.decode_status(bits)})")
+        for i, d in enumerate(self.counts):
+            if d is not None:
+                self.known[i], self.counts[i] = host.pop(0), None
+
+
 class TemporalNeighbor:
     """One hop: query q owns ``neighbors[root_start_ptr[q]:root_end_ptr[q]]`` (``root_start_ptr`` is the full
     exclusive prefix with one extra entry, ``root_end_ptr`` its shift by one).
@@ -80,25 +110,23 @@ class TemporalNeighbor:
 
     def __init__(self, hop: ops.Hop, owner: "TemporalResult" = None, n_queries: Optional[int] = None):
         self.hop = hop
-        # (not the result itself: the two would hold each other, and with them the arrays of every hop, until a garbage collection)
-        self._owner = None if owner is None else weakref.ref(owner)
-        self._status = None if owner is None else owner._status
-        self._before = owner.neighbors_list[-1] if owner is not None and owner.neighbors_list else None
+        self._sizes = None if owner is None else owner._sizes
+        self._at = None if owner is None else owner._sizes.add(hop.d_total)
+        last = owner.neighbors_list[-1] if owner is not None and owner.neighbors_list else None
+        self._at_before = last._at if last is not None and last._sizes is self._sizes else None
         self._n = None                  # number of sampled neighbours, once known on the host
         self._nq = n_queries            # number of queries (None: known only once the previous hop has been cut)
         self._neighbors_override = None
 
     def _cut(self) -> int:
         if self._n is None:
-            owner = None if self._owner is None else self._owner()
-            if owner is not None:
-                owner.materialize()
-            else:
-                if self._status is not None:
-                    self._status.check("sampling")
-                if self._nq is None and self._before is not None:
-                    self._nq = self._before._cut()
+            if self._sizes is None:
                 self._n = self.hop.total()
+            else:
+                self._sizes.read()
+                self._n = self._sizes.known[self._at]
+                if self._nq is None and self._at_before is not None:      # queries of hop l = neighbours of hop l - 1
+                    self._nq = self._sizes.known[self._at_before]
         return self._n
 
     @classmethod
@@ -158,9 +186,17 @@ class TemporalResult:
         self.roots = roots
         self.neg_roots = neg_roots
         self.neighbors_list: List[TemporalNeighbor] = []
-        self._remap_pieces = []          # (new global ids at capacity, device count) per relabelled list
+        self._remap_pieces = []          # (new global ids at capacity, where among the sizes their number is) per relabelled list
         self._remapper = None
-        self._status = None              # device status word of the graph that produced the result
+        self._sizes = _Sizes()
+
+    @property
+    def _status(self):
+        return self._sizes.status
+
+    @_status.setter
+    def _status(self, word):
+        self._sizes.status = word
 
     @property
     def neighbors(self):
@@ -168,30 +204,15 @@ class TemporalResult:
 
     def materialize(self):
         """The one read-back of a result: the sizes of every hop (and of every piece of the id map) in a single copy."""
-        hops = [nb for nb in self.neighbors_list if nb._n is None]
-        counts = [nb.hop.d_total for nb in hops] + [d for _, d in self._remap_pieces]
-        if not counts:
-            return
-        if self._status is not None:     # the kernels' error bits ride along in the same copy
-            counts = counts + [self._status.t.to(torch.int64)]
-        host = torch.cat(counts).tolist()
-        if self._status is not None:
-            bits = int(host.pop())
-            if bits:
-                self._status.t.zero_()
-                raise _C.SglError(f"sampling: device status {bits} ({_C.decode_status(bits)})")
-        for nb, n in zip(hops, host):
-            nb._n = int(n)
+        self._sizes.read()
         prev = None
         for nb in self.neighbors_list:      # queries of hop l+1 = neighbours of hop l
+            nb._cut()
             if nb._nq is None and prev is not None:
                 nb._nq = prev._n
             prev = nb
         if self._remap_pieces:
-            sizes = host[len(hops):]
-            dev = self.roots.roots.device
-            self._remapper = (torch.cat([ids[:int(c)] for (ids, _), c in zip(self._remap_pieces, sizes)])
-                              if sizes else _empty(dev))
+            self._remapper = torch.cat([ids[:self._sizes.known[i]] for ids, i in self._remap_pieces])
             self._remap_pieces = []
 
     @property
@@ -467,11 +488,11 @@ class CUDAGraph:
         pieces = result._remap_pieces
         loc, new_ids, d_new = self.relabel.insert(result.roots.roots, status=self.status)
         result.roots = TemporalRoot(loc, result.roots.ts_ptr, result.roots.ts, result.roots.q_ptr, result.roots.q_eid)
-        pieces.append((new_ids, d_new))
+        pieces.append((new_ids, result._sizes.add(d_new)))
         for nb in result.neighbors_list:      # capacity arrays + device counts: no read-back between the hops
             loc, new_ids, d_new = self.relabel.insert(nb.hop.nbr, d_n=nb.hop.d_total, status=self.status)
             nb.neighbors = loc
-            pieces.append((new_ids, d_new))
+            pieces.append((new_ids, result._sizes.add(d_new)))
 
     # ---- asynchronous queue ----------------------------------------------------------------------------------
     def submit_query(self, time_start, time_end, chunk_list, test_generate_samples, test_generate_samples_ts,

@@ -1,5 +1,7 @@
 #include "launch.cuh"
 
+#include <memory>
+
 namespace sgl {
 namespace {
 
@@ -89,9 +91,13 @@ int one_by_one(cudaStream_t stream) {
 
 int build(Cached& c) {
   const LaunchList& l = t_state.list;
+  std::vector<cudaGraphNode_t> nodes(l.used), deps;
+  // (before there is a graph: an entry with one has all of its notes, also after a failed allocation)
+  c.set.assign(l.used, {});
+  for (size_t i = 0; i < l.used; ++i) changed(c, i);
   cudaGraph_t graph = nullptr;
   SGL_CUDA_CHECK(cudaGraphCreate(&graph, 0));
-  std::vector<cudaGraphNode_t> nodes(l.used), deps;
+  std::unique_ptr<CUgraph_st, decltype(&cudaGraphDestroy)> made(graph, &cudaGraphDestroy);
   cudaError_t e = cudaSuccess;
   for (size_t i = 0; i < l.used && e == cudaSuccess; ++i) {
     deps.clear();
@@ -102,16 +108,13 @@ int build(Cached& c) {
   cudaGraphExec_t exec = nullptr;
   if (e == cudaSuccess) e = cudaGraphInstantiate(&exec, graph, 0);
   if (e != cudaSuccess) {
-    cudaGraphDestroy(graph);
     cudaGetLastError();
     c.refused = true;
     return SGL_OK;
   }
-  c.graph = graph;
+  c.graph = made.release();
   c.exec = exec;
   c.nodes = std::move(nodes);
-  c.set.resize(l.used);
-  for (size_t i = 0; i < l.used; ++i) changed(c, i);
   return SGL_OK;
 }
 

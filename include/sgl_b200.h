@@ -72,7 +72,8 @@ int sgl_radix_sort_u64_u32(uint64_t* keys, uint32_t* vals, uint64_t* keys_alt, u
                            int num_bits, int* h_result_in_alt, void* ws, size_t ws_bytes, void* stream);
 int64_t sgl_look_back_limit(int64_t ns);
 /* Composite entry points are submitted as one executable graph from the second call of a sequence of kernels on a stream on;
- * how many of them the calling thread holds (at most 32). */
+ * how many of them the calling thread holds (at most 32, and as many for the beginnings of batches and queries, which are submitted ahead
+ * of the rest and not counted here). */
 int sgl_launch_graphs(void);
 
 /* ------------------------------------------------------------------------------------------------

@@ -5,9 +5,11 @@
 namespace sgl {
 namespace {
 
-constexpr size_t kMaxGraphs = 32;     // per thread; the least recently used one makes room
+// per thread and kind (whole calls or the rest of one, beginnings that were submitted ahead): the least recently used one makes room
+constexpr size_t kMaxGraphs = 32;
 
 struct Cached {
+  bool ahead;                         // the beginning of a call
   int device;
   cudaStream_t stream;
   std::vector<const void*> funcs;
@@ -28,7 +30,7 @@ struct Thread {
   LaunchScope* open = nullptr;
   int plain = 0;
   LaunchList list;
-  std::vector<Cached*> graphs;
+  std::vector<Cached*> graphs;        // of both kinds
   uint64_t clock = 0;
   std::vector<void*> params;
   ~Thread() {
@@ -38,8 +40,8 @@ struct Thread {
 
 thread_local Thread t_state;
 
-bool same(const Cached& c, int device, cudaStream_t stream, const LaunchList& l) {
-  if (c.device != device || c.stream != stream || c.funcs.size() != l.used) return false;
+bool same(const Cached& c, bool ahead, int device, cudaStream_t stream, const LaunchList& l) {
+  if (c.ahead != ahead || c.device != device || c.stream != stream || c.funcs.size() != l.used) return false;
   for (size_t i = 0; i < l.used; ++i)
     if (c.funcs[i] != l.nodes[i].func || c.deps[i] != l.nodes[i].deps) return false;
   return true;
@@ -209,20 +211,20 @@ int LaunchScope::submit() {
   if (!owner_) return SGL_OK;
   owner_ = false;
   t_state.open = nullptr;
-  return no_throw([&] { return submit_list(); });
+  return no_throw([&] { return submit_list(false); });
 }
 
 int LaunchScope::flush() {
   if (!owner_) return SGL_OK;
   return no_throw([&] {
-    const int rc = submit_list();
+    const int rc = submit_list(true);
     t_state.list.clear();
     tails_.clear();                      // (what follows comes after all of it, in stream order)
     return rc;
   });
 }
 
-int LaunchScope::submit_list() {
+int LaunchScope::submit_list(bool ahead) {
   Thread& t = t_state;
   LaunchList& l = t.list;
   if (l.used == 0) return SGL_OK;
@@ -232,20 +234,24 @@ int LaunchScope::submit_list() {
   ++t.clock;
   Cached* c = nullptr;
   for (Cached* g : t.graphs)
-    if (same(*g, device, main_, l)) {
+    if (same(*g, ahead, device, main_, l)) {
       c = g;
       break;
     }
   if (c == nullptr) {
-    if (t.graphs.size() >= kMaxGraphs) {
-      size_t oldest = 0;
-      for (size_t i = 1; i < t.graphs.size(); ++i)
-        if (t.graphs[i]->last_use < t.graphs[oldest]->last_use) oldest = i;
+    size_t kind = 0, oldest = t.graphs.size();
+    for (size_t i = 0; i < t.graphs.size(); ++i) {
+      if (t.graphs[i]->ahead != ahead) continue;
+      ++kind;
+      if (oldest == t.graphs.size() || t.graphs[i]->last_use < t.graphs[oldest]->last_use) oldest = i;
+    }
+    if (kind >= kMaxGraphs) {
       Cached* old = t.graphs[oldest];
       delete old;
       t.graphs.erase(t.graphs.begin() + oldest);
     }
     c = new Cached;
+    c->ahead = ahead;
     c->device = device;
     c->stream = main_;
     for (size_t i = 0; i < l.used; ++i) {
@@ -276,7 +282,7 @@ int LaunchScope::submit_list() {
 
 extern "C" int sgl_launch_graphs(void) {
   int n = 0;
-  for (const sgl::Cached* c : sgl::t_state.graphs) n += c->exec != nullptr ? 1 : 0;
+  for (const sgl::Cached* c : sgl::t_state.graphs) n += c->exec != nullptr && !c->ahead ? 1 : 0;
   return n;
 }
 

@@ -91,7 +91,7 @@ class LaunchScope {
   int flush();
 
  private:
-  int submit_list();
+  int submit_list(bool ahead);
   bool owner_;
   cudaStream_t main_;
   struct Tail {

@@ -44,12 +44,13 @@ struct Digit {
 
 // Digit totals of every pass, each first.bits further up: one shared-memory counter table per pass.  A warp whose keys all carry the
 // same digit (high digits of a hub, ordered input) adds once.  Items that are checked on the way (Items::kChecked, edges) have check(i)
-// called once each, the words or-ed, and the result given to checked(); of their groups of 32 only the first that are alike are looked for.
+// called once each and the words or-ed; where refuses() says so of the result, *stop is set and the passes do nothing.  Of their groups of
+// 32 only the first that are alike are looked for.
 // 50 M edges: 276 us with their ids read (466 with a look at every group; 274 with that and the ids left to the scan, which took 262 and
 // not 184 us then); pairs of a batch, skewed in some groups and not in others, 14 M and 3.8 M: 181 us with a look at every group, 202.
 template <class Items>
 __global__ void __launch_bounds__(kHistThreads)
-lsd_hist_kernel(Items items, Digit first, int passes, unsigned long long* __restrict__ hist, int64_t* d_count) {
+lsd_hist_kernel(Items items, Digit first, int passes, unsigned long long* __restrict__ hist, int64_t* d_count, unsigned int* stop) {
   __shared__ uint32_t s_hist[kMaxPasses * kRadix];
   const int64_t n = items.begin();
   if (d_count && blockIdx.x == 0 && threadIdx.x == 0) *d_count = n;      // for the kernels behind the first pass
@@ -102,7 +103,8 @@ lsd_hist_kernel(Items items, Digit first, int passes, unsigned long long* __rest
   __syncthreads();
   for (int j = threadIdx.x; j < passes * kRadix; j += kHistThreads)
     if (s_hist[j]) atomicAdd(&hist[j], (unsigned long long)s_hist[j]);
-  if constexpr (Items::kChecked) items.checked(check);
+  if constexpr (Items::kChecked)
+    if (items.refuses(check)) *(volatile unsigned int*)stop = 1u;
 }
 
 // totals -> starts, one CTA per pass
@@ -126,6 +128,7 @@ struct LsdSmem {
   uint32_t cnt[kLsdWarps][kRadix];         // keys of the digit in the warp so far, then where the warp's start in the tile
   uint32_t out[kRadix];                    // global position of the tile's digit run minus its position in the tile (mod 2^32)
   int ticket;
+  unsigned int stop;
 };
 
 // Sum of what the tiles before this one hold of digit threadIdx.x; publishes it with the tile's own.
@@ -214,20 +217,25 @@ template <class V, class Items, class Out, bool kLoop>
 __global__ void __launch_bounds__(kLsdThreads, kLsdCtas)
 lsd_pass_kernel(Items items, Digit digit, int pass,
                 const unsigned long long* __restrict__ starts, unsigned int* __restrict__ ticket, uint64_t* state,
-                Out out, unsigned long long limit, unsigned int* gave_up, int32_t* d_status) {
+                Out out, unsigned long long limit, unsigned int* gave_up, const unsigned int* __restrict__ stop, int32_t* d_status) {
   extern __shared__ __align__(16) unsigned char smem[];
   LsdSmem<V>& sm = *(LsdSmem<V>*)smem;
   constexpr int kItems = kLsdItems<V>, kTile = kLsdTile<V>;
   const int64_t n = items.begin();
   if ((int64_t)blockIdx.x * kTile >= n) return;            // (capacity beyond the count; the others share the tickets)
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  if (tid == 0) sm.ticket = (int)atomicAdd(ticket, 1u);
+  if (tid == 0) {
+    const unsigned int s = *stop;        // (on its way together with the ticket; the same for all CTAs of a pass)
+    sm.ticket = (int)atomicAdd(ticket, 1u);
+    sm.stop = s;
+  }
   do {
     for (int j = tid; j < kLsdWarps * kRadix / 4; j += kLsdThreads) {
       ((uint4*)&sm.mask[0][0])[j] = make_uint4(0, 0, 0, 0);
       ((uint4*)&sm.cnt[0][0])[j] = make_uint4(0, 0, 0, 0);
     }
     __syncthreads();
+    if (sm.stop) break;
     const int tile = sm.ticket;
     const int64_t tile_base = (int64_t)tile * kTile;
     if (kLoop && tile_base >= n) break;
@@ -489,7 +497,7 @@ inline size_t lsd_ws_bytes(int64_t n) {
 
 // Sorts on key bits [first_bit, num_bits), at least one pass; the first pass reads from `items`, writes to (k1, v1), the next to
 // (k0, v0) and so on; *in_first says whether the result ends in (k1, v1).  With a `last` of another type than ArrayOut the last
-// pass writes there instead and its arrays stay free.  **gave_up on the device: a look-back ran into its time limit, the result
+// pass writes there instead and its arrays stay free.  Items that are refused (see lsd_hist_kernel) are not sorted.  **gave_up on the device: a look-back ran into its time limit, the result
 // is not to be used as positions.  d_n: number of items on the device (<= n); d_count: the count kernel writes it there, from items.
 template <class V, class Items, class Last, bool kLoop = false>
 int lsd_sort(const Items& items, uint64_t* k1, V* v1, uint64_t* k0, V* v0, int64_t n, const int64_t* d_n, int64_t* d_count, int first_bit, int num_bits,
@@ -502,11 +510,12 @@ int lsd_sort(const Items& items, uint64_t* k1, V* v1, uint64_t* k0, V* v0, int64
   unsigned long long* hist = c.take<unsigned long long>(kMaxPasses * kRadix + kMaxPasses);
   unsigned int* tickets = (unsigned int*)(hist + kMaxPasses * kRadix);
   *gave_up = tickets + kMaxPasses;
+  unsigned int* const stop = *gave_up + 1;
   uint64_t* state = c.take<uint64_t>((size_t)tiles * kRadix);
   SGL_REQUIRE(c.ok(), SGL_ERR_WORKSPACE, "radix sort: workspace too small for %lld keys", (long long)n);
   SGL_CHECK_RC(zero_async(hist, (size_t)((char*)(state + (size_t)tiles * kRadix) - (char*)hist), stream));     // (one behind the other)
   SGL_CHECK_RC(launch(lsd_hist_kernel<Items>, stream_grid(n, kHistThreads * 16, 4), kHistThreads, 0, stream, items, Digit{first_bit, bits},
-                      passes, hist, d_count));
+                      passes, hist, d_count, stop));
   SGL_CHECK_RC(launch(lsd_scan_kernel, passes, kRadix, 0, stream, hist));
   for (int p = 0; p < passes; ++p) {
     const Array out{p & 1 ? k0 : k1, p & 1 ? v0 : v1};
@@ -518,7 +527,7 @@ int lsd_sort(const Items& items, uint64_t* k1, V* v1, uint64_t* k0, V* v0, int64
       SGL_CUDA_CHECK(allow_smem((const void*)lsd_pass_kernel<V, From, To, kLoop>, done, sizeof(LsdSmem<V>)));
       const unsigned ctas = (unsigned)(kLoop && tiles > kNumSM * kLsdCtas ? kNumSM * kLsdCtas : tiles);
       return launch(lsd_pass_kernel<V, From, To, kLoop>, ctas, kLsdThreads, sizeof(LsdSmem<V>), stream, from, Digit{first_bit + p * bits, bits}, p,
-                    hist + p * kRadix, tickets + p, state, to, look_back_ns(), *gave_up, d_status);
+                    hist + p * kRadix, tickets + p, state, to, look_back_ns(), *gave_up, stop, d_status);
     };
     const bool to_last = !kArray && p == passes - 1;
     if (p == 0) SGL_CHECK_RC(to_last ? pass(items, last) : pass(items, out));

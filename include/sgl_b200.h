@@ -62,7 +62,8 @@ const char* sgl_build_info(void);
  * *h_result_in_alt tells whether the sorted data are in (keys, vals) [0] or in (keys_alt, vals_alt) [1].
  * Lists above 1,212,416 keys: the passes wait for each other's tiles, for 2 s at most; the call waits for their end and returns
  * SGL_ERR_CUDA if one gave up (a capturing stream: not reported).  sgl_look_back_limit sets that limit, in nanoseconds, for the
- * calls that the calling thread makes from then on (negative: unchanged) and returns the one before.
+ * calls that the calling thread makes from then on (negative: unchanged; 0: a sort of several tiles gives up whether it would have
+ * waited or not) and returns the one before.
  * Replaces: thrust::sort calls in csrc/include/starrygl/sample.cu.hpp:1078, :1197, :1795.
  * ---------------------------------------------------------------------------------------------- */
 size_t sgl_radix_sort_ws_bytes(int64_t n);

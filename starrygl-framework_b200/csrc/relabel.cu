@@ -65,7 +65,8 @@ constexpr int64_t kMaxRowTargets = 32;
 constexpr int kMapFanout = 32;
 inline int64_t rows_ctas(int64_t cap) { return (cap + kRowTile - 1) / kRowTile < 1 ? 1 : (cap + kRowTile - 1) / kRowTile; }
 
-// start[at]: edges of the items before `at` in its tile; sums: edges before the tile; from[at]: first edge of the item, and their number.
+// start[at]: edges of the items before `at` in its tile; sums: edges before the tile; from[at]: first edge of the item, and their number
+// (32 bits each: build_csc_rows takes fewer than 2^32 edges).
 // Targets of `drawn` or more edges may have drawn them.
 __global__ void __launch_bounds__(kThreads)
 csc_rows_count_kernel(const RowOrder ro, const int64_t* d_rows, const int64_t* __restrict__ offsets, int drawn, uint32_t* __restrict__ start,
@@ -397,6 +398,9 @@ int sgl::build_csc_rows(const RowOrder& ro, int64_t list_cap, const int64_t* row
                         const int64_t* d_n_edges, int64_t num_dst, const int64_t* d_num_dst, int dst_bits, int ts_bits, int64_t ts_base, int64_t* out_indptr, int64_t* out_indices,
                         int64_t* out_ts, float* out_dt, int64_t* out_eid, int32_t* d_status, void* ws, size_t ws_bytes, void* stream_) {
   cudaStream_t stream = (cudaStream_t)stream_;
+  // (list items and, in `from`, first edges of targets are 32-bit words; the sort of a row with too many targets has the same limit)
+  SGL_REQUIRE(n_edges >= 0 && n_edges < ((int64_t)1 << 32) && list_cap < ((int64_t)1 << 32), SGL_ERR_UNSUPPORTED,
+              "build_csc: %lld edges of %lld list items need 64-bit positions", (long long)n_edges, (long long)list_cap);
   SGL_REQUIRE(dst_bits >= 0 && ts_bits >= 0 && dst_bits + ts_bits <= 64, SGL_ERR_UNSUPPORTED,
               "build_csc: dst_bits %d + ts_bits %d exceed the 64-bit sort key", dst_bits, ts_bits);
   LaunchScope scope(stream);

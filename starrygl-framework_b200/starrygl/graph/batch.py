@@ -311,10 +311,10 @@ def build_batch(g, roots, root_ts, fanouts, policy="recent", **kw) -> List[dict]
     if last + 2 > len(words):
         return build_batch_async(g, roots, root_ts, fanouts, policy, **kw).finish()
     staged = bool(fanouts) and roots.numel() > 0 and last + 2 <= _EARLY
-    wait, sp, laid = _C.host().sgl_wait_word, _C.stream_ptr(), None
     try:
         db = _enqueue(g, roots, root_ts, fanouts, policy, g.ts_min, g.ts_max, kw.get("equal_root_time", False), kw.get("allowed_offset", -1),
                       kw.get("seed", 0), None, None, addr, early=addr + 8 * _EARLY if staged else None)
+        wait, sp, laid = _C.host().sgl_wait_word, _C.stream_ptr(), None     # (not in front of it: the device waits for nothing else)
         if staged:
             # laid out while the device merges the last list: a fifth of a small batch's time is the making of tensors
             wait(addr + 8 * (_EARLY + last), 1, sp)

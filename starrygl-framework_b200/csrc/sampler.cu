@@ -279,13 +279,14 @@ sample_count_kernel(const SampleArgs a) {
 // copy loop is then a handful of instructions around its three loads.  (It was issue bound: 100 - 170 instructions per edge,
 // 384,000 x 20 recent 101 us, a drawn hop of 4.2 M x 10 targets 458 us.)
 constexpr int kMapFanout = 32;
-// COPY: windows that are copied, up to kMapFanout edges each.  Without draws the kernel needs few registers, and the copy wants CTAs
-// (384,000 x 20 recent: one kernel for both, 62 registers, 90.6 us; bounded to six CTAs per SM 84.7, to eight 84.5, four elements in flight
-// per thread 86 - 111; 32, 128 and 256 targets per CTA 85, 86, 90).  Everything else keeps the kernel for both: one for draws alone was
-// slower (uniform, 16,384 targets: fan-out 33 53.2 -> 59.4 us, 100 158 -> 175), and so were six CTAs where there is no map (recent, 65,536
-// targets, fan-out 100: 70.3 -> 71.8).
-template <int CT, int FT, bool COPY>
-__global__ void __launch_bounds__(kCtaThreads, COPY ? 6 : 0)
+// Without draws the kernel needs few registers, and the copy wants CTAs (384,000 x 20 recent: one kernel for both, 62 registers, 90.6 us;
+// bounded to six CTAs per SM 84.7, to eight 84.5, four elements in flight per thread 86 - 111; 32, 128 and 256 targets per CTA 85, 86, 90).
+// Targets that draw, a lane each, were no faster with more CTAs and spills (in the code for both: uniform, 40,000 targets, fan-out 33
+// 176 -> 191 us).  A warp per target wants the CTAs, and draws best in the code for both: 40 registers, by itself 62 (uniform, 16,384 targets,
+// fan-out 33 59.4 us, so 53.6, 100 175 and 152).
+enum Fill { kCopies, kDraws, kEither };
+template <int CT, int FT, Fill MODE>
+__global__ void __launch_bounds__(kCtaThreads, MODE == kCopies ? 6 : MODE == kDraws ? 4 : 0)
 sample_fill_kernel(const SampleArgs a, int count_ctas) {
   static_assert(CT % FT == 0 && CT <= kCtaThreads && FT % kWarpsPerCta == 0, "fill CTAs tile the count CTAs");
   constexpr bool kLaneDraws = CT != kWarpsPerCta;          // picks by the target's lane instead of its warp
@@ -333,7 +334,7 @@ sample_fill_kernel(const SampleArgs a, int count_ctas) {
     base = a.cta_sums[count_cta];
     if (threadIdx.x == 0 && first + FT >= a.n_cap && a.total_out) *a.total_out = a.out_offsets[a.n_cap];
   }
-  const bool draws = !COPY && a.policy == SGL_POLICY_UNIFORM, has_map = COPY || fanout <= kMapFanout;
+  const bool draws = MODE == kEither ? a.policy == SGL_POLICY_UNIFORM : MODE == kDraws, has_map = fanout <= kMapFanout;
   const bool drawn = draws && cut - lo > fanout;           // (of this thread's target)
   if (mine) {
     s_ex[slot] = ex;
@@ -560,9 +561,9 @@ static int launch_sample(const SampleArgs& a, cudaStream_t stream, int64_t* host
   }
   if (a.fanout <= kMapFanout) smem += (size_t)FT * a.fanout;
   const unsigned fill_ctas = (unsigned)((a.n_cap + FT - 1) / FT);
-  return a.policy != SGL_POLICY_UNIFORM && a.fanout <= kMapFanout
-             ? launch(sample_fill_kernel<CT, FT, true>, fill_ctas, kCtaThreads, smem, stream, a, (int)ctas)
-             : launch(sample_fill_kernel<CT, FT, false>, fill_ctas, kCtaThreads, smem, stream, a, (int)ctas);
+  constexpr Fill kUniform = CT == kWarpsPerCta ? kEither : kDraws;
+  return a.policy == SGL_POLICY_UNIFORM ? launch(sample_fill_kernel<CT, FT, kUniform>, fill_ctas, kCtaThreads, smem, stream, a, (int)ctas)
+                                        : launch(sample_fill_kernel<CT, FT, kCopies>, fill_ctas, kCtaThreads, smem, stream, a, (int)ctas);
 }
 
 int sgl::check_sampling(int fanout, int policy, int64_t n_targets) {

@@ -24,7 +24,7 @@ def reference(table, ts, idx, rounds):
         idx = (idx + 2) % (table.shape[0] - 1)
 
 
-@pytest.mark.parametrize("dim", [1, 3, 100, 128, 186])      # 4-byte pieces, 16-byte pieces, the bulk copy
+@pytest.mark.parametrize("dim", [1, 3, 100, 128, 186])      # 4-byte pieces (1, 3, 186), the bulk copy
 @pytest.mark.parametrize("captured", [False, True])
 def test_each_round_sees_the_last_one(dim, captured):
     rows, n, rounds = 40_001, 8_000, 12

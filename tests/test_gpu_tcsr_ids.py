@@ -1,5 +1,5 @@
-"""T-CSR builds by radix passes (above 1,212,416 edges): ids beyond 32 bits anywhere in the input, among the first 303,104 edges that the
-scan looks at or behind them; skewed and ordered keys, for which a warp's digits are counted together."""
+"""T-CSR builds by radix passes (above 1,212,416 edges): ids beyond 32 bits anywhere in the input, among the first and last 303,104 edges that
+the scan looks at or between them; skewed and ordered keys, for which a warp's digits are counted together."""
 import numpy as np
 import pytest
 import torch

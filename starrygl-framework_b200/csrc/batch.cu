@@ -286,6 +286,8 @@ static int build_batch(const int64_t* indptr, const int64_t* nbr, const int64_t*
       }
       SGL_CHECK_RC(export_words(meta, host_ready, 0, l > 0 ? side : stream));
       host_ready = nullptr;
+      // (launched one by one, a stream of the caller's: it has to be joined behind this too; a chain of a graph needs no end)
+      if (forked && l > 0 && LaunchScope::current() == nullptr) SGL_CHECK_RC(order.mark(kCsc, side));
     }
     order_of = RowOrder{};
     if (l + 1 < n_hops && by_rows(e * fanouts[l + 1])) {
